@@ -1,0 +1,709 @@
+// Flash attention backward for sm_100a on tcgen05 tensor cores.
+//
+// Scores are computed transposed (rows = keys, columns = queries), so that the probabilities and
+// their gradients come out in the layout the products over queries read as their A operand:
+//     S^T  = K Q^T                      P^T  = exp2(S^T c - lse2)
+//     dP^T = V dO^T                     dS^T = P^T (dP^T - delta) scale
+//     dV += P^T dO     A = P^T straight from TMEM (16-bit), never in shared memory
+//     dK += dS^T Q     A = dS^T in shared memory, K-major
+//     dQ  = dS K       A = the same dS^T tile, read as an MN-major operand
+// Queries lie along the N side of the first two products and along the reduction of the next two,
+// so a ragged last query tile (ViT: 257 = 2 x 128 + 1) costs what its rows cost, not a full tile.
+//
+// One CTA per SM walks over (key tile, head, batch) items; roles of its 16 warps:
+//   warps 0-7    softmax side: thread <-> key row (TMEM lane), each warp half of the 128 queries
+//   warps 8-11   drain: dQ tiles out of TMEM into the fp32 sums (TMA reduce-add through swizzled
+//                boxes), and dK / dV at the end of an item while the next item is under way
+//   warp 12      TMA producer      warp 13  MMA issuer (one lane), TMEM owner (14, 15: idle)
+// What bounds it: per 128 x 128 tile pair 16384 exponentials (1024 cycles of the special-function
+// units) against 5 products (1400 cycles at head dim 64, 2560 at 128), so the tensor core must
+// never wait for the element-wise part.  Order of the MMA warp for tile i:
+//   head dim <= 64   S(i+1) as soon as S(i) is in registers, dV(i), dP(i+1), dK(i), dQ(i)
+//   96               S(i+1) as soon as S(i) is in registers, dV(i), dQ(i), dK(i), dP(i+1)
+//   128              dV(i), dQ(i), S(i+1), dK(i), dP(i+1)
+// TMEM (512 columns): S^T 128, dP^T 128, P^T 64 (16-bit), dV, dK, dQ one head dim each.  At 96 dQ
+// takes the columns of dP^T (dead once dS^T is in shared memory; the next dP^T waits until dQ is
+// drained), at 128 P^T also takes the columns of S^T.
+//
+// Measured (B200, CUDA events, L2 flushed, with the pre- and post-pass), against one CTA per key
+// tile that ran the five products and the element-wise part one after the other with scalar
+// reductions into dQ: [4, 4096, 10, 64] 1330 -> 877 us, [2, 2048, 16, 128] 445 -> 261,
+// causal [1, 2048, 32, 128] 302 -> 155, [24, 257, 16, 88] 192 -> 146.
+//
+// A pre-pass writes per query tile the row statistics [128 lse2 | 128 delta scale] (+inf / 0 beyond
+// the last query, which makes the probabilities there zero without a test) and clears the fp32 dQ
+// sums; a post-pass converts them.  With one key tile the dQ tiles are complete and go straight to
+// their 16-bit destination: no sums, no post-pass.
+#include "attn_common.cuh"
+#include "api.h"
+
+namespace pf {
+
+struct AttnBwdParams {
+  int B, H, Sq, Sk, D;
+  int causal;
+  float scale;
+  int fmt;              // 0 fp16, 1 bf16
+  const float* stats;   // [B*H][query tiles][256]: lse * log2(e), then delta * scale
+  void *dq, *dk, *dv;   // strides (batch, seq, head) in elements
+  long long sdq[3], sdkv[3];
+  int direct_dq;        // one key tile: dQ tiles are written as they are
+  int n_kt, n_qt;
+  int* status;
+};
+
+// One 8-lane group per (batch, padded query, head): delta = dO . O, statistics, cleared dQ sums.
+template <typename T>
+__global__ void __launch_bounds__(256)
+attn_bwd_prep_kernel(const T* __restrict__ dout, const T* __restrict__ out,
+                     const float* __restrict__ lse, float* __restrict__ stats,
+                     float* __restrict__ dq_accum, int B, int S, int H, int D, int n_qt,
+                     float scale) {
+  const int lane = threadIdx.x & 31, sub = lane & 7;
+  const long long g = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * 4 + (lane >> 3);
+  const int s_pad = n_qt * ATT_BM;
+  const bool in = g < (long long)B * s_pad * H;
+  const int h = in ? (int)(g % H) : 0;
+  const long long bs = g / H;
+  const int i = in ? (int)(bs % s_pad) : 0;
+  const long long b = in ? bs / s_pad : 0;
+  const bool live = in && i < S;
+  const long long row = (b * S + i) * H + h;
+  float s = 0.f;
+  if (live) {
+    const uint4* a = reinterpret_cast<const uint4*>(dout + row * D);
+    const uint4* c = reinterpret_cast<const uint4*>(out + row * D);
+    for (int v = sub; v < D / 8; v += 8) {
+      const uint4 ua = __ldg(a + v), uc = __ldg(c + v);
+      const T* ea = reinterpret_cast<const T*>(&ua);
+      const T* ec = reinterpret_cast<const T*>(&uc);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) s = fmaf(to_f32<T>(ea[j]), to_f32<T>(ec[j]), s);
+      if (dq_accum) {
+        float4* z = reinterpret_cast<float4*>(dq_accum + row * D) + 2 * v;
+        z[0] = make_float4(0.f, 0.f, 0.f, 0.f);
+        z[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    }
+  }
+  s += __shfl_xor_sync(0xffffffffu, s, 4);
+  s += __shfl_xor_sync(0xffffffffu, s, 2);
+  s += __shfl_xor_sync(0xffffffffu, s, 1);
+  if (in && sub == 0) {
+    float* st = stats + (((b * H + h) * n_qt + i / ATT_BM) * 2) * ATT_BM + i % ATT_BM;
+    st[0] = live ? lse[(b * H + h) * S + i] * LOG2E : INFINITY;
+    st[ATT_BM] = live ? s * scale : 0.f;
+  }
+}
+
+// dq[b, i, h, :] (strided) = convert(acc[b, i, h, :]) ; acc is contiguous [B*Sq*H, D]
+template <typename T>
+__global__ void __launch_bounds__(256)
+attn_dq_convert_kernel(const float* __restrict__ acc, T* __restrict__ dq, long long rows, int D,
+                       int Sq, int H, long long sb, long long ss, long long sh) {
+  const int dv = D / 8;
+  const long long total = rows * dv;
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
+    const long long row = i / dv;
+    const int c = (int)(i - row * dv);
+    const int h = (int)(row % H);
+    const long long bs = row / H;
+    const int si = (int)(bs % Sq);
+    const long long b = bs / Sq;
+    const float4 a0 = reinterpret_cast<const float4*>(acc + row * D)[2 * c];
+    const float4 a1 = reinterpret_cast<const float4*>(acc + row * D)[2 * c + 1];
+    uint4 q;
+    q.x = pack2<T>(a0.x, a0.y); q.y = pack2<T>(a0.z, a0.w);
+    q.z = pack2<T>(a1.x, a1.y); q.w = pack2<T>(a1.z, a1.w);
+    reinterpret_cast<uint4*>(dq + b * sb + (long long)si * ss + (long long)h * sh)[c] = q;
+  }
+}
+
+template <int DP>
+struct BwdCfg {
+  static constexpr int NBLK = (DP + 63) / 64;
+  static constexpr int TILE = NBLK * ATT_BLK;
+  static constexpr bool ALIAS_P = DP > 96;     // P^T in the columns of S^T
+  static constexpr bool ALIAS_DQ = DP > 64;    // dQ in the columns of dP^T
+  static constexpr int DOST = NBLK == 1 ? 2 : 1;   // dO stages (Q always has two)
+  static constexpr int NDS = NBLK == 1 ? 2 : 1;    // dS^T buffers
+  static constexpr int DS_BYTES = 2 * ATT_BLK;
+  static constexpr int OFF_V = TILE;
+  static constexpr int OFF_Q = 2 * TILE;
+  static constexpr int OFF_DO = OFF_Q + 2 * TILE;
+  static constexpr int OFF_DS = OFF_DO + DOST * TILE;
+  static constexpr int OFF_STG = OFF_DS + NDS * DS_BYTES;   // 4 warps x 2 boxes of 4 KB
+  static constexpr int OFF_STAT = OFF_STG + 4 * 2 * 4096;   // 2 stages x 1 KB
+  static constexpr int OFF_BAR = OFF_STAT + 2 * 1024;
+  static constexpr int SMEM = OFF_BAR + 256;
+  static constexpr int T_S = 0, T_DP = 128;
+  static constexpr int T_P = ALIAS_P ? 0 : 256;
+  static constexpr int P_HALF = ALIAS_P ? 64 : 32;   // column distance of P^T's query halves
+  static constexpr int T_DV = ALIAS_P ? 256 : 320;
+  static constexpr int T_DK = T_DV + DP;
+  static constexpr int T_DQ = ALIAS_DQ ? T_DP : T_DK + DP;
+  // four warpgroups of 128 registers a thread at launch
+  static constexpr int THREADS = 512;
+  static constexpr int REGS_SOFTMAX = 152, REGS_DRAIN = 120, REGS_OTHER = 88;
+  static_assert(2 * REGS_SOFTMAX + REGS_DRAIN + REGS_OTHER <= 4 * 128, "registers of the block");
+  static_assert(SMEM <= 232448, "shared memory per CTA");
+  static_assert((ALIAS_DQ ? T_DK : T_DQ) + DP <= 512, "TMEM columns");
+};
+
+struct BwdItem {
+  int k0, h, b, q_begin, n;    // first key, first visible query tile, number of query tiles
+};
+// Items of round `r`.  Causal key tiles see fewer queries the later they start: the long ones are
+// dealt first (all heads of a key tile next to each other) and every other round runs backwards,
+// so that a CTA with a long item in one round gets a short one in the next.  Otherwise the key
+// tiles of a head are neighbours, which lets them share its Q / dO in L2.
+__device__ __forceinline__ int bwd_index(int r) {
+  const int slot = (r & 1) ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;
+  return r * (int)gridDim.x + slot;
+}
+__device__ __forceinline__ BwdItem bwd_item(const AttnBwdParams& p, int w) {
+  BwdItem it;
+  int kt, bh;
+  if (p.causal) { kt = w / (p.B * p.H); bh = w - kt * (p.B * p.H); }
+  else { bh = w / p.n_kt; kt = w - bh * p.n_kt; }
+  it.k0 = kt * ATT_BN;
+  it.h = bh % p.H;
+  it.b = bh / p.H;
+  it.q_begin = p.causal ? max(0, it.k0 - (p.Sk - p.Sq)) / ATT_BM : 0;
+  it.n = max(0, p.n_qt - it.q_begin);
+  return it;
+}
+
+template <typename T, int DP>
+__global__ void __launch_bounds__(BwdCfg<DP>::THREADS, 1)
+attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
+                   const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo,
+                   const __grid_constant__ CUtensorMap tdq, const AttnBwdParams p,
+                   const int n_items) {
+  using C = BwdCfg<DP>;
+  constexpr int NBLK = C::NBLK, TILE = C::TILE;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::OFF_BAR);
+  uint64_t* kv_full = bars;          // K and V of the item
+  uint64_t* kv_empty = bars + 1;     // every product of the item has completed
+  uint64_t* q_full = bars + 2;       // [2] Q tile and its row statistics
+  uint64_t* q_empty = bars + 4;      // [2] dK has read Q (1), the softmax warps the statistics (8)
+  uint64_t* do_full = bars + 6;      // [2]
+  uint64_t* do_empty = bars + 8;     // [2] dV has read dO
+  uint64_t* s_full = bars + 10;
+  uint64_t* s_empty = bars + 11;     // S^T is in registers (used when P^T has its own columns)
+  uint64_t* p_ready = bars + 12;
+  uint64_t* dv_done = bars + 13;     // dV(i) has read P^T
+  uint64_t* dp_full = bars + 14;
+  uint64_t* ds_ready = bars + 15;
+  uint64_t* ds_empty = bars + 16;    // [2] dK and dQ have read dS^T
+  uint64_t* dq_full = bars + 18;
+  uint64_t* dq_empty = bars + 19;
+  uint64_t* acc_full = bars + 20;    // dK / dV of the item are complete
+  uint64_t* acc_empty = bars + 21;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 22);
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // the 128-byte swizzle works on absolute shared-memory addresses
+  if ((smem_u32(smem) & 1023u) != 0u) {
+    if (tid == 0) report(p.status, PF_ERR_BAD_ARG);
+    return;
+  }
+  if (tid == 0) {
+    tma_prefetch_desc(&tq); tma_prefetch_desc(&tk); tma_prefetch_desc(&tv);
+    tma_prefetch_desc(&tdo); tma_prefetch_desc(&tdq);
+    for (int i = 0; i < 22; ++i) mbar_init(&bars[i], 1);
+    for (int i = 0; i < 2; ++i) mbar_init(&q_empty[i], 1 + 8);
+    mbar_init(s_empty, 8);
+    mbar_init(p_ready, 8);
+    mbar_init(ds_ready, 8);
+    mbar_init(dq_empty, 4);
+    mbar_init(acc_empty, 4);
+    mbar_fence_init();
+  }
+  if (warp == 13) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  const int shift = p.Sk - p.Sq;
+
+  // one split per warpgroup: its four warps execute the same instruction
+  if (warp >= 12) {
+    regs_dec<C::REGS_OTHER>();
+    if (warp == 12) {
+      // ---------------------------------------------------------------- TMA producer
+      if (lane == 0) {
+        uint32_t g = 0, items = 0;
+        bool ok = true;
+        for (int r = 0; ok && r * (int)gridDim.x < n_items; ++r) {
+          const int w = bwd_index(r);
+          if (w >= n_items) continue;
+          const BwdItem it = bwd_item(p, w);
+          if (it.n == 0) continue;
+          for (int i = 0; i < it.n && ok; ++i, ++g) {
+            const int q0 = (it.q_begin + i) * ATT_BM, st = g & 1, ds = g % C::DOST;
+            ok = mbar_wait(&q_empty[st], ((g >> 1) & 1) ^ 1, p.status, PF_ERR_TIMEOUT_EMPTY);
+            if (!ok) break;
+            mbar_expect_tx(&q_full[st], TILE + 1024);
+#pragma unroll
+            for (int c = 0; c < NBLK; ++c)
+              tma_load_4d(smem + C::OFF_Q + st * TILE + c * ATT_BLK, &tq, &q_full[st], c * 64, it.h,
+                          q0, it.b);
+            bulk_load(smem + C::OFF_STAT + st * 1024,
+                      p.stats + ((long long)(it.b * p.H + it.h) * p.n_qt + it.q_begin + i) * 256,
+                      1024, &q_full[st]);
+            if (i == 0) {
+              ok = mbar_wait(kv_empty, (items & 1) ^ 1, p.status, PF_ERR_TIMEOUT_EMPTY);
+              if (!ok) break;
+              mbar_expect_tx(kv_full, 2 * TILE);
+#pragma unroll
+              for (int c = 0; c < NBLK; ++c) {
+                tma_load_4d(smem + c * ATT_BLK, &tk, kv_full, c * 64, it.h, it.k0, it.b);
+                tma_load_4d(smem + C::OFF_V + c * ATT_BLK, &tv, kv_full, c * 64, it.h, it.k0, it.b);
+              }
+            }
+            ok = mbar_wait(&do_empty[ds], ((g / C::DOST) & 1) ^ 1, p.status, PF_ERR_TIMEOUT_EMPTY);
+            if (!ok) break;
+            mbar_expect_tx(&do_full[ds], TILE);
+#pragma unroll
+            for (int c = 0; c < NBLK; ++c)
+              tma_load_4d(smem + C::OFF_DO + ds * TILE + c * ATT_BLK, &tdo, &do_full[ds], c * 64,
+                          it.h, q0, it.b);
+          }
+          ++items;
+        }
+      }
+      __syncwarp();
+    } else if (warp == 13) {
+      // ---------------------------------------------------------------- MMA issuer
+      if (lane == 0) {
+        const uint32_t sK = smem_u32(smem), sV = smem_u32(smem + C::OFF_V);
+        const uint32_t sQ = smem_u32(smem + C::OFF_Q), sdO = smem_u32(smem + C::OFF_DO);
+        const uint32_t sdS = smem_u32(smem + C::OFF_DS);
+        const uint32_t id_kd = make_idesc_f16(128, DP, p.fmt, 0, 1);   // P^T dO, dS^T Q
+        const uint32_t id_dq = make_idesc_f16(128, DP, p.fmt, 1, 1);   // dS K
+        uint32_t g = 0, items = 0;
+        bool ok = true;
+        auto cols_of = [&](int qt) { return (min(ATT_BM, p.Sq - qt * ATT_BM) + 15) / 16 * 16; };
+        // S^T of query tile `qt`, global tile number gg.  The columns of S^T must be free: either
+        // the softmax warps hold the previous scores in registers, or (P^T in the same columns) the
+        // previous dV has read its probabilities.
+        auto issue_s = [&](uint32_t gg, int qt) -> bool {
+          const int st = gg & 1;
+          if (!mbar_wait(&q_full[st], (gg >> 1) & 1, p.status, PF_ERR_TIMEOUT_FULL)) return false;
+          if (gg > 0 && !mbar_wait(C::ALIAS_P ? dv_done : s_empty, (gg - 1) & 1, p.status,
+                                   PF_ERR_TIMEOUT_TMEM_EMPTY))
+            return false;
+          tc_fence_after();
+          mma_kk<DP / 16>(tmem + C::T_S, sK, sQ + st * TILE,
+                          make_idesc_f16(128, cols_of(qt), p.fmt, 0, 0), false);
+          tc_commit(s_full);
+          return true;
+        };
+        // dP^T; its columns are free once dS^T of the previous tile is ready (waited for by the
+        // caller), and when dQ shares them, once that has been drained
+        auto issue_dp = [&](uint32_t gg, int qt) -> bool {
+          const int st = gg % C::DOST;
+          if (!mbar_wait(&do_full[st], (gg / C::DOST) & 1, p.status, PF_ERR_TIMEOUT_FULL))
+            return false;
+          if (C::ALIAS_DQ && gg > 0 &&
+              !mbar_wait(dq_empty, (gg - 1) & 1, p.status, PF_ERR_TIMEOUT_TMEM_EMPTY))
+            return false;
+          tc_fence_after();
+          mma_kk<DP / 16>(tmem + C::T_DP, sV, sdO + st * TILE,
+                          make_idesc_f16(128, cols_of(qt), p.fmt, 0, 0), false);
+          tc_commit(dp_full);
+          return true;
+        };
+        for (int r = 0; ok && r * (int)gridDim.x < n_items; ++r) {
+          const int w = bwd_index(r);
+          if (w >= n_items) continue;
+          const BwdItem it = bwd_item(p, w);
+          if (it.n == 0) continue;
+          const int k_steps = (min(ATT_BN, p.Sk - it.k0) + 15) / 16;
+          ok = mbar_wait(kv_full, items & 1, p.status, PF_ERR_TIMEOUT_FULL) &&
+               issue_s(g, it.q_begin) && issue_dp(g, it.q_begin);
+          for (int i = 0; i < it.n && ok; ++i, ++g) {
+            const int qt = it.q_begin + i, st = g & 1, dst = g % C::DOST, dsb = g % C::NDS;
+            const int q_steps = cols_of(qt) / 16;
+            const bool more = i + 1 < it.n;
+            if (!C::ALIAS_P && more && !(ok = issue_s(g + 1, qt + 1))) break;
+            // ---- dV
+            ok = mbar_wait(p_ready, g & 1, p.status, PF_ERR_TIMEOUT_FULL);
+            if (ok && i == 0)
+              ok = mbar_wait(acc_empty, (items & 1) ^ 1, p.status, PF_ERR_TIMEOUT_TMEM_EMPTY);
+            if (!ok) break;
+            tc_fence_after();
+#pragma unroll 1
+            for (int k = 0; k < q_steps; ++k)
+              tc_mma_f16_ts(tmem + C::T_DV, tmem + C::T_P + (k >> 2) * C::P_HALF + (k & 3) * 8,
+                            make_desc_sw128(sdO + dst * TILE + k * 2048, ATT_BLK, 1024), id_kd,
+                            i > 0 || k > 0);
+            tc_commit(&do_empty[dst]);
+            tc_commit(dv_done);
+            ok = mbar_wait(ds_ready, g & 1, p.status, PF_ERR_TIMEOUT_FULL);
+            if (!ok) break;
+            const uint32_t ds_tile = sdS + dsb * C::DS_BYTES;
+            auto issue_dk = [&]() {
+              tc_fence_after();
+              mma_k_mn(tmem + C::T_DK, ds_tile, sQ + st * TILE, id_kd, i > 0, q_steps);
+              tc_commit(&q_empty[st]);
+            };
+            auto issue_dq = [&]() {
+              tc_fence_after();
+              mma_mn_mn(tmem + C::T_DQ, ds_tile, sK, id_dq, false, k_steps);
+              tc_commit(dq_full);
+            };
+            if (C::ALIAS_DQ) {
+              issue_dq();
+              if (C::ALIAS_P && more && !(ok = issue_s(g + 1, qt + 1))) break;
+              issue_dk();
+              tc_commit(&ds_empty[dsb]);
+              if (more && !(ok = issue_dp(g + 1, qt + 1))) break;
+            } else {
+              if (more && !(ok = issue_dp(g + 1, qt + 1))) break;
+              issue_dk();
+              if (g > 0) ok = mbar_wait(dq_empty, (g - 1) & 1, p.status, PF_ERR_TIMEOUT_TMEM_EMPTY);
+              if (!ok) break;
+              issue_dq();
+              tc_commit(&ds_empty[dsb]);
+            }
+            if (!more) { tc_commit(acc_full); tc_commit(kv_empty); }
+          }
+          ++items;
+        }
+      }
+      __syncwarp();
+    }
+  } else if (warp >= 8) {
+    // ---------------------------------------------------------------- drain (4 warps)
+    regs_dec<C::REGS_DRAIN>();
+    const int quad = warp & 3;
+    const uint32_t lane_off = uint32_t(quad * 32) << 16;
+    uint8_t* boxes = smem + C::OFF_STG + quad * 8192;
+    uint32_t g = 0, items = 0, box = 0;
+    bool ok = true;
+    for (int r = 0; ok && r * (int)gridDim.x < n_items; ++r) {
+      const int w = bwd_index(r);
+      if (w >= n_items) continue;
+      const BwdItem it = bwd_item(p, w);
+      const int kj = it.k0 + quad * 32 + lane;
+      const long long off_kv = (long long)it.b * p.sdkv[0] + (long long)kj * p.sdkv[1] +
+                               (long long)it.h * p.sdkv[2];
+      T* dkp = reinterpret_cast<T*>(p.dk) + off_kv;
+      T* dvp = reinterpret_cast<T*>(p.dv) + off_kv;
+      if (it.n == 0) {             // no query sees this key tile: its gradients are zero
+        if (kj < p.Sk)
+          for (int c = 0; c < p.D / 8; ++c) {
+            reinterpret_cast<uint4*>(dkp)[c] = make_uint4(0, 0, 0, 0);
+            reinterpret_cast<uint4*>(dvp)[c] = make_uint4(0, 0, 0, 0);
+          }
+        continue;
+      }
+      for (int i = 0; i < it.n && ok; ++i, ++g) {
+        const int q0 = (it.q_begin + i) * ATT_BM + quad * 32;   // first query row of this warp
+        ok = mbar_wait(dq_full, g & 1, p.status, PF_ERR_TIMEOUT_TMEM_FULL);
+        if (!ok) break;
+        tc_fence_after();
+#pragma unroll
+        for (int c = 0; c < DP / 32; ++c) {
+          uint32_t raw[32];
+          tmem_ld32(tmem + C::T_DQ + lane_off + c * 32, raw);
+          tmem_ld_wait_for(raw);
+          if (c == DP / 32 - 1) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(dq_empty);
+          }
+          if (p.direct_dq) {
+            const int qi = q0 + lane;
+            if (qi < p.Sq) {
+              T* dst = reinterpret_cast<T*>(p.dq) + (long long)it.b * p.sdq[0] +
+                       (long long)qi * p.sdq[1] + (long long)it.h * p.sdq[2] + c * 32;
+#pragma unroll
+              for (int v = 0; v < 4; ++v)
+                if (c * 32 + v * 8 < p.D) reinterpret_cast<uint4*>(dst)[v] = pack8<T>(raw + v * 8);
+            }
+          } else {
+            // two boxes per warp: the reduce-add that last used this one must have read it
+            uint8_t* bx = boxes + (box & 1) * 4096;
+            if (lane == 0 && box >= 2) tma_store_wait_read_but_one();
+            __syncwarp();
+#pragma unroll
+            for (int v = 0; v < 8; ++v)
+              *reinterpret_cast<uint4*>(bx + lane * 128 + ((v ^ (lane & 7)) << 4)) =
+                  make_uint4(raw[v * 4], raw[v * 4 + 1], raw[v * 4 + 2], raw[v * 4 + 3]);
+            fence_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              // rows beyond the last query / columns beyond D are clipped by the TMA itself
+              if (q0 < p.Sq) tma_reduce_add_4d(&tdq, bx, c * 32, it.h, q0, it.b);
+              tma_store_commit();
+            }
+            ++box;
+          }
+        }
+      }
+      if (!ok) break;
+      ok = mbar_wait(acc_full, items & 1, p.status, PF_ERR_TIMEOUT_TMEM_FULL);
+      if (!ok) break;
+      tc_fence_after();
+#pragma unroll
+      for (int c = 0; c < DP / 32; ++c) {
+        uint32_t rk[32], rv[32];
+        tmem_ld32(tmem + C::T_DK + lane_off + c * 32, rk);
+        tmem_ld32(tmem + C::T_DV + lane_off + c * 32, rv);
+        tmem_ld_wait_for(rk);
+        tmem_ld_wait_for(rv);
+        if (c == DP / 32 - 1) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(acc_empty);
+        }
+        if (kj < p.Sk) {
+#pragma unroll
+          for (int v = 0; v < 4; ++v)
+            if (c * 32 + v * 8 < p.D) {
+              reinterpret_cast<uint4*>(dkp)[c * 4 + v] = pack8<T>(rk + v * 8);
+              reinterpret_cast<uint4*>(dvp)[c * 4 + v] = pack8<T>(rv + v * 8);
+            }
+        }
+      }
+      ++items;
+    }
+    if (lane == 0) tma_store_wait_all();
+  } else {
+    // ---------------------------------------------------------------- softmax side (8 warps)
+    regs_inc<C::REGS_SOFTMAX>();
+    const int quad = warp & 3, half = warp >> 2;
+    const int row = quad * 32 + lane;
+    const uint32_t lane_off = uint32_t(quad * 32) << 16;
+    const float c2 = p.scale * LOG2E;
+    const uint64_t c2v = f2_pack(c2, c2), scv = f2_pack(p.scale, p.scale);
+    uint32_t g = 0;
+    bool ok = true;
+    for (int r = 0; ok && r * (int)gridDim.x < n_items; ++r) {
+      const int w = bwd_index(r);
+      if (w >= n_items) continue;
+      const BwdItem it = bwd_item(p, w);
+      const bool ragged = it.k0 + ATT_BN > p.Sk;
+      const int kj = it.k0 + row;
+      // a warp all of whose keys lie beyond the last one (rounded to the reduction steps of dQ)
+      // has nothing to contribute: those rows of dK / dV are not stored, dQ does not read them
+      const bool warp_live = it.k0 + quad * 32 < (p.Sk + 15) / 16 * 16;
+      for (int i = 0; i < it.n && ok; ++i, ++g) {
+        const int q0 = (it.q_begin + i) * ATT_BM, st = g & 1, dsb = g % C::NDS;
+        const int cols = (min(ATT_BM, p.Sq - q0) + 15) / 16 * 16;
+        const float* lse2 =
+            reinterpret_cast<const float*>(smem + C::OFF_STAT + st * 1024) + half * 64;
+        const float* dlt = lse2 + 128;
+        const bool masked = ragged || (p.causal && it.k0 + ATT_BN - 1 > q0 + shift);
+        // queries of this half below `lim` do not see the key of this row
+        int lim = p.causal ? kj - shift - q0 - half * 64 : -1;
+        if (kj >= p.Sk) lim = ATT_BM;
+        ok = mbar_wait(&q_full[st], (g >> 1) & 1, p.status, PF_ERR_TIMEOUT_FULL) &&
+             mbar_wait(s_full, g & 1, p.status, PF_ERR_TIMEOUT_TMEM_FULL);
+        if (!C::ALIAS_P && ok && g > 0)     // the columns of P^T: dV of the previous tile read them
+          ok = mbar_wait(dv_done, (g - 1) & 1, p.status, PF_ERR_TIMEOUT_TMEM_EMPTY);
+        if (!ok) break;
+        tc_fence_after();
+        float pr[64];
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const bool work = warp_live && half * 64 + c * 32 < cols;     // warp-uniform
+          uint32_t s[32];
+          if (work) {
+            tmem_ld32(tmem + C::T_S + lane_off + half * 64 + c * 32, s);
+            tmem_ld_wait_for(s);
+          }
+          if (!C::ALIAS_P && c == 1) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(s_empty);
+          }
+          if (work) {
+            uint32_t pk[16];
+#pragma unroll
+            for (int j = 0; j < 32; j += 4) {
+              const float4 l4 = *reinterpret_cast<const float4*>(lse2 + c * 32 + j);
+              float x[4];
+              f2_unpack(fma2(f2_pack(__uint_as_float(s[j]), __uint_as_float(s[j + 1])), c2v,
+                             f2_pack(-l4.x, -l4.y)), x[0], x[1]);
+              f2_unpack(fma2(f2_pack(__uint_as_float(s[j + 2]), __uint_as_float(s[j + 3])), c2v,
+                             f2_pack(-l4.z, -l4.w)), x[2], x[3]);
+#pragma unroll
+              for (int u = 0; u < 4; ++u) {
+                float e = exp2f(x[u]);
+                if (masked && c * 32 + j + u < lim) e = 0.f;
+                pr[c * 32 + j + u] = e;
+              }
+              pk[j / 2] = pack2<T>(pr[c * 32 + j], pr[c * 32 + j + 1]);
+              pk[j / 2 + 1] = pack2<T>(pr[c * 32 + j + 2], pr[c * 32 + j + 3]);
+            }
+            tmem_st16(tmem + C::T_P + lane_off + half * C::P_HALF + c * 16, pk);
+          }
+        }
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(p_ready);
+        // ---- dS^T
+        ok = mbar_wait(dp_full, g & 1, p.status, PF_ERR_TIMEOUT_TMEM_FULL) &&
+             mbar_wait(&ds_empty[dsb], ((g / C::NDS) & 1) ^ 1, p.status, PF_ERR_TIMEOUT_EMPTY);
+        if (!ok) break;
+        tc_fence_after();
+        uint8_t* ds_row = smem + C::OFF_DS + dsb * C::DS_BYTES + half * ATT_BLK + row * 128;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          if (warp_live && half * 64 + c * 32 < cols) {
+            uint32_t s[32];
+            tmem_ld32(tmem + C::T_DP + lane_off + half * 64 + c * 32, s);
+            tmem_ld_wait_for(s);
+#pragma unroll
+            for (int j = 0; j < 32; j += 8) {
+              uint32_t o[4];
+#pragma unroll
+              for (int u = 0; u < 8; u += 4) {
+                const float4 d4 = *reinterpret_cast<const float4*>(dlt + c * 32 + j + u);
+                float a, b;
+                f2_unpack(mul2(f2_pack(pr[c * 32 + j + u], pr[c * 32 + j + u + 1]),
+                               fma2(f2_pack(__uint_as_float(s[j + u]),
+                                            __uint_as_float(s[j + u + 1])),
+                                    scv, f2_pack(-d4.x, -d4.y))), a, b);
+                o[u / 2] = pack2<T>(a, b);
+                f2_unpack(mul2(f2_pack(pr[c * 32 + j + u + 2], pr[c * 32 + j + u + 3]),
+                               fma2(f2_pack(__uint_as_float(s[j + u + 2]),
+                                            __uint_as_float(s[j + u + 3])),
+                                    scv, f2_pack(-d4.z, -d4.w))), a, b);
+                o[u / 2 + 1] = pack2<T>(a, b);
+              }
+              *reinterpret_cast<uint4*>(ds_row + (((c * 4 + j / 8) ^ (row & 7)) << 4)) =
+                  make_uint4(o[0], o[1], o[2], o[3]);
+            }
+          }
+        }
+        fence_async_smem();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) { mbar_arrive(ds_ready); mbar_arrive(&q_empty[st]); }
+      }
+    }
+  }
+
+  // teardown: every role reaches this point (all waits are bounded)
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 13) { tc_fence_after(); tmem_dealloc(tmem, 512); }
+}
+
+// ------------------------------------------------------------------------------- host side
+// fp32 [B, Sq, H, D] contiguous sums; box = 32 x 1 x 32 x 1 in the 128-byte swizzle
+static int make_tmap_dq(CUtensorMap* map, const void* base, int B, int S, int H, int D) {
+  EncodeTiledFn enc = attn_get_encode();
+  if (!enc) return -100;
+  cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)H, (cuuint64_t)S, (cuuint64_t)B};
+  cuuint64_t strides[3] = {(cuuint64_t)D * 4, (cuuint64_t)H * D * 4, (cuuint64_t)S * H * D * 4};
+  cuuint32_t box[4] = {32, 1, 32, 1};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<void*>(base), dims, strides,
+                   box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                   CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : -(1000 + (int)r);
+}
+
+template <typename T, int DP>
+static int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
+                      const CUtensorMap& tdo, const CUtensorMap& tdq, const AttnBwdParams& p,
+                      cudaStream_t st) {
+  using C = BwdCfg<DP>;
+  auto kern = attn_bwd_ws_kernel<T, DP>;
+  static bool done[64] = {};
+  int r = set_smem(kern, C::SMEM, done);
+  if (r) return r;
+  const int n_items = p.n_kt * p.H * p.B, sms = attn_sm_count();
+  kern<<<n_items < sms ? n_items : sms, C::THREADS, C::SMEM, st>>>(tq, tk, tv, tdo, tdq, p,
+                                                                   n_items);
+  PF_CHECK_LAUNCH();
+  return 0;
+}
+
+// one key tile that every query tile visits: its dQ tiles need no summation
+static bool bwd_direct(int Sq, int Sk, int causal) {
+  return Sk <= ATT_BN && (!causal || Sk >= Sq);
+}
+
+}  // namespace pf
+
+using namespace pf;
+
+// dout / out: [B, Sq, H, D] contiguous.  stats: fp32 scratch [B, H, ceil(Sq / 128), 256], 16-byte
+// aligned.  dq_accum: fp32 scratch [B, Sq, H, D], not needed (may be null) when
+// pf_attn_bwd_direct(Sq, Sk, causal).
+PF_API int pf_attn_bwd_direct(int Sq, int Sk, int causal) { return bwd_direct(Sq, Sk, causal); }
+
+PF_API int pf_attn_bwd(const void* dout, const void* q, const void* k, const void* v,
+                       const void* out, const void* lse, void* stats, void* dq_accum, void* dq,
+                       void* dk, void* dv, int B, int H, int Sq, int Sk, int D,
+                       const long long* sq, const long long* sk, const long long* sv,
+                       const long long* sdq, const long long* sdkv, int causal,
+                       float scale, int dtype, int* status, int sm_count, void* stream) {
+  if (dtype != PF_F16 && dtype != PF_BF16) return -1;
+  if (D % 8 || D > 128) return -3;
+  const bool direct = bwd_direct(Sq, Sk, causal);
+  if (!strides_ok(q, sq[0], sq[1], sq[2]) || !strides_ok(k, sk[0], sk[1], sk[2]) ||
+      !strides_ok(v, sv[0], sv[1], sv[2]) || (reinterpret_cast<uintptr_t>(dout) & 15) ||
+      (reinterpret_cast<uintptr_t>(out) & 15) || (reinterpret_cast<uintptr_t>(stats) & 15) ||
+      (!direct && (!dq_accum || (reinterpret_cast<uintptr_t>(dq_accum) & 15))) ||
+      !strides_ok(dq, sdq[0], sdq[1], sdq[2]) || !strides_ok(dk, sdkv[0], sdkv[1], sdkv[2]) ||
+      !strides_ok(dv, sdkv[0], sdkv[1], sdkv[2]))
+    return -2;
+  const int fmt = dtype == PF_BF16;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  AttnBwdParams p = {};
+  p.B = B; p.H = H; p.Sq = Sq; p.Sk = Sk; p.D = D; p.causal = causal; p.scale = scale;
+  p.fmt = fmt; p.stats = (const float*)stats; p.dq = dq; p.dk = dk; p.dv = dv; p.status = status;
+  p.direct_dq = direct;
+  p.n_kt = (Sk + ATT_BN - 1) / ATT_BN;
+  p.n_qt = (Sq + ATT_BM - 1) / ATT_BM;
+  for (int i = 0; i < 3; ++i) { p.sdq[i] = sdq[i]; p.sdkv[i] = sdkv[i]; }
+  CUtensorMap tq, tk, tv, tdo, tdq;
+  int r;
+  if ((r = make_tmap_bshd(&tq, q, fmt, B, Sq, H, D, sq[0], sq[1], sq[2]))) return r;
+  if ((r = make_tmap_bshd(&tk, k, fmt, B, Sk, H, D, sk[0], sk[1], sk[2]))) return r;
+  if ((r = make_tmap_bshd(&tv, v, fmt, B, Sk, H, D, sv[0], sv[1], sv[2]))) return r;
+  if ((r = make_tmap_bshd(&tdo, dout, fmt, B, Sq, H, D, (long long)Sq * H * D, (long long)H * D,
+                          D)))
+    return r;
+  if (direct) memset(&tdq, 0, sizeof(tdq));
+  else if ((r = make_tmap_dq(&tdq, dq_accum, B, Sq, H, D))) return r;
+  const long long pad_rows = (long long)B * p.n_qt * ATT_BM * H;
+  const unsigned prep = (unsigned)((pad_rows + 31) / 32);
+  float* sums = direct ? nullptr : (float*)dq_accum;
+  if (dtype == PF_F16)
+    attn_bwd_prep_kernel<__half><<<prep, 256, 0, st>>>((const __half*)dout, (const __half*)out,
+        (const float*)lse, (float*)stats, sums, B, Sq, H, D, p.n_qt, scale);
+  else
+    attn_bwd_prep_kernel<__nv_bfloat16><<<prep, 256, 0, st>>>((const __nv_bfloat16*)dout,
+        (const __nv_bfloat16*)out, (const float*)lse, (float*)stats, sums, B, Sq, H, D, p.n_qt,
+        scale);
+  PF_CHECK_LAUNCH();
+  {
+    auto run = [&]() -> int { PF_ATTN_DISPATCH(launch_bwd, tq, tk, tv, tdo, tdq, p, st); };
+    if ((r = run())) return r;
+  }
+  if (direct) return 0;
+  const long long rows = (long long)B * Sq * H, n = rows * (D / 8);
+  long long blocks = (n + 255) / 256;
+  const long long cap = (long long)(sm_count > 0 ? sm_count : 148) * 8;
+  if (blocks > cap) blocks = cap;
+  if (dtype == PF_F16)
+    attn_dq_convert_kernel<__half><<<(unsigned)blocks, 256, 0, st>>>(
+        (const float*)dq_accum, (__half*)dq, rows, D, Sq, H, sdq[0], sdq[1], sdq[2]);
+  else
+    attn_dq_convert_kernel<__nv_bfloat16><<<(unsigned)blocks, 256, 0, st>>>(
+        (const float*)dq_accum, (__nv_bfloat16*)dq, rows, D, Sq, H, sdq[0], sdq[1], sdq[2]);
+  PF_CHECK_LAUNCH();
+  return 0;
+}

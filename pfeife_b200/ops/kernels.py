@@ -440,9 +440,11 @@ def attn_bwd(do: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor
         dq = torch.empty((B, Sq, H, D), dtype=q.dtype, device=q.device)
         dk = torch.empty((B, Sk, H, D), dtype=q.dtype, device=q.device)
         dv = torch.empty((B, Sk, H, D), dtype=q.dtype, device=q.device)
-    delta = torch.empty((B, H, Sq), dtype=torch.float32, device=q.device)
-    acc = torch.empty((B, Sq, H, D), dtype=torch.float32, device=q.device)
-    check(L.pf_attn_bwd(ptr(do), ptr(q), ptr(k), ptr(v), ptr(o), ptr(lse), ptr(delta), ptr(acc),
+    # row statistics per query tile and, unless one key tile holds every key, fp32 sums of dq
+    stats = torch.empty((B, H, (Sq + 127) // 128, 256), dtype=torch.float32, device=q.device)
+    acc = None if L.pf_attn_bwd_direct(Sq, Sk, int(causal)) else \
+        torch.empty((B, Sq, H, D), dtype=torch.float32, device=q.device)
+    check(L.pf_attn_bwd(ptr(do), ptr(q), ptr(k), ptr(v), ptr(o), ptr(lse), ptr(stats), ptr(acc),
                         ptr(dq), ptr(dk), ptr(dv), B, H, Sq, Sk, D, _strides3(q), _strides3(k),
                         _strides3(v), _strides3(dq), _strides3(dk), int(causal), c_f(scale),
                         dt(q.dtype), ptr(status_word(q.device)), sm_count(q.device), stream()),

@@ -112,3 +112,50 @@ def test_packed_qkv_attention_writes_fused_gradient():
     o_ref.sum().backward()
     assert (out.float() - o_ref).abs().max() <= 2e-2
     assert (qkv.grad.float() - ref_in.grad).abs().max() <= 1e-1
+
+
+BWD_EDGES = [  # B, H, Sq, Sk, D, causal: tile edges, remainders, every head-dim class, empty key tiles
+    (1, 1, 1, 1, 8, False), (2, 3, 127, 128, 24, False), (1, 2, 129, 129, 32, False),
+    (2, 2, 257, 257, 88, True), (1, 2, 144, 272, 40, False), (1, 2, 385, 100, 64, False),
+    (1, 2, 100, 385, 64, True), (1, 2, 385, 100, 64, True), (1, 1, 300, 128, 72, True),
+    (2, 5, 513, 640, 128, True), (1, 3, 640, 513, 128, False), (40, 10, 65, 65, 96, False),
+    (7, 25, 130, 258, 128, False), (3, 67, 272, 272, 64, True),
+]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,H,Sq,Sk,D,causal", BWD_EDGES)
+def test_attention_fwd_bwd_at_tile_edges(dtype, B, H, Sq, Sk, D, causal):
+    """Outputs and gradients against 64 bits.  P, dS and the results are rounded to 16 bits, each
+    with a relative error of up to u = 2^-8 / 2^-11 and of u / 2 on average; 2 u bounds the 2-norm
+    of their sum."""
+    from pfeife_b200.ops import kernels as kx
+    g = torch.Generator(device="cuda").manual_seed(Sq * 7 + Sk)
+    mk = lambda S: torch.randn(B, S, H, D, device="cuda", generator=g).to(dtype)
+    q, k, v, do = mk(Sq), mk(Sk), mk(Sk), mk(Sq)
+    scale = 1.0 / math.sqrt(D)
+    o, lse = kx.attn_fwd(q, k, v, causal, scale)
+    grads = kx.attn_bwd(do, q, k, v, o, lse, causal, scale)
+    again = kx.attn_bwd(do, q, k, v, o, lse, causal, scale)   # buffers with earlier contents
+    torch.cuda.synchronize()
+    kx.check_status()
+    qr, kr, vr = (t.double().requires_grad_() for t in (q, k, v))
+    s = torch.einsum("bqhd,bkhd->bhqk", qr, kr) * scale
+    if causal:
+        seen = torch.ones(Sq, Sk, dtype=torch.bool, device="cuda").tril(Sk - Sq)
+        s = s.masked_fill(~seen, -1e30)      # rows that see no key: zeroed below
+        p = torch.softmax(s, -1) * seen
+    else:
+        p = torch.softmax(s, -1)
+    o_ref = torch.einsum("bhqk,bkhd->bqhd", p, vr)
+    o_ref.backward(do.double())
+    u = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    wants = (o_ref.detach(), qr.grad, kr.grad, vr.grad)
+    for name, got, want in zip(("o", "dq", "dk", "dv"), (o,) + grads, wants):
+        assert torch.isfinite(got.float()).all(), name
+        # the floor is what rounding dS, of the size of the probabilities' products, leaves in
+        # gradients that cancel (one key: dq and dk are zero)
+        floor = u * D ** 0.5 * want.numel() ** 0.5 * 0.5 if Sk == 1 else 0.0
+        assert (got.double() - want).norm() <= 2 * u * want.norm() + floor, name
+    for a, b in zip(grads, again):
+        assert (a.float() - b.float()).norm() <= u * a.float().norm()
