@@ -281,19 +281,22 @@ def linear_bwd(dy: Tensor, x: Tensor, w: Tensor, aux: Tensor, act: int, need_dx:
         if need_dw:
             x2 = _rows(x if x.dtype == cd else kx.cast(x, cd))
             ok = N % 8 == 0 and K % 8 == 0
+            # the epilogue rounds the fp32 sums to a 16-bit weight's type itself: one write of
+            # 2 bytes instead of 4 out, 4 back in and 2 out (4096 x 22016: 130 us less)
+            dt_w = w.dtype if w.dtype in (torch.float16, torch.bfloat16) else torch.float32
             if slot is not None and slot.main_grad is not None and ok:
                 kx.gemm(dy2, x2, a_mn=True, b_mn=True, out=slot.main_grad.view(N, K),
                         accumulate=True)
             elif ok:
-                dw = kx.gemm(dy2, x2, a_mn=True, b_mn=True, out_dtype=torch.float32)
+                dw = kx.gemm(dy2, x2, a_mn=True, b_mn=True, out_dtype=dt_w)
             elif N % 8 == 0:
                 # input width not a multiple of 8 (ViT patch embedding: 3 * 14 * 14 = 588):
                 # the same tensor-core GEMM on zero-padded columns, padding sliced off
                 dw = kx.gemm(dy2, _pad_k(x2), a_mn=True, b_mn=True,
-                             out_dtype=torch.float32)[:, :K].contiguous()
+                             out_dtype=dt_w)[:, :K].contiguous()
             else:
                 dw = dy2.float().t() @ x2.float()
-            if dw.numel() and w.dtype != torch.float32:
+            if dw.numel() and dw.dtype != w.dtype:
                 dw = dw.to(w.dtype)
         if need_db:
             bucket = _grad_bucket(bias)
