@@ -676,7 +676,7 @@ def _(logits, target, ignore_index):
 @torch.library.custom_op("pfeife::ce_bwd", mutates_args=())
 def ce_bwd(dloss: Tensor, logits: Tensor, target: Tensor, lse: Tensor, ignore_index: int) -> Tensor:
     if logits.is_cuda:
-        return kx.ce_bwd(logits.contiguous(), target, lse, dloss.float().contiguous(), ignore_index)
+        return kx.ce_bwd(logits.contiguous(), target, lse, dloss.float(), ignore_index)
     p = torch.exp(logits.float() - lse[:, None])
     valid = target != ignore_index
     onehot = torch.zeros_like(p)
@@ -704,18 +704,53 @@ ce_fwd.register_autograd(
     setup_context=_ce_setup)
 
 
+@torch.library.custom_op("pfeife::ce_mean_fwd", mutates_args=())
+def ce_mean_fwd(logits: Tensor, target: Tensor, ignore_index: int
+                ) -> Tuple[Tensor, Tensor, Tensor]:
+    """-> (mean loss over the rows that count, per-row log-sum-exp, one over their number)."""
+    if logits.is_cuda:
+        loss, lse = kx.ce_fwd(logits.contiguous(), target, ignore_index)
+        mean, inv = kx.ce_mean(loss, target, ignore_index)
+        return mean, lse, inv
+    lf = logits.float()
+    loss = F.cross_entropy(lf, target, reduction="none", ignore_index=ignore_index)
+    valid = (target != ignore_index).sum().clamp(min=1)
+    return loss.sum() / valid, torch.logsumexp(lf, -1), 1.0 / valid.float()
+
+
+@ce_mean_fwd.register_fake
+def _(logits, target, ignore_index):
+    m = logits.new_empty((), dtype=torch.float32)
+    return m, logits.new_empty(logits.shape[0], dtype=torch.float32), torch.empty_like(m)
+
+
+def _ce_mean_setup(ctx, inputs, output):
+    logits, target, ignore_index = inputs
+    ctx.set_materialize_grads(False)
+    ctx.save_for_backward(logits, target, output[1], output[2])
+    ctx.ignore_index = ignore_index
+
+
+def _ce_mean_backward(ctx, g, dlse, dinv):
+    logits, target, lse, inv = ctx.saved_tensors
+    if g is None:
+        return None, None, None
+    d = ce_bwd((g * inv).expand(logits.shape[0]), logits, target, lse, ctx.ignore_index)
+    return d, None, None
+
+
+ce_mean_fwd.register_autograd(_ce_mean_backward, setup_context=_ce_mean_setup)
+
+
 def cross_entropy(logits: Tensor, target: Tensor, ignore_index: int = -100,
                   reduction: str = "mean") -> Tensor:
     """Fused log-softmax + NLL over the last dim; the probabilities are never materialised in
     the forward and the backward is one pass over the logits."""
     V = logits.shape[-1]
+    if reduction not in ("none", "sum"):
+        return ce_mean_fwd(logits.reshape(-1, V), target.reshape(-1), ignore_index)[0]
     loss, _ = ce_fwd(logits.reshape(-1, V), target.reshape(-1), ignore_index)
-    if reduction == "none":
-        return loss.view(target.shape)
-    if reduction == "sum":
-        return loss.sum()
-    valid = (target.reshape(-1) != ignore_index).sum().clamp(min=1)
-    return loss.sum() / valid
+    return loss.view(target.shape) if reduction == "none" else loss.sum()
 
 
 @torch.library.custom_op("pfeife::mse_fwd", mutates_args=())

@@ -327,10 +327,24 @@ def ce_bwd(logits: torch.Tensor, target: torch.Tensor, lse: torch.Tensor,
     L = _lib.lib()
     rows, V = logits.shape
     d = torch.empty_like(logits)
+    if rows > 1 and gscale.stride(0) != 0:       # one value for all rows may come as an expand
+        gscale = gscale.contiguous()
     check(L.pf_ce_bwd(ptr(logits), ptr(target.contiguous()), ptr(lse), ptr(gscale), ptr(d),
                       c_ll(rows), V, c_ll(logits.stride(0)), c_ll(ignore_index),
-                      dt(logits.dtype), stream()), "pf_ce_bwd")
+                      c_ll(gscale.stride(0)), dt(logits.dtype), stream()), "pf_ce_bwd")
     return d
+
+
+def ce_mean(loss: torch.Tensor, target: torch.Tensor, ignore_index: int = -100
+            ) -> Tuple[torch.Tensor, torch.Tensor]:
+    """Row losses -> (their mean over the rows that count, one over the number of those)."""
+    L = _lib.lib()
+    assert loss.dtype == torch.float32 and loss.is_contiguous() and target.dtype == torch.int64
+    mean = torch.empty((), dtype=torch.float32, device=loss.device)
+    inv = torch.empty_like(mean)
+    check(L.pf_ce_mean(ptr(loss), ptr(target.contiguous()), ptr(mean), ptr(inv),
+                       c_ll(loss.numel()), c_ll(ignore_index), stream()), "pf_ce_mean")
+    return mean, inv
 
 
 def mse_fwd(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:

@@ -1,0 +1,65 @@
+"""Losses, norms and eager calls at the edges of their kernels' vector, slab and tile splits, against
+64-bit PyTorch."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+
+# unit roundoff of the result types
+U = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11, torch.float32: 2.0 ** -24}
+
+
+def close(got, want, rel):
+    """2-norm of the difference, relative; `rel` is the rounding of the result's type plus the
+    1e-5 of fp32 sums."""
+    got, want = got.double(), want.double()
+    assert torch.isfinite(got).all()
+    assert (got - want).norm() <= (rel + 1e-5) * want.norm() + 1e-12
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("rows,V", [(1, 1), (3, 7), (5, 1000), (17, 2049), (591, 33), (592, 4103),
+                                    (2, 50257), (1200, 1003)])
+def test_cross_entropy_edges(rows, V, dtype):
+    from pfeife_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(rows + V)
+    x = (torch.randn(rows, V, device="cuda", generator=g) * 3).to(dtype).requires_grad_()
+    t = torch.randint(0, V, (rows,), device="cuda", generator=g)
+    t[::3] = -100
+    xr = x.detach().double().requires_grad_()
+    for reduction in ("mean", "sum", "none"):
+        loss = ops.cross_entropy(x, t, reduction=reduction)
+        want = F.cross_entropy(xr, t, reduction="none")
+        want = want if reduction == "none" else want.sum() / (
+            max(1, int((t != -100).sum())) if reduction == "mean" else 1)
+        w = torch.randn(loss.shape, device="cuda", generator=g) + 2
+        (dx,) = torch.autograd.grad(loss, x, w)
+        (dr,) = torch.autograd.grad(want, xr, w.double())
+        close(loss, want, 0.0)
+        # fp16: small probabilities over many rows are subnormal, half a step of 2^-24 each
+        sub = 2.0 ** -25 * dr.numel() ** 0.5 if dtype == torch.float16 else 0.0
+        assert (dx.double() - dr).norm() <= (U[dtype] + 1e-5) * dr.norm() + sub
+
+
+def test_cross_entropy_masked_vocabulary_and_all_ignored():
+    """Logits of -inf and of the type's lowest value have no probability; a batch without a row
+    that counts has loss 0 and no gradient."""
+    from pfeife_b200 import ops
+    x = torch.randn(9, 3000, device="cuda").to(torch.bfloat16)
+    x[:, :1024] = float("-inf")
+    x[:, 2000:] = torch.finfo(torch.bfloat16).min
+    t = torch.randint(1024, 2000, (9,), device="cuda")
+    x.requires_grad_()
+    loss = ops.cross_entropy(x, t)
+    (dx,) = torch.autograd.grad(loss, x)
+    xr = x.detach().double().requires_grad_()
+    want = F.cross_entropy(xr, t)
+    (dr,) = torch.autograd.grad(want, xr)
+    close(loss, want, 0.0)
+    close(dx, dr, U[torch.bfloat16])
+    none = torch.full_like(t, -100)
+    y = torch.randn(9, 3000, device="cuda").to(torch.bfloat16).requires_grad_()
+    loss = ops.cross_entropy(y, none)
+    (dy,) = torch.autograd.grad(loss, y)
+    assert float(loss.detach()) == 0.0 and not dy.any()
