@@ -131,6 +131,10 @@ PF_DECL int pf_groupnorm_bwd(const void* dy, const void* x, const void* mean, co
                              const void* gamma, const void* beta, void* dx, void* dgamma,
                              void* dbeta, void* sums, int B, int HW, int C, int G, int act_silu,
                              int dtype, int sm_count, void* stream);
+PF_DECL int pf_conv_pack(const void* w, void* out, int Cout, int Cin, int taps, int cout8, int cin8,
+                         int flip, void* stream);
+PF_DECL int pf_conv_unpack(const void* src, void* dw, int Cout, int Cin, int taps, int cin8,
+                           int dtype, void* stream);
 PF_DECL int pf_upsample2x(const void* x, void* y, int B, int H, int W, int C, int backward,
                           int dtype, int sm_count, void* stream);
 

@@ -76,6 +76,71 @@ col2im_kernel(const T* __restrict__ dcols, T* __restrict__ dx, int B, int H, int
   }
 }
 
+// ------------------------------------------------------------------------------ conv weights
+// Between the [Cout, Cin, taps] order of a convolution's weight and the orders its products read.
+// Each CTA moves a tile through shared memory so that both sides are contiguous in global memory;
+// rows and channels beyond Cout / Cin (the products need multiples of 8) are zero.
+// Bound by latency at these sizes (7 MB at 640 channels): one launch for what took a strided copy
+// and, for the flipped taps, a second one.  Convolution forward and backward, bf16: 640 -> 640
+// channels on [4, 64, 64] 564 -> 538 us, 2560 -> 1280 on [1, 32, 32] 827 -> 666 us.
+constexpr int CONV_PACK_TAPS = 64;     // most taps (7 x 7 fits)
+
+// out[co, t, ci] = w[co, ci, t]
+__global__ void __launch_bounds__(128)
+conv_pack_kernel(const uint16_t* __restrict__ w, uint16_t* __restrict__ out, int Cout, int Cin,
+                 int taps, int cin8) {
+  __shared__ uint16_t tile[64 * CONV_PACK_TAPS];
+  const int co = blockIdx.x, ci0 = blockIdx.y * 64;
+  const int n_in = co < Cout ? max(0, min(64, Cin - ci0)) : 0, n_out = min(64, cin8 - ci0);
+  const uint16_t* src = w + ((long long)co * Cin + ci0) * taps;
+  for (int i = threadIdx.x; i < n_in * taps; i += 128) tile[i] = src[i];
+  __syncthreads();
+  for (int i = threadIdx.x; i < n_out * taps; i += 128) {
+    const int t = i / n_out, c = i - t * n_out;
+    out[((long long)co * taps + t) * cin8 + ci0 + c] = c < n_in ? tile[c * taps + t] : 0;
+  }
+}
+
+// out[ci, taps - 1 - t, co] = w[co, ci, t]: taps flipped, channel roles swapped
+__global__ void __launch_bounds__(256)
+conv_pack_flip_kernel(const uint16_t* __restrict__ w, uint16_t* __restrict__ out, int Cout, int Cin,
+                      int taps, int cout8, int cin8, int ci_per) {
+  extern __shared__ uint16_t ftile[];  // [64 co][ci_per * taps], rows padded by one
+  const int ci0 = blockIdx.x * ci_per, co0 = blockIdx.y * 64;
+  const int n_ci = max(0, min(ci_per, Cin - ci0)), n_co = min(64, Cout - co0);
+  const int row = n_ci * taps, pitch = ci_per * taps + 1;
+  for (int i = threadIdx.x; i < n_co * row; i += 256) {
+    const int c = i / row, k = i - c * row;
+    ftile[c * pitch + k] = w[((long long)(co0 + c) * Cin + ci0) * taps + k];
+  }
+  __syncthreads();
+  const int o_co = min(64, cout8 - co0), o_ci = min(ci_per, cin8 - ci0);
+  for (int i = threadIdx.x; i < o_ci * taps * o_co; i += 256) {
+    const int k = i / o_co, c = i - k * o_co, ci = k / taps, t = k - ci * taps;
+    out[((long long)(ci0 + ci) * taps + (taps - 1 - t)) * cout8 + co0 + c] =
+        (c < n_co && ci < n_ci) ? ftile[c * pitch + k] : 0;
+  }
+}
+
+// dw[co, ci, t] = src[co, t, ci] (fp32 sums with cin8 channels a row), converted to the weight's type
+template <typename T>
+__global__ void __launch_bounds__(128)
+conv_unpack_kernel(const float* __restrict__ src, T* __restrict__ dw, int Cin, int taps, int cin8) {
+  __shared__ float tile[64 * (CONV_PACK_TAPS + 1)];
+  const int co = blockIdx.x, ci0 = blockIdx.y * 64, n = min(64, Cin - ci0);
+  const int pitch = taps | 1;          // odd: the transposing stores hit different banks
+  for (int i = threadIdx.x; i < n * taps; i += 128) {
+    const int t = i / n, c = i - t * n;
+    tile[c * pitch + t] = src[((long long)co * taps + t) * cin8 + ci0 + c];
+  }
+  __syncthreads();
+  T* dst = dw + ((long long)co * Cin + ci0) * taps;
+  for (int i = threadIdx.x; i < n * taps; i += 128) {
+    const int c = i / taps, t = i - c * taps;
+    dst[i] = from_f32<T>(tile[c * pitch + t]);
+  }
+}
+
 // ------------------------------------------------------------------------------ GroupNorm
 // NHWC, C a multiple of 8.  All four passes read 16 bytes (8 channels) per thread and request.
 //
@@ -397,6 +462,40 @@ PF_API int pf_groupnorm_bwd(const void* dy, const void* x, const void* mean, con
         (const T*)dy, (const T*)x, (const float*)mean, (const float*)rstd, (const float*)gamma,
         (const float*)beta, sA, sB, (T*)dx, total_vec, HW, C, G, act_silu);
   });
+  PF_CHECK_LAUNCH();
+  return 0;
+}
+
+// 16-bit weights [Cout, Cin, taps] -> [cout8, taps, cin8], or with `flip` [cin8, taps reversed, cout8]
+PF_API int pf_conv_pack(const void* w, void* out, int Cout, int Cin, int taps, int cout8, int cin8,
+                        int flip, void* stream) {
+  if (taps < 1 || taps > CONV_PACK_TAPS) return -3;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  if (!flip) {
+    conv_pack_kernel<<<dim3(cout8, (cin8 + 63) / 64), 128, 0, st>>>(
+        (const uint16_t*)w, (uint16_t*)out, Cout, Cin, taps, cin8);
+  } else {
+    const int per = taps <= 16 ? 8 : 4;       // tile of at most 64 x 257 x 2 bytes
+    conv_pack_flip_kernel<<<dim3((cin8 + per - 1) / per, (cout8 + 63) / 64), 256,
+                            64 * (per * taps + 1) * 2, st>>>((const uint16_t*)w, (uint16_t*)out,
+                                                             Cout, Cin, taps, cout8, cin8, per);
+  }
+  PF_CHECK_LAUNCH();
+  return 0;
+}
+
+// fp32 [>= Cout, taps, cin8] -> [Cout, Cin, taps] of `dtype`
+PF_API int pf_conv_unpack(const void* src, void* dw, int Cout, int Cin, int taps, int cin8,
+                          int dtype, void* stream) {
+  if (taps < 1 || taps > CONV_PACK_TAPS) return -3;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  const dim3 grid(Cout, (Cin + 63) / 64);
+  switch (dtype) {
+    case PF_F32: conv_unpack_kernel<float><<<grid, 128, 0, st>>>((const float*)src, (float*)dw, Cin, taps, cin8); break;
+    case PF_F16: conv_unpack_kernel<__half><<<grid, 128, 0, st>>>((const float*)src, (__half*)dw, Cin, taps, cin8); break;
+    case PF_BF16: conv_unpack_kernel<__nv_bfloat16><<<grid, 128, 0, st>>>((const float*)src, (__nv_bfloat16*)dw, Cin, taps, cin8); break;
+    default: return -1;
+  }
   PF_CHECK_LAUNCH();
   return 0;
 }

@@ -1032,6 +1032,18 @@ def _pad_to8(n: int) -> int:
     return (n + 7) // 8 * 8
 
 
+def _conv_weight(w: Tensor, dtype: torch.dtype, cout8: int, cin8: int) -> Tensor:
+    """The weight as the B operand [cout8, KH*KW*cin8] (taps outermost) of the forward product."""
+    wc = _weight_as(w, dtype)
+    if w.shape[2:] == (1, 1) and w.shape[:2] == (cout8, cin8):
+        return wc.reshape(cout8, cin8)       # the same order already
+    return kx.conv_pack(wc, cout8, cin8)
+
+
+def _conv_dw_dtype(w: Tensor) -> torch.dtype:
+    return w.dtype if w.dtype in (torch.float16, torch.bfloat16) else torch.float32
+
+
 @torch.library.custom_op("pfeife::conv2d_fwd", mutates_args=())
 def conv2d_fwd(x: Tensor, w: Tensor, bias: Optional[Tensor], stride: int, pad: int) -> Tensor:
     """Channels-last convolution: x [B, H, W, Cin], w [Cout, Cin, KH, KW] -> [B, Ho, Wo, Cout].
@@ -1045,10 +1057,7 @@ def conv2d_fwd(x: Tensor, w: Tensor, bias: Optional[Tensor], stride: int, pad: i
         cin8, cout8 = _pad_to8(Cin), _pad_to8(Cout)
         if cin8 != Cin:
             xc = F.pad(xc, (0, cin8 - Cin))
-        w2 = _weight_as(w, cd).permute(0, 2, 3, 1)                      # [Cout, KH, KW, Cin]
-        if cin8 != Cin or cout8 != Cout:
-            w2 = F.pad(w2, (0, cin8 - Cin, 0, 0, 0, 0, 0, cout8 - Cout))
-        w2 = w2.reshape(cout8, KH * KW * cin8).contiguous()
+        w2 = _conv_weight(w, cd, cout8, cin8)
         Ho = (H + 2 * pad - KH) // stride + 1
         Wo = (W + 2 * pad - KW) // stride + 1
         b2 = None
@@ -1079,7 +1088,8 @@ def _(x, w, bias, stride, pad):
 @torch.library.custom_op("pfeife::conv2d_bwd", mutates_args=())
 def conv2d_bwd(dy: Tensor, x: Tensor, w: Tensor, stride: int, pad: int, need_dx: bool,
                need_db: bool) -> Tuple[Tensor, Tensor, Tensor]:
-    """-> (dx [B,H,W,Cin], dw fp32 [Cout,Cin,KH,KW], db fp32 [Cout])."""
+    """-> (dx [B,H,W,Cin], dw [Cout,Cin,KH,KW] in w's type (fp32 unless that is 16-bit), db fp32
+    [Cout])."""
     Cout, Cin, KH, KW = w.shape
     cd = dy.dtype
     if dy.is_cuda and cd in (torch.float16, torch.bfloat16):
@@ -1099,25 +1109,18 @@ def conv2d_bwd(dy: Tensor, x: Tensor, w: Tensor, stride: int, pad: int, need_dx:
         else:
             cols = xc.reshape(B * H * W, cin8) if one else kx.im2col(xc, KH, KW, stride, pad)
             dw2 = kx.gemm(dy2, cols, a_mn=True, b_mn=True, out_dtype=torch.float32)
-        dw = dw2.view(cout8, KH, KW, cin8)[:Cout, :, :, :Cin].permute(0, 3, 1, 2).contiguous()
+        dw = kx.conv_unpack(dw2, w.shape, cin8, _conv_dw_dtype(w))
         dx = dy.new_empty(0)
         if need_dx:
-            w2 = _weight_as(w, cd).permute(0, 2, 3, 1)
-            if cin8 != Cin or cout8 != Cout:
-                w2 = F.pad(w2, (0, cin8 - Cin, 0, 0, 0, 0, 0, cout8 - Cout))
-            w2 = w2.reshape(cout8, KH * KW * cin8).contiguous()
             dy4 = dy2.view(B, -1, dy.shape[2], cout8)
             if not one and stride == 1 and cout8 == Cout and \
                     kx.conv_gemm_supported(dy4, KH, KW, 1, KH - 1 - pad) and \
                     dy4.shape[1] + 2 * (KH - 1 - pad) - KH + 1 == H:
                 # dx = correlation of dy with the taps flipped and the channel roles swapped
-                wt = _weight_as(w, cd).flip(2, 3).permute(1, 2, 3, 0)     # [Cin, KH, KW, Cout]
-                if cin8 != Cin:
-                    wt = F.pad(wt, (0, 0, 0, 0, 0, 0, 0, cin8 - Cin))
-                wt = wt.reshape(cin8, KH * KW * cout8).contiguous()
+                wt = kx.conv_pack(_weight_as(w, cd), cout8, cin8, flip=True)
                 dxp = kx.conv_gemm(dy4, wt, KH, KW, 1, KH - 1 - pad)
             else:
-                dcols = kx.gemm(dy2, w2, b_mn=True)                              # [M, K]
+                dcols = kx.gemm(dy2, _conv_weight(w, cd, cout8, cin8), b_mn=True)                              # [M, K]
                 dxp = dcols.view(B, H, W, cin8) if one else \
                     kx.col2im(dcols, (B, H, W, cin8), KH, KW, stride, pad)
             dx = dxp[..., :Cin].contiguous() if cin8 != Cin else dxp
@@ -1129,13 +1132,13 @@ def conv2d_bwd(dy: Tensor, x: Tensor, w: Tensor, stride: int, pad: int, need_dx:
         .permute(0, 2, 3, 1).contiguous() if need_dx else dy.new_empty(0)
     dw = torch.nn.grad.conv2d_weight(xn.float(), w.shape, dyn.float(), stride=stride, padding=pad)
     db = dyn.float().sum((0, 2, 3)) if need_db else dy.new_empty(0, dtype=torch.float32)
-    return dx, dw.float(), db
+    return dx, dw.to(_conv_dw_dtype(w)), db
 
 
 @conv2d_bwd.register_fake
 def _(dy, x, w, stride, pad, need_dx, need_db):
     return (torch.empty_like(x, dtype=dy.dtype) if need_dx else dy.new_empty(0),
-            w.new_empty(w.shape, dtype=torch.float32),
+            w.new_empty(w.shape, dtype=_conv_dw_dtype(w)),
             dy.new_empty(w.shape[0] if need_db else 0, dtype=torch.float32))
 
 

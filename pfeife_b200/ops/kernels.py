@@ -537,6 +537,41 @@ def conv_wgrad(dy2: torch.Tensor, x: torch.Tensor, KH: int, KW: int, stride: int
     return out
 
 
+def conv_pack(w: torch.Tensor, cout8: int, cin8: int, flip: bool = False) -> torch.Tensor:
+    """w [Cout, Cin, KH, KW] (16-bit) -> [cout8, KH*KW*cin8], the B operand of the forward, or with
+    ``flip`` [cin8, KH*KW*cout8] with the taps reversed, that of the input gradient; channels
+    beyond Cout / Cin are zero."""
+    L = _lib.lib()
+    w = w.contiguous()
+    Cout, Cin, KH, KW = w.shape
+    taps = KH * KW
+    if taps > 64:                      # beyond the kernels' tile
+        w = torch.nn.functional.pad(w, (0, 0, 0, 0, 0, cin8 - Cin, 0, cout8 - Cout))
+        p = w.flip(2, 3).permute(1, 2, 3, 0) if flip else w.permute(0, 2, 3, 1)
+        return p.reshape(p.shape[0], -1).contiguous()
+    out = torch.empty((cin8, taps * cout8) if flip else (cout8, taps * cin8), dtype=w.dtype,
+                      device=w.device)
+    check(L.pf_conv_pack(ptr(w), ptr(out), Cout, Cin, taps, cout8, cin8, int(flip), stream()),
+          "pf_conv_pack")
+    return out
+
+
+def conv_unpack(dw2: torch.Tensor, shape, cin8: int, dtype: torch.dtype) -> torch.Tensor:
+    """fp32 sums [>= Cout, KH*KW*cin8] -> the weight gradient [Cout, Cin, KH, KW] in `dtype`."""
+    L = _lib.lib()
+    Cout, Cin, KH, KW = shape
+    assert dw2.dtype == torch.float32 and dw2.is_contiguous()
+    if KH * KW == 1 and cin8 == Cin and dtype == torch.float32:
+        return dw2[:Cout].view(Cout, Cin, 1, 1)
+    if KH * KW > 64:
+        p = dw2.view(-1, KH, KW, cin8)[:Cout, :, :, :Cin].permute(0, 3, 1, 2)
+        return p.to(dtype).contiguous()
+    dw = torch.empty((Cout, Cin, KH, KW), dtype=dtype, device=dw2.device)
+    check(L.pf_conv_unpack(ptr(dw2), ptr(dw), Cout, Cin, KH * KW, cin8, dt(dtype), stream()),
+          "pf_conv_unpack")
+    return dw
+
+
 def col2im(dcols: torch.Tensor, shape, KH: int, KW: int, stride: int, pad: int) -> torch.Tensor:
     L = _lib.lib()
     B, H, W, C = shape

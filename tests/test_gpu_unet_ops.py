@@ -146,3 +146,31 @@ def test_unet_model_gpu_matches_cpu():
     worst = max((gg[n] - gc[n]).abs().max().item() / max(1e-3, gc[n].abs().max().item())
                 for n in gc)
     assert worst < 0.25
+
+
+@pytest.mark.parametrize("w_dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("B,H,Cin,Cout,K,stride", [
+    (1, 8, 64, 64, 3, 1), (2, 16, 64, 72, 3, 2), (1, 16, 4, 320, 3, 1), (1, 16, 96, 4, 3, 1),
+    (1, 9, 13, 21, 3, 1), (1, 16, 128, 65, 1, 1), (1, 12, 8, 8, 5, 1), (1, 11, 3, 9, 9, 1)])
+def test_conv_weight_orders(B, H, Cin, Cout, K, stride, w_dtype):
+    """Output and gradients with the packed weights (padding, flipped taps, gradient order) against
+    64 bits; every product sums 16-bit values in fp32 and rounds once (twice through col2im)."""
+    from pfeife_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(Cin * 31 + Cout)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    x = rnd(B, H, H, Cin).to(torch.bfloat16).requires_grad_()
+    # fp32 weights that bf16 holds exactly: the cast in front of the product changes nothing
+    w = (0.1 * rnd(Cout, Cin, K, K)).to(torch.bfloat16).to(w_dtype).requires_grad_()
+    b = rnd(Cout).requires_grad_()
+    y = ops.conv2d(x, w, b, stride, K // 2)
+    dy = rnd(*y.shape).to(torch.bfloat16)
+    grads = torch.autograd.grad(y, (x, w, b), dy)
+    xr, wr, br = (t.detach().double().requires_grad_() for t in (x, w, b))
+    yr = torch.nn.functional.conv2d(xr.permute(0, 3, 1, 2).cpu(), wr.cpu(), br.cpu(),
+                                    stride=stride, padding=K // 2).permute(0, 2, 3, 1)
+    wants = torch.autograd.grad(yr, (xr, wr, br), dy.double().cpu())
+    u = 2.0 ** -8
+    for got, want in ((y, yr), (grads[0], wants[0]), (grads[1], wants[1]), (grads[2], wants[2])):
+        want = want.to(got.device)
+        assert (got.double() - want).norm() <= 1.5 * u * want.norm()
+    assert grads[1].dtype == w_dtype
