@@ -405,123 +405,204 @@ norm_bwd_param_kernel(const T* __restrict__ dy, const T* __restrict__ h,
   }
 }
 
-// Backward for rows of up to 2048 16-bit elements: one WARP per row (no CTA-wide barrier on the
-// row path), 8 warps per CTA, rows strided over a persistent grid.  Each lane keeps the packed
-// dy / h vectors of its row slice in registers, expands them twice (reduction pass, output
-// pass) and carries dgamma / dbeta partials for its columns across rows.  At the end the 8
-// warps of a CTA fold their partials through shared memory into scratch[blockIdx][2][N].
+// Backward for rows of up to 2048 16-bit elements, everything in one pass over memory.  A
+// persistent CTA walks over tiles of 8 rows that asynchronous copies bring into shared memory, one
+// tile ahead; dy and h are then read there twice:
+//   by rows      warp <-> row: two shuffle reductions, dx
+//   by columns   thread <-> 8 columns of a share of the 8 rows: sums of dy * xhat and dy, kept in
+//                registers over all tiles of the CTA
+// The CTA's sums go to scratch[blockIdx][2][N], folded by norm_bwd_finish_kernel.
+// Bound by HBM: 4 tensors cross it once, where a pass for dx and one for the sums read dy and h
+// twice.  bf16, with the fold: 6168 x 1408 50 -> 38 us, 50000 x 1408 249 -> 153 us (3.7 TB/s),
+// 20000 x 2048 173 -> 112 us.  Longer rows keep the two passes: two stages of 8 of them do not fit.
+constexpr int NORM_TILE_ROWS = 8;
 template <typename T, int NV>
 __global__ void __launch_bounds__(256)
-norm_bwd_warp_kernel(const T* __restrict__ dy, const T* __restrict__ h,
-                     const float* __restrict__ gamma, const float* __restrict__ mean,
-                     const float* __restrict__ rstd, const T* __restrict__ dres,
-                     T* __restrict__ dx, float* __restrict__ scratch, long long rows, int N,
-                     int rms) {
-  constexpr int V = 16 / sizeof(T);
-  extern __shared__ float sacc[];          // [2][N]
-  const int nvec = N / V;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int i = threadIdx.x; i < 2 * N; i += 256) sacc[i] = 0.f;
-  __syncthreads();
-  float dg[NV][V], db[NV][V];
-#pragma unroll
-  for (int i = 0; i < NV; ++i)
-#pragma unroll
-    for (int j = 0; j < V; ++j) { dg[i][j] = 0.f; db[i][j] = 0.f; }
+norm_bwd_fused_kernel(const T* __restrict__ dy, const T* __restrict__ h,
+                      const float* __restrict__ gamma, const float* __restrict__ mean,
+                      const float* __restrict__ rstd, const T* __restrict__ dres,
+                      T* __restrict__ dx, float* __restrict__ scratch, long long rows, int N,
+                      int rms) {
+  constexpr int V = 8, R = NORM_TILE_ROWS;
+  extern __shared__ __align__(128) uint8_t nsmem[];     // [2 stages][dy, h][R][N]
+  const int nvec = N / V, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int tile_vec = R * nvec;
+  auto stage_ptr = [&](int st, int which) {
+    return reinterpret_cast<uint4*>(nsmem) + (st * 2 + which) * tile_vec;
+  };
+  const long long n_tiles = (rows + R - 1) / R;
+  // the rows of a tile are one contiguous piece of each tensor
+  auto fetch = [&](long long t, int st) {
+    if (t < n_tiles) {
+      const int n = (int)min((long long)R, rows - t * R) * nvec;
+      const uint4* gd = reinterpret_cast<const uint4*>(dy + t * R * N);
+      const uint4* gh = reinterpret_cast<const uint4*>(h + t * R * N);
+      for (int i = threadIdx.x; i < n; i += 256) {
+        cp_async16(stage_ptr(st, 0) + i, gd + i);
+        cp_async16(stage_ptr(st, 1) + i, gh + i);
+      }
+    }
+    cp_async_commit();                 // an empty group past the last tile
+  };
+  fetch(blockIdx.x, 0);
+  // column share: vector cv of rows grp, grp + groups, ...
+  const int groups = min(R, 256 / nvec), grp = threadIdx.x / nvec, cv = threadIdx.x - grp * nvec;
+  float ag[V] = {0, 0, 0, 0, 0, 0, 0, 0}, ab[V] = {0, 0, 0, 0, 0, 0, 0, 0};
   const float inv_n = 1.f / N;
-  for (long long row = (long long)blockIdx.x * 8 + warp; row < rows;
-       row += (long long)gridDim.x * 8) {
-    const float mu = rms ? 0.f : mean[row];
-    const float rs = rstd[row];
-    uint4 qd[NV], qh[NV];
-    float s1 = 0.f, s2 = 0.f;
+  int st = 0;
+  for (long long t = blockIdx.x; t < n_tiles; t += gridDim.x, st ^= 1) {
+    // the other stage was read in the previous round, which ended with a barrier
+    fetch(t + gridDim.x, st ^ 1);
+    const int live = (int)min((long long)R, rows - t * R);
+    const long long row = t * R + warp;
+    uint4 qr[NV];
+    float mu = 0.f, rs = 0.f;
+    if (warp < live) {
+      if (!rms) mu = mean[row];
+      rs = rstd[row];
+      if (dres) {
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      const int idx = lane + i * 32;
-      if (idx < nvec) {
-        qd[i] = reinterpret_cast<const uint4*>(dy + row * N)[idx];
-        qh[i] = reinterpret_cast<const uint4*>(h + row * N)[idx];
-        const T* ed = reinterpret_cast<const T*>(&qd[i]);
-        const T* eh = reinterpret_cast<const T*>(&qh[i]);
-        const float4* g4 = reinterpret_cast<const float4*>(gamma + idx * V);
+        for (int i = 0; i < NV; ++i)
+          if (lane + i * 32 < nvec)
+            qr[i] = __ldg(reinterpret_cast<const uint4*>(dres + row * N) + lane + i * 32);
+      }
+    }
+    cp_async_wait_but_one();           // this tile has landed, the next one may be under way
+    __syncthreads();
+    const uint4 *sd = stage_ptr(st, 0), *sh = stage_ptr(st, 1);
+    if (warp < live) {
+      const uint4 *rd = sd + warp * nvec, *rh = sh + warp * nvec;
+      float s1 = 0.f, s2 = 0.f;
 #pragma unroll
-        for (int j4 = 0; j4 < V / 4; ++j4) {
-          const float4 g = __ldg(g4 + j4);
-          const float gg[4] = {g.x, g.y, g.z, g.w};
+      for (int i = 0; i < NV; ++i) {
+        const int idx = lane + i * 32;
+        if (idx < nvec) {
+          const uint4 qd = rd[idx], qh = rh[idx];
+          const T* ed = reinterpret_cast<const T*>(&qd);
+          const T* eh = reinterpret_cast<const T*>(&qh);
+          const float4 g0 = __ldg(reinterpret_cast<const float4*>(gamma + idx * V));
+          const float4 g1 = __ldg(reinterpret_cast<const float4*>(gamma + idx * V) + 1);
+          const float g[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const int j = j4 * 4 + u;
-            const float d = to_f32<T>(ed[j]);
-            const float xhat = (to_f32<T>(eh[j]) - mu) * rs;
-            const float dyg = d * gg[u];
+          for (int j = 0; j < V; ++j) {
+            const float dyg = to_f32<T>(ed[j]) * g[j];
             s1 += dyg;
-            s2 += dyg * xhat;
-            dg[i][j] += d * xhat;
-            db[i][j] += d;
+            s2 += dyg * (to_f32<T>(eh[j]) - mu) * rs;
           }
         }
       }
-    }
-    const float m1 = rms ? 0.f : warp_sum(s1) * inv_n;
-    const float m2 = warp_sum(s2) * inv_n;
+      const float m1 = rms ? 0.f : warp_sum(s1) * inv_n;
+      const float m2 = warp_sum(s2) * inv_n;
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      const int idx = lane + i * 32;
-      if (idx < nvec) {
-        const T* ed = reinterpret_cast<const T*>(&qd[i]);
-        const T* eh = reinterpret_cast<const T*>(&qh[i]);
-        uint4 qr;
-        if (dres) qr = reinterpret_cast<const uint4*>(dres + row * N)[idx];
-        const T* er = reinterpret_cast<const T*>(&qr);
-        uint4 q;
-        T* e = reinterpret_cast<T*>(&q);
-        const float4* g4 = reinterpret_cast<const float4*>(gamma + idx * V);
+      for (int i = 0; i < NV; ++i) {
+        const int idx = lane + i * 32;
+        if (idx < nvec) {
+          const uint4 qd = rd[idx], qh = rh[idx];
+          const T* ed = reinterpret_cast<const T*>(&qd);
+          const T* eh = reinterpret_cast<const T*>(&qh);
+          const float4 g0 = __ldg(reinterpret_cast<const float4*>(gamma + idx * V));
+          const float4 g1 = __ldg(reinterpret_cast<const float4*>(gamma + idx * V) + 1);
+          const float g[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+          const T* er = reinterpret_cast<const T*>(&qr[i]);
+          uint4 q;
+          T* e = reinterpret_cast<T*>(&q);
 #pragma unroll
-        for (int j4 = 0; j4 < V / 4; ++j4) {
-          const float4 g = __ldg(g4 + j4);
-          const float gg[4] = {g.x, g.y, g.z, g.w};
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const int j = j4 * 4 + u;
+          for (int j = 0; j < V; ++j) {
             const float xhat = (to_f32<T>(eh[j]) - mu) * rs;
-            float o = rs * (to_f32<T>(ed[j]) * gg[u] - m1 - xhat * m2);
+            float o = rs * (to_f32<T>(ed[j]) * g[j] - m1 - xhat * m2);
             if (dres) o += to_f32<T>(er[j]);
             e[j] = from_f32<T>(o);
           }
+          reinterpret_cast<uint4*>(dx + row * N)[idx] = q;
         }
-        reinterpret_cast<uint4*>(dx + row * N)[idx] = q;
       }
     }
-  }
+    if (grp < groups) {
+      for (int r = grp; r < live; r += groups) {
+        const float mr = rms ? 0.f : __ldg(mean + t * R + r), rr = __ldg(rstd + t * R + r);
+        const uint4 qd = sd[r * nvec + cv], qh = sh[r * nvec + cv];
+        const T* ed = reinterpret_cast<const T*>(&qd);
+        const T* eh = reinterpret_cast<const T*>(&qh);
 #pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    const int idx = lane + i * 32;
-    if (idx < nvec) {
-#pragma unroll
-      for (int j = 0; j < V; ++j) {
-        atomicAdd(&sacc[idx * V + j], dg[i][j]);
-        atomicAdd(&sacc[N + idx * V + j], db[i][j]);
+        for (int j = 0; j < V; ++j) {
+          const float d = to_f32<T>(ed[j]);
+          ag[j] += d * (to_f32<T>(eh[j]) - mr) * rr;
+          ab[j] += d;
+        }
       }
+    }
+    __syncthreads();
+  }
+  // fold the row groups through the (now unused) tiles: [groups][2][N] floats
+  float* red = reinterpret_cast<float*>(nsmem);
+  if (grp < groups) {
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+      red[grp * 2 * N + cv * V + j] = ag[j];
+      red[grp * 2 * N + N + cv * V + j] = ab[j];
     }
   }
   __syncthreads();
   float* out = scratch + (long long)blockIdx.x * 2 * N;
-  for (int i = threadIdx.x; i < 2 * N; i += 256) out[i] = sacc[i];
+  for (int i = threadIdx.x; i < 2 * N; i += 256) {
+    float v = red[i];
+    for (int k = 1; k < groups; ++k) v += red[k * 2 * N + i];
+    out[i] = v;
+  }
 }
 
-// dgamma[c] (+)= sum_g scratch[g][0][c] ; dbeta likewise
-__global__ void __launch_bounds__(256)
+// dgamma[c] (+)= sum_g scratch[g][0][c] ; dbeta likewise.  A CTA owns 32 columns, its 32 warps share
+// the G rows (one thread per column over all rows took 29 us of latency at G = 296).
+__global__ void __launch_bounds__(1024)
 norm_bwd_finish_kernel(const float* __restrict__ scratch, float* __restrict__ dgamma,
                        float* __restrict__ dbeta, int G, int N, int accumulate) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= N) return;
+  __shared__ float red[2][32][33];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = blockIdx.x * 32 + lane;
   float a = 0.f, b = 0.f;
-  for (int g = 0; g < G; ++g) {
-    a += scratch[(long long)g * 2 * N + c];
-    b += scratch[(long long)g * 2 * N + N + c];
+  if (c < N) {
+#pragma unroll 4
+    for (int g = warp; g < G; g += 32) {
+      a += scratch[(long long)g * 2 * N + c];
+      b += scratch[(long long)g * 2 * N + N + c];
+    }
   }
-  dgamma[c] = accumulate ? dgamma[c] + a : a;
-  if (dbeta) dbeta[c] = accumulate ? dbeta[c] + b : b;
+  red[0][lane][warp] = a;
+  red[1][lane][warp] = b;
+  __syncthreads();
+  // warp w finishes column w of the 32
+  const int cw = blockIdx.x * 32 + warp;
+  a = warp_sum(red[0][warp][lane]);
+  b = warp_sum(red[1][warp][lane]);
+  if (lane == 0 && cw < N) {
+    // a gradient bucket may be added to by other kernels at the same time
+    if (accumulate) atomicAdd(dgamma + cw, a);
+    else dgamma[cw] = a;
+    if (dbeta && accumulate) atomicAdd(dbeta + cw, b);
+    else if (dbeta) dbeta[cw] = b;
+  }
+}
+
+// the fused backward needs two stages of a tile in shared memory (at most 128 KB)
+template <typename T, int NV>
+static int norm_bwd_fused_launch(const void* dy, const void* h, const float* gamma,
+                                 const float* mean, const float* rstd, const void* dres, void* dx,
+                                 float* scratch, int G, long long rows, int N, int rms,
+                                 cudaStream_t st) {
+  auto kern = norm_bwd_fused_kernel<T, NV>;
+  const int bytes = max(4 * NORM_TILE_ROWS * N * 2, 16384);
+  static bool done[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64 || !done[dev]) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         4 * NORM_TILE_ROWS * 2048 * 2);
+    if (e != cudaSuccess) return (int)e;
+    if (dev >= 0 && dev < 64) done[dev] = true;
+  }
+  kern<<<G, 256, bytes, st>>>((const T*)dy, (const T*)h, gamma, mean, rstd, (const T*)dres,
+                              (T*)dx, scratch, rows, N, rms);
+  return 0;
 }
 
 template <typename T>
@@ -565,6 +646,15 @@ static int norm_bwd_launch(const void* dy, const void* h, const float* gamma, co
   constexpr int V = 16 / sizeof(T);
   if (N % V) return -2;
   const int nvec = N / V;
+  if (sizeof(T) == 2 && nvec <= 32 * 8) {
+#define PF_NORM_BWD_FUSED(NV)                                                                     \
+    norm_bwd_fused_launch<T, NV>(dy, h, gamma, mean, rstd, dres, dx, scratch, G, rows, N, rms, st)
+    if (nvec <= 32 * 2) return PF_NORM_BWD_FUSED(2);
+    if (nvec <= 32 * 4) return PF_NORM_BWD_FUSED(4);
+    if (nvec <= 32 * 6) return PF_NORM_BWD_FUSED(6);
+    return PF_NORM_BWD_FUSED(8);
+#undef PF_NORM_BWD_FUSED
+  }
   if (sizeof(T) == 2 && nvec <= 32 * 16) {
     // input gradient: warp per row (rows of up to 4096 16-bit elements: Llama's hidden size);
     // parameter gradients: column reduction over row slabs
@@ -572,11 +662,7 @@ static int norm_bwd_launch(const void* dy, const void* h, const float* gamma, co
 #define PF_NORM_BWD_DX(NV)                                                                   \
     norm_bwd_dx_kernel<T, NV><<<grid, 256, 0, st>>>((const T*)dy, (const T*)h, gamma, mean,  \
         rstd, (const T*)dres, (T*)dx, rows, N, rms)
-    if (nvec <= 32 * 2) PF_NORM_BWD_DX(2);
-    else if (nvec <= 32 * 4) PF_NORM_BWD_DX(4);
-    else if (nvec <= 32 * 6) PF_NORM_BWD_DX(6);
-    else if (nvec <= 32 * 8) PF_NORM_BWD_DX(8);
-    else if (nvec <= 32 * 12) PF_NORM_BWD_DX(12);
+    if (nvec <= 32 * 12) PF_NORM_BWD_DX(12);
     else PF_NORM_BWD_DX(16);
 #undef PF_NORM_BWD_DX
     // enough row slabs to fill the GPU once with (column blocks x slabs) CTAs, few enough
@@ -657,8 +743,8 @@ PF_API int pf_norm_bwd(const void* dy, const void* h, const void* gamma, const v
   if (r) return r;
   PF_CHECK_LAUNCH();
   if (G > 0) {
-    norm_bwd_finish_kernel<<<(N + 255) / 256, 256, 0, st>>>((const float*)scratch, (float*)dgamma,
-                                                            (float*)dbeta, G, N, accumulate);
+    norm_bwd_finish_kernel<<<(N + 31) / 32, 1024, 0, st>>>((const float*)scratch, (float*)dgamma,
+                                                           (float*)dbeta, G, N, accumulate);
     PF_CHECK_LAUNCH();
   }
   return 0;

@@ -63,3 +63,44 @@ def test_cross_entropy_masked_vocabulary_and_all_ignored():
     loss = ops.cross_entropy(y, none)
     (dy,) = torch.autograd.grad(loss, y)
     assert float(loss.detach()) == 0.0 and not dy.any()
+
+
+@pytest.mark.parametrize("rms", [False, True])
+@pytest.mark.parametrize("rows,N", [(1, 8), (7, 24), (8, 192), (9, 256), (300, 264), (2371, 1408),
+                                    (5, 2040), (4999, 2048), (33, 2056), (640, 520)])
+def test_norm_backward_tiles(rows, N, rms):
+    """Gradients of the residual norm at the edges of the row tiles and column shares; twice, the
+    second time into recycled scratch, and into existing gradients."""
+    from pfeife_b200 import ops
+    from pfeife_b200.ops import kernels as kx
+    g = torch.Generator(device="cuda").manual_seed(rows + N)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    dtype = torch.bfloat16
+    x, res, gy, gh = ((rnd(rows, N) * 2).to(dtype) for _ in range(4))
+    w, b = 1 + 0.1 * rnd(N), 0.1 * rnd(N)
+    xr, wr, br = (t.double().requires_grad_() for t in ((x + res), w, b))
+    if rms:
+        want = xr * torch.rsqrt(xr.square().mean(-1, keepdim=True) + 1e-5) * wr
+    else:
+        want = F.layer_norm(xr, (N,), wr, br, 1e-5)
+    wants = torch.autograd.grad(want, (xr, wr) if rms else (xr, wr, br), gy.double())
+    for _ in range(2):
+        leaves = [t.clone().requires_grad_() for t in (x, res, w, b)]
+        if rms:
+            y, h = ops.rms_norm(leaves[0], leaves[2], 1e-5, residual=leaves[1])
+        else:
+            y, h = ops.layer_norm(*[leaves[i] for i in (0, 2, 3)], 1e-5, residual=leaves[1])
+        wrt = (leaves[0], leaves[2]) if rms else (leaves[0], leaves[2], leaves[3])
+        grads = torch.autograd.grad((y, h), wrt, (gy, gh))
+        close(y, want, U[dtype])
+        # dx is rounded once, after the gradient of the sum was added to it
+        close(grads[0], wants[0] + gh.double(), 1.5 * U[dtype])
+        for got, ref in zip(grads[1:], wants[1:]):
+            close(got, ref, 1e-5)
+    _, _, mean, rstd = kx.norm_fwd(x + res, w, None if rms else b, 1e-5, rms)
+    dw, db = torch.ones(N, device="cuda"), torch.ones(N, device="cuda")
+    kx.norm_bwd(gy, x + res, w, mean, rstd, rms, dgamma=dw, dbeta=None if rms else db,
+                accumulate=True, want_dbeta=False)
+    close(dw, wants[1] + 1, 1e-5)
+    if not rms:
+        close(db, wants[2] + 1, 1e-5)
