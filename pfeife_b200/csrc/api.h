@@ -124,17 +124,14 @@ PF_DECL int pf_im2col(const void* x, void* cols, int B, int H, int W, int C, int
 PF_DECL int pf_col2im(const void* dcols, void* dx, int B, int H, int W, int C, int KH, int KW,
                       int Ho, int Wo, int stride, int pad, long long ldc, int dtype, int sm_count,
                       void* stream);
+PF_DECL int pf_groupnorm_slabs(int B, int HW, int C, int sm_count);
 PF_DECL int pf_groupnorm_fwd(const void* x, const void* gamma, const void* beta, void* y,
-                             void* mean, void* rstd, int B, int HW, int C, int G, float eps,
-                             int act_silu, int dtype, int sm_count, void* stream);
+                             void* mean, void* rstd, void* scratch, int B, int HW, int C, int G,
+                             float eps, int act_silu, int dtype, int sm_count, void* stream);
 PF_DECL int pf_groupnorm_bwd(const void* dy, const void* x, const void* mean, const void* rstd,
                              const void* gamma, const void* beta, void* dx, void* dgamma,
-                             void* dbeta, void* sums, int B, int HW, int C, int G, int act_silu,
-                             int dtype, int sm_count, void* stream);
-PF_DECL int pf_conv_pack(const void* w, void* out, int Cout, int Cin, int taps, int cout8, int cin8,
-                         int flip, void* stream);
-PF_DECL int pf_conv_unpack(const void* src, void* dw, int Cout, int Cin, int taps, int cin8,
-                           int dtype, void* stream);
+                             void* dbeta, void* sums, void* scratch, int B, int HW, int C, int G,
+                             int act_silu, int accumulate, int dtype, int sm_count, void* stream);
 PF_DECL int pf_upsample2x(const void* x, void* y, int B, int H, int W, int C, int backward,
                           int dtype, int sm_count, void* stream);
 

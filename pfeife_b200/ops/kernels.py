@@ -584,6 +584,11 @@ def col2im(dcols: torch.Tensor, shape, KH: int, KW: int, stride: int, pad: int) 
     return dx
 
 
+def _groupnorm_scratch(L, B: int, HW: int, C: int, width: int, device) -> torch.Tensor:
+    slabs = L.pf_groupnorm_slabs(B, HW, C, sm_count(device))
+    return torch.empty((B, slabs, 2, width), dtype=torch.float32, device=device)
+
+
 def groupnorm_fwd(x: torch.Tensor, gamma: torch.Tensor, beta: torch.Tensor, groups: int,
                   eps: float, silu: bool):
     """x NHWC [B, H, W, C] -> (y, mean[B*G], rstd[B*G])."""
@@ -593,9 +598,10 @@ def groupnorm_fwd(x: torch.Tensor, gamma: torch.Tensor, beta: torch.Tensor, grou
     y = torch.empty_like(x)
     mean = torch.empty(B * groups, dtype=torch.float32, device=x.device)
     rstd = torch.empty_like(mean)
+    scratch = _groupnorm_scratch(L, B, H * W, C, groups, x.device)
     check(L.pf_groupnorm_fwd(ptr(x), ptr(gamma.float()), ptr(beta.float()), ptr(y), ptr(mean),
-                             ptr(rstd), B, H * W, C, groups, c_f(eps), int(silu), dt(x.dtype),
-                             sm_count(x.device), stream()), "pf_groupnorm_fwd")
+                             ptr(rstd), ptr(scratch), B, H * W, C, groups, c_f(eps), int(silu),
+                             dt(x.dtype), sm_count(x.device), stream()), "pf_groupnorm_fwd")
     return y, mean, rstd
 
 
@@ -604,13 +610,14 @@ def groupnorm_bwd(dy, x, mean, rstd, gamma, beta, groups: int, silu: bool):
     x, dy = x.contiguous(), dy.contiguous()
     B, H, W, C = x.shape
     dx = torch.empty_like(x)
-    dgamma = torch.zeros(C, dtype=torch.float32, device=x.device)
-    dbeta = torch.zeros(C, dtype=torch.float32, device=x.device)
+    dgamma = torch.empty(C, dtype=torch.float32, device=x.device)
+    dbeta = torch.empty(C, dtype=torch.float32, device=x.device)
     sums = torch.empty(2 * B * groups, dtype=torch.float32, device=x.device)
+    scratch = _groupnorm_scratch(L, B, H * W, C, C + groups, x.device)
     check(L.pf_groupnorm_bwd(ptr(dy), ptr(x), ptr(mean), ptr(rstd), ptr(gamma.float()),
-                             ptr(beta.float()), ptr(dx), ptr(dgamma), ptr(dbeta), ptr(sums), B,
-                             H * W, C, groups, int(silu), dt(x.dtype), sm_count(x.device),
-                             stream()), "pf_groupnorm_bwd")
+                             ptr(beta.float()), ptr(dx), ptr(dgamma), ptr(dbeta), ptr(sums),
+                             ptr(scratch), B, H * W, C, groups, int(silu), 0, dt(x.dtype),
+                             sm_count(x.device), stream()), "pf_groupnorm_bwd")
     return dx, dgamma, dbeta
 
 

@@ -65,6 +65,31 @@ def test_cross_entropy_masked_vocabulary_and_all_ignored():
     assert float(loss.detach()) == 0.0 and not dy.any()
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("silu", [True, False])
+@pytest.mark.parametrize("B,H,W,C,G", [(1, 1, 1, 32, 8), (2, 5, 7, 8, 2), (3, 16, 16, 32, 8),
+                                       (1, 37, 37, 320, 32), (2, 9, 3, 2048, 32),
+                                       (1, 4, 4, 2560, 32), (5, 64, 64, 96, 32)])
+def test_group_norm_edges(B, H, W, C, G, silu, dtype):
+    from pfeife_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(C + H)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    x = (rnd(B, H, W, C) * 2 + rnd(C)).to(dtype).requires_grad_()
+    w, b = (1 + 0.2 * rnd(C)).requires_grad_(), (0.2 * rnd(C)).requires_grad_()
+    dy = rnd(B, H, W, C).to(dtype)
+    xr, wr, br = (t.detach().double().requires_grad_() for t in (x, w, b))
+    want = F.group_norm(xr.permute(0, 3, 1, 2), G, wr, br, 1e-5).permute(0, 2, 3, 1)
+    want = F.silu(want) if silu else want
+    wants = torch.autograd.grad(want, (xr, wr, br), dy.double())
+    for _ in range(2):               # the second time into recycled scratch
+        y = ops.group_norm(x, w, b, G, 1e-5, silu)
+        grads = torch.autograd.grad(y, (x, w, b), dy)
+        close(y, want, U[dtype])
+        for got, ref in zip(grads, wants):
+            # groups of a few values lose digits in E[x^2] - E[x]^2 and in the differences of dx
+            close(got, ref, (U[dtype] if got.dtype == dtype else 0.0) + (2e-4 if H * W < 64 else 0))
+
+
 @pytest.mark.parametrize("rms", [False, True])
 @pytest.mark.parametrize("rows,N", [(1, 8), (7, 24), (8, 192), (9, 256), (300, 264), (2371, 1408),
                                     (5, 2040), (4999, 2048), (33, 2056), (640, 520)])
