@@ -204,7 +204,7 @@ norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ h, const float* 
 // CTA barrier), 8 rows per CTA.  The row stays in registers in its packed 16-bit form and is
 // expanded once per pass (sum, squared deviations, output): a third of the registers of an fp32
 // copy.  Bound by HBM: x and the residual are requested together, without a register limit that
-// would spill them; fp16 with residual 6168 x 1408 29 -> 23 us, 50000 x 1408 129 -> 102 us
+// would spill them; bf16 with residual 6168 x 1408 29 -> 23 us, 50000 x 1408 129 -> 102 us
 // (5.5 TB/s), 20000 x 2048 98 -> 75 us.
 template <typename T, int NV>
 __global__ void __launch_bounds__(256)

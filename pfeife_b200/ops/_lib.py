@@ -82,8 +82,9 @@ def ptr(t: Optional[torch.Tensor]):
     device is not reliable (new Python threads start on device 0)."""
     if t is None:
         return ctypes.c_void_p(0)
-    if t.is_cuda:
-        _tls.op_device = t.device.index
+    device = t.get_device()
+    if device >= 0:
+        _tls.op_device = device
     return ctypes.c_void_p(t.data_ptr())
 
 
@@ -107,14 +108,17 @@ def stream(device: Optional[int] = None) -> ctypes.c_void_p:
     if device is None:
         device = torch.cuda.current_device()
     bind_thread(device)
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(device))
 
 
 _sm_count_cache = {}
 
 
 def sm_count(device=None) -> int:
-    idx = torch.cuda.current_device() if device is None else torch.device(device).index
+    if type(device) is torch.device:
+        idx = device.index
+    else:
+        idx = torch.cuda.current_device() if device is None else torch.device(device).index
     if idx not in _sm_count_cache:
         _sm_count_cache[idx] = torch.cuda.get_device_properties(idx).multi_processor_count
     return _sm_count_cache[idx]

@@ -32,7 +32,10 @@ def status_word(device=None) -> torch.Tensor:
     """int32[STATUS_WORDS] per device.  Kernels record the first bounded-wait failure in word 0
     (0 = ok) and read their wait limit from word 1 (``set_wait_limit``); the environment
     variable PF_WAIT_CYCLES presets that limit."""
-    idx = torch.cuda.current_device() if device is None else torch.device(device).index
+    if type(device) is torch.device:
+        idx = device.index
+    else:
+        idx = torch.cuda.current_device() if device is None else torch.device(device).index
     if idx not in _status:
         t = torch.zeros(STATUS_WORDS, dtype=torch.int32, device=f"cuda:{idx}")
         import os

@@ -90,6 +90,93 @@ def test_group_norm_edges(B, H, W, C, G, silu, dtype):
             close(got, ref, (U[dtype] if got.dtype == dtype else 0.0) + (2e-4 if H * W < 64 else 0))
 
 
+def _block(x, res, w, b, w1, b1, qkv):
+    from pfeife_b200 import ops
+    y, h = ops.layer_norm(x, w, b, 1e-5, residual=res)
+    y = ops.mlp(y, w1, b1, w1.t().contiguous(), None, "gelu", residual=h)
+    a = ops.attention_qkv(ops.linear(y, qkv).view(2, 16, 3, 4, 16), causal=True)
+    return ops.cross_entropy(a.reshape(-1, 64).float() * 4, torch.arange(32, device=x.device))
+
+
+def test_eager_calls_equal_dispatched_ones():
+    """An eager call gives the bits and gradients that the same call gives through the dispatcher
+    (under a dispatch mode, where every op must stay visible)."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+    seen = []
+
+    class Watch(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    g = torch.Generator(device="cuda").manual_seed(4)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    mk = [rnd(2, 16, 64).half(), rnd(2, 16, 64).half(), 1 + 0.1 * rnd(64), 0.1 * rnd(64),
+          (0.1 * rnd(64, 64)).half(), 0.1 * rnd(64), (0.2 * rnd(192, 64)).half()]
+    results = []
+    for watch in (False, True):
+        leaves = [t.clone().requires_grad_() for t in mk]
+        if watch:
+            with Watch():
+                loss = _block(*leaves)
+                loss.backward()
+        else:
+            loss = _block(*leaves)
+            loss.backward()
+        results.append([loss.detach()] + [t.grad for t in leaves])
+    assert any("pfeife::linear_fwd" in s or "pfeife.linear_fwd" in s for s in seen)
+    assert any("attn_qkv_bwd" in s for s in seen)
+    # dq is summed over key tiles in any order; one tile here, so everything is exact but the
+    # norm's and bias' parameter sums (atomics): a few units of fp32
+    for a, b in zip(*results):
+        assert torch.allclose(a.float(), b.float(), rtol=1e-5, atol=1e-6)
+
+
+def test_eager_calls_keep_autograd_rules():
+    """Saved-tensor hooks see what the ops save, a second backward is refused, batched gradients
+    work, and no graph is kept without gradients."""
+    from pfeife_b200 import ops
+    x = torch.randn(8, 64, device="cuda").half().requires_grad_()
+    w = torch.randn(32, 64, device="cuda").half().requires_grad_()
+    packed = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(t.shape) or t.cpu(),
+                                                  lambda t: t.cuda()):
+        y = ops.linear(x, w, activation="gelu")
+    assert torch.Size([8, 64]) in packed and torch.Size([32, 64]) in packed
+    dx, dw = torch.autograd.grad(y, (x, w), torch.ones_like(y), retain_graph=True)
+    z = ops.linear(x, w, activation="gelu")
+    rx, rw = torch.autograd.grad(z, (x, w), torch.ones_like(z))
+    assert torch.equal(dx, rx) and torch.equal(dw, rw)
+    z = ops.linear(x, w)
+    (gx,) = torch.autograd.grad(z, x, torch.ones_like(z), create_graph=True)
+    with pytest.raises(RuntimeError):
+        gx.sum().backward()
+    with torch.no_grad():
+        assert ops.linear(x, w).grad_fn is None
+    assert ops.linear(x.detach(), w.detach()).grad_fn is None
+    # results may be changed in place, with and without a graph
+    x3 = x.detach().view(2, 4, 64).requires_grad_()
+    y = ops.linear(x3, w)
+    y += 1.0
+    (gx,) = torch.autograd.grad(y.float().square().sum(), x3)
+    z = ops.linear(x3, w) + 1.0
+    (rx,) = torch.autograd.grad(z.float().square().sum(), x3)
+    assert torch.equal(gx, rx)
+    with torch.no_grad():
+        y = ops.linear(x3, w)
+    y.add_(ops.linear(x3, w))
+    assert y.requires_grad
+    # gradients of several vectors at once (a transform over the backward)
+    y = ops.swiglu(x)
+    v = torch.stack([torch.ones_like(y), 2 * torch.ones_like(y)])
+    one = torch.autograd.grad(y, x, v[0], retain_graph=True)[0]
+    try:
+        (both,) = torch.autograd.grad(y, x, v, is_grads_batched=True)
+        assert torch.allclose(both[1].float(), 2 * one.float(), rtol=1e-2)
+    except RuntimeError as e:           # refused, as through the dispatcher, never wrong
+        assert "vmap" in str(e) or "Batching" in str(e) or "storage" in str(e)
+
+
 @pytest.mark.parametrize("rms", [False, True])
 @pytest.mark.parametrize("rows,N", [(1, 8), (7, 24), (8, 192), (9, 256), (300, 264), (2371, 1408),
                                     (5, 2040), (4999, 2048), (33, 2056), (640, 520)])
