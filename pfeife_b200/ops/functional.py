@@ -1094,9 +1094,9 @@ def attn_qkv_bwd(do: Tensor, qkv: Tensor, o: Tensor, lse: Tensor, causal: bool,
     """-> d(qkv) [B, S, 3, H, D], written in place by the backward kernels (no concatenation)."""
     q, k, v = qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2]
     if _native(qkv) and kx.attention_supported(q, k, v):
-        dq, _, _ = kx.attn_bwd(do, q, k, v, o, lse, causal, scale, packed=True)
-        return dq._base if dq._base is not None else torch.stack(
-            kx.attn_bwd(do, q, k, v, o, lse, causal, scale), dim=2)
+        dqkv = torch.empty(qkv.shape, dtype=qkv.dtype, device=qkv.device)
+        kx.attn_bwd(do, q, k, v, o, lse, causal, scale, packed=True, dqkv=dqkv)
+        return dqkv
     dq, dk, dv = attn_bwd.plain(do, q, k, v, o, lse, causal, scale)
     return torch.stack([dq, dk, dv], dim=2)
 

@@ -439,10 +439,11 @@ def attn_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: bool, sc
 
 def attn_bwd(do: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
              o: torch.Tensor, lse: torch.Tensor, causal: bool, scale: float,
-             packed: bool = False) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+             packed: bool = False, dqkv: Optional[torch.Tensor] = None
+             ) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     """-> (dq, dk, dv).  With ``packed`` (self-attention on slices of one fused projection) the
-    three gradients are slices of a single [B, S, 3, H, D] buffer, i.e. the gradient of the
-    fused projection needs no concatenation."""
+    three gradients are slices of a single [B, S, 3, H, D] buffer, ``dqkv`` when given, i.e. the
+    gradient of the fused projection needs no concatenation."""
     L = _lib.lib()
     B, Sq, H, D = q.shape
     Sk = k.shape[1]
@@ -451,7 +452,9 @@ def attn_bwd(do: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor
     q, k, v = fix(q), fix(k), fix(v)
     do, o = do.contiguous(), o.contiguous()
     if packed and Sq == Sk:
-        dqkv = torch.empty((B, Sq, 3, H, D), dtype=q.dtype, device=q.device)
+        if dqkv is None:
+            dqkv = torch.empty((B, Sq, 3, H, D), dtype=q.dtype, device=q.device)
+        assert dqkv.shape == (B, Sq, 3, H, D) and dqkv.dtype == q.dtype and dqkv.is_contiguous()
         dq, dk, dv = dqkv[:, :, 0], dqkv[:, :, 1], dqkv[:, :, 2]
     else:
         dq = torch.empty((B, Sq, H, D), dtype=q.dtype, device=q.device)

@@ -132,6 +132,17 @@ def test_eager_calls_equal_dispatched_ones():
         assert torch.allclose(a.float(), b.float(), rtol=1e-5, atol=1e-6)
 
 
+def test_eager_backward_launches_each_kernel_once():
+    """The packed attention backward is one native call, whichever way the op was called."""
+    from pfeife_b200 import ops
+    from pfeife_b200.ops import _lib
+    qkv = torch.randn(1, 64, 3, 2, 32, device="cuda").half().requires_grad_()
+    o = ops.attention_qkv(qkv)
+    before = _lib.launch_count()
+    (dqkv,) = torch.autograd.grad(o, qkv, torch.ones_like(o))
+    assert _lib.launch_count() == before + 1 and dqkv.is_contiguous()
+
+
 def test_eager_calls_keep_autograd_rules():
     """Saved-tensor hooks see what the ops save, a second backward is refused, batched gradients
     work, and no graph is kept without gradients."""
