@@ -6,22 +6,35 @@
 // (88 for ViT-g/14 runs as 96 with zero-filled tails: the tensor map's inner extent is D, so
 // the tail of the last 64-element block is filled with zeros by TMA, never with the next head).
 //
-// Forward: a persistent kernel, one CTA per SM walking over (q tile of 128, head, batch) items,
-// with a TMA producer warp (K and V rings), an MMA issuer warp and four softmax warps (thread
-// <-> query row <-> TMEM lane); per 128-row K/V tile:
-//     S = Q K^T            tcgen05.mma, smem x smem -> one of two S buffers in TMEM; the next
-//                          tile's S is issued before this tile's probabilities are waited for
-//     online softmax       one tcgen05.ld of S -> registers (base-2 exponent, running max / sum)
-//     P -> smem            16-bit, in the 128B-swizzled K-major layout the MMA reads; two buffers
-//     O += P V             tcgen05.mma, V in place as an MN-major operand, O accumulated in TMEM
-//                          and rescaled there only when the row maximum grew by more than 2^8
-// The score matrix never exists in global memory.  (Details at attn_fwd_ws_kernel.)
+// A persistent kernel, one CTA per SM, walks over items of up to 256 query rows of one (head,
+// batch): two query tiles of 128 that share every K / V tile it loads.  Its warps:
+//   warps 0-3 / 4-7   softmax of query tile 0 / 1, thread <-> query row <-> TMEM lane
+//   warp 8            TMA producer (K and V rings; runs ahead, across item boundaries too)
+//   warp 9            MMA issuer, TMEM owner                   warps 10, 11  idle
+// Per query tile t and key tile j:
+//     S_t = Q_t K_j^T   tcgen05.mma, shared memory x shared memory -> TMEM
+//     online softmax    S_t read once into registers, base-2 exponent, running maximum and sum
+//     P_t -> TMEM       16-bit, read by the next product as its A operand; P never touches
+//                       shared memory
+//     O_t += P_t V_j    accumulated in TMEM and rescaled there only when the row maximum grew by
+//                       more than 2^8 since it was last set (P stays below 2^8, which both 16-bit
+//                       formats hold, and most tiles need no rescaling)
+// What bounds it: 16384 exponentials per tile, 1024 cycles of the special-function units, against
+// 16 x head dim cycles of tensor core.  Two tiles in flight keep one tile's products under the
+// other's exponentials.
+// Measured (B200, CUDA events, L2 flushed), against one query tile per CTA with P in shared
+// memory: [4, 4096, 10, 64] 402 -> 346 us, causal [1, 2048, 32, 128] 87 -> 59,
+// [2, 2048, 16, 128] 114 -> 96, causal [6, 1782, 21, 32] 200 -> 117, 77 keys [4, 1024, 20, 64]
+// 32 -> 22, [24, 257, 16, 88] 62 -> 58.
+// TMEM (512 columns): S_0, S_1 128 each, O_0, O_1 one head dim each.  Up to head dim 64 P_0, P_1
+// have 64 columns of their own, so S of the next key tile is issued as soon as this one's scores
+// are in registers; above, P_t takes the columns of S_t and the next S_t waits until P_t V has
+// read it.
 //
 // Short tails.  A sequence length just above a multiple of 128 (ViT: 257 = 2 x 128 + the class
-// token) would spend a whole 128-row query tile on a few rows.  When at most ATT_TAIL_MAX rows are
-// left over, the tensor-core tiles cover only the full multiples and a small CUDA-core kernel
-// computes the leftover query rows.
-#include <cstdlib>
+// token) would spend a whole item on a few rows.  When at most ATT_TAIL_MAX rows are left over, the
+// tensor-core tiles cover only the full multiples and a small CUDA-core kernel computes the
+// leftover query rows ([24, 257, 16, 88]: 68 -> 58 us).
 #include "attn_common.cuh"
 #include "api.h"
 
@@ -34,14 +47,16 @@ struct AttnParams {
   int B, H, Sq, Sk, D;
   int causal;
   float scale;
-  int fmt;  // 0 fp16, 1 bf16
-  void* o;              // fwd: out [B,Sq,H,D] contiguous
+  int fmt;              // 0 fp16, 1 bf16
+  void* o;              // [B,Sq,H,D] contiguous
   float* lse;           // [B,H,Sq]
   int* status;
-  // raw views for the CUDA-core tail path of the forward (element strides: batch, seq, head)
+  int q_rows;           // query rows of the tensor-core kernel; the others are leftover rows
+  int q_pairs;          // items per head: ceil(q_rows / 256)
+  int q_tail;           // leftover rows
+  // raw views for the leftover rows (element strides: batch, seq, head)
   const void* q; const void* k; const void* v;
   long long sq[3], sk[3], sv[3];
-  int q_tiles, q_tail;  // tensor-core query tiles; leftover query rows after them
 };
 
 __device__ __forceinline__ float block_reduce(float v, float* red, bool is_max) {
@@ -152,60 +167,127 @@ __device__ void attn_fwd_tail_row(const AttnParams& p, uint8_t* smem, int qi, in
     p.lse[((long long)b * p.H + h) * p.Sq + qi] = (l > 0.f) ? (mx + log2f(l)) * LN2 : -INFINITY;
 }
 
-
 // Leftover rows in kernels of their own: small shared memory and block size, so that many of
 // these latency-bound CTAs share an SM instead of each holding a tensor-core CTA's resources.
 template <typename T>
 __global__ void __launch_bounds__(128)
 attn_fwd_tail_kernel(const AttnParams p) {
   extern __shared__ uint8_t tail_smem[];
-  attn_fwd_tail_row<T>(p, tail_smem, p.q_tiles * ATT_BM + (int)blockIdx.x, blockIdx.y, blockIdx.z);
+  attn_fwd_tail_row<T>(p, tail_smem, p.q_rows + (int)blockIdx.x, blockIdx.y, blockIdx.z);
 }
-// ================================================================================ forward
-// Persistent, warp-specialised forward.  One CTA per SM walks over (q tile, head, batch) work
-// items; its 6 warps have fixed roles:
-//   warp 0     TMA producer: Q of the item, then K / V tiles into a ring of ST stages; it runs
-//              ahead of the consumers, across item boundaries too
-//   warp 1     MMA issuer: S_j = Q K_j^T into one of two S buffers in TMEM, O (+)= P_j V_j into
-//              the O accumulator in TMEM.  S_{j+1} is issued BEFORE it waits for P_j, so the
-//              tensor core computes the next scores while the softmax warps work on this tile
-//   warps 2-5  softmax, thread <-> query row <-> TMEM lane: one read of S, running maximum,
-//              P = exp2(S c - m) written to shared memory in the layout the P V product reads
-// P has two buffers, so a tile's probabilities are computed and stored while the previous
-// tile's P V still runs.  O stays in TMEM for the whole item.  The row maximum that scales P is only raised when the
-// true maximum has grown by more than 2^8 since it was last set; then the row of O (and the
-// running sum) is rescaled in place (tcgen05.ld / st).  P therefore stays below 2^8, which both
-// 16-bit formats hold, and most tiles need no rescaling at all.
-// TMEM: S0 [0,128) S1 [128,256) O [256, 256+DP) of 512 allocated columns.
+
+// Products over [128 rows x 64] blocks in shared memory, issued by a converged warp (`on`: its
+// issuing lane).  Fully unrolled, so that a step costs an addition per operand.
+// A[128 x K] (K-major blocks) . B[N x K]^T (K-major blocks), K = KSTEPS * 16
+template <int KSTEPS>
+__device__ __forceinline__ void mma_kk_on(uint32_t on, uint32_t d_tmem, uint32_t sa, uint32_t sb,
+                                          uint32_t idesc) {
+  const uint32_t a = desc_lo(sa, 16), b = desc_lo(sb, 16);
+#pragma unroll
+  for (int k = 0; k < KSTEPS; ++k) {
+    const uint32_t off = ((k >> 2) * ATT_BLK + (k & 3) * 32) >> 4;
+    tc_mma_f16_on(on, d_tmem, a + off, b + off, idesc, k > 0);
+  }
+}
+// A in TMEM (16-bit pairs, 8 columns per step), B given as [K=128 rows][N] (N contiguous)
+__device__ __forceinline__ void mma_t_mn_on(uint32_t on, uint32_t d_tmem, uint32_t ta, uint32_t sb,
+                                            uint32_t idesc, bool accumulate_first, int ksteps) {
+  const uint32_t b = desc_lo(sb, ATT_BLK);
+#pragma unroll
+  for (int k = 0; k < 8; ++k)
+    if (k < ksteps)
+      tc_mma_f16_ts_on(on, d_tmem, ta + k * 8, b + (k * 2048 >> 4), idesc,
+                       k > 0 || accumulate_first);
+}
+
+
 template <int DP>
 struct FwdCfg {
   static constexpr int NBLK = (DP + 63) / 64;
   static constexpr int TILE = NBLK * ATT_BLK;
-  static constexpr int ST = NBLK >= 2 ? 2 : 3;          // K/V ring stages
-  static constexpr int OFF_K = TILE;
+  static constexpr bool ALIAS_P = DP > 64;
+  static constexpr int ST = NBLK >= 2 ? 2 : 4;          // K/V ring stages
+  static constexpr int OFF_K = 2 * TILE;
   static constexpr int OFF_V = OFF_K + ST * TILE;
-  static constexpr int OFF_P = OFF_V + ST * TILE;       // two buffers of [128 q][128 kv] 16-bit
-  static constexpr int P_BYTES = 2 * ATT_BLK;           // (two swizzled blocks each)
-  static constexpr int OFF_BAR = OFF_P + 2 * P_BYTES;
-  static constexpr int SMEM = OFF_BAR + 256 + 1024;     // barriers + alignment slack
-  static constexpr int THREADS = 192;
+  static constexpr int OFF_BAR = OFF_V + ST * TILE;
+  static constexpr int SMEM = OFF_BAR + 256;
+  static constexpr int T_O = 256;                        // + t * DP
+  static constexpr int T_P = ALIAS_P ? 0 : 256 + 2 * DP;
+  static constexpr int P_TILE = ALIAS_P ? 128 : 64;      // column distance of P_0 and P_1
+  // three warpgroups of 168 registers a thread at launch; the softmax ones hold a row of scores
+  static constexpr int THREADS = 384;
+  static constexpr int REGS_SOFTMAX = 216, REGS_OTHER = 72;
+  static_assert(2 * REGS_SOFTMAX + REGS_OTHER <= 3 * 168, "registers of the block");
+  static_assert(SMEM <= 232448, "shared memory per CTA");
+  static_assert((ALIAS_P ? T_O + 2 * DP : T_P + 128) <= 512, "TMEM columns");
 };
 
 struct FwdItem {
-  int q0, h, b, n_tiles;
+  int q0, h, b, n[2];    // first query row; key tiles seen by the two query tiles
 };
 __device__ __forceinline__ FwdItem fwd_item(const AttnParams& p, int w) {
   FwdItem it;
-  // causal: the later query tiles see more keys; they go first so the long items start early
-  const int qt = p.causal ? (p.q_tiles - 1 - w % p.q_tiles) : (w % p.q_tiles);
-  it.q0 = qt * ATT_BM;
-  const int r = w / p.q_tiles;
-  it.h = r % p.H;
-  it.b = r / p.H;
-  int kv_end = p.Sk;
-  if (p.causal) kv_end = min(p.Sk, it.q0 + ATT_BM + (p.Sk - p.Sq));
-  it.n_tiles = kv_end > 0 ? (kv_end + ATT_BN - 1) / ATT_BN : 0;
+  int qp, bh;
+  if (p.causal) {
+    // later queries see more keys: the long items of every head are dealt first
+    qp = w / (p.B * p.H);
+    bh = w - qp * (p.B * p.H);
+    qp = p.q_pairs - 1 - qp;
+  } else {
+    bh = w / p.q_pairs;
+    qp = w - bh * p.q_pairs;
+  }
+  it.q0 = qp * 2 * ATT_BM;
+  it.h = bh % p.H;
+  it.b = bh / p.H;
+#pragma unroll
+  for (int t = 0; t < 2; ++t) {
+    const int q0 = it.q0 + t * ATT_BM;
+    int kv_end = p.Sk;
+    if (p.causal) kv_end = min(p.Sk, q0 + ATT_BM + (p.Sk - p.Sq));
+    it.n[t] = (q0 < p.q_rows && kv_end > 0) ? (kv_end + ATT_BN - 1) / ATT_BN : 0;
+  }
   return it;
+}
+// rounds run alternately forwards and backwards over the CTAs, so that a CTA with a long item in
+// one round gets a short one in the next
+__device__ __forceinline__ int fwd_index(int r) {
+  const int slot = (r & 1) ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;
+  return r * (int)gridDim.x + slot;
+}
+
+// Probabilities of one row, packed to 16 bits; returns their fp32 sum (of the unrounded values).
+template <typename T, bool MASKED>
+__device__ __forceinline__ float probs(const uint32_t (&s)[4][32], uint32_t (&pk)[4][16], float c2,
+                                       float m_sub, int n_chunks, int lim) {
+  const uint64_t c2v = f2_pack(c2, c2), nm = f2_pack(-m_sub, -m_sub);
+  uint64_t r01 = 0, r23 = 0;                  // pairs of fp32 sums
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    if (!MASKED || c < n_chunks) {
+#pragma unroll
+      for (int i = 0; i < 32; i += 4) {
+        float e[4];
+        f2_unpack(fma2(f2_pack(__uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1])), c2v, nm),
+                  e[0], e[1]);
+        f2_unpack(fma2(f2_pack(__uint_as_float(s[c][i + 2]), __uint_as_float(s[c][i + 3])), c2v,
+                       nm), e[2], e[3]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          e[u] = exp2f(e[u]);
+          if (MASKED && c * 32 + i + u >= lim) e[u] = 0.f;
+        }
+        r01 = add2(r01, f2_pack(e[0], e[1]));
+        r23 = add2(r23, f2_pack(e[2], e[3]));
+        pk[c][i / 2] = pack2<T>(e[0], e[1]);
+        pk[c][i / 2 + 1] = pack2<T>(e[2], e[3]);
+      }
+    }
+  }
+  float a, b, d, e;
+  f2_unpack(r01, a, b);
+  f2_unpack(r23, d, e);
+  return (a + b) + (d + e);
 }
 
 template <typename T, int DP>
@@ -214,311 +296,311 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
                    const __grid_constant__ CUtensorMap tv, const AttnParams p, const int n_items) {
   using C = FwdCfg<DP>;
   constexpr int NBLK = C::NBLK, TILE = C::TILE, ST = C::ST;
-  constexpr uint32_t TMEM_COLS = 512;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                             ~uintptr_t(1023));
-  uint8_t* sQ = smem;
-  uint8_t* sK = smem + C::OFF_K;
-  uint8_t* sV = smem + C::OFF_V;
-  uint8_t* sP = smem + C::OFF_P;
+  extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::OFF_BAR);
-  uint64_t* bar_q_full = bars;            // TMA bytes of Q
-  uint64_t* bar_q_empty = bars + 1;       // last S product of the item has read Q
-  uint64_t* bar_k_full = bars + 2;        // [ST]
-  uint64_t* bar_v_full = bars + 2 + ST;   // [ST]
-  uint64_t* bar_k_empty = bars + 2 + 2 * ST;    // [ST] Q K^T of the tile has completed
-  uint64_t* bar_v_empty = bars + 2 + 3 * ST;    // [ST] P V of the tile has completed
-  uint64_t* bar_s_full = bars + 2 + 4 * ST;     // [2]
-  uint64_t* bar_s_empty = bar_s_full + 2;       // [2] the softmax warps hold S in registers
-  uint64_t* bar_p_full = bar_s_empty + 2;       // P is in shared memory (and O rescaled)
-  uint64_t* bar_pv_done = bar_p_full + 1;       // [2], by tile parity: P V has completed (that P
-                                                // buffer is free, O holds every tile up to it)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_pv_done + 2);
-  constexpr int N_BARS = 2 + 4 * ST + 7;
+  uint64_t* q_full = bars;               // [2] by query tile
+  uint64_t* q_empty = bars + 2;          // [2] the item's last S product of that tile is done
+  uint64_t* s_full = bars + 4;           // [2]
+  uint64_t* s_empty = bars + 6;          // [2] scores are in registers (P in columns of its own)
+  uint64_t* p_full = bars + 8;           // [2] P is in TMEM (and O rescaled)
+  uint64_t* pv_done = bars + 10;         // [2] P V has completed
+  uint64_t* k_full = bars + 12;          // [ST]
+  uint64_t* k_empty = k_full + ST;
+  uint64_t* v_full = k_empty + ST;
+  uint64_t* v_empty = v_full + ST;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(v_empty + ST);
+  constexpr int N_BARS = 12 + 4 * ST;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // the 128-byte swizzle works on absolute shared-memory addresses
+  if ((smem_u32(smem) & 1023u) != 0u) {
+    if (tid == 0) report(p.status, PF_ERR_BAD_ARG);
+    return;
+  }
   if (tid == 0) {
     tma_prefetch_desc(&tq); tma_prefetch_desc(&tk); tma_prefetch_desc(&tv);
     for (int i = 0; i < N_BARS; ++i) mbar_init(&bars[i], 1);
-    for (int i = 0; i < 2; ++i) mbar_init(&bar_s_empty[i], 4);   // lane 0 of each softmax warp
-    mbar_init(bar_p_full, 4);
+    for (int t = 0; t < 2; ++t) { mbar_init(&s_empty[t], 4); mbar_init(&p_full[t], 4); }
     mbar_fence_init();
   }
-  if (warp == 1) { tmem_alloc(tmem_slot, TMEM_COLS); tmem_relinquish(); }
+  if (warp == 9) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t t_o = tmem + 256;
 
-  if (warp == 0) {
-    // ---------------------------------------------------------------- TMA producer
-    if (lane == 0) {
-      uint32_t g = 0, qc = 0;
-      bool ok = true;
-      for (int w = blockIdx.x; w < n_items && ok; w += gridDim.x) {
-        const FwdItem it = fwd_item(p, w);
-        if (it.n_tiles == 0) continue;
-        ok = mbar_wait(bar_q_empty, (qc & 1) ^ 1, p.status, PF_ERR_TIMEOUT_EMPTY);
-        if (!ok) break;
-        load_tile<NBLK>(sQ, &tq, bar_q_full, it.h, it.q0, it.b);
-        ++qc;
-        // K runs one tile ahead of V: a K stage is free as soon as its Q K^T has completed, a V
-        // stage only after its P V, and the next scores are wanted first
-        auto load_v = [&](int j, uint32_t gv) -> bool {
-          const int st = gv % ST;
-          if (!mbar_wait(&bar_v_empty[st], ((gv / ST) & 1) ^ 1, p.status, PF_ERR_TIMEOUT_EMPTY))
-            return false;
-          load_tile<NBLK>(sV + st * TILE, &tv, &bar_v_full[st], it.h, j * ATT_BN, it.b);
-          return true;
-        };
-        for (int j = 0; j < it.n_tiles && ok; ++j) {
-          const uint32_t gk = g + j;
-          const int st = gk % ST;
-          ok = mbar_wait(&bar_k_empty[st], ((gk / ST) & 1) ^ 1, p.status, PF_ERR_TIMEOUT_EMPTY);
-          if (!ok) break;
-          load_tile<NBLK>(sK + st * TILE, &tk, &bar_k_full[st], it.h, j * ATT_BN, it.b);
-          if (j > 0) ok = load_v(j - 1, gk - 1);
+  // one split per warpgroup: its four warps execute the same instruction
+  if (warp >= 8) {
+    regs_dec<C::REGS_OTHER>();
+    if (warp == 8) {
+      // ---------------------------------------------------------------- TMA producer
+      if (lane == 0) {
+        uint32_t g = 0, qc[2] = {0, 0};
+        bool ok = true;
+        for (int r = 0; ok && r * (int)gridDim.x < n_items; ++r) {
+          const int w = fwd_index(r);
+          if (w >= n_items) continue;
+          const FwdItem it = fwd_item(p, w);
+          const int nmax = max(it.n[0], it.n[1]);
+          for (int j = 0; j < nmax && ok; ++j, ++g) {
+            const int st = g % ST;
+            if (j == 0 && it.n[0] > 0) {
+              ok = mbar_wait(&q_empty[0], (qc[0] & 1) ^ 1, p.status, PF_ERR_TIMEOUT_EMPTY);
+              if (!ok) break;
+              load_tile<NBLK>(smem, &tq, &q_full[0], it.h, it.q0, it.b);
+              ++qc[0];
+            }
+            ok = mbar_wait(&k_empty[st], ((g / ST) & 1) ^ 1, p.status, PF_ERR_TIMEOUT_EMPTY);
+            if (!ok) break;
+            load_tile<NBLK>(smem + C::OFF_K + st * TILE, &tk, &k_full[st], it.h, j * ATT_BN, it.b);
+            if (j == 0 && it.n[1] > 0) {
+              ok = mbar_wait(&q_empty[1], (qc[1] & 1) ^ 1, p.status, PF_ERR_TIMEOUT_EMPTY);
+              if (!ok) break;
+              load_tile<NBLK>(smem + TILE, &tq, &q_full[1], it.h, it.q0 + ATT_BM, it.b);
+              ++qc[1];
+            }
+            ok = mbar_wait(&v_empty[st], ((g / ST) & 1) ^ 1, p.status, PF_ERR_TIMEOUT_EMPTY);
+            if (!ok) break;
+            load_tile<NBLK>(smem + C::OFF_V + st * TILE, &tv, &v_full[st], it.h, j * ATT_BN, it.b);
+          }
         }
-        if (ok) ok = load_v(it.n_tiles - 1, g + it.n_tiles - 1);
-        g += it.n_tiles;
       }
-    }
-    __syncwarp();
-  } else if (warp == 1) {
-    // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
-      const uint32_t idesc_s = make_idesc_f16(128, 128, p.fmt, 0, 0);
-      const uint32_t idesc_o = make_idesc_f16(128, DP, p.fmt, 0, 1);
-      uint32_t g = 0, qc = 0;
-      bool ok = true;
-      // S of global tile `gg` (tile j of the item)
-      auto issue_s = [&](uint32_t gg, int j) -> bool {
-        const int st = gg % ST, sb = gg & 1;
-        if (!mbar_wait(&bar_k_full[st], (gg / ST) & 1, p.status, PF_ERR_TIMEOUT_FULL)) return false;
-        if (!mbar_wait(&bar_s_empty[sb], ((gg >> 1) & 1) ^ 1, p.status, PF_ERR_TIMEOUT_TMEM_EMPTY))
-          return false;
-        tc_fence_after();
-        const int rem = min(ATT_BN, p.Sk - j * ATT_BN);
-        const int n_mma = (rem + 15) / 16 * 16;
-        const uint32_t id = (n_mma == ATT_BN) ? idesc_s : make_idesc_f16(128, n_mma, p.fmt, 0, 0);
-        mma_kk<DP / 16>(tmem + sb * 128, smem_u32(sQ), smem_u32(sK + st * TILE), id, false);
-        tc_commit(&bar_k_empty[st]);
-        tc_commit(&bar_s_full[sb]);
-        return true;
-      };
-      for (int w = blockIdx.x; w < n_items && ok; w += gridDim.x) {
-        const FwdItem it = fwd_item(p, w);
-        if (it.n_tiles == 0) continue;
-        ok = mbar_wait(bar_q_full, qc & 1, p.status, PF_ERR_TIMEOUT_FULL);
-        ++qc;
-        ok = ok && issue_s(g, 0);
-        for (int j = 0; j < it.n_tiles && ok; ++j) {
-          const uint32_t gg = g + j;
-          if (j + 1 < it.n_tiles) ok = issue_s(gg + 1, j + 1);
-          else tc_commit(bar_q_empty);     // every S product of this item has been issued
-          if (!ok) break;
+      __syncwarp();
+    } else if (warp == 9) {
+      // ---------------------------------------------------------------- MMA issuer
+      {
+        const uint32_t on = lane == 0;
+        const uint32_t id_s = make_idesc_f16(128, 128, p.fmt, 0, 0);
+        const uint32_t id_o = make_idesc_f16(128, DP, p.fmt, 0, 1);
+        uint32_t g = 0, qc[2] = {0, 0}, cnt[2] = {0, 0};    // cnt: S tiles issued per query tile
+        bool ok = true;
+        // S_t of key tile j (ring position gg).  Its columns must be free: the previous scores are
+        // in registers, or (P in the same columns) the previous P V has read its probabilities.
+        auto issue_s = [&](int t, uint32_t gg, int j, int n, bool last_of_tile) -> bool {
           const int st = gg % ST;
-          ok = mbar_wait(bar_p_full, gg & 1, p.status, PF_ERR_TIMEOUT_FULL) &&
-               mbar_wait(&bar_v_full[st], (gg / ST) & 1, p.status, PF_ERR_TIMEOUT_FULL);
-          if (!ok) break;
+          if (j == 0) {
+            if (!mbar_wait_warp(&q_full[t], qc[t] & 1, p.status, PF_ERR_TIMEOUT_FULL)) return false;
+            ++qc[t];
+          }
+          if (!mbar_wait_warp(&k_full[st], (gg / ST) & 1, p.status, PF_ERR_TIMEOUT_FULL))
+            return false;
+          if (cnt[t] > 0 && !mbar_wait_warp(C::ALIAS_P ? &pv_done[t] : &s_empty[t],
+                                            (cnt[t] - 1) & 1, p.status,
+                                            PF_ERR_TIMEOUT_TMEM_EMPTY))
+            return false;
           tc_fence_after();
           const int rem = min(ATT_BN, p.Sk - j * ATT_BN);
-          mma_k_mn(t_o, smem_u32(sP + (gg & 1) * C::P_BYTES), smem_u32(sV + st * TILE), idesc_o,
-                   j > 0, (rem + 15) / 16);
-          tc_commit(&bar_v_empty[st]);
-          tc_commit(&bar_pv_done[gg & 1]);
+          const int n_mma = (rem + 15) / 16 * 16;
+          const uint32_t id = n_mma == ATT_BN ? id_s : make_idesc_f16(128, n_mma, p.fmt, 0, 0);
+          mma_kk_on<DP / 16>(on, tmem + t * 128, smem_u32(smem + t * TILE),
+                          smem_u32(smem + C::OFF_K + st * TILE), id);
+          if (last_of_tile) tc_commit_on(on, &k_empty[st]);
+          tc_commit_on(on, &s_full[t]);
+          if (j == n - 1) tc_commit_on(on, &q_empty[t]);
+          ++cnt[t];
+          return true;
+        };
+        for (int r = 0; ok && r * (int)gridDim.x < n_items; ++r) {
+          const int w = fwd_index(r);
+          if (w >= n_items) continue;
+          const FwdItem it = fwd_item(p, w);
+          const int nmax = max(it.n[0], it.n[1]);
+          // tile 1 reads every key tile that tile 0 reads, and after it
+          auto last_reader = [&](int t, int j) { return t == 1 || j >= it.n[1]; };
+#pragma unroll
+          for (int t = 0; t < 2; ++t)
+            if (ok && it.n[t] > 0) ok = issue_s(t, g, 0, it.n[t], last_reader(t, 0));
+          for (int j = 0; j < nmax && ok; ++j) {
+            const uint32_t gg = g + j;
+            const int st = gg % ST;
+            if (!C::ALIAS_P) {
+#pragma unroll
+              for (int t = 0; t < 2; ++t)
+                if (ok && j + 1 < it.n[t])
+                  ok = issue_s(t, gg + 1, j + 1, it.n[t], last_reader(t, j + 1));
+              if (!ok) break;
+            }
+            ok = mbar_wait_warp(&v_full[st], (gg / ST) & 1, p.status, PF_ERR_TIMEOUT_FULL);
+            if (!ok) break;
+            const int k_steps = (min(ATT_BN, p.Sk - j * ATT_BN) + 15) / 16;
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+              if (!ok || j >= it.n[t]) continue;
+              // the tile whose probabilities are waited for is the one before any S issued above
+              const uint32_t c = cnt[t] - 1 - ((!C::ALIAS_P && j + 1 < it.n[t]) ? 1u : 0u);
+              ok = mbar_wait_warp(&p_full[t], c & 1, p.status, PF_ERR_TIMEOUT_FULL);
+              if (!ok) continue;
+              tc_fence_after();
+              const uint32_t sV = smem_u32(smem + C::OFF_V + st * TILE);
+              const uint32_t t_p = tmem + C::T_P + t * C::P_TILE;
+              mma_t_mn_on(on, tmem + C::T_O + t * DP, t_p, sV, id_o, j > 0, k_steps);
+              if (last_reader(t, j)) tc_commit_on(on, &v_empty[st]);
+              tc_commit_on(on, &pv_done[t]);
+              if (C::ALIAS_P && j + 1 < it.n[t])
+                ok = issue_s(t, gg + 1, j + 1, it.n[t], last_reader(t, j + 1));
+            }
+          }
+          g += nmax;
         }
-        g += it.n_tiles;
       }
+      __syncwarp();
     }
-    __syncwarp();
   } else {
-    // ---------------------------------------------------------------- softmax (4 warps)
-    const int quad = warp & 3;                       // TMEM lane quadrant of this warp
+    // ---------------------------------------------------------------- softmax (2 x 4 warps)
+    regs_inc<C::REGS_SOFTMAX>();
+    const int t = warp >> 2, quad = warp & 3;
     const int row = quad * 32 + lane;
     const uint32_t lane_off = uint32_t(quad * 32) << 16;
+    const uint32_t t_s = tmem + t * 128 + lane_off;
+    const uint32_t t_o = tmem + C::T_O + t * DP + lane_off;
+    const uint32_t t_p = tmem + C::T_P + t * C::P_TILE + lane_off;
     const float c2 = p.scale * LOG2E;
     const int shift = p.Sk - p.Sq;
-    uint32_t g = 0;
+    uint32_t cnt = 0;
     bool ok = true;
-    for (int w = blockIdx.x; w < n_items && ok; w += gridDim.x) {
+    for (int r = 0; ok && r * (int)gridDim.x < n_items; ++r) {
+      const int w = fwd_index(r);
+      if (w >= n_items) continue;
       const FwdItem it = fwd_item(p, w);
-      const int qi = it.q0 + row;
+      const int q0 = it.q0 + t * ATT_BM, n_tiles = t ? it.n[1] : it.n[0];
+      const int qi = q0 + row;
+      if (q0 >= p.q_rows) continue;
       T* dst = reinterpret_cast<T*>(p.o) + (((long long)it.b * p.Sq + qi) * p.H + it.h) * p.D;
       float* lse_dst = p.lse + ((long long)it.b * p.H + it.h) * p.Sq + qi;
-      if (it.n_tiles == 0) {       // no key is visible to this query tile
+      if (n_tiles == 0) {          // no key is visible to this query tile
         if (qi < p.Sq) {
-          for (int c = 0; c < p.D / 8; ++c) reinterpret_cast<uint4*>(dst)[c] = make_uint4(0, 0, 0, 0);
+          for (int c = 0; c < p.D / 8; ++c)
+            reinterpret_cast<uint4*>(dst)[c] = make_uint4(0, 0, 0, 0);
           *lse_dst = -INFINITY;
         }
         continue;
       }
+      // a warp whose rows all lie beyond the last query only keeps the barriers going
+      const bool warp_live = q0 + quad * 32 < p.Sq;
       float m_used = -INFINITY, l = 0.f;
-      for (int j = 0; j < it.n_tiles && ok; ++j) {
-        const uint32_t gg = g + j;
-        const int sb = gg & 1;
+      for (int j = 0; j < n_tiles && ok; ++j, ++cnt) {
         const int k0 = j * ATT_BN;
         const int rem = min(ATT_BN, p.Sk - k0);
         const int n_chunks = ((rem + 15) / 16 * 16 + 31) / 32;
         // a tile needs masks when it is ragged or crosses the causal diagonal of this q tile
-        const bool masked = rem < ATT_BN || (p.causal && k0 + ATT_BN - 1 > it.q0 + shift);
-        ok = mbar_wait(&bar_s_full[sb], (gg >> 1) & 1, p.status, PF_ERR_TIMEOUT_TMEM_FULL);
+        const bool masked = rem < ATT_BN || (p.causal && k0 + ATT_BN - 1 > q0 + shift);
+        ok = mbar_wait(&s_full[t], cnt & 1, p.status, PF_ERR_TIMEOUT_TMEM_FULL);
         if (!ok) break;
         tc_fence_after();
         uint32_t s[4][32];
-        const uint32_t t_s = tmem + sb * 128 + lane_off;
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
-          if (c < n_chunks) tmem_ld32(t_s + c * 32, s[c]);
+        for (int c = 0; c < 4; ++c) tmem_ld32(t_s + c * 32, s[c]);
         tmem_ld_wait();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&bar_s_empty[sb]);
-        float mx = -INFINITY;
-        if (!masked) {
-          // full tile: four independent chains, no visibility tests
-          float m0 = -INFINITY, m1 = -INFINITY, m2 = -INFINITY, m3 = -INFINITY;
+        if (!C::ALIAS_P) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&s_empty[t]);
+        }
+        // keys of this tile below `lim` are visible to this row
+        const int lim = p.causal ? min(p.Sk, qi + shift + 1) - k0 : p.Sk - k0;
+        uint32_t pk[4][16];
+        float alpha = 1.f;
+        if (warp_live) {
+          float mx = -INFINITY;
+          if (!masked) {
+            float m0 = -INFINITY, m1 = -INFINITY, m2 = -INFINITY, m3 = -INFINITY;
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
+            for (int c = 0; c < 4; ++c) {
 #pragma unroll
-            for (int i = 0; i < 32; i += 4) {
-              m0 = fmaxf(m0, __uint_as_float(s[c][i]));
-              m1 = fmaxf(m1, __uint_as_float(s[c][i + 1]));
-              m2 = fmaxf(m2, __uint_as_float(s[c][i + 2]));
-              m3 = fmaxf(m3, __uint_as_float(s[c][i + 3]));
+              for (int i = 0; i < 32; i += 4) {
+                m0 = fmaxf(m0, __uint_as_float(s[c][i]));
+                m1 = fmaxf(m1, __uint_as_float(s[c][i + 1]));
+                m2 = fmaxf(m2, __uint_as_float(s[c][i + 2]));
+                m3 = fmaxf(m3, __uint_as_float(s[c][i + 3]));
+              }
             }
-          }
-          mx = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
-        } else {
+            mx = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
+          } else {
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            if (c < n_chunks) {
+            for (int c = 0; c < 4; ++c) {
+              if (c < n_chunks) {
 #pragma unroll
-              for (int i = 0; i < 32; ++i) {
-                const int kj = k0 + c * 32 + i;
-                const bool vis = kj < p.Sk && !(p.causal && kj > qi + shift);
-                if (vis) mx = fmaxf(mx, __uint_as_float(s[c][i]));
+                for (int i = 0; i < 32; ++i)
+                  if (c * 32 + i < lim) mx = fmaxf(mx, __uint_as_float(s[c][i]));
               }
             }
           }
+          mx *= c2;                                   // c2 > 0; -inf stays -inf
+          if (j == 0) {
+            m_used = mx;
+          } else if (mx > m_used + 8.f) {             // also true when m_used is still -inf
+            alpha = exp2f(m_used - mx);               // exp2(-inf) = 0: nothing had accumulated
+            m_used = mx;
+          }
+          const float m_sub = (m_used == -INFINITY) ? 0.f : m_used;
+          const float rs = masked ? probs<T, true>(s, pk, c2, m_sub, n_chunks, lim)
+                                  : probs<T, false>(s, pk, c2, m_sub, 4, ATT_BN);
+          l = l * alpha + rs;
         }
-        mx *= c2;                                   // c2 > 0; -inf stays -inf
-        float alpha = 1.f;
-        if (j == 0) {
-          m_used = mx;
-        } else if (mx > m_used + 8.f) {             // also true when m_used is still -inf
-          alpha = exp2f(m_used - mx);               // exp2(-inf) = 0: nothing had accumulated
-          m_used = mx;
-        }
-        const float m_sub = (m_used == -INFINITY) ? 0.f : m_used;
-        // This tile's P buffer was last read by the P V of the tile before the previous one
-        // (any item): long done, so the probabilities below are computed while the previous
-        // tile's P V still runs.  (Parity of the phase before this tile's own on that barrier;
-        // on a fresh barrier the wait passes.)
-        uint8_t* sPj = sP + (gg & 1) * C::P_BYTES;
-        ok = mbar_wait(&bar_pv_done[gg & 1], ((gg >> 1) & 1) ^ 1, p.status,
-                       PF_ERR_TIMEOUT_TMEM_FULL);
-        if (!ok) break;
-        if (j > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
-          // rare: the row maximum grew by more than 2^8.  O must hold every earlier tile of
-          // the item before it is rescaled: wait for the previous tile's P V
-          ok = mbar_wait(&bar_pv_done[(gg - 1) & 1], ((gg - 1) >> 1) & 1, p.status,
-                         PF_ERR_TIMEOUT_TMEM_FULL);
+        // The previous P V must have read its probabilities, and O must hold every earlier tile
+        // before it is rescaled (a short wait: that product ran under the work above).  It also
+        // keeps a warp without live rows from arriving twice on one phase of p_full.
+        if (j > 0) {
+          ok = mbar_wait(&pv_done[t], (cnt - 1) & 1, p.status, PF_ERR_TIMEOUT_TMEM_FULL);
           if (!ok) break;
           tc_fence_after();
-          {
+        }
+        if (warp_live) {
+          if (j > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
 #pragma unroll
             for (int c = 0; c < DP / 32; ++c) {
               uint32_t o[32];
-              tmem_ld32(t_o + lane_off + c * 32, o);
-              tmem_ld_wait();
+              tmem_ld32(t_o + c * 32, o);
+              tmem_ld_wait_for(o);
 #pragma unroll
               for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-              tmem_st32(t_o + lane_off + c * 32, o);
+              tmem_st32(t_o + c * 32, o);
             }
-            tmem_st_wait();
           }
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            if (c < n_chunks) tmem_st16(t_p + c * 16, pk[c]);
+          tmem_st_wait();
         }
-        float rs = 0.f;
-        if (!masked) {
-          float r0 = 0.f, r1 = 0.f, r2 = 0.f, r3 = 0.f;
-          const float nm = -m_sub;
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            float pv[32];
-#pragma unroll
-            for (int i = 0; i < 32; i += 4) {
-              pv[i] = exp2f(fmaf(__uint_as_float(s[c][i]), c2, nm));
-              pv[i + 1] = exp2f(fmaf(__uint_as_float(s[c][i + 1]), c2, nm));
-              pv[i + 2] = exp2f(fmaf(__uint_as_float(s[c][i + 2]), c2, nm));
-              pv[i + 3] = exp2f(fmaf(__uint_as_float(s[c][i + 3]), c2, nm));
-              r0 += pv[i]; r1 += pv[i + 1]; r2 += pv[i + 2]; r3 += pv[i + 3];
-            }
-            store_p_chunk<T>(sPj, row, c * 32, pv);
-          }
-          rs = (r0 + r1) + (r2 + r3);
-        } else {
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            if (c < n_chunks) {
-              float pv[32];
-#pragma unroll
-              for (int i = 0; i < 32; ++i) {
-                const int kj = k0 + c * 32 + i;
-                const bool vis = kj < p.Sk && !(p.causal && kj > qi + shift);
-                pv[i] = vis ? exp2f(fmaf(__uint_as_float(s[c][i]), c2, -m_sub)) : 0.f;
-                rs += pv[i];
-              }
-              store_p_chunk<T>(sPj, row, c * 32, pv);
-            }
-          }
-        }
-        l = l * alpha + rs;
-        fence_async_smem();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar_p_full);
+        if (lane == 0) mbar_arrive(&p_full[t]);
       }
       if (!ok) break;
-      g += it.n_tiles;
-      // ---- epilogue of the item: O / l
-      ok = mbar_wait(&bar_pv_done[(g - 1) & 1], ((g - 1) >> 1) & 1, p.status,
-                     PF_ERR_TIMEOUT_TMEM_FULL);
+      // ---- epilogue of the tile: O / l
+      ok = mbar_wait(&pv_done[t], (cnt - 1) & 1, p.status, PF_ERR_TIMEOUT_TMEM_FULL);
       if (!ok) break;
       tc_fence_after();
-      const float inv = l > 0.f ? 1.f / l : 0.f;
+      if (warp_live) {
+        const float inv = l > 0.f ? 1.f / l : 0.f;
 #pragma unroll
-      for (int c = 0; c < DP / 32; ++c) {
-        uint32_t o[32];
-        tmem_ld32(t_o + lane_off + c * 32, o);
-        tmem_ld_wait();
-        if (qi < p.Sq) {
+        for (int c = 0; c < DP / 32; ++c) {
+          uint32_t o[32];
+          tmem_ld32(t_o + c * 32, o);
+          tmem_ld_wait_for(o);
 #pragma unroll
-          for (int v8 = 0; v8 < 4; ++v8) {
-            if (c * 32 + v8 * 8 < p.D) {
-              uint4 q;
-              q.x = pack2<T>(__uint_as_float(o[v8 * 8 + 0]) * inv, __uint_as_float(o[v8 * 8 + 1]) * inv);
-              q.y = pack2<T>(__uint_as_float(o[v8 * 8 + 2]) * inv, __uint_as_float(o[v8 * 8 + 3]) * inv);
-              q.z = pack2<T>(__uint_as_float(o[v8 * 8 + 4]) * inv, __uint_as_float(o[v8 * 8 + 5]) * inv);
-              q.w = pack2<T>(__uint_as_float(o[v8 * 8 + 6]) * inv, __uint_as_float(o[v8 * 8 + 7]) * inv);
-              reinterpret_cast<uint4*>(dst)[c * 4 + v8] = q;
-            }
+          for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * inv);
+          if (qi < p.Sq) {
+#pragma unroll
+            for (int v = 0; v < 4; ++v)
+              if (c * 32 + v * 8 < p.D)
+                reinterpret_cast<uint4*>(dst)[c * 4 + v] = pack8<T>(o + v * 8);
           }
         }
+        if (qi < p.Sq) *lse_dst = (l > 0.f) ? (m_used + log2f(l)) * LN2 : -INFINITY;
       }
-      if (qi < p.Sq) *lse_dst = (l > 0.f) ? (m_used + log2f(l)) * LN2 : -INFINITY;
-      // the reads of O above have completed (tcgen05.wait::ld); the next item's first P V,
-      // which overwrites O, is ordered after them by this warp's next arrival on bar_p_full
+      // the reads of O above have completed (tcgen05.wait::ld); the next item's first P V of this
+      // tile, which overwrites O, is ordered after them by this warp's next arrival on p_full
       tc_fence_before();
     }
   }
 
+  // teardown: every role reaches this point (all waits are bounded)
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem, TMEM_COLS); }
+  if (warp == 9) { tc_fence_after(); tmem_dealloc(tmem, 512); }
 }
+
 template <typename T, int DP>
 static int launch_fwd_ws(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                          const AttnParams& p, cudaStream_t st) {
@@ -527,9 +609,8 @@ static int launch_fwd_ws(const CUtensorMap& tq, const CUtensorMap& tk, const CUt
   static bool done[64] = {};
   int r = set_smem(kern, C::SMEM, done);
   if (r) return r;
-  const int n_items = p.q_tiles * p.H * p.B;
+  const int n_items = p.q_pairs * p.H * p.B, sms = attn_sm_count();
   if (n_items > 0) {
-    const int sms = attn_sm_count();
     kern<<<n_items < sms ? n_items : sms, C::THREADS, C::SMEM, st>>>(tq, tk, tv, p, n_items);
     PF_CHECK_LAUNCH();
   }
@@ -540,26 +621,6 @@ static int launch_fwd_ws(const CUtensorMap& tq, const CUtensorMap& tk, const CUt
     PF_CHECK_LAUNCH();
   }
   return 0;
-}
-
-// Tensor-core tiles and leftover rows of a sequence of length S: a short leftover (at most
-// ATT_TAIL_MAX rows after at least one full tile) goes to the CUDA-core paths, which stage the
-// other sequence dimension (`other`) in shared memory; otherwise the last tile is ragged.
-static void split_tail(int S, int other, int* tiles, int* tail) {
-  const int left = S % ATT_BM;
-  if (S > ATT_BM && left > 0 && left <= ATT_TAIL_MAX && other <= ATT_TAIL_SEQ_MAX) {
-    *tiles = S / ATT_BM;
-    *tail = left;
-  } else {
-    *tiles = (S + ATT_BM - 1) / ATT_BM;
-    *tail = 0;
-  }
-}
-
-static void set_views(AttnParams& p, const void* q, const void* k, const void* v,
-                      const long long* sq, const long long* sk, const long long* sv) {
-  p.q = q; p.k = k; p.v = v;
-  for (int i = 0; i < 3; ++i) { p.sq[i] = sq[i]; p.sk[i] = sk[i]; p.sv[i] = sv[i]; }
 }
 
 }  // namespace pf
@@ -585,8 +646,14 @@ PF_API int pf_attn_fwd(const void* q, const void* k, const void* v, void* o, voi
   AttnParams p = {};
   p.B = B; p.H = H; p.Sq = Sq; p.Sk = Sk; p.D = D; p.causal = causal; p.scale = scale;
   p.fmt = fmt; p.o = o; p.lse = (float*)lse; p.status = status;
-  set_views(p, q, k, v, sq, sk, sv);
-  split_tail(Sq, Sk, &p.q_tiles, &p.q_tail);
+  p.q = q; p.k = k; p.v = v;
+  for (int i = 0; i < 3; ++i) { p.sq[i] = sq[i]; p.sk[i] = sk[i]; p.sv[i] = sv[i]; }
+  // A short leftover (at most ATT_TAIL_MAX rows after at least one full tile) goes to the CUDA-core
+  // kernel, which stages the keys' scores in shared memory; otherwise the last tile is ragged.
+  const int left = Sq % ATT_BM;
+  p.q_tail = (Sq > ATT_BM && left > 0 && left <= ATT_TAIL_MAX && Sk <= ATT_TAIL_SEQ_MAX) ? left : 0;
+  p.q_rows = Sq - p.q_tail;
+  p.q_pairs = (p.q_rows + 2 * ATT_BM - 1) / (2 * ATT_BM);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   PF_ATTN_DISPATCH(launch_fwd_ws, tq, tk, tv, p, st);
 }
