@@ -490,7 +490,8 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
         uint32_t s[4][32];
 #pragma unroll
         for (int c = 0; c < 4; ++c) tmem_ld32(t_s + c * 32, s[c]);
-        tmem_ld_wait();
+#pragma unroll
+        for (int c = 0; c < 4; ++c) tmem_ld_wait_for(s[c]);
         if (!C::ALIAS_P) {
           tc_fence_before();
           __syncwarp();

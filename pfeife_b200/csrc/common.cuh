@@ -451,11 +451,8 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
       : "r"(taddr)
       : "memory");
 }
-__device__ __forceinline__ void tmem_ld_wait() {
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-// The same wait with the loaded registers named as operands, so that no use of them can be
-// scheduled ahead of it when other work sits between the load and the wait.
+// Wait for the TMEM loads in flight, with the loaded registers named as operands: a use of them is
+// no memory access and could otherwise be scheduled ahead of the wait.
 __device__ __forceinline__ void tmem_ld_wait_for(uint32_t (&r)[32]) {
   asm volatile(
       "tcgen05.wait::ld.sync.aligned;"
