@@ -18,10 +18,12 @@ struct RowSplit {
   }
 };
 
-// (max, sum of exp(x - max)) of two parts of a row; a part without a finite element is (-inf, 0)
+// (max, sum of exp(x - max)) of two parts of a row; a part without a finite element is (-inf, 0), and
+// (-inf, NaN) when it holds a NaN, which no maximum shows: the sums are always added, and -inf, which
+// cannot be subtracted from itself, counts as 0 there.
 __device__ __forceinline__ void ce_merge(float& m, float& s, float m2, float s2) {
-  const float mm = fmaxf(m, m2);
-  s = (m == -INFINITY ? 0.f : s * __expf(m - mm)) + (m2 == -INFINITY ? 0.f : s2 * __expf(m2 - mm));
+  const float mm = fmaxf(m, m2), sub = mm == -INFINITY ? 0.f : mm;
+  s = s * __expf(m - sub) + s2 * __expf(m2 - sub);
   m = mm;
 }
 
@@ -56,8 +58,8 @@ ce_fwd_kernel(const T* __restrict__ logits, const long long* __restrict__ target
 #pragma unroll
         for (int j = 0; j < VN; ++j) lm = fmaxf(lm, to_f32<T>(e[j]));
       }
-    // a NaN does not move the maximum but reaches the sum below; parts that are -inf so far
-    // subtract 0, which leaves their exponentials at zero
+    // a NaN does not move the maximum but reaches the sum below, and every merge keeps it; parts
+    // that are -inf so far subtract 0, which leaves their exponentials at zero
     const float mm = fmaxf(m, lm), sub = (mm == -INFINITY) ? 0.f : mm;
     if (lm > m) s *= __expf(m - sub);
     float a = 0.f;

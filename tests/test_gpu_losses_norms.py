@@ -65,6 +65,34 @@ def test_cross_entropy_masked_vocabulary_and_all_ignored():
     assert float(loss.detach()) == 0.0 and not dy.any()
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows", [9, 700])       # both sizes of CTA
+@pytest.mark.parametrize("V", [2, 7, 10, 1000, 2048, 3001])
+def test_cross_entropy_keeps_nan_and_skips_masked(V, rows, dtype):
+    """A NaN logit outside the target's column makes the row's loss NaN, whatever part of the row a
+    thread owns; -inf logits (a masked vocabulary) count as zero probability."""
+    from pfeife_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(V + rows)
+    x = torch.randn(rows, V, device="cuda", generator=g).to(dtype)
+    t = torch.zeros(rows, dtype=torch.int64, device="cuda")
+    masked = torch.rand(rows, V, device="cuda", generator=g) < 0.7
+    masked[:, 0] = False
+    x = x.masked_fill(masked, float("-inf"))
+    want = F.cross_entropy(x.double(), t, reduction="none")
+    got = ops.cross_entropy(x, t, reduction="none")
+    # the targets' own rounding aside, fp32 sums: u of the loss and of the logits it is the difference of
+    assert torch.allclose(got.double(), want, rtol=1e-5, atol=1e-5)
+    r = torch.arange(rows, device="cuda")
+    one = x.clone()
+    one[r, 1 + r % (V - 1)] = float("nan")
+    run = x.clone()                       # eight NaNs side by side: the whole of one 16-byte load
+    for k in range(8):
+        run[r, (1 + (8 * r + k) % (V - 1))] = float("nan")
+    for bad in (one, run):
+        assert torch.isnan(ops.cross_entropy(bad, t, reduction="none")).all()
+        assert torch.isnan(ops.cross_entropy(bad, t))
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("silu", [True, False])
 @pytest.mark.parametrize("B,H,W,C,G", [(1, 1, 1, 32, 8), (2, 5, 7, 8, 2), (3, 16, 16, 32, 8),
