@@ -214,6 +214,10 @@ def _rows(x: Tensor) -> Tensor:
 # images, logits: 4.7 -> 2.9 ms; LayerNorm with residual, forward and backward: 246 -> 175 us.)
 # The implementation runs below autograd, as the dispatcher has it, so that what it returns is no
 # view to autograd and may be changed in place.
+_DIRECT_DEVICE = "cuda"
+_below_autograd = torch._C._AutoDispatchBelowADInplaceOrView
+
+
 def _custom_op(name: str):
     """``torch.library.custom_op`` that keeps the undecorated function as ``.plain``; an op that is
     part of another op's implementation is called through it."""
@@ -232,7 +236,7 @@ def _autograd(op, n_out: int, backward, setup) -> None:
     class Direct(torch.autograd.Function):
         @staticmethod
         def forward(ctx, *args):
-            with torch._C._AutoDispatchBelowADInplaceOrView():
+            with _below_autograd():
                 out = op.plain(*args)
             ctx.plain = True
             setup(ctx, args, out)
@@ -247,19 +251,24 @@ def _autograd(op, n_out: int, backward, setup) -> None:
         def backward(ctx, *grads):
             if not _unobserved():
                 return backward(ctx, *grads, *ctx.more)
-            with torch._C._AutoDispatchBelowADInplaceOrView():
+            with _below_autograd():
                 return backward(ctx, *grads, *ctx.more)
 
     op.direct, op.n_out = Direct, n_out
 
 
+_DispatchKey, _KeySet = torch._C.DispatchKey, torch._C.DispatchKeySet
+_VIEWS = _KeySet(_DispatchKey.ADInplaceOrView).raw_repr()      # absent in inference mode
+_NO_LAYER = _KeySet(_DispatchKey.BackendSelect).raw_repr() | _VIEWS
+
+
 def _unobserved() -> bool:
-    """No compiler, tracer, dispatch or function mode, functorch transform or forward-mode level is
-    active: nothing but the kernels and autograd needs to see an op."""
-    return not (torch.compiler.is_compiling() or torch._C._len_torch_dispatch_stack()
-                or torch._C._len_torch_function_stack() or forward_ad._current_level >= 0
-                or torch._C._functorch.peek_interpreter_stack() is not None
-                or torch._C._get_tracing_state() is not None)
+    """No compiler, tracer, dispatch or function mode, transform (of either vmap) or forward-mode level
+    is active: nothing but the kernels and autograd needs to see an op.  All but three of these put
+    a layer of their own on the dispatcher of this thread."""
+    return not (torch.compiler.is_compiling() or torch._C._len_torch_function_stack()
+                or forward_ad._current_level >= 0) and \
+        torch._C._dispatch_tls_local_include_set().raw_repr() | _VIEWS == _NO_LAYER
 
 
 def _bwd(ctx, op):
@@ -279,7 +288,7 @@ def _plain_call(args) -> bool:
                 return False
             if device is None:
                 device = a.device
-                if device.type != "cuda":
+                if device.type != _DIRECT_DEVICE:
                     return False
             elif a.device != device:
                 return False
@@ -293,7 +302,7 @@ def _call(op, *args):
             for a in args:
                 if isinstance(a, Tensor) and a.requires_grad:
                     return op.direct.apply(*args)
-        with torch._C._AutoDispatchBelowADInplaceOrView():
+        with _below_autograd():
             out = op.plain(*args)
     else:
         out = op(*args)

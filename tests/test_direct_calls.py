@@ -1,0 +1,80 @@
+"""An eager call on plain tensors goes straight to its implementation; transforms, tracers, hooks and
+higher derivatives still have to work as they do through the dispatcher.  On CPU the direct way is
+switched on for CPU tensors."""
+import pytest
+import torch
+
+from pfeife_b200 import ops
+from pfeife_b200.ops import functional
+
+DEVICES = ["cpu", pytest.param("cuda", marks=pytest.mark.gpu)]
+
+
+@pytest.fixture(params=DEVICES)
+def device(request, monkeypatch):
+    monkeypatch.setattr(functional, "_DIRECT_DEVICE", request.param, raising=False)
+    return request.param
+
+
+def _cases(device):
+    """name -> (function of the leaves, leaves)"""
+    dt = torch.float32 if device == "cpu" else torch.bfloat16
+    g = torch.Generator().manual_seed(5)
+
+    def r(*shape, scale=1.0, dtype=dt):
+        return (torch.randn(*shape, generator=g) * scale).to(device=device, dtype=dtype)
+
+    def v(n):
+        return r(n, dtype=torch.float32)
+
+    cos, sin = ops.rope_tables(16, 16, device=device)
+    ids = torch.randint(0, 24, (2, 16), generator=g).to(device)
+    return {
+        "linear": (lambda x, w, b, res: ops.linear(x, w, b, "gelu", res),
+                   [r(16, 64), r(32, 64, scale=0.2), v(32), r(16, 32)]),
+        "mlp": (lambda x, w1, b1, w2, b2, res: ops.mlp(x, w1, b1, w2, b2, "gelu", res),
+                [r(16, 64), r(96, 64, scale=0.2), v(96), r(64, 96, scale=0.2), v(64), r(16, 64)]),
+        "layer_norm": (lambda x, w, b, res: ops.layer_norm(x, w, b, 1e-5, residual=res)[0],
+                       [r(16, 64), v(64), v(64), r(16, 64)]),
+        "rms_norm": (lambda x, w: ops.rms_norm(x, w), [r(16, 64), v(64)]),
+        "gelu": (ops.gelu, [r(16, 64)]),
+        "swiglu": (ops.swiglu, [r(16, 64)]),
+        "cross_entropy": (lambda x: ops.cross_entropy(x, ids.view(-1)), [r(32, 24)]),
+        "cross_entropy_rows": (lambda x: ops.cross_entropy(x, ids.view(-1), reduction="none"),
+                               [r(32, 24)]),
+        "mse": (lambda a: ops.mse_loss(a, a.detach() + 1), [r(16, 64)]),
+        "embedding": (lambda t: ops.embedding(ids, t, dt), [r(24, 32)]),
+        "rope": (lambda x: ops.rope(x, cos, sin), [r(2, 16, 2, 16)]),
+        "attention": (lambda q, k, v: ops.attention(q, k, v, causal=True),
+                      [r(2, 16, 2, 16), r(2, 16, 2, 16), r(2, 16, 2, 16)]),
+        "attention_qkv": (lambda qkv: ops.attention_qkv(qkv), [r(2, 16, 3, 2, 16)]),
+        "conv2d": (lambda x, w, b: ops.conv2d(x, w, b, 1, 1),
+                   [r(1, 8, 8, 16), r(24, 16, 3, 3, scale=0.2), v(24)]),
+        "group_norm": (lambda x, w, b: ops.group_norm(x, w, b, 4, silu=True),
+                       [r(2, 4, 4, 32), v(32), v(32)]),
+        "upsample": (ops.upsample_nearest2x, [r(2, 4, 4, 32)]),
+    }
+
+
+NAMES = list(_cases("cpu"))
+# two correct computations of one 16-bit result differ by a rounding; sums with atomics by less
+TOL = {"cpu": 1e-5, "cuda": 2.0 ** -7}
+
+
+def _near(a, b, device):
+    a, b = a.double(), b.double()
+    assert a.shape == b.shape and (a - b).norm() <= TOL[device] * b.norm() + 1e-6
+
+
+@pytest.mark.parametrize("name", NAMES)
+def test_gradients_of_several_vectors_at_once(name, device):
+    fn, leaves = _cases(device)[name]
+    leaves = [t.requires_grad_() for t in leaves]
+    y = fn(*leaves)
+    assert "Direct" in y.grad_fn.name() or name in ("cross_entropy_rows", "embedding")
+    vs = torch.stack([torch.ones_like(y), torch.randn_like(y), torch.zeros_like(y)])
+    batched = torch.autograd.grad(y, leaves, vs, is_grads_batched=True, retain_graph=True)
+    for i in range(len(vs)):
+        one = torch.autograd.grad(y, leaves, vs[i], retain_graph=True)
+        for a, b in zip(batched, one):
+            _near(a[i], b, device)
