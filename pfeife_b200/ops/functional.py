@@ -249,8 +249,6 @@ def _autograd(op, n_out: int, backward, setup) -> None:
         @staticmethod
         @once_differentiable
         def backward(ctx, *grads):
-            if not _unobserved():
-                return backward(ctx, *grads, *ctx.more)
             with _below_autograd():
                 return backward(ctx, *grads, *ctx.more)
 
@@ -274,11 +272,14 @@ def _unobserved() -> bool:
 def _bwd(ctx, op):
     """The form of the backward op that matches how the forward was called (batched gradients
     arrive under a transform whatever the forward was)."""
-    return op.plain if getattr(ctx, "plain", False) and _unobserved() else op
+    if not getattr(ctx, "plain", False):
+        return op
+    return lambda *args: (op.plain if _plain_call(args) else op)(*args)
 
 
 def _plain_call(args) -> bool:
-    """True for plain CUDA tensors of one device that nothing else observes."""
+    """True for plain CUDA tensors of one device that nothing else observes and whose memory holds
+    their values: no view with a negative bit, no wrapper that outlived its transform."""
     if not _unobserved():
         return False
     device = None
@@ -291,6 +292,8 @@ def _plain_call(args) -> bool:
                 if device.type != _DIRECT_DEVICE:
                     return False
             elif a.device != device:
+                return False
+            if a.is_neg() or torch._C._functorch.is_functorch_wrapped_tensor(a):
                 return False
     return device is not None
 

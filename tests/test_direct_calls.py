@@ -78,3 +78,23 @@ def test_gradients_of_several_vectors_at_once(name, device):
         one = torch.autograd.grad(y, leaves, vs[i], retain_graph=True)
         for a, b in zip(batched, one):
             _near(a[i], b, device)
+
+
+def test_lazily_negated_inputs(device, monkeypatch):
+    """A view with the negative bit set holds the wrong sign in memory: no implementation gets one."""
+    for op in (functional.act_fwd, functional.act_bwd):
+        def plain(x, *args, plain=op.plain):
+            assert not x.is_neg()
+            return plain(x, *args)
+        monkeypatch.setattr(op, "plain", plain)
+    dtype = torch.float32 if device == "cpu" else torch.bfloat16
+    x = torch.randn(8, 64).to(device=device, dtype=dtype)
+    flip = torch._neg_view(x).requires_grad_()
+    y, want = ops.gelu(flip), ops.gelu((-x).requires_grad_())
+    _near(y, want, device)
+    v = torch.randn_like(x)
+    for out in (y, want):
+        (g,) = torch.autograd.grad(out, out.grad_fn.next_functions[0][0].variable, torch._neg_view(v),
+                                   retain_graph=True)
+        (w,) = torch.autograd.grad(out, out.grad_fn.next_functions[0][0].variable, -v)
+        _near(g, w, device)
