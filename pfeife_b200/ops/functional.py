@@ -252,12 +252,13 @@ def _autograd(op, n_out: int, backward, setup) -> None:
             with _below_autograd():
                 return backward(ctx, *grads, *ctx.more)
 
-    op.direct, op.n_out = Direct, n_out
+    op.direct, op.n_out, op.n_all = Direct, n_out, len(op._opoverload._schema.returns)
 
 
 _DispatchKey, _KeySet = torch._C.DispatchKey, torch._C.DispatchKeySet
 _VIEWS = _KeySet(_DispatchKey.ADInplaceOrView).raw_repr()      # absent in inference mode
 _NO_LAYER = _KeySet(_DispatchKey.BackendSelect).raw_repr() | _VIEWS
+_PLAIN_VALUES = frozenset((type(None), bool, int, float, torch.dtype))
 
 
 def _unobserved() -> bool:
@@ -279,14 +280,14 @@ def _bwd(ctx, op):
 
 def _plain_call(args) -> bool:
     """True for plain CUDA tensors of one device that nothing else observes and whose memory holds
-    their values: no view with a negative bit, no wrapper that outlived its transform."""
+    their values: no view with a negative bit, no wrapper that outlived its transform.  Anything but
+    tensors and plain values (the proxy of a symbolic trace) is for the dispatcher to handle."""
     if not _unobserved():
         return False
     device = None
     for a in args:
-        if isinstance(a, Tensor):
-            if type(a) is not Tensor and type(a) is not torch.nn.Parameter:
-                return False
+        kind = type(a)
+        if kind is Tensor or kind is torch.nn.Parameter:
             if device is None:
                 device = a.device
                 if device.type != _DIRECT_DEVICE:
@@ -295,6 +296,8 @@ def _plain_call(args) -> bool:
                 return False
             if a.is_neg() or torch._C._functorch.is_functorch_wrapped_tensor(a):
                 return False
+        elif kind not in _PLAIN_VALUES:
+            return False
     return device is not None
 
 
@@ -309,9 +312,9 @@ def _call(op, *args):
             out = op.plain(*args)
     else:
         out = op(*args)
-    if not isinstance(out, tuple):
+    if op.n_all == 1:
         return out
-    return out[0] if op.n_out == 1 else out[:op.n_out]
+    return out[0] if op.n_out == 1 else tuple(out[i] for i in range(op.n_out))
 
 
 # =========================================================================== linear

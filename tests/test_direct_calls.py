@@ -98,3 +98,19 @@ def test_lazily_negated_inputs(device, monkeypatch):
                                    retain_graph=True)
         (w,) = torch.autograd.grad(out, out.grad_fn.next_functions[0][0].variable, -v)
         _near(g, w, device)
+
+
+@pytest.mark.parametrize("name", ["linear", "layer_norm", "rope", "cross_entropy", "attention_qkv"])
+def test_symbolic_traces_beside_real_tensors(name, device):
+    """A proxy input next to tensors that exist (weights, tables): the call is recorded."""
+    fn, leaves = _cases(device)[name]
+    rest = leaves[1:]
+    if name == "attention_qkv":
+        fn = lambda qkv: ops.attention_qkv(qkv, scale=0.25)
+    if name == "cross_entropy":
+        ids = torch.arange(32, device=device) % 24
+        fn = lambda x: functional._call(functional.ce_mean_fwd, x, ids, -100)
+    gm = torch.fx.symbolic_trace(lambda x: fn(x, *rest))
+    assert any("pfeife" in str(n.target) for n in gm.graph.nodes)
+    with torch.no_grad():
+        assert torch.equal(gm(leaves[0]), fn(*leaves))
