@@ -27,7 +27,6 @@ import torch.nn.functional as F
 from torch import Tensor
 from torch._subclasses.fake_tensor import FakeTensor
 from torch.autograd import forward_ad
-from torch.autograd.function import once_differentiable
 
 from . import kernels as kx
 
@@ -247,8 +246,9 @@ def _autograd(op, n_out: int, backward, setup) -> None:
             return out[0] if n_out == 1 else out[:n_out]
 
         @staticmethod
-        @once_differentiable
         def backward(ctx, *grads):
+            if torch.is_grad_enabled():
+                return backward(ctx, *grads, *ctx.more)
             with _below_autograd():
                 return backward(ctx, *grads, *ctx.more)
 
@@ -272,8 +272,9 @@ def _unobserved() -> bool:
 
 def _bwd(ctx, op):
     """The form of the backward op that matches how the forward was called (batched gradients
-    arrive under a transform whatever the forward was)."""
-    if not getattr(ctx, "plain", False):
+    arrive under a transform whatever the forward was).  A backward that is itself recorded
+    (``create_graph``) goes through the dispatcher, whose ops have autograd formulas."""
+    if not getattr(ctx, "plain", False) or torch.is_grad_enabled():
         return op
     return lambda *args: (op.plain if _plain_call(args) else op)(*args)
 

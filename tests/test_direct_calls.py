@@ -3,6 +3,7 @@ higher derivatives still have to work as they do through the dispatcher.  On CPU
 switched on for CPU tensors."""
 import pytest
 import torch
+from torch.utils._python_dispatch import TorchDispatchMode
 
 from pfeife_b200 import ops
 from pfeife_b200.ops import functional
@@ -14,6 +15,13 @@ DEVICES = ["cpu", pytest.param("cuda", marks=pytest.mark.gpu)]
 def device(request, monkeypatch):
     monkeypatch.setattr(functional, "_DIRECT_DEVICE", request.param, raising=False)
     return request.param
+
+
+class Watch(TorchDispatchMode):
+    """Lets every op be seen, which keeps all calls on the dispatcher."""
+
+    def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+        return func(*args, **(kwargs or {}))
 
 
 def _cases(device):
@@ -98,6 +106,36 @@ def test_lazily_negated_inputs(device, monkeypatch):
                                    retain_graph=True)
         (w,) = torch.autograd.grad(out, out.grad_fn.next_functions[0][0].variable, -v)
         _near(g, w, device)
+
+
+@pytest.mark.parametrize("name", ["rope", "upsample", "linear", "mlp"])
+def test_second_derivatives_where_the_backward_is_linear(name, device):
+    """The gradients of rope, of upsampling and of a residual are linear in the result's gradient
+    and are made of ops that can be differentiated again."""
+    fn, leaves = _cases(device)[name]
+    leaves = [t.requires_grad_() for t in leaves]
+    x = leaves[-1]                       # the residual, or the only input
+    out = []
+    for watched in (False, True):
+        v = torch.full_like(fn(*leaves), 0.5).requires_grad_()
+        if watched:
+            with Watch():
+                (gx,) = torch.autograd.grad(fn(*leaves), x, v, create_graph=True)
+                (gv,) = torch.autograd.grad(gx.square().sum(), v)
+        else:
+            (gx,) = torch.autograd.grad(fn(*leaves), x, v, create_graph=True)
+            (gv,) = torch.autograd.grad(gx.square().sum(), v)
+        out.append((gx.detach(), gv))
+    for a, b in zip(*out):
+        assert torch.equal(a, b) and b.any()
+
+
+def test_second_derivatives_of_the_others_are_refused(device):
+    fn, leaves = _cases(device)["linear"]
+    leaves = [t.requires_grad_() for t in leaves]
+    (gx,) = torch.autograd.grad(fn(*leaves).sum(), leaves[0], create_graph=True)
+    with pytest.raises(RuntimeError):
+        gx.sum().backward()
 
 
 @pytest.mark.parametrize("name", ["linear", "layer_norm", "rope", "cross_entropy", "attention_qkv"])
