@@ -247,10 +247,7 @@ def _autograd(op, n_out: int, backward, setup) -> None:
 
         @staticmethod
         def backward(ctx, *grads):
-            if torch.is_grad_enabled():
-                return backward(ctx, *grads, *ctx.more)
-            with _below_autograd():
-                return backward(ctx, *grads, *ctx.more)
+            return backward(ctx, *grads, *ctx.more)
 
     op.direct, op.n_out, op.n_all = Direct, n_out, len(op._opoverload._schema.returns)
 
@@ -273,10 +270,18 @@ def _unobserved() -> bool:
 def _bwd(ctx, op):
     """The form of the backward op that matches how the forward was called (batched gradients
     arrive under a transform whatever the forward was).  A backward that is itself recorded
-    (``create_graph``) goes through the dispatcher, whose ops have autograd formulas."""
+    (``create_graph``) goes through the dispatcher, whose ops have autograd formulas.  Only the op
+    runs below autograd, not the formula around it: unpacking a saved tensor may call hooks that
+    record (a checkpoint runs its forward again)."""
     if not getattr(ctx, "plain", False) or torch.is_grad_enabled():
         return op
-    return lambda *args: (op.plain if _plain_call(args) else op)(*args)
+
+    def direct(*args):
+        if not _plain_call(args):
+            return op(*args)
+        with _below_autograd():
+            return op.plain(*args)
+    return direct
 
 
 def _plain_call(args) -> bool:
@@ -812,13 +817,14 @@ def _ce_setup(ctx, inputs, output):
     ctx.ignore_index = ignore_index
 
 
-_autograd(
-    ce_fwd, 1,
-    lambda ctx, dloss, dlse: ((None if dloss is None else
-                               _bwd(ctx, ce_bwd)(dloss.contiguous(), ctx.saved_tensors[0],
-                                                 ctx.saved_tensors[1], ctx.saved_tensors[2],
-                                                 ctx.ignore_index)), None, None),
-    setup=_ce_setup)
+def _ce_backward(ctx, dloss, dlse):
+    if dloss is None:
+        return None, None, None
+    logits, target, lse = ctx.saved_tensors
+    return _bwd(ctx, ce_bwd)(dloss.contiguous(), logits, target, lse, ctx.ignore_index), None, None
+
+
+_autograd(ce_fwd, 1, _ce_backward, setup=_ce_setup)
 
 
 @_custom_op("pfeife::ce_mean_fwd")
@@ -985,11 +991,12 @@ def _rope_setup(ctx, inputs, output):
     ctx.inverse = inputs[3]
 
 
-_autograd(
-    rope_apply, 1,
-    lambda ctx, dy: (_bwd(ctx, rope_apply)(dy.contiguous(), ctx.saved_tensors[0],
-                                           ctx.saved_tensors[1], not ctx.inverse), None, None, None),
-    setup=_rope_setup)
+def _rope_backward(ctx, dy):
+    cos, sin = ctx.saved_tensors
+    return _bwd(ctx, rope_apply)(dy.contiguous(), cos, sin, not ctx.inverse), None, None, None
+
+
+_autograd(rope_apply, 1, _rope_backward, setup=_rope_setup)
 
 
 def rope(x: Tensor, cos: Tensor, sin: Tensor) -> Tensor:

@@ -152,3 +152,34 @@ def test_symbolic_traces_beside_real_tensors(name, device):
     assert any("pfeife" in str(n.target) for n in gm.graph.nodes)
     with torch.no_grad():
         assert torch.equal(gm(leaves[0]), fn(*leaves))
+
+
+@pytest.mark.parametrize("name", NAMES)
+def test_recomputing_checkpoints(name, device):
+    """Saved tensors come back through hooks that may themselves run recorded ops, once each."""
+    from torch.utils.checkpoint import checkpoint
+    fn, leaves = _cases(device)[name]
+    leaves = [t.requires_grad_() for t in leaves]
+    y = fn(*leaves)
+    want = torch.autograd.grad(y, leaves, torch.ones_like(y))
+    y = checkpoint(lambda *a: fn(a[0] * 1, *a[1:]), *leaves, use_reentrant=False)
+    got = torch.autograd.grad(y, leaves, torch.ones_like(y))
+    for a, b in zip(got, want):
+        _near(a, b, device)
+
+
+def test_unpacking_hooks_run_recorded(device):
+    seen = []
+
+    def unpack(t):
+        leaf = torch.ones(2, device=t.device, requires_grad=True)
+        with torch.enable_grad():
+            seen.append((leaf * 2).requires_grad)
+        return t
+
+    fn, leaves = _cases(device)["linear"]
+    leaves = [t.requires_grad_() for t in leaves]
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, unpack):
+        y = fn(*leaves)
+    torch.autograd.grad(y, leaves, torch.ones_like(y))
+    assert seen and all(seen)
