@@ -255,6 +255,10 @@ def _autograd(op, n_out: int, backward, setup) -> None:
 _DispatchKey, _KeySet = torch._C.DispatchKey, torch._C.DispatchKeySet
 _VIEWS = _KeySet(_DispatchKey.ADInplaceOrView).raw_repr()      # absent in inference mode
 _NO_LAYER = _KeySet(_DispatchKey.BackendSelect).raw_repr() | _VIEWS
+_AUTOGRAD = _DispatchKey.AutogradOther                         # excluded inside other ops
+_layers, _excluded = (torch._C._dispatch_tls_local_include_set,
+                      torch._C._dispatch_tls_is_dispatch_key_excluded)
+_wrapped, _Parameter = torch._C._functorch.is_functorch_wrapped_tensor, torch.nn.Parameter
 _PLAIN_VALUES = frozenset((type(None), bool, int, float, torch.dtype))
 
 
@@ -264,7 +268,7 @@ def _unobserved() -> bool:
     a layer of their own on the dispatcher of this thread."""
     return not (torch.compiler.is_compiling() or torch._C._len_torch_function_stack()
                 or forward_ad._current_level >= 0) and \
-        torch._C._dispatch_tls_local_include_set().raw_repr() | _VIEWS == _NO_LAYER
+        _layers().raw_repr() | _VIEWS == _NO_LAYER
 
 
 def _bwd(ctx, op):
@@ -284,36 +288,38 @@ def _bwd(ctx, op):
     return direct
 
 
-def _plain_call(args) -> bool:
-    """True for plain CUDA tensors of one device that nothing else observes and whose memory holds
-    their values: no view with a negative bit, no wrapper that outlived its transform.  Anything but
-    tensors and plain values (the proxy of a symbolic trace) is for the dispatcher to handle."""
+def _plain_call(args) -> int:
+    """Non-zero for plain CUDA tensors of one device that nothing else observes and whose memory
+    holds their values: no view with a negative bit, no wrapper that outlived its transform.
+    Anything but tensors and plain values (the proxy of a symbolic trace) is for the dispatcher to
+    handle.  2 when one of them requires a gradient, else 1."""
     if not _unobserved():
-        return False
-    device = None
+        return 0
+    device, found = None, 1
     for a in args:
         kind = type(a)
-        if kind is Tensor or kind is torch.nn.Parameter:
+        if kind is Tensor or kind is _Parameter:
             if device is None:
                 device = a.device
                 if device.type != _DIRECT_DEVICE:
-                    return False
+                    return 0
             elif a.device != device:
-                return False
-            if a.is_neg() or torch._C._functorch.is_functorch_wrapped_tensor(a):
-                return False
+                return 0
+            if a.is_neg() or _wrapped(a):
+                return 0
+            if a.requires_grad:
+                found = 2
         elif kind not in _PLAIN_VALUES:
-            return False
-    return device is not None
+            return 0
+    return found if device is not None else 0
 
 
 def _call(op, *args):
     """The first ``n_out`` outputs of `op`."""
-    if _plain_call(args):
-        if torch.is_grad_enabled():
-            for a in args:
-                if isinstance(a, Tensor) and a.requires_grad:
-                    return op.direct.apply(*args)
+    found = _plain_call(args)
+    if found == 2 and torch.is_grad_enabled() and not _excluded(_AUTOGRAD):
+        return op.direct.apply(*args)
+    if found:
         with _below_autograd():
             out = op.plain(*args)
     else:

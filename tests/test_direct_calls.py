@@ -183,3 +183,13 @@ def test_unpacking_hooks_run_recorded(device):
         y = fn(*leaves)
     torch.autograd.grad(y, leaves, torch.ones_like(y))
     assert seen and all(seen)
+
+
+def test_calls_inside_another_op_are_not_recorded(device):
+    """Below autograd (the implementation of a user's own op) a call keeps no graph, whatever its
+    weights ask for."""
+    w = torch.randn(32, 64).to(device=device, dtype=torch.float32 if device == "cpu" else torch.bfloat16)
+    x, w = torch.ones_like(w), w.requires_grad_()
+    with torch._C._AutoDispatchBelowAutograd():
+        assert ops.linear(x, w).grad_fn is None
+    assert ops.linear(x, w).grad_fn is not None
