@@ -1169,7 +1169,7 @@ def _conv_weight(w: Tensor, dtype: torch.dtype, cout8: int, cin8: int) -> Tensor
     """The weight as the B operand [cout8, KH*KW*cin8] (taps outermost) of the forward product."""
     wc = _weight_as(w, dtype)
     if w.shape[2:] == (1, 1) and w.shape[:2] == (cout8, cin8):
-        return wc.reshape(cout8, cin8)       # the same order already
+        return wc.reshape(cout8, cin8).contiguous()      # the same order already
     return kx.conv_pack(wc, cout8, cin8)
 
 

@@ -174,3 +174,26 @@ def test_conv_weight_orders(B, H, Cin, Cout, K, stride, w_dtype):
         want = want.to(got.device)
         assert (got.double() - want).norm() <= 1.5 * u * want.norm()
     assert grads[1].dtype == w_dtype
+
+
+@pytest.mark.parametrize("w_dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("K", [1, 3])
+@pytest.mark.parametrize("layout", ["transposed", "sliced", "channels_last", "expanded"])
+def test_conv_weight_views(layout, K, w_dtype):
+    """Weights that are views of something else: the same values as a contiguous copy gives."""
+    from pfeife_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(K)
+    rnd = lambda *s: (0.1 * torch.randn(*s, device="cuda", generator=g)).to(w_dtype)
+    Cout, Cin = 64, 72
+    w = {"transposed": lambda: rnd(Cin, Cout, K, K).transpose(0, 1),
+         "sliced": lambda: rnd(Cout, Cin + 3, K, K)[:, 3:],
+         "channels_last": lambda: rnd(Cout, Cin, K, K).to(memory_format=torch.channels_last),
+         "expanded": lambda: rnd(Cout, 1, K, K).expand(Cout, Cin, K, K)}[layout]()
+    x = torch.randn(2, 8, 8, Cin, device="cuda", generator=g).to(torch.bfloat16)
+    out = []
+    for weight in (w, w.clone(memory_format=torch.contiguous_format)):
+        leaves = x.clone().requires_grad_(), weight.detach().requires_grad_()
+        y = ops.conv2d(*leaves, None, 1, K // 2)
+        out.append((y,) + torch.autograd.grad(y, leaves, torch.ones_like(y)))
+    for a, b in zip(*out):
+        assert torch.equal(a, b)
