@@ -66,12 +66,13 @@ PF_DECL int pf_loss_scale_update(void* state, void* found_inf, float growth, flo
 // ---- loss_embed.cu
 PF_DECL int pf_ce_fwd(const void* logits, const void* target, void* loss, void* lse,
                       long long rows, int V, long long ld, long long ignore_index, int dtype,
-                      void* stream);
-PF_DECL int pf_ce_mean(const void* loss, const void* target, void* mean, void* inv, long long rows,
-                       long long ignore_index, void* stream);
+                      int sm_count, void* stream);
+PF_DECL int pf_ce_mean_parts(long long rows, int sm_count);
+PF_DECL int pf_ce_mean(const void* loss, const void* target, void* scratch, void* mean, void* inv,
+                       long long rows, long long ignore_index, int sm_count, void* stream);
 PF_DECL int pf_ce_bwd(const void* logits, const void* target, const void* lse, const void* gscale,
                       void* dlogits, long long rows, int V, long long ld, long long ignore_index,
-                      long long gstride, int dtype, void* stream);
+                      long long gstride, int dtype, int sm_count, void* stream);
 PF_DECL int pf_mse_fwd(const void* a, const void* b, void* out_f32, long long n, int dtype,
                        int sm_count, void* stream);
 PF_DECL int pf_mse_bwd(const void* a, const void* b, const void* gout_f32, void* da, long long n,

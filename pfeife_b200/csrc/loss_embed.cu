@@ -18,34 +18,37 @@ struct RowSplit {
   }
 };
 
-// (max, sum of exp(x - max)) of two parts of a row; a part without a finite element is (-inf, 0), and
-// (-inf, NaN) when it holds a NaN, which no maximum shows: the sums are always added, and -inf, which
-// cannot be subtracted from itself, counts as 0 there.
+// (max, sum of exp(x - max)) of two parts of a row; a part without a finite element is (-inf, 0),
+// and (-inf, NaN) when it holds a NaN, which no maximum shows: the sums are always added, and
+// -inf, which cannot be subtracted from itself, counts as 0 there.
 __device__ __forceinline__ void ce_merge(float& m, float& s, float m2, float s2) {
   const float mm = fmaxf(m, m2), sub = mm == -INFINITY ? 0.f : mm;
   s = s * __expf(m - sub) + s2 * __expf(m2 - sub);
   m = mm;
 }
 
-// One CTA per row of logits, one pass: every thread keeps the maximum and the sum of exponentials
-// of its elements, raised once per 32 elements.  The per-row log-sum-exp is saved so the backward
-// never re-reduces.  loss[row] = lse - x[target] (0 for ignore_index rows).
-// Bound by HBM: four 16-byte loads per thread are in flight; THREADS is 256, and 1024 for calls
-// of too few rows to fill the SMs with small CTAs (183 x 32000: 18 -> 12 us).  2047 x 32000 bf16:
-// 53 -> 37 us, 3.5 TB/s (2-byte loads and a maximum raised per element before).
+// One pass over a row of logits by THREADS threads: every thread keeps the maximum and the sum of
+// exponentials of its elements, raised once per 32 elements.  The per-row log-sum-exp is saved so
+// the backward never re-reduces.  loss[row] = lse - x[target] (0 for ignore_index rows).
+// Bound by HBM: four 16-byte loads per thread are in flight (2047 x 32000 bf16: 53 -> 37 us,
+// 3.5 TB/s, against 2-byte loads and a maximum raised per element).
 template <typename T, int THREADS>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS < 256 ? 256 : THREADS)
 ce_fwd_kernel(const T* __restrict__ logits, const long long* __restrict__ target,
-              float* __restrict__ loss, float* __restrict__ lse, int V, long long ld,
+              float* __restrict__ loss, float* __restrict__ lse, long long rows, int V, long long ld,
               long long ignore_index) {
   constexpr int W = THREADS / 32, VN = RowSplit<T>::V, U = 4;
+  constexpr int ROWS = THREADS < 256 ? 256 / THREADS : 1;       // rows per CTA, whole warps each
+  static_assert(ROWS == 1 || W == 1, "rows that share a CTA are a warp each");
   __shared__ float smax[W], ssum[W];
-  const long long row = blockIdx.x;
+  const long long row = (long long)blockIdx.x * ROWS + threadIdx.x / THREADS;
+  if (row >= rows) return;
+  const int tid = threadIdx.x % THREADS;
   const T* x = logits + row * ld;
   const RowSplit<T> part(x, V);
   float m = -INFINITY, s = 0.f;
   const uint4* xv = reinterpret_cast<const uint4*>(x + part.head);
-  for (int i0 = threadIdx.x; i0 < part.nvec; i0 += U * THREADS) {
+  for (int i0 = tid; i0 < part.nvec; i0 += U * THREADS) {
     uint4 q[U];
 #pragma unroll
     for (int u = 0; u < U; ++u)
@@ -74,72 +77,99 @@ ce_fwd_kernel(const T* __restrict__ logits, const long long* __restrict__ target
     m = mm;
   }
   // the elements before the first and after the last vector (at most 2 (V - 1))
-  for (int i = threadIdx.x; i < V - part.nvec * VN; i += THREADS) {
+  for (int i = tid; i < V - part.nvec * VN; i += THREADS) {
     const float v = to_f32<T>(x[i < part.head ? i : part.nvec * VN + i]);
     ce_merge(m, s, v, 1.f);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1)
     ce_merge(m, s, __shfl_xor_sync(0xffffffffu, m, o), __shfl_xor_sync(0xffffffffu, s, o));
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  if (l == 0) { smax[w] = m; ssum[w] = s; }
-  __syncthreads();
-  if (w == 0) {
+  if (W > 1) {
+    const int w = tid >> 5, l = tid & 31;
+    if (l == 0) { smax[w] = m; ssum[w] = s; }
+    __syncthreads();
+    if (w > 0) return;
     m = l < W ? smax[l] : -INFINITY;
     s = l < W ? ssum[l] : 0.f;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
       ce_merge(m, s, __shfl_xor_sync(0xffffffffu, m, o), __shfl_xor_sync(0xffffffffu, s, o));
-    if (l == 0) {
-      const float L = m + logf(s);
-      lse[row] = L;
-      const long long t = target[row];
-      loss[row] = (t == ignore_index || t < 0 || t >= V) ? 0.f : L - to_f32<T>(x[t]);
-    }
+  }
+  if (tid == 0) {
+    const float L = m + logf(s);
+    lse[row] = L;
+    const long long t = target[row];
+    loss[row] = (t == ignore_index || t < 0 || t >= V) ? 0.f : L - to_f32<T>(x[t]);
   }
 }
 
-// Mean of the row losses over the rows whose target is not ignore_index: mean = sum / count,
-// inv = 1 / count (count at least 1).  One CTA: a call has few thousand rows of one float, and
-// one launch takes the place of five of elementwise and reduction kernels.
-__global__ void __launch_bounds__(1024)
-ce_mean_kernel(const float* __restrict__ loss, const long long* __restrict__ target,
-               float* __restrict__ mean, float* __restrict__ inv, long long rows,
-               long long ignore_index) {
+// sums over a CTA of 1024 threads, for its first warp
+__device__ __forceinline__ void ce_mean_fold(float& s, int& n) {
   __shared__ float ssum[32];
   __shared__ int scnt[32];
-  float s = 0.f;
-  int n = 0;
-  for (long long i = threadIdx.x; i < rows; i += 1024) {
-    s += loss[i];
-    n += target[i] != ignore_index;
-  }
   s = warp_sum(s);
   n = __reduce_add_sync(0xffffffffu, n);
   if ((threadIdx.x & 31) == 0) { ssum[threadIdx.x >> 5] = s; scnt[threadIdx.x >> 5] = n; }
   __syncthreads();
   if (threadIdx.x < 32) {
     s = warp_sum(ssum[threadIdx.x]);
-    n = max(1, __reduce_add_sync(0xffffffffu, scnt[threadIdx.x]));
-    if (threadIdx.x == 0) {
-      *mean = __fdiv_rn(s, (float)n);
-      *inv = __fdiv_rn(1.f, (float)n);
-    }
+    n = __reduce_add_sync(0xffffffffu, scnt[threadIdx.x]);
   }
 }
 
+// Mean of the row losses over the rows whose target is not ignore_index: mean = sum / count,
+// inv = 1 / count (count at least 1).  A call of some thousand rows is one CTA, one launch in the
+// place of five of elementwise and reduction kernels; beyond CE_MEAN_ROWS (per-pixel losses) the
+// CTAs of ce_mean_part_kernel leave a sum and a count each, and `target` is null here: a million
+// rows 86 -> 6 us.
+constexpr int CE_MEAN_ROWS = 16384;
+__global__ void __launch_bounds__(1024)
+ce_mean_kernel(const float* __restrict__ loss, const int* __restrict__ counts,
+               const long long* __restrict__ target, float* __restrict__ mean,
+               float* __restrict__ inv, int n_in, long long ignore_index) {
+  float s = 0.f;
+  int n = 0;
+  for (int i = threadIdx.x; i < n_in; i += 1024) {
+    s += loss[i];
+    n += target ? (int)(target[i] != ignore_index) : counts[i];
+  }
+  ce_mean_fold(s, n);
+  if (threadIdx.x == 0) {
+    n = max(1, n);
+    *mean = __fdiv_rn(s, (float)n);
+    *inv = __fdiv_rn(1.f, (float)n);
+  }
+}
+__global__ void __launch_bounds__(1024)
+ce_mean_part_kernel(const float* __restrict__ loss, const long long* __restrict__ target,
+                    float* __restrict__ sums, int* __restrict__ counts, long long rows,
+                    long long ignore_index) {
+  float s = 0.f;
+  int n = 0;
+#pragma unroll 4
+  for (long long i = (long long)blockIdx.x * 1024 + threadIdx.x; i < rows;
+       i += gridDim.x * 1024ll) {
+    s += loss[i];
+    n += target[i] != ignore_index;
+  }
+  ce_mean_fold(s, n);
+  if (threadIdx.x == 0) { sums[blockIdx.x] = s; counts[blockIdx.x] = n; }
+}
+
 // dlogits[row, i] = (exp(x - lse) - [i == target]) * gscale[row]
-// gscale = upstream gradient per row, or one for all rows (gstride 0: the mean's, already divided
-// by the number of valid rows).  The grid is (row, slab of the row): calls of few rows still fill the SMs.  Vectors are used when
-// the row and its gradient lie equally to 16 bytes.  2047 x 32000 bf16: 70 -> 51 us, 5.1 TB/s.
-template <typename T>
+// gscale = upstream gradient per row, or one for all rows (gstride 0: the mean's, already divided by
+// the number of valid rows).  THREADS threads per row; with 256 the grid is (row, slab of the row),
+// so that calls of few rows still fill the SMs.  Vectors are used when the row and its gradient lie
+// equally to 16 bytes.  2047 x 32000 bf16: 70 -> 51 us, 5.1 TB/s.
+template <typename T, int THREADS>
 __global__ void __launch_bounds__(256)
 ce_bwd_kernel(const T* __restrict__ logits, const long long* __restrict__ target,
               const float* __restrict__ lse, const float* __restrict__ gscale,
-              T* __restrict__ dlogits, int V, long long ld, long long ignore_index,
+              T* __restrict__ dlogits, long long rows, int V, long long ld, long long ignore_index,
               long long gstride) {
-  constexpr int VN = RowSplit<T>::V;
-  const long long row = blockIdx.x;
+  constexpr int VN = RowSplit<T>::V, UNROLL = THREADS < 128 ? 1 : THREADS < 256 ? 2 : 4;
+  const long long row = (long long)blockIdx.x * (256 / THREADS) + threadIdx.x / THREADS;
+  if (row >= rows) return;
   const T* x = logits + row * ld;
   T* d = dlogits + row * ld;
   const long long t = target[row];
@@ -150,13 +180,13 @@ ce_bwd_kernel(const T* __restrict__ logits, const long long* __restrict__ target
     if (i == t) p -= 1.f;
     return p * g;
   };
-  const int first = blockIdx.y * 256 + threadIdx.x, step = gridDim.y * 256;
+  const int first = blockIdx.y * THREADS + threadIdx.x % THREADS, step = gridDim.y * THREADS;
   if (((reinterpret_cast<uintptr_t>(x) ^ reinterpret_cast<uintptr_t>(d)) & 15) != 0) {
     for (int i = first; i < V; i += step) d[i] = from_f32<T>(grad(to_f32<T>(x[i]), i));
     return;
   }
   const RowSplit<T> part(x, V);
-#pragma unroll 4
+#pragma unroll UNROLL
   for (int i = first; i < part.nvec; i += step) {
     const uint4 q = __ldg(reinterpret_cast<const uint4*>(x + part.head) + i);
     const T* e = reinterpret_cast<const T*>(&q);
@@ -313,28 +343,69 @@ using namespace pf;
     default: return -1;                                        \
   }
 
+// Threads per row of the forward: with a CTA per short row a call is bound by the rate of CTAs, so
+// a row of up to 1024 elements is a warp's (200000 x 300 bf16: 351 -> 77 us, one row 2.6 -> 2.4); at
+// 1500 a CTA of 256 is ahead for few rows (64: 2.8 against 3.0 us).  Calls of no more rows than SMs
+// give a long row 1024 threads: 64 x 12000 3.8 -> 3.5 us, 1 x 60001 8.9 -> 5.8, but 64 x 8192
+// 3.1 -> 3.4 and 400 x 32000 8.2 -> 8.7.
+static int ce_fwd_threads(long long rows, int V, int sm_count) {
+  if (V <= 1024) return 32;
+  return rows <= sm_count && V > 8192 ? 1024 : 256;
+}
+// Threads per row of the backward, by the vectors of a row: a warp up to 64 (200000 x 512 bf16:
+// 284 -> 77 us), half a CTA up to 512 (20000 x 2048 fp32: 66 -> 54 us) unless the rows are too
+// few to fill the SMs (64 x 4096 bf16: 3.2 against 2.4 us).
+template <typename T>
+static int ce_bwd_threads(long long rows, int V, int sm_count) {
+  const int nvec = V / RowSplit<T>::V;
+  if (nvec <= 64) return 32;
+  return nvec <= 512 && rows > 2 * sm_count ? 128 : 256;
+}
+
 PF_API int pf_ce_fwd(const void* logits, const void* target, void* loss, void* lse, long long rows,
-                     int V, long long ld, long long ignore_index, int dtype, void* stream) {
+                     int V, long long ld, long long ignore_index, int dtype, int sm_count,
+                     void* stream) {
   if (rows <= 0) return 0;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (rows < 4 * 148) {
-    PF_DISPATCH3(dtype, (ce_fwd_kernel<T, 1024><<<(unsigned)rows, 1024, 0, st>>>(
-        (const T*)logits, (const long long*)target, (float*)loss, (float*)lse, V, ld,
-        ignore_index)));
-  } else {
-    PF_DISPATCH3(dtype, (ce_fwd_kernel<T, 256><<<(unsigned)rows, 256, 0, st>>>(
-        (const T*)logits, (const long long*)target, (float*)loss, (float*)lse, V, ld,
-        ignore_index)));
-  }
+#define PF_CE_FWD(THREADS)                                                                       \
+  ce_fwd_kernel<T, THREADS><<<(unsigned)(THREADS < 256 ? (rows + 7) / 8 : rows),                 \
+                              THREADS < 256 ? 256 : THREADS, 0, st>>>(                           \
+      (const T*)logits, (const long long*)target, (float*)loss, (float*)lse, rows, V, ld,        \
+      ignore_index)
+  PF_DISPATCH3(dtype, {
+    const int threads = ce_fwd_threads(rows, V, sm_count);
+    if (threads == 32) PF_CE_FWD(32);
+    else if (threads == 256) PF_CE_FWD(256);
+    else PF_CE_FWD(1024);
+  });
+#undef PF_CE_FWD
   PF_CHECK_LAUNCH();
   return 0;
 }
 
+// CTAs that share the sum of the row losses; more than one need scratch of that many floats and ints
+PF_API int pf_ce_mean_parts(long long rows, int sm_count) {
+  if (rows <= CE_MEAN_ROWS) return 1;
+  const long long n = (rows + CE_MEAN_ROWS / 4 - 1) / (CE_MEAN_ROWS / 4);
+  return (int)(n < sm_count ? n : sm_count);
+}
+
 // mean loss over the rows that count, and one over their number
-PF_API int pf_ce_mean(const void* loss, const void* target, void* mean, void* inv, long long rows,
-                      long long ignore_index, void* stream) {
-  ce_mean_kernel<<<1, 1024, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      (const float*)loss, (const long long*)target, (float*)mean, (float*)inv, rows, ignore_index);
+PF_API int pf_ce_mean(const void* loss, const void* target, void* scratch, void* mean, void* inv,
+                      long long rows, long long ignore_index, int sm_count, void* stream) {
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  const int parts = pf_ce_mean_parts(rows, sm_count);
+  if (parts > 1) {
+    float* sums = (float*)scratch;
+    int* counts = (int*)scratch + parts;
+    ce_mean_part_kernel<<<parts, 1024, 0, st>>>((const float*)loss, (const long long*)target, sums,
+                                                counts, rows, ignore_index);
+    ce_mean_kernel<<<1, 1024, 0, st>>>(sums, counts, nullptr, (float*)mean, (float*)inv, parts,
+                                       ignore_index);
+  } else {
+    ce_mean_kernel<<<1, 1024, 0, st>>>((const float*)loss, nullptr, (const long long*)target,
+                                       (float*)mean, (float*)inv, (int)rows, ignore_index);
+  }
   PF_CHECK_LAUNCH();
   return 0;
 }
@@ -342,16 +413,26 @@ PF_API int pf_ce_mean(const void* loss, const void* target, void* mean, void* in
 // gscale: one value per row (gstride 1) or one for all (gstride 0)
 PF_API int pf_ce_bwd(const void* logits, const void* target, const void* lse, const void* gscale,
                      void* dlogits, long long rows, int V, long long ld, long long ignore_index,
-                     long long gstride, int dtype, void* stream) {
+                     long long gstride, int dtype, int sm_count, void* stream) {
   if (rows <= 0) return 0;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  // at least eight CTAs per SM where the row length allows it (a slab: 256 vectors or more)
-  long long slabs = (8 * 148 + rows - 1) / rows;
+  // up to the eight CTAs that an SM holds where the row length allows it (a slab: 256 vectors or
+  // more); one more would be a second round (591 x 8192 bf16: 5.9 -> 5.1 us)
+  long long slabs = 8ll * sm_count / rows;
   const long long most = (V + 2047) / 2048;
   if (slabs > most) slabs = most;
-  PF_DISPATCH3(dtype, (ce_bwd_kernel<T><<<dim3((unsigned)rows, (unsigned)slabs), 256, 0, st>>>(
-      (const T*)logits, (const long long*)target, (const float*)lse, (const float*)gscale,
-      (T*)dlogits, V, ld, ignore_index, gstride)));
+  if (slabs < 1) slabs = 1;
+#define PF_CE_BWD(THREADS, GRID)                                                                 \
+  ce_bwd_kernel<T, THREADS><<<GRID, 256, 0, st>>>(                                               \
+      (const T*)logits, (const long long*)target, (const float*)lse, (const float*)gscale,       \
+      (T*)dlogits, rows, V, ld, ignore_index, gstride)
+  PF_DISPATCH3(dtype, {
+    const int threads = ce_bwd_threads<T>(rows, V, sm_count);
+    if (threads == 32) PF_CE_BWD(32, (unsigned)((rows + 7) / 8));
+    else if (threads == 128) PF_CE_BWD(128, (unsigned)((rows + 1) / 2));
+    else PF_CE_BWD(256, dim3((unsigned)rows, (unsigned)slabs));
+  });
+#undef PF_CE_BWD
   PF_CHECK_LAUNCH();
   return 0;
 }

@@ -320,8 +320,8 @@ def ce_fwd(logits: torch.Tensor, target: torch.Tensor, ignore_index: int = -100
     loss = torch.empty(rows, dtype=torch.float32, device=logits.device)
     lse = torch.empty(rows, dtype=torch.float32, device=logits.device)
     check(L.pf_ce_fwd(ptr(logits), ptr(target.contiguous()), ptr(loss), ptr(lse), c_ll(rows), V,
-                      c_ll(logits.stride(0)), c_ll(ignore_index), dt(logits.dtype), stream()),
-          "pf_ce_fwd")
+                      c_ll(logits.stride(0)), c_ll(ignore_index), dt(logits.dtype),
+                      sm_count(logits.device), stream()), "pf_ce_fwd")
     return loss, lse
 
 
@@ -334,7 +334,8 @@ def ce_bwd(logits: torch.Tensor, target: torch.Tensor, lse: torch.Tensor,
         gscale = gscale.contiguous()
     check(L.pf_ce_bwd(ptr(logits), ptr(target.contiguous()), ptr(lse), ptr(gscale), ptr(d),
                       c_ll(rows), V, c_ll(logits.stride(0)), c_ll(ignore_index),
-                      c_ll(gscale.stride(0)), dt(logits.dtype), stream()), "pf_ce_bwd")
+                      c_ll(gscale.stride(0)), dt(logits.dtype), sm_count(logits.device), stream()),
+          "pf_ce_bwd")
     return d
 
 
@@ -345,8 +346,11 @@ def ce_mean(loss: torch.Tensor, target: torch.Tensor, ignore_index: int = -100
     assert loss.dtype == torch.float32 and loss.is_contiguous() and target.dtype == torch.int64
     mean = torch.empty((), dtype=torch.float32, device=loss.device)
     inv = torch.empty_like(mean)
-    check(L.pf_ce_mean(ptr(loss), ptr(target.contiguous()), ptr(mean), ptr(inv),
-                       c_ll(loss.numel()), c_ll(ignore_index), stream()), "pf_ce_mean")
+    rows, sms = loss.numel(), sm_count(loss.device)
+    parts = L.pf_ce_mean_parts(c_ll(rows), sms)
+    scratch = torch.empty(2 * parts, dtype=torch.float32, device=loss.device) if parts > 1 else None
+    check(L.pf_ce_mean(ptr(loss), ptr(target.contiguous()), ptr(scratch), ptr(mean), ptr(inv),
+                       c_ll(rows), c_ll(ignore_index), sms, stream()), "pf_ce_mean")
     return mean, inv
 
 

@@ -42,6 +42,20 @@ def test_cross_entropy_edges(rows, V, dtype):
         assert (dx.double() - dr).norm() <= (U[dtype] + 1e-5) * dr.norm() + sub
 
 
+@pytest.mark.parametrize("rows", [16384, 16385, 20000, 700001])
+def test_cross_entropy_of_many_rows(rows):
+    """Per-pixel losses: several CTAs sum the rows; the mean is that of the rows that count."""
+    from pfeife_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x = torch.randn(rows, 5, device="cuda", generator=g).requires_grad_()
+    t = torch.randint(0, 5, (rows,), device="cuda", generator=g)
+    t[1::3] = -100
+    xr = x.detach().double().requires_grad_()
+    loss, want = ops.cross_entropy(x, t), F.cross_entropy(xr, t)
+    close(loss, want, 0.0)
+    close(torch.autograd.grad(loss, x)[0], torch.autograd.grad(want, xr)[0], 0.0)
+
+
 def test_cross_entropy_masked_vocabulary_and_all_ignored():
     """Logits of -inf and of the type's lowest value have no probability; a batch without a row
     that counts has loss 0 and no gradient."""
