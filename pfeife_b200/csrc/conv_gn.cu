@@ -78,66 +78,112 @@ col2im_kernel(const T* __restrict__ dcols, T* __restrict__ dx, int B, int H, int
 
 // ------------------------------------------------------------------------------ conv weights
 // Between the [Cout, Cin, taps] order of a convolution's weight and the orders its products read.
-// Each CTA moves a tile through shared memory so that both sides are contiguous in global memory;
-// rows and channels beyond Cout / Cin (the products need multiples of 8) are zero.
-// Bound by latency at these sizes (7 MB at 640 channels): one launch for what took a strided copy
-// and, for the flipped taps, a second one.  Convolution forward and backward, bf16: 640 -> 640
-// channels on [4, 64, 64] 564 -> 538 us, 2560 -> 1280 on [1, 32, 32] 827 -> 666 us.
+// Each CTA moves a tile through shared memory so that both sides are contiguous in global memory,
+// 16 bytes a thread and request (`vec`: the weight's rows start on 16 bytes; else element by
+// element); rows and channels beyond Cout / Cin (the products need multiples of 8) are zero.
+// Bound by the latency of one short pass through L2.  640 x 640 x 9 bf16: packed 4.2 us, flipped
+// 6.0, gradient 7.8 (with 2 bytes a request 9.9, 17.4 and 12.6, as strided copies 8.1, 25.5 and
+// 12.9).  Convolution forward and backward, bf16: 640 -> 640 channels on [4, 64, 64] 546 -> 509 us
+// against strided copies, 2560 -> 1280 on [1, 32, 32] 807 -> 511 us.
 constexpr int CONV_PACK_TAPS = 64;     // most taps (7 x 7 fits)
+constexpr int CONV_TILE = 4096;        // elements of a tile: 8 channels of 64 taps fit
 
-// out[co, t, ci] = w[co, ci, t]
+// out[co, t, ci] = w[co, ci, t]; a tile is `per` channels (a multiple of 8) of one co
 __global__ void __launch_bounds__(128)
 conv_pack_kernel(const uint16_t* __restrict__ w, uint16_t* __restrict__ out, int Cout, int Cin,
-                 int taps, int cin8) {
-  __shared__ uint16_t tile[64 * CONV_PACK_TAPS];
-  const int co = blockIdx.x, ci0 = blockIdx.y * 64;
-  const int n_in = co < Cout ? max(0, min(64, Cin - ci0)) : 0, n_out = min(64, cin8 - ci0);
+                 int taps, int cin8, int per, int vec) {
+  __shared__ __align__(16) uint16_t tile[CONV_TILE];
+  const int co = blockIdx.x, ci0 = blockIdx.y * per;
+  const int n_in = co < Cout ? max(0, min(per, Cin - ci0)) : 0, n_out = min(per, cin8 - ci0) / 8;
   const uint16_t* src = w + ((long long)co * Cin + ci0) * taps;
-  for (int i = threadIdx.x; i < n_in * taps; i += 128) tile[i] = src[i];
+  if (vec) {
+    for (int i = threadIdx.x; i < n_in * taps / 8; i += 128)
+      reinterpret_cast<uint4*>(tile)[i] = __ldg(reinterpret_cast<const uint4*>(src) + i);
+  } else {
+    for (int i = threadIdx.x; i < n_in * taps; i += 128) tile[i] = src[i];
+  }
   __syncthreads();
-  for (int i = threadIdx.x; i < n_out * taps; i += 128) {
-    const int t = i / n_out, c = i - t * n_out;
-    out[((long long)co * taps + t) * cin8 + ci0 + c] = c < n_in ? tile[c * taps + t] : 0;
+  uint16_t* dst = out + (long long)co * taps * cin8 + ci0;
+  for (int i = threadIdx.x; i < taps * n_out; i += 128) {
+    const int t = i / n_out, c = (i - t * n_out) * 8;
+    uint4 q;
+    uint16_t* e = reinterpret_cast<uint16_t*>(&q);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) e[j] = c + j < n_in ? tile[(c + j) * taps + t] : 0;
+    *reinterpret_cast<uint4*>(dst + (long long)t * cin8 + c) = q;
   }
 }
 
-// out[ci, taps - 1 - t, co] = w[co, ci, t]: taps flipped, channel roles swapped
+// out[ci, taps - 1 - t, co] = w[co, ci, t]: taps flipped, channel roles swapped; a tile is 8 input
+// channels of `per` output channels (a multiple of 8)
 __global__ void __launch_bounds__(256)
 conv_pack_flip_kernel(const uint16_t* __restrict__ w, uint16_t* __restrict__ out, int Cout, int Cin,
-                      int taps, int cout8, int cin8, int ci_per) {
-  extern __shared__ uint16_t ftile[];  // [64 co][ci_per * taps], rows padded by one
-  const int ci0 = blockIdx.x * ci_per, co0 = blockIdx.y * 64;
-  const int n_ci = max(0, min(ci_per, Cin - ci0)), n_co = min(64, Cout - co0);
-  const int row = n_ci * taps, pitch = ci_per * taps + 1;
-  for (int i = threadIdx.x; i < n_co * row; i += 256) {
-    const int c = i / row, k = i - c * row;
-    ftile[c * pitch + k] = w[((long long)(co0 + c) * Cin + ci0) * taps + k];
+                      int taps, int cout8, int per, int vec) {
+  // [per][8 * taps + 2]: rows lie an odd number of words apart
+  extern __shared__ __align__(16) uint16_t ftile[];
+  const int ci0 = blockIdx.x * 8, co0 = blockIdx.y * per;
+  const int n_ci = max(0, min(8, Cin - ci0)), n_co = max(0, min(per, Cout - co0));
+  const int row = n_ci * taps, pitch = 8 * taps + 2;
+  const uint16_t* src = w + ((long long)co0 * Cin + ci0) * taps;
+  if (vec) {
+    for (int i = threadIdx.x; i < n_co * (row / 8); i += 256) {
+      const int c = i / (row / 8), k = (i - c * (row / 8)) * 8;
+      const uint4 q = __ldg(reinterpret_cast<const uint4*>(src + (long long)c * Cin * taps + k));
+      uint32_t* d = reinterpret_cast<uint32_t*>(ftile + c * pitch + k);
+      d[0] = q.x; d[1] = q.y; d[2] = q.z; d[3] = q.w;
+    }
+  } else {
+    for (int i = threadIdx.x; i < n_co * row; i += 256) {
+      const int c = i / row, k = i - c * row;
+      ftile[c * pitch + k] = src[(long long)c * Cin * taps + k];
+    }
   }
   __syncthreads();
-  const int o_co = min(64, cout8 - co0), o_ci = min(ci_per, cin8 - ci0);
-  for (int i = threadIdx.x; i < o_ci * taps * o_co; i += 256) {
-    const int k = i / o_co, c = i - k * o_co, ci = k / taps, t = k - ci * taps;
-    out[((long long)(ci0 + ci) * taps + (taps - 1 - t)) * cout8 + co0 + c] =
-        (c < n_co && ci < n_ci) ? ftile[c * pitch + k] : 0;
+  const int o_co = min(per, cout8 - co0) / 8;
+  for (int i = threadIdx.x; i < 8 * taps * o_co; i += 256) {
+    const int k = i / o_co, c = (i - k * o_co) * 8, ci = k / taps, t = k - ci * taps;
+    uint4 q;
+    uint16_t* e = reinterpret_cast<uint16_t*>(&q);
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      e[j] = (c + j < n_co && ci < n_ci) ? ftile[(c + j) * pitch + k] : 0;
+    *reinterpret_cast<uint4*>(out + ((long long)(ci0 + ci) * taps + (taps - 1 - t)) * cout8 + co0 +
+                              c) = q;
   }
 }
 
-// dw[co, ci, t] = src[co, t, ci] (fp32 sums with cin8 channels a row), converted to the weight's type
+// dw[co, ci, t] = src[co, t, ci] (fp32 sums with cin8 channels a row), converted to the weight's
+// type; a tile is `per` channels (a multiple of 8) of one co
 template <typename T>
 __global__ void __launch_bounds__(128)
-conv_unpack_kernel(const float* __restrict__ src, T* __restrict__ dw, int Cin, int taps, int cin8) {
-  __shared__ float tile[64 * (CONV_PACK_TAPS + 1)];
-  const int co = blockIdx.x, ci0 = blockIdx.y * 64, n = min(64, Cin - ci0);
-  const int pitch = taps | 1;          // odd: the transposing stores hit different banks
-  for (int i = threadIdx.x; i < n * taps; i += 128) {
-    const int t = i / n, c = i - t * n;
-    tile[c * pitch + t] = src[((long long)co * taps + t) * cin8 + ci0 + c];
+conv_unpack_kernel(const float* __restrict__ src, T* __restrict__ dw, int Cin, int taps, int cin8,
+                   int per, int vec) {
+  constexpr int V = 16 / sizeof(T);
+  __shared__ float tile[CONV_TILE + 64];
+  const int co = blockIdx.x, ci0 = blockIdx.y * per, n = min(per, Cin - ci0);
+  const int pitch = taps | 1;          // odd: the transposing stores spread over the banks
+  const int n4 = (n + 3) / 4;          // a row of sums has channels up to a multiple of 8
+  const float* s0 = src + (long long)co * taps * cin8 + ci0;
+  for (int i = threadIdx.x; i < taps * n4; i += 128) {
+    const int t = i / n4, c = (i - t * n4) * 4;
+    const float4 q = __ldg(reinterpret_cast<const float4*>(s0 + (long long)t * cin8 + c));
+    float* d = tile + c * pitch + t;
+    d[0] = q.x; d[pitch] = q.y; d[2 * pitch] = q.z; d[3 * pitch] = q.w;
   }
   __syncthreads();
   T* dst = dw + ((long long)co * Cin + ci0) * taps;
-  for (int i = threadIdx.x; i < n * taps; i += 128) {
-    const int c = i / taps, t = i - c * taps;
-    dst[i] = from_f32<T>(tile[c * pitch + t]);
+  const int step = vec ? V : 1;
+  for (int i = threadIdx.x * step; i < n * taps; i += 128 * step) {
+    int c = i / taps, t = i - c * taps;
+    if (!vec) { dst[i] = from_f32<T>(tile[c * pitch + t]); continue; }
+    uint4 q;
+    T* e = reinterpret_cast<T*>(&q);
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+      e[j] = from_f32<T>(tile[c * pitch + t]);
+      if (++t == taps) { t = 0; ++c; }
+    }
+    *reinterpret_cast<uint4*>(dst + i) = q;
   }
 }
 
@@ -565,34 +611,49 @@ PF_API int pf_groupnorm_bwd(const void* dy, const void* x, const void* mean, con
   return 0;
 }
 
-// 16-bit weights [Cout, Cin, taps] -> [cout8, taps, cin8], or with `flip` [cin8, taps reversed, cout8]
+// Channels per tile: equal shares, multiples of 8, of no more than `most`.
+static inline int conv_share(int channels, int most) {
+  const int tiles = (channels + most - 1) / most;
+  return ((channels + tiles - 1) / tiles + 7) / 8 * 8;
+}
+
+// 16-bit weights [Cout, Cin, taps] -> [cout8, taps, cin8], or with `flip` [cin8, taps reversed,
+// cout8]; cout8 / cin8 are multiples of 8, `out` lies on 16 bytes
 PF_API int pf_conv_pack(const void* w, void* out, int Cout, int Cin, int taps, int cout8, int cin8,
                         int flip, void* stream) {
-  if (taps < 1 || taps > CONV_PACK_TAPS) return -3;
+  if (taps < 1 || taps > CONV_PACK_TAPS || cout8 % 8 || cin8 % 8) return -3;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  const int vec = (reinterpret_cast<uintptr_t>(w) & 15) == 0 && (long long)Cin * taps % 8 == 0;
   if (!flip) {
-    conv_pack_kernel<<<dim3(cout8, (cin8 + 63) / 64), 128, 0, st>>>(
-        (const uint16_t*)w, (uint16_t*)out, Cout, Cin, taps, cin8);
+    const int per = conv_share(cin8, CONV_TILE / taps / 8 * 8);
+    conv_pack_kernel<<<dim3(cout8, (cin8 + per - 1) / per), 128, 0, st>>>(
+        (const uint16_t*)w, (uint16_t*)out, Cout, Cin, taps, cin8, per, vec);
   } else {
-    const int per = taps <= 16 ? 8 : 4;       // tile of at most 64 x 257 x 2 bytes
-    conv_pack_flip_kernel<<<dim3((cin8 + per - 1) / per, (cout8 + 63) / 64), 256,
-                            64 * (per * taps + 1) * 2, st>>>((const uint16_t*)w, (uint16_t*)out,
-                                                             Cout, Cin, taps, cout8, cin8, per);
+    // tiles of 5 to 8 thousand elements; 64 channels make whole 128-byte lines of the output
+    const int per = taps <= 9 ? 64 : taps <= 25 ? 32 : 16;
+    conv_pack_flip_kernel<<<dim3(cin8 / 8, (cout8 + per - 1) / per), 256,
+                            per * (8 * taps + 2) * 2, st>>>((const uint16_t*)w, (uint16_t*)out,
+                                                            Cout, Cin, taps, cout8, per, vec);
   }
   PF_CHECK_LAUNCH();
   return 0;
 }
 
-// fp32 [>= Cout, taps, cin8] -> [Cout, Cin, taps] of `dtype`
+// fp32 [>= Cout, taps, cin8] on 16 bytes -> [Cout, Cin, taps] of `dtype`; cin8 is a multiple of 8
 PF_API int pf_conv_unpack(const void* src, void* dw, int Cout, int Cin, int taps, int cin8,
                           int dtype, void* stream) {
-  if (taps < 1 || taps > CONV_PACK_TAPS) return -3;
+  if (taps < 1 || taps > CONV_PACK_TAPS || cin8 % 8) return -3;
+  if (reinterpret_cast<uintptr_t>(src) & 15) return -2;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  const dim3 grid(Cout, (Cin + 63) / 64);
+  const int per = conv_share(cin8, CONV_TILE / (taps | 1) / 8 * 8);
+  const dim3 grid(Cout, (Cin + per - 1) / per);
+  const int vec = (reinterpret_cast<uintptr_t>(dw) & 15) == 0 &&
+                  (long long)Cin * taps % (dtype == PF_F32 ? 4 : 8) == 0;
+  const float* s = (const float*)src;
   switch (dtype) {
-    case PF_F32: conv_unpack_kernel<float><<<grid, 128, 0, st>>>((const float*)src, (float*)dw, Cin, taps, cin8); break;
-    case PF_F16: conv_unpack_kernel<__half><<<grid, 128, 0, st>>>((const float*)src, (__half*)dw, Cin, taps, cin8); break;
-    case PF_BF16: conv_unpack_kernel<__nv_bfloat16><<<grid, 128, 0, st>>>((const float*)src, (__nv_bfloat16*)dw, Cin, taps, cin8); break;
+    case PF_F32: conv_unpack_kernel<float><<<grid, 128, 0, st>>>(s, (float*)dw, Cin, taps, cin8, per, vec); break;
+    case PF_F16: conv_unpack_kernel<__half><<<grid, 128, 0, st>>>(s, (__half*)dw, Cin, taps, cin8, per, vec); break;
+    case PF_BF16: conv_unpack_kernel<__nv_bfloat16><<<grid, 128, 0, st>>>(s, (__nv_bfloat16*)dw, Cin, taps, cin8, per, vec); break;
     default: return -1;
   }
   PF_CHECK_LAUNCH();

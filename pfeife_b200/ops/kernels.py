@@ -556,7 +556,8 @@ def conv_pack(w: torch.Tensor, cout8: int, cin8: int, flip: bool = False) -> tor
     Cout, Cin, KH, KW = w.shape
     taps = KH * KW
     if taps > 64:                      # beyond the kernels' tile
-        w = torch.nn.functional.pad(w, (0, 0, 0, 0, 0, cin8 - Cin, 0, cout8 - Cout))
+        if cin8 != Cin or cout8 != Cout:
+            w = torch.nn.functional.pad(w, (0, 0, 0, 0, 0, cin8 - Cin, 0, cout8 - Cout))
         p = w.flip(2, 3).permute(1, 2, 3, 0) if flip else w.permute(0, 2, 3, 1)
         return p.reshape(p.shape[0], -1).contiguous()
     out = torch.empty((cin8, taps * cout8) if flip else (cout8, taps * cin8), dtype=w.dtype,
@@ -571,8 +572,9 @@ def conv_unpack(dw2: torch.Tensor, shape, cin8: int, dtype: torch.dtype) -> torc
     L = _lib.lib()
     Cout, Cin, KH, KW = shape
     assert dw2.dtype == torch.float32 and dw2.is_contiguous()
-    if KH * KW == 1 and cin8 == Cin and dtype == torch.float32:
-        return dw2[:Cout].view(Cout, Cin, 1, 1)
+    if KH * KW == 1 and cin8 == Cin:
+        p = dw2[:Cout].view(Cout, Cin, 1, 1)               # the same order already
+        return p.to(dtype)
     if KH * KW > 64:
         p = dw2.view(-1, KH, KW, cin8)[:Cout, :, :, :Cin].permute(0, 3, 1, 2)
         return p.to(dtype).contiguous()

@@ -197,3 +197,27 @@ def test_conv_weight_views(layout, K, w_dtype):
         out.append((y,) + torch.autograd.grad(y, leaves, torch.ones_like(y)))
     for a, b in zip(*out):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("Cout,Cin,taps", [
+    (8, 8, 1), (1, 1, 1), (21, 13, 1), (9, 4104, 1), (64, 64, 4), (64, 520, 9), (17, 455, 9),
+    (72, 9, 25), (16, 96, 49), (5, 3, 49), (33, 120, 63), (24, 65, 64), (7, 16, 65)])
+def test_conv_weight_kernels_move_every_element(Cout, Cin, taps):
+    """Packed, flipped and gradient orders at the edges of the tiles (64 taps, whole and ragged
+    vectors, several shares of the channels), bit for bit."""
+    from pfeife_b200.ops import kernels as kx
+    cout8, cin8 = (Cout + 7) // 8 * 8, (Cin + 7) // 8 * 8
+    w = torch.randn(Cout, Cin, taps, 1, device="cuda").to(torch.bfloat16)
+    full = w.new_zeros(cout8, cin8, taps)
+    full[:Cout, :Cin] = w[..., 0]
+    shifted = torch.empty(w.numel() + 1, dtype=w.dtype, device="cuda")[1:].view(w.shape).copy_(w)
+    for src in (w, shifted):                      # 16-byte aligned or not
+        assert torch.equal(kx.conv_pack(src, cout8, cin8),
+                           full.permute(0, 2, 1).reshape(cout8, -1))
+        assert torch.equal(kx.conv_pack(src, cout8, cin8, flip=True),
+                           full.flip(2).permute(1, 2, 0).reshape(cin8, -1))
+    sums = torch.randn(cout8, taps * cin8, device="cuda")
+    want = sums.view(cout8, taps, cin8)[:Cout, :, :Cin].permute(0, 2, 1).reshape(w.shape)
+    for dtype in (torch.float32, torch.bfloat16, torch.float16):
+        got = kx.conv_unpack(sums, w.shape, cin8, dtype)
+        assert got.is_contiguous() and torch.equal(got, want.to(dtype))
