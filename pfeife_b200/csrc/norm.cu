@@ -205,9 +205,11 @@ norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ h, const float* 
 // expanded once per pass (sum, squared deviations, output): a third of the registers of an fp32
 // copy.  Bound by HBM: x and the residual are requested together, without a register limit that
 // would spill them; bf16 with residual 6168 x 1408 29 -> 23 us, 50000 x 1408 129 -> 102 us
-// (5.5 TB/s), 20000 x 2048 98 -> 75 us.
-template <typename T, int NV>
-__global__ void __launch_bounds__(256)
+// (5.5 TB/s), 20000 x 2048 98 -> 75 us.  Rows of one or two vectors a lane without a residual are
+// bound by the instructions around their loads and have a form of their own (MAY_RES false):
+// 200000 x 64 47.5 -> 43.7 us.
+template <typename T, int NV, bool MAY_RES>
+__global__ void __launch_bounds__(256, MAY_RES ? 0 : 4)
 norm_fwd_warp_kernel(const T* __restrict__ x, const T* __restrict__ res,
                      const float* __restrict__ gamma, const float* __restrict__ beta,
                      T* __restrict__ y, T* __restrict__ h_out, float* __restrict__ mean_out,
@@ -217,24 +219,24 @@ norm_fwd_warp_kernel(const T* __restrict__ x, const T* __restrict__ res,
   const int lane = threadIdx.x & 31;
   const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (row >= rows) return;
-  uint4 q[NV], qr[NV];
+  uint4 q[NV], qr[MAY_RES ? NV : 1];
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     const int idx = lane + i * 32;
     if (idx < nvec) q[i] = reinterpret_cast<const uint4*>(x + row * N)[idx];
   }
-  if (res) {      // h = x + residual, rounded to the storage type like the unfused sequence
+  if (MAY_RES && res) {   // h = x + residual, rounded to the storage type like the unfused sequence
     // both streams are requested before either is used
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       const int idx = lane + i * 32;
-      if (idx < nvec) qr[i] = reinterpret_cast<const uint4*>(res + row * N)[idx];
+      if (idx < nvec) qr[MAY_RES ? i : 0] = reinterpret_cast<const uint4*>(res + row * N)[idx];
     }
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       const int idx = lane + i * 32;
       if (idx < nvec) {
-        const T* er = reinterpret_cast<const T*>(&qr[i]);
+        const T* er = reinterpret_cast<const T*>(&qr[MAY_RES ? i : 0]);
         T* e = reinterpret_cast<T*>(&q[i]);
 #pragma unroll
         for (int j = 0; j < V; ++j) e[j] = from_f32<T>(to_f32<T>(e[j]) + to_f32<T>(er[j]));
@@ -619,15 +621,16 @@ static int norm_fwd_launch(const void* x, const void* res, const float* gamma, c
   constexpr int V = 16 / sizeof(T);
   if (N % V) return -2;
   const int nvec = N / V;
-  if (sizeof(T) == 2 && nvec <= 32 * 8) {
+  if constexpr (sizeof(T) == 2) if (nvec <= 32 * 8) {
     const unsigned grid = (unsigned)((rows + 7) / 8);
-#define PF_NORM_FWD_WARP(NV)                                                                  \
-    norm_fwd_warp_kernel<T, NV><<<grid, 256, 0, st>>>((const T*)x, (const T*)res, gamma, beta, \
-        (T*)y, (T*)h_out, mean, rstd, rows, N, eps, rms)
-    if (nvec <= 32 * 2) PF_NORM_FWD_WARP(2);
-    else if (nvec <= 32 * 4) PF_NORM_FWD_WARP(4);
-    else if (nvec <= 32 * 6) PF_NORM_FWD_WARP(6);
-    else PF_NORM_FWD_WARP(8);
+#define PF_NORM_FWD_WARP(NV, MAY_RES)                                                         \
+    norm_fwd_warp_kernel<T, NV, MAY_RES><<<grid, 256, 0, st>>>((const T*)x, (const T*)res, gamma, \
+        beta, (T*)y, (T*)h_out, mean, rstd, rows, N, eps, rms)
+    if (nvec <= 32 * 2 && !res) PF_NORM_FWD_WARP(2, false);
+    else if (nvec <= 32 * 2) PF_NORM_FWD_WARP(2, true);
+    else if (nvec <= 32 * 4) PF_NORM_FWD_WARP(4, true);
+    else if (nvec <= 32 * 6) PF_NORM_FWD_WARP(6, true);
+    else PF_NORM_FWD_WARP(8, true);
 #undef PF_NORM_FWD_WARP
     return 0;
   }
