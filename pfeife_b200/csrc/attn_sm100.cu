@@ -7,8 +7,9 @@
 // the tail of the last 64-element block is filled with zeros by TMA, never with the next head).
 //
 // A persistent kernel, one CTA per SM, walks over items of up to 256 query rows of one (head,
-// batch): two query tiles of 128 that share every K / V tile it loads.  Its warps:
-//   warps 0-3 / 4-7   softmax of query tile 0 / 1, thread <-> query row <-> TMEM lane
+// batch): two query tiles of 128 that share every K / V tile it loads (or, where pairs would leave
+// SMs idle, one tile whose keys are shared out: see FwdItem).  Its warps:
+//   warps 0-3 / 4-7   softmax of side 0 / 1, thread <-> query row <-> TMEM lane
 //   warp 8            TMA producer (K and V rings; runs ahead, across item boundaries too)
 //   warp 9            MMA issuer, TMEM owner                   warps 10, 11  idle
 // Per query tile t and key tile j:
@@ -20,8 +21,8 @@
 //                       more than 2^8 since it was last set (P stays below 2^8, which both 16-bit
 //                       formats hold, and most tiles need no rescaling)
 // What bounds it: 16384 exponentials per tile, 1024 cycles of the special-function units, against
-// 16 x head dim cycles of tensor core.  Two tiles in flight keep one tile's products under the
-// other's exponentials.
+// 8 x head dim cycles of tensor core (512 at head dim 64; at 128 both take 1024).  Two tiles in
+// flight keep one tile's products under the other's exponentials.
 // Measured (B200, CUDA events, L2 flushed), against one query tile per CTA with P in shared
 // memory: [4, 4096, 10, 64] 402 -> 346 us, causal [1, 2048, 32, 128] 87 -> 59,
 // [2, 2048, 16, 128] 114 -> 96, causal [6, 1782, 21, 32] 200 -> 117, 77 keys [4, 1024, 20, 64]
@@ -52,7 +53,8 @@ struct AttnParams {
   float* lse;           // [B,H,Sq]
   int* status;
   int q_rows;           // query rows of the tensor-core kernel; the others are leftover rows
-  int q_pairs;          // items per head: ceil(q_rows / 256)
+  int q_pairs;          // pairs of query tiles per head: ceil(q_rows / 256)
+  int n_pair;           // the first items are pairs, the others split tiles (see FwdItem)
   int q_tail;           // leftover rows
   // raw views for the leftover rows (element strides: batch, seq, head)
   const void* q; const void* k; const void* v;
@@ -209,7 +211,8 @@ struct FwdCfg {
   static constexpr int ST = NBLK >= 2 ? 2 : 4;          // K/V ring stages
   static constexpr int OFF_K = 2 * TILE;
   static constexpr int OFF_V = OFF_K + ST * TILE;
-  static constexpr int OFF_BAR = OFF_V + ST * TILE;
+  static constexpr int OFF_SIDE = OFF_V + ST * TILE;     // maxima and sums of a split tile's side 1
+  static constexpr int OFF_BAR = OFF_SIDE + 2 * ATT_BM * 4;
   static constexpr int SMEM = OFF_BAR + 256;
   static constexpr int T_O = 256;                        // + t * DP
   static constexpr int T_P = ALIAS_P ? 0 : 256 + 2 * DP;
@@ -222,31 +225,50 @@ struct FwdCfg {
   static_assert((ALIAS_P ? T_O + 2 * DP : T_P + 128) <= 512, "TMEM columns");
 };
 
+// An item is a pair of query tiles that read the same key tiles or, when the pairs left over after
+// whole rounds of the SMs are no more than half of those, one query tile whose key tiles are dealt to
+// the two sides in turn; each side then has the maximum, sum and output of its own keys, which side 0
+// joins at the end.  A split tile takes half the steps of a pair; it is always its CTA's last item.
+// Head dim 128, 2048 tokens: 8 heads (64 pairs) 45 us as pairs, 28 split; 20 heads (160 pairs) 89
+// and 72.  Head dim 64, [1, 2048, 8, 64]: 38 and 24 us.
+template <bool SPLIT>     // some items are split tiles
 struct FwdItem {
-  int q0, h, b, n[2];    // first query row; key tiles seen by the two query tiles
+  int q0, q1, h, b;      // first query row of the two sides
+  int n[2], keys;        // key tiles that each side sees; key tiles to load
+  bool split;
+  // key tile of step i of side t
+  __device__ __forceinline__ int key(int t, int i) const {
+    return SPLIT && split ? 2 * i + t : i;
+  }
 };
-__device__ __forceinline__ FwdItem fwd_item(const AttnParams& p, int w) {
-  FwdItem it;
+template <bool SPLIT>
+__device__ __forceinline__ FwdItem<SPLIT> fwd_item(const AttnParams& p, int w) {
+  FwdItem<SPLIT> it;
+  it.split = SPLIT && w >= p.n_pair;
+  const int u = w - p.n_pair, pair = it.split ? p.n_pair + (u >> 1) : w;
   int qp, bh;
   if (p.causal) {
     // later queries see more keys: the long items of every head are dealt first
-    qp = w / (p.B * p.H);
-    bh = w - qp * (p.B * p.H);
+    qp = pair / (p.B * p.H);
+    bh = pair - qp * (p.B * p.H);
     qp = p.q_pairs - 1 - qp;
   } else {
-    bh = w / p.q_pairs;
-    qp = w - bh * p.q_pairs;
+    bh = pair / p.q_pairs;
+    qp = pair - bh * p.q_pairs;
   }
-  it.q0 = qp * 2 * ATT_BM;
+  it.q0 = qp * 2 * ATT_BM + (it.split && (u & 1) ? ATT_BM : 0);
+  it.q1 = it.split ? it.q0 : it.q0 + ATT_BM;
   it.h = bh % p.H;
   it.b = bh / p.H;
-#pragma unroll
-  for (int t = 0; t < 2; ++t) {
-    const int q0 = it.q0 + t * ATT_BM;
+  auto tiles = [&](int q0) {
     int kv_end = p.Sk;
     if (p.causal) kv_end = min(p.Sk, q0 + ATT_BM + (p.Sk - p.Sq));
-    it.n[t] = (q0 < p.q_rows && kv_end > 0) ? (kv_end + ATT_BN - 1) / ATT_BN : 0;
-  }
+    return (q0 < p.q_rows && kv_end > 0) ? (kv_end + ATT_BN - 1) / ATT_BN : 0;
+  };
+  const int n0 = tiles(it.q0), n1 = it.split ? 0 : tiles(it.q1);
+  it.keys = max(n0, n1);
+  it.n[0] = it.split ? (n0 + 1) / 2 : n0;
+  it.n[1] = it.split ? n0 / 2 : n1;
   return it;
 }
 // rounds run alternately forwards and backwards over the CTAs, so that a CTA with a long item in
@@ -290,11 +312,12 @@ __device__ __forceinline__ float probs(const uint32_t (&s)[4][32], uint32_t (&pk
   return (a + b) + (d + e);
 }
 
-template <typename T, int DP>
+template <typename T, int DP, bool SPLIT>
 __global__ void __launch_bounds__(FwdCfg<DP>::THREADS, 1)
 attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                    const __grid_constant__ CUtensorMap tv, const AttnParams p, const int n_items) {
   using C = FwdCfg<DP>;
+  using Item = FwdItem<SPLIT>;
   constexpr int NBLK = C::NBLK, TILE = C::TILE, ST = C::ST;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::OFF_BAR);
@@ -308,8 +331,10 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
   uint64_t* k_empty = k_full + ST;
   uint64_t* v_full = k_empty + ST;
   uint64_t* v_empty = v_full + ST;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(v_empty + ST);
-  constexpr int N_BARS = 12 + 4 * ST;
+  uint64_t* joined = v_empty + ST;       // side 1 of a split tile has left its maxima and sums
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(joined + 1);
+  constexpr int N_BARS = 13 + 4 * ST;
+  float* side1 = reinterpret_cast<float*>(smem + C::OFF_SIDE);   // [2][128]
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // the 128-byte swizzle works on absolute shared-memory addresses
@@ -321,6 +346,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
     tma_prefetch_desc(&tq); tma_prefetch_desc(&tk); tma_prefetch_desc(&tv);
     for (int i = 0; i < N_BARS; ++i) mbar_init(&bars[i], 1);
     for (int t = 0; t < 2; ++t) { mbar_init(&s_empty[t], 4); mbar_init(&p_full[t], 4); }
+    mbar_init(joined, 4);
     mbar_fence_init();
   }
   if (warp == 9) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
@@ -340,9 +366,8 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
         for (int r = 0; ok && r * (int)gridDim.x < n_items; ++r) {
           const int w = fwd_index(r);
           if (w >= n_items) continue;
-          const FwdItem it = fwd_item(p, w);
-          const int nmax = max(it.n[0], it.n[1]);
-          for (int j = 0; j < nmax && ok; ++j, ++g) {
+          const Item it = fwd_item<SPLIT>(p, w);
+          for (int j = 0; j < it.keys && ok; ++j, ++g) {
             const int st = g % ST;
             if (j == 0 && it.n[0] > 0) {
               ok = mbar_wait(&q_empty[0], (qc[0] & 1) ^ 1, p.status, PF_ERR_TIMEOUT_EMPTY);
@@ -356,7 +381,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
             if (j == 0 && it.n[1] > 0) {
               ok = mbar_wait(&q_empty[1], (qc[1] & 1) ^ 1, p.status, PF_ERR_TIMEOUT_EMPTY);
               if (!ok) break;
-              load_tile<NBLK>(smem + TILE, &tq, &q_full[1], it.h, it.q0 + ATT_BM, it.b);
+              load_tile<NBLK>(smem + TILE, &tq, &q_full[1], it.h, it.q1, it.b);
               ++qc[1];
             }
             ok = mbar_wait(&v_empty[st], ((g / ST) & 1) ^ 1, p.status, PF_ERR_TIMEOUT_EMPTY);
@@ -372,75 +397,78 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
         const uint32_t on = lane == 0;
         const uint32_t id_s = make_idesc_f16(128, 128, p.fmt, 0, 0);
         const uint32_t id_o = make_idesc_f16(128, DP, p.fmt, 0, 1);
-        uint32_t g = 0, qc[2] = {0, 0}, cnt[2] = {0, 0};    // cnt: S tiles issued per query tile
+        uint32_t g = 0, qc[2] = {0, 0}, cnt[2] = {0, 0};    // cnt: S tiles issued per side
         bool ok = true;
-        // S_t of key tile j (ring position gg).  Its columns must be free: the previous scores are
-        // in registers, or (P in the same columns) the previous P V has read its probabilities.
-        auto issue_s = [&](int t, uint32_t gg, int j, int n, bool last_of_tile) -> bool {
-          const int st = gg % ST;
-          if (j == 0) {
+        // in a pair, tile 1 reads every key tile that tile 0 reads, and after it
+        auto last_reader = [](const Item& it, int t, int i) {
+          return (SPLIT && it.split) || t == 1 || i >= it.n[1];
+        };
+        // S of step i of side t.  Its columns must be free: the previous scores are in registers,
+        // or (P in the same columns) the previous P V has read its probabilities.
+        auto issue_s = [&](const Item& it, int t, int i) -> bool {
+          const int kt = it.key(t, i), st = (g + kt) % ST;
+          if (i == 0) {
             if (!mbar_wait_warp(&q_full[t], qc[t] & 1, p.status, PF_ERR_TIMEOUT_FULL)) return false;
             ++qc[t];
           }
-          if (!mbar_wait_warp(&k_full[st], (gg / ST) & 1, p.status, PF_ERR_TIMEOUT_FULL))
+          if (!mbar_wait_warp(&k_full[st], ((g + kt) / ST) & 1, p.status, PF_ERR_TIMEOUT_FULL))
             return false;
           if (cnt[t] > 0 && !mbar_wait_warp(C::ALIAS_P ? &pv_done[t] : &s_empty[t],
                                             (cnt[t] - 1) & 1, p.status,
                                             PF_ERR_TIMEOUT_TMEM_EMPTY))
             return false;
           tc_fence_after();
-          const int rem = min(ATT_BN, p.Sk - j * ATT_BN);
+          const int rem = min(ATT_BN, p.Sk - kt * ATT_BN);
           const int n_mma = (rem + 15) / 16 * 16;
           const uint32_t id = n_mma == ATT_BN ? id_s : make_idesc_f16(128, n_mma, p.fmt, 0, 0);
           mma_kk_on<DP / 16>(on, tmem + t * 128, smem_u32(smem + t * TILE),
                           smem_u32(smem + C::OFF_K + st * TILE), id);
-          if (last_of_tile) tc_commit_on(on, &k_empty[st]);
+          if (last_reader(it, t, i)) tc_commit_on(on, &k_empty[st]);
           tc_commit_on(on, &s_full[t]);
-          if (j == n - 1) tc_commit_on(on, &q_empty[t]);
+          if (i == it.n[t] - 1) tc_commit_on(on, &q_empty[t]);
           ++cnt[t];
           return true;
         };
         for (int r = 0; ok && r * (int)gridDim.x < n_items; ++r) {
           const int w = fwd_index(r);
           if (w >= n_items) continue;
-          const FwdItem it = fwd_item(p, w);
-          const int nmax = max(it.n[0], it.n[1]);
-          // tile 1 reads every key tile that tile 0 reads, and after it
-          auto last_reader = [&](int t, int j) { return t == 1 || j >= it.n[1]; };
+          const Item it = fwd_item<SPLIT>(p, w);
+          const int steps = max(it.n[0], it.n[1]);
 #pragma unroll
           for (int t = 0; t < 2; ++t)
-            if (ok && it.n[t] > 0) ok = issue_s(t, g, 0, it.n[t], last_reader(t, 0));
-          for (int j = 0; j < nmax && ok; ++j) {
-            const uint32_t gg = g + j;
-            const int st = gg % ST;
+            if (ok && it.n[t] > 0) ok = issue_s(it, t, 0);
+          for (int i = 0; i < steps && ok; ++i) {
             if (!C::ALIAS_P) {
 #pragma unroll
               for (int t = 0; t < 2; ++t)
-                if (ok && j + 1 < it.n[t])
-                  ok = issue_s(t, gg + 1, j + 1, it.n[t], last_reader(t, j + 1));
+                if (ok && i + 1 < it.n[t]) ok = issue_s(it, t, i + 1);
               if (!ok) break;
             }
-            ok = mbar_wait_warp(&v_full[st], (gg / ST) & 1, p.status, PF_ERR_TIMEOUT_FULL);
-            if (!ok) break;
-            const int k_steps = (min(ATT_BN, p.Sk - j * ATT_BN) + 15) / 16;
+            if (!SPLIT)        // one V tile for both sides
+              ok = mbar_wait_warp(&v_full[(g + i) % ST], ((g + i) / ST) & 1, p.status,
+                                  PF_ERR_TIMEOUT_FULL);
 #pragma unroll
             for (int t = 0; t < 2; ++t) {
-              if (!ok || j >= it.n[t]) continue;
-              // the tile whose probabilities are waited for is the one before any S issued above
-              const uint32_t c = cnt[t] - 1 - ((!C::ALIAS_P && j + 1 < it.n[t]) ? 1u : 0u);
-              ok = mbar_wait_warp(&p_full[t], c & 1, p.status, PF_ERR_TIMEOUT_FULL);
+              if (!ok || i >= it.n[t]) continue;
+              const int kt = it.key(t, i), st = (g + kt) % ST;
+              // the probabilities waited for are those of the step before any S issued above
+              const uint32_t c = cnt[t] - 1 - ((!C::ALIAS_P && i + 1 < it.n[t]) ? 1u : 0u);
+              if (SPLIT)
+                ok = mbar_wait_warp(&v_full[st], ((g + kt) / ST) & 1, p.status,
+                                    PF_ERR_TIMEOUT_FULL);
+              ok = ok && mbar_wait_warp(&p_full[t], c & 1, p.status, PF_ERR_TIMEOUT_FULL);
               if (!ok) continue;
               tc_fence_after();
+              const int k_steps = (min(ATT_BN, p.Sk - kt * ATT_BN) + 15) / 16;
               const uint32_t sV = smem_u32(smem + C::OFF_V + st * TILE);
               const uint32_t t_p = tmem + C::T_P + t * C::P_TILE;
-              mma_t_mn_on(on, tmem + C::T_O + t * DP, t_p, sV, id_o, j > 0, k_steps);
-              if (last_reader(t, j)) tc_commit_on(on, &v_empty[st]);
+              mma_t_mn_on(on, tmem + C::T_O + t * DP, t_p, sV, id_o, i > 0, k_steps);
+              if (last_reader(it, t, i)) tc_commit_on(on, &v_empty[st]);
               tc_commit_on(on, &pv_done[t]);
-              if (C::ALIAS_P && j + 1 < it.n[t])
-                ok = issue_s(t, gg + 1, j + 1, it.n[t], last_reader(t, j + 1));
+              if (C::ALIAS_P && i + 1 < it.n[t]) ok = issue_s(it, t, i + 1);
             }
           }
-          g += nmax;
+          g += it.keys;
         }
       }
       __syncwarp();
@@ -461,13 +489,13 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
     for (int r = 0; ok && r * (int)gridDim.x < n_items; ++r) {
       const int w = fwd_index(r);
       if (w >= n_items) continue;
-      const FwdItem it = fwd_item(p, w);
-      const int q0 = it.q0 + t * ATT_BM, n_tiles = t ? it.n[1] : it.n[0];
+      const Item it = fwd_item<SPLIT>(p, w);
+      const int q0 = t ? it.q1 : it.q0, n_tiles = t ? it.n[1] : it.n[0];
       const int qi = q0 + row;
-      if (q0 >= p.q_rows) continue;
+      if (q0 >= p.q_rows || (SPLIT && t && it.split && it.n[0] == 0)) continue;
       T* dst = reinterpret_cast<T*>(p.o) + (((long long)it.b * p.Sq + qi) * p.H + it.h) * p.D;
       float* lse_dst = p.lse + ((long long)it.b * p.H + it.h) * p.Sq + qi;
-      if (n_tiles == 0) {          // no key is visible to this query tile
+      if (n_tiles == 0 && !(SPLIT && t && it.split)) {      // no key is visible to this query tile
         if (qi < p.Sq) {
           for (int c = 0; c < p.D / 8; ++c)
             reinterpret_cast<uint4*>(dst)[c] = make_uint4(0, 0, 0, 0);
@@ -479,7 +507,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
       const bool warp_live = q0 + quad * 32 < p.Sq;
       float m_used = -INFINITY, l = 0.f;
       for (int j = 0; j < n_tiles && ok; ++j, ++cnt) {
-        const int k0 = j * ATT_BN;
+        const int k0 = it.key(t, j) * ATT_BN;
         const int rem = min(ATT_BN, p.Sk - k0);
         const int n_chunks = ((rem + 15) / 16 * 16 + 31) / 32;
         // a tile needs masks when it is ragged or crosses the causal diagonal of this q tile
@@ -569,18 +597,49 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
       }
       if (!ok) break;
       // ---- epilogue of the tile: O / l
-      ok = mbar_wait(&pv_done[t], (cnt - 1) & 1, p.status, PF_ERR_TIMEOUT_TMEM_FULL);
-      if (!ok) break;
-      tc_fence_after();
+      if (!SPLIT || n_tiles > 0) {
+        ok = mbar_wait(&pv_done[t], (cnt - 1) & 1, p.status, PF_ERR_TIMEOUT_TMEM_FULL);
+        if (!ok) break;
+        tc_fence_after();
+      }
+      float w0 = 1.f, w1 = 0.f;              // weights of the two sides' outputs
+      if (SPLIT && it.split) {
+        if (t) {                             // the thread of this row on side 0 finishes it
+          side1[row] = m_used;
+          side1[ATT_BM + row] = l;
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(joined);
+          continue;
+        }
+        ok = mbar_wait(joined, 0, p.status, PF_ERR_TIMEOUT_TMEM_FULL);
+        if (!ok) break;
+        tc_fence_after();
+        const float m1 = side1[row], m = fmaxf(m_used, m1), m_sub = (m == -INFINITY) ? 0.f : m;
+        w0 = exp2f(m_used - m_sub);
+        w1 = exp2f(m1 - m_sub);
+        l = l * w0 + side1[ATT_BM + row] * w1;
+        m_used = m;
+      }
       if (warp_live) {
         const float inv = l > 0.f ? 1.f / l : 0.f;
+        w0 *= inv;
+        w1 *= inv;
 #pragma unroll
         for (int c = 0; c < DP / 32; ++c) {
           uint32_t o[32];
           tmem_ld32(t_o + c * 32, o);
           tmem_ld_wait_for(o);
 #pragma unroll
-          for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * inv);
+          for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * w0);
+          if (SPLIT && it.split && it.n[1] > 0) {     // the same row of the other side's columns
+            uint32_t o1[32];
+            tmem_ld32(t_o + DP + c * 32, o1);
+            tmem_ld_wait_for(o1);
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              o[i] = __float_as_uint(fmaf(__uint_as_float(o1[i]), w1, __uint_as_float(o[i])));
+          }
           if (qi < p.Sq) {
 #pragma unroll
             for (int v = 0; v < 4; ++v)
@@ -606,11 +665,13 @@ template <typename T, int DP>
 static int launch_fwd_ws(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                          const AttnParams& p, cudaStream_t st) {
   using C = FwdCfg<DP>;
-  auto kern = attn_fwd_ws_kernel<T, DP>;
-  static bool done[64] = {};
-  int r = set_smem(kern, C::SMEM, done);
+  const int pairs = p.q_pairs * p.H * p.B, n_items = p.n_pair + 2 * (pairs - p.n_pair);
+  const int sms = attn_sm_count();
+  const bool split = p.n_pair < pairs;
+  auto kern = split ? attn_fwd_ws_kernel<T, DP, true> : attn_fwd_ws_kernel<T, DP, false>;
+  static bool done[2][64] = {};
+  int r = set_smem(kern, C::SMEM, done[split]);
   if (r) return r;
-  const int n_items = p.q_pairs * p.H * p.B, sms = attn_sm_count();
   if (n_items > 0) {
     kern<<<n_items < sms ? n_items : sms, C::THREADS, C::SMEM, st>>>(tq, tk, tv, p, n_items);
     PF_CHECK_LAUNCH();
@@ -655,6 +716,14 @@ PF_API int pf_attn_fwd(const void* q, const void* k, const void* v, void* o, voi
   p.q_tail = (Sq > ATT_BM && left > 0 && left <= ATT_TAIL_MAX && Sk <= ATT_TAIL_SEQ_MAX) ? left : 0;
   p.q_rows = Sq - p.q_tail;
   p.q_pairs = (p.q_rows + 2 * ATT_BM - 1) / (2 * ATT_BM);
+  // Pairs left over after whole rounds are split into tiles when these fit one round (FwdItem).  The
+  // form of the kernel that can do both takes 4 to 9 % longer over a pair, so that after four whole
+  // rounds the gain is used up (640 pairs of head dim 64: 340 us either way).  Causal items differ in
+  // length and are dealt by it: there only a call without a whole round is split.
+  const int pairs = p.q_pairs * H * B, left_over = pairs % attn_sm_count();
+  const int rounds = pairs / attn_sm_count();
+  const bool split = 2 * left_over <= attn_sm_count() && rounds <= (causal ? 0 : 4);
+  p.n_pair = split ? pairs - left_over : pairs;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   PF_ATTN_DISPATCH(launch_fwd_ws, tq, tk, tv, p, st);
 }

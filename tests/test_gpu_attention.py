@@ -120,6 +120,9 @@ BWD_EDGES = [  # B, H, Sq, Sk, D, causal: tile edges, remainders, every head-dim
     (1, 2, 100, 385, 64, True), (1, 2, 385, 100, 64, True), (1, 1, 300, 128, 72, True),
     (2, 5, 513, 640, 128, True), (1, 3, 640, 513, 128, False), (40, 10, 65, 65, 96, False),
     (7, 25, 130, 258, 128, False), (3, 67, 272, 272, 64, True),
+    # whole rounds of query tile pairs, then single tiles whose keys are shared out (one, some, empty)
+    (5, 31, 300, 300, 64, False), (1, 150, 40, 200, 32, False), (2, 75, 256, 128, 96, False),
+    (1, 1, 1024, 1024, 128, True), (1, 3, 700, 1500, 64, True),
 ]
 
 
