@@ -132,7 +132,7 @@ PF_DECL int pf_groupnorm_fwd(const void* x, const void* gamma, const void* beta,
 PF_DECL int pf_groupnorm_bwd(const void* dy, const void* x, const void* mean, const void* rstd,
                              const void* gamma, const void* beta, void* dx, void* dgamma,
                              void* dbeta, void* sums, void* scratch, int B, int HW, int C, int G,
-                             int act_silu, int accumulate, int dtype, int sm_count, void* stream);
+                             int act_silu, int dtype, int sm_count, void* stream);
 PF_DECL int pf_upsample2x(const void* x, void* y, int B, int H, int W, int C, int backward,
                           int dtype, int sm_count, void* stream);
 

@@ -58,24 +58,6 @@ __device__ __forceinline__ uint4 pack8(const uint32_t* r) {
                     pack2<T>(__uint_as_float(r[6]), __uint_as_float(r[7])));
 }
 
-// Writes 32 consecutive 16-bit values of row `r`, columns [c0, c0+32), into a [128 x 128]
-// K-major tile made of two swizzled [128 x 64] blocks.
-template <typename T>
-__device__ __forceinline__ void store_p_chunk(uint8_t* tile, int r, int c0, const float (&v)[32]) {
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const int c = c0 + j * 8;
-    const int blk = c >> 6;
-    const int chunk = (c & 63) >> 3;
-    uint4 q;
-    q.x = pack2<T>(v[j * 8 + 0], v[j * 8 + 1]);
-    q.y = pack2<T>(v[j * 8 + 2], v[j * 8 + 3]);
-    q.z = pack2<T>(v[j * 8 + 4], v[j * 8 + 5]);
-    q.w = pack2<T>(v[j * 8 + 6], v[j * 8 + 7]);
-    *reinterpret_cast<uint4*>(tile + blk * ATT_BLK + r * 128 + ((chunk ^ (r & 7)) << 4)) = q;
-  }
-}
-
 // one [128 rows x DP] tile = DP/64 (rounded up) swizzled blocks, loaded with one TMA per block
 template <int NBLK>
 __device__ __forceinline__ void load_tile(uint8_t* dst, const CUtensorMap* map, uint64_t* bar,

@@ -376,7 +376,7 @@ __global__ void gn_bwd_stats_kernel(const T* __restrict__ dy, const T* __restric
 __global__ void __launch_bounds__(1024)
 gn_bwd_fold_kernel(const float* __restrict__ part, const float* __restrict__ gpart,
                    float* __restrict__ sumA, float* __restrict__ sumB, float* __restrict__ dgamma,
-                   float* __restrict__ dbeta, int B, int slabs, int C, int G, int accumulate) {
+                   float* __restrict__ dbeta, int B, int slabs, int C, int G) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int group_ctas = (B * G + 31) / 32;
   if ((int)blockIdx.x < group_ctas) {
@@ -413,8 +413,8 @@ gn_bwd_fold_kernel(const float* __restrict__ part, const float* __restrict__ gpa
   g = warp_sum(red[0][warp][lane]);
   d = warp_sum(red[1][warp][lane]);
   if (lane == 0 && cw < C) {
-    dgamma[cw] = accumulate ? dgamma[cw] + g : g;
-    dbeta[cw] = accumulate ? dbeta[cw] + d : d;
+    dgamma[cw] = g;
+    dbeta[cw] = d;
   }
 }
 
@@ -576,12 +576,11 @@ PF_API int pf_groupnorm_fwd(const void* x, const void* gamma, const void* beta, 
   return 0;
 }
 
-// sums: fp32 scratch [2][B*G]; dgamma / dbeta fp32 [C], added to when `accumulate`
+// sums: fp32 scratch [2][B*G]; dgamma / dbeta fp32 [C]
 PF_API int pf_groupnorm_bwd(const void* dy, const void* x, const void* mean, const void* rstd,
                             const void* gamma, const void* beta, void* dx, void* dgamma,
                             void* dbeta, void* sums, void* scratch, int B, int HW, int C, int G,
-                            int act_silu, int accumulate, int dtype, int sm_count,
-                            void* stream) {
+                            int act_silu, int dtype, int sm_count, void* stream) {
   if (C % G || C % 8) return -2;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   float* sA = (float*)sums;
@@ -601,7 +600,7 @@ PF_API int pf_groupnorm_bwd(const void* dy, const void* x, const void* mean, con
                  G, rows);
     }
     gn_bwd_fold_kernel<<<(B * G + 31) / 32 + (C + 31) / 32, 1024, 0, st>>>(
-        part, gpart, sA, sB, (float*)dgamma, (float*)dbeta, B, slabs, C, G, accumulate);
+        part, gpart, sA, sB, (float*)dgamma, (float*)dbeta, B, slabs, C, G);
     const int smem = 0;
     PF_GN_SILU(gn_bwd_apply_kernel, (const T*)dy, (const T*)x, (const float*)mean,
                (const float*)rstd, (const float*)gamma, (const float*)beta, sA, sB, (T*)dx, HW, C,

@@ -656,7 +656,7 @@ static int norm_bwd_launch(const void* dy, const void* h, const float* gamma, co
   constexpr int V = 16 / sizeof(T);
   if (N % V) return -2;
   const int nvec = N / V;
-  if (sizeof(T) == 2 && nvec <= 32 * 8) {
+  if constexpr (sizeof(T) == 2) if (nvec <= 32 * 8) {
 #define PF_NORM_BWD_FUSED(NV)                                                                     \
     norm_bwd_fused_launch<T, NV>(dy, h, gamma, mean, rstd, dres, dx, scratch, G, rows, N, rms, st)
     if (nvec <= 32 * 2) return PF_NORM_BWD_FUSED(2);
@@ -665,7 +665,7 @@ static int norm_bwd_launch(const void* dy, const void* h, const float* gamma, co
     return PF_NORM_BWD_FUSED(8);
 #undef PF_NORM_BWD_FUSED
   }
-  if (sizeof(T) == 2 && nvec <= 32 * 16) {
+  if constexpr (sizeof(T) == 2) if (nvec <= 32 * 16) {
     // input gradient: warp per row (rows of up to 4096 16-bit elements: Llama's hidden size);
     // parameter gradients: column reduction over row slabs
     const unsigned grid = (unsigned)((rows + 7) / 8);

@@ -628,7 +628,7 @@ def groupnorm_bwd(dy, x, mean, rstd, gamma, beta, groups: int, silu: bool):
     scratch = _groupnorm_scratch(L, B, H * W, C, C + groups, x.device)
     check(L.pf_groupnorm_bwd(ptr(dy), ptr(x), ptr(mean), ptr(rstd), ptr(gamma.float()),
                              ptr(beta.float()), ptr(dx), ptr(dgamma), ptr(dbeta), ptr(sums),
-                             ptr(scratch), B, H * W, C, groups, int(silu), 0, dt(x.dtype),
+                             ptr(scratch), B, H * W, C, groups, int(silu), dt(x.dtype),
                              sm_count(x.device), stream()), "pf_groupnorm_bwd")
     return dx, dgamma, dbeta
 
