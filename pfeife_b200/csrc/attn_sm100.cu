@@ -722,7 +722,7 @@ PF_API int pf_attn_fwd(const void* q, const void* k, const void* v, void* o, voi
   // length and are dealt by it: there only a call without a whole round is split.
   const int pairs = p.q_pairs * H * B, left_over = pairs % attn_sm_count();
   const int rounds = pairs / attn_sm_count();
-  const bool split = 2 * left_over <= attn_sm_count() && rounds <= (causal ? 0 : 4);
+  const bool split = 2 * left_over <= attn_sm_count() && rounds <= (causal ? 0 : 3);
   p.n_pair = split ? pairs - left_over : pairs;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   PF_ATTN_DISPATCH(launch_fwd_ws, tq, tk, tv, p, st);
