@@ -213,8 +213,10 @@ def _rows(x: Tensor) -> Tensor:
 # images, logits: 4.7 -> 2.9 ms; LayerNorm with residual, forward and backward: 246 -> 175 us.)
 # The implementation runs below autograd, as the dispatcher has it, so that what it returns is no
 # view to autograd and may be changed in place.
-_DIRECT_DEVICE = "cuda"
+_FIRST_DEVICE = 0            # the least device index of tensors that are called directly (CPU: -1)
 _below_autograd = torch._C._AutoDispatchBelowADInplaceOrView
+_Parameter = torch.nn.Parameter
+_PLAIN_VALUES = frozenset((type(None), bool, int, float, torch.dtype))
 
 
 def _custom_op(name: str):
@@ -252,23 +254,13 @@ def _autograd(op, n_out: int, backward, setup) -> None:
     op.direct, op.n_out, op.n_all = Direct, n_out, len(op._opoverload._schema.returns)
 
 
-_DispatchKey, _KeySet = torch._C.DispatchKey, torch._C.DispatchKeySet
-_VIEWS = _KeySet(_DispatchKey.ADInplaceOrView).raw_repr()      # absent in inference mode
-_NO_LAYER = _KeySet(_DispatchKey.BackendSelect).raw_repr() | _VIEWS
-_AUTOGRAD = _DispatchKey.AutogradOther                         # excluded inside other ops
-_layers, _excluded = (torch._C._dispatch_tls_local_include_set,
-                      torch._C._dispatch_tls_is_dispatch_key_excluded)
-_wrapped, _Parameter = torch._C._functorch.is_functorch_wrapped_tensor, torch.nn.Parameter
-_PLAIN_VALUES = frozenset((type(None), bool, int, float, torch.dtype))
-
-
 def _unobserved() -> bool:
-    """No compiler, tracer, dispatch or function mode, transform (of either vmap) or forward-mode level
-    is active: nothing but the kernels and autograd needs to see an op.  All but three of these put
-    a layer of their own on the dispatcher of this thread."""
-    return not (torch.compiler.is_compiling() or torch._C._len_torch_function_stack()
-                or forward_ad._current_level >= 0) and \
-        _layers().raw_repr() | _VIEWS == _NO_LAYER
+    """No compiler, tracer, dispatch or function mode, functorch transform or forward-mode level is
+    active: nothing but the kernels and autograd needs to see an op."""
+    return not (torch.compiler.is_compiling() or torch._C._len_torch_dispatch_stack()
+                or torch._C._len_torch_function_stack() or forward_ad._current_level >= 0
+                or torch._C._functorch.peek_interpreter_stack() is not None
+                or torch._C._get_tracing_state() is not None)
 
 
 def _bwd(ctx, op):
@@ -290,34 +282,39 @@ def _bwd(ctx, op):
 
 def _plain_call(args) -> int:
     """Non-zero for plain CUDA tensors of one device that nothing else observes and whose memory
-    holds their values: no view with a negative bit, no wrapper that outlived its transform.
-    Anything but tensors and plain values (the proxy of a symbolic trace) is for the dispatcher to
-    handle.  2 when one of them requires a gradient, else 1."""
+    holds their values: no view with a negative bit, no wrapper (``data_ptr`` raises or is null for a
+    tensor of the older vmap and for one that outlived its transform).  Anything but tensors and
+    plain values (the proxy of a symbolic trace) is for the dispatcher to handle.  2 when one of them
+    requires a gradient, else 1."""
     if not _unobserved():
         return 0
     device, found = None, 1
-    for a in args:
-        kind = type(a)
-        if kind is Tensor or kind is _Parameter:
-            if device is None:
-                device = a.device
-                if device.type != _DIRECT_DEVICE:
+    try:
+        for a in args:
+            kind = type(a)
+            if kind is Tensor or kind is _Parameter:
+                if device is None:
+                    device = a.get_device()
+                    if device < _FIRST_DEVICE:
+                        return 0
+                elif a.get_device() != device:
                     return 0
-            elif a.device != device:
+                if a.is_neg() or not a.data_ptr():
+                    return 0
+                if a.requires_grad:
+                    found = 2
+            elif kind not in _PLAIN_VALUES:
                 return 0
-            if a.is_neg() or _wrapped(a):
-                return 0
-            if a.requires_grad:
-                found = 2
-        elif kind not in _PLAIN_VALUES:
-            return 0
+    except RuntimeError:
+        return 0
     return found if device is not None else 0
 
 
 def _call(op, *args):
     """The first ``n_out`` outputs of `op`."""
     found = _plain_call(args)
-    if found == 2 and torch.is_grad_enabled() and not _excluded(_AUTOGRAD):
+    if found == 2 and torch.is_grad_enabled() and not \
+            torch._C._dispatch_tls_is_dispatch_key_excluded(torch._C.DispatchKey.AutogradOther):
         return op.direct.apply(*args)
     if found:
         with _below_autograd():

@@ -13,7 +13,7 @@ DEVICES = ["cpu", pytest.param("cuda", marks=pytest.mark.gpu)]
 
 @pytest.fixture(params=DEVICES)
 def device(request, monkeypatch):
-    monkeypatch.setattr(functional, "_DIRECT_DEVICE", request.param, raising=False)
+    monkeypatch.setattr(functional, "_FIRST_DEVICE", -1 if request.param == "cpu" else 0)
     return request.param
 
 
@@ -106,6 +106,17 @@ def test_lazily_negated_inputs(device, monkeypatch):
                                    retain_graph=True)
         (w,) = torch.autograd.grad(out, out.grad_fn.next_functions[0][0].variable, -v)
         _near(g, w, device)
+
+
+def test_wrappers_that_outlive_their_transform(device):
+    """A tensor kept from inside a transform has no memory of its own; the dispatcher unwraps it."""
+    dtype = torch.float32 if device == "cpu" else torch.bfloat16
+    x, kept = torch.randn(8, 64).to(device=device, dtype=dtype), []
+    torch.func.grad(lambda t: (kept.append(t), t.sum())[1])(x)
+    torch.func.functionalize(lambda t: (kept.append(t), t + 1)[1])(x)
+    for t in kept:
+        assert not functional._plain_call((t,))
+    assert torch.equal(ops.gelu(kept[0]), ops.gelu(x))
 
 
 @pytest.mark.parametrize("name", ["rope", "upsample", "linear", "mlp"])
