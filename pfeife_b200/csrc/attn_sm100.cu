@@ -231,44 +231,43 @@ struct FwdCfg {
 // joins at the end.  A split tile takes half the steps of a pair; it is always its CTA's last item.
 // Head dim 128, 2048 tokens: 8 heads (64 pairs) 45 us as pairs, 28 split; 20 heads (160 pairs) 89
 // and 72.  Head dim 64, [1, 2048, 8, 64]: 38 and 24 us.
-template <bool SPLIT>     // some items are split tiles
 struct FwdItem {
-  int q0, q1, h, b;      // first query row of the two sides
-  int n[2], keys;        // key tiles that each side sees; key tiles to load
-  bool split;
-  // key tile of step i of side t
-  __device__ __forceinline__ int key(int t, int i) const {
-    return SPLIT && split ? 2 * i + t : i;
-  }
+  int q0, h, b, n[2];    // first query row; key tiles seen by the two query tiles
 };
-template <bool SPLIT>
-__device__ __forceinline__ FwdItem<SPLIT> fwd_item(const AttnParams& p, int w) {
-  FwdItem<SPLIT> it;
-  it.split = SPLIT && w >= p.n_pair;
-  const int u = w - p.n_pair, pair = it.split ? p.n_pair + (u >> 1) : w;
+__device__ __forceinline__ FwdItem fwd_item(const AttnParams& p, int w) {
+  FwdItem it;
   int qp, bh;
   if (p.causal) {
     // later queries see more keys: the long items of every head are dealt first
-    qp = pair / (p.B * p.H);
-    bh = pair - qp * (p.B * p.H);
+    qp = w / (p.B * p.H);
+    bh = w - qp * (p.B * p.H);
     qp = p.q_pairs - 1 - qp;
   } else {
-    bh = pair / p.q_pairs;
-    qp = pair - bh * p.q_pairs;
+    bh = w / p.q_pairs;
+    qp = w - bh * p.q_pairs;
   }
-  it.q0 = qp * 2 * ATT_BM + (it.split && (u & 1) ? ATT_BM : 0);
-  it.q1 = it.split ? it.q0 : it.q0 + ATT_BM;
+  it.q0 = qp * 2 * ATT_BM;
   it.h = bh % p.H;
   it.b = bh / p.H;
-  auto tiles = [&](int q0) {
+#pragma unroll
+  for (int t = 0; t < 2; ++t) {
+    const int q0 = it.q0 + t * ATT_BM;
     int kv_end = p.Sk;
     if (p.causal) kv_end = min(p.Sk, q0 + ATT_BM + (p.Sk - p.Sq));
-    return (q0 < p.q_rows && kv_end > 0) ? (kv_end + ATT_BN - 1) / ATT_BN : 0;
-  };
-  const int n0 = tiles(it.q0), n1 = it.split ? 0 : tiles(it.q1);
-  it.keys = max(n0, n1);
-  it.n[0] = it.split ? (n0 + 1) / 2 : n0;
-  it.n[1] = it.split ? n0 / 2 : n1;
+    it.n[t] = (q0 < p.q_rows && kv_end > 0) ? (kv_end + ATT_BN - 1) / ATT_BN : 0;
+  }
+  return it;
+}
+// item `w` of a kernel whose items from n_pair on are split tiles (`split` says whether this one is)
+__device__ __forceinline__ FwdItem fwd_item(const AttnParams& p, int w, bool& split) {
+  split = w >= p.n_pair;
+  if (!split) return fwd_item(p, w);
+  const int u = w - p.n_pair, t = u & 1;
+  FwdItem it = fwd_item(p, p.n_pair + (u >> 1));
+  const int n = t ? it.n[1] : it.n[0];
+  it.q0 += t * ATT_BM;
+  it.n[0] = (n + 1) / 2;
+  it.n[1] = n / 2;
   return it;
 }
 // rounds run alternately forwards and backwards over the CTAs, so that a CTA with a long item in
@@ -317,7 +316,6 @@ __global__ void __launch_bounds__(FwdCfg<DP>::THREADS, 1)
 attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                    const __grid_constant__ CUtensorMap tv, const AttnParams p, const int n_items) {
   using C = FwdCfg<DP>;
-  using Item = FwdItem<SPLIT>;
   constexpr int NBLK = C::NBLK, TILE = C::TILE, ST = C::ST;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::OFF_BAR);
@@ -366,8 +364,10 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
         for (int r = 0; ok && r * (int)gridDim.x < n_items; ++r) {
           const int w = fwd_index(r);
           if (w >= n_items) continue;
-          const Item it = fwd_item<SPLIT>(p, w);
-          for (int j = 0; j < it.keys && ok; ++j, ++g) {
+          bool split = false;
+          const FwdItem it = SPLIT ? fwd_item(p, w, split) : fwd_item(p, w);
+          const int nmax = split ? it.n[0] + it.n[1] : max(it.n[0], it.n[1]);
+          for (int j = 0; j < nmax && ok; ++j, ++g) {
             const int st = g % ST;
             if (j == 0 && it.n[0] > 0) {
               ok = mbar_wait(&q_empty[0], (qc[0] & 1) ^ 1, p.status, PF_ERR_TIMEOUT_EMPTY);
@@ -381,7 +381,8 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
             if (j == 0 && it.n[1] > 0) {
               ok = mbar_wait(&q_empty[1], (qc[1] & 1) ^ 1, p.status, PF_ERR_TIMEOUT_EMPTY);
               if (!ok) break;
-              load_tile<NBLK>(smem + TILE, &tq, &q_full[1], it.h, it.q1, it.b);
+              load_tile<NBLK>(smem + TILE, &tq, &q_full[1], it.h,
+                              split ? it.q0 : it.q0 + ATT_BM, it.b);
               ++qc[1];
             }
             ok = mbar_wait(&v_empty[st], ((g / ST) & 1) ^ 1, p.status, PF_ERR_TIMEOUT_EMPTY);
@@ -399,19 +400,16 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
         const uint32_t id_o = make_idesc_f16(128, DP, p.fmt, 0, 1);
         uint32_t g = 0, qc[2] = {0, 0}, cnt[2] = {0, 0};    // cnt: S tiles issued per side
         bool ok = true;
-        // in a pair, tile 1 reads every key tile that tile 0 reads, and after it
-        auto last_reader = [](const Item& it, int t, int i) {
-          return (SPLIT && it.split) || t == 1 || i >= it.n[1];
-        };
-        // S of step i of side t.  Its columns must be free: the previous scores are in registers,
-        // or (P in the same columns) the previous P V has read its probabilities.
-        auto issue_s = [&](const Item& it, int t, int i) -> bool {
-          const int kt = it.key(t, i), st = (g + kt) % ST;
-          if (i == 0) {
+        // S of step j of side t: key tile kt (ring position gg).  Its columns must be free: the
+        // previous scores are in registers, or (P in the same columns) the previous P V has read
+        // its probabilities.
+        auto issue_s = [&](int t, uint32_t gg, int j, int kt, int n, bool last_of_tile) -> bool {
+          const int st = gg % ST;
+          if (j == 0) {
             if (!mbar_wait_warp(&q_full[t], qc[t] & 1, p.status, PF_ERR_TIMEOUT_FULL)) return false;
             ++qc[t];
           }
-          if (!mbar_wait_warp(&k_full[st], ((g + kt) / ST) & 1, p.status, PF_ERR_TIMEOUT_FULL))
+          if (!mbar_wait_warp(&k_full[st], (gg / ST) & 1, p.status, PF_ERR_TIMEOUT_FULL))
             return false;
           if (cnt[t] > 0 && !mbar_wait_warp(C::ALIAS_P ? &pv_done[t] : &s_empty[t],
                                             (cnt[t] - 1) & 1, p.status,
@@ -423,52 +421,66 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
           const uint32_t id = n_mma == ATT_BN ? id_s : make_idesc_f16(128, n_mma, p.fmt, 0, 0);
           mma_kk_on<DP / 16>(on, tmem + t * 128, smem_u32(smem + t * TILE),
                           smem_u32(smem + C::OFF_K + st * TILE), id);
-          if (last_reader(it, t, i)) tc_commit_on(on, &k_empty[st]);
+          if (last_of_tile) tc_commit_on(on, &k_empty[st]);
           tc_commit_on(on, &s_full[t]);
-          if (i == it.n[t] - 1) tc_commit_on(on, &q_empty[t]);
+          if (j == n - 1) tc_commit_on(on, &q_empty[t]);
           ++cnt[t];
           return true;
         };
         for (int r = 0; ok && r * (int)gridDim.x < n_items; ++r) {
           const int w = fwd_index(r);
           if (w >= n_items) continue;
-          const Item it = fwd_item<SPLIT>(p, w);
-          const int steps = max(it.n[0], it.n[1]);
+          bool split = false;
+          const FwdItem it = SPLIT ? fwd_item(p, w, split) : fwd_item(p, w);
+          const int nmax = max(it.n[0], it.n[1]);
+          // in a pair, tile 1 reads every key tile that tile 0 reads, and after it
+          auto last_reader = [&](int t, int j) {
+            return (SPLIT && split) || t == 1 || j >= it.n[1];
+          };
+          // key tile of step j of side t
+          auto key = [&](int t, int j) { return (SPLIT && split) ? 2 * j + t : j; };
 #pragma unroll
           for (int t = 0; t < 2; ++t)
-            if (ok && it.n[t] > 0) ok = issue_s(it, t, 0);
-          for (int i = 0; i < steps && ok; ++i) {
+            if (ok && it.n[t] > 0)
+              ok = issue_s(t, g + key(t, 0), 0, key(t, 0), it.n[t], last_reader(t, 0));
+          for (int j = 0; j < nmax && ok; ++j) {
             if (!C::ALIAS_P) {
 #pragma unroll
               for (int t = 0; t < 2; ++t)
-                if (ok && i + 1 < it.n[t]) ok = issue_s(it, t, i + 1);
+                if (ok && j + 1 < it.n[t])
+                  ok = issue_s(t, g + key(t, j + 1), j + 1, key(t, j + 1), it.n[t],
+                               last_reader(t, j + 1));
               if (!ok) break;
             }
-            if (!SPLIT)        // one V tile for both sides
-              ok = mbar_wait_warp(&v_full[(g + i) % ST], ((g + i) / ST) & 1, p.status,
+            if (!SPLIT) {        // one V tile for both sides
+              ok = mbar_wait_warp(&v_full[(g + j) % ST], ((g + j) / ST) & 1, p.status,
                                   PF_ERR_TIMEOUT_FULL);
+              if (!ok) break;
+            }
 #pragma unroll
             for (int t = 0; t < 2; ++t) {
-              if (!ok || i >= it.n[t]) continue;
-              const int kt = it.key(t, i), st = (g + kt) % ST;
-              // the probabilities waited for are those of the step before any S issued above
-              const uint32_t c = cnt[t] - 1 - ((!C::ALIAS_P && i + 1 < it.n[t]) ? 1u : 0u);
+              if (!ok || j >= it.n[t]) continue;
+              const uint32_t gg = g + key(t, j);
+              const int st = gg % ST;
               if (SPLIT)
-                ok = mbar_wait_warp(&v_full[st], ((g + kt) / ST) & 1, p.status,
-                                    PF_ERR_TIMEOUT_FULL);
+                ok = mbar_wait_warp(&v_full[st], (gg / ST) & 1, p.status, PF_ERR_TIMEOUT_FULL);
+              const int k_steps = (min(ATT_BN, p.Sk - key(t, j) * ATT_BN) + 15) / 16;
+              // the probabilities waited for are those of the step before any S issued above
+              const uint32_t c = cnt[t] - 1 - ((!C::ALIAS_P && j + 1 < it.n[t]) ? 1u : 0u);
               ok = ok && mbar_wait_warp(&p_full[t], c & 1, p.status, PF_ERR_TIMEOUT_FULL);
               if (!ok) continue;
               tc_fence_after();
-              const int k_steps = (min(ATT_BN, p.Sk - kt * ATT_BN) + 15) / 16;
               const uint32_t sV = smem_u32(smem + C::OFF_V + st * TILE);
               const uint32_t t_p = tmem + C::T_P + t * C::P_TILE;
-              mma_t_mn_on(on, tmem + C::T_O + t * DP, t_p, sV, id_o, i > 0, k_steps);
-              if (last_reader(it, t, i)) tc_commit_on(on, &v_empty[st]);
+              mma_t_mn_on(on, tmem + C::T_O + t * DP, t_p, sV, id_o, j > 0, k_steps);
+              if (last_reader(t, j)) tc_commit_on(on, &v_empty[st]);
               tc_commit_on(on, &pv_done[t]);
-              if (C::ALIAS_P && i + 1 < it.n[t]) ok = issue_s(it, t, i + 1);
+              if (C::ALIAS_P && j + 1 < it.n[t])
+                ok = issue_s(t, g + key(t, j + 1), j + 1, key(t, j + 1), it.n[t],
+                             last_reader(t, j + 1));
             }
           }
-          g += it.keys;
+          g += (SPLIT && split) ? it.n[0] + it.n[1] : nmax;
         }
       }
       __syncwarp();
@@ -489,13 +501,14 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
     for (int r = 0; ok && r * (int)gridDim.x < n_items; ++r) {
       const int w = fwd_index(r);
       if (w >= n_items) continue;
-      const Item it = fwd_item<SPLIT>(p, w);
-      const int q0 = t ? it.q1 : it.q0, n_tiles = t ? it.n[1] : it.n[0];
+      bool split = false;
+      const FwdItem it = SPLIT ? fwd_item(p, w, split) : fwd_item(p, w);
+      const int q0 = it.q0 + (split ? 0 : t * ATT_BM), n_tiles = t ? it.n[1] : it.n[0];
       const int qi = q0 + row;
-      if (q0 >= p.q_rows || (SPLIT && t && it.split && it.n[0] == 0)) continue;
+      if (q0 >= p.q_rows || (split && t && it.n[0] == 0)) continue;
       T* dst = reinterpret_cast<T*>(p.o) + (((long long)it.b * p.Sq + qi) * p.H + it.h) * p.D;
       float* lse_dst = p.lse + ((long long)it.b * p.H + it.h) * p.Sq + qi;
-      if (n_tiles == 0 && !(SPLIT && t && it.split)) {      // no key is visible to this query tile
+      if (n_tiles == 0 && !(split && t)) {      // no key is visible to this query tile
         if (qi < p.Sq) {
           for (int c = 0; c < p.D / 8; ++c)
             reinterpret_cast<uint4*>(dst)[c] = make_uint4(0, 0, 0, 0);
@@ -507,7 +520,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
       const bool warp_live = q0 + quad * 32 < p.Sq;
       float m_used = -INFINITY, l = 0.f;
       for (int j = 0; j < n_tiles && ok; ++j, ++cnt) {
-        const int k0 = it.key(t, j) * ATT_BN;
+        const int k0 = (split ? 2 * j + t : j) * ATT_BN;
         const int rem = min(ATT_BN, p.Sk - k0);
         const int n_chunks = ((rem + 15) / 16 * 16 + 31) / 32;
         // a tile needs masks when it is ragged or crosses the causal diagonal of this q tile
@@ -603,7 +616,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
         tc_fence_after();
       }
       float w0 = 1.f, w1 = 0.f;              // weights of the two sides' outputs
-      if (SPLIT && it.split) {
+      if (split) {
         if (t) {                             // the thread of this row on side 0 finishes it
           side1[row] = m_used;
           side1[ATT_BM + row] = l;
@@ -632,7 +645,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
           tmem_ld_wait_for(o);
 #pragma unroll
           for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * w0);
-          if (SPLIT && it.split && it.n[1] > 0) {     // the same row of the other side's columns
+          if (split && it.n[1] > 0) {     // the same row of the other side's columns
             uint32_t o1[32];
             tmem_ld32(t_o + DP + c * 32, o1);
             tmem_ld_wait_for(o1);
@@ -722,7 +735,10 @@ PF_API int pf_attn_fwd(const void* q, const void* k, const void* v, void* o, voi
   // length and are dealt by it: there only a call without a whole round is split.
   const int pairs = p.q_pairs * H * B, left_over = pairs % attn_sm_count();
   const int rounds = pairs / attn_sm_count();
-  const bool split = 2 * left_over <= attn_sm_count() && rounds <= (causal ? 0 : 3);
+  // One tile per head is no pair to begin with: its keys are shared out from the third key tile on
+  // ([1, 128, 4, 128] 7.2 us whole, 7.8 split).
+  const bool split = 2 * left_over <= attn_sm_count() && rounds <= (causal ? 0 : 3) &&
+                     (p.q_rows > ATT_BM || Sk > 2 * ATT_BN);
   p.n_pair = split ? pairs - left_over : pairs;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   PF_ATTN_DISPATCH(launch_fwd_ws, tq, tk, tv, p, st);

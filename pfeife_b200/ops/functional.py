@@ -215,6 +215,10 @@ def _rows(x: Tensor) -> Tensor:
 # view to autograd and may be changed in place.
 _FIRST_DEVICE = 0            # the least device index of tensors that are called directly (CPU: -1)
 _below_autograd = torch._C._AutoDispatchBelowADInplaceOrView
+_is_compiling, _tracing = torch.compiler.is_compiling, torch._C._get_tracing_state
+_dispatch_modes = torch._C._len_torch_dispatch_stack
+_function_modes = torch._C._len_torch_function_stack
+_interpreters = torch._C._functorch.peek_interpreter_stack
 _Parameter = torch.nn.Parameter
 _PLAIN_VALUES = frozenset((type(None), bool, int, float, torch.dtype))
 
@@ -257,10 +261,9 @@ def _autograd(op, n_out: int, backward, setup) -> None:
 def _unobserved() -> bool:
     """No compiler, tracer, dispatch or function mode, functorch transform or forward-mode level is
     active: nothing but the kernels and autograd needs to see an op."""
-    return not (torch.compiler.is_compiling() or torch._C._len_torch_dispatch_stack()
-                or torch._C._len_torch_function_stack() or forward_ad._current_level >= 0
-                or torch._C._functorch.peek_interpreter_stack() is not None
-                or torch._C._get_tracing_state() is not None)
+    return not (_is_compiling() or _dispatch_modes() or _function_modes()
+                or forward_ad._current_level >= 0 or _interpreters() is not None
+                or _tracing() is not None)
 
 
 def _bwd(ctx, op):
