@@ -14,7 +14,7 @@
 //   warps 0-7    softmax side: thread <-> key row (TMEM lane), each warp half of the 128 queries
 //   warps 8-11   drain: dQ tiles out of TMEM into the fp32 sums (TMA reduce-add through swizzled
 //                boxes), and dK / dV at the end of an item while the next item is under way
-//   warp 12      TMA producer      warp 13  MMA issuer (one lane), TMEM owner (14, 15: idle)
+//   warp 12      TMA producer      warp 13  MMA issuer, TMEM owner (14, 15: idle)
 // What bounds it: per 128 x 128 tile pair 16384 exponentials (1024 cycles of the special-function
 // units) against 5 products (1400 cycles at head dim 64, 2560 at 128), so the tensor core must
 // never wait for the element-wise part.  Order of the MMA warp for tile i:
@@ -27,7 +27,8 @@
 //
 // Measured (B200, CUDA events, L2 flushed, with the pre- and post-pass), against one CTA per key
 // tile that ran the five products and the element-wise part one after the other with scalar
-// reductions into dQ: [4, 4096, 10, 64] 1330 -> 877 us, [2, 2048, 16, 128] 445 -> 261,
+// reductions into dQ: [4, 4096, 10, 64] 1330 -> 877 us (670 since one elected thread issues the
+// products: before, issuing the 28 of a tile pair took 4000 cycles), [2, 2048, 16, 128] 445 -> 261,
 // causal [1, 2048, 32, 128] 302 -> 155, [24, 257, 16, 88] 192 -> 146.
 //
 // A pre-pass writes per query tile the row statistics [128 lse2 | 128 delta scale] (+inf / 0 beyond
@@ -226,7 +227,7 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = tmem_base_of(tmem_slot);
   const int shift = p.Sk - p.Sq;
 
   // one split per warpgroup: its four warps execute the same instruction
@@ -234,7 +235,7 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
     regs_dec<C::REGS_OTHER>();
     if (warp == 12) {
       // ---------------------------------------------------------------- TMA producer
-      if (lane == 0) {
+      if (elect_one()) {
         uint32_t g = 0, items = 0;
         bool ok = true;
         for (int r = 0; ok && r * (int)gridDim.x < n_items; ++r) {
@@ -278,7 +279,7 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
       __syncwarp();
     } else if (warp == 13) {
       // ---------------------------------------------------------------- MMA issuer
-      if (lane == 0) {
+      if (elect_one()) {
         const uint32_t sK = smem_u32(smem), sV = smem_u32(smem + C::OFF_V);
         const uint32_t sQ = smem_u32(smem + C::OFF_Q), sdO = smem_u32(smem + C::OFF_DO);
         const uint32_t sdS = smem_u32(smem + C::OFF_DS);
@@ -298,7 +299,7 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
             return false;
           tc_fence_after();
           mma_kk<DP / 16>(tmem + C::T_S, sK, sQ + st * TILE,
-                          make_idesc_f16(128, cols_of(qt), p.fmt, 0, 0), false);
+                          make_idesc_f16(128, cols_of(qt), p.fmt, 0, 0));
           tc_commit(s_full);
           return true;
         };
@@ -313,7 +314,7 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
             return false;
           tc_fence_after();
           mma_kk<DP / 16>(tmem + C::T_DP, sV, sdO + st * TILE,
-                          make_idesc_f16(128, cols_of(qt), p.fmt, 0, 0), false);
+                          make_idesc_f16(128, cols_of(qt), p.fmt, 0, 0));
           tc_commit(dp_full);
           return true;
         };
@@ -336,11 +337,7 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
               ok = mbar_wait(acc_empty, (items & 1) ^ 1, p.status, PF_ERR_TIMEOUT_TMEM_EMPTY);
             if (!ok) break;
             tc_fence_after();
-#pragma unroll 1
-            for (int k = 0; k < q_steps; ++k)
-              tc_mma_f16_ts(tmem + C::T_DV, tmem + C::T_P + (k >> 2) * C::P_HALF + (k & 3) * 8,
-                            make_desc_sw128(sdO + dst * TILE + k * 2048, ATT_BLK, 1024), id_kd,
-                            i > 0 || k > 0);
+            mma_t_mn(tmem + C::T_DV, tmem + C::T_P, C::P_HALF, sdO + dst * TILE, id_kd, i > 0, q_steps);
             tc_commit(&do_empty[dst]);
             tc_commit(dv_done);
             ok = mbar_wait(ds_ready, g & 1, p.status, PF_ERR_TIMEOUT_FULL);
@@ -353,7 +350,7 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
             };
             auto issue_dq = [&]() {
               tc_fence_after();
-              mma_mn_mn(tmem + C::T_DQ, ds_tile, sK, id_dq, false, k_steps);
+              mma_mn_mn(tmem + C::T_DQ, ds_tile, sK, id_dq, k_steps);
               tc_commit(dq_full);
             };
             if (C::ALIAS_DQ) {

@@ -67,35 +67,46 @@ __device__ __forceinline__ void load_tile(uint8_t* dst, const CUtensorMap* map, 
   for (int i = 0; i < NBLK; ++i) tma_load_4d(dst + i * ATT_BLK, map, bar, i * 64, h, s0, b);
 }
 
+// Products over [128 rows x 64] blocks in shared memory, by the issuing thread.  Unrolled, so that a
+// step costs an addition per operand.
 // A[128 x K] (K-major blocks) . B[N x K]^T (K-major blocks), K = KSTEPS * 16
 template <int KSTEPS>
-__device__ __forceinline__ void mma_kk(uint32_t d_tmem, uint32_t sa, uint32_t sb, uint32_t idesc,
-                                       bool accumulate_first) {
+__device__ __forceinline__ void mma_kk(uint32_t d_tmem, uint32_t sa, uint32_t sb, uint32_t idesc) {
+  const uint32_t a = desc_lo(sa, 16), b = desc_lo(sb, 16);
 #pragma unroll
   for (int k = 0; k < KSTEPS; ++k) {
-    const uint32_t off = (k >> 2) * ATT_BLK + (k & 3) * 32;
-    tc_mma_f16(d_tmem, make_desc_sw128(sa + off, 16, 1024), make_desc_sw128(sb + off, 16, 1024),
-               idesc, (k > 0) || accumulate_first);
+    const uint32_t off = ((k >> 2) * ATT_BLK + (k & 3) * 32) >> 4;
+    tc_mma_f16(d_tmem, a + off, b + off, idesc, k > 0);
   }
 }
 // A[128 x 128] K-major . B given as [K=128 rows][N] (N contiguous, MN-major blocks of 64)
 __device__ __forceinline__ void mma_k_mn(uint32_t d_tmem, uint32_t sa, uint32_t sb, uint32_t idesc,
-                                         bool accumulate_first, int ksteps = 8) {
-#pragma unroll 1
-  for (int k = 0; k < ksteps; ++k) {
-    const uint32_t aoff = (k >> 2) * ATT_BLK + (k & 3) * 32;
-    tc_mma_f16(d_tmem, make_desc_sw128(sa + aoff, 16, 1024),
-               make_desc_sw128(sb + k * 2048, ATT_BLK, 1024), idesc, (k > 0) || accumulate_first);
-  }
+                                         bool accumulate_first, int ksteps) {
+  const uint32_t a = desc_lo(sa, 16), b = desc_lo(sb, ATT_BLK);
+#pragma unroll
+  for (int k = 0; k < 8; ++k)
+    if (k < ksteps)
+      tc_mma_f16(d_tmem, a + (((k >> 2) * ATT_BLK + (k & 3) * 32) >> 4), b + (k * 2048 >> 4), idesc,
+                 (k > 0) || accumulate_first);
 }
 // A given as [K=128 rows][M=128] (M contiguous) . B given as [K=128 rows][N] (N contiguous)
 __device__ __forceinline__ void mma_mn_mn(uint32_t d_tmem, uint32_t sa, uint32_t sb, uint32_t idesc,
-                                          bool accumulate_first, int ksteps = 8) {
-#pragma unroll 1
-  for (int k = 0; k < ksteps; ++k) {
-    tc_mma_f16(d_tmem, make_desc_sw128(sa + k * 2048, ATT_BLK, 1024),
-               make_desc_sw128(sb + k * 2048, ATT_BLK, 1024), idesc, (k > 0) || accumulate_first);
-  }
+                                          int ksteps) {
+  const uint32_t a = desc_lo(sa, ATT_BLK), b = desc_lo(sb, ATT_BLK);
+#pragma unroll
+  for (int k = 0; k < 8; ++k)
+    if (k < ksteps) tc_mma_f16(d_tmem, a + (k * 2048 >> 4), b + (k * 2048 >> 4), idesc, k > 0);
+}
+// A in TMEM (16-bit pairs, 8 columns per step; its second half `half_cols` columns after the first),
+// B given as [K=128 rows][N] (N contiguous)
+__device__ __forceinline__ void mma_t_mn(uint32_t d_tmem, uint32_t ta, uint32_t half_cols, uint32_t sb,
+                                         uint32_t idesc, bool accumulate_first, int ksteps) {
+  const uint32_t b = desc_lo(sb, ATT_BLK);
+#pragma unroll
+  for (int k = 0; k < 8; ++k)
+    if (k < ksteps)
+      tc_mma_f16_ts(d_tmem, ta + (k >> 2) * half_cols + (k & 3) * 8, b + (k * 2048 >> 4), idesc,
+                    (k > 0) || accumulate_first);
 }
 
 // ------------------------------------------------------------------------------- host side

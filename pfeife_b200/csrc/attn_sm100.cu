@@ -24,7 +24,7 @@
 // 8 x head dim cycles of tensor core (512 at head dim 64; at 128 both take 1024).  Two tiles in
 // flight keep one tile's products under the other's exponentials.
 // Measured (B200, CUDA events, L2 flushed), against one query tile per CTA with P in shared
-// memory: [4, 4096, 10, 64] 402 -> 346 us, causal [1, 2048, 32, 128] 87 -> 59,
+// memory: [4, 4096, 10, 64] 402 -> 346 us (310 since one elected thread issues the products), causal [1, 2048, 32, 128] 87 -> 59,
 // [2, 2048, 16, 128] 114 -> 96, causal [6, 1782, 21, 32] 200 -> 117, 77 keys [4, 1024, 20, 64]
 // 32 -> 22, [24, 257, 16, 88] 62 -> 58.
 // TMEM (512 columns): S_0, S_1 128 each, O_0, O_1 one head dim each.  Up to head dim 64 P_0, P_1
@@ -178,31 +178,6 @@ attn_fwd_tail_kernel(const AttnParams p) {
   attn_fwd_tail_row<T>(p, tail_smem, p.q_rows + (int)blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
-// Products over [128 rows x 64] blocks in shared memory, issued by a converged warp (`on`: its
-// issuing lane).  Fully unrolled, so that a step costs an addition per operand.
-// A[128 x K] (K-major blocks) . B[N x K]^T (K-major blocks), K = KSTEPS * 16
-template <int KSTEPS>
-__device__ __forceinline__ void mma_kk_on(uint32_t on, uint32_t d_tmem, uint32_t sa, uint32_t sb,
-                                          uint32_t idesc) {
-  const uint32_t a = desc_lo(sa, 16), b = desc_lo(sb, 16);
-#pragma unroll
-  for (int k = 0; k < KSTEPS; ++k) {
-    const uint32_t off = ((k >> 2) * ATT_BLK + (k & 3) * 32) >> 4;
-    tc_mma_f16_on(on, d_tmem, a + off, b + off, idesc, k > 0);
-  }
-}
-// A in TMEM (16-bit pairs, 8 columns per step), B given as [K=128 rows][N] (N contiguous)
-__device__ __forceinline__ void mma_t_mn_on(uint32_t on, uint32_t d_tmem, uint32_t ta, uint32_t sb,
-                                            uint32_t idesc, bool accumulate_first, int ksteps) {
-  const uint32_t b = desc_lo(sb, ATT_BLK);
-#pragma unroll
-  for (int k = 0; k < 8; ++k)
-    if (k < ksteps)
-      tc_mma_f16_ts_on(on, d_tmem, ta + k * 8, b + (k * 2048 >> 4), idesc,
-                       k > 0 || accumulate_first);
-}
-
-
 template <int DP>
 struct FwdCfg {
   static constexpr int NBLK = (DP + 63) / 64;
@@ -351,14 +326,14 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = tmem_base_of(tmem_slot);
 
   // one split per warpgroup: its four warps execute the same instruction
   if (warp >= 8) {
     regs_dec<C::REGS_OTHER>();
     if (warp == 8) {
       // ---------------------------------------------------------------- TMA producer
-      if (lane == 0) {
+      if (elect_one()) {
         uint32_t g = 0, qc[2] = {0, 0};
         bool ok = true;
         for (int r = 0; ok && r * (int)gridDim.x < n_items; ++r) {
@@ -394,8 +369,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
       __syncwarp();
     } else if (warp == 9) {
       // ---------------------------------------------------------------- MMA issuer
-      {
-        const uint32_t on = lane == 0;
+      if (elect_one()) {
         const uint32_t id_s = make_idesc_f16(128, 128, p.fmt, 0, 0);
         const uint32_t id_o = make_idesc_f16(128, DP, p.fmt, 0, 1);
         uint32_t g = 0, qc[2] = {0, 0}, cnt[2] = {0, 0};    // cnt: S tiles issued per side
@@ -406,12 +380,12 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
         auto issue_s = [&](int t, uint32_t gg, int j, int kt, int n, bool last_of_tile) -> bool {
           const int st = gg % ST;
           if (j == 0) {
-            if (!mbar_wait_warp(&q_full[t], qc[t] & 1, p.status, PF_ERR_TIMEOUT_FULL)) return false;
+            if (!mbar_wait(&q_full[t], qc[t] & 1, p.status, PF_ERR_TIMEOUT_FULL)) return false;
             ++qc[t];
           }
-          if (!mbar_wait_warp(&k_full[st], (gg / ST) & 1, p.status, PF_ERR_TIMEOUT_FULL))
+          if (!mbar_wait(&k_full[st], (gg / ST) & 1, p.status, PF_ERR_TIMEOUT_FULL))
             return false;
-          if (cnt[t] > 0 && !mbar_wait_warp(C::ALIAS_P ? &pv_done[t] : &s_empty[t],
+          if (cnt[t] > 0 && !mbar_wait(C::ALIAS_P ? &pv_done[t] : &s_empty[t],
                                             (cnt[t] - 1) & 1, p.status,
                                             PF_ERR_TIMEOUT_TMEM_EMPTY))
             return false;
@@ -419,11 +393,11 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
           const int rem = min(ATT_BN, p.Sk - kt * ATT_BN);
           const int n_mma = (rem + 15) / 16 * 16;
           const uint32_t id = n_mma == ATT_BN ? id_s : make_idesc_f16(128, n_mma, p.fmt, 0, 0);
-          mma_kk_on<DP / 16>(on, tmem + t * 128, smem_u32(smem + t * TILE),
-                          smem_u32(smem + C::OFF_K + st * TILE), id);
-          if (last_of_tile) tc_commit_on(on, &k_empty[st]);
-          tc_commit_on(on, &s_full[t]);
-          if (j == n - 1) tc_commit_on(on, &q_empty[t]);
+          mma_kk<DP / 16>(tmem + t * 128, smem_u32(smem + t * TILE),
+                       smem_u32(smem + C::OFF_K + st * TILE), id);
+          if (last_of_tile) tc_commit(&k_empty[st]);
+          tc_commit(&s_full[t]);
+          if (j == n - 1) tc_commit(&q_empty[t]);
           ++cnt[t];
           return true;
         };
@@ -453,7 +427,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
               if (!ok) break;
             }
             if (!SPLIT) {        // one V tile for both sides
-              ok = mbar_wait_warp(&v_full[(g + j) % ST], ((g + j) / ST) & 1, p.status,
+              ok = mbar_wait(&v_full[(g + j) % ST], ((g + j) / ST) & 1, p.status,
                                   PF_ERR_TIMEOUT_FULL);
               if (!ok) break;
             }
@@ -463,18 +437,18 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
               const uint32_t gg = g + key(t, j);
               const int st = gg % ST;
               if (SPLIT)
-                ok = mbar_wait_warp(&v_full[st], (gg / ST) & 1, p.status, PF_ERR_TIMEOUT_FULL);
+                ok = mbar_wait(&v_full[st], (gg / ST) & 1, p.status, PF_ERR_TIMEOUT_FULL);
               const int k_steps = (min(ATT_BN, p.Sk - key(t, j) * ATT_BN) + 15) / 16;
               // the probabilities waited for are those of the step before any S issued above
               const uint32_t c = cnt[t] - 1 - ((!C::ALIAS_P && j + 1 < it.n[t]) ? 1u : 0u);
-              ok = ok && mbar_wait_warp(&p_full[t], c & 1, p.status, PF_ERR_TIMEOUT_FULL);
+              ok = ok && mbar_wait(&p_full[t], c & 1, p.status, PF_ERR_TIMEOUT_FULL);
               if (!ok) continue;
               tc_fence_after();
               const uint32_t sV = smem_u32(smem + C::OFF_V + st * TILE);
               const uint32_t t_p = tmem + C::T_P + t * C::P_TILE;
-              mma_t_mn_on(on, tmem + C::T_O + t * DP, t_p, sV, id_o, j > 0, k_steps);
-              if (last_reader(t, j)) tc_commit_on(on, &v_empty[st]);
-              tc_commit_on(on, &pv_done[t]);
+              mma_t_mn(tmem + C::T_O + t * DP, t_p, 32, sV, id_o, j > 0, k_steps);
+              if (last_reader(t, j)) tc_commit(&v_empty[st]);
+              tc_commit(&pv_done[t]);
               if (C::ALIAS_P && j + 1 < it.n[t])
                 ok = issue_s(t, g + key(t, j + 1), j + 1, key(t, j + 1), it.n[t],
                              last_reader(t, j + 1));

@@ -222,6 +222,10 @@ __device__ __forceinline__ void tmem_alloc(uint32_t* smem_slot, uint32_t ncols) 
                "r"(ncols)
                : "memory");
 }
+// the allocated base address, known to be the same for all lanes (every lane of the warp calls)
+__device__ __forceinline__ uint32_t tmem_base_of(const uint32_t* smem_slot) {
+  return __shfl_sync(0xffffffffu, *reinterpret_cast<const volatile uint32_t*>(smem_slot), 0);
+}
 __device__ __forceinline__ void tmem_relinquish() {
   asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 }
@@ -339,91 +343,62 @@ __device__ __forceinline__ void tc_commit_pair(uint64_t* bar, uint16_t cta_mask)
       "h"(cta_mask)
       : "memory");
 }
-// D (256 rows over the two CTAs' TMEM) (+)= A (128 rows per CTA) * B (N/2 rows per CTA)
-__device__ __forceinline__ void tc_mma_f16_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b,
-                                                uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
-      :
-      : "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-// D[tmem] (+)= A[smem] * B[smem], 16-bit inputs, fp32 accumulate.  One thread issues.
-__device__ __forceinline__ void tc_mma_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b,
-                                           uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
-      :
-      : "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// A operand from TMEM (used by attention: P stays on chip)
-__device__ __forceinline__ void tc_mma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b,
-                                              uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n"
-      :
-      : "r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-// Issue from a converged warp: every lane executes these with warp-uniform operands and the one
-// whose `on` is non-zero performs them.  Descriptors come as the low word that varies (start
-// address and LBO) and a constant high word (128-byte swizzle, SBO 1024), so that a step to the next
-// slice of an operand is one 32-bit addition.  (The attention forward on [4, 4096, 10, 64] took
-// 382 us when one divergent lane issued with 64-bit descriptors built per instruction, 349 us this
-// way.)
+// D[tmem] (+)= A * B, 16-bit inputs, fp32 accumulate.  One thread issues, chosen by elect_one() for
+// the whole of its role, with operands that are the same for all lanes of its warp: the compiler then
+// keeps them in uniform registers, where the instruction reads them.  Descriptors come as the low word
+// that varies (start address and LBO) and a constant high word (128-byte swizzle, SBO 1024), so that a
+// step to the next slice of an operand is one 32-bit addition.
+// Cycles from one product to the next, M = 128, K = 16 (B200, 1 CTA, eight other warps busy), by the
+// form of the issue: a lane chosen by `lane == 0` in a loop that builds 64-bit descriptors 109-124
+// whatever N; a converged warp in which a predicate picks the lane 61-70; elected, unrolled: 32 at
+// N = 64 with A in TMEM (what the arithmetic takes), 50 at N = 64 with A in shared memory (48 to
+// fetch the operands), 66 at N = 128 (64).
+// Shared-memory matrix descriptor for tcgen05.mma (version 1 = Blackwell), 128-byte swizzle.
+//   K-major operand : rows of 128 B (64 x 16-bit along K); 8 rows = one 1024 B swizzle atom;
+//                     SBO = distance between 8-row groups; LBO unused (1).
+//   MN-major operand: rows of 128 B (64 x 16-bit along M/N), one row per K index; 8 K-rows =
+//                     one atom; SBO = distance between 8-K-row groups, LBO = distance between
+//                     64-element blocks along M/N.
 constexpr uint32_t TC_DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29);
 __device__ __forceinline__ uint32_t desc_lo(uint32_t smem_addr, uint32_t lbo_bytes) {
   return ((smem_addr & 0x3FFFF) >> 4) | ((lbo_bytes >> 4) << 16);
 }
-__device__ __forceinline__ void tc_mma_f16_on(uint32_t on, uint32_t tmem_d, uint32_t a_lo,
-                                              uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void tc_mma_f16(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo,
+                                           uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p, e;\n\t.reg .b64 da, db;\n\t"
-      "setp.ne.b32 e, %0, 0;\n\t"
-      "setp.ne.b32 p, %5, 0;\n\t"
-      "mov.b64 da, {%2, %6};\n\t"
-      "mov.b64 db, {%3, %6};\n\t"
-      "@e tcgen05.mma.cta_group::1.kind::f16 [%1], da, db, %4, p;\n\t}\n"
+      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "mov.b64 da, {%1, %5};\n\t"
+      "mov.b64 db, {%2, %5};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n\t}\n"
       :
-      : "r"(on), "r"(tmem_d), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(TC_DESC_HI)
+      : "r"(tmem_d), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(TC_DESC_HI)
       : "memory");
 }
 // A operand from TMEM (attention: P stays on chip)
-__device__ __forceinline__ void tc_mma_f16_ts_on(uint32_t on, uint32_t tmem_d, uint32_t tmem_a,
-                                                 uint32_t b_lo, uint32_t idesc,
-                                                 uint32_t accumulate) {
+__device__ __forceinline__ void tc_mma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo,
+                                              uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p, e;\n\t.reg .b64 db;\n\t"
-      "setp.ne.b32 e, %0, 0;\n\t"
-      "setp.ne.b32 p, %5, 0;\n\t"
-      "mov.b64 db, {%3, %6};\n\t"
-      "@e tcgen05.mma.cta_group::1.kind::f16 [%1], [%2], db, %4, p;\n\t}\n"
+      "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "mov.b64 db, {%2, %5};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n\t}\n"
       :
-      : "r"(on), "r"(tmem_d), "r"(tmem_a), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(TC_DESC_HI)
+      : "r"(tmem_d), "r"(tmem_a), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(TC_DESC_HI)
       : "memory");
 }
-__device__ __forceinline__ void tc_commit_on(uint32_t on, uint64_t* bar) {
+// D (256 rows over the two CTAs' TMEM) (+)= A (128 rows per CTA) * B (N/2 rows per CTA)
+__device__ __forceinline__ void tc_mma_f16_pair(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo,
+                                                uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred e;\n\t"
-      "setp.ne.b32 e, %0, 0;\n\t"
-      "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%1];\n\t}\n"
+      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "mov.b64 da, {%1, %5};\n\t"
+      "mov.b64 db, {%2, %5};\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %3, p;\n\t}\n"
       :
-      : "r"(on), "r"(smem_u32(bar))
+      : "r"(tmem_d), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(TC_DESC_HI)
       : "memory");
-}
-// bounded wait of a whole warp, with one answer for all lanes
-__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int* status,
-                                               int code) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, status, code));
 }
 
 // 32 lanes x 32 columns of fp32: thread i of the warp receives 32 consecutive columns of TMEM
@@ -489,23 +464,6 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
 }
 __device__ __forceinline__ void tmem_st_wait() {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-}
-
-// Shared-memory matrix descriptor for tcgen05.mma (version 1 = Blackwell), 128-byte swizzle.
-//   K-major operand : rows of 128 B (64 x 16-bit along K); 8 rows = one 1024 B swizzle atom;
-//                     SBO = distance between 8-row groups; LBO unused (1).
-//   MN-major operand: rows of 128 B (64 x 16-bit along M/N), one row per K index; 8 K-rows =
-//                     one atom; SBO = distance between 8-K-row groups, LBO = distance between
-//                     64-element blocks along M/N.
-__device__ __forceinline__ uint64_t make_desc_sw128(uint32_t smem_addr, uint32_t lbo_bytes,
-                                                    uint32_t sbo_bytes) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((smem_addr & 0x3FFFF) >> 4);
-  d |= static_cast<uint64_t>((lbo_bytes >> 4) & 0x3FFF) << 16;
-  d |= static_cast<uint64_t>((sbo_bytes >> 4) & 0x3FFF) << 32;
-  d |= 1ull << 46;  // descriptor version
-  d |= 2ull << 61;  // SWIZZLE_128B
-  return d;
 }
 
 // Instruction descriptor, kind::f16, fp32 accumulate.  fmt: 0 = fp16, 1 = bf16.

@@ -12,9 +12,10 @@
 // pre-activation to `aux`), multiply by gelu'(aux) (dGELU), + residual[m,n], accumulate into C
 // (fp32 gradient buckets), cast to the output dtype.
 //
-// Role layout of the 320-thread CTA: warp 0 = TMA producer (one lane), warp 1 = TMEM owner and
-// MMA issuer (one lane), warps 2..9 = epilogue (one accumulator row per thread; two warps share a
-// TMEM lane quadrant and split the tile's columns, which halves the epilogue latency per tile);
+// Role layout of the 320-thread CTA: warp 0 = TMA producer, warp 1 = TMEM owner and MMA
+// issuer (one elected thread each), warps 2..9 = epilogue (one accumulator row per thread; two warps
+// share a TMEM lane quadrant and split the tile's columns, which halves the epilogue latency per
+// tile);
 // the instantiation that fuses an all-gather of B adds two warps that copy the remote rows.
 #include <cstring>
 #include "common.cuh"
@@ -237,11 +238,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
   __syncthreads();
   if (PAIR) cluster_sync();   // the peer's barriers exist before anything is sent to them
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = tmem_base_of(tmem_slot);
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -357,11 +358,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && cta_rank == 0) {
+    if (cta_rank == 0 && elect_one()) {
       const uint32_t idesc = make_idesc_f16(BMT, BNT, p.fmt, p.a_mn, p.b_mn);
-      // per-UMMA_K advance of the descriptor start address and its LBO/SBO
-      const uint32_t a_adv = p.a_mn ? 2048u : 32u;
-      const uint32_t b_adv = p.b_mn ? 2048u : 32u;
+      // per-UMMA_K advance of the descriptor start address (in its units of 16 bytes) and its LBO
+      const uint32_t a_adv = (p.a_mn ? 2048u : 32u) >> 4;
+      const uint32_t b_adv = (p.b_mn ? 2048u : 32u) >> 4;
       const uint32_t a_lbo = p.a_mn ? 8192u : 16u;
       const uint32_t b_lbo = p.b_mn ? 8192u : 16u;
       int stage = 0;
@@ -388,14 +389,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
           if (!ok) break;
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + stage * S::STAGE_BYTES);
-          const uint32_t sb = sa + S::A_BYTES;
+          const uint32_t a_lo = desc_lo(sa, a_lbo), b_lo = desc_lo(sa + S::A_BYTES, b_lbo);
 #pragma unroll
           for (int k = 0; k < GEMM_BK / GEMM_UMMA_K; ++k) {
-            const uint64_t da = make_desc_sw128(sa + k * a_adv, a_lbo, 1024);
-            const uint64_t db = make_desc_sw128(sb + k * b_adv, b_lbo, 1024);
             const uint32_t acc_on = (kb != kb_begin) || (k != 0);
-            if (PAIR) tc_mma_f16_pair(d_tmem, da, db, idesc_t, acc_on);
-            else tc_mma_f16(d_tmem, da, db, idesc_t, acc_on);
+            if (PAIR) tc_mma_f16_pair(d_tmem, a_lo + k * a_adv, b_lo + k * b_adv, idesc_t, acc_on);
+            else tc_mma_f16(d_tmem, a_lo + k * a_adv, b_lo + k * b_adv, idesc_t, acc_on);
           }
           // smem slot reusable (in both CTAs of a pair) once these MMAs retire
           if (PAIR) tc_commit_pair(&empty_bar[stage], 3);
