@@ -20,20 +20,23 @@
 // never wait for the element-wise part.  Order of the MMA warp for tile i:
 //   head dim <= 64   S(i+1) as soon as S(i) is in registers, dV(i), dP(i+1), dK(i), dQ(i)
 //   96               S(i+1) as soon as S(i) is in registers, dV(i), dQ(i), dK(i), dP(i+1)
-//   128              dV(i), dQ(i), S(i+1), dK(i), dP(i+1)
+//   128              dV(i), S(i+1) once dV(i) has read P^T, dQ(i), dK(i), dP(i+1)
 // TMEM (512 columns): S^T 128, dP^T 128, P^T 64 (16-bit), dV, dK, dQ one head dim each.  At 96 dQ
 // takes the columns of dP^T (dead once dS^T is in shared memory; the next dP^T waits until dQ is
 // drained), at 128 P^T also takes the columns of S^T.
 //
 // Measured (B200, CUDA events, L2 flushed, with the pre- and post-pass), against one CTA per key
 // tile that ran the five products and the element-wise part one after the other with scalar
-// reductions into dQ: [4, 4096, 10, 64] 1330 -> 877 us (670 since one elected thread issues the
-// products: before, issuing the 28 of a tile pair took 4000 cycles), [2, 2048, 16, 128] 445 -> 261,
-// causal [1, 2048, 32, 128] 302 -> 155, [24, 257, 16, 88] 192 -> 146.
+// reductions into dQ: [4, 4096, 10, 64] 1330 -> 590 us, [2, 2048, 16, 128] 445 -> 222,
+// causal [1, 2048, 32, 128] 302 -> 138, [24, 257, 16, 88] 192 -> 142.  Steps on the way at
+// [4, 4096, 10, 64]: 877; 690 with one elected thread issuing the products (before, issuing the 28 of
+// a tile pair took 4000 cycles); 590 with tile paths free of masks, barriers looked at together, the
+// next 32 columns on their way while the last are worked on, and negated statistics.  At head dim
+// 128: 261; 222 with S(i+1) issued under the dS^T of tile i and dQ leaving TMEM ahead of its boxes.
 //
-// A pre-pass writes per query tile the row statistics [128 lse2 | 128 delta scale] (+inf / 0 beyond
-// the last query, which makes the probabilities there zero without a test) and clears the fp32 dQ
-// sums; a post-pass converts them.  With one key tile the dQ tiles are complete and go straight to
+// A pre-pass writes per query tile the row statistics [128 x -lse2 | 128 x -delta scale] (-inf / 0
+// beyond the last query, which makes the probabilities there zero without a test) and clears the fp32
+// dQ sums; a post-pass converts them.  With one key tile the dQ tiles are complete and go straight to
 // their 16-bit destination: no sums, no post-pass.
 #include "attn_common.cuh"
 #include "api.h"
@@ -45,7 +48,7 @@ struct AttnBwdParams {
   int causal;
   float scale;
   int fmt;              // 0 fp16, 1 bf16
-  const float* stats;   // [B*H][query tiles][256]: lse * log2(e), then delta * scale
+  const float* stats;   // [B*H][query tiles][256]: -lse * log2(e), then -delta * scale
   void *dq, *dk, *dv;   // strides (batch, seq, head) in elements
   long long sdq[3], sdkv[3];
   int direct_dq;        // one key tile: dQ tiles are written as they are
@@ -92,8 +95,8 @@ attn_bwd_prep_kernel(const T* __restrict__ dout, const T* __restrict__ out,
   s += __shfl_xor_sync(0xffffffffu, s, 1);
   if (in && sub == 0) {
     float* st = stats + (((b * H + h) * n_qt + i / ATT_BM) * 2) * ATT_BM + i % ATT_BM;
-    st[0] = live ? lse[(b * H + h) * S + i] * LOG2E : INFINITY;
-    st[ATT_BM] = live ? s * scale : 0.f;
+    st[0] = live ? -lse[(b * H + h) * S + i] * LOG2E : -INFINITY;
+    st[ATT_BM] = live ? -s * scale : 0.f;
   }
 }
 
@@ -146,7 +149,7 @@ struct BwdCfg {
   static constexpr int T_DQ = ALIAS_DQ ? T_DP : T_DK + DP;
   // four warpgroups of 128 registers a thread at launch
   static constexpr int THREADS = 512;
-  static constexpr int REGS_SOFTMAX = 152, REGS_DRAIN = 120, REGS_OTHER = 88;
+  static constexpr int REGS_SOFTMAX = 152, REGS_DRAIN = 104, REGS_OTHER = 104;
   static_assert(2 * REGS_SOFTMAX + REGS_DRAIN + REGS_OTHER <= 4 * 128, "registers of the block");
   static_assert(SMEM <= 232448, "shared memory per CTA");
   static_assert((ALIAS_DQ ? T_DK : T_DQ) + DP <= 512, "TMEM columns");
@@ -174,6 +177,57 @@ __device__ __forceinline__ BwdItem bwd_item(const AttnBwdParams& p, int w) {
   it.q_begin = p.causal ? max(0, it.k0 - (p.Sk - p.Sq)) / ATT_BM : 0;
   it.n = max(0, p.n_qt - it.q_begin);
   return it;
+}
+
+// Probabilities of 32 queries for this thread's key: kept in fp32, packed to 16 bits in the columns
+// of P^T.  Queries below `lim` do not see the key.
+template <typename T, bool MASKED>
+__device__ __forceinline__ void bwd_probs(const uint32_t (&s)[32], float* pr, const float* nlse2,
+                                          uint64_t c2v, int lim, uint32_t t_p) {
+  uint32_t pk[16];
+#pragma unroll
+  for (int j = 0; j < 32; j += 4) {
+    const float4 l4 = *reinterpret_cast<const float4*>(nlse2 + j);
+    float x[4];
+    f2_unpack(fma2(f2_pack(__uint_as_float(s[j]), __uint_as_float(s[j + 1])), c2v,
+                   f2_pack(l4.x, l4.y)), x[0], x[1]);
+    f2_unpack(fma2(f2_pack(__uint_as_float(s[j + 2]), __uint_as_float(s[j + 3])), c2v,
+                   f2_pack(l4.z, l4.w)), x[2], x[3]);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const float e = exp2f(x[u]);
+      pr[j + u] = (MASKED && j + u < lim) ? 0.f : e;
+    }
+    pk[j / 2] = pack2<T>(pr[j], pr[j + 1]);
+    pk[j / 2 + 1] = pack2<T>(pr[j + 2], pr[j + 3]);
+  }
+  tmem_st16(t_p, pk);
+}
+
+// dS^T of the same 32 queries: 16-bit, into this key's row of the swizzled tile from its 16-byte
+// chunk `c0` on
+template <typename T>
+__device__ __forceinline__ void bwd_ds(const uint32_t (&s)[32], const float* pr, const float* ndlt,
+                                       uint64_t scv, uint8_t* ds_row, int row, int c0) {
+#pragma unroll
+  for (int j = 0; j < 32; j += 8) {
+    uint32_t o[4];
+#pragma unroll
+    for (int u = 0; u < 8; u += 4) {
+      const float4 d4 = *reinterpret_cast<const float4*>(ndlt + j + u);
+      float a, b;
+      f2_unpack(mul2(f2_pack(pr[j + u], pr[j + u + 1]),
+                     fma2(f2_pack(__uint_as_float(s[j + u]), __uint_as_float(s[j + u + 1])), scv,
+                          f2_pack(d4.x, d4.y))), a, b);
+      o[u / 2] = pack2<T>(a, b);
+      f2_unpack(mul2(f2_pack(pr[j + u + 2], pr[j + u + 3]),
+                     fma2(f2_pack(__uint_as_float(s[j + u + 2]), __uint_as_float(s[j + u + 3])), scv,
+                          f2_pack(d4.z, d4.w))), a, b);
+      o[u / 2 + 1] = pack2<T>(a, b);
+    }
+    *reinterpret_cast<uint4*>(ds_row + (((c0 + j / 8) ^ (row & 7)) << 4)) =
+        make_uint4(o[0], o[1], o[2], o[3]);
+  }
 }
 
 template <typename T, int DP>
@@ -340,6 +394,7 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
             mma_t_mn(tmem + C::T_DV, tmem + C::T_P, C::P_HALF, sdO + dst * TILE, id_kd, i > 0, q_steps);
             tc_commit(&do_empty[dst]);
             tc_commit(dv_done);
+            if (C::ALIAS_P && more && !(ok = issue_s(g + 1, qt + 1))) break;
             ok = mbar_wait(ds_ready, g & 1, p.status, PF_ERR_TIMEOUT_FULL);
             if (!ok) break;
             const uint32_t ds_tile = sdS + dsb * C::DS_BYTES;
@@ -355,7 +410,6 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
             };
             if (C::ALIAS_DQ) {
               issue_dq();
-              if (C::ALIAS_P && more && !(ok = issue_s(g + 1, qt + 1))) break;
               issue_dk();
               tc_commit(&ds_empty[dsb]);
               if (more && !(ok = issue_dp(g + 1, qt + 1))) break;
@@ -404,42 +458,52 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
         ok = mbar_wait(dq_full, g & 1, p.status, PF_ERR_TIMEOUT_TMEM_FULL);
         if (!ok) break;
         tc_fence_after();
+        // two chunks of 32 columns at a time: the columns of dQ are free as soon as the last pair is
+        // in registers, whatever the boxes wait for
 #pragma unroll
-        for (int c = 0; c < DP / 32; ++c) {
-          uint32_t raw[32];
-          tmem_ld32(tmem + C::T_DQ + lane_off + c * 32, raw);
-          tmem_ld_wait_for(raw);
-          if (c == DP / 32 - 1) {
+        for (int c0 = 0; c0 < DP / 32; c0 += 2) {
+          uint32_t raw[2][32];
+          tmem_ld32(tmem + C::T_DQ + lane_off + c0 * 32, raw[0]);
+          if (c0 + 1 < DP / 32) tmem_ld32(tmem + C::T_DQ + lane_off + c0 * 32 + 32, raw[1]);
+          tmem_ld_wait_for(raw[0]);
+          if (c0 + 1 < DP / 32) tmem_ld_wait_for(raw[1]);
+          if (c0 + 2 >= DP / 32) {
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(dq_empty);
           }
-          if (p.direct_dq) {
-            const int qi = q0 + lane;
-            if (qi < p.Sq) {
-              T* dst = reinterpret_cast<T*>(p.dq) + (long long)it.b * p.sdq[0] +
-                       (long long)qi * p.sdq[1] + (long long)it.h * p.sdq[2] + c * 32;
 #pragma unroll
-              for (int v = 0; v < 4; ++v)
-                if (c * 32 + v * 8 < p.D) reinterpret_cast<uint4*>(dst)[v] = pack8<T>(raw + v * 8);
-            }
-          } else {
-            // two boxes per warp: the reduce-add that last used this one must have read it
-            uint8_t* bx = boxes + (box & 1) * 4096;
-            if (lane == 0 && box >= 2) tma_store_wait_read_but_one();
-            __syncwarp();
+          for (int u = 0; u < 2; ++u) {
+            const int c = c0 + u;
+            if (c >= DP / 32) continue;
+            if (p.direct_dq) {
+              const int qi = q0 + lane;
+              if (qi < p.Sq) {
+                T* dst = reinterpret_cast<T*>(p.dq) + (long long)it.b * p.sdq[0] +
+                         (long long)qi * p.sdq[1] + (long long)it.h * p.sdq[2] + c * 32;
 #pragma unroll
-            for (int v = 0; v < 8; ++v)
-              *reinterpret_cast<uint4*>(bx + lane * 128 + ((v ^ (lane & 7)) << 4)) =
-                  make_uint4(raw[v * 4], raw[v * 4 + 1], raw[v * 4 + 2], raw[v * 4 + 3]);
-            fence_async_smem();
-            __syncwarp();
-            if (lane == 0) {
-              // rows beyond the last query / columns beyond D are clipped by the TMA itself
-              if (q0 < p.Sq) tma_reduce_add_4d(&tdq, bx, c * 32, it.h, q0, it.b);
-              tma_store_commit();
+                for (int v = 0; v < 4; ++v)
+                  if (c * 32 + v * 8 < p.D)
+                    reinterpret_cast<uint4*>(dst)[v] = pack8<T>(raw[u] + v * 8);
+              }
+            } else {
+              // two boxes per warp: the reduce-add that last used this one must have read it
+              uint8_t* bx = boxes + (box & 1) * 4096;
+              if (lane == 0 && box >= 2) tma_store_wait_read_but_one();
+              __syncwarp();
+#pragma unroll
+              for (int v = 0; v < 8; ++v)
+                *reinterpret_cast<uint4*>(bx + lane * 128 + ((v ^ (lane & 7)) << 4)) = make_uint4(
+                    raw[u][v * 4], raw[u][v * 4 + 1], raw[u][v * 4 + 2], raw[u][v * 4 + 3]);
+              fence_async_smem();
+              __syncwarp();
+              if (lane == 0) {
+                // rows beyond the last query / columns beyond D are clipped by the TMA itself
+                if (q0 < p.Sq) tma_reduce_add_4d(&tdq, bx, c * 32, it.h, q0, it.b);
+                tma_store_commit();
+              }
+              ++box;
             }
-            ++box;
           }
         }
       }
@@ -493,91 +557,91 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
       for (int i = 0; i < it.n && ok; ++i, ++g) {
         const int q0 = (it.q_begin + i) * ATT_BM, st = g & 1, dsb = g % C::NDS;
         const int cols = (min(ATT_BM, p.Sq - q0) + 15) / 16 * 16;
-        const float* lse2 =
+        const float* nlse2 =
             reinterpret_cast<const float*>(smem + C::OFF_STAT + st * 1024) + half * 64;
-        const float* dlt = lse2 + 128;
+        const float* ndlt = nlse2 + 128;
         const bool masked = ragged || (p.causal && it.k0 + ATT_BN - 1 > q0 + shift);
         // queries of this half below `lim` do not see the key of this row
         int lim = p.causal ? kj - shift - q0 - half * 64 : -1;
         if (kj >= p.Sk) lim = ATT_BM;
-        ok = mbar_wait(&q_full[st], (g >> 1) & 1, p.status, PF_ERR_TIMEOUT_FULL) &&
-             mbar_wait(s_full, g & 1, p.status, PF_ERR_TIMEOUT_TMEM_FULL);
-        if (!C::ALIAS_P && ok && g > 0)     // the columns of P^T: dV of the previous tile read them
-          ok = mbar_wait(dv_done, (g - 1) & 1, p.status, PF_ERR_TIMEOUT_TMEM_EMPTY);
+        // A wait that is satisfied still takes some 130 cycles: all barriers are looked at together
+        // first.  (The columns of P^T must have been read by dV of the previous tile.)
+        const bool chk_dv = !C::ALIAS_P && g > 0;
+        const bool seen_q = mbar_test(&q_full[st], (g >> 1) & 1), seen_s = mbar_test(s_full, g & 1);
+        const bool seen_v = !chk_dv || mbar_test(dv_done, (g - 1) & 1);
+        if (!(seen_q && seen_s && seen_v)) {
+          ok = mbar_wait(&q_full[st], (g >> 1) & 1, p.status, PF_ERR_TIMEOUT_FULL) &&
+               mbar_wait(s_full, g & 1, p.status, PF_ERR_TIMEOUT_TMEM_FULL);
+          if (chk_dv && ok) ok = mbar_wait(dv_done, (g - 1) & 1, p.status, PF_ERR_TIMEOUT_TMEM_EMPTY);
+        }
         if (!ok) break;
         tc_fence_after();
         float pr[64];
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          const bool work = warp_live && half * 64 + c * 32 < cols;     // warp-uniform
-          uint32_t s[32];
-          if (work) {
-            tmem_ld32(tmem + C::T_S + lane_off + half * 64 + c * 32, s);
-            tmem_ld_wait_for(s);
-          }
-          if (!C::ALIAS_P && c == 1) {
+        const uint32_t t_p = tmem + C::T_P + lane_off + half * C::P_HALF;
+        const uint32_t t_s = tmem + C::T_S + lane_off + half * 64;
+        const uint32_t t_dp = tmem + C::T_DP + lane_off + half * 64;
+        // the usual tile: nothing masked, all of this warp's columns and rows exist
+        const bool whole = warp_live && !masked && half * 64 + 64 <= cols;
+        if (whole) {
+          uint32_t s0[32], s1[32];
+          tmem_ld32(t_s, s0);
+          tmem_ld_wait_for(s0);
+          tmem_ld32(t_s + 32, s1);          // travels while the first half is worked on
+          bwd_probs<T, false>(s0, pr, nlse2, c2v, 0, t_p);
+          tmem_ld_wait_for(s1);
+          if (!C::ALIAS_P) {
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(s_empty);
           }
-          if (work) {
-            uint32_t pk[16];
+          bwd_probs<T, false>(s1, pr + 32, nlse2 + 32, c2v, 0, t_p + 16);
+        } else {
 #pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-              const float4 l4 = *reinterpret_cast<const float4*>(lse2 + c * 32 + j);
-              float x[4];
-              f2_unpack(fma2(f2_pack(__uint_as_float(s[j]), __uint_as_float(s[j + 1])), c2v,
-                             f2_pack(-l4.x, -l4.y)), x[0], x[1]);
-              f2_unpack(fma2(f2_pack(__uint_as_float(s[j + 2]), __uint_as_float(s[j + 3])), c2v,
-                             f2_pack(-l4.z, -l4.w)), x[2], x[3]);
-#pragma unroll
-              for (int u = 0; u < 4; ++u) {
-                float e = exp2f(x[u]);
-                if (masked && c * 32 + j + u < lim) e = 0.f;
-                pr[c * 32 + j + u] = e;
-              }
-              pk[j / 2] = pack2<T>(pr[c * 32 + j], pr[c * 32 + j + 1]);
-              pk[j / 2 + 1] = pack2<T>(pr[c * 32 + j + 2], pr[c * 32 + j + 3]);
+          for (int c = 0; c < 2; ++c) {
+            const bool work = warp_live && half * 64 + c * 32 < cols;     // warp-uniform
+            uint32_t s[32];
+            if (work) {
+              tmem_ld32(t_s + c * 32, s);
+              tmem_ld_wait_for(s);
             }
-            tmem_st16(tmem + C::T_P + lane_off + half * C::P_HALF + c * 16, pk);
+            if (!C::ALIAS_P && c == 1) {
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(s_empty);
+            }
+            if (work)
+              bwd_probs<T, true>(s, pr + c * 32, nlse2 + c * 32, c2v, lim - c * 32, t_p + c * 16);
           }
         }
+        const bool seen_dp = mbar_test(dp_full, g & 1);
+        const bool seen_ds = mbar_test(&ds_empty[dsb], ((g / C::NDS) & 1) ^ 1);
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(p_ready);
         // ---- dS^T
-        ok = mbar_wait(dp_full, g & 1, p.status, PF_ERR_TIMEOUT_TMEM_FULL) &&
-             mbar_wait(&ds_empty[dsb], ((g / C::NDS) & 1) ^ 1, p.status, PF_ERR_TIMEOUT_EMPTY);
+        if (!(seen_dp && seen_ds))
+          ok = mbar_wait(dp_full, g & 1, p.status, PF_ERR_TIMEOUT_TMEM_FULL) &&
+               mbar_wait(&ds_empty[dsb], ((g / C::NDS) & 1) ^ 1, p.status, PF_ERR_TIMEOUT_EMPTY);
         if (!ok) break;
         tc_fence_after();
         uint8_t* ds_row = smem + C::OFF_DS + dsb * C::DS_BYTES + half * ATT_BLK + row * 128;
+        if (whole) {
+          uint32_t s0[32], s1[32];
+          tmem_ld32(t_dp, s0);
+          tmem_ld_wait_for(s0);
+          tmem_ld32(t_dp + 32, s1);
+          bwd_ds<T>(s0, pr, ndlt, scv, ds_row, row, 0);
+          tmem_ld_wait_for(s1);
+          bwd_ds<T>(s1, pr + 32, ndlt + 32, scv, ds_row, row, 4);
+        } else {
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          if (warp_live && half * 64 + c * 32 < cols) {
-            uint32_t s[32];
-            tmem_ld32(tmem + C::T_DP + lane_off + half * 64 + c * 32, s);
-            tmem_ld_wait_for(s);
-#pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-              uint32_t o[4];
-#pragma unroll
-              for (int u = 0; u < 8; u += 4) {
-                const float4 d4 = *reinterpret_cast<const float4*>(dlt + c * 32 + j + u);
-                float a, b;
-                f2_unpack(mul2(f2_pack(pr[c * 32 + j + u], pr[c * 32 + j + u + 1]),
-                               fma2(f2_pack(__uint_as_float(s[j + u]),
-                                            __uint_as_float(s[j + u + 1])),
-                                    scv, f2_pack(-d4.x, -d4.y))), a, b);
-                o[u / 2] = pack2<T>(a, b);
-                f2_unpack(mul2(f2_pack(pr[c * 32 + j + u + 2], pr[c * 32 + j + u + 3]),
-                               fma2(f2_pack(__uint_as_float(s[j + u + 2]),
-                                            __uint_as_float(s[j + u + 3])),
-                                    scv, f2_pack(-d4.z, -d4.w))), a, b);
-                o[u / 2 + 1] = pack2<T>(a, b);
-              }
-              *reinterpret_cast<uint4*>(ds_row + (((c * 4 + j / 8) ^ (row & 7)) << 4)) =
-                  make_uint4(o[0], o[1], o[2], o[3]);
+          for (int c = 0; c < 2; ++c) {
+            if (warp_live && half * 64 + c * 32 < cols) {
+              uint32_t s[32];
+              tmem_ld32(t_dp + c * 32, s);
+              tmem_ld_wait_for(s);
+              bwd_ds<T>(s, pr + c * 32, ndlt + c * 32, scv, ds_row, row, c * 4);
             }
           }
         }
