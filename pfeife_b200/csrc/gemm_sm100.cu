@@ -876,19 +876,34 @@ PF_API int pf_gemm(const void* A, const void* B, void* C, int M, int N, int K, l
                 !(aux && out_dtype == PF_F32);
   // Split-K: a gradient-accumulating GEMM whose tiles do not fill the GPU divides each tile's
   // reduction among several work items; they all reduce-add into C, which costs nothing extra
-  // because the epilogue accumulates anyway.
+  // because the epilogue accumulates anyway.  The weight gradient of a convolution, whose long
+  // reduction over the output pixels meets few tiles, does so too when it does not accumulate: C is
+  // small beside the operands and is cleared first (3 x 3, 320 filters of 320 channels over
+  // [4, 128, 128]: 24 pair tiles, 301 us whole, 123 in three).
   p.split_k = 1;
-  if (p.tma_store && accumulate && out_dtype == PF_F32 && !g_gather.on_any() && !g_conv.on &&
-      !bias && !residual && epilogue == EPI_NONE && !(tile_n & 8192)) {
+  const bool clear_first = !accumulate && g_conv.on == 2 && ldc == N;
+  if (p.vec_ok && out_dtype == PF_F32 && (accumulate || clear_first) && !(tile_n & 1024) && !aux &&
+      !g_gather.on_any() && g_conv.on != 1 && !bias && !residual && epilogue == EPI_NONE &&
+      !(tile_n & 8192)) {
     const int bm = pair ? 256 : 128, bn = pair ? 256 : BN;
     const long long tiles = (long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn);
     const long long slots = pair ? sm_count / 2 : sm_count;
     const int nkb = (K + GEMM_BK - 1) / GEMM_BK;
     double best = 1e30;
     for (int sk = 1; sk <= 4 && sk * 8 <= nkb; ++sk) {
-      const double waves = (double)((tiles * sk + slots - 1) / slots) / sk + 0.03 * (sk - 1);
+      double waves = (double)((tiles * sk + slots - 1) / slots) / sk + 0.03 * (sk - 1);
+      // clearing C and adding to it from L2 moves some 4 MB per us, a k-block of a full wave takes
+      // 0.36 us ([1, 32, 32, 1280] with 1280 filters, 59 MB of C: 40 us whole, 60 in two)
+      if (clear_first && sk > 1)
+        waves += (double)M * N * (1 + 2 * sk) / 1e6 / (0.36 * nkb);
       if (waves < best - 1e-9) { best = waves; p.split_k = sk; }
     }
+  }
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  if (p.split_k > 1 && clear_first) {
+    cudaError_t e = cudaMemsetAsync(C, 0, sizeof(float) * (size_t)M * (size_t)N, st);
+    if (e != cudaSuccess) return (int)e;
+    p.accumulate = 1;
   }
   CUtensorMap tc, taux;
   memset(&tc, 0, sizeof(tc));
@@ -899,7 +914,6 @@ PF_API int pf_gemm(const void* A, const void* B, void* C, int M, int N, int K, l
                                     epilogue == EPI_SILU);
     if (aux_is_out && (r = make_tmap_out(&taux, aux, out_dtype, N, M, ldaux))) return r;
   }
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
 
   const bool gather = g_gather.world > 1;
 #define PF_GEMM_DISPATCH(T)                                                                    \

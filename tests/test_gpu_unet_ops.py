@@ -221,3 +221,31 @@ def test_conv_weight_kernels_move_every_element(Cout, Cin, taps):
     for dtype in (torch.float32, torch.bfloat16, torch.float16):
         got = kx.conv_unpack(sums, w.shape, cin8, dtype)
         assert got.is_contiguous() and torch.equal(got, want.to(dtype))
+
+
+@pytest.mark.parametrize("batch,hw,cin,cout,stride", [
+    (1, 8, 64, 64, 1),        # one k-block per image row group, one tile, nothing to split
+    (3, 8, 128, 72, 1),       # k-blocks of eight output rows, image after image
+    (2, 32, 64, 320, 1),      # the reduction in several parts: C is cleared and added to
+    (2, 128, 64, 64, 1),      # a k-block is half an output row
+    (2, 32, 64, 128, 2),      # stride 2: 16 x 16 outputs
+])
+def test_conv_wgrad_steps_through_pixels(batch, hw, cin, cout, stride):
+    """Weight gradients over every way a k-block of 64 output pixels can lie in an image, also into a
+    buffer that holds something else before (the split reduction clears it).  Products are exact in
+    fp32, so only the order of the sums differs: 2^-24 of the root of the number of terms."""
+    from pfeife_b200.ops import kernels as kx
+    torch.manual_seed(3)
+    x = torch.randn(batch, hw, hw, cin, device="cuda").to(torch.bfloat16)
+    ho = (hw - 1) // stride + 1
+    dy = torch.randn(batch, ho, ho, cout, device="cuda").to(torch.bfloat16)
+    assert kx.conv_wgrad_supported(x, cout, 3, 3, stride, 1)
+    out = torch.full((cout, 9 * cin), 7.0, device="cuda")
+    kx.conv_wgrad(dy.view(-1, cout), x, 3, 3, stride, 1, out=out)
+    more = kx.conv_wgrad(dy.view(-1, cout), x, 3, 3, stride, 1, out=out.clone(), accumulate=True)
+    ref = torch.nn.grad.conv2d_weight(x.double().permute(0, 3, 1, 2), (cout, cin, 3, 3),
+                                      dy.double().permute(0, 3, 1, 2), stride=stride, padding=1)
+    ref = ref.permute(0, 2, 3, 1).reshape(cout, 9 * cin)
+    kx.check_status()
+    assert ((out - ref).norm() / ref.norm()).item() < 1e-5
+    assert ((more - 2 * ref).norm() / ref.norm()).item() < 2e-5
