@@ -203,9 +203,9 @@ __device__ __forceinline__ void cp_async16(void* smem_dst, const void* src) {
 __device__ __forceinline__ void cp_async_commit() {
   asm volatile("cp.async.commit_group;" ::: "memory");
 }
-// all but the most recently committed group have landed (for the calling thread's copies)
-__device__ __forceinline__ void cp_async_wait_but_one() {
-  asm volatile("cp.async.wait_group 1;" ::: "memory");
+// all but the N most recently committed groups have landed (for the calling thread's copies)
+template <int N> __device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 __device__ __forceinline__ void tma_store_commit() {
   asm volatile("cp.async.bulk.commit_group;" ::: "memory");

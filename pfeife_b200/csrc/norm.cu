@@ -293,127 +293,6 @@ norm_fwd_warp_kernel(const T* __restrict__ x, const T* __restrict__ res,
   }
 }
 
-// Backward, input gradient only: one warp per row, packed dy / h kept in registers, two
-// shuffle reductions.  The parameter gradients come from norm_bwd_param_kernel.
-template <typename T, int NV>
-__global__ void __launch_bounds__(256)
-norm_bwd_dx_kernel(const T* __restrict__ dy, const T* __restrict__ h,
-                   const float* __restrict__ gamma, const float* __restrict__ mean,
-                   const float* __restrict__ rstd, const T* __restrict__ dres,
-                   T* __restrict__ dx, long long rows, int N, int rms) {
-  constexpr int V = 8;
-  const int nvec = N / V;
-  const int lane = threadIdx.x & 31;
-  const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (row >= rows) return;
-  const float mu = rms ? 0.f : mean[row];
-  const float rs = rstd[row];
-  uint4 qd[NV], qh[NV];
-  float s1 = 0.f, s2 = 0.f;
-#pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    const int idx = lane + i * 32;
-    if (idx < nvec) {
-      qd[i] = reinterpret_cast<const uint4*>(dy + row * N)[idx];
-      qh[i] = reinterpret_cast<const uint4*>(h + row * N)[idx];
-      const T* ed = reinterpret_cast<const T*>(&qd[i]);
-      const T* eh = reinterpret_cast<const T*>(&qh[i]);
-      const float4 g0 = __ldg(reinterpret_cast<const float4*>(gamma + idx * V));
-      const float4 g1 = __ldg(reinterpret_cast<const float4*>(gamma + idx * V) + 1);
-      const float g[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-#pragma unroll
-      for (int j = 0; j < V; ++j) {
-        const float dyg = to_f32<T>(ed[j]) * g[j];
-        s1 += dyg;
-        s2 += dyg * (to_f32<T>(eh[j]) - mu) * rs;
-      }
-    }
-  }
-  const float m1 = rms ? 0.f : warp_sum(s1) / N;
-  const float m2 = warp_sum(s2) / N;
-#pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    const int idx = lane + i * 32;
-    if (idx < nvec) {
-      const T* ed = reinterpret_cast<const T*>(&qd[i]);
-      const T* eh = reinterpret_cast<const T*>(&qh[i]);
-      const float4 g0 = __ldg(reinterpret_cast<const float4*>(gamma + idx * V));
-      const float4 g1 = __ldg(reinterpret_cast<const float4*>(gamma + idx * V) + 1);
-      const float g[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-      uint4 qr;
-      if (dres) qr = reinterpret_cast<const uint4*>(dres + row * N)[idx];
-      const T* er = reinterpret_cast<const T*>(&qr);
-      uint4 q;
-      T* e = reinterpret_cast<T*>(&q);
-#pragma unroll
-      for (int j = 0; j < V; ++j) {
-        const float xhat = (to_f32<T>(eh[j]) - mu) * rs;
-        float o = rs * (to_f32<T>(ed[j]) * g[j] - m1 - xhat * m2);
-        if (dres) o += to_f32<T>(er[j]);
-        e[j] = from_f32<T>(o);
-      }
-      reinterpret_cast<uint4*>(dx + row * N)[idx] = q;
-    }
-  }
-}
-
-// dgamma[c] += sum_r dy[r,c] * xhat[r,c] ; dbeta[c] += sum_r dy[r,c].  Each CTA owns 256
-// columns (lane = 8 consecutive columns, 16-byte loads) and a slab of rows split over its 8
-// warps; warps are combined through shared memory and the CTA writes its partial sums to the
-// scratch buffer, which norm_bwd_finish_kernel folds (deterministic, nothing to zero).
-template <typename T>
-__global__ void __launch_bounds__(256)
-norm_bwd_param_kernel(const T* __restrict__ dy, const T* __restrict__ h,
-                      const float* __restrict__ mean, const float* __restrict__ rstd,
-                      float* __restrict__ scratch, float* __restrict__ acc_gamma,
-                      float* __restrict__ acc_beta, long long rows, int N, int rows_per_cta,
-                      int rms) {
-  __shared__ float red[2][8][256];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int c0 = blockIdx.x * 256 + lane * 8;
-  const long long r0 = (long long)blockIdx.y * rows_per_cta;
-  const long long r1 = min(rows, r0 + rows_per_cta);
-  float ag[8] = {0, 0, 0, 0, 0, 0, 0, 0}, ab[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  if (c0 < N) {
-    for (long long r = r0 + warp; r < r1; r += 8) {
-      const float mu = rms ? 0.f : mean[r];
-      const float rs = rstd[r];
-      const uint4 qd = *reinterpret_cast<const uint4*>(dy + r * N + c0);
-      const uint4 qh = *reinterpret_cast<const uint4*>(h + r * N + c0);
-      const T* ed = reinterpret_cast<const T*>(&qd);
-      const T* eh = reinterpret_cast<const T*>(&qh);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float d = to_f32<T>(ed[j]);
-        ag[j] += d * (to_f32<T>(eh[j]) - mu) * rs;
-        ab[j] += d;
-      }
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    red[0][warp][lane * 8 + j] = ag[j];
-    red[1][warp][lane * 8 + j] = ab[j];
-  }
-  __syncthreads();
-  const int c = blockIdx.x * 256 + threadIdx.x;
-  if (c < N) {
-    float g = 0.f, b = 0.f;
-#pragma unroll
-    for (int w = 0; w < 8; ++w) { g += red[0][w][threadIdx.x]; b += red[1][w][threadIdx.x]; }
-    if (acc_gamma) {
-      // accumulating into existing gradients (the framework's gradient bucket): add this row
-      // slab's sums directly, no folding pass
-      atomicAdd(acc_gamma + c, g);
-      if (acc_beta) atomicAdd(acc_beta + c, b);
-    } else {
-      // partial sums of this row slab: scratch[slab][0][c] (dgamma), scratch[slab][1][c] (dbeta)
-      scratch[((long long)blockIdx.y * 2) * N + c] = g;
-      scratch[((long long)blockIdx.y * 2 + 1) * N + c] = b;
-    }
-  }
-}
-
 // Backward for rows of up to 2048 16-bit elements, everything in one pass over memory.  A
 // persistent CTA walks over tiles of 8 rows that asynchronous copies bring into shared memory, one
 // tile ahead; dy and h are then read there twice:
@@ -423,7 +302,7 @@ norm_bwd_param_kernel(const T* __restrict__ dy, const T* __restrict__ h,
 // The CTA's sums go to scratch[blockIdx][2][N], folded by norm_bwd_finish_kernel.
 // Bound by HBM: 4 tensors cross it once, where a pass for dx and one for the sums read dy and h
 // twice.  bf16, with the fold: 6168 x 1408 50 -> 38 us, 50000 x 1408 249 -> 153 us (3.7 TB/s),
-// 20000 x 2048 173 -> 112 us.  Longer rows keep the two passes: two stages of 8 of them do not fit.
+// 20000 x 2048 173 -> 112 us.  Longer rows: norm_bwd_wide_kernel.
 constexpr int NORM_TILE_ROWS = 8;
 template <typename T, int NV>
 __global__ void __launch_bounds__(256)
@@ -476,7 +355,7 @@ norm_bwd_fused_kernel(const T* __restrict__ dy, const T* __restrict__ h,
             qr[i] = __ldg(reinterpret_cast<const uint4*>(dres + row * N) + lane + i * 32);
       }
     }
-    cp_async_wait_but_one();           // this tile has landed, the next one may be under way
+    cp_async_wait<1>();           // this tile has landed, the next one may be under way
     __syncthreads();
     const uint4 *sd = stage_ptr(st, 0), *sh = stage_ptr(st, 1);
     if (warp < live) {
@@ -560,6 +439,138 @@ norm_bwd_fused_kernel(const T* __restrict__ dy, const T* __restrict__ h,
   }
 }
 
+// Backward for rows of 2056 to 4096 16-bit elements, in one pass as well: two stages of eight such
+// rows do not fit in shared memory, so a thread owns 8 columns for good and keeps their parameter sums
+// in registers, and a row's two sums go through the CTA (one barrier per NORM_WIDE_ROWS rows).  A
+// thread only ever reads what it copied itself, so the ring that its asynchronous copies fill three
+// batches ahead (144 KB on their way per SM at 4096 columns) needs no barriers.  One CTA per SM.
+// Bound by HBM: 4 tensors cross it once.  bf16, with the fold, against a pass for dx (one warp per row,
+// 16 vectors of two tensors in registers) and one for the sums: 2048 x 4096 62 -> 28 us,
+// 20000 x 4096 441 -> 132, 50000 x 4096 1066 -> 308 (5.3 TB/s), 9000 x 3072 120 -> 60.
+constexpr int NORM_WIDE_ROWS = 2, NORM_WIDE_STAGES = 4;
+template <typename T, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1)
+norm_bwd_wide_kernel(const T* __restrict__ dy, const T* __restrict__ h,
+                     const float* __restrict__ gamma, const float* __restrict__ mean,
+                     const float* __restrict__ rstd, const T* __restrict__ dres,
+                     T* __restrict__ dx, float* __restrict__ scratch, long long rows, int N,
+                     int rms) {
+  constexpr int V = 8, R = NORM_WIDE_ROWS, S = NORM_WIDE_STAGES, WARPS = THREADS / 32;
+  static_assert(WARPS <= 32 && R == 2, "one lane per warp folds the sums of two rows");
+  __shared__ float4 red[2][WARPS];             // per warp: s1, s2 of both rows; two batches
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, cv = threadIdx.x;
+  const bool on = cv < N / V;
+  float g[V], ag[V], ab[V];
+#pragma unroll
+  for (int j = 0; j < V; ++j) {
+    g[j] = on ? __ldg(gamma + cv * V + j) : 0.f;
+    ag[j] = ab[j] = 0.f;
+  }
+  const float inv_n = 1.f / N;
+  const long long n_batches = (rows + R - 1) / R;
+  extern __shared__ __align__(128) uint8_t wsmem[];     // [stage][row][dy, h, dres][thread]
+  auto slot = [&](int st, int r, int which) {
+    return reinterpret_cast<uint4*>(wsmem) + ((st * R + r) * 3 + which) * THREADS + cv;
+  };
+  auto fetch = [&](long long b, int st) {
+    if (on && b < n_batches) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const long long row = b * R + r;
+        if (row < rows) {
+          cp_async16(slot(st, r, 0), reinterpret_cast<const uint4*>(dy + row * N) + cv);
+          cp_async16(slot(st, r, 1), reinterpret_cast<const uint4*>(h + row * N) + cv);
+          if (dres) cp_async16(slot(st, r, 2), reinterpret_cast<const uint4*>(dres + row * N) + cv);
+        }
+      }
+    }
+    cp_async_commit();                 // an empty group past the last batch
+  };
+  const long long step = gridDim.x;
+  long long b = blockIdx.x;
+#pragma unroll
+  for (int i = 0; i < S - 1; ++i) fetch(b + i * step, i);
+  int st = 0;
+  for (int parity = 0; b < n_batches; b += step, parity ^= 1) {
+    uint4 qd[R], qh[R], qr[R];
+    float mu[R], rs[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const long long row = min(b * R + r, rows - 1);
+      mu[r] = rms ? 0.f : __ldg(mean + row);
+      rs[r] = __ldg(rstd + row);
+      qd[r] = qh[r] = qr[r] = make_uint4(0, 0, 0, 0);
+    }
+    cp_async_wait<S - 2>();            // this batch has landed, the later ones may be under way
+    if (on) {
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (b * R + r < rows) {
+          qd[r] = *slot(st, r, 0);
+          qh[r] = *slot(st, r, 1);
+          if (dres) qr[r] = *slot(st, r, 2);
+        }
+    }
+    // into the slots read in the previous round
+    fetch(b + (S - 1) * step, st == 0 ? S - 1 : st - 1);
+    st = st == S - 1 ? 0 : st + 1;
+    float s[2 * R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const T* ed = reinterpret_cast<const T*>(&qd[r]);
+      const T* eh = reinterpret_cast<const T*>(&qh[r]);
+      float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+      for (int j = 0; j < V; ++j) {
+        const float d = to_f32<T>(ed[j]), xhat = (to_f32<T>(eh[j]) - mu[r]) * rs[r];
+        const float dyg = d * g[j];
+        s1 += dyg;
+        s2 += dyg * xhat;
+        ag[j] += d * xhat;
+        ab[j] += d;
+      }
+      s[2 * r] = on ? s1 : 0.f;
+      s[2 * r + 1] = on ? s2 : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < 2 * R; ++i) s[i] = warp_sum(s[i]);
+    if (lane == 0) red[parity][warp] = make_float4(s[0], s[1], s[2], s[3]);
+    // the buffer of two batches ago is free: every warp has passed the barrier since it read it
+    __syncthreads();
+    float4 f = lane < WARPS ? red[parity][lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+    f.x = warp_sum(f.x); f.y = warp_sum(f.y); f.z = warp_sum(f.z); f.w = warp_sum(f.w);
+    const float m1[R] = {rms ? 0.f : f.x * inv_n, rms ? 0.f : f.z * inv_n};
+    const float m2[R] = {f.y * inv_n, f.w * inv_n};
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const long long row = b * R + r;
+      if (on && row < rows) {
+        const T* ed = reinterpret_cast<const T*>(&qd[r]);
+        const T* eh = reinterpret_cast<const T*>(&qh[r]);
+        const T* er = reinterpret_cast<const T*>(&qr[r]);
+        uint4 q;
+        T* e = reinterpret_cast<T*>(&q);
+#pragma unroll
+        for (int j = 0; j < V; ++j) {
+          const float xhat = (to_f32<T>(eh[j]) - mu[r]) * rs[r];
+          float o = rs[r] * (to_f32<T>(ed[j]) * g[j] - m1[r] - xhat * m2[r]);
+          if (dres) o += to_f32<T>(er[j]);
+          e[j] = from_f32<T>(o);
+        }
+        reinterpret_cast<uint4*>(dx + row * N)[cv] = q;
+      }
+    }
+  }
+  if (on) {
+    float4* og = reinterpret_cast<float4*>(scratch + (long long)blockIdx.x * 2 * N + cv * V);
+    float4* ob = reinterpret_cast<float4*>(scratch + (long long)blockIdx.x * 2 * N + N + cv * V);
+    og[0] = make_float4(ag[0], ag[1], ag[2], ag[3]);
+    og[1] = make_float4(ag[4], ag[5], ag[6], ag[7]);
+    ob[0] = make_float4(ab[0], ab[1], ab[2], ab[3]);
+    ob[1] = make_float4(ab[4], ab[5], ab[6], ab[7]);
+  }
+}
+
 // dgamma[c] (+)= sum_g scratch[g][0][c] ; dbeta likewise.  A CTA owns 32 columns, its 32 warps share
 // the G rows (one thread per column over all rows took 29 us of latency at G = 296).
 __global__ void __launch_bounds__(1024)
@@ -614,6 +625,26 @@ static int norm_bwd_fused_launch(const void* dy, const void* h, const float* gam
   return 0;
 }
 
+template <typename T, int THREADS>
+static int norm_bwd_wide_launch(const void* dy, const void* h, const float* gamma,
+                                const float* mean, const float* rstd, const void* dres, void* dx,
+                                float* scratch, int G, long long rows, int N, int rms,
+                                cudaStream_t st) {
+  auto kern = norm_bwd_wide_kernel<T, THREADS>;
+  constexpr int bytes = NORM_WIDE_STAGES * NORM_WIDE_ROWS * 3 * THREADS * 16;
+  static bool done[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64 || !done[dev]) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess) return (int)e;
+    if (dev >= 0 && dev < 64) done[dev] = true;
+  }
+  kern<<<G, THREADS, bytes, st>>>((const T*)dy, (const T*)h, gamma, mean, rstd, (const T*)dres,
+                                  (T*)dx, scratch, rows, N, rms);
+  return 0;
+}
+
 template <typename T>
 static int norm_fwd_launch(const void* x, const void* res, const float* gamma, const float* beta,
                            void* y, void* h_out, float* mean, float* rstd, long long rows, int N,
@@ -651,8 +682,7 @@ static int norm_fwd_launch(const void* x, const void* res, const float* gamma, c
 template <typename T>
 static int norm_bwd_launch(const void* dy, const void* h, const float* gamma, const float* mean,
                            const float* rstd, const void* dres, void* dx, float* scratch, int& G,
-                           long long rows, int N, int rms, cudaStream_t st,
-                           float* acc_gamma = nullptr, float* acc_beta = nullptr) {
+                           long long rows, int N, int rms, cudaStream_t st) {
   constexpr int V = 16 / sizeof(T);
   if (N % V) return -2;
   const int nvec = N / V;
@@ -666,29 +696,12 @@ static int norm_bwd_launch(const void* dy, const void* h, const float* gamma, co
 #undef PF_NORM_BWD_FUSED
   }
   if constexpr (sizeof(T) == 2) if (nvec <= 32 * 16) {
-    // input gradient: warp per row (rows of up to 4096 16-bit elements: Llama's hidden size);
-    // parameter gradients: column reduction over row slabs
-    const unsigned grid = (unsigned)((rows + 7) / 8);
-#define PF_NORM_BWD_DX(NV)                                                                   \
-    norm_bwd_dx_kernel<T, NV><<<grid, 256, 0, st>>>((const T*)dy, (const T*)h, gamma, mean,  \
-        rstd, (const T*)dres, (T*)dx, rows, N, rms)
-    if (nvec <= 32 * 12) PF_NORM_BWD_DX(12);
-    else PF_NORM_BWD_DX(16);
-#undef PF_NORM_BWD_DX
-    // enough row slabs to fill the GPU once with (column blocks x slabs) CTAs, few enough
-    // that folding them (norm_bwd_finish_kernel) stays negligible
-    const int col_blocks = (N + 255) / 256;
-    int slabs = (2 * 148 + col_blocks - 1) / col_blocks;
-    if (slabs > (int)((rows + 31) / 32)) slabs = (int)((rows + 31) / 32);
-    if (slabs > G) slabs = G;
-    if (slabs < 1) slabs = 1;
-    const int rows_per = (int)((rows + slabs - 1) / slabs);
-    slabs = (int)((rows + rows_per - 1) / rows_per);
-    norm_bwd_param_kernel<T><<<dim3((N + 255) / 256, slabs), 256, 0, st>>>(
-        (const T*)dy, (const T*)h, mean, rstd, scratch, acc_gamma, acc_beta, rows, N, rows_per,
-        rms);
-    G = acc_gamma ? 0 : slabs;      // 0: the sums are already where they belong
-    return 0;
+    // rows of up to 4096 16-bit elements (Llama's hidden size): one CTA per SM fills its shared memory
+    if (G > 148) G = 148;
+#define PF_NORM_BWD_WIDE(THREADS)                                                                 \
+    norm_bwd_wide_launch<T, THREADS>(dy, h, gamma, mean, rstd, dres, dx, scratch, G, rows, N, rms, st)
+    return nvec <= 384 ? PF_NORM_BWD_WIDE(384) : PF_NORM_BWD_WIDE(512);
+#undef PF_NORM_BWD_WIDE
   }
   if (nvec <= 128 * NORM_MAX_VEC)
     norm_bwd_kernel<T, 128><<<G, 128, 0, st>>>((const T*)dy, (const T*)h, gamma, mean, rstd,
@@ -740,23 +753,17 @@ PF_API int pf_norm_bwd(const void* dy, const void* h, const void* gamma, const v
   if (rows <= 0) return 0;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   int G = pf_norm_bwd_ctas(rows, sm_count);   // rows of scratch; the launch may use fewer
-  // when the sums are added to existing gradients the row slabs add them directly (G comes
-  // back 0) instead of leaving partial sums for the folding kernel
-  float* ag = accumulate ? (float*)dgamma : nullptr;
-  float* ab = accumulate ? (float*)dbeta : nullptr;
   int r = -1;
   switch (dtype) {
-    case PF_F32: r = norm_bwd_launch<float>(dy, h, (const float*)gamma, (const float*)mean, (const float*)rstd, dres, dx, (float*)scratch, G, rows, N, rms, st, ag, ab); break;
-    case PF_F16: r = norm_bwd_launch<__half>(dy, h, (const float*)gamma, (const float*)mean, (const float*)rstd, dres, dx, (float*)scratch, G, rows, N, rms, st, ag, ab); break;
-    case PF_BF16: r = norm_bwd_launch<__nv_bfloat16>(dy, h, (const float*)gamma, (const float*)mean, (const float*)rstd, dres, dx, (float*)scratch, G, rows, N, rms, st, ag, ab); break;
+    case PF_F32: r = norm_bwd_launch<float>(dy, h, (const float*)gamma, (const float*)mean, (const float*)rstd, dres, dx, (float*)scratch, G, rows, N, rms, st); break;
+    case PF_F16: r = norm_bwd_launch<__half>(dy, h, (const float*)gamma, (const float*)mean, (const float*)rstd, dres, dx, (float*)scratch, G, rows, N, rms, st); break;
+    case PF_BF16: r = norm_bwd_launch<__nv_bfloat16>(dy, h, (const float*)gamma, (const float*)mean, (const float*)rstd, dres, dx, (float*)scratch, G, rows, N, rms, st); break;
   }
   if (r) return r;
   PF_CHECK_LAUNCH();
-  if (G > 0) {
-    norm_bwd_finish_kernel<<<(N + 31) / 32, 1024, 0, st>>>((const float*)scratch, (float*)dgamma,
-                                                           (float*)dbeta, G, N, accumulate);
-    PF_CHECK_LAUNCH();
-  }
+  norm_bwd_finish_kernel<<<(N + 31) / 32, 1024, 0, st>>>((const float*)scratch, (float*)dgamma,
+                                                         (float*)dbeta, G, N, accumulate);
+  PF_CHECK_LAUNCH();
   return 0;
 }
 

@@ -262,3 +262,11 @@ def test_norm_backward_tiles(rows, N, rms):
     close(dw, wants[1] + 1, 1e-5)
     if not rms:
         close(db, wants[2] + 1, 1e-5)
+
+
+@pytest.mark.parametrize("rms", [False, True])
+@pytest.mark.parametrize("rows,N", [(1, 4096), (2, 2056), (3, 3072), (591, 3080), (2500, 4096)])
+def test_norm_backward_wide_rows(rows, N, rms):
+    """Rows that one CTA holds two at a time: fewer batches than the ring has stages, an odd last
+    row, threads without columns, several batches per CTA."""
+    test_norm_backward_tiles(rows, N, rms)
