@@ -84,6 +84,8 @@ PF_DECL int pf_embed_bwd(const void* dout, const void* ids, void* dtable_f32, lo
 PF_DECL int pf_rope(const void* x, void* out, const void* cos_t, const void* sin_t, long long B,
                     int S, int H, int D, long long stride_b, long long stride_s,
                     long long stride_h, int inverse, int dtype, int sm_count, void* stream);
+PF_DECL int pf_rope_qkv(const void* x, void* out, const void* cos_t, const void* sin_t,
+                        long long rows, int S, int H, int D, int inverse, int dtype, void* stream);
 
 // ---- attn_sm100.cu : flash attention on tcgen05 (strides in elements: batch, seq, head)
 PF_DECL int pf_attn_fwd(const void* q, const void* k, const void* v, void* o, void* lse, int B,

@@ -304,6 +304,52 @@ rope_vec_kernel(const T* __restrict__ x, T* __restrict__ out, const float* __res
   }
 }
 
+// The same rotation over a whole fused projection [rows = B*S][3][H][D]: slices 0 and 1 (queries, keys)
+// are rotated, slice 2 is copied, so that one kernel per direction takes the place of two rotations
+// and, in the backward, of the fills, strided copies and additions that join the gradients of three
+// slices.  One CTA per row; bound by HBM: the tensor is read and written once.  [1, 2048, 3, 32, 128]
+// bf16: 18 us in a decoder layer (26 with L2 flushed) and as much backward, where 34 us went into
+// rotations and 137 into joining slices.
+template <typename T>
+__global__ void __launch_bounds__(256)
+rope_qkv_kernel(const T* __restrict__ x, T* __restrict__ out, const float* __restrict__ cos_t,
+                const float* __restrict__ sin_t, int S, int H, int D, int inverse) {
+  const int half = D / 2, hv = half / 8;
+  const long long row = blockIdx.x;
+  const T* src = x + row * 3 * H * D;
+  T* dst = out + row * 3 * H * D;
+  const float* ct = cos_t + (row % S) * half;
+  const float* st = sin_t + (row % S) * half;
+  const int n_rot = 2 * H * hv;
+  for (int i = threadIdx.x; i < n_rot; i += 256) {
+    const int jh = i / hv, v = i - jh * hv, off = jh * D + v * 8;
+    const uint4 u1 = *reinterpret_cast<const uint4*>(src + off);
+    const uint4 u2 = *reinterpret_cast<const uint4*>(src + off + half);
+    const float4* cp = reinterpret_cast<const float4*>(ct + v * 8);
+    const float4* sp = reinterpret_cast<const float4*>(st + v * 8);
+    const float4 c0 = __ldg(cp), c1 = __ldg(cp + 1), s0 = __ldg(sp), s1 = __ldg(sp + 1);
+    const float c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+    const float sn[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+    const T* e1 = reinterpret_cast<const T*>(&u1);
+    const T* e2 = reinterpret_cast<const T*>(&u2);
+    uint4 o1, o2;
+    T* q1 = reinterpret_cast<T*>(&o1);
+    T* q2 = reinterpret_cast<T*>(&o2);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float x1 = to_f32<T>(e1[j]), x2 = to_f32<T>(e2[j]);
+      const float sj = inverse ? -sn[j] : sn[j];
+      q1[j] = from_f32<T>(x1 * c[j] - x2 * sj);
+      q2[j] = from_f32<T>(x2 * c[j] + x1 * sj);
+    }
+    *reinterpret_cast<uint4*>(dst + off) = o1;
+    *reinterpret_cast<uint4*>(dst + off + half) = o2;
+  }
+  const uint4* vs = reinterpret_cast<const uint4*>(src + 2 * H * D);
+  uint4* vd = reinterpret_cast<uint4*>(dst + 2 * H * D);
+  for (int i = threadIdx.x; i < H * D / 8; i += 256) vd[i] = vs[i];
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256)
 rope_kernel(const T* __restrict__ x, T* __restrict__ out, const float* __restrict__ cos_t,
@@ -487,6 +533,27 @@ PF_API int pf_embed_bwd(const void* dout, const void* ids, void* dtable_f32, lon
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   PF_DISPATCH3(dtype, (embed_bwd_kernel<T><<<(unsigned)tokens, 256, 0, st>>>(
       (const T*)dout, (const long long*)ids, (float*)dtable_f32, D, vocab)));
+  PF_CHECK_LAUNCH();
+  return 0;
+}
+
+// x, out: [rows = B*S][3][H][D] 16-bit, contiguous; cos / sin fp32 [S, D/2].  Needs D a multiple of 16
+// and 16-byte aligned pointers (-2 otherwise).
+PF_API int pf_rope_qkv(const void* x, void* out, const void* cos_t, const void* sin_t,
+                       long long rows, int S, int H, int D, int inverse, int dtype, void* stream) {
+  if (rows <= 0) return 0;
+  if (dtype != PF_F16 && dtype != PF_BF16) return -1;
+  if (D % 16 || rows > 0x7fffffffll || (reinterpret_cast<uintptr_t>(x) & 15) ||
+      (reinterpret_cast<uintptr_t>(out) & 15) || (reinterpret_cast<uintptr_t>(cos_t) & 15) ||
+      (reinterpret_cast<uintptr_t>(sin_t) & 15))
+    return -2;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  if (dtype == PF_F16)
+    rope_qkv_kernel<__half><<<(unsigned)rows, 256, 0, st>>>((const __half*)x, (__half*)out,
+        (const float*)cos_t, (const float*)sin_t, S, H, D, inverse);
+  else
+    rope_qkv_kernel<__nv_bfloat16><<<(unsigned)rows, 256, 0, st>>>((const __nv_bfloat16*)x,
+        (__nv_bfloat16*)out, (const float*)cos_t, (const float*)sin_t, S, H, D, inverse);
   PF_CHECK_LAUNCH();
   return 0;
 }

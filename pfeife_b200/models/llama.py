@@ -65,9 +65,7 @@ class LlamaBlock(nn.Module):
         else:
             y, x = ops.rms_norm(delta, self.input_norm, self.eps, residual=x)
         qkv = ops.linear(y, self.qkv.weight).view(B, S, 3, H, d // H)
-        q = ops.rope(qkv[:, :, 0], cos, sin)
-        k = ops.rope(qkv[:, :, 1], cos, sin)
-        a = ops.attention(q, k, qkv[:, :, 2], causal=True).view(B, S, d)
+        a = ops.attention_qkv(ops.rope_qkv(qkv, cos, sin), causal=True).view(B, S, d)
         delta = ops.linear(a, self.o_proj.weight)
         y, x = ops.rms_norm(delta, self.post_norm, self.eps, residual=x)
         g = ops.swiglu(ops.linear(y, self.gate_up.weight))

@@ -1009,6 +1009,35 @@ def rope(x: Tensor, cos: Tensor, sin: Tensor) -> Tensor:
     return _call(rope_apply, x, cos, sin, False)
 
 
+@_custom_op("pfeife::rope_qkv_apply")
+def rope_qkv_apply(qkv: Tensor, cos: Tensor, sin: Tensor, inverse: bool) -> Tensor:
+    """qkv [B, S, 3, H, D] -> a contiguous tensor with the queries and keys rotated."""
+    if _native(qkv):
+        qkv = qkv.contiguous()
+        if kx.rope_qkv_supported(qkv):
+            return kx.rope_qkv(qkv, cos.float(), sin.float(), inverse)
+    q, k = (rope_apply.plain(qkv[:, :, j], cos, sin, inverse) for j in (0, 1))
+    return torch.stack([q, k, qkv[:, :, 2]], dim=2)
+
+
+@rope_qkv_apply.register_fake
+def _(qkv, cos, sin, inverse):
+    return qkv.new_empty(qkv.shape)
+
+
+def _rope_qkv_backward(ctx, dy):
+    cos, sin = ctx.saved_tensors
+    return _bwd(ctx, rope_qkv_apply)(dy.contiguous(), cos, sin, not ctx.inverse), None, None, None
+
+
+_autograd(rope_qkv_apply, 1, _rope_qkv_backward, setup=_rope_setup)
+
+
+def rope_qkv(qkv: Tensor, cos: Tensor, sin: Tensor) -> Tensor:
+    """``rope`` of the queries and keys of a fused projection [B, S, 3, H, D], for ``attention_qkv``."""
+    return _call(rope_qkv_apply, qkv, cos, sin, False)
+
+
 def rope_tables(seq_len: int, head_dim: int, theta: float = 10000.0, device=None
                 ) -> Tuple[Tensor, Tensor]:
     inv = 1.0 / (theta ** (torch.arange(0, head_dim, 2, device=device, dtype=torch.float32)

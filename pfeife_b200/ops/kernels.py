@@ -407,6 +407,25 @@ def rope(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, inverse: bool = 
     return out
 
 
+def rope_qkv_supported(x: torch.Tensor) -> bool:
+    """True when the kernel over a whole fused projection covers x [B, S, 3, H, D]."""
+    return (x.dtype in (torch.float16, torch.bfloat16) and x.shape[-1] % 16 == 0
+            and x.is_contiguous() and x.data_ptr() % 16 == 0)
+
+
+def rope_qkv(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, inverse: bool = False
+             ) -> torch.Tensor:
+    """x: [B, S, 3, H, D] contiguous -> the same with slices 0 and 1 rotated; cos/sin: fp32 [S, D/2]."""
+    L = _lib.lib()
+    B, S, three, H, D = x.shape
+    assert three == 3 and x.is_contiguous() and cos.shape == sin.shape == (S, D // 2)
+    out = torch.empty_like(x)
+    fix = lambda t: t if t.is_contiguous() and t.data_ptr() % 16 == 0 else t.clone()
+    check(L.pf_rope_qkv(ptr(x), ptr(out), ptr(fix(cos)), ptr(fix(sin)), c_ll(B * S), S, H, D,
+                        int(inverse), dt(x.dtype), stream()), "pf_rope_qkv")
+    return out
+
+
 # --------------------------------------------------------------------------- attention
 def attention_supported(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> bool:
     """True when the native flash-attention kernels cover this problem."""

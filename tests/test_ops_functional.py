@@ -215,3 +215,22 @@ def test_registered_param_accumulates_into_bucket(device):
         _check(bucket.view(48, 64), ref, tol)
     finally:
         ops.unregister_params()
+
+
+@pytest.mark.parametrize("device", DEVICES)
+@pytest.mark.parametrize("B,S,H,D", [(1, 1, 1, 16), (2, 9, 3, 32), (1, 33, 5, 88), (2, 5, 2, 128)])
+def test_rope_of_a_fused_projection(device, B, S, H, D):
+    """The same values and gradients, bit for bit, as rotating the slices one by one (a head dim of 88
+    or a view takes the route over the slices)."""
+    torch.manual_seed(4)
+    dt = torch.bfloat16 if device == "cuda" else torch.float32
+    cos, sin = ops.rope_tables(S, D, device=device)
+    for strided in (False, True):
+        base = torch.randn(B, S, 3, H, D + 8 * strided, device=device, dtype=dt)
+        a = base[..., :D].detach().requires_grad_()
+        b = base[..., :D].detach().clone().requires_grad_()
+        y = ops.rope_qkv(a, cos, sin)
+        r = torch.stack([ops.rope(b[:, :, 0], cos, sin), ops.rope(b[:, :, 1], cos, sin), b[:, :, 2]], 2)
+        g = torch.randn(B, S, 3, H, D, device=device, dtype=dt)
+        assert torch.equal(y, r)
+        assert torch.equal(torch.autograd.grad(y, a, g)[0], torch.autograd.grad(r, b, g)[0])
