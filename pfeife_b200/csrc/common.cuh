@@ -499,32 +499,72 @@ __device__ __forceinline__ float dgelu_erf(float x) {
   const float pdf = 0.3989422804014327f * __expf(-0.5f * x * x);
   return cdf + x * pdf;
 }
-// erf-GELU and its derivative for fused GEMM epilogues: erf through the five-term rational
-// approximation 1 - (a1 t + ... + a5 t^5) exp(-z^2), t = 1 / (1 + p z) (absolute error
-// 1.5e-7), which costs two special-function instructions and about a dozen FMAs per value;
-// gelu and gelu' are exact to 4e-7 absolute.  Phi(x) = y for x < 0 and 1 - y for x >= 0 with
-// y = 0.5 poly exp(-x^2 / 2).
-__device__ __forceinline__ float gelu_half_tail(float ax, float* e_out) {
-  const float a = ax * 0.70710678118654752f;
-  const float t = __fdividef(1.0f, fmaf(0.3275911f, a, 1.0f));
-  float poly = fmaf(t, 0.5f * 1.061405429f, 0.5f * -1.453152027f);
-  poly = fmaf(t, poly, 0.5f * 1.421413741f);
-  poly = fmaf(t, poly, 0.5f * -0.284496736f);
-  poly = fmaf(t, poly, 0.5f * 0.254829592f);
-  const float e = exp2f(-(a * a) * 1.4426950408889634f);
-  *e_out = e;
-  return poly * t * e;
+// pairs of fp32 values in one 64-bit register: one issue slot for two operations
+__device__ __forceinline__ uint64_t f2_pack(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
 }
-__device__ __forceinline__ float gelu_erf_fast(float x) {
-  float e;
-  const float xy = x * gelu_half_tail(fabsf(x), &e);
-  return x >= 0.f ? x - xy : xy;
+__device__ __forceinline__ void f2_unpack(uint64_t v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
 }
-__device__ __forceinline__ float dgelu_erf_fast(float x) {
-  float e;
-  const float y = gelu_half_tail(fabsf(x), &e);
-  const float cdf = x >= 0.f ? 1.0f - y : y;
-  return fmaf(x * 0.3989422804014327f, e, cdf);
+// two fp32 fused multiply-adds in one issue slot
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
+__device__ __forceinline__ float rcp_approx(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// erf-GELU and its derivative for fused GEMM epilogues, two values at a time: erf through the
+// five-term rational approximation 1 - (a1 t + ... + a5 t^5) exp(-z^2), t = 1 / (1 + p z)
+// (Abramowitz and Stegun 7.1.26, absolute error 1.5e-7), which costs two special-function
+// instructions per value and nine packed ones per pair; gelu and gelu' are exact to 4e-7 absolute.
+// With y = 0.5 poly exp(-x^2 / 2) >= 0, Phi(x) = y for x < 0 and 1 - y for x >= 0, so that
+// gelu(x) = max(x, 0) - |x| y and Phi(x) = 0.5 + sign(x) (0.5 - y).
+// Returns -y for |x| (`ax`) and leaves exp(-x^2 / 2) in `e`.
+__device__ __forceinline__ uint64_t gelu_neg_tail2(uint64_t ax, uint64_t& e) {
+  float d0, d1, q0, q1;
+  f2_unpack(fma2(ax, f2_pack(0.23164188f, 0.23164188f), f2_pack(1.f, 1.f)), d0, d1);  // p / sqrt(2)
+  f2_unpack(mul2(mul2(ax, ax), f2_pack(-0.72134752f, -0.72134752f)), q0, q1);    // -log2(e) / 2
+  const uint64_t t = f2_pack(rcp_approx(d0), rcp_approx(d1));
+  e = f2_pack(exp2f(q0), exp2f(q1));
+  uint64_t poly = fma2(t, f2_pack(-0.5f * 1.061405429f, -0.5f * 1.061405429f),
+                       f2_pack(0.5f * 1.453152027f, 0.5f * 1.453152027f));
+  poly = fma2(t, poly, f2_pack(-0.5f * 1.421413741f, -0.5f * 1.421413741f));
+  poly = fma2(t, poly, f2_pack(0.5f * 0.284496736f, 0.5f * 0.284496736f));
+  poly = fma2(t, poly, f2_pack(-0.5f * 0.254829592f, -0.5f * 0.254829592f));
+  return mul2(mul2(poly, t), e);
+}
+// (a, b) -> gelu of both
+__device__ __forceinline__ void gelu_erf_fast2(float& a, float& b) {
+  uint64_t e;
+  const uint64_t ax = f2_pack(fabsf(a), fabsf(b));
+  f2_unpack(fma2(ax, gelu_neg_tail2(ax, e), f2_pack(fmaxf(a, 0.f), fmaxf(b, 0.f))), a, b);
+}
+// (a, b) *= gelu' of (x, y)
+__device__ __forceinline__ void dgelu_erf_fast2(float& a, float& b, float x, float y) {
+  uint64_t e;
+  const uint64_t ny = gelu_neg_tail2(f2_pack(fabsf(x), fabsf(y)), e);
+  float h0, h1;
+  f2_unpack(add2(ny, f2_pack(0.5f, 0.5f)), h0, h1);                 // 0.5 - y, not negative
+  const uint64_t cdf = add2(f2_pack(copysignf(h0, x), copysignf(h1, y)), f2_pack(0.5f, 0.5f));
+  const uint64_t pdf_x = mul2(f2_pack(x, y), f2_pack(0.3989422804014327f, 0.3989422804014327f));
+  f2_unpack(mul2(f2_pack(a, b), fma2(pdf_x, e, cdf)), a, b);
 }
 __device__ __forceinline__ float gelu_tanh(float x) {
   const float u = 0.7978845608028654f * (x + 0.044715f * x * x * x);

@@ -15,7 +15,10 @@
 // Role layout of the 320-thread CTA: warp 0 = TMA producer, warp 1 = TMEM owner and MMA
 // issuer (one elected thread each), warps 2..9 = epilogue (one accumulator row per thread; two warps
 // share a TMEM lane quadrant and split the tile's columns, which halves the epilogue latency per
-// tile);
+// tile).  Over 6144 x 6144 outputs the epilogue takes 36 us plain, 68 with GELU and its saved
+// pre-activations and 65 with GELU' (70, 74 and 80 with one value at a time and the saved values
+// fetched when they are needed), so that at K = 1408, whose products take 71 us, it still shows:
+// ViT-g/14's first layer 101 -> 94 us, its input gradient 99 -> 90;
 // the instantiation that fuses an all-gather of B adds two warps that copy the remote rows.
 #include <cstring>
 #include "common.cuh"
@@ -500,17 +503,30 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
     int staged = 0;        // chunks handed to the TMA so far (saturates at 2)
     const bool vec = p.vec_ok != 0;
     const bool tma_out = p.tma_store != 0;
+    // saved pre-activations (16-bit) are requested a chunk of 32 columns ahead
+    const bool dgelu = p.epilogue == EPI_DGELU || p.epilogue == EPI_DGELU_TANH;
+    const bool aux_ahead = sizeof(OutT) == 2 && vec;
+    uint4 aux_q[4];
+    auto fetch_aux = [&](int r, int col) {
+      if (aux_ahead && col + 32 <= p.N) {
+        const uint4* src = reinterpret_cast<const uint4*>(AUX + (long long)r * p.ldaux + col);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) aux_q[i] = __ldg(src + i);
+      }
+    };
     const bool bias_vec = p.bias && p.bias_dtype == PF_F32 &&
                           (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0;
     for (int round = 0, item = item_of(0); item < num_tiles && ok; item = item_of(++round)) {
       const int tile = item % num_mn;
       const int m0 = (tile % num_m) * BMT + int(cta_rank) * GEMM_BM;
       const int n0 = ((tile / num_m + n_rot) % num_n) * BNT;
+      const int row = m0 + row_in_tile;
+      const bool row_ok = row < p.M;
+      // the first saved values of this tile travel while its products are computed
+      if (dgelu && row_ok) fetch_aux(row, n0 + c_begin);
       ok = mbar_wait(&tmem_full[acc], acc_phase, p.status, PF_ERR_TIMEOUT_TMEM_FULL);
       if (!ok) break;
       tc_fence_after();
-      const int row = m0 + row_in_tile;
-      const bool row_ok = row < p.M;
       const uint32_t t_row = tmem_base + (uint32_t(quad * 32) << 16) + acc * BNT;
       uint32_t raw[32];
       if (n0 + c_begin < p.N) tmem_ld32(t_row + c_begin, raw);   // uniform across the warp
@@ -563,7 +579,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
           }
           if (p.epilogue == EPI_GELU) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = gelu_erf_fast(v[i]);
+            for (int i = 0; i < 32; i += 2) gelu_erf_fast2(v[i], v[i + 1]);
           } else if (p.epilogue == EPI_GELU_TANH) {
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[i] = gelu_tanh(v[i]);
@@ -571,12 +587,22 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[i] = silu(v[i]);
           }
-        } else if ((p.epilogue == EPI_DGELU || p.epilogue == EPI_DGELU_TANH) && row_ok) {
+        } else if (dgelu && row_ok) {
           float z[32];
-          load_row32<OutT>(AUX + (long long)row * p.ldaux + col, vec, nvalid, z);
+          if (aux_ahead && nvalid == 32) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const OutT* e = reinterpret_cast<const OutT*>(&aux_q[i]);
+#pragma unroll
+              for (int j = 0; j < 8; ++j) z[i * 8 + j] = to_f32<OutT>(e[j]);
+            }
+          } else {
+            load_row32<OutT>(AUX + (long long)row * p.ldaux + col, vec, nvalid, z);
+          }
+          if (c + 32 < c_end) fetch_aux(row, col + 32);
           if (p.epilogue == EPI_DGELU) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] *= dgelu_erf_fast(z[i]);
+            for (int i = 0; i < 32; i += 2) dgelu_erf_fast2(v[i], v[i + 1], z[i], z[i + 1]);
           } else {
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[i] *= dgelu_tanh(z[i]);
