@@ -829,6 +829,9 @@ PF_API int pf_gemm(const void* A, const void* B, void* C, int M, int N, int K, l
   // the split reduction (tests, benches)
   const int tn = tile_n & 1023;
   if (sm_count <= 0) sm_count = 148;
+  const bool one_round =
+      (long long)((M + 127) / 128) * ((N + 127) / 128) <= sm_count &&
+      !(out_dtype == PF_F32 && (accumulate || g_conv.on == 2));
   bool pair = false;
   if (g_gather.world <= 1 && !(tile_n & 4096) && sm_count >= 2) {
     if (tile_n & 2048) {
@@ -843,7 +846,11 @@ PF_API int pf_gemm(const void* A, const void* B, void* C, int M, int N, int K, l
       const long long t1 = (long long)((M + 127) / 128) * ((N + 255) / 256);
       const long long w2 = (t2 + sm_count / 2 - 1) / (sm_count / 2);
       const long long w1 = (t1 + sm_count - 1) / sm_count;
-      pair = 93 * w2 <= 100 * w1;
+      // Where 128 x 128 tiles all run at once, the time is that of one tile, and the small ones are
+      // the soonest done: 1024 x 768 x 3072 24.2 us as pairs, 19.5 as 128 x 128; 300 x 4096 x 1024
+      // 20.1 and 14.0; 2048 x 1024 x 4096 28.3 and 24.2; 788 x 768 x 192 16.0 and 10.6.
+      // (Outputs whose reduction may be split fill the SMs that way, with the large tiles.)
+      pair = !one_round && 93 * w2 <= 100 * w1;
     }
   }
   int bn_auto = N <= 128 ? 128 : 256;
@@ -853,7 +860,7 @@ PF_API int pf_gemm(const void* A, const void* B, void* C, int M, int N, int K, l
     const long long th = (long long)((M + 127) / 128) * ((N + 127) / 128);
     const long long w1 = (t1 + sm_count - 1) / sm_count;
     const long long wh = (th + sm_count - 1) / sm_count;
-    if (11 * wh < 20 * w1) bn_auto = 128;
+    if (11 * wh < 20 * w1 || one_round) bn_auto = 128;
   }
   const int BN = pair ? 128 : (tn == 128 || tn == 256) ? tn : bn_auto;
 

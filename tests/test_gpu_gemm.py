@@ -166,3 +166,16 @@ def test_gather_rows_one_device():
     kx.gather_rows(copies[rank], _table([c.data_ptr() for c in copies]), world, rank, ends)
     torch.cuda.synchronize()
     assert torch.equal(copies[rank], w)
+
+
+@pytest.mark.parametrize("M,N", [(4736, 512), (4737, 512), (129, 136), (136, 4096)])
+@pytest.mark.parametrize("K", [72, 1088])
+def test_gemm_around_one_round_of_small_tiles(M, N, K):
+    """Sizes on both sides of the line up to which 128 x 128 tiles all run at once (148 SMs)."""
+    from pfeife_b200.ops import kernels as kx
+    a, b = _mk(M, N, K, False, False, torch.bfloat16)
+    out = kx.gemm(a, b, out_dtype=torch.float32)
+    ref = a.double() @ b.double().t()
+    kx.check_status()
+    # products of 16-bit values are exact in fp32; K fp32 additions in some order
+    assert ((out - ref).norm() / ref.norm()).item() < K * 2.0 ** -24
