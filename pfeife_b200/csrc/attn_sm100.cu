@@ -24,9 +24,11 @@
 // 8 x head dim cycles of tensor core (512 at head dim 64; at 128 both take 1024).  Two tiles in
 // flight keep one tile's products under the other's exponentials.
 // Measured (B200, CUDA events, L2 flushed), against one query tile per CTA with P in shared
-// memory: [4, 4096, 10, 64] 402 -> 346 us (310 since one elected thread issues the products), causal [1, 2048, 32, 128] 87 -> 59,
-// [2, 2048, 16, 128] 114 -> 96, causal [6, 1782, 21, 32] 200 -> 117, 77 keys [4, 1024, 20, 64]
-// 32 -> 22, [24, 257, 16, 88] 62 -> 58.
+// memory: [4, 4096, 10, 64] 402 -> 273 us, causal [1, 2048, 32, 128] 87 -> 51,
+// [2, 2048, 16, 128] 114 -> 82, causal [6, 1782, 21, 32] 200 -> 104, 77 keys [4, 1024, 20, 64]
+// 32 -> 20, [24, 257, 16, 88] 62 -> 52.  Steps on the way at [4, 4096, 10, 64]: 346 with two query
+// tiles per CTA, 305 with one elected thread issuing the products, 292 with the maximum found in the
+// pass over the exponentials, 273 with the pairs beyond whole rounds split.
 // TMEM (512 columns): S_0, S_1 128 each, O_0, O_1 one head dim each.  Up to head dim 64 P_0, P_1
 // have 64 columns of their own, so S of the next key tile is issued as soon as this one's scores
 // are in registers; above, P_t takes the columns of S_t and the next S_t waits until P_t V has
@@ -42,6 +44,7 @@
 namespace pf {
 
 constexpr int ATT_TAIL_MAX = 4;      // leftover rows handled on CUDA cores
+constexpr int ATT_TWO_LAUNCH_TILES = 12;   // key tiles from which a second launch pays (see FwdItem)
 constexpr int ATT_TAIL_SEQ_MAX = 2048;  // longest other dimension the CUDA-core paths stage in smem
 
 struct AttnParams {
@@ -55,6 +58,7 @@ struct AttnParams {
   int q_rows;           // query rows of the tensor-core kernel; the others are leftover rows
   int q_pairs;          // pairs of query tiles per head: ceil(q_rows / 256)
   int n_pair;           // the first items are pairs, the others split tiles (see FwdItem)
+  int item0;            // first item of this launch
   int q_tail;           // leftover rows
   // raw views for the leftover rows (element strides: batch, seq, head)
   const void* q; const void* k; const void* v;
@@ -235,6 +239,7 @@ __device__ __forceinline__ FwdItem fwd_item(const AttnParams& p, int w) {
 }
 // item `w` of a kernel whose items from n_pair on are split tiles (`split` says whether this one is)
 __device__ __forceinline__ FwdItem fwd_item(const AttnParams& p, int w, bool& split) {
+  w += p.item0;
   split = w >= p.n_pair;
   if (!split) return fwd_item(p, w);
   const int u = w - p.n_pair, t = u & 1;
@@ -252,22 +257,35 @@ __device__ __forceinline__ int fwd_index(int r) {
   return r * (int)gridDim.x + slot;
 }
 
-// Probabilities of one row, packed to 16 bits; returns their fp32 sum (of the unrounded values).
-template <typename T, bool MASKED>
-__device__ __forceinline__ float probs(const uint32_t (&s)[4][32], uint32_t (&pk)[4][16], float c2,
-                                       float m_sub, int n_chunks, int lim) {
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+// Probabilities of one row under the maximum `m_sub`, packed to 16 bits and stored to the columns of P
+// chunk by chunk; returns their fp32 sum (of the unrounded values).  With MAX the largest score is
+// found on the way: its comparisons go to another unit than the exponentials that bound the loop.
+template <typename T, bool MASKED, bool MAX>
+__device__ __forceinline__ float probs(const uint32_t (&s)[4][32], uint32_t t_p, float c2, float m_sub,
+                                       int n_chunks, int lim, float& mx) {
   const uint64_t c2v = f2_pack(c2, c2), nm = f2_pack(-m_sub, -m_sub);
   uint64_t r01 = 0, r23 = 0;                  // pairs of fp32 sums
+  float m0 = -INFINITY, m1 = -INFINITY;
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
     if (!MASKED || c < n_chunks) {
+      uint32_t pk[16];
 #pragma unroll
       for (int i = 0; i < 32; i += 4) {
-        float e[4];
-        f2_unpack(fma2(f2_pack(__uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1])), c2v, nm),
-                  e[0], e[1]);
-        f2_unpack(fma2(f2_pack(__uint_as_float(s[c][i + 2]), __uint_as_float(s[c][i + 3])), c2v,
-                       nm), e[2], e[3]);
+        float x[4], e[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) x[u] = __uint_as_float(s[c][i + u]);
+        if (MAX) {
+          m0 = max3(m0, x[0], x[1]);
+          m1 = max3(m1, x[2], x[3]);
+        }
+        f2_unpack(fma2(f2_pack(x[0], x[1]), c2v, nm), e[0], e[1]);
+        f2_unpack(fma2(f2_pack(x[2], x[3]), c2v, nm), e[2], e[3]);
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           e[u] = exp2f(e[u]);
@@ -275,11 +293,13 @@ __device__ __forceinline__ float probs(const uint32_t (&s)[4][32], uint32_t (&pk
         }
         r01 = add2(r01, f2_pack(e[0], e[1]));
         r23 = add2(r23, f2_pack(e[2], e[3]));
-        pk[c][i / 2] = pack2<T>(e[0], e[1]);
-        pk[c][i / 2 + 1] = pack2<T>(e[2], e[3]);
+        pk[i / 2] = pack2<T>(e[0], e[1]);
+        pk[i / 2 + 1] = pack2<T>(e[2], e[3]);
       }
+      tmem_st16(t_p + c * 16, pk);
     }
   }
+  if (MAX) mx = fmaxf(m0, m1);
   float a, b, d, e;
   f2_unpack(r01, a, b);
   f2_unpack(r23, d, e);
@@ -493,15 +513,18 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
       // a warp whose rows all lie beyond the last query only keeps the barriers going
       const bool warp_live = q0 + quad * 32 < p.Sq;
       float m_used = -INFINITY, l = 0.f;
+      bool s_seen = false;                   // the scores of this step are known to be there
       for (int j = 0; j < n_tiles && ok; ++j, ++cnt) {
         const int k0 = (split ? 2 * j + t : j) * ATT_BN;
         const int rem = min(ATT_BN, p.Sk - k0);
         const int n_chunks = ((rem + 15) / 16 * 16 + 31) / 32;
         // a tile needs masks when it is ragged or crosses the causal diagonal of this q tile
         const bool masked = rem < ATT_BN || (p.causal && k0 + ATT_BN - 1 > q0 + shift);
-        ok = mbar_wait(&s_full[t], cnt & 1, p.status, PF_ERR_TIMEOUT_TMEM_FULL);
+        if (!s_seen) ok = mbar_wait(&s_full[t], cnt & 1, p.status, PF_ERR_TIMEOUT_TMEM_FULL);
         if (!ok) break;
         tc_fence_after();
+        // looked at here, needed below: even a wait that is satisfied takes some 130 cycles
+        const bool pv_seen = C::ALIAS_P || j == 0 || mbar_test(&pv_done[t], (cnt - 1) & 1);
         uint32_t s[4][32];
 #pragma unroll
         for (int c = 0; c < 4; ++c) tmem_ld32(t_s + c * 32, s[c]);
@@ -514,23 +537,37 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
         }
         // keys of this tile below `lim` are visible to this row
         const int lim = p.causal ? min(p.Sk, qi + shift + 1) - k0 : p.Sk - k0;
-        uint32_t pk[4][16];
-        float alpha = 1.f;
+        // P in columns of its own: the previous P V must have read its probabilities before they are
+        // overwritten (that product ran while the scores were fetched), and O must hold every
+        // earlier tile before it is rescaled.  The wait also keeps a warp without live rows from
+        // arriving twice on one phase of p_full.  With P in the columns of S the scores were only
+        // computed after that product.
+        if (!pv_seen) ok = mbar_wait(&pv_done[t], (cnt - 1) & 1, p.status, PF_ERR_TIMEOUT_TMEM_FULL);
+        if (!ok) break;
+        tc_fence_after();
         if (warp_live) {
-          float mx = -INFINITY;
-          if (!masked) {
-            float m0 = -INFINITY, m1 = -INFINITY, m2 = -INFINITY, m3 = -INFINITY;
+          // The maximum in use only moves when the row's grew by more than 2^8, which is rare after
+          // the first tiles: the probabilities are computed under the old one while the new maximum
+          // is looked for, and once more if a row of the warp turns out to need it.
+          // (Two passes, maximum first, took 490 cycles of the 3470 of a step at head dim 64.)
+          float mx = -INFINITY, rs = 0.f;
+          bool again = j == 0 || masked;
+          if (!again) {
+            rs = probs<T, false, true>(s, t_p, c2, (m_used == -INFINITY) ? 0.f : m_used, 4, ATT_BN, mx);
+            mx *= c2;                                 // c2 > 0; -inf stays -inf
+            again = __any_sync(0xffffffffu, mx > m_used + 8.f);
+            if (again) tmem_st_wait();
+          } else if (!masked) {
+            float m0 = -INFINITY, m1 = -INFINITY;
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
 #pragma unroll
               for (int i = 0; i < 32; i += 4) {
-                m0 = fmaxf(m0, __uint_as_float(s[c][i]));
-                m1 = fmaxf(m1, __uint_as_float(s[c][i + 1]));
-                m2 = fmaxf(m2, __uint_as_float(s[c][i + 2]));
-                m3 = fmaxf(m3, __uint_as_float(s[c][i + 3]));
+                m0 = max3(m0, __uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1]));
+                m1 = max3(m1, __uint_as_float(s[c][i + 2]), __uint_as_float(s[c][i + 3]));
               }
             }
-            mx = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
+            mx = fmaxf(m0, m1) * c2;
           } else {
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
@@ -540,42 +577,34 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
                   if (c * 32 + i < lim) mx = fmaxf(mx, __uint_as_float(s[c][i]));
               }
             }
+            mx *= c2;
           }
-          mx *= c2;                                   // c2 > 0; -inf stays -inf
-          if (j == 0) {
-            m_used = mx;
-          } else if (mx > m_used + 8.f) {             // also true when m_used is still -inf
-            alpha = exp2f(m_used - mx);               // exp2(-inf) = 0: nothing had accumulated
-            m_used = mx;
-          }
-          const float m_sub = (m_used == -INFINITY) ? 0.f : m_used;
-          const float rs = masked ? probs<T, true>(s, pk, c2, m_sub, n_chunks, lim)
-                                  : probs<T, false>(s, pk, c2, m_sub, 4, ATT_BN);
-          l = l * alpha + rs;
-        }
-        // The previous P V must have read its probabilities, and O must hold every earlier tile
-        // before it is rescaled (a short wait: that product ran under the work above).  It also
-        // keeps a warp without live rows from arriving twice on one phase of p_full.
-        if (j > 0) {
-          ok = mbar_wait(&pv_done[t], (cnt - 1) & 1, p.status, PF_ERR_TIMEOUT_TMEM_FULL);
-          if (!ok) break;
-          tc_fence_after();
-        }
-        if (warp_live) {
-          if (j > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
+          if (again) {
+            float alpha = 1.f;
+            if (j == 0) {
+              m_used = mx;
+            } else if (mx > m_used + 8.f) {           // also true when m_used is still -inf
+              alpha = exp2f(m_used - mx);             // exp2(-inf) = 0: nothing had accumulated
+              m_used = mx;
+            }
+            const float m_sub = (m_used == -INFINITY) ? 0.f : m_used;
+            rs = masked ? probs<T, true, false>(s, t_p, c2, m_sub, n_chunks, lim, mx)
+                        : probs<T, false, false>(s, t_p, c2, m_sub, 4, ATT_BN, mx);
+            if (j > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
+              l *= alpha;
 #pragma unroll
-            for (int c = 0; c < DP / 32; ++c) {
-              uint32_t o[32];
-              tmem_ld32(t_o + c * 32, o);
-              tmem_ld_wait_for(o);
+              for (int c = 0; c < DP / 32; ++c) {
+                uint32_t o[32];
+                tmem_ld32(t_o + c * 32, o);
+                tmem_ld_wait_for(o);
 #pragma unroll
-              for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-              tmem_st32(t_o + c * 32, o);
+                for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                tmem_st32(t_o + c * 32, o);
+              }
             }
           }
-#pragma unroll
-          for (int c = 0; c < 4; ++c)
-            if (c < n_chunks) tmem_st16(t_p + c * 16, pk[c]);
+          l += rs;
+          if (!C::ALIAS_P) s_seen = j + 1 < n_tiles && mbar_test(&s_full[t], (cnt + 1) & 1);
           tmem_st_wait();
         }
         tc_fence_before();
@@ -650,18 +679,26 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 
 template <typename T, int DP>
 static int launch_fwd_ws(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
-                         const AttnParams& p, cudaStream_t st) {
+                         const AttnParams& p, bool two_launches, cudaStream_t st) {
   using C = FwdCfg<DP>;
-  const int pairs = p.q_pairs * p.H * p.B, n_items = p.n_pair + 2 * (pairs - p.n_pair);
-  const int sms = attn_sm_count();
-  const bool split = p.n_pair < pairs;
-  auto kern = split ? attn_fwd_ws_kernel<T, DP, true> : attn_fwd_ws_kernel<T, DP, false>;
+  const int pairs = p.q_pairs * p.H * p.B, tiles = 2 * (pairs - p.n_pair);
   static bool done[2][64] = {};
-  int r = set_smem(kern, C::SMEM, done[split]);
-  if (r) return r;
-  if (n_items > 0) {
-    kern<<<n_items < sms ? n_items : sms, C::THREADS, C::SMEM, st>>>(tq, tk, tv, p, n_items);
+  auto run = [&](const AttnParams& q, bool split, int n) -> int {
+    if (n <= 0) return 0;
+    auto kern = split ? attn_fwd_ws_kernel<T, DP, true> : attn_fwd_ws_kernel<T, DP, false>;
+    const int r = set_smem(kern, C::SMEM, done[split]), sms = attn_sm_count();
+    if (r) return r;
+    kern<<<n < sms ? n : sms, C::THREADS, C::SMEM, st>>>(tq, tk, tv, q, n);
     PF_CHECK_LAUNCH();
+    return 0;
+  };
+  int r;
+  if (two_launches) {
+    AttnParams rest = p;
+    rest.item0 = p.n_pair;
+    if ((r = run(p, false, p.n_pair)) || (r = run(rest, true, tiles))) return r;
+  } else if ((r = run(p, tiles > 0, p.n_pair + tiles))) {
+    return r;
   }
   if (p.q_tail > 0) {
     // [q 128 | red 32 | scores max(Sk, 8 x 128 for the fold)] floats
@@ -704,16 +741,23 @@ PF_API int pf_attn_fwd(const void* q, const void* k, const void* v, void* o, voi
   p.q_rows = Sq - p.q_tail;
   p.q_pairs = (p.q_rows + 2 * ATT_BM - 1) / (2 * ATT_BM);
   // Pairs left over after whole rounds are split into tiles when these fit one round (FwdItem).  The
-  // form of the kernel that can do both takes 4 to 9 % longer over a pair, so that after four whole
-  // rounds the gain is used up (640 pairs of head dim 64: 340 us either way).  Causal items differ in
-  // length and are dealt by it: there only a call without a whole round is split.
+  // form of the kernel that can do both takes 4 to 9 % longer over a pair: up to three rounds it gains
+  // all the same ([4, 1024, 20, 64] 56 us whole, 48 split, [2, 2048, 20, 128] 116 and 103), after more
+  // it does not.  There the whole rounds go to the form without and the tiles to a second launch, which
+  // costs some 5 us: no gain with 8 key tiles, [4, 4096, 10, 64], which has 32, 292 us whole and 273
+  // in two.  Causal items differ in length and are dealt by it: there only a call without a whole
+  // round is split.
   const int pairs = p.q_pairs * H * B, left_over = pairs % attn_sm_count();
   const int rounds = pairs / attn_sm_count();
+  const bool fits = left_over > 0 && 2 * left_over <= attn_sm_count();
+  const bool two_launches =
+      fits && !causal && rounds > 3 && Sk > (ATT_TWO_LAUNCH_TILES - 1) * ATT_BN;
   // One tile per head is no pair to begin with: its keys are shared out from the third key tile on
   // ([1, 128, 4, 128] 7.2 us whole, 7.8 split).
-  const bool split = 2 * left_over <= attn_sm_count() && rounds <= (causal ? 0 : 3) &&
-                     (p.q_rows > ATT_BM || Sk > 2 * ATT_BN);
+  const bool split = two_launches ||
+                     (fits && rounds <= (causal ? 0 : 3) &&
+                      (p.q_rows > ATT_BM || Sk > 2 * ATT_BN));
   p.n_pair = split ? pairs - left_over : pairs;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  PF_ATTN_DISPATCH(launch_fwd_ws, tq, tk, tv, p, st);
+  PF_ATTN_DISPATCH(launch_fwd_ws, tq, tk, tv, p, two_launches, st);
 }

@@ -162,3 +162,21 @@ def test_attention_fwd_bwd_at_tile_edges(dtype, B, H, Sq, Sk, D, causal):
         assert (got.double() - want).norm() <= 2 * u * want.norm() + floor, name
     for a, b in zip(grads, again):
         assert (a.float() - b.float()).norm() <= u * a.float().norm()
+
+
+@pytest.mark.parametrize("Sq,Sk,H", [(250, 1500, 600), (256, 1409, 666), (129, 1408, 600)])
+def test_attention_forward_with_pairs_beyond_whole_rounds(Sq, Sk, H):
+    """More than four rounds of pairs of query tiles on 148 SMs: the pairs left over are split and go to
+    a launch of their own from 12 key tiles on, and stay whole below (the last case).  Heads on both
+    sides of the line against 64 bits; u / 2 per rounding (probabilities, result) on average."""
+    from pfeife_b200.ops import kernels as kx
+    g = torch.Generator(device="cuda").manual_seed(Sk)
+    q, k, v = (torch.randn(1, S, H, 32, device="cuda", generator=g).to(torch.bfloat16)
+               for S in (Sq, Sk, Sk))
+    o, lse = kx.attn_fwd(q, k, v, False, 32 ** -0.5)
+    kx.check_status()
+    pick = [0, 147, 591, 592, H - 1]
+    s = torch.einsum("qhd,khd->hqk", q[0, :, pick].double(), k[0, :, pick].double()) * 32 ** -0.5
+    want = torch.einsum("hqk,khd->qhd", s.softmax(-1), v[0, :, pick].double())
+    assert ((o[0, :, pick] - want).norm() / want.norm()).item() < 2 * 2.0 ** -8
+    assert (lse[0, pick] - s.logsumexp(-1)).abs().max().item() < 1e-4
