@@ -5,7 +5,7 @@
 //     S^T  = K Q^T                      P^T  = exp2(S^T c - lse2)
 //     dP^T = V dO^T                     dS^T = P^T (dP^T - delta) scale
 //     dV += P^T dO     A = P^T straight from TMEM (16-bit), never in shared memory
-//     dK += dS^T Q     A = dS^T in shared memory, K-major
+//     dK += dS^T Q     A = dS^T in shared memory, K-major, or up to head dim 64 in the columns of dP^T
 //     dQ  = dS K       A = the same dS^T tile, read as an MN-major operand
 // Queries lie along the N side of the first two products and along the reduction of the next two,
 // so a ragged last query tile (ViT: 257 = 2 x 128 + 1) costs what its rows cost, not a full tile.
@@ -18,7 +18,8 @@
 // What bounds it: per 128 x 128 tile pair 16384 exponentials (1024 cycles of the special-function
 // units) against 5 products (1400 cycles at head dim 64, 2560 at 128), so the tensor core must
 // never wait for the element-wise part.  Order of the MMA warp for tile i:
-//   head dim <= 64   S(i+1) as soon as S(i) is in registers, dV(i), dP(i+1), dK(i), dQ(i)
+//   head dim <= 64   S(i+1) as soon as S(i) is in registers, dV(i), dK(i), dQ(i), dP(i+1), or with
+//                    one key tile dP(i+1) before dK(i)
 //   96               S(i+1) as soon as S(i) is in registers, dV(i), dQ(i), dK(i), dP(i+1)
 //   128              dV(i), S(i+1) once dV(i) has read P^T, dQ(i), dK(i), dP(i+1)
 // TMEM (512 columns): S^T 128, dP^T 128, P^T 64 (16-bit), dV, dK, dQ one head dim each.  At 96 dQ
@@ -27,17 +28,19 @@
 //
 // Measured (B200, CUDA events, L2 flushed, with the pre- and post-pass), against one CTA per key
 // tile that ran the five products and the element-wise part one after the other with scalar
-// reductions into dQ: [4, 4096, 10, 64] 1330 -> 590 us, [2, 2048, 16, 128] 445 -> 222,
+// reductions into dQ: [4, 4096, 10, 64] 1330 -> 549 us, [2, 2048, 16, 128] 445 -> 222,
 // causal [1, 2048, 32, 128] 302 -> 138, [24, 257, 16, 88] 192 -> 142.  Steps on the way at
 // [4, 4096, 10, 64]: 877; 690 with one elected thread issuing the products (before, issuing the 28 of
 // a tile pair took 4000 cycles); 590 with tile paths free of masks, barriers looked at together, the
-// next 32 columns on their way while the last are worked on, and negated statistics.  At head dim
-// 128: 261; 222 with S(i+1) issued under the dS^T of tile i and dQ leaving TMEM ahead of its boxes.
+// next 32 columns on their way while the last are worked on, and negated statistics; 549 with dS^T
+// for dK in tensor memory.  At head dim 128: 261; 222 with S(i+1) issued under the dS^T of tile i and
+// dQ leaving TMEM ahead of its boxes.
 //
 // A pre-pass writes per query tile the row statistics [128 x -lse2 | 128 x -delta scale] (-inf / 0
 // beyond the last query, which makes the probabilities there zero without a test) and clears the fp32
 // dQ sums; a post-pass converts them.  With one key tile the dQ tiles are complete and go straight to
 // their 16-bit destination: no sums, no post-pass.
+#include <type_traits>
 #include "attn_common.cuh"
 #include "api.h"
 
@@ -124,7 +127,7 @@ attn_dq_convert_kernel(const float* __restrict__ acc, T* __restrict__ dq, long l
   }
 }
 
-template <int DP>
+template <int DP, bool DS_TMEM>
 struct BwdCfg {
   static constexpr int NBLK = (DP + 63) / 64;
   static constexpr int TILE = NBLK * ATT_BLK;
@@ -149,7 +152,9 @@ struct BwdCfg {
   static constexpr int T_DQ = ALIAS_DQ ? T_DP : T_DK + DP;
   // four warpgroups of 128 registers a thread at launch
   static constexpr int THREADS = 512;
-  static constexpr int REGS_SOFTMAX = 152, REGS_DRAIN = 104, REGS_OTHER = 104;
+  static constexpr int REGS_SOFTMAX = DS_TMEM ? 160 : 152, REGS_DRAIN = 104;
+  static constexpr int REGS_OTHER = DS_TMEM ? 88 : 104;
+  static_assert(!(DS_TMEM && ALIAS_DQ), "dS^T and dQ would share columns");
   static_assert(2 * REGS_SOFTMAX + REGS_DRAIN + REGS_OTHER <= 4 * 128, "registers of the block");
   static_assert(SMEM <= 232448, "shared memory per CTA");
   static_assert((ALIAS_DQ ? T_DK : T_DQ) + DP <= 512, "TMEM columns");
@@ -205,13 +210,15 @@ __device__ __forceinline__ void bwd_probs(const uint32_t (&s)[32], float* pr, co
 }
 
 // dS^T of the same 32 queries: 16-bit, into this key's row of the swizzled tile from its 16-byte
-// chunk `c0` on
-template <typename T>
+// chunk `c0` on, and with TMEM also to the columns at `t_ds`, whose dP^T has been read
+template <typename T, bool TMEM>
 __device__ __forceinline__ void bwd_ds(const uint32_t (&s)[32], const float* pr, const float* ndlt,
-                                       uint64_t scv, uint8_t* ds_row, int row, int c0) {
+                                       uint64_t scv, uint8_t* ds_row, int row, int c0,
+                                       uint32_t t_ds) {
+  uint32_t pk[16];
 #pragma unroll
   for (int j = 0; j < 32; j += 8) {
-    uint32_t o[4];
+    uint32_t* o = pk + j / 2;
 #pragma unroll
     for (int u = 0; u < 8; u += 4) {
       const float4 d4 = *reinterpret_cast<const float4*>(ndlt + j + u);
@@ -228,15 +235,19 @@ __device__ __forceinline__ void bwd_ds(const uint32_t (&s)[32], const float* pr,
     *reinterpret_cast<uint4*>(ds_row + (((c0 + j / 8) ^ (row & 7)) << 4)) =
         make_uint4(o[0], o[1], o[2], o[3]);
   }
+  if (TMEM) tmem_st16(t_ds, pk);
 }
 
-template <typename T, int DP>
-__global__ void __launch_bounds__(BwdCfg<DP>::THREADS, 1)
+// DS_TMEM: dK reads dS^T from tensor memory: 256 of the 3100 cycles' worth of shared-memory accesses of a
+// tile pair less ([4, 4096, 10, 64] 579 -> 549 us).  dP(i+1) then waits for dK(i), which costs more
+// than that where one key tile holds every key ([4, 1024, 20, 64] with 77 keys: 35 -> 37 us).
+template <typename T, int DP, bool DS_TMEM>
+__global__ void __launch_bounds__(BwdCfg<DP, DS_TMEM>::THREADS, 1)
 attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                    const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo,
                    const __grid_constant__ CUtensorMap tdq, const AttnBwdParams p,
                    const int n_items) {
-  using C = BwdCfg<DP>;
+  using C = BwdCfg<DP, DS_TMEM>;
   constexpr int NBLK = C::NBLK, TILE = C::TILE;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::OFF_BAR);
@@ -257,7 +268,8 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
   uint64_t* dq_empty = bars + 19;
   uint64_t* acc_full = bars + 20;    // dK / dV of the item are complete
   uint64_t* acc_empty = bars + 21;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 22);
+  uint64_t* dk_done = bars + 22;     // dK(i) has read dS^T from the columns of dP^T (head dim <= 64)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 23);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // the 128-byte swizzle works on absolute shared-memory addresses
@@ -268,7 +280,7 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
   if (tid == 0) {
     tma_prefetch_desc(&tq); tma_prefetch_desc(&tk); tma_prefetch_desc(&tv);
     tma_prefetch_desc(&tdo); tma_prefetch_desc(&tdq);
-    for (int i = 0; i < 22; ++i) mbar_init(&bars[i], 1);
+    for (int i = 0; i < 23; ++i) mbar_init(&bars[i], 1);
     for (int i = 0; i < 2; ++i) mbar_init(&q_empty[i], 1 + 8);
     mbar_init(s_empty, 8);
     mbar_init(p_ready, 8);
@@ -283,7 +295,6 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
   tc_fence_after();
   const uint32_t tmem = tmem_base_of(tmem_slot);
   const int shift = p.Sk - p.Sq;
-
   // one split per warpgroup: its four warps execute the same instruction
   if (warp >= 12) {
     regs_dec<C::REGS_OTHER>();
@@ -357,14 +368,15 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
           tc_commit(s_full);
           return true;
         };
-        // dP^T; its columns are free once dS^T of the previous tile is ready (waited for by the
-        // caller), and when dQ shares them, once that has been drained
+        // dP^T; its columns are free once the previous dK has read dS^T there, or when dQ shares them,
+        // once that has been drained
         auto issue_dp = [&](uint32_t gg, int qt) -> bool {
           const int st = gg % C::DOST;
           if (!mbar_wait(&do_full[st], (gg / C::DOST) & 1, p.status, PF_ERR_TIMEOUT_FULL))
             return false;
-          if (C::ALIAS_DQ && gg > 0 &&
-              !mbar_wait(dq_empty, (gg - 1) & 1, p.status, PF_ERR_TIMEOUT_TMEM_EMPTY))
+          if ((C::ALIAS_DQ || DS_TMEM) && gg > 0 &&
+              !mbar_wait(C::ALIAS_DQ ? dq_empty : dk_done, (gg - 1) & 1, p.status,
+                         PF_ERR_TIMEOUT_TMEM_EMPTY))
             return false;
           tc_fence_after();
           mma_kk<DP / 16>(tmem + C::T_DP, sV, sdO + st * TILE,
@@ -400,8 +412,12 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
             const uint32_t ds_tile = sdS + dsb * C::DS_BYTES;
             auto issue_dk = [&]() {
               tc_fence_after();
-              mma_k_mn(tmem + C::T_DK, ds_tile, sQ + st * TILE, id_kd, i > 0, q_steps);
+              if (DS_TMEM)
+                mma_t_mn(tmem + C::T_DK, tmem + C::T_DP, 64, sQ + st * TILE, id_kd, i > 0, q_steps);
+              else
+                mma_k_mn(tmem + C::T_DK, ds_tile, sQ + st * TILE, id_kd, i > 0, q_steps);
               tc_commit(&q_empty[st]);
+              if (DS_TMEM) tc_commit(dk_done);
             };
             auto issue_dq = [&]() {
               tc_fence_after();
@@ -414,12 +430,13 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
               tc_commit(&ds_empty[dsb]);
               if (more && !(ok = issue_dp(g + 1, qt + 1))) break;
             } else {
-              if (more && !(ok = issue_dp(g + 1, qt + 1))) break;
+              if (!DS_TMEM && more && !(ok = issue_dp(g + 1, qt + 1))) break;
               issue_dk();
               if (g > 0) ok = mbar_wait(dq_empty, (g - 1) & 1, p.status, PF_ERR_TIMEOUT_TMEM_EMPTY);
               if (!ok) break;
               issue_dq();
               tc_commit(&ds_empty[dsb]);
+              if (DS_TMEM && more && !(ok = issue_dp(g + 1, qt + 1))) break;
             }
             if (!more) { tc_commit(acc_full); tc_commit(kv_empty); }
           }
@@ -631,9 +648,9 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
           tmem_ld32(t_dp, s0);
           tmem_ld_wait_for(s0);
           tmem_ld32(t_dp + 32, s1);
-          bwd_ds<T>(s0, pr, ndlt, scv, ds_row, row, 0);
+          bwd_ds<T, DS_TMEM>(s0, pr, ndlt, scv, ds_row, row, 0, t_dp);
           tmem_ld_wait_for(s1);
-          bwd_ds<T>(s1, pr + 32, ndlt + 32, scv, ds_row, row, 4);
+          bwd_ds<T, DS_TMEM>(s1, pr + 32, ndlt + 32, scv, ds_row, row, 4, t_dp + 16);
         } else {
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
@@ -641,11 +658,13 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
               uint32_t s[32];
               tmem_ld32(t_dp + c * 32, s);
               tmem_ld_wait_for(s);
-              bwd_ds<T>(s, pr + c * 32, ndlt + c * 32, scv, ds_row, row, c * 4);
+              bwd_ds<T, DS_TMEM>(s, pr + c * 32, ndlt + c * 32, scv, ds_row, row, c * 4,
+                                 t_dp + c * 16);
             }
           }
         }
         fence_async_smem();
+        if (DS_TMEM) tmem_st_wait();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) { mbar_arrive(ds_ready); mbar_arrive(&q_empty[st]); }
@@ -678,16 +697,22 @@ template <typename T, int DP>
 static int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                       const CUtensorMap& tdo, const CUtensorMap& tdq, const AttnBwdParams& p,
                       cudaStream_t st) {
-  using C = BwdCfg<DP>;
-  auto kern = attn_bwd_ws_kernel<T, DP>;
-  static bool done[64] = {};
-  int r = set_smem(kern, C::SMEM, done);
-  if (r) return r;
   const int n_items = p.n_kt * p.H * p.B, sms = attn_sm_count();
-  kern<<<n_items < sms ? n_items : sms, C::THREADS, C::SMEM, st>>>(tq, tk, tv, tdo, tdq, p,
-                                                                   n_items);
-  PF_CHECK_LAUNCH();
-  return 0;
+  const int grid = n_items < sms ? n_items : sms;
+  auto run = [&](auto ds_tmem) -> int {
+    using C = BwdCfg<DP, decltype(ds_tmem)::value>;
+    auto kern = attn_bwd_ws_kernel<T, DP, decltype(ds_tmem)::value>;
+    static bool done[64] = {};       // one per instantiation of this lambda
+    const int r = set_smem(kern, C::SMEM, done);
+    if (r) return r;
+    kern<<<grid, C::THREADS, C::SMEM, st>>>(tq, tk, tv, tdo, tdq, p, n_items);
+    PF_CHECK_LAUNCH();
+    return 0;
+  };
+  if constexpr (DP <= 64) {
+    if (!p.direct_dq) return run(std::true_type());
+  }
+  return run(std::false_type());
 }
 
 // one key tile that every query tile visits: its dQ tiles need no summation
