@@ -127,6 +127,10 @@ PF_DECL int pf_im2col(const void* x, void* cols, int B, int H, int W, int C, int
 PF_DECL int pf_col2im(const void* dcols, void* dx, int B, int H, int W, int C, int KH, int KW,
                       int Ho, int Wo, int stride, int pad, long long ldc, int dtype, int sm_count,
                       void* stream);
+PF_DECL int pf_conv_pack(const void* w, void* out, int Cout, int Cin, int taps, int cout8, int cin8,
+                         int flip, void* stream);
+PF_DECL int pf_conv_unpack(const void* src, void* dw, int Cout, int Cin, int taps, int cin8,
+                           int dtype, void* stream);
 PF_DECL int pf_groupnorm_slabs(int B, int HW, int C, int sm_count);
 PF_DECL int pf_groupnorm_fwd(const void* x, const void* gamma, const void* beta, void* y,
                              void* mean, void* rstd, void* scratch, int B, int HW, int C, int G,

@@ -5,6 +5,7 @@
 Outputs, next to the package's ``__init__.py``:
   * ``libpfeife_b200_kernels.so`` - every CUDA kernel, compiled for sm_100a only
   * ``libpfeife_b200_host.so``    - host-side C++ (planner evaluator, step executor helpers)
+  * ``libpfeife_b200_calls.so``   - the kernel library's entry points as a Python module
 
 Objects are cached under ``build/`` keyed by source mtime, so rebuilding after a one-file edit
 recompiles one file.
@@ -17,6 +18,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 CSRC = Path(__file__).resolve().parent
@@ -25,6 +27,8 @@ BUILD = PKG.parent / "build" / "pfeife_b200"
 
 KERNEL_LIB = PKG / "libpfeife_b200_kernels.so"
 HOST_LIB = PKG / "libpfeife_b200_host.so"
+CALLS_LIB = PKG / "libpfeife_b200_calls.so"
+CALLS_SRC = CSRC / "calls.cpp"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -67,7 +71,7 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) 
     BUILD.mkdir(parents=True, exist_ok=True)
     headers = sorted(CSRC.glob("*.h")) + sorted(CSRC.glob("*.cuh"))
     cu = sorted(CSRC.glob("*.cu"))
-    cpp = sorted(CSRC.glob("*.cpp"))
+    cpp = [p for p in sorted(CSRC.glob("*.cpp")) if p != CALLS_SRC]
     nvcc = _nvcc()
     jobs = []
     objs_cu, objs_cpp = [], []
@@ -91,6 +95,9 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) 
               "-gencode", "arch=compute_100a,code=sm_100a"], verbose)
     if objs_cpp and (force or jobs or _stale(HOST_LIB, objs_cpp)):
         _run(["g++", "-shared", "-o", str(HOST_LIB), *map(str, objs_cpp), "-pthread"], verbose)
+    if force or _stale(CALLS_LIB, [CALLS_SRC, CSRC / "api.h"]):
+        _run(["g++", *CXX_FLAGS, "-shared", "-I", sysconfig.get_paths()["include"], "-I", str(CSRC),
+              str(CALLS_SRC), "-o", str(CALLS_LIB)], verbose)
 
 
 def main(argv=None) -> int:

@@ -8,6 +8,8 @@ implementations, which is what the CPU/gloo tests run.
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import threading
 from pathlib import Path
 from typing import Optional
@@ -18,7 +20,10 @@ _PKG = Path(__file__).resolve().parent.parent
 _KERNEL_LIB = _PKG / "libpfeife_b200_kernels.so"
 _HOST_LIB = _PKG / "libpfeife_b200_host.so"
 
+_CALLS_LIB = _PKG / "libpfeife_b200_calls.so"
+
 _lib: Optional[ctypes.CDLL] = None
+_calls = None
 _host: Optional[ctypes.CDLL] = None
 _tried = False
 _launches = 0  # kernels launched through this module (reported by bench.py)
@@ -57,6 +62,22 @@ def lib() -> Optional[ctypes.CDLL]:
     torch.cuda.init()
     _lib = ctypes.CDLL(str(_KERNEL_LIB), mode=ctypes.RTLD_GLOBAL)
     return _lib
+
+
+def calls():
+    """The kernel library's entry points as a Python module, which takes tensors, None, numbers and
+    tuples of strides as they are (csrc/calls.cpp); None on a machine without CUDA."""
+    global _calls
+    if _calls is None and lib() is not None:
+        if not _CALLS_LIB.exists():
+            raise KernelError(f"{_CALLS_LIB.name} is missing on a CUDA machine; run "
+                              "`python -m pfeife_b200.csrc.build`")
+        loader = importlib.machinery.ExtensionFileLoader("pfeife_b200_calls", str(_CALLS_LIB))
+        spec = importlib.util.spec_from_loader("pfeife_b200_calls", loader)
+        module = importlib.util.module_from_spec(spec)
+        loader.exec_module(module)
+        _calls = module
+    return _calls
 
 
 def host_lib() -> Optional[ctypes.CDLL]:
@@ -109,6 +130,17 @@ def stream(device: Optional[int] = None) -> ctypes.c_void_p:
         device = torch.cuda.current_device()
     bind_thread(device)
     return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(device))
+
+
+def stream_of(t: torch.Tensor) -> int:
+    """The torch stream that is current for the device of `t`, for ``calls()``; binds the calling
+    thread to that device like ``stream``."""
+    device = t.get_device()
+    if device < 0:
+        raise KernelError("a kernel was called on a tensor that is not on a CUDA device")
+    if getattr(_tls, "dev", None) != device:
+        bind_thread(device)
+    return torch._C._cuda_getCurrentRawStream(device)
 
 
 _sm_count_cache = {}

@@ -330,6 +330,10 @@ def _call(op, *args):
 
 
 # =========================================================================== linear
+_EPI_OF_ACT = {ACT_NONE: kx.EPI_NONE, ACT_GELU: kx.EPI_GELU, ACT_GELU_TANH: kx.EPI_GELU_TANH,
+               ACT_SILU: kx.EPI_SILU}
+
+
 @_custom_op("pfeife::linear_fwd")
 def linear_fwd(x: Tensor, w: Tensor, bias: Optional[Tensor], residual: Optional[Tensor],
                act: int) -> Tuple[Tensor, Tensor]:
@@ -350,8 +354,7 @@ def linear_fwd(x: Tensor, w: Tensor, bias: Optional[Tensor], residual: Optional[
         M = x2.shape[0]
         y = torch.empty((M, N), dtype=cd, device=x.device)
         aux = torch.empty((M, N), dtype=cd, device=x.device) if act else None
-        epi = {ACT_NONE: kx.EPI_NONE, ACT_GELU: kx.EPI_GELU, ACT_GELU_TANH: kx.EPI_GELU_TANH,
-               ACT_SILU: kx.EPI_SILU}[act]
+        epi = _EPI_OF_ACT[act]
         if fused_gather:
             # first use of this weight since the optimizer step: the GEMM pulls the other
             # ranks' rows over NVLink while it computes the tiles whose rows are local
@@ -386,14 +389,13 @@ def linear_bwd(dy: Tensor, x: Tensor, w: Tensor, aux: Tensor, act: int, need_dx:
     registered gradient bucket, comes back as an empty tensor."""
     cd = dy.dtype
     N, K = w.shape
-    empty = dy.new_empty(0)
     slot = _slot(w)
     if dy.is_cuda and cd in (torch.float16, torch.bfloat16):
         dy2 = _rows(dy)
         if act:
             kop = {ACT_GELU: kx.EW_DGELU, ACT_GELU_TANH: kx.EW_DGELU_TANH, ACT_SILU: kx.EW_DSILU}[act]
             dy2 = kx.elementwise(kop, dy2, _rows(aux))
-        dx, dw, db = dy.new_empty(0), dy.new_empty(0), dy.new_empty(0)
+        dx = dw = db = None
         if need_dx:
             w2 = _weight_as(w, cd)
             if N % 8 == 0 and K % 8 == 0:
@@ -420,7 +422,7 @@ def linear_bwd(dy: Tensor, x: Tensor, w: Tensor, aux: Tensor, act: int, need_dx:
                              out_dtype=dt_w)[:, :K].contiguous()
             else:
                 dw = dy2.float().t() @ x2.float()
-            if dw.numel() and dw.dtype != w.dtype:
+            if dw is not None and dw.dtype != w.dtype:
                 dw = dw.to(w.dtype)
         if need_db:
             bucket = _grad_bucket(bias)
@@ -428,7 +430,7 @@ def linear_bwd(dy: Tensor, x: Tensor, w: Tensor, aux: Tensor, act: int, need_dx:
                 kx.colsum(dy2, out=bucket)      # adds into the registered gradient
             else:
                 db = kx.colsum(dy2)
-        return dx, dw, db
+        return tuple(dy.new_empty(0) if t is None else t for t in (dx, dw, db))
     dz = dy if not act else (dy.float() * _dact_ref(aux, act)).to(cd)
     dz2 = dz.reshape(-1, N)
     dx = (dz2 @ w.to(cd)).view(x.shape[:-1] + (K,)) if need_dx else dy.new_empty(0)

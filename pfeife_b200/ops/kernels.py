@@ -11,7 +11,7 @@ from typing import Optional, Tuple
 import torch
 
 from . import _lib
-from ._lib import c_f, c_ll, check, dt, ptr, sm_count, stream
+from ._lib import c_f, c_ll, check, dt, ptr, sm_count, stream, stream_of   # ptr, c_*: ctypes
 
 # GEMM epilogue codes (gemm_sm100.cu)
 EPI_NONE, EPI_GELU, EPI_DGELU, EPI_GELU_TANH, EPI_DGELU_TANH, EPI_SILU = 0, 1, 2, 3, 4, 5
@@ -98,7 +98,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     a: [M,K] (K-major) or [K,M] when ``a_mn``; b: [N,K] (K-major) or [K,N] when ``b_mn``.
     Inputs are fp16 or bf16 2-D tensors with unit inner stride and 16-byte aligned pitch.
     """
-    L = _lib.lib()
+    L = _lib.calls()
     assert a.dim() == 2 and b.dim() == 2 and a.dtype == b.dtype
     assert a.stride(1) == 1 and b.stride(1) == 1
     if a_mn:
@@ -117,12 +117,12 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         assert residual.shape == (M, N) and residual.dtype == out.dtype and residual.stride(1) == 1
     if aux is not None:
         assert aux.shape == (M, N) and aux.dtype == out.dtype and aux.stride(1) == 1
-    code = L.pf_gemm(ptr(a), ptr(b), ptr(out), M, N, K, c_ll(a.stride(0)), c_ll(b.stride(0)),
-                     c_ll(out.stride(0)), int(a_mn), int(b_mn), dt(a.dtype), dt(out.dtype),
-                     ptr(bias), dt(bias.dtype) if bias is not None else 0, ptr(residual),
-                     c_ll(residual.stride(0) if residual is not None else 0), ptr(aux),
-                     c_ll(aux.stride(0) if aux is not None else 0), epilogue, int(accumulate),
-                     c_f(alpha), ptr(status_word(a.device)), sm_count(a.device), tile_n, stream())
+    code = L.pf_gemm(a, b, out, M, N, K, a.stride(0), b.stride(0),
+                     out.stride(0), int(a_mn), int(b_mn), dt(a.dtype), dt(out.dtype),
+                     bias, dt(bias.dtype) if bias is not None else 0, residual,
+                     residual.stride(0) if residual is not None else 0, aux,
+                     aux.stride(0) if aux is not None else 0, epilogue, int(accumulate),
+                     alpha, status_word(a.device), sm_count(a.device), tile_n, stream_of(a))
     if code != 0:
         check(code, f"pf_gemm(M={M}, N={N}, K={K}, a={tuple(a.shape)}/{a.stride()}/{a.dtype}/"
                     f"{a.data_ptr() % 256}, b={tuple(b.shape)}/{b.stride()}/{b.data_ptr() % 256}, "
@@ -133,78 +133,78 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
 
 def elementwise(op: int, a: torch.Tensor, b: Optional[torch.Tensor] = None,
                 out: Optional[torch.Tensor] = None) -> torch.Tensor:
-    L = _lib.lib()
+    L = _lib.calls()
     a = a.contiguous()
     if b is not None:
         b = b.contiguous()
         assert b.shape == a.shape and b.dtype == a.dtype
     if out is None:
         out = torch.empty_like(a)
-    check(L.pf_elementwise(ptr(a), ptr(b), ptr(out), c_ll(a.numel()), op, dt(a.dtype),
-                           sm_count(a.device), stream()), "pf_elementwise")
+    check(L.pf_elementwise(a, b, out, a.numel(), op, dt(a.dtype),
+                           sm_count(a.device), stream_of(a)), "pf_elementwise")
     return out
 
 
 def glu_fwd(gu: torch.Tensor, gelu: bool) -> torch.Tensor:
-    L = _lib.lib()
+    L = _lib.calls()
     gu = gu.contiguous()
     H = gu.shape[-1] // 2
     out = torch.empty(gu.shape[:-1] + (H,), dtype=gu.dtype, device=gu.device)
     rows = gu.numel() // (2 * H)
-    check(L.pf_glu_fwd(ptr(gu), ptr(out), c_ll(rows), H, int(gelu), dt(gu.dtype),
-                       sm_count(gu.device), stream()), "pf_glu_fwd")
+    check(L.pf_glu_fwd(gu, out, rows, H, int(gelu), dt(gu.dtype),
+                       sm_count(gu.device), stream_of(gu)), "pf_glu_fwd")
     return out
 
 
 def glu_bwd(gu: torch.Tensor, dout: torch.Tensor, gelu: bool) -> torch.Tensor:
-    L = _lib.lib()
+    L = _lib.calls()
     gu = gu.contiguous()
     dout = dout.contiguous()
     H = gu.shape[-1] // 2
     dgu = torch.empty_like(gu)
     rows = gu.numel() // (2 * H)
-    check(L.pf_glu_bwd(ptr(gu), ptr(dout), ptr(dgu), c_ll(rows), H, int(gelu), dt(gu.dtype),
-                       sm_count(gu.device), stream()), "pf_glu_bwd")
+    check(L.pf_glu_bwd(gu, dout, dgu, rows, H, int(gelu), dt(gu.dtype),
+                       sm_count(gu.device), stream_of(gu)), "pf_glu_bwd")
     return dgu
 
 
 def axpy_f32(dst: torch.Tensor, src: torch.Tensor, scale: float = 1.0,
              accumulate: bool = True) -> torch.Tensor:
-    L = _lib.lib()
+    L = _lib.calls()
     assert dst.dtype == torch.float32 and dst.is_contiguous() and dst.numel() == src.numel()
     src = src.contiguous()
-    check(L.pf_axpy_f32(ptr(dst), ptr(src), c_ll(src.numel()), c_f(scale), int(accumulate),
-                        dt(src.dtype), sm_count(src.device), stream()), "pf_axpy_f32")
+    check(L.pf_axpy_f32(dst, src, src.numel(), scale, int(accumulate),
+                        dt(src.dtype), sm_count(src.device), stream_of(dst)), "pf_axpy_f32")
     return dst
 
 
 def cast(src: torch.Tensor, dtype: torch.dtype, out: Optional[torch.Tensor] = None) -> torch.Tensor:
-    L = _lib.lib()
+    L = _lib.calls()
     src = src.contiguous()
     if out is None:
         out = torch.empty(src.shape, dtype=dtype, device=src.device)
-    check(L.pf_cast(ptr(src), ptr(out), c_ll(src.numel()), dt(src.dtype), dt(dtype),
-                    sm_count(src.device), stream()), "pf_cast")
+    check(L.pf_cast(src, out, src.numel(), dt(src.dtype), dt(dtype),
+                    sm_count(src.device), stream_of(src)), "pf_cast")
     return out
 
 
 def colsum(x: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """out[c] += sum over rows of x[r, c]; ``out`` fp32, zero-filled when not given."""
-    L = _lib.lib()
+    L = _lib.calls()
     assert x.dim() == 2 and x.stride(1) == 1
     if out is None:
         out = torch.zeros(x.shape[1], dtype=torch.float32, device=x.device)
-    check(L.pf_colsum(ptr(x), ptr(out), c_ll(x.shape[0]), x.shape[1], c_ll(x.stride(0)),
-                      dt(x.dtype), sm_count(x.device), stream()), "pf_colsum")
+    check(L.pf_colsum(x, out, x.shape[0], x.shape[1], x.stride(0),
+                      dt(x.dtype), sm_count(x.device), stream_of(x)), "pf_colsum")
     return out
 
 
 def transpose16(x: torch.Tensor) -> torch.Tensor:
-    L = _lib.lib()
+    L = _lib.calls()
     assert x.dim() == 2 and x.element_size() == 2 and x.stride(1) == 1
     out = torch.empty((x.shape[1], x.shape[0]), dtype=x.dtype, device=x.device)
-    check(L.pf_transpose16(ptr(x), ptr(out), x.shape[0], x.shape[1], c_ll(x.stride(0)),
-                           c_ll(out.stride(0)), stream()), "pf_transpose16")
+    check(L.pf_transpose16(x, out, x.shape[0], x.shape[1], x.stride(0),
+                           out.stride(0), stream_of(x)), "pf_transpose16")
     return out
 
 
@@ -212,7 +212,7 @@ def norm_fwd(x: torch.Tensor, gamma: torch.Tensor, beta: Optional[torch.Tensor],
              rms: bool, residual: Optional[torch.Tensor] = None
              ) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor]:
     """Returns (y, h, mean, rstd); h = x + residual (h is x itself when residual is None)."""
-    L = _lib.lib()
+    L = _lib.calls()
     N = x.shape[-1]
     x2 = x.contiguous().view(-1, N)
     rows = x2.shape[0]
@@ -223,15 +223,15 @@ def norm_fwd(x: torch.Tensor, gamma: torch.Tensor, beta: Optional[torch.Tensor],
     rstd = torch.empty(rows, dtype=torch.float32, device=x.device)
     g = gamma if gamma.dtype == torch.float32 else gamma.float()
     b = None if beta is None else (beta if beta.dtype == torch.float32 else beta.float())
-    check(L.pf_norm_fwd(ptr(x2), ptr(res2), ptr(g), ptr(b), ptr(y),
-                        ptr(h) if residual is not None else ptr(None), ptr(mean), ptr(rstd),
-                        c_ll(rows), N, c_f(eps), int(rms), dt(x.dtype), stream()), "pf_norm_fwd")
+    check(L.pf_norm_fwd(x2, res2, g, b, y,
+                        h if residual is not None else None, mean, rstd,
+                        rows, N, eps, int(rms), dt(x.dtype), stream_of(x2)), "pf_norm_fwd")
     return y.view(x.shape), h.view(x.shape), mean, rstd
 
 
 def norm_bwd_scratch_shape(rows: int, N: int, device=None) -> Tuple[int, int, int]:
-    L = _lib.lib()
-    return (L.pf_norm_bwd_ctas(c_ll(rows), sm_count(device)), 2, N)
+    L = _lib.calls()
+    return (L.pf_norm_bwd_ctas(rows, sm_count(device)), 2, N)
 
 
 def norm_bwd(dy: torch.Tensor, h: torch.Tensor, gamma: torch.Tensor, mean: torch.Tensor,
@@ -239,7 +239,7 @@ def norm_bwd(dy: torch.Tensor, h: torch.Tensor, gamma: torch.Tensor, mean: torch
              dgamma: Optional[torch.Tensor] = None, dbeta: Optional[torch.Tensor] = None,
              accumulate: bool = False, want_dbeta: bool = True
              ) -> Tuple[torch.Tensor, torch.Tensor, Optional[torch.Tensor]]:
-    L = _lib.lib()
+    L = _lib.calls()
     N = h.shape[-1]
     dy2 = dy.contiguous().view(-1, N)
     h2 = h.contiguous().view(-1, N)
@@ -254,16 +254,17 @@ def norm_bwd(dy: torch.Tensor, h: torch.Tensor, gamma: torch.Tensor, mean: torch
         dbeta = torch.empty(N, dtype=torch.float32, device=h.device)
     scratch = torch.empty(norm_bwd_scratch_shape(rows, N, h.device), dtype=torch.float32,
                           device=h.device)
-    check(L.pf_norm_bwd(ptr(dy2), ptr(h2), ptr(g), ptr(mean), ptr(rstd), ptr(dres2), ptr(dx),
-                        ptr(dgamma), ptr(dbeta), ptr(scratch), c_ll(rows), N, int(rms),
-                        int(accumulate), dt(h.dtype), sm_count(h.device), stream()), "pf_norm_bwd")
+    check(L.pf_norm_bwd(dy2, h2, g, mean, rstd, dres2, dx,
+                        dgamma, dbeta, scratch, rows, N, int(rms),
+                        int(accumulate), dt(h.dtype), sm_count(h.device), stream_of(dy2)),
+          "pf_norm_bwd")
     return dx.view(h.shape), dgamma, dbeta
 
 
 def nonfinite(g: torch.Tensor, found_inf: torch.Tensor) -> None:
-    L = _lib.lib()
+    L = _lib.calls()
     assert g.dtype == torch.float32 and g.is_contiguous()
-    check(L.pf_nonfinite(ptr(g), c_ll(g.numel()), ptr(found_inf), sm_count(g.device), stream()),
+    check(L.pf_nonfinite(g, g.numel(), found_inf, sm_count(g.device), stream_of(g)),
           "pf_nonfinite")
 
 
@@ -275,21 +276,21 @@ def adamw(p: torch.Tensor, g: torch.Tensor, m: torch.Tensor, v: torch.Tensor, *,
           applied_steps: Optional[torch.Tensor] = None) -> None:
     """`applied_steps` (int32 device scalar): when given, the bias correction uses its value + 1
     instead of `step`; advance it with ``step_advance`` after every group was updated."""
-    L = _lib.lib()
+    L = _lib.calls()
     for t in (p, g, m, v):
         assert t.dtype == torch.float32 and t.is_contiguous() and t.numel() == p.numel()
-    check(L.pf_adamw(ptr(p), ptr(g), ptr(m), ptr(v), ptr(lp), c_ll(p.numel()), ptr(found_inf),
-                     ptr(loss_scale), c_f(lr), c_f(beta1), c_f(beta2), c_f(eps),
-                     c_f(weight_decay), int(step), ptr(applied_steps), c_f(grad_scale),
+    check(L.pf_adamw(p, g, m, v, lp, p.numel(), found_inf,
+                     loss_scale, lr, beta1, beta2, eps,
+                     weight_decay, int(step), applied_steps, grad_scale,
                      int(decoupled),
                      int(zero_grad), dt(lp.dtype) if lp is not None else 0, sm_count(p.device),
-                     stream()), "pf_adamw")
+                     stream_of(p)), "pf_adamw")
 
 
 def step_advance(applied_steps: torch.Tensor, found_inf: Optional[torch.Tensor]) -> None:
     """applied_steps += 1 unless `found_inf` is set (the step was skipped)."""
-    L = _lib.lib()
-    check(L.pf_step_advance(ptr(applied_steps), ptr(found_inf), stream()), "pf_step_advance")
+    L = _lib.calls()
+    check(L.pf_step_advance(applied_steps, found_inf, stream_of(applied_steps)), "pf_step_advance")
 
 
 def sgd(p: torch.Tensor, g: torch.Tensor, mom: Optional[torch.Tensor], *, lr: float,
@@ -298,43 +299,45 @@ def sgd(p: torch.Tensor, g: torch.Tensor, mom: Optional[torch.Tensor], *, lr: fl
         zero_grad: bool = True, lp: Optional[torch.Tensor] = None,
         found_inf: Optional[torch.Tensor] = None,
         loss_scale: Optional[torch.Tensor] = None) -> None:
-    L = _lib.lib()
-    check(L.pf_sgd(ptr(p), ptr(g), ptr(mom), ptr(lp), c_ll(p.numel()), ptr(found_inf),
-                   ptr(loss_scale), c_f(lr), c_f(momentum), c_f(dampening), c_f(weight_decay),
-                   int(nesterov), int(first_step), c_f(grad_scale), int(zero_grad),
-                   dt(lp.dtype) if lp is not None else 0, sm_count(p.device), stream()), "pf_sgd")
+    L = _lib.calls()
+    check(L.pf_sgd(p, g, mom, lp, p.numel(), found_inf,
+                   loss_scale, lr, momentum, dampening, weight_decay,
+                   int(nesterov), int(first_step), grad_scale, int(zero_grad),
+                   dt(lp.dtype) if lp is not None else 0, sm_count(p.device), stream_of(p)),
+          "pf_sgd")
 
 
 def loss_scale_update(state: torch.Tensor, found_inf: torch.Tensor, growth: float = 2.0,
                       backoff: float = 0.5, interval: int = 2000) -> None:
-    L = _lib.lib()
-    check(L.pf_loss_scale_update(ptr(state), ptr(found_inf), c_f(growth), c_f(backoff),
-                                 int(interval), stream()), "pf_loss_scale_update")
+    L = _lib.calls()
+    check(L.pf_loss_scale_update(state, found_inf, growth, backoff,
+                                 int(interval), stream_of(state)), "pf_loss_scale_update")
 
 
 def ce_fwd(logits: torch.Tensor, target: torch.Tensor, ignore_index: int = -100
            ) -> Tuple[torch.Tensor, torch.Tensor]:
-    L = _lib.lib()
+    L = _lib.calls()
     assert logits.dim() == 2 and logits.stride(1) == 1 and target.dtype == torch.int64
     rows, V = logits.shape
     loss = torch.empty(rows, dtype=torch.float32, device=logits.device)
     lse = torch.empty(rows, dtype=torch.float32, device=logits.device)
-    check(L.pf_ce_fwd(ptr(logits), ptr(target.contiguous()), ptr(loss), ptr(lse), c_ll(rows), V,
-                      c_ll(logits.stride(0)), c_ll(ignore_index), dt(logits.dtype),
-                      sm_count(logits.device), stream()), "pf_ce_fwd")
+    check(L.pf_ce_fwd(logits, target.contiguous(), loss, lse, rows, V,
+                      logits.stride(0), ignore_index, dt(logits.dtype),
+                      sm_count(logits.device), stream_of(logits)), "pf_ce_fwd")
     return loss, lse
 
 
 def ce_bwd(logits: torch.Tensor, target: torch.Tensor, lse: torch.Tensor,
            gscale: torch.Tensor, ignore_index: int = -100) -> torch.Tensor:
-    L = _lib.lib()
+    L = _lib.calls()
     rows, V = logits.shape
     d = torch.empty_like(logits)
     if rows > 1 and gscale.stride(0) != 0:       # one value for all rows may come as an expand
         gscale = gscale.contiguous()
-    check(L.pf_ce_bwd(ptr(logits), ptr(target.contiguous()), ptr(lse), ptr(gscale), ptr(d),
-                      c_ll(rows), V, c_ll(logits.stride(0)), c_ll(ignore_index),
-                      c_ll(gscale.stride(0)), dt(logits.dtype), sm_count(logits.device), stream()),
+    check(L.pf_ce_bwd(logits, target.contiguous(), lse, gscale, d,
+                      rows, V, logits.stride(0), ignore_index,
+                      gscale.stride(0), dt(logits.dtype), sm_count(logits.device),
+                      stream_of(logits)),
           "pf_ce_bwd")
     return d
 
@@ -342,54 +345,54 @@ def ce_bwd(logits: torch.Tensor, target: torch.Tensor, lse: torch.Tensor,
 def ce_mean(loss: torch.Tensor, target: torch.Tensor, ignore_index: int = -100
             ) -> Tuple[torch.Tensor, torch.Tensor]:
     """Row losses -> (their mean over the rows that count, one over the number of those)."""
-    L = _lib.lib()
+    L = _lib.calls()
     assert loss.dtype == torch.float32 and loss.is_contiguous() and target.dtype == torch.int64
     mean = torch.empty((), dtype=torch.float32, device=loss.device)
     inv = torch.empty_like(mean)
     rows, sms = loss.numel(), sm_count(loss.device)
-    parts = L.pf_ce_mean_parts(c_ll(rows), sms)
+    parts = L.pf_ce_mean_parts(rows, sms)
     scratch = torch.empty(2 * parts, dtype=torch.float32, device=loss.device) if parts > 1 else None
-    check(L.pf_ce_mean(ptr(loss), ptr(target.contiguous()), ptr(scratch), ptr(mean), ptr(inv),
-                       c_ll(rows), c_ll(ignore_index), sms, stream()), "pf_ce_mean")
+    check(L.pf_ce_mean(loss, target.contiguous(), scratch, mean, inv,
+                       rows, ignore_index, sms, stream_of(loss)), "pf_ce_mean")
     return mean, inv
 
 
 def mse_fwd(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
-    L = _lib.lib()
+    L = _lib.calls()
     a, b = a.contiguous(), b.contiguous()
     out = torch.empty(1, dtype=torch.float32, device=a.device)
-    check(L.pf_mse_fwd(ptr(a), ptr(b), ptr(out), c_ll(a.numel()), dt(a.dtype),
-                       sm_count(a.device), stream()), "pf_mse_fwd")
+    check(L.pf_mse_fwd(a, b, out, a.numel(), dt(a.dtype),
+                       sm_count(a.device), stream_of(a)), "pf_mse_fwd")
     return out
 
 
 def mse_bwd(a: torch.Tensor, b: torch.Tensor, gout: torch.Tensor) -> torch.Tensor:
-    L = _lib.lib()
+    L = _lib.calls()
     a, b = a.contiguous(), b.contiguous()
     da = torch.empty_like(a)
-    check(L.pf_mse_bwd(ptr(a), ptr(b), ptr(gout.float().contiguous()), ptr(da), c_ll(a.numel()),
-                       dt(a.dtype), sm_count(a.device), stream()), "pf_mse_bwd")
+    check(L.pf_mse_bwd(a, b, gout.float().contiguous(), da, a.numel(),
+                       dt(a.dtype), sm_count(a.device), stream_of(a)), "pf_mse_bwd")
     return da
 
 
 def embed_fwd(table: torch.Tensor, ids: torch.Tensor, out_dtype: torch.dtype) -> torch.Tensor:
-    L = _lib.lib()
+    L = _lib.calls()
     ids_c = ids.contiguous()
     D = table.shape[1]
     out = torch.empty(ids.shape + (D,), dtype=out_dtype, device=table.device)
-    check(L.pf_embed_fwd(ptr(table), ptr(ids_c), ptr(out), c_ll(ids_c.numel()), D,
-                         c_ll(table.shape[0]), dt(table.dtype), dt(out_dtype), stream()),
+    check(L.pf_embed_fwd(table, ids_c, out, ids_c.numel(), D,
+                         table.shape[0], dt(table.dtype), dt(out_dtype), stream_of(table)),
           "pf_embed_fwd")
     return out
 
 
 def embed_bwd(dout: torch.Tensor, ids: torch.Tensor, dtable: torch.Tensor) -> torch.Tensor:
-    L = _lib.lib()
+    L = _lib.calls()
     assert dtable.dtype == torch.float32 and dtable.is_contiguous()
     dout = dout.contiguous()
     ids_c = ids.contiguous()
-    check(L.pf_embed_bwd(ptr(dout), ptr(ids_c), ptr(dtable), c_ll(ids_c.numel()),
-                         dtable.shape[1], c_ll(dtable.shape[0]), dt(dout.dtype), stream()),
+    check(L.pf_embed_bwd(dout, ids_c, dtable, ids_c.numel(),
+                         dtable.shape[1], dtable.shape[0], dt(dout.dtype), stream_of(dout)),
           "pf_embed_bwd")
     return dtable
 
@@ -397,13 +400,13 @@ def embed_bwd(dout: torch.Tensor, ids: torch.Tensor, dtable: torch.Tensor) -> to
 def rope(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, inverse: bool = False
          ) -> torch.Tensor:
     """x: [B, S, H, D] with unit stride on D; cos/sin: fp32 [S, D/2]."""
-    L = _lib.lib()
+    L = _lib.calls()
     assert x.dim() == 4 and x.stride(3) == 1
     B, S, H, D = x.shape
     out = torch.empty((B, S, H, D), dtype=x.dtype, device=x.device)
-    check(L.pf_rope(ptr(x), ptr(out), ptr(cos.contiguous()), ptr(sin.contiguous()), c_ll(B), S, H,
-                    D, c_ll(x.stride(0)), c_ll(x.stride(1)), c_ll(x.stride(2)), int(inverse),
-                    dt(x.dtype), sm_count(x.device), stream()), "pf_rope")
+    check(L.pf_rope(x, out, cos.contiguous(), sin.contiguous(), B, S, H,
+                    D, x.stride(0), x.stride(1), x.stride(2), int(inverse),
+                    dt(x.dtype), sm_count(x.device), stream_of(x)), "pf_rope")
     return out
 
 
@@ -415,21 +418,22 @@ def rope_qkv_supported(x: torch.Tensor) -> bool:
 
 def rope_qkv(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, inverse: bool = False
              ) -> torch.Tensor:
-    """x: [B, S, 3, H, D] contiguous -> the same with slices 0 and 1 rotated; cos/sin: fp32 [S, D/2]."""
-    L = _lib.lib()
+    """x: [B, S, 3, H, D] contiguous -> the same with slices 0 and 1 rotated; cos/sin: fp32
+    [S, D/2]."""
+    L = _lib.calls()
     B, S, three, H, D = x.shape
     assert three == 3 and x.is_contiguous() and cos.shape == sin.shape == (S, D // 2)
     out = torch.empty_like(x)
     fix = lambda t: t if t.is_contiguous() and t.data_ptr() % 16 == 0 else t.clone()
-    check(L.pf_rope_qkv(ptr(x), ptr(out), ptr(fix(cos)), ptr(fix(sin)), c_ll(B * S), S, H, D,
-                        int(inverse), dt(x.dtype), stream()), "pf_rope_qkv")
+    check(L.pf_rope_qkv(x, out, fix(cos), fix(sin), B * S, S, H, D,
+                        int(inverse), dt(x.dtype), stream_of(x)), "pf_rope_qkv")
     return out
 
 
 # --------------------------------------------------------------------------- attention
 def attention_supported(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> bool:
     """True when the native flash-attention kernels cover this problem."""
-    L = _lib.lib()
+    L = _lib.calls()
     return L is not None and hasattr(L, "pf_attn_fwd") and _attn_ok(q, k, v)
 
 
@@ -440,13 +444,13 @@ def _attn_ok(q, k, v) -> bool:
 
 
 def _strides3(t: torch.Tensor):
-    return (ctypes.c_longlong * 3)(t.stride(0), t.stride(1), t.stride(2))
+    return t.stride()[:3]
 
 
 def attn_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: bool, scale: float
              ) -> Tuple[torch.Tensor, torch.Tensor]:
     """q [B,Sq,H,D], k/v [B,Sk,H,D] (strided views allowed) -> (o [B,Sq,H,D], lse [B,H,Sq])."""
-    L = _lib.lib()
+    L = _lib.calls()
     B, Sq, H, D = q.shape
     Sk = k.shape[1]
     fix = lambda t: t if (t.stride(3) == 1 and t.data_ptr() % 16 == 0 and
@@ -454,9 +458,9 @@ def attn_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: bool, sc
     q, k, v = fix(q), fix(k), fix(v)
     o = torch.empty((B, Sq, H, D), dtype=q.dtype, device=q.device)
     lse = torch.empty((B, H, Sq), dtype=torch.float32, device=q.device)
-    check(L.pf_attn_fwd(ptr(q), ptr(k), ptr(v), ptr(o), ptr(lse), B, H, Sq, Sk, D, _strides3(q),
-                        _strides3(k), _strides3(v), int(causal), c_f(scale), dt(q.dtype),
-                        ptr(status_word(q.device)), stream()), "pf_attn_fwd")
+    check(L.pf_attn_fwd(q, k, v, o, lse, B, H, Sq, Sk, D, _strides3(q),
+                        _strides3(k), _strides3(v), int(causal), scale, dt(q.dtype),
+                        status_word(q.device), stream_of(q)), "pf_attn_fwd")
     return o, lse
 
 
@@ -467,7 +471,7 @@ def attn_bwd(do: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor
     """-> (dq, dk, dv).  With ``packed`` (self-attention on slices of one fused projection) the
     three gradients are slices of a single [B, S, 3, H, D] buffer, ``dqkv`` when given, i.e. the
     gradient of the fused projection needs no concatenation."""
-    L = _lib.lib()
+    L = _lib.calls()
     B, Sq, H, D = q.shape
     Sk = k.shape[1]
     fix = lambda t: t if (t.stride(3) == 1 and t.data_ptr() % 16 == 0 and
@@ -487,23 +491,24 @@ def attn_bwd(do: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor
     stats = torch.empty((B, H, (Sq + 127) // 128, 256), dtype=torch.float32, device=q.device)
     acc = None if L.pf_attn_bwd_direct(Sq, Sk, int(causal)) else \
         torch.empty((B, Sq, H, D), dtype=torch.float32, device=q.device)
-    check(L.pf_attn_bwd(ptr(do), ptr(q), ptr(k), ptr(v), ptr(o), ptr(lse), ptr(stats), ptr(acc),
-                        ptr(dq), ptr(dk), ptr(dv), B, H, Sq, Sk, D, _strides3(q), _strides3(k),
-                        _strides3(v), _strides3(dq), _strides3(dk), int(causal), c_f(scale),
-                        dt(q.dtype), ptr(status_word(q.device)), sm_count(q.device), stream()),
+    check(L.pf_attn_bwd(do, q, k, v, o, lse, stats, acc,
+                        dq, dk, dv, B, H, Sq, Sk, D, _strides3(q), _strides3(k),
+                        _strides3(v), _strides3(dq), _strides3(dk), int(causal), scale,
+                        dt(q.dtype), status_word(q.device), sm_count(q.device), stream_of(do)),
           "pf_attn_bwd")
     return dq, dk, dv
 
 
 # --------------------------------------------------------------------------- UNet kernels (NHWC)
 def im2col(x: torch.Tensor, KH: int, KW: int, stride: int, pad: int) -> torch.Tensor:
-    L = _lib.lib()
+    L = _lib.calls()
     B, H, W, C = x.shape
     Ho = (H + 2 * pad - KH) // stride + 1
     Wo = (W + 2 * pad - KW) // stride + 1
     cols = torch.empty((B * Ho * Wo, KH * KW * C), dtype=x.dtype, device=x.device)
-    check(L.pf_im2col(ptr(x.contiguous()), ptr(cols), B, H, W, C, KH, KW, Ho, Wo, stride, pad,
-                      c_ll(cols.stride(0)), dt(x.dtype), sm_count(x.device), stream()), "pf_im2col")
+    check(L.pf_im2col(x.contiguous(), cols, B, H, W, C, KH, KW, Ho, Wo, stride, pad,
+                      cols.stride(0), dt(x.dtype), sm_count(x.device), stream_of(cols)),
+          "pf_im2col")
     return cols
 
 
@@ -524,7 +529,7 @@ def conv_gemm(x: torch.Tensor, w2: torch.Tensor, KH: int, KW: int, stride: int, 
     channels innermost) -> [B, Ho, Wo, Cout].  The patches are never materialised: the GEMM's A
     tiles come straight from x through a 4-D tensor map whose out-of-bounds fill is the zero
     padding."""
-    L = _lib.lib()
+    L = _lib.calls()
     B, H, W, C = x.shape
     Cout = w2.shape[0]
     Ho = (H + 2 * pad - KH) // stride + 1
@@ -532,11 +537,11 @@ def conv_gemm(x: torch.Tensor, w2: torch.Tensor, KH: int, KW: int, stride: int, 
     assert w2.shape[1] == KH * KW * C and w2.stride(1) == 1 and w2.dtype == x.dtype
     y = torch.empty((B, Ho, Wo, Cout), dtype=x.dtype, device=x.device)
     r2 = residual.reshape(-1, Cout) if residual is not None else None
-    check(L.pf_conv_gemm(ptr(x), ptr(w2), ptr(y), B, H, W, C, Cout, KH, KW, stride, pad,
-                         c_ll(w2.stride(0)), c_ll(Cout), dt(x.dtype), dt(y.dtype), ptr(bias),
-                         dt(bias.dtype) if bias is not None else 0, ptr(r2),
-                         c_ll(r2.stride(0) if r2 is not None else 0), epilogue,
-                         ptr(status_word(x.device)), sm_count(x.device), stream()),
+    check(L.pf_conv_gemm(x, w2, y, B, H, W, C, Cout, KH, KW, stride, pad,
+                         w2.stride(0), Cout, dt(x.dtype), dt(y.dtype), bias,
+                         dt(bias.dtype) if bias is not None else 0, r2,
+                         r2.stride(0) if r2 is not None else 0, epilogue,
+                         status_word(x.device), sm_count(x.device), stream_of(x)),
           "pf_conv_gemm")
     return y
 
@@ -553,16 +558,16 @@ def conv_wgrad_supported(x: torch.Tensor, cout: int, KH: int, KW: int, stride: i
 def conv_wgrad(dy2: torch.Tensor, x: torch.Tensor, KH: int, KW: int, stride: int, pad: int,
                out: Optional[torch.Tensor] = None, accumulate: bool = False) -> torch.Tensor:
     """dw2 [Cout, KH*KW*C] fp32 (+)= dy2[B*Ho*Wo, Cout]^T . patches(x) without an im2col buffer."""
-    L = _lib.lib()
+    L = _lib.calls()
     B, H, W, C = x.shape
     Cout = dy2.shape[1]
     assert dy2.is_contiguous() and dy2.dtype == x.dtype
     if out is None:
         out = torch.empty((Cout, KH * KW * C), dtype=torch.float32, device=x.device)
         accumulate = False
-    check(L.pf_conv_wgrad(ptr(dy2), ptr(x), ptr(out), B, H, W, C, Cout, KH, KW, stride, pad,
-                          dt(x.dtype), int(accumulate), ptr(status_word(x.device)),
-                          sm_count(x.device), stream()), "pf_conv_wgrad")
+    check(L.pf_conv_wgrad(dy2, x, out, B, H, W, C, Cout, KH, KW, stride, pad,
+                          dt(x.dtype), int(accumulate), status_word(x.device),
+                          sm_count(x.device), stream_of(dy2)), "pf_conv_wgrad")
     return out
 
 
@@ -570,7 +575,7 @@ def conv_pack(w: torch.Tensor, cout8: int, cin8: int, flip: bool = False) -> tor
     """w [Cout, Cin, KH, KW] (16-bit) -> [cout8, KH*KW*cin8], the B operand of the forward, or with
     ``flip`` [cin8, KH*KW*cout8] with the taps reversed, that of the input gradient; channels
     beyond Cout / Cin are zero."""
-    L = _lib.lib()
+    L = _lib.calls()
     w = w.contiguous()
     Cout, Cin, KH, KW = w.shape
     taps = KH * KW
@@ -581,14 +586,14 @@ def conv_pack(w: torch.Tensor, cout8: int, cin8: int, flip: bool = False) -> tor
         return p.reshape(p.shape[0], -1).contiguous()
     out = torch.empty((cin8, taps * cout8) if flip else (cout8, taps * cin8), dtype=w.dtype,
                       device=w.device)
-    check(L.pf_conv_pack(ptr(w), ptr(out), Cout, Cin, taps, cout8, cin8, int(flip), stream()),
+    check(L.pf_conv_pack(w, out, Cout, Cin, taps, cout8, cin8, int(flip), stream_of(w)),
           "pf_conv_pack")
     return out
 
 
 def conv_unpack(dw2: torch.Tensor, shape, cin8: int, dtype: torch.dtype) -> torch.Tensor:
     """fp32 sums [>= Cout, KH*KW*cin8] -> the weight gradient [Cout, Cin, KH, KW] in `dtype`."""
-    L = _lib.lib()
+    L = _lib.calls()
     Cout, Cin, KH, KW = shape
     assert dw2.dtype == torch.float32 and dw2.is_contiguous()
     if KH * KW == 1 and cin8 == Cin:
@@ -598,19 +603,19 @@ def conv_unpack(dw2: torch.Tensor, shape, cin8: int, dtype: torch.dtype) -> torc
         p = dw2.view(-1, KH, KW, cin8)[:Cout, :, :, :Cin].permute(0, 3, 1, 2)
         return p.to(dtype).contiguous()
     dw = torch.empty((Cout, Cin, KH, KW), dtype=dtype, device=dw2.device)
-    check(L.pf_conv_unpack(ptr(dw2), ptr(dw), Cout, Cin, KH * KW, cin8, dt(dtype), stream()),
+    check(L.pf_conv_unpack(dw2, dw, Cout, Cin, KH * KW, cin8, dt(dtype), stream_of(dw2)),
           "pf_conv_unpack")
     return dw
 
 
 def col2im(dcols: torch.Tensor, shape, KH: int, KW: int, stride: int, pad: int) -> torch.Tensor:
-    L = _lib.lib()
+    L = _lib.calls()
     B, H, W, C = shape
     Ho = (H + 2 * pad - KH) // stride + 1
     Wo = (W + 2 * pad - KW) // stride + 1
     dx = torch.empty(shape, dtype=dcols.dtype, device=dcols.device)
-    check(L.pf_col2im(ptr(dcols), ptr(dx), B, H, W, C, KH, KW, Ho, Wo, stride, pad,
-                      c_ll(dcols.stride(0)), dt(dcols.dtype), sm_count(dcols.device), stream()),
+    check(L.pf_col2im(dcols, dx, B, H, W, C, KH, KW, Ho, Wo, stride, pad,
+                      dcols.stride(0), dt(dcols.dtype), sm_count(dcols.device), stream_of(dcols)),
           "pf_col2im")
     return dx
 
@@ -623,21 +628,21 @@ def _groupnorm_scratch(L, B: int, HW: int, C: int, width: int, device) -> torch.
 def groupnorm_fwd(x: torch.Tensor, gamma: torch.Tensor, beta: torch.Tensor, groups: int,
                   eps: float, silu: bool):
     """x NHWC [B, H, W, C] -> (y, mean[B*G], rstd[B*G])."""
-    L = _lib.lib()
+    L = _lib.calls()
     x = x.contiguous()
     B, H, W, C = x.shape
     y = torch.empty_like(x)
     mean = torch.empty(B * groups, dtype=torch.float32, device=x.device)
     rstd = torch.empty_like(mean)
     scratch = _groupnorm_scratch(L, B, H * W, C, groups, x.device)
-    check(L.pf_groupnorm_fwd(ptr(x), ptr(gamma.float()), ptr(beta.float()), ptr(y), ptr(mean),
-                             ptr(rstd), ptr(scratch), B, H * W, C, groups, c_f(eps), int(silu),
-                             dt(x.dtype), sm_count(x.device), stream()), "pf_groupnorm_fwd")
+    check(L.pf_groupnorm_fwd(x, gamma.float(), beta.float(), y, mean,
+                             rstd, scratch, B, H * W, C, groups, eps, int(silu),
+                             dt(x.dtype), sm_count(x.device), stream_of(x)), "pf_groupnorm_fwd")
     return y, mean, rstd
 
 
 def groupnorm_bwd(dy, x, mean, rstd, gamma, beta, groups: int, silu: bool):
-    L = _lib.lib()
+    L = _lib.calls()
     x, dy = x.contiguous(), dy.contiguous()
     B, H, W, C = x.shape
     dx = torch.empty_like(x)
@@ -645,15 +650,15 @@ def groupnorm_bwd(dy, x, mean, rstd, gamma, beta, groups: int, silu: bool):
     dbeta = torch.empty(C, dtype=torch.float32, device=x.device)
     sums = torch.empty(2 * B * groups, dtype=torch.float32, device=x.device)
     scratch = _groupnorm_scratch(L, B, H * W, C, C + groups, x.device)
-    check(L.pf_groupnorm_bwd(ptr(dy), ptr(x), ptr(mean), ptr(rstd), ptr(gamma.float()),
-                             ptr(beta.float()), ptr(dx), ptr(dgamma), ptr(dbeta), ptr(sums),
-                             ptr(scratch), B, H * W, C, groups, int(silu), dt(x.dtype),
-                             sm_count(x.device), stream()), "pf_groupnorm_bwd")
+    check(L.pf_groupnorm_bwd(dy, x, mean, rstd, gamma.float(),
+                             beta.float(), dx, dgamma, dbeta, sums,
+                             scratch, B, H * W, C, groups, int(silu), dt(x.dtype),
+                             sm_count(x.device), stream_of(dy)), "pf_groupnorm_bwd")
     return dx, dgamma, dbeta
 
 
 def upsample2x(x: torch.Tensor, backward: bool = False) -> torch.Tensor:
-    L = _lib.lib()
+    L = _lib.calls()
     x = x.contiguous()
     B, H, W, C = x.shape
     if backward:
@@ -661,8 +666,8 @@ def upsample2x(x: torch.Tensor, backward: bool = False) -> torch.Tensor:
         y = torch.empty((B, H, W, C), dtype=x.dtype, device=x.device)
     else:
         y = torch.empty((B, 2 * H, 2 * W, C), dtype=x.dtype, device=x.device)
-    check(L.pf_upsample2x(ptr(x), ptr(y), B, H, W, C, int(backward), dt(x.dtype),
-                          sm_count(x.device), stream()), "pf_upsample2x")
+    check(L.pf_upsample2x(x, y, B, H, W, C, int(backward), dt(x.dtype),
+                          sm_count(x.device), stream_of(x)), "pf_upsample2x")
     return y
 
 
