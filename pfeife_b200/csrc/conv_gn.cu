@@ -4,6 +4,7 @@
 //     1x1 convolutions skip these kernels entirely (they are plain GEMMs on the NHWC tensor).
 //   * GroupNorm with optional fused SiLU, forward and backward.
 //   * nearest-neighbour 2x upsampling and its backward.
+#include <type_traits>
 #include "common.cuh"
 #include "api.h"
 
@@ -196,7 +197,7 @@ conv_unpack_kernel(const float* __restrict__ src, T* __restrict__ dw, int Cin, i
 // go to scratch (per group [B, slabs, 2, G], in the backward per channel [B, slabs, 2, C] as well):
 // nothing to clear, no atomics, the same result every time.
 // Bound by memory and, below some 10 MB, by the latency of three dependent launches.
-// [4, 128, 128, 320] bf16, L2 flushed: forward 82 -> 46 us, backward 124 -> 83 us (atomics into
+// [4, 128, 128, 320] bf16, L2 flushed: forward 82 -> 46 us, backward 124 -> 83, now 64 (atomics into
 // cleared sums, a division and four lookups per element before).
 
 // rows of C/8 threads in a CTA
@@ -211,6 +212,35 @@ static inline int gn_slabs(int B, int HW, int rows, int sm_count, int per_sm) {
   const int most = (HW + 8 * rows - 1) / (8 * rows);
   if (slabs > most) slabs = most;
   return slabs < 1 ? 1 : slabs;
+}
+
+// The backward's two passes over dy and x run out of registers before they have enough loads under
+// way: each thread keeps a ring of its next pixels in shared memory, filled by asynchronous copies of
+// its own, which needs no barriers.  Three sizes of CTA: up to 256 threads (2048 channels) and up to 400
+// with a ring, beyond without (at 80 registers no more than 800 threads fit).  Backward, both passes
+// and the fold, L2 flushed: [4, 128, 128, 320] 78 -> 64 us, [4, 128, 128, 640] 141 -> 102,
+// [4, 64, 64, 1920] 108 -> 85, [4, 32, 32, 2560] 65 -> 57.
+constexpr int GN_RING = 6, GN_RING_THREADS = 400;
+// fold and ring of 400 threads
+constexpr int GN_MAX_SMEM = 2 * 8 * GN_RING_THREADS * 4 + GN_RING * 2 * GN_RING_THREADS * 16;
+constexpr int gn_min_ctas(int max_threads) {
+  return max_threads <= 256 ? GN_BWD_PER_SM : max_threads <= GN_RING_THREADS ? 2 : 1;
+}
+static inline int gn_ring_smem(int threads) {
+  return threads <= GN_RING_THREADS ? GN_RING * 2 * threads * 16 : 0;
+}
+
+// dz of two channels: dy times the derivative of the activation at z = xhat * gamma + beta
+template <bool SILU>
+__device__ __forceinline__ uint64_t gn_dz2(uint64_t dy, uint64_t xhat, uint64_t ga, uint64_t be) {
+  if (!SILU) return dy;
+  const uint64_t z = fma2(xhat, ga, be), one = f2_pack(1.f, 1.f);
+  float a, b;
+  f2_unpack(mul2(z, f2_pack(-1.4426950408889634f, -1.4426950408889634f)), a, b);
+  f2_unpack(add2(f2_pack(exp2f(a), exp2f(b)), one), a, b);
+  const uint64_t s = f2_pack(rcp_approx(a), rcp_approx(b));
+  // s (1 + z (1 - s))
+  return mul2(dy, mul2(s, fma2(z, fma2(s, f2_pack(-1.f, -1.f), one), one)));
 }
 
 // shared memory of a fold: [rows][2][C] sums (16 KB, or 8 bytes per channel when rows is 1)
@@ -321,43 +351,93 @@ __global__ void gn_apply_kernel(const T* __restrict__ x, const float* __restrict
   }
 }
 
+// Calls f(p, x, dy) for pixels p = p0, p0 + rows, ... below p1 with a thread's 8 channels of both
+// tensors as pairs of fp32 values
+template <typename T, bool RING, typename F>
+__device__ __forceinline__ void gn_pixels(const T* x, const T* dy, float* ring, int p0, int p1,
+                                          int rows, int C, F f) {
+  auto work = [&](int p, const uint4& ux, const uint4& ud) {
+    const T* ex = reinterpret_cast<const T*>(&ux);
+    const T* ed = reinterpret_cast<const T*>(&ud);
+    uint64_t vx[4], vd[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      vx[j] = f2_pack(to_f32<T>(ex[2 * j]), to_f32<T>(ex[2 * j + 1]));
+      vd[j] = f2_pack(to_f32<T>(ed[2 * j]), to_f32<T>(ed[2 * j + 1]));
+    }
+    f(p, vx, vd);
+  };
+  if constexpr (RING) {
+    auto slot = [&](int st, int which) {
+      return reinterpret_cast<uint4*>(ring) + (st * 2 + which) * blockDim.x + threadIdx.x;
+    };
+    auto fetch = [&](int p, int st) {
+      if (p < p1) {
+        cp_async16(slot(st, 0), x + (long long)p * C);
+        cp_async16(slot(st, 1), dy + (long long)p * C);
+      }
+      cp_async_commit();               // an empty group past the last pixel
+    };
+#pragma unroll
+    for (int i = 0; i < GN_RING - 1; ++i) fetch(p0 + i * rows, i);
+    int st = 0;
+    for (int p = p0; p < p1; p += rows) {
+      cp_async_wait<GN_RING - 2>();
+      const uint4 ux = *slot(st, 0), ud = *slot(st, 1);
+      fetch(p + (GN_RING - 1) * rows, st == 0 ? GN_RING - 1 : st - 1);   // read in the last round
+      st = st == GN_RING - 1 ? 0 : st + 1;
+      work(p, ux, ud);
+    }
+  } else {
+#pragma unroll 2
+    for (int p = p0; p < p1; p += rows)
+      work(p, *reinterpret_cast<const uint4*>(x + (long long)p * C),
+           *reinterpret_cast<const uint4*>(dy + (long long)p * C));
+  }
+}
+
 // Backward pass 1: per-channel sums of dz * xhat and dz (dz = dy * act'(z)); over all slabs they
 // are the parameter gradients (dgamma, dbeta) and, weighted by gamma and folded per group, the two
 // sums A = sum(dz * gamma), Bq = sum(dz * gamma * xhat) the second pass needs.
-template <typename T, bool SILU>
-__global__ void gn_bwd_stats_kernel(const T* __restrict__ dy, const T* __restrict__ x,
-                                    const float* __restrict__ mean, const float* __restrict__ rstd,
-                                    const float* __restrict__ gamma, const float* __restrict__ beta,
-                                    float* __restrict__ part, float* __restrict__ gpart, int HW,
-                                    int C, int G, int rows) {
-  extern __shared__ __align__(16) float chan[];       // [rows][2][C]: sum dz * xhat, sum dz
+template <typename T, bool SILU, int MAXT>
+__global__ void __launch_bounds__(MAXT, gn_min_ctas(MAXT))
+gn_bwd_stats_kernel(const T* __restrict__ dy, const T* __restrict__ x,
+                    const float* __restrict__ mean, const float* __restrict__ rstd,
+                    const float* __restrict__ gamma, const float* __restrict__ beta,
+                    float* __restrict__ part, float* __restrict__ gpart, int HW,
+                    int C, int G, int rows) {
+  extern __shared__ __align__(16) float chan[];       // [rows][2][C]: sum dz * xhat, sum dz; the ring
   const int ncv = C / 8, cpg = C / G;
   const int cv = threadIdx.x % ncv, r = threadIdx.x / ncv;
   const int b = blockIdx.y, c0 = cv * 8;
-  float m[8], rs[8], ga[8], be[8];
+  uint64_t nm[4], rs[4], ga[4], be[4];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const int sg = b * G + (c0 + j) / cpg;
-    m[j] = mean[sg]; rs[j] = rstd[sg]; ga[j] = gamma[c0 + j]; be[j] = beta[c0 + j];
+  for (int j = 0; j < 4; ++j) {
+    const int s0 = b * G + (c0 + 2 * j) / cpg, s1 = b * G + (c0 + 2 * j + 1) / cpg;
+    nm[j] = f2_pack(-mean[s0], -mean[s1]);
+    rs[j] = f2_pack(rstd[s0], rstd[s1]);
+    ga[j] = f2_pack(gamma[c0 + 2 * j], gamma[c0 + 2 * j + 1]);
+    be[j] = f2_pack(beta[c0 + 2 * j], beta[c0 + 2 * j + 1]);
   }
   const int per = (HW + gridDim.x - 1) / gridDim.x;
   const int p0 = blockIdx.x * per, p1 = min(HW, p0 + per);
-  float sx[8] = {0, 0, 0, 0, 0, 0, 0, 0}, sd[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  uint64_t sx2[4] = {0, 0, 0, 0}, sd2[4] = {0, 0, 0, 0};
   const long long off = (long long)b * HW * C + c0;
-#pragma unroll 2
-  for (int p = p0 + r; p < p1; p += rows) {
-    const uint4 ux = *reinterpret_cast<const uint4*>(x + off + (long long)p * C);
-    const uint4 ud = *reinterpret_cast<const uint4*>(dy + off + (long long)p * C);
-    const T* ex = reinterpret_cast<const T*>(&ux);
-    const T* ed = reinterpret_cast<const T*>(&ud);
+  gn_pixels<T, (MAXT <= GN_RING_THREADS)>(x + off, dy + off, chan + rows * 2 * C, p0 + r, p1, rows, C,
+                     [&](int, const uint64_t (&vx)[4], const uint64_t (&vd)[4]) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float xhat = (to_f32<T>(ex[j]) - m[j]) * rs[j];
-      float dz = to_f32<T>(ed[j]);
-      if (SILU) dz *= dsilu(fmaf(xhat, ga[j], be[j]));
-      sd[j] += dz;
-      sx[j] = fmaf(dz, xhat, sx[j]);
+    for (int j = 0; j < 4; ++j) {
+      const uint64_t xhat = mul2(add2(vx[j], nm[j]), rs[j]);
+      const uint64_t dz = gn_dz2<SILU>(vd[j], xhat, ga[j], be[j]);
+      sd2[j] = add2(sd2[j], dz);
+      sx2[j] = fma2(dz, xhat, sx2[j]);
     }
+  });
+  float sx[8], sd[8];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    f2_unpack(sx2[j], sx[2 * j], sx[2 * j + 1]);
+    f2_unpack(sd2[j], sd[2 * j], sd[2 * j + 1]);
   }
   gn_fold(chan, sx, sd, c0, r, rows, C);
   const long long slab = (long long)b * gridDim.x + blockIdx.x;
@@ -419,46 +499,49 @@ gn_bwd_fold_kernel(const float* __restrict__ part, const float* __restrict__ gpa
 }
 
 // Backward pass 2: dx = rstd * (dz*gamma - A/n - xhat * B/n)
-template <typename T, bool SILU>
-__global__ void gn_bwd_apply_kernel(const T* __restrict__ dy, const T* __restrict__ x,
-                                    const float* __restrict__ mean, const float* __restrict__ rstd,
-                                    const float* __restrict__ gamma, const float* __restrict__ beta,
-                                    const float* __restrict__ sumA, const float* __restrict__ sumB,
-                                    T* __restrict__ dx, int HW, int C, int G, int rows) {
+template <typename T, bool SILU, int MAXT>
+__global__ void __launch_bounds__(MAXT, gn_min_ctas(MAXT))
+gn_bwd_apply_kernel(const T* __restrict__ dy, const T* __restrict__ x,
+                    const float* __restrict__ mean, const float* __restrict__ rstd,
+                    const float* __restrict__ gamma, const float* __restrict__ beta,
+                    const float* __restrict__ sumA, const float* __restrict__ sumB,
+                    T* __restrict__ dx, int HW, int C, int G, int rows) {
+  extern __shared__ __align__(16) float ring[];
   const int ncv = C / 8, cpg = C / G;
   const float inv_n = 1.f / ((float)HW * cpg);
   const int cv = threadIdx.x % ncv, r = threadIdx.x / ncv;
   const int b = blockIdx.y, c0 = cv * 8;
-  float m[8], rs[8], ga[8], be[8], A[8], Bq[8];
+  uint64_t nm[4], rs[4], ga[4], be[4], nA[4], nB[4];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const int sg = b * G + (c0 + j) / cpg;
-    m[j] = mean[sg]; rs[j] = rstd[sg]; ga[j] = gamma[c0 + j]; be[j] = beta[c0 + j];
-    A[j] = sumA[sg] * inv_n; Bq[j] = sumB[sg] * inv_n;
+  for (int j = 0; j < 4; ++j) {
+    const int s0 = b * G + (c0 + 2 * j) / cpg, s1 = b * G + (c0 + 2 * j + 1) / cpg;
+    nm[j] = f2_pack(-mean[s0], -mean[s1]);
+    rs[j] = f2_pack(rstd[s0], rstd[s1]);
+    ga[j] = f2_pack(gamma[c0 + 2 * j], gamma[c0 + 2 * j + 1]);
+    be[j] = f2_pack(beta[c0 + 2 * j], beta[c0 + 2 * j + 1]);
+    nA[j] = f2_pack(-sumA[s0] * inv_n, -sumA[s1] * inv_n);
+    nB[j] = f2_pack(-sumB[s0] * inv_n, -sumB[s1] * inv_n);
   }
   const int per = (HW + gridDim.x - 1) / gridDim.x;
   const int p0 = blockIdx.x * per, p1 = min(HW, p0 + per);
   const long long off = (long long)b * HW * C + c0;
-#pragma unroll 2
-  for (int p = p0 + r; p < p1; p += rows) {
-    const uint4 ux = *reinterpret_cast<const uint4*>(x + off + (long long)p * C);
-    const uint4 ud = *reinterpret_cast<const uint4*>(dy + off + (long long)p * C);
-    const T* ex = reinterpret_cast<const T*>(&ux);
-    const T* ed = reinterpret_cast<const T*>(&ud);
+  gn_pixels<T, (MAXT <= GN_RING_THREADS)>(x + off, dy + off, ring, p0 + r, p1, rows, C,
+                     [&](int p, const uint64_t (&vx)[4], const uint64_t (&vd)[4]) {
     uint4 o;
     T* oe = reinterpret_cast<T*>(&o);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float xhat = (to_f32<T>(ex[j]) - m[j]) * rs[j];
-      float dz = to_f32<T>(ed[j]);
-      if (SILU) dz *= dsilu(fmaf(xhat, ga[j], be[j]));
-      oe[j] = from_f32<T>(rs[j] * (dz * ga[j] - A[j] - xhat * Bq[j]));
+    for (int j = 0; j < 4; ++j) {
+      const uint64_t xhat = mul2(add2(vx[j], nm[j]), rs[j]);
+      const uint64_t dz = gn_dz2<SILU>(vd[j], xhat, ga[j], be[j]);
+      float a0, a1;
+      f2_unpack(mul2(rs[j], fma2(xhat, nB[j], fma2(dz, ga[j], nA[j]))), a0, a1);
+      oe[2 * j] = from_f32<T>(a0);
+      oe[2 * j + 1] = from_f32<T>(a1);
     }
     *reinterpret_cast<uint4*>(dx + off + (long long)p * C) = o;
-  }
+  });
 }
 
-// nearest 2x upsample (NHWC) and its backward (sum of the 4 children)
 template <typename T>
 __global__ void __launch_bounds__(256)
 upsample2x_kernel(const T* __restrict__ x, T* __restrict__ y, int B, int H, int W, int C,
@@ -576,6 +659,31 @@ PF_API int pf_groupnorm_fwd(const void* x, const void* gamma, const void* beta, 
   return 0;
 }
 
+// `done`: per kernel and device, whether it may already use more than 48 KB of shared memory
+template <typename... P, typename... A>
+static int gn_launch(void (*kern)(P...), bool* done, dim3 grid, int threads, int smem,
+                     cudaStream_t st, A... args) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (smem > 48 * 1024 && (dev < 0 || dev >= 64 || !done[dev])) {
+    const cudaError_t e = cudaFuncSetAttribute((const void*)kern,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, GN_MAX_SMEM);
+    if (e != cudaSuccess) return (int)e;
+    if (dev >= 0 && dev < 64) done[dev] = true;
+  }
+  kern<<<grid, threads, smem, st>>>(args...);
+  return 0;
+}
+template <typename F>
+static int gn_bwd_launch(int act_silu, int threads, F f) {
+  auto sized = [&](auto silu) {
+    if (threads <= 256) return f(silu, std::integral_constant<int, 256>());
+    if (threads <= GN_RING_THREADS) return f(silu, std::integral_constant<int, GN_RING_THREADS>());
+    return f(silu, std::integral_constant<int, 800>());
+  };
+  return act_silu ? sized(std::true_type()) : sized(std::false_type());
+}
+
 // sums: fp32 scratch [2][B*G]; dgamma / dbeta fp32 [C]
 PF_API int pf_groupnorm_bwd(const void* dy, const void* x, const void* mean, const void* rstd,
                             const void* gamma, const void* beta, void* dx, void* dgamma,
@@ -593,18 +701,27 @@ PF_API int pf_groupnorm_bwd(const void* dy, const void* x, const void* mean, con
   float* part = (float*)scratch;
   float* gpart = part + (long long)B * slabs * 2 * C;
   PF_DISPATCH_H(dtype, {
-    {
-      const int smem = gn_smem(rows, C);
-      PF_GN_SILU(gn_bwd_stats_kernel, (const T*)dy, (const T*)x, (const float*)mean,
-                 (const float*)rstd, (const float*)gamma, (const float*)beta, part, gpart, HW, C,
-                 G, rows);
-    }
+    int r = gn_bwd_launch(act_silu, threads, [&](auto silu, auto most) {
+      constexpr bool S = decltype(silu)::value;
+      constexpr int R = decltype(most)::value;
+      static bool done[64] = {};       // one per instantiation
+      return gn_launch(gn_bwd_stats_kernel<T, S, R>, done, grid, threads,
+                       gn_smem(rows, C) + gn_ring_smem(threads), st, (const T*)dy, (const T*)x,
+                       (const float*)mean, (const float*)rstd, (const float*)gamma,
+                       (const float*)beta, part, gpart, HW, C, G, rows);
+    });
+    if (r) return r;
     gn_bwd_fold_kernel<<<(B * G + 31) / 32 + (C + 31) / 32, 1024, 0, st>>>(
         part, gpart, sA, sB, (float*)dgamma, (float*)dbeta, B, slabs, C, G);
-    const int smem = 0;
-    PF_GN_SILU(gn_bwd_apply_kernel, (const T*)dy, (const T*)x, (const float*)mean,
-               (const float*)rstd, (const float*)gamma, (const float*)beta, sA, sB, (T*)dx, HW, C,
-               G, rows);
+    r = gn_bwd_launch(act_silu, threads, [&](auto silu, auto most) {
+      constexpr bool S = decltype(silu)::value;
+      constexpr int R = decltype(most)::value;
+      static bool done[64] = {};       // one per instantiation
+      return gn_launch(gn_bwd_apply_kernel<T, S, R>, done, grid, threads, gn_ring_smem(threads), st,
+                       (const T*)dy, (const T*)x, (const float*)mean, (const float*)rstd,
+                       (const float*)gamma, (const float*)beta, sA, sB, (T*)dx, HW, C, G, rows);
+    });
+    if (r) return r;
   });
   PF_CHECK_LAUNCH();
   return 0;

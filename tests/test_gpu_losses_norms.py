@@ -270,3 +270,11 @@ def test_norm_backward_wide_rows(rows, N, rms):
     """Rows that one CTA holds two at a time: fewer batches than the ring has stages, an odd last
     row, threads without columns, several batches per CTA."""
     test_norm_backward_tiles(rows, N, rms)
+
+
+@pytest.mark.parametrize("silu", [True, False])
+@pytest.mark.parametrize("B,H,W,C,G", [(1, 5, 5, 3200, 32), (1, 5, 5, 3328, 32), (2, 64, 41, 320, 32)])
+def test_group_norm_forms_of_the_backward(B, H, W, C, G, silu):
+    """The largest CTA with a ring of pixels, the form without one, and more pixels per thread than a
+    ring has places."""
+    test_group_norm_edges(B, H, W, C, G, silu, torch.bfloat16)
