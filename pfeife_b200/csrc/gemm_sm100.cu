@@ -909,12 +909,12 @@ PF_API int pf_gemm(const void* A, const void* B, void* C, int M, int N, int K, l
                 !(aux && out_dtype == PF_F32);
   // Split-K: a gradient-accumulating GEMM whose tiles do not fill the GPU divides each tile's
   // reduction among several work items; they all reduce-add into C, which costs nothing extra
-  // because the epilogue accumulates anyway.  The weight gradient of a convolution, whose long
-  // reduction over the output pixels meets few tiles, does so too when it does not accumulate: C is
+  // because the epilogue accumulates anyway.  Other fp32 outputs, above all weight gradients of
+  // convolutions, whose long reduction over the output pixels meets few tiles, are split too: C is
   // small beside the operands and is cleared first (3 x 3, 320 filters of 320 channels over
   // [4, 128, 128]: 24 pair tiles, 301 us whole, 123 in three).
   p.split_k = 1;
-  const bool clear_first = !accumulate && g_conv.on == 2 && ldc == N;
+  const bool clear_first = !accumulate && ldc == N;
   if (p.vec_ok && out_dtype == PF_F32 && (accumulate || clear_first) && !(tile_n & 1024) && !aux &&
       !g_gather.on_any() && g_conv.on != 1 && !bias && !residual && epilogue == EPI_NONE &&
       !(tile_n & 8192)) {
@@ -923,8 +923,11 @@ PF_API int pf_gemm(const void* A, const void* B, void* C, int M, int N, int K, l
     const long long slots = pair ? sm_count / 2 : sm_count;
     const int nkb = (K + GEMM_BK - 1) / GEMM_BK;
     double best = 1e30;
-    for (int sk = 1; sk <= 4 && sk * 8 <= nkb; ++sk) {
-      double waves = (double)((tiles * sk + slots - 1) / slots) / sk + 0.03 * (sk - 1);
+    // Very few tiles under a very long reduction: up to 64 parts, each of which costs its first loads
+    // and its epilogue, some 8 k-blocks (320 x 72 x 65536: 282 us whole, 21 in 48).
+    for (int sk = 1; sk <= 64 && sk * 8 <= nkb; sk += sk < 4 ? 1 : sk < 8 ? 2 : sk < 16 ? 4 : 16) {
+      const double items = (double)((tiles * sk + slots - 1) / slots);
+      double waves = sk <= 4 ? items / sk + 0.03 * (sk - 1) : items * (1.0 / sk + 8.0 / nkb) + 0.09;
       // clearing C and adding to it from L2 moves some 4 MB per us, a k-block of a full wave takes
       // 0.36 us ([1, 32, 32, 1280] with 1280 filters, 59 MB of C: 40 us whole, 60 in two)
       if (clear_first && sk > 1)

@@ -179,3 +179,18 @@ def test_gemm_around_one_round_of_small_tiles(M, N, K):
     kx.check_status()
     # products of 16-bit values are exact in fp32; K fp32 additions in some order
     assert ((out - ref).norm() / ref.norm()).item() < K * 2.0 ** -24
+
+
+@pytest.mark.parametrize("M,N,K,a_mn,b_mn", [(320, 72, 32768, True, True), (8, 2880, 4096, True, True),
+                                             (128, 128, 512, False, False), (136, 72, 4160, False, True)])
+def test_gemm_fp32_output_split_into_many_parts(M, N, K, a_mn, b_mn):
+    """Few tiles under a long reduction, written and not accumulated: the parts add into an output that
+    held something else before."""
+    from pfeife_b200.ops import kernels as kx
+    a, b = _mk(M, N, K, a_mn, b_mn, torch.bfloat16)
+    out = torch.full((M, N), float("nan"), device="cuda")
+    kx.gemm(a, b, a_mn=a_mn, b_mn=b_mn, out=out)
+    ref = (a.double().t() if a_mn else a.double()) @ (b.double() if b_mn else b.double().t())
+    kx.check_status()
+    # products of 16-bit values are exact in fp32; K fp32 additions in some order
+    assert ((out - ref).norm() / ref.norm()).item() < K * 2.0 ** -24
