@@ -512,10 +512,13 @@ def im2col(x: torch.Tensor, KH: int, KW: int, stride: int, pad: int) -> torch.Te
     return cols
 
 
-def conv_gemm_supported(x: torch.Tensor, KH: int, KW: int, stride: int, pad: int) -> bool:
-    """True when the implicit-GEMM convolution covers this problem: x NHWC with C % 64 == 0,
-    tiles of 128 output pixels made of whole output rows of one image, stride 1 or 2."""
+def conv_gemm_supported(x: torch.Tensor, KH: int, KW: int, stride: int, pad: int,
+                        channels: Optional[int] = None) -> bool:
+    """True when the implicit-GEMM convolution covers this problem: x NHWC with C % 64 == 0 (C is
+    ``channels`` when x is still to be padded to that many), tiles of 128 output pixels made of
+    whole output rows of one image, stride 1 or 2."""
     B, H, W, C = x.shape
+    C = C if channels is None else channels
     Ho = (H + 2 * pad - KH) // stride + 1
     Wo = (W + 2 * pad - KW) // stride + 1
     return (x.is_contiguous() and C % 64 == 0 and 0 < Wo <= 128 and 128 % Wo == 0
