@@ -15,10 +15,10 @@
 // Role layout of the 320-thread CTA: warp 0 = TMA producer, warp 1 = TMEM owner and MMA
 // issuer (one elected thread each), warps 2..9 = epilogue (one accumulator row per thread; two warps
 // share a TMEM lane quadrant and split the tile's columns, which halves the epilogue latency per
-// tile).  Over 6144 x 6144 outputs the epilogue takes 36 us plain, 68 with GELU and its saved
-// pre-activations and 65 with GELU' (70, 74 and 80 with one value at a time and the saved values
-// fetched when they are needed), so that at K = 1408, whose products take 71 us, it still shows:
-// ViT-g/14's first layer 101 -> 94 us, its input gradient 99 -> 90;
+// tile).  Over 6144 x 6144 outputs at K = 64 a GEMM takes 39 us plain, 75 with GELU and its saved
+// pre-activations and 72 with GELU' (77 and 82 with one value at a time and the saved values fetched
+// when they are needed), so that at K = 1408, 84 us plain, the epilogue still shows: ViT-g/14's first
+// layer 104 -> 98 us, its input gradient 104 -> 94 (CUDA events, L2 flushed);
 // the instantiation that fuses an all-gather of B adds two warps that copy the remote rows.
 #include <cstring>
 #include "common.cuh"

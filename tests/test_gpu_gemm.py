@@ -194,3 +194,42 @@ def test_gemm_fp32_output_split_into_many_parts(M, N, K, a_mn, b_mn):
     kx.check_status()
     # products of 16-bit values are exact in fp32; K fp32 additions in some order
     assert ((out - ref).norm() / ref.norm()).item() < K * 2.0 ** -24
+
+
+def _pieces(z):
+    """fp32 values as the sum of three bf16 columns of a GEMM operand."""
+    a = torch.zeros(z.numel(), 64, device="cuda", dtype=torch.bfloat16)
+    rest = z.clone()
+    for j in range(3):
+        a[:, j] = rest.to(torch.bfloat16)
+        rest = rest - a[:, j].float()
+    assert not rest.any()
+    b = torch.zeros(64, 64, device="cuda", dtype=torch.bfloat16)
+    b[:, :3] = 1
+    return a, b
+
+
+# (x, gelu(x)) as the bits of fp32: what the formula gives when each of its steps rounds once
+GELU_BITS = [
+    (0xc0f24df9, 0xaa1dfac3), (0xc0c3eae2, 0xb142a258), (0xc0a381d2, 0xb55dcbf1),
+    (0xc0971fcc, 0xb6b8aed8), (0xc07f9b80, 0xb9082db1), (0xc090bfc8, 0xb7671e4c),
+    (0xc0012341, 0xbd343b7f), (0xbfc13a61, 0xbdcabafc), (0xc0074344, 0xbd15967a),
+    (0xbf3ff460, 0xbe2e0cb2), (0xbf06f443, 0xbe216d2f), (0xbf51ac69, 0xbe2d1785),
+    (0x3e8c2846, 0x3e2a6456), (0x3e5d506f, 0x3e01977e), (0x3ed7f86c, 0x3e8f477c),
+    (0x3f05ac43, 0x3ebaef04), (0x3f78d47c, 0x3f4fa452), (0x3f836242, 0x3f5ebca0),
+    (0x4005bd43, 0x400349ec), (0x402e9d57, 0x402e0f12), (0x402f4958, 0x402ebf02)]
+
+
+def test_gelu_epilogue_keeps_its_bits():
+    """A last bit of GELU turns 16-bit roundings that every later layer carries on: the logits of a
+    whole model change with it.  Values at which fused or folded steps give other bits."""
+    from pfeife_b200.ops import kernels as kx
+    bits = torch.tensor(GELU_BITS, dtype=torch.int64).to(torch.int32).cuda()
+    z = bits[:, 0].contiguous().view(torch.float32)
+    a, b = _pieces(z)
+    out = torch.empty(z.numel(), 64, device="cuda")
+    kx.gemm(a, b, out=out)
+    assert torch.equal(out, z[:, None].expand_as(out))
+    kx.gemm(a, b, out=out, epilogue=kx.EPI_GELU)
+    kx.check_status()
+    assert torch.equal(out.view(torch.int32), bits[:, 1:].expand_as(out))
