@@ -535,7 +535,8 @@ __device__ __forceinline__ float rcp_approx(float x) {
 // (Abramowitz and Stegun 7.1.26, absolute error 1.5e-7), which costs two special-function
 // instructions per value and nine packed ones per pair; gelu and gelu' are exact to 4e-7 absolute.
 // With y = 0.5 poly exp(-x^2 / 2) >= 0, Phi(x) = y for x < 0 and 1 - y for x >= 0, so that
-// gelu(x) = max(x, 0) - |x| y and Phi(x) = 0.5 + sign(x) (0.5 - y).
+// gelu(x) = max(x, 0) - |x| y.  Phi is selected and not folded into 0.5 + sign(x) (0.5 - y): below -4 that
+// would leave a few bits of y, and gelu' with a relative error of up to 3e-2 for 1.5e-4.
 // Returns -y for |x| (`ax`) and leaves exp(-x^2 / 2) in `e`.  Every step rounds where the form for one
 // value did, as does the last product of gelu: folding 1 / sqrt(2) into p and into the exponent, and that
 // product into the sum, saves two instructions per pair and turns last bits, which twelve layers of
@@ -568,9 +569,10 @@ __device__ __forceinline__ void gelu_erf_fast2(float& a, float& b) {
 __device__ __forceinline__ void dgelu_erf_fast2(float& a, float& b, float x, float y) {
   uint64_t e;
   const uint64_t ny = gelu_neg_tail2(f2_pack(fabsf(x), fabsf(y)), e);
-  float h0, h1;
-  f2_unpack(add2(ny, f2_pack(0.5f, 0.5f)), h0, h1);                 // 0.5 - y, not negative
-  const uint64_t cdf = add2(f2_pack(copysignf(h0, x), copysignf(h1, y)), f2_pack(0.5f, 0.5f));
+  float y0, y1, c0, c1;
+  f2_unpack(ny, y0, y1);
+  f2_unpack(add2(ny, f2_pack(1.f, 1.f)), c0, c1);
+  const uint64_t cdf = f2_pack(x >= 0.f ? c0 : -y0, y >= 0.f ? c1 : -y1);
   const uint64_t pdf_x = mul2(f2_pack(x, y), f2_pack(0.3989422804014327f, 0.3989422804014327f));
   f2_unpack(mul2(f2_pack(a, b), fma2(pdf_x, e, cdf)), a, b);
 }

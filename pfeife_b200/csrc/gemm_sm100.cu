@@ -16,7 +16,7 @@
 // issuer (one elected thread each), warps 2..9 = epilogue (one accumulator row per thread; two warps
 // share a TMEM lane quadrant and split the tile's columns, which halves the epilogue latency per
 // tile).  Over 6144 x 6144 outputs at K = 64 a GEMM takes 39 us plain, 75 with GELU and its saved
-// pre-activations and 72 with GELU' (77 and 82 with one value at a time and the saved values fetched
+// pre-activations and 74 with GELU' (77 and 82 with one value at a time and the saved values fetched
 // when they are needed), so that at K = 1408, 84 us plain, the epilogue still shows: ViT-g/14's first
 // layer 104 -> 98 us, its input gradient 104 -> 94 (CUDA events, L2 flushed);
 // the instantiation that fuses an all-gather of B adds two warps that copy the remote rows.

@@ -233,3 +233,30 @@ def test_gelu_epilogue_keeps_its_bits():
     kx.gemm(a, b, out=out, epilogue=kx.EPI_GELU)
     kx.check_status()
     assert torch.equal(out.view(torch.int32), bits[:, 1:].expand_as(out))
+
+
+def test_dgelu_epilogue_by_value():
+    """GELU' over [-8, 8], where a norm shows nothing of the tail.  Against the same formula in 64 bits
+    (Abramowitz and Stegun 7.1.26): its exponent, up to 46 in fp32, gives 46 ln 2 / 2^24 = 2e-6, every
+    other step some 2^-23; between -2 and 8, where terms cancel, absolutely, with 1.5e-7 of the
+    formula's own."""
+    from pfeife_b200.ops import kernels as kx
+    z = torch.linspace(-8, 8, 8192, device="cuda")
+    a, b = _pieces(z)
+    aux = kx.gemm(a, b, out_dtype=torch.float32)
+    one = torch.zeros_like(a)
+    one[:, 0] = 1
+    got = kx.gemm(one, b, out_dtype=torch.float32, aux=aux, epilogue=kx.EPI_DGELU)[:, 0].double()
+    kx.check_status()
+    x = aux[:, 0].double()
+    s = x.abs() * 0.5 ** 0.5
+    t = 1 / (1 + 0.3275911 * s)
+    poly = ((((1.061405429 * t - 1.453152027) * t + 1.421413741) * t - 0.284496736) * t
+            + 0.254829592) * t
+    e = torch.exp(-s * s)
+    y = 0.5 * poly * e
+    want = torch.where(x >= 0, 1 - y, y) + x * e * 0.3989422804014327
+    tail = x < -2
+    assert ((got - want) / want)[tail].abs().max().item() < 1e-5
+    exact = 0.5 * torch.erfc(-x * 0.5 ** 0.5) + x * torch.exp(-x * x / 2) * 0.3989422804014327
+    assert (got - exact)[~tail].abs().max().item() < 4e-7
