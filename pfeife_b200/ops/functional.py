@@ -1281,9 +1281,9 @@ def conv2d_bwd(dy: Tensor, x: Tensor, w: Tensor, stride: int, pad: int, need_dx:
             # stay in fp32 and no [pixels, taps * Cin] buffer is written and read (4 filters over
             # [4, 128, 128, 320]: 314 us through that buffer, 37 padded).
             wide = 64 if cout8 < 64 else cout8
-            if not one and stride == 1 and (cout8 == Cout or wide != cout8) and \
-                    kx.conv_gemm_supported(dy4, KH, KW, 1, KH - 1 - pad, wide) and \
-                    dy4.shape[1] + 2 * (KH - 1 - pad) - KH + 1 == H:
+            # One padding, KH - 1 - pad, serves both axes of that route: square kernels only.
+            if not one and stride == 1 and KH == KW and (cout8 == Cout or wide != cout8) and \
+                    kx.conv_gemm_supported(dy4, KH, KW, 1, KH - 1 - pad, wide):
                 # dx = correlation of dy with the taps flipped and the channel roles swapped
                 if wide != cout8:
                     dy4 = F.pad(dy4, (0, wide - cout8))

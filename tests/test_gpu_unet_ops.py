@@ -264,3 +264,27 @@ def test_conv_input_gradient_of_few_filters(cout, hw):
     ref = torch.nn.grad.conv2d_input((2, 64, hw, hw), w.double(), gy.double().permute(0, 3, 1, 2),
                                      padding=1).permute(0, 2, 3, 1)
     assert ((dx - ref).norm() / ref.norm()).item() < 2.0 ** -8
+
+
+@pytest.mark.parametrize("KH,KW,pad,H,W,cout", [
+    (1, 3, 0, 32, 36, 8), (3, 1, 1, 28, 28, 4), (1, 3, 0, 32, 36, 64), (3, 5, 1, 32, 34, 128),
+    (1, 1, 1, 16, 32, 8), (5, 5, 1, 18, 34, 8), (3, 3, 1, 16, 32, 4)])
+def test_conv_gradients_of_any_kernel_shape(KH, KW, pad, H, W, cout):
+    """The implicit route of the input gradient has one padding for both axes: kernels that are not square
+    go through the column buffer.  One rounding, of the columns too on that route: sqrt(2) 2^-9 at most
+    on average."""
+    from pfeife_b200 import ops
+    torch.manual_seed(7)
+    x = torch.randn(1, H, W, 64, device="cuda").to(torch.bfloat16).requires_grad_()
+    w = (torch.randn(cout, 64, KH, KW, device="cuda") * 0.1).to(torch.bfloat16).requires_grad_()
+    y = ops.conv2d(x, w, None, 1, pad)
+    xd, wd = x.detach().double().permute(0, 3, 1, 2), w.detach().double()
+    gy = torch.randn(y.shape, device="cuda").to(torch.bfloat16)
+    gd = gy.double().permute(0, 3, 1, 2)
+    dx, dw = torch.autograd.grad(y, (x, w), gy)
+    ref = torch.nn.functional.conv2d(xd, wd, padding=pad).permute(0, 2, 3, 1)
+    refx = torch.nn.grad.conv2d_input(xd.shape, wd, gd, padding=pad).permute(0, 2, 3, 1)
+    refw = torch.nn.grad.conv2d_weight(xd, wd.shape, gd, padding=pad)
+    for got, want in ((y, ref), (dx, refx), (dw, refw)):
+        assert got.shape == want.shape
+        assert ((got - want).norm() / want.norm()).item() < 1.5 * 2.0 ** -9
