@@ -1016,7 +1016,7 @@ def rope_qkv_apply(qkv: Tensor, cos: Tensor, sin: Tensor, inverse: bool) -> Tens
     """qkv [B, S, 3, H, D] -> a contiguous tensor with the queries and keys rotated."""
     if _native(qkv):
         qkv = qkv.contiguous()
-        if kx.rope_qkv_supported(qkv):
+        if kx.rope_qkv_supported(qkv, cos, sin):
             return kx.rope_qkv(qkv, cos.float(), sin.float(), inverse)
     q, k = (rope_apply.plain(qkv[:, :, j], cos, sin, inverse) for j in (0, 1))
     return torch.stack([q, k, qkv[:, :, 2]], dim=2)

@@ -403,6 +403,7 @@ def rope(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, inverse: bool = 
     L = _lib.calls()
     assert x.dim() == 4 and x.stride(3) == 1
     B, S, H, D = x.shape
+    assert min(cos.numel(), sin.numel()) >= S * (D // 2)      # the first S rows are read
     out = torch.empty((B, S, H, D), dtype=x.dtype, device=x.device)
     check(L.pf_rope(x, out, cos.contiguous(), sin.contiguous(), B, S, H,
                     D, x.stride(0), x.stride(1), x.stride(2), int(inverse),
@@ -410,19 +411,21 @@ def rope(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, inverse: bool = 
     return out
 
 
-def rope_qkv_supported(x: torch.Tensor) -> bool:
-    """True when the kernel over a whole fused projection covers x [B, S, 3, H, D]."""
-    return (x.dtype in (torch.float16, torch.bfloat16) and x.shape[-1] % 16 == 0
-            and x.is_contiguous() and x.data_ptr() % 16 == 0)
+def rope_qkv_supported(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor) -> bool:
+    """True when the kernel over a whole fused projection covers x [B, S, 3, H, D] and these tables."""
+    S, D = x.shape[1], x.shape[-1]
+    return (x.dtype in (torch.float16, torch.bfloat16) and D % 16 == 0
+            and x.is_contiguous() and x.data_ptr() % 16 == 0
+            and all(t.dim() == 2 and t.shape[0] >= S and t.shape[1] == D // 2 for t in (cos, sin)))
 
 
 def rope_qkv(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, inverse: bool = False
              ) -> torch.Tensor:
     """x: [B, S, 3, H, D] contiguous -> the same with slices 0 and 1 rotated; cos/sin: fp32
-    [S, D/2]."""
+    [>= S, D/2], of which the first S rows are used (as ``rope`` does)."""
     L = _lib.calls()
     B, S, three, H, D = x.shape
-    assert three == 3 and x.is_contiguous() and cos.shape == sin.shape == (S, D // 2)
+    assert three == 3 and rope_qkv_supported(x, cos, sin)
     out = torch.empty_like(x)
     fix = lambda t: t if t.is_contiguous() and t.data_ptr() % 16 == 0 else t.clone()
     check(L.pf_rope_qkv(x, out, fix(cos), fix(sin), B * S, S, H, D,

@@ -234,3 +234,22 @@ def test_rope_of_a_fused_projection(device, B, S, H, D):
         g = torch.randn(B, S, 3, H, D, device=device, dtype=dt)
         assert torch.equal(y, r)
         assert torch.equal(torch.autograd.grad(y, a, g)[0], torch.autograd.grad(r, b, g)[0])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D", [16, 24])
+def test_decoder_block_takes_longer_rotary_tables(D):
+    """Tables for the longest sequence: the block uses their first rows.  Shorter ones are refused."""
+    from pfeife_b200.models.llama import LlamaBlock, llama_config
+    torch.manual_seed(8)
+    with torch.device("cuda"):
+        block = LlamaBlock(llama_config("llama2_7b", hidden_size=4 * D, num_heads=4,
+                                        intermediate_size=64, num_layers=1)).to(torch.bfloat16)
+    x = torch.randn(2, 9, 4 * D, device="cuda").to(torch.bfloat16)
+    cos, sin = ops.rope_tables(32, D, device="cuda")
+    want = block(x, None, cos[:9], sin[:9])
+    for tables in ((cos, sin), (cos[None, :9], sin[None, :9])):
+        for got, ref in zip(block(x, None, *tables), want):
+            assert torch.equal(got, ref)
+    with pytest.raises(AssertionError):
+        block(x, None, cos[:8], sin[:8])
