@@ -65,7 +65,12 @@ class LlamaBlock(nn.Module):
         else:
             y, x = ops.rms_norm(delta, self.input_norm, self.eps, residual=x)
         qkv = ops.linear(y, self.qkv.weight).view(B, S, 3, H, d // H)
-        a = ops.attention_qkv(ops.rope_qkv(qkv, cos, sin), causal=True).view(B, S, d)
+        if ops.rope_qkv_in_one(qkv):
+            a = ops.attention_qkv(ops.rope_qkv(qkv, cos, sin), causal=True)
+        else:
+            q, k = ops.rope(qkv[:, :, 0], cos, sin), ops.rope(qkv[:, :, 1], cos, sin)
+            a = ops.attention(q, k, qkv[:, :, 2], causal=True)
+        a = a.view(B, S, d)
         delta = ops.linear(a, self.o_proj.weight)
         y, x = ops.rms_norm(delta, self.post_norm, self.eps, residual=x)
         g = ops.swiglu(ops.linear(y, self.gate_up.weight))

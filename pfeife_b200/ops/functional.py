@@ -1040,6 +1040,12 @@ def rope_qkv(qkv: Tensor, cos: Tensor, sin: Tensor) -> Tensor:
     return _call(rope_qkv_apply, qkv, cos, sin, False)
 
 
+def rope_qkv_in_one(qkv: Tensor) -> bool:
+    """True when ``rope_qkv`` is one kernel over the projection.  Elsewhere it rotates the slices and
+    stacks all three, a copy that ``rope`` of the slices and ``attention`` do without."""
+    return _native(qkv) and qkv.shape[-1] % 16 == 0
+
+
 def rope_tables(seq_len: int, head_dim: int, theta: float = 10000.0, device=None
                 ) -> Tuple[Tensor, Tensor]:
     inv = 1.0 / (theta ** (torch.arange(0, head_dim, 2, device=device, dtype=torch.float32)

@@ -253,3 +253,21 @@ def test_decoder_block_takes_longer_rotary_tables(D):
             assert torch.equal(got, ref)
     with pytest.raises(AssertionError):
         block(x, None, cos[:8], sin[:8])
+
+
+@pytest.mark.parametrize("device", DEVICES)
+@pytest.mark.parametrize("D", [16, 24])
+def test_decoder_block_does_not_stack_slices(device, D, monkeypatch):
+    """Where no kernel rotates the whole projection, the block copies none of it: the values go to the
+    attention as they are."""
+    from pfeife_b200.models.llama import LlamaBlock, llama_config
+    dt = torch.bfloat16 if device == "cuda" else torch.float32
+    with torch.device(device):
+        block = LlamaBlock(llama_config("llama2_7b", hidden_size=4 * D, num_heads=4,
+                                        intermediate_size=64, num_layers=1)).to(dt)
+    stacked = []
+    stack = torch.stack
+    monkeypatch.setattr(torch, "stack", lambda *a, **k: stacked.append(1) or stack(*a, **k))
+    x = torch.randn(2, 9, 4 * D, device=device).to(dt)
+    out = block(x, None, *ops.rope_tables(9, D, device=device))
+    assert out[1].shape == x.shape and not stacked
