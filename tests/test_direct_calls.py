@@ -53,6 +53,7 @@ def _cases(device):
         "mse": (lambda a: ops.mse_loss(a, a.detach() + 1), [r(16, 64)]),
         "embedding": (lambda t: ops.embedding(ids, t, dt), [r(24, 32)]),
         "rope": (lambda x: ops.rope(x, cos, sin), [r(2, 16, 2, 16)]),
+        "rope_qkv": (lambda x: ops.rope_qkv(x, cos, sin), [r(2, 16, 3, 2, 16)]),
         "attention": (lambda q, k, v: ops.attention(q, k, v, causal=True),
                       [r(2, 16, 2, 16), r(2, 16, 2, 16), r(2, 16, 2, 16)]),
         "attention_qkv": (lambda qkv: ops.attention_qkv(qkv), [r(2, 16, 3, 2, 16)]),
@@ -119,7 +120,7 @@ def test_wrappers_that_outlive_their_transform(device):
     assert torch.equal(ops.gelu(kept[0]), ops.gelu(x))
 
 
-@pytest.mark.parametrize("name", ["rope", "upsample", "linear", "mlp"])
+@pytest.mark.parametrize("name", ["rope", "rope_qkv", "upsample", "linear", "mlp"])
 def test_second_derivatives_where_the_backward_is_linear(name, device):
     """The gradients of rope, of upsampling and of a residual are linear in the result's gradient
     and are made of ops that can be differentiated again."""
@@ -149,7 +150,8 @@ def test_second_derivatives_of_the_others_are_refused(device):
         gx.sum().backward()
 
 
-@pytest.mark.parametrize("name", ["linear", "layer_norm", "rope", "cross_entropy", "attention_qkv"])
+@pytest.mark.parametrize("name", ["linear", "layer_norm", "rope", "rope_qkv", "cross_entropy",
+                                  "attention_qkv"])
 def test_symbolic_traces_beside_real_tensors(name, device):
     """A proxy input next to tensors that exist (weights, tables): the call is recorded."""
     fn, leaves = _cases(device)[name]
