@@ -5,7 +5,8 @@
 Outputs, next to the package's ``__init__.py``:
   * ``libpfeife_b200_kernels.so`` - every CUDA kernel, compiled for sm_100a only
   * ``libpfeife_b200_host.so``    - host-side C++ (planner evaluator, step executor helpers)
-  * ``libpfeife_b200_calls.so``   - the kernel library's entry points as a Python module
+  * ``libpfeife_b200_calls.<abi>.so`` - the kernel library's entry points as a Python module, for the
+    Python that builds it; left out where that has no headers (calls then go through ctypes)
 
 Objects are cached under ``build/`` keyed by source mtime, so rebuilding after a one-file edit
 recompiles one file.
@@ -27,7 +28,7 @@ BUILD = PKG.parent / "build" / "pfeife_b200"
 
 KERNEL_LIB = PKG / "libpfeife_b200_kernels.so"
 HOST_LIB = PKG / "libpfeife_b200_host.so"
-CALLS_LIB = PKG / "libpfeife_b200_calls.so"
+CALLS_LIB = PKG / ("libpfeife_b200_calls" + sysconfig.get_config_var("EXT_SUFFIX"))
 CALLS_SRC = CSRC / "calls.cpp"
 
 NVCC_FLAGS = [
@@ -95,8 +96,12 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) 
               "-gencode", "arch=compute_100a,code=sm_100a"], verbose)
     if objs_cpp and (force or jobs or _stale(HOST_LIB, objs_cpp)):
         _run(["g++", "-shared", "-o", str(HOST_LIB), *map(str, objs_cpp), "-pthread"], verbose)
-    if force or _stale(CALLS_LIB, [CALLS_SRC, CSRC / "api.h"]):
-        _run(["g++", *CXX_FLAGS, "-shared", "-I", sysconfig.get_paths()["include"], "-I", str(CSRC),
+    include = Path(sysconfig.get_paths()["include"])
+    if not (include / "Python.h").exists():
+        CALLS_LIB.unlink(missing_ok=True)      # of another state of the sources, perhaps
+        print(f"no Python.h in {include}: {CALLS_LIB.name} is not built, calls go through ctypes")
+    elif force or _stale(CALLS_LIB, [CALLS_SRC, CSRC / "api.h"]):
+        _run(["g++", *CXX_FLAGS, "-shared", "-I", str(include), "-I", str(CSRC),
               str(CALLS_SRC), "-o", str(CALLS_LIB)], verbose)
 
 

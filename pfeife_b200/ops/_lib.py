@@ -10,6 +10,8 @@ from __future__ import annotations
 import ctypes
 import importlib.machinery
 import importlib.util
+import re
+import sysconfig
 import threading
 from pathlib import Path
 from typing import Optional
@@ -20,7 +22,8 @@ _PKG = Path(__file__).resolve().parent.parent
 _KERNEL_LIB = _PKG / "libpfeife_b200_kernels.so"
 _HOST_LIB = _PKG / "libpfeife_b200_host.so"
 
-_CALLS_LIB = _PKG / "libpfeife_b200_calls.so"
+# built for one Python: the name carries its ABI
+_CALLS_LIB = _PKG / ("libpfeife_b200_calls" + sysconfig.get_config_var("EXT_SUFFIX"))
 
 _lib: Optional[ctypes.CDLL] = None
 _calls = None
@@ -64,19 +67,51 @@ def lib() -> Optional[ctypes.CDLL]:
     return _lib
 
 
+class _CtypesCalls:
+    """The entry points of csrc/api.h with the arguments csrc/calls.cpp takes, through ctypes: for a
+    Python without headers to build that module against.  A call costs some 5 us more."""
+
+    def __init__(self, library: ctypes.CDLL):
+        header = (_PKG / "csrc" / "api.h").read_text()
+        for name, params in re.findall(r"PF_DECL int (pf_\w+)\(([^)]*)\)", header):
+            kinds = [None if "*" in p else ctypes.c_longlong if "long long" in p
+                     else ctypes.c_float if "float" in p else ctypes.c_int
+                     for p in params.split(",") if p.strip()]
+            setattr(self, name, self._entry(getattr(library, name), kinds))
+
+    @staticmethod
+    def _pointer(v):
+        if v is None or isinstance(v, int):
+            return ctypes.c_void_p(v)
+        if isinstance(v, tuple):
+            return (ctypes.c_longlong * len(v))(*v)
+        return ctypes.c_void_p(v.data_ptr())
+
+    def _entry(self, fn, kinds):
+        def call(*args):
+            if len(args) != len(kinds):
+                raise TypeError(f"expected {len(kinds)} arguments, got {len(args)}")
+            return fn(*(self._pointer(a) if k is None else k(a) for k, a in zip(kinds, args)))
+        return call
+
+
+def load_calls(library: ctypes.CDLL):
+    """The Python module of the entry points of `library`, which is loaded with its symbols global."""
+    if not _CALLS_LIB.exists():
+        return _CtypesCalls(library)
+    loader = importlib.machinery.ExtensionFileLoader("pfeife_b200_calls", str(_CALLS_LIB))
+    spec = importlib.util.spec_from_loader("pfeife_b200_calls", loader)
+    module = importlib.util.module_from_spec(spec)
+    loader.exec_module(module)
+    return module
+
+
 def calls():
     """The kernel library's entry points as a Python module, which takes tensors, None, numbers and
     tuples of strides as they are (csrc/calls.cpp); None on a machine without CUDA."""
     global _calls
     if _calls is None and lib() is not None:
-        if not _CALLS_LIB.exists():
-            raise KernelError(f"{_CALLS_LIB.name} is missing on a CUDA machine; run "
-                              "`python -m pfeife_b200.csrc.build`")
-        loader = importlib.machinery.ExtensionFileLoader("pfeife_b200_calls", str(_CALLS_LIB))
-        spec = importlib.util.spec_from_loader("pfeife_b200_calls", loader)
-        module = importlib.util.module_from_spec(spec)
-        loader.exec_module(module)
-        _calls = module
+        _calls = load_calls(_lib)
     return _calls
 
 

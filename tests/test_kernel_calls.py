@@ -1,0 +1,81 @@
+"""How Python values reach the kernel library's entry points: through the module built for this Python and
+through ctypes where there is none.  The entry points called here return before they touch a device."""
+import ctypes
+
+import pytest
+import torch
+
+from pfeife_b200.csrc import build
+from pfeife_b200.ops import _lib
+
+
+@pytest.fixture(params=["module", "ctypes"])
+def calls(request, monkeypatch):
+    if not build.KERNEL_LIB.exists():
+        pytest.skip("the kernel library is not built")
+    library = ctypes.CDLL(str(build.KERNEL_LIB), mode=ctypes.RTLD_GLOBAL)
+    if request.param == "ctypes":
+        monkeypatch.setattr(_lib, "_CALLS_LIB", build.PKG / "missing.so")
+    elif not build.CALLS_LIB.exists():
+        pytest.skip("the module is not built: this Python has no headers")
+    out = _lib.load_calls(library)
+    assert isinstance(out, _lib._CtypesCalls) == (request.param == "ctypes")
+    return out
+
+
+def _gemm(calls, a, b, M=8, dtype=_lib.PF_BF16, lda=64, alpha=1.0):
+    return calls.pf_gemm(a, b, None, M, 8, 64, lda, 64, 8, 0, 0, dtype, dtype, None, 0, None, 0, None, 0,
+                         0, 0, alpha, None, 148, 0, None)
+
+
+def test_values_arrive(calls):
+    assert calls.pf_norm_bwd_ctas(1, 148) == 1
+    assert calls.pf_norm_bwd_ctas(1 << 40, 148) == calls.pf_norm_bwd_ctas(1 << 20, 148) > 148
+    assert calls.pf_attn_bwd_direct(256, 128, False) == 1
+    assert calls.pf_attn_bwd_direct(256, 129, 0) == 0
+    t = torch.zeros(64, 64, dtype=torch.bfloat16)
+    assert _gemm(calls, t, t, M=0) == 0
+    assert _gemm(calls, t, t, dtype=7) == -1
+    assert _gemm(calls, t, t, lda=63) == -2
+    assert _gemm(calls, t[0, 1:], t) == -2                 # 2 bytes off, as a tensor and as a number
+    assert _gemm(calls, t.data_ptr(), t.data_ptr() + 2) == -2
+    assert calls.pf_rope_qkv(t, t, None, None, 0, 1, 1, 16, 0, _lib.PF_BF16, None) == 0
+    # strides as a tuple: rows of queries that are no multiple of 16 bytes
+    z = (64, 64, 64)
+    args = [t, t, t, t, t, 1, 1, 8, 8, 64, (64, 60, 64), z, z, 0, 1.0, _lib.PF_BF16, None, None]
+    assert calls.pf_attn_fwd(*args) == -2
+
+
+def test_what_does_not_fit_is_refused(calls):
+    t = torch.zeros(64, 64, dtype=torch.bfloat16)
+    with pytest.raises(TypeError):
+        calls.pf_norm_bwd_ctas(1)
+    with pytest.raises(TypeError):
+        calls.pf_norm_bwd_ctas(1.5, 148)
+    with pytest.raises((TypeError, AttributeError)):
+        _gemm(calls, "tensor", t)
+    with pytest.raises(TypeError):
+        _gemm(calls, t, t, alpha="1")
+    if not isinstance(calls, _lib._CtypesCalls):           # ctypes wraps numbers and takes any tuple
+        with pytest.raises(OverflowError):
+            calls.pf_norm_bwd_ctas(1, 1 << 31)
+        with pytest.raises(OverflowError):
+            calls.pf_norm_bwd_ctas(1 << 63, 148)
+        with pytest.raises(ValueError):
+            calls.pf_attn_fwd(t, t, t, t, t, 1, 1, 8, 8, 64, (1,) * 9, None, None, 0, 1.0, 2, None, None)
+
+
+def test_a_tensor_on_the_cpu_is_refused():
+    with pytest.raises(_lib.KernelError):
+        _lib.stream_of(torch.zeros(1))
+
+
+def test_the_module_is_optional(monkeypatch, tmp_path, capsys):
+    """Without Python's headers everything else is built, and no module of another state stays."""
+    left = tmp_path / "calls.so"
+    left.write_bytes(b"")
+    monkeypatch.setattr(build, "CALLS_LIB", left)
+    monkeypatch.setattr(build.sysconfig, "get_paths", lambda: {"include": str(tmp_path)})
+    monkeypatch.setattr(build, "_stale", lambda *a: False)
+    build.build()
+    assert not left.exists() and "ctypes" in capsys.readouterr().out
