@@ -20,7 +20,10 @@ PF_DECL int pf_gemm(const void* A, const void* B, void* C, int M, int N, int K, 
                     long long ldb, long long ldc, int a_mn, int b_mn, int in_dtype, int out_dtype,
                     const void* bias, int bias_dtype, const void* residual, long long ldr,
                     void* aux, long long ldaux, int epilogue, int accumulate, float alpha,
-                    int* status, int sm_count, int tile_n, void* stream);
+                    int* status, int sm_count, int tile_n, void* workspace, int workspace_kib,
+                    void* stream);
+PF_DECL int pf_gemm_workspace(int M, int N, int K, int accumulate, int conv, int sm_count,
+                              int tile_n);
 
 // ---- elementwise.cu
 PF_DECL int pf_elementwise(const void* a, const void* b, void* out, long long n, int op, int dtype,
@@ -151,7 +154,8 @@ PF_DECL int pf_conv_gemm(const void* x, const void* w2, void* y, int B, int H, i
 
 PF_DECL int pf_conv_wgrad(const void* dy, const void* x, void* dw2, int B, int H, int W, int C,
                           int Cout, int KH, int KW, int stride, int pad, int in_dtype,
-                          int accumulate, int* status, int sm_count, void* stream);
+                          int accumulate, int* status, int sm_count, void* workspace,
+                          int workspace_kib, void* stream);
 
 // ---- gemm_sm100.cu : GEMM with the all-gather of a row-sharded weight fused in
 PF_DECL int pf_gemm_allgather(const void* A, void* w_full, void* const* copies, int world,

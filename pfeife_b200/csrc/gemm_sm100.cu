@@ -58,8 +58,9 @@ struct GemmParams {
   int a_mn, b_mn;
   int fmt;        // 0 = fp16 inputs, 1 = bf16 inputs
   int* status;
-  int split_k;    // > 1: each tile's k-blocks are divided among this many work items, which all
-                  // add into C (needs accumulate through the TMA reduce-add epilogue)
+  int split_k;    // > 1: each tile's k-blocks are divided among this many work items, which either
+                  // all add into C (needs accumulate through the TMA reduce-add epilogue) or, with
+  int part_rows;  // part_rows > 0, store to rows of their own: part i from row i * part_rows of C on
   // ---- fused all-gather of the B operand (weights sharded by rows over `gather_world` ranks)
   int gather_world;            // 0: B is an ordinary local operand
   int gather_rank;
@@ -522,6 +523,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
       const int n0 = ((tile / num_m + n_rot) % num_n) * BNT;
       const int row = m0 + row_in_tile;
       const bool row_ok = row < p.M;
+      const int part_row0 = sizeof(OutT) == 4 ? (item / num_mn) * p.part_rows : 0;
       // the first saved values of this tile travel while its products are computed
       if (dgelu && row_ok) fetch_aux(row, n0 + c_begin);
       ok = mbar_wait(&tmem_full[acc], acc_phase, p.status, PF_ERR_TIMEOUT_TMEM_FULL);
@@ -622,7 +624,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
           const int row0 = m0 + quad * 32;
           if (lane == 0 && row0 < p.M) {
             if (p.accumulate) tma_reduce_add_2d(&tmap_c, stage_c, col, row0);
-            else tma_store_2d(&tmap_c, stage_c, col, row0);
+            else tma_store_2d(&tmap_c, stage_c, col, row0 + part_row0);
             if (aux_out) tma_store_2d(&tmap_aux, stage_aux, col, row0);
           }
           // an (empty) group is committed even for a clipped chunk so that the group count
@@ -662,6 +664,55 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
     tc_fence_after();
     if (PAIR) tmem_dealloc_pair(tmem_base, TMEM_COLS);
     else tmem_dealloc(tmem_base, TMEM_COLS);
+  }
+}
+
+// C[m, n] (+)= the sum over parts of ws[part][m, n], in the order of the parts: the same bits every time.
+// Bound by L2, where the parts have just been written, or by latency when there is little of them; a
+// thread takes 4 columns, or one where that leaves SMs idle, and has 8 parts on their way at a time.
+template <int V>
+__global__ void __launch_bounds__(256)
+gemm_fold_kernel(const float* __restrict__ ws, float* __restrict__ C, int M, int N, int parts,
+                 long long part_size, int pitch, long long ldc, int accumulate) {
+  const int nv = (N + V - 1) / V;
+  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (i >= (long long)M * nv) return;
+  const int m = (int)(i / nv), n = (int)(i - (long long)m * nv) * V;
+  const float* src = ws + (long long)m * pitch + n;
+  float* dst = C + (long long)m * ldc + n;
+  float s[V], b[8][V];
+  auto load = [&](const float* from, float (&to)[V]) {
+    if constexpr (V == 4) {
+      const float4 q = *reinterpret_cast<const float4*>(from);
+      to[0] = q.x; to[1] = q.y; to[2] = q.z; to[3] = q.w;
+    } else {
+      to[0] = *from;
+    }
+  };
+#pragma unroll
+  for (int v = 0; v < V; ++v) s[v] = 0.f;
+  for (int p0 = 0; p0 < parts; p0 += 8) {
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (p0 + u < parts) load(src + (p0 + u) * part_size, b[u]);
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (p0 + u < parts) {
+#pragma unroll
+        for (int v = 0; v < V; ++v) s[v] += b[u][v];
+      }
+  }
+  if (accumulate) {
+#pragma unroll
+    for (int v = 0; v < V; ++v)
+      if (n + v < N) s[v] += dst[v];
+  }
+  if (V == 4 && n + 4 <= N && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+    *reinterpret_cast<float4*>(dst) = make_float4(s[0], s[1 % V], s[2 % V], s[3 % V]);
+  } else {
+#pragma unroll
+    for (int v = 0; v < V; ++v)
+      if (n + v < N) dst[v] = s[v];
   }
 }
 
@@ -812,30 +863,29 @@ struct GatherArgs {
 };
 static thread_local GatherArgs g_gather;
 
-PF_API int pf_gemm(const void* A, const void* B, void* C, int M, int N, int K, long long lda,
-                   long long ldb, long long ldc, int a_mn, int b_mn, int in_dtype, int out_dtype,
-                   const void* bias, int bias_dtype, const void* residual, long long ldr,
-                   void* aux, long long ldaux, int epilogue, int accumulate, float alpha,
-                   int* status, int sm_count, int tile_n, void* stream) {
-  if (M <= 0 || N <= 0 || K <= 0) return 0;
-  if (in_dtype != PF_F16 && in_dtype != PF_BF16) return -1;
-  if ((g_conv.on != 1 && (lda % 8)) || (g_conv.on != 2 && (ldb % 8)) ||
-      (reinterpret_cast<uintptr_t>(A) & 15) ||
-      (reinterpret_cast<uintptr_t>(B) & 15))
-    return -2;  // TMA needs 16-byte aligned bases and pitches
-  const int fmt = in_dtype == PF_BF16 ? 1 : 0;
-  // tile_n: low bits 0 / 128 / 256 = tile width of the single-CTA form; bit 10 forces the
-  // direct-store epilogue, bit 11 forces the CTA-pair form, bit 12 forbids it, bit 13 forbids
-  // the split reduction (tests, benches)
+// Tiles and parts of a call.
+struct GemmPlan {
+  bool pair = false;       // 256 x 256 tiles of a CTA pair, else 128 x bn
+  int bn = 128;
+  int parts = 1;           // work items that share a tile's reduction
+  bool ordered = false;    // they write to a workspace that is folded afterwards
+  // of a part in the workspace
+  int rows = 0, pitch = 0;
+  long long ws_floats() const { return ordered ? (long long)parts * rows * pitch : 0; }
+};
+
+// `may_split`: an fp32 output, written whole by the TMA with nothing fused; `conv`: 2 for the weight
+// gradient of a convolution.
+static GemmPlan gemm_plan(int M, int N, int K, int out_dtype, bool accumulate, int conv, bool gather,
+                          bool may_split, int tile_n, int sm_count) {
+  GemmPlan g;
   const int tn = tile_n & 1023;
-  if (sm_count <= 0) sm_count = 148;
   const bool one_round =
       (long long)((M + 127) / 128) * ((N + 127) / 128) <= sm_count &&
-      !(out_dtype == PF_F32 && (accumulate || g_conv.on == 2));
-  bool pair = false;
-  if (g_gather.world <= 1 && !(tile_n & 4096) && sm_count >= 2) {
+      !(out_dtype == PF_F32 && (accumulate || conv == 2));
+  if (!gather && !(tile_n & 4096) && sm_count >= 2) {
     if (tile_n & 2048) {
-      pair = true;
+      g.pair = true;
     } else if (tn == 0 && M > 128 && N > 128) {
       // rounds of 256 x 256 pair tiles over sm_count / 2 pairs against rounds of 128 x 256 tiles
       // over sm_count CTAs.  Measured on B200, a pair tile costs each SM 0.9-0.95 of a single
@@ -849,12 +899,15 @@ PF_API int pf_gemm(const void* A, const void* B, void* C, int M, int N, int K, l
       // Where 128 x 128 tiles all run at once, the time is that of one tile, and the small ones are
       // the soonest done: 1024 x 768 x 3072 24.2 us as pairs, 19.5 as 128 x 128; 300 x 4096 x 1024
       // 20.1 and 14.0; 2048 x 1024 x 4096 28.3 and 24.2; 788 x 768 x 192 16.0 and 10.6.
-      // (Outputs whose reduction may be split fill the SMs that way, with the large tiles.)
-      pair = !one_round && 93 * w2 <= 100 * w1;
+      // Accumulating fp32 outputs and convolution gradients keep the large tiles, whose reduction is
+      // split where they leave SMs idle; the other fp32 outputs are split over 128 x 128 tiles, which
+      // was no slower: 320 x 320 x 65536 40 us over 128 x 128, 46 as pairs, 1280 x 1280 x 4096 27.6
+      // and 29.7, 1408 x 1408 x 6168 36 and 38, 640 x 640 x 16384 33.8 and 31.7.
+      g.pair = !one_round && 93 * w2 <= 100 * w1;
     }
   }
   int bn_auto = N <= 128 ? 128 : 256;
-  if (!pair && tn == 0 && N > 128) {
+  if (!g.pair && tn == 0 && N > 128) {
     // 128 x 128 tiles (0.55 of a 128 x 256 tile each) when they fill the waves better
     const long long t1 = (long long)((M + 127) / 128) * ((N + 255) / 256);
     const long long th = (long long)((M + 127) / 128) * ((N + 127) / 128);
@@ -862,7 +915,87 @@ PF_API int pf_gemm(const void* A, const void* B, void* C, int M, int N, int K, l
     const long long wh = (th + sm_count - 1) / sm_count;
     if (11 * wh < 20 * w1 || one_round) bn_auto = 128;
   }
-  const int BN = pair ? 128 : (tn == 128 || tn == 256) ? tn : bn_auto;
+  g.bn = g.pair ? 128 : (tn == 128 || tn == 256) ? tn : bn_auto;
+  if (!may_split || out_dtype != PF_F32 || gather || conv == 1 || (tile_n & (1024 | 8192))) return g;
+
+  const int bm = g.pair ? 256 : 128, bn = g.pair ? 256 : g.bn;
+  const long long tiles = (long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn);
+  const long long slots = g.pair ? sm_count / 2 : sm_count;
+  const int nkb = (K + GEMM_BK - 1) / GEMM_BK;
+  double best = 1e30;
+  if (accumulate && conv == 0) {
+    // A gradient-accumulating GEMM of a linear layer: up to four parts that all reduce-add into C,
+    // which costs nothing extra because the epilogue accumulates anyway.  (The order in which they
+    // arrive is not fixed, and neither are the last bits of the sum.)
+    for (int sk = 1; sk <= 4 && sk * 8 <= nkb; ++sk) {
+      const double waves = (double)((tiles * sk + slots - 1) / slots) / sk + 0.03 * (sk - 1);
+      if (waves < best - 1e-9) { best = waves; g.parts = sk; }
+    }
+    return g;
+  }
+  // Other fp32 outputs, above all weight gradients of convolutions, whose long reduction over the output
+  // pixels meets few tiles: the parts go to a workspace and are folded in their order (3 x 3, 320 filters
+  // of 320 channels over [4, 128, 128]: 24 pair tiles, 302 us whole, 124 in three).  Up to 64 parts, each
+  // of which costs its first loads and its epilogue, some 8 k-blocks (320 x 72 x 65536: 284 us whole, 28
+  // in 32).  What writing and folding them costs, in units of a k-block (0.36 us of a pair, 0.26 of
+  // 128 columns): a launch of some 2 us, and 5 MB per us of parts written and read and C written
+  // ([1, 32, 32, 1280] with 1280 filters, 59 MB of C: 42 us whole, 87 in two; 1024 x 1024 x 2048: 19.5
+  // and 21.5; [1, 64, 64, 320] with 640 filters: 31.7 and 29.7).  Against parts that add into a cleared C
+  // in any order, sizes of the UNet take 0 to 2 us longer and 320 x 72 x 65536 4.
+  g.rows = (M + bm - 1) / bm * bm;
+  g.pitch = (N + 3) / 4 * 4;
+  const double whole_us = (g.pair ? 0.36 : g.bn == 256 ? 0.3 : 0.26) * nkb;
+  for (int sk = 1; sk <= 64 && sk * 8 <= nkb; sk += sk < 4 ? 1 : sk < 8 ? 2 : sk < 16 ? 4 : 16) {
+    const double items = (double)((tiles * sk + slots - 1) / slots);
+    double waves = sk <= 4 ? items / sk + 0.03 * (sk - 1) : items * (1.0 / sk + 8.0 / nkb) + 0.09;
+    if (sk > 1) waves += (2.0 + (double)M * N * (1 + 2 * sk) / 1.25e6) / whole_us;
+    if (waves < best - 1e-9) { best = waves; g.parts = sk; }
+  }
+  g.ordered = g.parts > 1;
+  return g;
+}
+
+// KiB of workspace with which pf_gemm (conv 0) or pf_conv_wgrad (conv 2: M = Cout, N = KH * KW * C,
+// K = B * Ho * Wo) splits the reduction of an fp32 output with nothing fused into its epilogue; 0 when
+// it stays whole.  Without the workspace such a call is not split.
+PF_API int pf_gemm_workspace(int M, int N, int K, int accumulate, int conv, int sm_count, int tile_n) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  const GemmPlan g = gemm_plan(M, N, K, PF_F32, accumulate, conv, false, true, tile_n,
+                               sm_count > 0 ? sm_count : 148);
+  return (int)((g.ws_floats() + 255) / 256);
+}
+
+PF_API int pf_gemm(const void* A, const void* B, void* C, int M, int N, int K, long long lda,
+                   long long ldb, long long ldc, int a_mn, int b_mn, int in_dtype, int out_dtype,
+                   const void* bias, int bias_dtype, const void* residual, long long ldr,
+                   void* aux, long long ldaux, int epilogue, int accumulate, float alpha,
+                   int* status, int sm_count, int tile_n, void* workspace, int workspace_kib,
+                   void* stream) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if (in_dtype != PF_F16 && in_dtype != PF_BF16) return -1;
+  if ((g_conv.on != 1 && (lda % 8)) || (g_conv.on != 2 && (ldb % 8)) ||
+      (reinterpret_cast<uintptr_t>(A) & 15) ||
+      (reinterpret_cast<uintptr_t>(B) & 15))
+    return -2;  // TMA needs 16-byte aligned bases and pitches
+  const int fmt = in_dtype == PF_BF16 ? 1 : 0;
+  // tile_n: low bits 0 / 128 / 256 = tile width of the single-CTA form; bit 10 forces the
+  // direct-store epilogue, bit 11 forces the CTA-pair form, bit 12 forbids it, bit 13 forbids
+  // the split reduction (tests, benches).  workspace: pf_gemm_workspace, 16-byte aligned
+  if (sm_count <= 0) sm_count = 148;
+  const size_t es = out_dtype == PF_F32 ? 4 : 2;
+  auto aligned = [&](const void* ptr, long long ld) {
+    return ptr == nullptr || ((reinterpret_cast<uintptr_t>(ptr) & 15) == 0 && (ld * es) % 16 == 0);
+  };
+  const bool vec_ok = aligned(C, ldc) && aligned(residual, ldr) && aligned(aux, ldaux);
+  const bool may_split = vec_ok && !bias && !residual && !aux && epilogue == EPI_NONE;
+  GemmPlan plan = gemm_plan(M, N, K, out_dtype, accumulate, g_conv.on, g_gather.on_any(), may_split,
+                            tile_n, sm_count);
+  if (plan.ordered && (!workspace || workspace_kib * 256ll < plan.ws_floats())) {
+    plan.parts = 1;
+    plan.ordered = false;
+  }
+  const bool pair = plan.pair;
+  const int BN = plan.bn;
 
   CUtensorMap ta, tb;
   int r;
@@ -898,54 +1031,28 @@ PF_API int pf_gemm(const void* A, const void* B, void* C, int M, int N, int K, l
     p.conv_c64 = g_conv.C / 64; p.conv_kw = g_conv.KW; p.conv_pad = g_conv.pad;
     p.conv_stride = g_conv.stride; p.conv_wo = g_conv.Wo; p.conv_howo = g_conv.Ho * g_conv.Wo;
   }
-  const size_t es = out_dtype == PF_F32 ? 4 : 2;
-  auto aligned = [&](const void* ptr, long long ld) {
-    return ptr == nullptr || ((reinterpret_cast<uintptr_t>(ptr) & 15) == 0 && (ld * es) % 16 == 0);
-  };
-  p.vec_ok = aligned(C, ldc) && aligned(residual, ldr) && aligned(aux, ldaux);
+  p.vec_ok = vec_ok;
   // TMA-store epilogue: needs aligned outputs; fp32 accumulation uses the reduce-add store,
   // 16-bit accumulation (unused by the framework) stays on the direct path
   p.tma_store = p.vec_ok && !(accumulate && out_dtype != PF_F32) && !(tile_n & 1024) &&
                 !(aux && out_dtype == PF_F32);
-  // Split-K: a gradient-accumulating GEMM whose tiles do not fill the GPU divides each tile's
-  // reduction among several work items; they all reduce-add into C, which costs nothing extra
-  // because the epilogue accumulates anyway.  Other fp32 outputs, above all weight gradients of
-  // convolutions, whose long reduction over the output pixels meets few tiles, are split too: C is
-  // small beside the operands and is cleared first (3 x 3, 320 filters of 320 channels over
-  // [4, 128, 128]: 24 pair tiles, 301 us whole, 123 in three).
-  p.split_k = 1;
-  const bool clear_first = !accumulate && ldc == N;
-  if (p.vec_ok && out_dtype == PF_F32 && (accumulate || clear_first) && !(tile_n & 1024) && !aux &&
-      !g_gather.on_any() && g_conv.on != 1 && !bias && !residual && epilogue == EPI_NONE &&
-      !(tile_n & 8192)) {
-    const int bm = pair ? 256 : 128, bn = pair ? 256 : BN;
-    const long long tiles = (long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn);
-    const long long slots = pair ? sm_count / 2 : sm_count;
-    const int nkb = (K + GEMM_BK - 1) / GEMM_BK;
-    double best = 1e30;
-    // Very few tiles under a very long reduction: up to 64 parts, each of which costs its first loads
-    // and its epilogue, some 8 k-blocks (320 x 72 x 65536: 282 us whole, 21 in 48).
-    for (int sk = 1; sk <= 64 && sk * 8 <= nkb; sk += sk < 4 ? 1 : sk < 8 ? 2 : sk < 16 ? 4 : 16) {
-      const double items = (double)((tiles * sk + slots - 1) / slots);
-      double waves = sk <= 4 ? items / sk + 0.03 * (sk - 1) : items * (1.0 / sk + 8.0 / nkb) + 0.09;
-      // clearing C and adding to it from L2 moves some 4 MB per us, a k-block of a full wave takes
-      // 0.36 us ([1, 32, 32, 1280] with 1280 filters, 59 MB of C: 40 us whole, 60 in two)
-      if (clear_first && sk > 1)
-        waves += (double)M * N * (1 + 2 * sk) / 1e6 / (0.36 * nkb);
-      if (waves < best - 1e-9) { best = waves; p.split_k = sk; }
-    }
+  p.split_k = plan.parts;
+  p.part_rows = 0;
+  void* dst = C;
+  long long dst_rows = M, dst_ld = ldc;
+  if (plan.ordered) {
+    p.accumulate = 0;
+    p.part_rows = plan.rows;
+    dst = workspace;
+    dst_rows = (long long)plan.parts * plan.rows;
+    dst_ld = plan.pitch;
   }
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (p.split_k > 1 && clear_first) {
-    cudaError_t e = cudaMemsetAsync(C, 0, sizeof(float) * (size_t)M * (size_t)N, st);
-    if (e != cudaSuccess) return (int)e;
-    p.accumulate = 1;
-  }
   CUtensorMap tc, taux;
   memset(&tc, 0, sizeof(tc));
   memset(&taux, 0, sizeof(taux));
   if (p.tma_store) {
-    if ((r = make_tmap_out(&tc, C, out_dtype, N, M, ldc))) return r;
+    if ((r = make_tmap_out(&tc, dst, out_dtype, N, dst_rows, dst_ld))) return r;
     const bool aux_is_out = aux && (epilogue == EPI_GELU || epilogue == EPI_GELU_TANH ||
                                     epilogue == EPI_SILU);
     if (aux_is_out && (r = make_tmap_out(&taux, aux, out_dtype, N, M, ldaux))) return r;
@@ -958,7 +1065,17 @@ PF_API int pf_gemm(const void* A, const void* B, void* C, int M, int N, int K, l
    : BN == 256 ? launch_gemm<T, 256, 4, 4096, false, false>(ta, tb, tc, taux, p, sm_count, st) \
                : launch_gemm<T, 128, 5, 8192, false, false>(ta, tb, tc, taux, p, sm_count, st))
   switch (out_dtype) {
-    case PF_F32: return PF_GEMM_DISPATCH(float);
+    case PF_F32: {
+      if ((r = PF_GEMM_DISPATCH(float)) || !plan.ordered) return r;
+      const long long part = (long long)plan.rows * plan.pitch, quads = (long long)M * (plan.pitch / 4);
+      const bool wide = quads >= 256ll * sm_count;
+      const unsigned grid = (unsigned)(((wide ? quads : (long long)M * N) + 255) / 256);
+      auto fold = wide ? gemm_fold_kernel<4> : gemm_fold_kernel<1>;
+      fold<<<grid, 256, 0, st>>>((const float*)workspace, (float*)C, M, N, plan.parts, part,
+                                 plan.pitch, ldc, accumulate);
+      PF_CHECK_LAUNCH();
+      return 0;
+    }
     case PF_F16: return PF_GEMM_DISPATCH(__half);
     case PF_BF16: return PF_GEMM_DISPATCH(__nv_bfloat16);
   }
@@ -993,7 +1110,7 @@ PF_API int pf_gemm_allgather(const void* A, void* w_full, void* const* copies, i
   }
   const int r = pf_gemm(A, w_full, C, M, N, K, lda, ldb, ldc, 0, 0, in_dtype, out_dtype, bias,
                         bias_dtype, residual, ldr, aux, ldaux, epilogue, 0, alpha, status,
-                        sm_count, 256, stream);
+                        sm_count, 256, nullptr, 0, stream);
   g_gather = GatherArgs();
   return r;
 }
@@ -1014,7 +1131,7 @@ PF_API int pf_conv_gemm(const void* x, const void* w2, void* y, int B, int H, in
   g_conv.KW = KW; g_conv.stride = stride; g_conv.pad = pad; g_conv.Ho = Ho; g_conv.Wo = Wo;
   const int r = pf_gemm(x, w2, y, B * Ho * Wo, Cout, KH * KW * C, 0, ldw, ldy, 0, 0, in_dtype,
                         out_dtype, bias, bias_dtype, residual, ldr, nullptr, 0, epilogue, 0, 1.0f,
-                        status, sm_count, 0, stream);
+                        status, sm_count, 0, nullptr, 0, stream);
   g_conv = ConvArgs();
   return r;
 }
@@ -1025,7 +1142,8 @@ PF_API int pf_conv_gemm(const void* x, const void* w2, void* y, int B, int H, in
 // a multiple of it, (Ho * Wo) % 64 == 0, stride 1 or 2; returns -3 otherwise.
 PF_API int pf_conv_wgrad(const void* dy, const void* x, void* dw2, int B, int H, int W, int C,
                          int Cout, int KH, int KW, int stride, int pad, int in_dtype,
-                         int accumulate, int* status, int sm_count, void* stream) {
+                         int accumulate, int* status, int sm_count, void* workspace,
+                         int workspace_kib, void* stream) {
   const int Ho = (H + 2 * pad - KH) / stride + 1, Wo = (W + 2 * pad - KW) / stride + 1;
   if (C % 64 || Cout % 8 || Wo <= 0 || (64 % Wo && Wo % 64) || (Ho * Wo) % 64 ||
       (stride != 1 && stride != 2))
@@ -1034,7 +1152,8 @@ PF_API int pf_conv_wgrad(const void* dy, const void* x, void* dw2, int B, int H,
   g_conv.KW = KW; g_conv.stride = stride; g_conv.pad = pad; g_conv.Ho = Ho; g_conv.Wo = Wo;
   const int r = pf_gemm(dy, x, dw2, Cout, KH * KW * C, B * Ho * Wo, Cout, 0,
                         (long long)KH * KW * C, 1, 1, in_dtype, PF_F32, nullptr, 0, nullptr, 0,
-                        nullptr, 0, 0, accumulate, 1.0f, status, sm_count, 0, stream);
+                        nullptr, 0, 0, accumulate, 1.0f, status, sm_count, 0, workspace,
+                        workspace_kib, stream);
   g_conv = ConvArgs();
   return r;
 }

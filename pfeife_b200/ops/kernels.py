@@ -88,6 +88,13 @@ def poll_status(device=None) -> None:
     ent["event"] = ev
 
 
+def _split_workspace(L, M: int, N: int, K: int, accumulate: bool, conv: int, tile_n: int, device
+                     ) -> Tuple[Optional[torch.Tensor], int]:
+    """(workspace, KiB) in which the parts of a split reduction wait to be added in their order."""
+    kib = L.pf_gemm_workspace(M, N, K, int(accumulate), conv, sm_count(device), tile_n)
+    return (torch.empty(kib * 256, dtype=torch.float32, device=device) if kib else None), kib
+
+
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False,
          out: Optional[torch.Tensor] = None, out_dtype: Optional[torch.dtype] = None,
          bias: Optional[torch.Tensor] = None, residual: Optional[torch.Tensor] = None,
@@ -117,12 +124,17 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         assert residual.shape == (M, N) and residual.dtype == out.dtype and residual.stride(1) == 1
     if aux is not None:
         assert aux.shape == (M, N) and aux.dtype == out.dtype and aux.stride(1) == 1
+    ws, kib = None, 0
+    if out.dtype == torch.float32 and not accumulate and epilogue == EPI_NONE and bias is None \
+            and residual is None and aux is None:
+        ws, kib = _split_workspace(L, M, N, K, False, 0, tile_n, a.device)
     code = L.pf_gemm(a, b, out, M, N, K, a.stride(0), b.stride(0),
                      out.stride(0), int(a_mn), int(b_mn), dt(a.dtype), dt(out.dtype),
                      bias, dt(bias.dtype) if bias is not None else 0, residual,
                      residual.stride(0) if residual is not None else 0, aux,
                      aux.stride(0) if aux is not None else 0, epilogue, int(accumulate),
-                     alpha, status_word(a.device), sm_count(a.device), tile_n, stream_of(a))
+                     alpha, status_word(a.device), sm_count(a.device), tile_n, ws, kib,
+                     stream_of(a))
     if code != 0:
         check(code, f"pf_gemm(M={M}, N={N}, K={K}, a={tuple(a.shape)}/{a.stride()}/{a.dtype}/"
                     f"{a.data_ptr() % 256}, b={tuple(b.shape)}/{b.stride()}/{b.data_ptr() % 256}, "
@@ -571,9 +583,10 @@ def conv_wgrad(dy2: torch.Tensor, x: torch.Tensor, KH: int, KW: int, stride: int
     if out is None:
         out = torch.empty((Cout, KH * KW * C), dtype=torch.float32, device=x.device)
         accumulate = False
+    ws, kib = _split_workspace(L, Cout, KH * KW * C, dy2.shape[0], accumulate, 2, 0, x.device)
     check(L.pf_conv_wgrad(dy2, x, out, B, H, W, C, Cout, KH, KW, stride, pad,
                           dt(x.dtype), int(accumulate), status_word(x.device),
-                          sm_count(x.device), stream_of(dy2)), "pf_conv_wgrad")
+                          sm_count(x.device), ws, kib, stream_of(dy2)), "pf_conv_wgrad")
     return out
 
 

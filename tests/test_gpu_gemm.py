@@ -184,8 +184,8 @@ def test_gemm_around_one_round_of_small_tiles(M, N, K):
 @pytest.mark.parametrize("M,N,K,a_mn,b_mn", [(320, 72, 32768, True, True), (8, 2880, 4096, True, True),
                                              (128, 128, 512, False, False), (136, 72, 4160, False, True)])
 def test_gemm_fp32_output_split_into_many_parts(M, N, K, a_mn, b_mn):
-    """Few tiles under a long reduction, written and not accumulated: the parts add into an output that
-    held something else before."""
+    """Few tiles under a long reduction, written and not accumulated, into an output that held something
+    else before."""
     from pfeife_b200.ops import kernels as kx
     a, b = _mk(M, N, K, a_mn, b_mn, torch.bfloat16)
     out = torch.full((M, N), float("nan"), device="cuda")
@@ -260,3 +260,20 @@ def test_dgelu_epilogue_by_value():
     assert ((got - want) / want)[tail].abs().max().item() < 1e-5
     exact = 0.5 * torch.erfc(-x * 0.5 ** 0.5) + x * torch.exp(-x * x / 2) * 0.3989422804014327
     assert (got - exact)[~tail].abs().max().item() < 4e-7
+
+
+@pytest.mark.parametrize("M,N,K,a_mn,b_mn", [(320, 72, 32768, True, True), (130, 260, 4104, False, False),
+                                             (8, 2880, 16384, True, True), (592, 1408, 6168, True, True)])
+def test_gemm_split_outputs_repeat(M, N, K, a_mn, b_mn):
+    """An fp32 output has the same bits every time, however its reduction is divided; also into rows
+    longer than the output's, whose rest stays as it is."""
+    from pfeife_b200.ops import _lib, kernels as kx
+    assert _lib.calls().pf_gemm_workspace(M, N, K, 0, 0, 148, 0) > 0
+    a, b = _mk(M, N, K, a_mn, b_mn, torch.bfloat16)
+    first = kx.gemm(a, b, a_mn=a_mn, b_mn=b_mn, out_dtype=torch.float32)
+    for _ in range(20):
+        assert torch.equal(kx.gemm(a, b, a_mn=a_mn, b_mn=b_mn, out_dtype=torch.float32), first)
+    wide = torch.full((M, N + 8), 3.0, device="cuda")
+    kx.gemm(a, b, a_mn=a_mn, b_mn=b_mn, out=wide[:, :N])
+    assert torch.equal(wide[:, :N], first) and (wide[:, N:] == 3).all()
+    kx.check_status()

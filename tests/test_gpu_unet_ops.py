@@ -226,13 +226,13 @@ def test_conv_weight_kernels_move_every_element(Cout, Cin, taps):
 @pytest.mark.parametrize("batch,hw,cin,cout,stride", [
     (1, 8, 64, 64, 1),        # one k-block per image row group, one tile, nothing to split
     (3, 8, 128, 72, 1),       # k-blocks of eight output rows, image after image
-    (2, 32, 64, 320, 1),      # the reduction in several parts: C is cleared and added to
+    (2, 32, 64, 320, 1),      # the reduction in several parts
     (2, 128, 64, 64, 1),      # a k-block is half an output row
     (2, 32, 64, 128, 2),      # stride 2: 16 x 16 outputs
 ])
 def test_conv_wgrad_steps_through_pixels(batch, hw, cin, cout, stride):
     """Weight gradients over every way a k-block of 64 output pixels can lie in an image, also into a
-    buffer that holds something else before (the split reduction clears it).  Products are exact in
+    buffer that holds something else before.  Products are exact in
     fp32, so only the order of the sums differs: 2^-24 of the root of the number of terms."""
     from pfeife_b200.ops import kernels as kx
     torch.manual_seed(3)
@@ -288,3 +288,24 @@ def test_conv_gradients_of_any_kernel_shape(KH, KW, pad, H, W, cout):
     for got, want in ((y, ref), (dx, refx), (dw, refw)):
         assert got.shape == want.shape
         assert ((got - want).norm() / want.norm()).item() < 1.5 * 2.0 ** -9
+
+
+@pytest.mark.parametrize("batch,hw,cin,cout,stride", [(2, 32, 64, 320, 1), (2, 128, 320, 8, 1),
+                                                      (4, 64, 320, 320, 2)])
+def test_conv_weight_gradients_repeat(batch, hw, cin, cout, stride):
+    """The same bits every time, written and accumulated, where the reduction is divided."""
+    from pfeife_b200.ops import _lib, kernels as kx
+    torch.manual_seed(4)
+    x = torch.randn(batch, hw, hw, cin, device="cuda").to(torch.bfloat16)
+    ho = (hw - 1) // stride + 1
+    dy = torch.randn(batch * ho * ho, cout, device="cuda").to(torch.bfloat16)
+    assert _lib.calls().pf_gemm_workspace(cout, 9 * cin, batch * ho * ho, 0, 2, 148, 0) > 0
+    start = torch.randn(cout, 9 * cin, device="cuda")
+    first = None
+    for _ in range(20):
+        got = (kx.conv_wgrad(dy, x, 3, 3, stride, 1),
+               kx.conv_wgrad(dy, x, 3, 3, stride, 1, out=start.clone(), accumulate=True))
+        first = first or got
+        assert all(torch.equal(a, b) for a, b in zip(got, first))
+    assert torch.equal(first[1], start + first[0])
+    kx.check_status()

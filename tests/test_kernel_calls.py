@@ -25,7 +25,7 @@ def calls(request, monkeypatch):
 
 def _gemm(calls, a, b, M=8, dtype=_lib.PF_BF16, lda=64, alpha=1.0):
     return calls.pf_gemm(a, b, None, M, 8, 64, lda, 64, 8, 0, 0, dtype, dtype, None, 0, None, 0, None, 0,
-                         0, 0, alpha, None, 148, 0, None)
+                         0, 0, alpha, None, 148, 0, None, 0, None)
 
 
 def test_values_arrive(calls):
