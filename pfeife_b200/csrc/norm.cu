@@ -682,7 +682,7 @@ static int norm_fwd_launch(const void* x, const void* res, const float* gamma, c
 template <typename T>
 static int norm_bwd_launch(const void* dy, const void* h, const float* gamma, const float* mean,
                            const float* rstd, const void* dres, void* dx, float* scratch, int& G,
-                           long long rows, int N, int rms, cudaStream_t st) {
+                           long long rows, int N, int rms, int sm_count, cudaStream_t st) {
   constexpr int V = 16 / sizeof(T);
   if (N % V) return -2;
   const int nvec = N / V;
@@ -697,7 +697,7 @@ static int norm_bwd_launch(const void* dy, const void* h, const float* gamma, co
   }
   if constexpr (sizeof(T) == 2) if (nvec <= 32 * 16) {
     // rows of up to 4096 16-bit elements (Llama's hidden size): one CTA per SM fills its shared memory
-    if (G > 148) G = 148;
+    if (G > sm_count) G = sm_count;
 #define PF_NORM_BWD_WIDE(THREADS)                                                                 \
     norm_bwd_wide_launch<T, THREADS>(dy, h, gamma, mean, rstd, dres, dx, scratch, G, rows, N, rms, st)
     return nvec <= 384 ? PF_NORM_BWD_WIDE(384) : PF_NORM_BWD_WIDE(512);
@@ -751,13 +751,14 @@ PF_API int pf_norm_bwd(const void* dy, const void* h, const void* gamma, const v
                        void* scratch, long long rows, int N, int rms, int accumulate, int dtype,
                        int sm_count, void* stream) {
   if (rows <= 0) return 0;
+  if (sm_count <= 0) sm_count = 148;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   int G = pf_norm_bwd_ctas(rows, sm_count);   // rows of scratch; the launch may use fewer
   int r = -1;
   switch (dtype) {
-    case PF_F32: r = norm_bwd_launch<float>(dy, h, (const float*)gamma, (const float*)mean, (const float*)rstd, dres, dx, (float*)scratch, G, rows, N, rms, st); break;
-    case PF_F16: r = norm_bwd_launch<__half>(dy, h, (const float*)gamma, (const float*)mean, (const float*)rstd, dres, dx, (float*)scratch, G, rows, N, rms, st); break;
-    case PF_BF16: r = norm_bwd_launch<__nv_bfloat16>(dy, h, (const float*)gamma, (const float*)mean, (const float*)rstd, dres, dx, (float*)scratch, G, rows, N, rms, st); break;
+    case PF_F32: r = norm_bwd_launch<float>(dy, h, (const float*)gamma, (const float*)mean, (const float*)rstd, dres, dx, (float*)scratch, G, rows, N, rms, sm_count, st); break;
+    case PF_F16: r = norm_bwd_launch<__half>(dy, h, (const float*)gamma, (const float*)mean, (const float*)rstd, dres, dx, (float*)scratch, G, rows, N, rms, sm_count, st); break;
+    case PF_BF16: r = norm_bwd_launch<__nv_bfloat16>(dy, h, (const float*)gamma, (const float*)mean, (const float*)rstd, dres, dx, (float*)scratch, G, rows, N, rms, sm_count, st); break;
   }
   if (r) return r;
   PF_CHECK_LAUNCH();

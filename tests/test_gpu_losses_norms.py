@@ -278,3 +278,20 @@ def test_group_norm_forms_of_the_backward(B, H, W, C, G, silu):
     """The largest CTA with a ring of pixels, the form without one, and more pixels per thread than a
     ring has places."""
     test_group_norm_edges(B, H, W, C, G, silu, torch.bfloat16)
+
+
+def test_norm_backward_wide_rows_on_some_of_the_sms():
+    """The caller's number of SMs bounds the CTAs, each of which writes one row of scratch."""
+    from pfeife_b200.ops import _lib
+    rows, N, sms = 1000, 3072, 16
+    L = _lib.calls()
+    h, dy = (torch.randn(rows, N, device="cuda").to(torch.bfloat16) for _ in range(2))
+    w = torch.ones(N, device="cuda")
+    mean, rstd = torch.zeros(rows, device="cuda"), torch.ones(rows, device="cuda")
+    scratch = torch.full((L.pf_norm_bwd_ctas(rows, sms), 2, N), float("nan"), device="cuda")
+    dx, dw, db = torch.empty_like(h), torch.empty_like(w), torch.empty_like(w)
+    assert L.pf_norm_bwd(dy, h, w, mean, rstd, None, dx, dw, db, scratch, rows, N, 1, 0, _lib.PF_BF16, sms,
+                         _lib.stream_of(h)) == 0
+    assert scratch[:sms].isfinite().all() and scratch[sms:].isnan().all()
+    want = (dy.double() * h.double()).sum(0)
+    assert (dw - want).norm() <= 1e-5 * want.norm()
