@@ -203,9 +203,9 @@ conv_unpack_kernel(const float* __restrict__ src, T* __restrict__ dw, int Cin, i
 // rows of C/8 threads in a CTA
 static inline int gn_rows(int C) { const int ncv = C / 8; return ncv >= 256 ? 1 : 256 / ncv; }
 
-// Slabs of pixels per image, at least eight pixels per thread.  `per_sm` CTAs per SM make one
-// wave: 4 of the forward's at 56 registers, 3 of the backward's at 80 (4 left a third of them to a
-// second wave: 110 us against 83).
+// Slabs of pixels per image, at least eight pixels per thread.  `per_sm` CTAs of up to 256 threads per
+// SM make one wave: 4 of the forward's at 56 registers, 3 of the backward's at 80 (4 left a third of
+// them to a second wave: 110 us against 83).
 constexpr int GN_FWD_PER_SM = 4, GN_BWD_PER_SM = 3;
 static inline int gn_slabs(int B, int HW, int rows, int sm_count, int per_sm) {
   int slabs = (per_sm * (sm_count > 0 ? sm_count : 148)) / B;
@@ -216,9 +216,12 @@ static inline int gn_slabs(int B, int HW, int rows, int sm_count, int per_sm) {
 
 // The backward's two passes over dy and x run out of registers before they have enough loads under
 // way: each thread keeps a ring of its next pixels in shared memory, filled by asynchronous copies of
-// its own, which needs no barriers.  Three sizes of CTA: up to 256 threads (2048 channels) and up to 400
-// with a ring, beyond without (at 80 registers no more than 800 threads fit).  Backward, both passes
-// and the fold, L2 flushed: [4, 128, 128, 320] 78 -> 64 us, [4, 128, 128, 640] 141 -> 102,
+// its own, which needs no barriers.  Four sizes of CTA: up to 256 threads (2048 channels) and up to 400
+// with a ring, up to 800 and up to 1024 (8192 channels) without.  They compile to 80, 72, 72 and 64
+// registers; the second pass with SiLU spills 44, 64, 96 and 176 bytes per thread, the first 4, 32, 0 and
+// 256, the others next to nothing.  Up to 256 threads three CTAs share an SM, up to 400 two, beyond one,
+// while the slabs are cut for three: wider images take more than one wave.  Backward, both passes and
+// the fold, L2 flushed: [4, 128, 128, 320] 78 -> 64 us, [4, 128, 128, 640] 141 -> 102,
 // [4, 64, 64, 1920] 108 -> 85, [4, 32, 32, 2560] 65 -> 57.
 constexpr int GN_RING = 6, GN_RING_THREADS = 400;
 // fold and ring of 400 threads
@@ -542,6 +545,7 @@ gn_bwd_apply_kernel(const T* __restrict__ dy, const T* __restrict__ x,
   });
 }
 
+// nearest 2x upsample (NHWC) and its backward (sum of the 4 children)
 template <typename T>
 __global__ void __launch_bounds__(256)
 upsample2x_kernel(const T* __restrict__ x, T* __restrict__ y, int B, int H, int W, int C,
@@ -635,30 +639,6 @@ PF_API int pf_groupnorm_slabs(int B, int HW, int C, int sm_count) {
     else KERN<T, false><<<grid, threads, smem, st>>>(__VA_ARGS__);         \
   } while (0)
 
-PF_API int pf_groupnorm_fwd(const void* x, const void* gamma, const void* beta, void* y,
-                            void* mean, void* rstd, void* scratch, int B, int HW, int C, int G,
-                            float eps, int act_silu, int dtype, int sm_count, void* stream) {
-  if (C % G || C % 8) return -2;
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  const int rows = gn_rows(C);
-  const int threads = rows * (C / 8);
-  if (threads > 1024) return -2;
-  const int slabs = gn_slabs(B, HW, rows, sm_count, GN_FWD_PER_SM);
-  const dim3 grid(slabs, B);
-  PF_DISPATCH_H(dtype, {
-    gn_stats_kernel<T><<<grid, threads, gn_smem(rows, C), st>>>((const T*)x, (float*)scratch, HW,
-                                                               C, G, rows);
-    gn_finalize_kernel<<<(B * G + 3) / 4, 128, 0, st>>>(
-        (const float*)scratch, (float*)mean, (float*)rstd, slabs, G, B * G,
-        1.f / ((float)HW * (C / G)), eps);
-    const int smem = 0;
-    PF_GN_SILU(gn_apply_kernel, (const T*)x, (const float*)mean, (const float*)rstd,
-               (const float*)gamma, (const float*)beta, (T*)y, HW, C, G, rows);
-  });
-  PF_CHECK_LAUNCH();
-  return 0;
-}
-
 // `done`: per kernel and device, whether it may already use more than 48 KB of shared memory
 template <typename... P, typename... A>
 static int gn_launch(void (*kern)(P...), bool* done, dim3 grid, int threads, int smem,
@@ -672,14 +652,42 @@ static int gn_launch(void (*kern)(P...), bool* done, dim3 grid, int threads, int
     if (dev >= 0 && dev < 64) done[dev] = true;
   }
   kern<<<grid, threads, smem, st>>>(args...);
+  return (int)cudaGetLastError();
+}
+
+PF_API int pf_groupnorm_fwd(const void* x, const void* gamma, const void* beta, void* y,
+                            void* mean, void* rstd, void* scratch, int B, int HW, int C, int G,
+                            float eps, int act_silu, int dtype, int sm_count, void* stream) {
+  if (C % G || C % 8) return -2;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  const int rows = gn_rows(C);
+  const int threads = rows * (C / 8);
+  if (threads > 1024) return -2;
+  const int slabs = gn_slabs(B, HW, rows, sm_count, GN_FWD_PER_SM);
+  const dim3 grid(slabs, B);
+  PF_DISPATCH_H(dtype, {
+    static bool done[64] = {};
+    const int r = gn_launch(gn_stats_kernel<T>, done, grid, threads, gn_smem(rows, C), st,
+                            (const T*)x, (float*)scratch, HW, C, G, rows);
+    if (r) return r;
+    gn_finalize_kernel<<<(B * G + 3) / 4, 128, 0, st>>>(
+        (const float*)scratch, (float*)mean, (float*)rstd, slabs, G, B * G,
+        1.f / ((float)HW * (C / G)), eps);
+    const int smem = 0;
+    PF_GN_SILU(gn_apply_kernel, (const T*)x, (const float*)mean, (const float*)rstd,
+               (const float*)gamma, (const float*)beta, (T*)y, HW, C, G, rows);
+  });
+  PF_CHECK_LAUNCH();
   return 0;
 }
+
 template <typename F>
 static int gn_bwd_launch(int act_silu, int threads, F f) {
   auto sized = [&](auto silu) {
     if (threads <= 256) return f(silu, std::integral_constant<int, 256>());
     if (threads <= GN_RING_THREADS) return f(silu, std::integral_constant<int, GN_RING_THREADS>());
-    return f(silu, std::integral_constant<int, 800>());
+    if (threads <= 800) return f(silu, std::integral_constant<int, 800>());
+    return f(silu, std::integral_constant<int, 1024>());
   };
   return act_silu ? sized(std::true_type()) : sized(std::false_type());
 }

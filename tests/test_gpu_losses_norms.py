@@ -295,3 +295,11 @@ def test_norm_backward_wide_rows_on_some_of_the_sms():
     assert scratch[:sms].isfinite().all() and scratch[sms:].isnan().all()
     want = (dy.double() * h.double()).sum(0)
     assert (dw - want).norm() <= 1e-5 * want.norm()
+
+
+@pytest.mark.parametrize("silu", [True, False])
+@pytest.mark.parametrize("C", [6144, 6152, 6400, 6408, 8192])
+def test_group_norm_of_many_channels(C, silu):
+    """Sums of more than 6144 channels take more than 48 KB of shared memory, and beyond 6400 a CTA has
+    more than 800 threads."""
+    test_group_norm_edges(1, 5, 5, C, 8, silu, torch.bfloat16)
