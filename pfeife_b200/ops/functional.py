@@ -1283,12 +1283,12 @@ def conv2d_bwd(dy: Tensor, x: Tensor, w: Tensor, stride: int, pad: int, need_dx:
         dx = dy.new_empty(0)
         if need_dx:
             dy4 = dy2.view(B, -1, dy.shape[2], cout8)
-            # Few filters are padded to the 64 channels the implicit GEMM reads at a time: its sums
+            # Up to 64 filters are padded to the 64 channels the implicit GEMM reads at a time: its sums
             # stay in fp32 and no [pixels, taps * Cin] buffer is written and read (4 filters over
             # [4, 128, 128, 320]: 314 us through that buffer, 37 padded).
-            wide = 64 if cout8 < 64 else cout8
+            wide = max(cout8, 64)
             # One padding, KH - 1 - pad, serves both axes of that route: square kernels only.
-            if not one and stride == 1 and KH == KW and (cout8 == Cout or wide != cout8) and \
+            if not one and stride == 1 and KH == KW and (cout8 == Cout or wide == 64) and \
                     kx.conv_gemm_supported(dy4, KH, KW, 1, KH - 1 - pad, wide):
                 # dx = correlation of dy with the taps flipped and the channel roles swapped
                 if wide != cout8:

@@ -251,19 +251,25 @@ def test_conv_wgrad_steps_through_pixels(batch, hw, cin, cout, stride):
     assert ((more - 2 * ref).norm() / ref.norm()).item() < 2e-5
 
 
-@pytest.mark.parametrize("cout,hw", [(4, 16), (8, 32), (56, 16), (3, 128)])
-def test_conv_input_gradient_of_few_filters(cout, hw):
-    """Fewer than 64 filters: the gradient is padded to the width the implicit GEMM reads.  fp32 sums
-    and one rounding: u = 2^-8 at most, half of it on average."""
+@pytest.mark.parametrize("cout,hw", [(4, 16), (8, 32), (56, 16), (3, 128), (60, 16), (64, 16)])
+def test_conv_input_gradient_of_few_filters(cout, hw, monkeypatch):
+    """Up to 64 filters: the gradient is padded to the width the implicit GEMM reads.  fp32 sums and one
+    rounding: the error is that of the exact result rounded to 16 bits, give or take the roundings that
+    fp32 sums of up to 576 terms turn (columns of 16 bits would add as much again)."""
     from pfeife_b200 import ops
+    from pfeife_b200.ops import kernels as kx
     torch.manual_seed(6)
     x = torch.randn(2, hw, hw, 64, device="cuda").to(torch.bfloat16).requires_grad_()
     w = (torch.randn(cout, 64, 3, 3, device="cuda") * 0.1).to(torch.bfloat16)
     gy = torch.randn(2, hw, hw, cout, device="cuda").to(torch.bfloat16)
-    dx, = torch.autograd.grad(ops.conv2d(x, w, None, 1, 1), x, gy)
+    y = ops.conv2d(x, w, None, 1, 1)
+    calls, conv_gemm = [], kx.conv_gemm
+    monkeypatch.setattr(kx, "conv_gemm", lambda *a, **k: calls.append(1) or conv_gemm(*a, **k))
+    dx, = torch.autograd.grad(y, x, gy)
+    assert calls
     ref = torch.nn.grad.conv2d_input((2, 64, hw, hw), w.double(), gy.double().permute(0, 3, 1, 2),
                                      padding=1).permute(0, 2, 3, 1)
-    assert ((dx - ref).norm() / ref.norm()).item() < 2.0 ** -8
+    assert (dx - ref).norm() < 1.1 * (ref.to(torch.bfloat16) - ref).norm()
 
 
 @pytest.mark.parametrize("KH,KW,pad,H,W,cout", [
