@@ -177,8 +177,9 @@ def test_gemm_around_one_round_of_small_tiles(M, N, K):
     out = kx.gemm(a, b, out_dtype=torch.float32)
     ref = a.double() @ b.double().t()
     kx.check_status()
-    # products of 16-bit values are exact in fp32; K fp32 additions in some order
-    assert ((out - ref).norm() / ref.norm()).item() < K * 2.0 ** -24
+    # products of 16-bit values are exact in fp32; K fp32 additions in some order, whose roundings add
+    # up like a random walk over sums that grow like one: sqrt(K) 2^-24 at most
+    assert ((out - ref).norm() / ref.norm()).item() < K ** 0.5 * 2.0 ** -24
 
 
 @pytest.mark.parametrize("M,N,K,a_mn,b_mn", [(320, 72, 32768, True, True), (8, 2880, 4096, True, True),
@@ -192,8 +193,9 @@ def test_gemm_fp32_output_split_into_many_parts(M, N, K, a_mn, b_mn):
     kx.gemm(a, b, a_mn=a_mn, b_mn=b_mn, out=out)
     ref = (a.double().t() if a_mn else a.double()) @ (b.double() if b_mn else b.double().t())
     kx.check_status()
-    # products of 16-bit values are exact in fp32; K fp32 additions in some order
-    assert ((out - ref).norm() / ref.norm()).item() < K * 2.0 ** -24
+    # products of 16-bit values are exact in fp32; K fp32 additions in some order, whose roundings add
+    # up like a random walk over sums that grow like one: sqrt(K) 2^-24 at most
+    assert ((out - ref).norm() / ref.norm()).item() < K ** 0.5 * 2.0 ** -24
 
 
 def _pieces(z):
