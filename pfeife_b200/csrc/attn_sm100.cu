@@ -743,10 +743,11 @@ PF_API int pf_attn_fwd(const void* q, const void* k, const void* v, void* o, voi
   // Pairs left over after whole rounds are split into tiles when these fit one round (FwdItem).  The
   // form of the kernel that can do both takes 4 to 9 % longer over a pair: up to three rounds it gains
   // all the same ([4, 1024, 20, 64] 56 us whole, 48 split, [2, 2048, 20, 128] 116 and 103), after more
-  // it does not.  There the whole rounds go to the form without and the tiles to a second launch, which
-  // costs some 5 us: no gain with 8 key tiles, [4, 4096, 10, 64], which has 32, 292 us whole and 273
-  // in two.  Causal items differ in length and are dealt by it: there only a call without a whole
-  // round is split.
+  // it does not.  There the whole rounds go to the form without and the tiles to a second launch.  640
+  // pairs of head dim 64, whole and in two, by key tiles: 8 94 and 94 us, 12 129 and 128, 14 145 and 143,
+  // 16 163 and 159, 24 229 and 220, 32 297 and 282; head dims 32 and 128, 600 and 664 pairs alike, 900
+  // (six rounds) 1 to 3 % from 20 tiles on, 1500 (ten) 3 % at 128 and nothing at 64.  Causal items differ
+  // in length and are dealt by it: there only a call without a whole round is split.
   const int pairs = p.q_pairs * H * B, left_over = pairs % attn_sm_count();
   const int rounds = pairs / attn_sm_count();
   const bool fits = left_over > 0 && 2 * left_over <= attn_sm_count();

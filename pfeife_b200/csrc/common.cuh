@@ -355,26 +355,28 @@ __device__ __forceinline__ void tc_commit_pair(uint64_t* bar, uint16_t cta_mask)
       "h"(cta_mask)
       : "memory");
 }
-// D[tmem] (+)= A * B, 16-bit inputs, fp32 accumulate.  One thread issues, chosen by elect_one() for
-// the whole of its role, with operands that are the same for all lanes of its warp: the compiler then
-// keeps them in uniform registers, where the instruction reads them.  Descriptors come as the low word
-// that varies (start address and LBO) and a constant high word (128-byte swizzle, SBO 1024), so that a
-// step to the next slice of an operand is one 32-bit addition.
-// Cycles from one product to the next, M = 128, K = 16 (B200, 1 CTA, eight other warps busy), by the
-// form of the issue: a lane chosen by `lane == 0` in a loop that builds 64-bit descriptors 109-124
-// whatever N; a converged warp in which a predicate picks the lane 61-70; elected, unrolled: 32 at
-// N = 64 with A in TMEM (what the arithmetic takes), 50 at N = 64 with A in shared memory (48 to
-// fetch the operands), 66 at N = 128 (64).
 // Shared-memory matrix descriptor for tcgen05.mma (version 1 = Blackwell), 128-byte swizzle.
 //   K-major operand : rows of 128 B (64 x 16-bit along K); 8 rows = one 1024 B swizzle atom;
 //                     SBO = distance between 8-row groups; LBO unused (1).
 //   MN-major operand: rows of 128 B (64 x 16-bit along M/N), one row per K index; 8 K-rows =
 //                     one atom; SBO = distance between 8-K-row groups, LBO = distance between
 //                     64-element blocks along M/N.
+// The high word is constant (SBO 1024); the low one holds the start address and LBO, so that a step to
+// the next slice of an operand is one 32-bit addition.
 constexpr uint32_t TC_DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29);
 __device__ __forceinline__ uint32_t desc_lo(uint32_t smem_addr, uint32_t lbo_bytes) {
   return ((smem_addr & 0x3FFFF) >> 4) | ((lbo_bytes >> 4) << 16);
 }
+
+// D[tmem] (+)= A * B, 16-bit inputs, fp32 accumulate.  One thread issues, chosen by elect_one() for
+// the whole of its role, with operands that are the same for all lanes of its warp: the compiler then
+// keeps them in uniform registers, where the instruction reads them.  a_lo, b_lo: the descriptors' low
+// words.
+// Cycles from one product to the next, M = 128, K = 16 (B200, 1 CTA, eight other warps busy), by the
+// form of the issue: a lane chosen by `lane == 0` in a loop that builds 64-bit descriptors 109-124
+// whatever N; a converged warp in which a predicate picks the lane 61-70; elected, unrolled: 32 at
+// N = 64 with A in TMEM (what the arithmetic takes), 50 at N = 64 with A in shared memory (48 to
+// fetch the operands), 66 at N = 128 (64).
 __device__ __forceinline__ void tc_mma_f16(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo,
                                            uint32_t idesc, uint32_t accumulate) {
   asm volatile(

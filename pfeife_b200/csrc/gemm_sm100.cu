@@ -18,7 +18,9 @@
 // tile).  Over 6144 x 6144 outputs at K = 64 a GEMM takes 39 us plain, 75 with GELU and its saved
 // pre-activations and 74 with GELU' (77 and 82 with one value at a time and the saved values fetched
 // when they are needed), so that at K = 1408, 84 us plain, the epilogue still shows: ViT-g/14's first
-// layer 104 -> 98 us, its input gradient 104 -> 94 (CUDA events, L2 flushed);
+// layer 104 -> 98 us, its input gradient 104 -> 94 (CUDA events, L2 flushed).  There the epilogue is
+// bound by latency: at K = 64 the issue slots are 34 % busy, the special-function unit 27 %, with two
+// epilogue warps per scheduler;
 // the instantiation that fuses an all-gather of B adds two warps that copy the remote rows.
 #include <cstring>
 #include "common.cuh"
