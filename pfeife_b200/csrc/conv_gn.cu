@@ -218,8 +218,9 @@ static inline int gn_slabs(int B, int HW, int rows, int sm_count, int per_sm) {
 // way: each thread keeps a ring of its next pixels in shared memory, filled by asynchronous copies of
 // its own, which needs no barriers.  Four sizes of CTA: up to 256 threads (2048 channels) and up to 400
 // with a ring, up to 800 and up to 1024 (8192 channels) without.  They compile to 80, 72, 72 and 64
-// registers; the second pass with SiLU spills 44, 64, 96 and 176 bytes per thread, the first 4, 32, 0 and
-// 256, the others next to nothing.  Up to 256 threads three CTAs share an SM, up to 400 two, beyond one,
+// registers; the second pass with SiLU spills 44, 64, 8 and 88 bytes per thread, the first 4, 32, 36 and
+// 124, the others next to nothing.  Without a ring the loads of two pixels go out together only as
+// read-only ones, past the store between them ([4, 32, 32, 6080] 134 us, now 116).  Up to 256 threads three CTAs share an SM, up to 400 two, beyond one,
 // while the slabs are cut for three: wider images take more than one wave.  Backward, both passes and
 // the fold, L2 flushed: [4, 128, 128, 320] 78 -> 64 us, [4, 128, 128, 640] 141 -> 102,
 // [4, 64, 64, 1920] 108 -> 85, [4, 32, 32, 2560] 65 -> 57.
@@ -394,8 +395,8 @@ __device__ __forceinline__ void gn_pixels(const T* x, const T* dy, float* ring, 
   } else {
 #pragma unroll 2
     for (int p = p0; p < p1; p += rows)
-      work(p, *reinterpret_cast<const uint4*>(x + (long long)p * C),
-           *reinterpret_cast<const uint4*>(dy + (long long)p * C));
+      work(p, __ldg(reinterpret_cast<const uint4*>(x + (long long)p * C)),
+           __ldg(reinterpret_cast<const uint4*>(dy + (long long)p * C)));
   }
 }
 
