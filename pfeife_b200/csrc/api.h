@@ -98,8 +98,9 @@ PF_DECL int pf_attn_fwd(const void* q, const void* k, const void* v, void* o, vo
 
 // ---- attn_bwd_sm100.cu
 PF_DECL int pf_attn_bwd_direct(int Sq, int Sk, int causal);
+PF_DECL int pf_attn_bwd_scratch(int B, int H, int Sq, int Sk, int D, int causal);
 PF_DECL int pf_attn_bwd(const void* dout, const void* q, const void* k, const void* v,
-                        const void* out, const void* lse, void* stats, void* dq_accum, void* dq,
+                        const void* out, const void* lse, void* stats, void* scratch, void* dq,
                         void* dk, void* dv, int B, int H, int Sq, int Sk, int D,
                         const long long* sq, const long long* sk, const long long* sv,
                         const long long* sdq, const long long* sdkv, int causal, float scale,

@@ -8,7 +8,9 @@
 //     dK += dS^T Q     A = dS^T in shared memory, K-major, or up to head dim 64 in the columns of dP^T
 //     dQ  = dS K       A = the same dS^T tile, read as an MN-major operand
 // Queries lie along the N side of the first two products and along the reduction of the next two,
-// so a ragged last query tile (ViT: 257 = 2 x 128 + 1) costs what its rows cost, not a full tile.
+// so a ragged last query tile costs what its rows cost, not a full tile; a ragged last key tile costs a
+// full one.  One or two tokens beyond full tiles (ViT: 257 = 2 x 128 + the class token) are taken out of
+// the tiles and handled by attn_bwd_edge_kernel.
 //
 // One CTA per SM walks over (key tile, head, batch) items; roles of its 16 warps:
 //   warps 0-7    softmax side: thread <-> key row (TMEM lane), each warp half of the 128 queries
@@ -36,6 +38,12 @@
 // for dK in tensor memory.  At head dim 128: 261; 222 with S(i+1) issued under the dS^T of tile i and
 // dQ leaving TMEM ahead of its boxes.
 //
+// Where a CTA takes all key tiles of a head (DQ_WHOLE), dQ needs neither clearing, adding in memory nor
+// converting, and dK and dV leave through boxes (rotating inputs, everything included): [24, 257, 16, 88]
+// 136 -> 107 us with its leftover token, [64, 257, 16, 64] 286 -> 163, [16, 256, 16, 64] 52 -> 42.5,
+// [24, 400, 24, 32] 218 -> 167.  At head dim 88 the items of a head are bound by waits: dQ's way out through
+// the columns of dP^T, and K and V, which have one place and arrive after the last product of the item before.
+//
 // A pre-pass writes per query tile the row statistics [128 x -lse2 | 128 x -delta scale] (-inf / 0
 // beyond the last query, which makes the probabilities there zero without a test) and clears the fp32
 // dQ sums; a post-pass converts them.  With one key tile the dQ tiles are complete and go straight to
@@ -46,6 +54,9 @@
 
 namespace pf {
 
+constexpr int BWD_LEFT_MAX = 2;       // leftover tokens of a head handled on CUDA cores (see bwd_plan)
+constexpr int BWD_WHOLE_TILES = 8;    // most query tiles of a head that one CTA takes whole: its sums stay in L2
+
 struct AttnBwdParams {
   int B, H, Sq, Sk, D;
   int causal;
@@ -54,10 +65,21 @@ struct AttnBwdParams {
   const float* stats;   // [B*H][query tiles][256]: -lse * log2(e), then -delta * scale
   void *dq, *dk, *dv;   // strides (batch, seq, head) in elements
   long long sdq[3], sdkv[3];
-  int direct_dq;        // one key tile: dQ tiles are written as they are
   int n_kt, n_qt;
   int* status;
+  float4* part;         // DQ_WHOLE: per CTA the dQ of its head so far, [query tile][DP / 4][128 rows]
+  // leftover rows (attn_bwd_edge_kernel): their number, their weights, and where q, k, dO begin
+  int left;
+  float* edge;          // [B*H][left][3][n_qt * 128]: P and dS of query n + t by key, dS of key n + t by query
+  const void *q, *k, *dout;
+  long long sq[3], sk[3];
 };
+
+// What becomes of a dQ tile.  DQ_SUMS: added to fp32 sums in memory, which a post-pass converts.
+// DQ_DIRECT: one key tile, it is complete.  DQ_WHOLE: a CTA takes all key tiles of a head in turn, so the
+// thread that drains a row of dQ keeps that row's sum, in a buffer of the CTA's own that never leaves L2,
+// and writes 16 bits after the last one: nothing to clear, to add in memory or to convert.
+enum DqMode : int { DQ_SUMS = 0, DQ_DIRECT = 1, DQ_WHOLE = 2 };
 
 // One 8-lane group per (batch, padded query, head): delta = dO . O, statistics, cleared dQ sums.
 template <typename T>
@@ -100,6 +122,199 @@ attn_bwd_prep_kernel(const T* __restrict__ dout, const T* __restrict__ out,
     float* st = stats + (((b * H + h) * n_qt + i / ATT_BM) * 2) * ATT_BM + i % ATT_BM;
     st[0] = live ? -lse[(b * H + h) * S + i] * LOG2E : -INFINITY;
     st[ATT_BM] = live ? -s * scale : 0.f;
+  }
+}
+
+// What the leftover rows of a head of n + left tokens (n a multiple of 128) take part in, on CUDA cores:
+// one CTA per head walks over its tokens x once per leftover token r with
+//     weights of query r by key x      P_r[x] = exp2(q_r k_x c - lse2_r),  dS_r[x] = P (dO_r v_x - delta_r) scale
+//     weights of key r by query x      P[x], dS[x] likewise from q_x k_r, dO_x v_r
+//     dQ_r = sum dS_r[x] k_x,  dV_r = sum P[x] dO_x,  dK_r = sum dS[x] q_x          (complete, written here)
+// and leaves the weights that touch the other tokens to the kernel below (AttnBwdParams::edge), with the
+// row statistics of the pre-pass, whose reads of O and dO it shares.
+// Four lanes share a token: with 8 or 16 the sums over lanes and the reads of token r's values from shared
+// memory bound it ([24, 257, 16, 88] 35 us, now 30).  A thread asks for its next token's five rows while it
+// works on this one's, in slots of its own, so that the loop has no barrier.
+template <int DP>
+struct EdgeCfg {
+  static constexpr int NV = DP / 32;                     // vectors of 8 columns per lane
+  static constexpr int THREADS = 128, GROUPS = THREADS / 4;
+  static constexpr int CTAS = NV > 3 ? 2 : 3;            // per SM
+  static constexpr int RING = 2 * 5 * NV * THREADS * 16;
+  static constexpr int OFF_VECS = RING, OFF_LSE = OFF_VECS + 4 * DP * 4;
+  static constexpr int SMEM = OFF_LSE + (BWD_WHOLE_TILES * ATT_BM + BWD_LEFT_MAX) * 4;
+  static_assert(4 * 3 * DP * 4 <= RING, "the warps' sums lie over the ring");
+};
+
+template <typename T, int DP>
+__global__ void __launch_bounds__(EdgeCfg<DP>::THREADS, EdgeCfg<DP>::CTAS)
+attn_bwd_edge_kernel(const AttnBwdParams p, const T* __restrict__ v, const T* __restrict__ out,
+                     const float* __restrict__ lse, float* __restrict__ stats, const long long sv0,
+                     const long long sv1, const long long sv2) {
+  using C = EdgeCfg<DP>;
+  constexpr int NV = C::NV, THREADS = C::THREADS, GROUPS = C::GROUPS;
+  extern __shared__ __align__(16) uint8_t edge_smem[];
+  uint4* ring = reinterpret_cast<uint4*>(edge_smem) + threadIdx.x;              // [2][5][NV][THREADS]
+  float* vecs = reinterpret_cast<float*>(edge_smem + C::OFF_VECS);              // q, k, v, dO of token r
+  float* nlse = reinterpret_cast<float*>(edge_smem + C::OFF_LSE);
+  float (*red)[3][DP] = reinterpret_cast<float (*)[3][DP]>(edge_smem);          // after the loop
+  const int h = blockIdx.x, b = blockIdx.y, n = p.Sq, S = n + p.left;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane & 3, grp = threadIdx.x >> 2;
+  const long long bh = (long long)b * p.H + h;
+  const float c2 = p.scale * LOG2E;
+  // rows of q, k, v, dO, O; this lane's columns are vectors sub, sub + 4, ...
+  const T* base[5] = {reinterpret_cast<const T*>(p.q) + b * p.sq[0] + h * p.sq[2],
+                      reinterpret_cast<const T*>(p.k) + b * p.sk[0] + h * p.sk[2],
+                      v + b * sv0 + h * sv2,
+                      reinterpret_cast<const T*>(p.dout) + (b * (long long)S * p.H + h) * p.D,
+                      out + (b * (long long)S * p.H + h) * p.D};
+  const long long so = (long long)p.H * p.D;
+  const long long stride[5] = {p.sq[1], p.sk[1], sv1, so, so};
+  auto in = [&](int i) { return (sub + 4 * i) * 8 < p.D; };
+  for (int x = threadIdx.x; x < S; x += THREADS) nlse[x] = -lse[bh * S + x] * LOG2E;
+  const int trips = (S + GROUPS - 1) / GROUPS;           // the same for every lane
+  auto fetch = [&](int trip) {
+    const int x = min(trip * GROUPS + grp, S - 1);
+    uint4* slot = ring + (trip & 1) * 5 * NV * THREADS;
+    if (trip < trips) {
+#pragma unroll
+      for (int a = 0; a < 5; ++a)
+#pragma unroll
+        for (int i = 0; i < NV; ++i)
+          if (in(i)) cp_async16(slot + (a * NV + i) * THREADS, base[a] + x * stride[a] + (sub + 4 * i) * 8);
+    }
+    cp_async_commit();
+  };
+  auto widen = [](const uint4& u, float* f) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) f[j] = to_f32<T>(reinterpret_cast<const T*>(&u)[j]);
+  };
+  auto dot = [](const float (&a)[8 * NV], const float (&c)[8 * NV]) {
+    float s[NV] = {};
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+      for (int i = 0; i < NV; ++i) s[i] = fmaf(a[i * 8 + j], c[i * 8 + j], s[i]);
+    float r = s[0];
+#pragma unroll
+    for (int i = 1; i < NV; ++i) r += s[i];
+    return r;
+  };
+  auto over_lanes = [](float s) {      // whole warps take part, whichever of their tokens exist
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    return s + __shfl_xor_sync(0xffffffffu, s, 1);
+  };
+  for (int t = 0; t < p.left; ++t) {
+    const int r = n + t;
+#pragma unroll
+    for (int i = 0; i < 2 * 5 * NV; ++i)                 // columns beyond D count as zeros
+      if (!in(i % NV)) ring[i * THREADS] = make_uint4(0, 0, 0, 0);
+    fetch(0);
+    if (threadIdx.x < DP)
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+        vecs[a * DP + threadIdx.x] =
+            (int)threadIdx.x < p.D ? to_f32<T>(base[a][r * stride[a] + threadIdx.x]) : 0.f;
+    float f[8 * NV], g[8 * NV], w[8 * NV], dq[8 * NV] = {}, dk[8 * NV] = {}, dv[8 * NV] = {};
+    auto own = [&](const T* row, float (&to)[8 * NV]) {
+#pragma unroll
+      for (int i = 0; i < NV; ++i)
+        widen(in(i) ? __ldg(reinterpret_cast<const uint4*>(row) + sub + 4 * i) : make_uint4(0, 0, 0, 0),
+              to + i * 8);
+    };
+    own(base[3] + r * so, g);
+    own(base[4] + r * so, f);
+    const float delta_r = over_lanes(dot(g, f));
+    __syncthreads();
+    const float nlse_r = nlse[r];
+    auto vec = [&](int a, float (&to)[8 * NV]) {
+#pragma unroll
+      for (int i = 0; i < NV; ++i)
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const float4 q = *reinterpret_cast<const float4*>(vecs + a * DP + (sub + 4 * i) * 8 + u * 4);
+          float* o = to + i * 8 + u * 4;
+          o[0] = q.x; o[1] = q.y; o[2] = q.z; o[3] = q.w;
+        }
+    };
+    float* e = p.edge + (bh * p.left + t) * 3 * n;
+    for (int trip = 0; trip < trips; ++trip) {
+      fetch(trip + 1);
+      cp_async_wait<1>();
+      const int x = trip * GROUPS + grp;
+      const bool live = x < S;
+      const uint4* slot = ring + (trip & 1) * 5 * NV * THREADS;
+      auto row = [&](int a, float (&to)[8 * NV]) {
+#pragma unroll
+        for (int i = 0; i < NV; ++i) widen(slot[(a * NV + i) * THREADS], to + i * 8);
+      };
+      const float nlse_x = nlse[min(x, S - 1)];
+      row(3, g);
+      row(4, f);
+      const float delta_x = over_lanes(dot(g, f));
+      vec(2, w);
+      const float dp_x = over_lanes(dot(g, w));           // dO_x v_r
+      row(2, f);
+      vec(3, w);
+      const float dp_r = over_lanes(dot(f, w));           // dO_r v_x
+      row(1, f);
+      vec(0, w);
+      const float s_r = over_lanes(dot(f, w));
+      const float p_r = live ? exp2f(fmaf(s_r, c2, nlse_r)) : 0.f;
+      const float ds_r = p_r * (dp_r - delta_r) * p.scale;
+#pragma unroll
+      for (int j = 0; j < 8 * NV; ++j) dq[j] = fmaf(ds_r, f[j], dq[j]);
+      row(0, f);
+      vec(1, w);
+      const float s_x = over_lanes(dot(f, w));
+      const float p_x = live ? exp2f(fmaf(s_x, c2, nlse_x)) : 0.f;
+      const float ds_x = p_x * (dp_x - delta_x) * p.scale;
+#pragma unroll
+      for (int j = 0; j < 8 * NV; ++j) {
+        dk[j] = fmaf(ds_x, f[j], dk[j]);
+        dv[j] = fmaf(p_x, g[j], dv[j]);
+      }
+      if (sub == 0 && x < n) {
+        e[x] = p_r;
+        e[n + x] = ds_r;
+        e[2 * n + x] = ds_x;
+        if (t == 0) {
+          float* st = stats + ((bh * p.n_qt + x / ATT_BM) * 2) * ATT_BM + x % ATT_BM;
+          st[0] = nlse_x;
+          st[ATT_BM] = -delta_x * p.scale;
+        }
+      }
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    // over the eight groups of a warp, then over the warps
+#pragma unroll
+    for (int j = 0; j < 8 * NV; ++j) {
+#pragma unroll
+      for (int m = 4; m < 32; m <<= 1) {
+        dq[j] += __shfl_xor_sync(0xffffffffu, dq[j], m);
+        dk[j] += __shfl_xor_sync(0xffffffffu, dk[j], m);
+        dv[j] += __shfl_xor_sync(0xffffffffu, dv[j], m);
+      }
+      if (lane < 4) {
+        const int d = (sub + 4 * (j / 8)) * 8 + j % 8;
+        red[warp][0][d] = dq[j];
+        red[warp][1][d] = dk[j];
+        red[warp][2][d] = dv[j];
+      }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < 3 * DP; i += THREADS) {
+      const int a = i / DP, d = i - a * DP;
+      if (d < p.D) {
+        const float s = (red[0][a][d] + red[1][a][d]) + (red[2][a][d] + red[3][a][d]);
+        T* dst = a == 0 ? reinterpret_cast<T*>(p.dq) + b * p.sdq[0] + r * p.sdq[1] + h * p.sdq[2]
+                        : reinterpret_cast<T*>(a == 1 ? p.dk : p.dv) + b * p.sdkv[0] +
+                              r * p.sdkv[1] + h * p.sdkv[2];
+        dst[d] = from_f32<T>(s);
+      }
+    }
+    __syncthreads();
   }
 }
 
@@ -161,7 +376,7 @@ struct BwdCfg {
 };
 
 struct BwdItem {
-  int k0, h, b, q_begin, n;    // first key, first visible query tile, number of query tiles
+  int kt, k0, h, b, q_begin, n;    // key tile, its first key, first visible query tile, query tiles
 };
 // Items of round `r`.  Causal key tiles see fewer queries the later they start: the long ones are
 // dealt first (all heads of a key tile next to each other) and every other round runs backwards,
@@ -171,17 +386,57 @@ __device__ __forceinline__ int bwd_index(int r) {
   const int slot = (r & 1) ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;
   return r * (int)gridDim.x + slot;
 }
-__device__ __forceinline__ BwdItem bwd_item(const AttnBwdParams& p, int w) {
-  BwdItem it;
+// In DQ_WHOLE the items are heads and their key tiles rounds of their own.
+template <int MODE>
+__device__ __forceinline__ int bwd_rounds(const AttnBwdParams& p, int n_items) {
+  const int rounds = (n_items + (int)gridDim.x - 1) / (int)gridDim.x;
+  return MODE == DQ_WHOLE ? rounds * p.n_kt : rounds;
+}
+// the item of round `r`; false when this CTA has none
+template <int MODE>
+__device__ __forceinline__ bool bwd_item(const AttnBwdParams& p, int r, int n_items, BwdItem& it) {
   int kt, bh;
-  if (p.causal) { kt = w / (p.B * p.H); bh = w - kt * (p.B * p.H); }
-  else { bh = w / p.n_kt; kt = w - bh * p.n_kt; }
+  if (MODE == DQ_WHOLE) {
+    const int head = r / p.n_kt;
+    kt = r - head * p.n_kt;
+    bh = bwd_index(head);
+    if (bh >= n_items) return false;
+  } else {
+    const int w = bwd_index(r);
+    if (w >= n_items) return false;
+    if (p.causal) { kt = w / (p.B * p.H); bh = w - kt * (p.B * p.H); }
+    else { bh = w / p.n_kt; kt = w - bh * p.n_kt; }
+  }
+  it.kt = kt;
   it.k0 = kt * ATT_BN;
   it.h = bh % p.H;
   it.b = bh / p.H;
   it.q_begin = p.causal ? max(0, it.k0 - (p.Sk - p.Sq)) / ATT_BM : 0;
   it.n = max(0, p.n_qt - it.q_begin);
-  return it;
+  return true;
+}
+
+// 32 values of row `r` of a 16-bit box of 32 x 32 in the 64-byte swizzle
+template <typename T>
+__device__ __forceinline__ void box_row16(uint8_t* box, int r, const uint32_t (&v)[32]) {
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+    *reinterpret_cast<uint4*>(box + r * 64 + ((c ^ ((r >> 1) & 3)) << 4)) = pack8<T>(v + c * 8);
+}
+
+// acc[0..31] += w * (columns c0 .. c0 + 31 of a 16-bit row of D values); every lane reads the same row
+template <typename T>
+__device__ __forceinline__ void axpy_row32(uint32_t (&acc)[32], float w, const T* row, int c0, int D) {
+#pragma unroll
+  for (int v = 0; v < 4; ++v) {
+    if (c0 + v * 8 < D) {
+      const uint4 u = __ldg(reinterpret_cast<const uint4*>(row + c0) + v);
+      const T* e = reinterpret_cast<const T*>(&u);
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        acc[v * 8 + j] = __float_as_uint(fmaf(w, to_f32<T>(e[j]), __uint_as_float(acc[v * 8 + j])));
+    }
+  }
 }
 
 // Probabilities of 32 queries for this thread's key: kept in fp32, packed to 16 bits in the columns
@@ -241,11 +496,12 @@ __device__ __forceinline__ void bwd_ds(const uint32_t (&s)[32], const float* pr,
 // DS_TMEM: dK reads dS^T from tensor memory: 256 of the 3100 cycles' worth of shared-memory accesses of a
 // tile pair less ([4, 4096, 10, 64] 579 -> 549 us).  dP(i+1) then waits for dK(i), which costs more
 // than that where one key tile holds every key ([4, 1024, 20, 64] with 77 keys: 35 -> 37 us).
-template <typename T, int DP, bool DS_TMEM>
+template <typename T, int DP, int MODE, bool DS_TMEM>
 __global__ void __launch_bounds__(BwdCfg<DP, DS_TMEM>::THREADS, 1)
 attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                    const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo,
-                   const __grid_constant__ CUtensorMap tdq, const AttnBwdParams p,
+                   const __grid_constant__ CUtensorMap tdq, const __grid_constant__ CUtensorMap tdk,
+                   const __grid_constant__ CUtensorMap tdv, const AttnBwdParams p,
                    const int n_items) {
   using C = BwdCfg<DP, DS_TMEM>;
   constexpr int NBLK = C::NBLK, TILE = C::TILE;
@@ -279,7 +535,7 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
   }
   if (tid == 0) {
     tma_prefetch_desc(&tq); tma_prefetch_desc(&tk); tma_prefetch_desc(&tv);
-    tma_prefetch_desc(&tdo); tma_prefetch_desc(&tdq);
+    tma_prefetch_desc(&tdo); tma_prefetch_desc(&tdq); tma_prefetch_desc(&tdk); tma_prefetch_desc(&tdv);
     for (int i = 0; i < 23; ++i) mbar_init(&bars[i], 1);
     for (int i = 0; i < 2; ++i) mbar_init(&q_empty[i], 1 + 8);
     mbar_init(s_empty, 8);
@@ -294,7 +550,7 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_base_of(tmem_slot);
-  const int shift = p.Sk - p.Sq;
+  const int shift = p.Sk - p.Sq, rounds = bwd_rounds<MODE>(p, n_items);
   // one split per warpgroup: its four warps execute the same instruction
   if (warp >= 12) {
     regs_dec<C::REGS_OTHER>();
@@ -303,11 +559,9 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
       if (elect_one()) {
         uint32_t g = 0, items = 0;
         bool ok = true;
-        for (int r = 0; ok && r * (int)gridDim.x < n_items; ++r) {
-          const int w = bwd_index(r);
-          if (w >= n_items) continue;
-          const BwdItem it = bwd_item(p, w);
-          if (it.n == 0) continue;
+        for (int r = 0; ok && r < rounds; ++r) {
+          BwdItem it;
+          if (!bwd_item<MODE>(p, r, n_items, it) || it.n == 0) continue;
           for (int i = 0; i < it.n && ok; ++i, ++g) {
             const int q0 = (it.q_begin + i) * ATT_BM, st = g & 1, ds = g % C::DOST;
             ok = mbar_wait(&q_empty[st], ((g >> 1) & 1) ^ 1, p.status, PF_ERR_TIMEOUT_EMPTY);
@@ -384,11 +638,9 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
           tc_commit(dp_full);
           return true;
         };
-        for (int r = 0; ok && r * (int)gridDim.x < n_items; ++r) {
-          const int w = bwd_index(r);
-          if (w >= n_items) continue;
-          const BwdItem it = bwd_item(p, w);
-          if (it.n == 0) continue;
+        for (int r = 0; ok && r < rounds; ++r) {
+          BwdItem it;
+          if (!bwd_item<MODE>(p, r, n_items, it) || it.n == 0) continue;
           const int k_steps = (min(ATT_BN, p.Sk - it.k0) + 15) / 16;
           ok = mbar_wait(kv_full, items & 1, p.status, PF_ERR_TIMEOUT_FULL) &&
                issue_s(g, it.q_begin) && issue_dp(g, it.q_begin);
@@ -451,12 +703,19 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
     const int quad = warp & 3;
     const uint32_t lane_off = uint32_t(quad * 32) << 16;
     uint8_t* boxes = smem + C::OFF_STG + quad * 8192;
+    const int n_pad = p.n_qt * ATT_BM;
+    float4* part = p.part + (long long)blockIdx.x * n_pad * (DP / 4);
     uint32_t g = 0, items = 0, box = 0;
     bool ok = true;
-    for (int r = 0; ok && r * (int)gridDim.x < n_items; ++r) {
-      const int w = bwd_index(r);
-      if (w >= n_items) continue;
-      const BwdItem it = bwd_item(p, w);
+    // two boxes per warp: the store that last used this one must have read it
+    auto next_box = [&]() -> uint8_t* {
+      if (lane == 0 && box >= 2) tma_store_wait_read_but_one();
+      __syncwarp();
+      return boxes + (box++ & 1) * 4096;
+    };
+    for (int r = 0; ok && r < rounds; ++r) {
+      BwdItem it;
+      if (!bwd_item<MODE>(p, r, n_items, it)) continue;
       const int kj = it.k0 + quad * 32 + lane;
       const long long off_kv = (long long)it.b * p.sdkv[0] + (long long)kj * p.sdkv[1] +
                                (long long)it.h * p.sdkv[2];
@@ -470,8 +729,12 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
           }
         continue;
       }
+      const float* edge = p.edge + (long long)(it.b * p.H + it.h) * p.left * 3 * n_pad;
       for (int i = 0; i < it.n && ok; ++i, ++g) {
         const int q0 = (it.q_begin + i) * ATT_BM + quad * 32;   // first query row of this warp
+        // DQ_WHOLE: the last key tile that this query tile sees
+        const int last_kt =
+            p.causal ? min(p.n_kt - 1, ((it.q_begin + i + 1) * ATT_BM - 1 + shift) / ATT_BN) : p.n_kt - 1;
         ok = mbar_wait(dq_full, g & 1, p.status, PF_ERR_TIMEOUT_TMEM_FULL);
         if (!ok) break;
         tc_fence_after();
@@ -493,33 +756,51 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
           for (int u = 0; u < 2; ++u) {
             const int c = c0 + u;
             if (c >= DP / 32) continue;
-            if (p.direct_dq) {
+            if (MODE == DQ_WHOLE) {
               const int qi = q0 + lane;
-              if (qi < p.Sq) {
-                T* dst = reinterpret_cast<T*>(p.dq) + (long long)it.b * p.sdq[0] +
-                         (long long)qi * p.sdq[1] + (long long)it.h * p.sdq[2] + c * 32;
+              float4* sum = part + ((it.q_begin + i) * (DP / 4) + c * 8) * ATT_BM + quad * 32 + lane;
+              if (it.kt > 0) {
 #pragma unroll
-                for (int v = 0; v < 4; ++v)
-                  if (c * 32 + v * 8 < p.D)
-                    reinterpret_cast<uint4*>(dst)[v] = pack8<T>(raw[u] + v * 8);
+                for (int v = 0; v < 8; ++v) {
+                  const float4 s = sum[v * ATT_BM];
+                  raw[u][v * 4] = __float_as_uint(__uint_as_float(raw[u][v * 4]) + s.x);
+                  raw[u][v * 4 + 1] = __float_as_uint(__uint_as_float(raw[u][v * 4 + 1]) + s.y);
+                  raw[u][v * 4 + 2] = __float_as_uint(__uint_as_float(raw[u][v * 4 + 2]) + s.z);
+                  raw[u][v * 4 + 3] = __float_as_uint(__uint_as_float(raw[u][v * 4 + 3]) + s.w);
+                }
               }
-            } else {
-              // two boxes per warp: the reduce-add that last used this one must have read it
-              uint8_t* bx = boxes + (box & 1) * 4096;
-              if (lane == 0 && box >= 2) tma_store_wait_read_but_one();
-              __syncwarp();
+              if (it.kt < last_kt) {
+#pragma unroll
+                for (int v = 0; v < 8; ++v)
+                  sum[v * ATT_BM] = make_float4(
+                      __uint_as_float(raw[u][v * 4]), __uint_as_float(raw[u][v * 4 + 1]),
+                      __uint_as_float(raw[u][v * 4 + 2]), __uint_as_float(raw[u][v * 4 + 3]));
+                continue;
+              }
+              for (int t = 0; t < p.left; ++t)         // the leftover keys' part
+                axpy_row32<T>(raw[u], edge[(t * 3 + 2) * n_pad + qi],
+                              reinterpret_cast<const T*>(p.k) + (long long)it.b * p.sk[0] +
+                                  (long long)(p.Sk + t) * p.sk[1] + (long long)it.h * p.sk[2],
+                              c * 32, p.D);
+            }
+            uint8_t* bx = next_box();
+            if (MODE == DQ_SUMS) {
 #pragma unroll
               for (int v = 0; v < 8; ++v)
                 *reinterpret_cast<uint4*>(bx + lane * 128 + ((v ^ (lane & 7)) << 4)) = make_uint4(
                     raw[u][v * 4], raw[u][v * 4 + 1], raw[u][v * 4 + 2], raw[u][v * 4 + 3]);
-              fence_async_smem();
-              __syncwarp();
-              if (lane == 0) {
-                // rows beyond the last query / columns beyond D are clipped by the TMA itself
-                if (q0 < p.Sq) tma_reduce_add_4d(&tdq, bx, c * 32, it.h, q0, it.b);
-                tma_store_commit();
+            } else {
+              box_row16<T>(bx, lane, raw[u]);
+            }
+            fence_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              // rows beyond the last query / columns beyond D are clipped by the TMA itself
+              if (q0 < p.Sq) {
+                if (MODE == DQ_SUMS) tma_reduce_add_4d(&tdq, bx, c * 32, it.h, q0, it.b);
+                else tma_store_4d(&tdq, bx, c * 32, it.h, q0, it.b);
               }
-              ++box;
+              tma_store_commit();
             }
           }
         }
@@ -540,13 +821,42 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
           __syncwarp();
           if (lane == 0) mbar_arrive(acc_empty);
         }
-        if (kj < p.Sk) {
+        if (MODE == DQ_SUMS) {
+          if (kj < p.Sk) {
 #pragma unroll
-          for (int v = 0; v < 4; ++v)
-            if (c * 32 + v * 8 < p.D) {
-              reinterpret_cast<uint4*>(dkp)[c * 4 + v] = pack8<T>(rk + v * 8);
-              reinterpret_cast<uint4*>(dvp)[c * 4 + v] = pack8<T>(rv + v * 8);
-            }
+            for (int v = 0; v < 4; ++v)
+              if (c * 32 + v * 8 < p.D) {
+                reinterpret_cast<uint4*>(dkp)[c * 4 + v] = pack8<T>(rk + v * 8);
+                reinterpret_cast<uint4*>(dvp)[c * 4 + v] = pack8<T>(rv + v * 8);
+              }
+          }
+          continue;
+        }
+        // A row's 16 bytes per thread take some 6800 cycles to leave at head dim 88, more than the products
+        // of a short item: they go through boxes.  Among the boxes of DQ_SUMS they would only wait
+        // ([12, 513, 25, 64] 181 -> 200 us).
+        for (int t = 0; t < p.left; ++t) {       // the leftover queries' part
+          const long long r = p.Sq + t;
+          axpy_row32<T>(rk, edge[(t * 3 + 1) * n_pad + kj],
+                        reinterpret_cast<const T*>(p.q) + (long long)it.b * p.sq[0] + r * p.sq[1] +
+                            (long long)it.h * p.sq[2],
+                        c * 32, p.D);
+          axpy_row32<T>(rv, edge[t * 3 * n_pad + kj],
+                        reinterpret_cast<const T*>(p.dout) +
+                            (((long long)it.b * (p.Sq + p.left) + r) * p.H + it.h) * p.D,
+                        c * 32, p.D);
+        }
+        uint8_t* bx = next_box();                // half a box each
+        box_row16<T>(bx, lane, rk);
+        box_row16<T>(bx + 2048, lane, rv);
+        fence_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          if (it.k0 + quad * 32 < p.Sk) {
+            tma_store_4d(&tdk, bx, c * 32, it.h, it.k0 + quad * 32, it.b);
+            tma_store_4d(&tdv, bx + 2048, c * 32, it.h, it.k0 + quad * 32, it.b);
+          }
+          tma_store_commit();
         }
       }
       ++items;
@@ -562,10 +872,9 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
     const uint64_t c2v = f2_pack(c2, c2), scv = f2_pack(p.scale, p.scale);
     uint32_t g = 0;
     bool ok = true;
-    for (int r = 0; ok && r * (int)gridDim.x < n_items; ++r) {
-      const int w = bwd_index(r);
-      if (w >= n_items) continue;
-      const BwdItem it = bwd_item(p, w);
+    for (int r = 0; ok && r < rounds; ++r) {
+      BwdItem it;
+      if (!bwd_item<MODE>(p, r, n_items, it)) continue;
       const bool ragged = it.k0 + ATT_BN > p.Sk;
       const int kj = it.k0 + row;
       // a warp all of whose keys lie beyond the last one (rounded to the reduction steps of dQ)
@@ -693,26 +1002,59 @@ static int make_tmap_dq(CUtensorMap* map, const void* base, int B, int S, int H,
   return r == CUDA_SUCCESS ? 0 : -(1000 + (int)r);
 }
 
+// 16-bit [B, S, H, D] view with element strides; box = 32 x 1 x 32 x 1 in the 64-byte swizzle
+static int make_tmap_grad(CUtensorMap* map, const void* base, int fmt, int B, int S, int H, int D,
+                          const long long* st) {
+  EncodeTiledFn enc = attn_get_encode();
+  if (!enc) return -100;
+  cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)H, (cuuint64_t)S, (cuuint64_t)B};
+  cuuint64_t strides[3] = {(cuuint64_t)st[2] * 2, (cuuint64_t)st[1] * 2, (cuuint64_t)st[0] * 2};
+  cuuint32_t box[4] = {32, 1, 32, 1};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUresult r = enc(map, fmt ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
+                   4, const_cast<void*>(base), dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
+                   CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : -(1000 + (int)r);
+}
+
 template <typename T, int DP>
 static int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
-                      const CUtensorMap& tdo, const CUtensorMap& tdq, const AttnBwdParams& p,
-                      cudaStream_t st) {
-  const int n_items = p.n_kt * p.H * p.B, sms = attn_sm_count();
+                      const CUtensorMap& tdo, const CUtensorMap& tdq, const CUtensorMap& tdk,
+                      const CUtensorMap& tdv, const AttnBwdParams& p, int mode, cudaStream_t st) {
+  const int n_items = (mode == DQ_WHOLE ? 1 : p.n_kt) * p.H * p.B, sms = attn_sm_count();
   const int grid = n_items < sms ? n_items : sms;
-  auto run = [&](auto ds_tmem) -> int {
+  auto run = [&](auto m, auto ds_tmem) -> int {
     using C = BwdCfg<DP, decltype(ds_tmem)::value>;
-    auto kern = attn_bwd_ws_kernel<T, DP, decltype(ds_tmem)::value>;
+    auto kern = attn_bwd_ws_kernel<T, DP, decltype(m)::value, decltype(ds_tmem)::value>;
     static bool done[64] = {};       // one per instantiation of this lambda
     const int r = set_smem(kern, C::SMEM, done);
     if (r) return r;
-    kern<<<grid, C::THREADS, C::SMEM, st>>>(tq, tk, tv, tdo, tdq, p, n_items);
+    kern<<<grid, C::THREADS, C::SMEM, st>>>(tq, tk, tv, tdo, tdq, tdk, tdv, p, n_items);
     PF_CHECK_LAUNCH();
     return 0;
   };
-  if constexpr (DP <= 64) {
-    if (!p.direct_dq) return run(std::true_type());
-  }
-  return run(std::false_type());
+  std::integral_constant<int, DQ_SUMS> sums;
+  std::integral_constant<int, DQ_DIRECT> direct;
+  std::integral_constant<int, DQ_WHOLE> whole;
+  constexpr std::bool_constant<(DP <= 64)> in_tmem{};
+  constexpr std::false_type in_smem{};
+  if (mode == DQ_SUMS) return run(sums, in_tmem);
+  if (mode == DQ_DIRECT) return run(direct, in_smem);
+  return p.n_kt > 1 ? run(whole, in_tmem) : run(whole, in_smem);
+}
+
+template <typename T, int DP>
+static int launch_edge(const AttnBwdParams& p, const void* v, const void* out, const void* lse, void* stats,
+                       const long long* sv, cudaStream_t st) {
+  using C = EdgeCfg<DP>;
+  static bool done[64] = {};
+  const int r = set_smem(attn_bwd_edge_kernel<T, DP>, C::SMEM, done);
+  if (r) return r;
+  attn_bwd_edge_kernel<T, DP><<<dim3(p.H, p.B), C::THREADS, C::SMEM, st>>>(
+      p, (const T*)v, (const T*)out, (const float*)lse, (float*)stats, sv[0], sv[1], sv[2]);
+  PF_CHECK_LAUNCH();
+  return 0;
 }
 
 // one key tile that every query tile visits: its dQ tiles need no summation
@@ -720,41 +1062,79 @@ static bool bwd_direct(int Sq, int Sk, int causal) {
   return Sk <= ATT_BN && (!causal || Sk >= Sq);
 }
 
+struct BwdPlan {
+  int mode, left, n_kt, n_qt;
+  long long part, edge;               // floats of scratch: dQ so far (or the fp32 sums), leftover weights
+};
+// Heads are taken whole where that takes no more rounds of key tiles than dealing the key tiles one by one.
+// The leftover token then saves a key tile and a query tile per head; each costs a pass over the head (some
+// 15 us per 200 heads of 257 tokens up to head dim 64, twice that above).  [12, 258, 25, 64] 87 us in tiles
+// and 83 so, [12, 260, 25, 64] 86 and 121; [24, 257, 16, 88] 123 and 107, [24, 258, 16, 88] 125 and 147.
+static BwdPlan bwd_plan(int B, int H, int Sq, int Sk, int D, int causal) {
+  const long long heads = (long long)B * H, sms = attn_sm_count();
+  auto tiles = [](int n) { return (n + ATT_BN - 1) / ATT_BN; };
+  BwdPlan g = {bwd_direct(Sq, Sk, causal) ? DQ_DIRECT : DQ_SUMS, 0, tiles(Sk), tiles(Sq), 0, 0};
+  const int left = Sq % ATT_BM, left_max = D > 64 ? 1 : BWD_LEFT_MAX;
+  const bool edge = !causal && Sq == Sk && Sq > ATT_BM && left > 0 && left <= left_max;
+  const int n_kt = edge ? g.n_kt - 1 : g.n_kt, n_qt = edge ? g.n_qt - 1 : g.n_qt;
+  const long long whole = (heads + sms - 1) / sms * n_kt, apart = (heads * g.n_kt + sms - 1) / sms;
+  if (g.mode == DQ_SUMS && n_qt <= BWD_WHOLE_TILES && (!causal || Sk >= Sq) && whole <= apart) {
+    g.mode = DQ_WHOLE;
+    g.left = edge ? left : 0;
+    g.n_kt = n_kt;
+    g.n_qt = n_qt;
+    const int dp = (D + 31) / 32 * 32;
+    g.part = (heads < sms ? heads : sms) * n_qt * ATT_BM * dp;
+    g.edge = heads * g.left * 3 * n_qt * ATT_BM;
+  } else if (g.mode == DQ_SUMS) {
+    g.part = heads * Sq * D;
+  }
+  return g;
+}
+
 }  // namespace pf
 
 using namespace pf;
 
-// dout / out: [B, Sq, H, D] contiguous.  stats: fp32 scratch [B, H, ceil(Sq / 128), 256], 16-byte
-// aligned.  dq_accum: fp32 scratch [B, Sq, H, D], not needed (may be null) when
-// pf_attn_bwd_direct(Sq, Sk, causal).
 PF_API int pf_attn_bwd_direct(int Sq, int Sk, int causal) { return bwd_direct(Sq, Sk, causal); }
 
+// KiB of scratch that pf_attn_bwd needs on the current device (0: none)
+PF_API int pf_attn_bwd_scratch(int B, int H, int Sq, int Sk, int D, int causal) {
+  const BwdPlan g = bwd_plan(B, H, Sq, Sk, D, causal);
+  return (int)((g.part + g.edge + 255) / 256);
+}
+
+// dout / out: [B, Sq, H, D] contiguous.  stats: fp32 scratch [B, H, ceil(Sq / 128), 256]; scratch: of
+// pf_attn_bwd_scratch KiB; both 16-byte aligned.
 PF_API int pf_attn_bwd(const void* dout, const void* q, const void* k, const void* v,
-                       const void* out, const void* lse, void* stats, void* dq_accum, void* dq,
+                       const void* out, const void* lse, void* stats, void* scratch, void* dq,
                        void* dk, void* dv, int B, int H, int Sq, int Sk, int D,
                        const long long* sq, const long long* sk, const long long* sv,
                        const long long* sdq, const long long* sdkv, int causal,
                        float scale, int dtype, int* status, int sm_count, void* stream) {
   if (dtype != PF_F16 && dtype != PF_BF16) return -1;
   if (D % 8 || D > 128) return -3;
-  const bool direct = bwd_direct(Sq, Sk, causal);
+  const BwdPlan plan = bwd_plan(B, H, Sq, Sk, D, causal);
   if (!strides_ok(q, sq[0], sq[1], sq[2]) || !strides_ok(k, sk[0], sk[1], sk[2]) ||
       !strides_ok(v, sv[0], sv[1], sv[2]) || (reinterpret_cast<uintptr_t>(dout) & 15) ||
       (reinterpret_cast<uintptr_t>(out) & 15) || (reinterpret_cast<uintptr_t>(stats) & 15) ||
-      (!direct && (!dq_accum || (reinterpret_cast<uintptr_t>(dq_accum) & 15))) ||
+      (plan.part && (!scratch || (reinterpret_cast<uintptr_t>(scratch) & 15))) ||
       !strides_ok(dq, sdq[0], sdq[1], sdq[2]) || !strides_ok(dk, sdkv[0], sdkv[1], sdkv[2]) ||
       !strides_ok(dv, sdkv[0], sdkv[1], sdkv[2]))
     return -2;
   const int fmt = dtype == PF_BF16;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   AttnBwdParams p = {};
-  p.B = B; p.H = H; p.Sq = Sq; p.Sk = Sk; p.D = D; p.causal = causal; p.scale = scale;
-  p.fmt = fmt; p.stats = (const float*)stats; p.dq = dq; p.dk = dk; p.dv = dv; p.status = status;
-  p.direct_dq = direct;
-  p.n_kt = (Sk + ATT_BN - 1) / ATT_BN;
-  p.n_qt = (Sq + ATT_BM - 1) / ATT_BM;
-  for (int i = 0; i < 3; ++i) { p.sdq[i] = sdq[i]; p.sdkv[i] = sdkv[i]; }
-  CUtensorMap tq, tk, tv, tdo, tdq;
+  // with leftover rows the tensor-core kernel sees the tokens before them
+  p.B = B; p.H = H; p.Sq = Sq - plan.left; p.Sk = Sk - plan.left; p.D = D; p.causal = causal;
+  p.scale = scale; p.fmt = fmt; p.stats = (const float*)stats; p.dq = dq; p.dk = dk; p.dv = dv;
+  p.status = status; p.n_kt = plan.n_kt; p.n_qt = plan.n_qt;
+  p.part = (float4*)scratch; p.left = plan.left; p.edge = (float*)scratch + plan.part;
+  p.q = q; p.k = k; p.dout = dout;
+  for (int i = 0; i < 3; ++i) {
+    p.sdq[i] = sdq[i]; p.sdkv[i] = sdkv[i]; p.sq[i] = sq[i]; p.sk[i] = sk[i];
+  }
+  CUtensorMap tq, tk, tv, tdo, tdq, tdk, tdv;
   int r;
   if ((r = make_tmap_bshd(&tq, q, fmt, B, Sq, H, D, sq[0], sq[1], sq[2]))) return r;
   if ((r = make_tmap_bshd(&tk, k, fmt, B, Sk, H, D, sk[0], sk[1], sk[2]))) return r;
@@ -762,34 +1142,42 @@ PF_API int pf_attn_bwd(const void* dout, const void* q, const void* k, const voi
   if ((r = make_tmap_bshd(&tdo, dout, fmt, B, Sq, H, D, (long long)Sq * H * D, (long long)H * D,
                           D)))
     return r;
-  if (direct) memset(&tdq, 0, sizeof(tdq));
-  else if ((r = make_tmap_dq(&tdq, dq_accum, B, Sq, H, D))) return r;
-  const long long pad_rows = (long long)B * p.n_qt * ATT_BM * H;
-  const unsigned prep = (unsigned)((pad_rows + 31) / 32);
-  float* sums = direct ? nullptr : (float*)dq_accum;
-  if (dtype == PF_F16)
-    attn_bwd_prep_kernel<__half><<<prep, 256, 0, st>>>((const __half*)dout, (const __half*)out,
-        (const float*)lse, (float*)stats, sums, B, Sq, H, D, p.n_qt, scale);
-  else
-    attn_bwd_prep_kernel<__nv_bfloat16><<<prep, 256, 0, st>>>((const __nv_bfloat16*)dout,
-        (const __nv_bfloat16*)out, (const float*)lse, (float*)stats, sums, B, Sq, H, D, p.n_qt,
-        scale);
+  float* sums = plan.mode == DQ_SUMS ? (float*)scratch : nullptr;
+  if ((r = sums ? make_tmap_dq(&tdq, sums, B, Sq, H, D)
+                : make_tmap_grad(&tdq, dq, fmt, B, Sq, H, D, sdq)) ||
+      (r = make_tmap_grad(&tdk, dk, fmt, B, Sk, H, D, sdkv)) ||
+      (r = make_tmap_grad(&tdv, dv, fmt, B, Sk, H, D, sdkv)))
+    return r;
+  if (plan.left) {
+    auto run = [&]() -> int { PF_ATTN_DISPATCH(launch_edge, p, v, out, lse, stats, sv, st); };
+    if ((r = run())) return r;
+  } else {
+    const long long pad_rows = (long long)B * p.n_qt * ATT_BM * H;
+    const unsigned prep = (unsigned)((pad_rows + 31) / 32);
+    if (dtype == PF_F16)
+      attn_bwd_prep_kernel<__half><<<prep, 256, 0, st>>>((const __half*)dout, (const __half*)out,
+          (const float*)lse, (float*)stats, sums, B, Sq, H, D, p.n_qt, scale);
+    else
+      attn_bwd_prep_kernel<__nv_bfloat16><<<prep, 256, 0, st>>>((const __nv_bfloat16*)dout,
+          (const __nv_bfloat16*)out, (const float*)lse, (float*)stats, sums, B, Sq, H, D, p.n_qt,
+          scale);
+  }
   PF_CHECK_LAUNCH();
   {
-    auto run = [&]() -> int { PF_ATTN_DISPATCH(launch_bwd, tq, tk, tv, tdo, tdq, p, st); };
+    auto run = [&]() -> int { PF_ATTN_DISPATCH(launch_bwd, tq, tk, tv, tdo, tdq, tdk, tdv, p, plan.mode, st); };
     if ((r = run())) return r;
   }
-  if (direct) return 0;
+  if (!sums) return 0;
   const long long rows = (long long)B * Sq * H, n = rows * (D / 8);
   long long blocks = (n + 255) / 256;
   const long long cap = (long long)(sm_count > 0 ? sm_count : 148) * 8;
   if (blocks > cap) blocks = cap;
   if (dtype == PF_F16)
     attn_dq_convert_kernel<__half><<<(unsigned)blocks, 256, 0, st>>>(
-        (const float*)dq_accum, (__half*)dq, rows, D, Sq, H, sdq[0], sdq[1], sdq[2]);
+        sums, (__half*)dq, rows, D, Sq, H, sdq[0], sdq[1], sdq[2]);
   else
     attn_dq_convert_kernel<__nv_bfloat16><<<(unsigned)blocks, 256, 0, st>>>(
-        (const float*)dq_accum, (__nv_bfloat16*)dq, rows, D, Sq, H, sdq[0], sdq[1], sdq[2]);
+        sums, (__nv_bfloat16*)dq, rows, D, Sq, H, sdq[0], sdq[1], sdq[2]);
   PF_CHECK_LAUNCH();
   return 0;
 }

@@ -504,12 +504,13 @@ def attn_bwd(do: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor
         dv = torch.empty((B, Sk, H, D), dtype=q.dtype, device=q.device)
     # row statistics per query tile and, unless one key tile holds every key, fp32 sums of dq
     stats = torch.empty((B, H, (Sq + 127) // 128, 256), dtype=torch.float32, device=q.device)
-    acc = None if L.pf_attn_bwd_direct(Sq, Sk, int(causal)) else \
-        torch.empty((B, Sq, H, D), dtype=torch.float32, device=q.device)
+    stream = stream_of(do)               # binds the thread to the device that the next call asks
+    kib = L.pf_attn_bwd_scratch(B, H, Sq, Sk, D, int(causal))
+    acc = torch.empty(kib * 256, dtype=torch.float32, device=q.device) if kib else None
     check(L.pf_attn_bwd(do, q, k, v, o, lse, stats, acc,
                         dq, dk, dv, B, H, Sq, Sk, D, _strides3(q), _strides3(k),
                         _strides3(v), _strides3(dq), _strides3(dk), int(causal), scale,
-                        dt(q.dtype), status_word(q.device), sm_count(q.device), stream_of(do)),
+                        dt(q.dtype), status_word(q.device), sm_count(q.device), stream),
           "pf_attn_bwd")
     return dq, dk, dv
 

@@ -180,3 +180,25 @@ def test_attention_forward_with_pairs_beyond_whole_rounds(Sq, Sk, H):
     want = torch.einsum("hqk,khd->qhd", s.softmax(-1), v[0, :, pick].double())
     assert ((o[0, :, pick] - want).norm() / want.norm()).item() < 2 * 2.0 ** -8
     assert (lse[0, pick] - s.logsumexp(-1)).abs().max().item() < 1e-4
+
+
+WHOLE = [  # B, H, Sq, Sk, D, causal: enough heads that the backward takes each whole, with one and with two
+    # tokens beyond full tiles, ragged tiles, key tiles that not every query tile sees
+    (10, 16, 257, 257, 88, False), (8, 20, 129, 129, 32, False), (8, 19, 130, 130, 64, False),
+    (10, 16, 258, 258, 48, False), (4, 37, 513, 513, 40, False), (10, 16, 257, 257, 128, False),
+    (7, 20, 300, 300, 64, True), (7, 20, 130, 300, 96, True), (7, 20, 300, 130, 72, False),
+    (7, 20, 256, 256, 8, False), (37, 8, 385, 257, 32, False),
+]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,H,Sq,Sk,D,causal", WHOLE)
+def test_attention_backward_of_whole_heads(dtype, B, H, Sq, Sk, D, causal):
+    """The same bounds as at the tile edges; and dQ, whose sums one thread keeps, repeats bit for bit."""
+    from pfeife_b200.ops import kernels as kx
+    test_attention_fwd_bwd_at_tile_edges(dtype, B, H, Sq, Sk, D, causal)
+    q, do = (torch.randn(B, Sq, H, D, device="cuda").to(dtype) for _ in range(2))
+    k, v = (torch.randn(B, Sk, H, D, device="cuda").to(dtype) for _ in range(2))
+    o, lse = kx.attn_fwd(q, k, v, causal, D ** -0.5)
+    first, second = (kx.attn_bwd(do, q, k, v, o, lse, causal, D ** -0.5) for _ in range(2))
+    assert all(torch.equal(a, b) for a, b in zip(first, second))
