@@ -416,14 +416,6 @@ __device__ __forceinline__ bool bwd_item(const AttnBwdParams& p, int r, int n_it
   return true;
 }
 
-// 32 values of row `r` of a 16-bit box of 32 x 32 in the 64-byte swizzle
-template <typename T>
-__device__ __forceinline__ void box_row16(uint8_t* box, int r, const uint32_t (&v)[32]) {
-#pragma unroll
-  for (int c = 0; c < 4; ++c)
-    *reinterpret_cast<uint4*>(box + r * 64 + ((c ^ ((r >> 1) & 3)) << 4)) = pack8<T>(v + c * 8);
-}
-
 // acc[0..31] += w * (columns c0 .. c0 + 31 of a 16-bit row of D values); every lane reads the same row
 template <typename T>
 __device__ __forceinline__ void axpy_row32(uint32_t (&acc)[32], float w, const T* row, int c0, int D) {
@@ -1002,22 +994,6 @@ static int make_tmap_dq(CUtensorMap* map, const void* base, int B, int S, int H,
   return r == CUDA_SUCCESS ? 0 : -(1000 + (int)r);
 }
 
-// 16-bit [B, S, H, D] view with element strides; box = 32 x 1 x 32 x 1 in the 64-byte swizzle
-static int make_tmap_grad(CUtensorMap* map, const void* base, int fmt, int B, int S, int H, int D,
-                          const long long* st) {
-  EncodeTiledFn enc = attn_get_encode();
-  if (!enc) return -100;
-  cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)H, (cuuint64_t)S, (cuuint64_t)B};
-  cuuint64_t strides[3] = {(cuuint64_t)st[2] * 2, (cuuint64_t)st[1] * 2, (cuuint64_t)st[0] * 2};
-  cuuint32_t box[4] = {32, 1, 32, 1};
-  cuuint32_t estr[4] = {1, 1, 1, 1};
-  CUresult r = enc(map, fmt ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
-                   4, const_cast<void*>(base), dims, strides, box, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
-                   CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? 0 : -(1000 + (int)r);
-}
-
 template <typename T, int DP>
 static int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                       const CUtensorMap& tdo, const CUtensorMap& tdq, const CUtensorMap& tdk,
@@ -1144,9 +1120,9 @@ PF_API int pf_attn_bwd(const void* dout, const void* q, const void* k, const voi
     return r;
   float* sums = plan.mode == DQ_SUMS ? (float*)scratch : nullptr;
   if ((r = sums ? make_tmap_dq(&tdq, sums, B, Sq, H, D)
-                : make_tmap_grad(&tdq, dq, fmt, B, Sq, H, D, sdq)) ||
-      (r = make_tmap_grad(&tdk, dk, fmt, B, Sk, H, D, sdkv)) ||
-      (r = make_tmap_grad(&tdv, dv, fmt, B, Sk, H, D, sdkv)))
+                : make_tmap_box32(&tdq, dq, fmt, B, Sq, H, D, sdq)) ||
+      (r = make_tmap_box32(&tdk, dk, fmt, B, Sk, H, D, sdkv)) ||
+      (r = make_tmap_box32(&tdv, dv, fmt, B, Sk, H, D, sdkv)))
     return r;
   if (plan.left) {
     auto run = [&]() -> int { PF_ATTN_DISPATCH(launch_edge, p, v, out, lse, stats, sv, st); };

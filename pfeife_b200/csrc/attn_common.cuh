@@ -32,6 +32,14 @@ __device__ __forceinline__ uint4 pack8(const uint32_t* r) {
                     pack2<T>(__uint_as_float(r[6]), __uint_as_float(r[7])));
 }
 
+// 32 values of row `r` of a 16-bit box of 32 x 32 in the 64-byte swizzle
+template <typename T>
+__device__ __forceinline__ void box_row16(uint8_t* box, int r, const uint32_t (&v)[32]) {
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+    *reinterpret_cast<uint4*>(box + r * 64 + ((c ^ ((r >> 1) & 3)) << 4)) = pack8<T>(v + c * 8);
+}
+
 // one [128 rows x DP] tile = DP/64 (rounded up) swizzled blocks, loaded with one TMA per block
 template <int NBLK>
 __device__ __forceinline__ void load_tile(uint8_t* dst, const CUtensorMap* map, uint64_t* bar,
@@ -113,6 +121,22 @@ inline int make_tmap_bshd(CUtensorMap* map, const void* base, int fmt, int B, in
                    4, const_cast<void*>(base), dims, strides, box, estr,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : -(1000 + (int)r);
+}
+
+// 16-bit [B, S, H, D] view with element strides; box = 32 x 1 x 32 x 1 in the 64-byte swizzle
+inline int make_tmap_box32(CUtensorMap* map, const void* base, int fmt, int B, int S, int H, int D,
+                          const long long* st) {
+  EncodeTiledFn enc = attn_get_encode();
+  if (!enc) return -100;
+  cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)H, (cuuint64_t)S, (cuuint64_t)B};
+  cuuint64_t strides[3] = {(cuuint64_t)st[2] * 2, (cuuint64_t)st[1] * 2, (cuuint64_t)st[0] * 2};
+  cuuint32_t box[4] = {32, 1, 32, 1};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUresult r = enc(map, fmt ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
+                   4, const_cast<void*>(base), dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
+                   CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : -(1000 + (int)r);
 }
 

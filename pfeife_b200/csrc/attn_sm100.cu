@@ -191,7 +191,8 @@ struct FwdCfg {
   static constexpr int OFF_K = 2 * TILE;
   static constexpr int OFF_V = OFF_K + ST * TILE;
   static constexpr int OFF_SIDE = OFF_V + ST * TILE;     // maxima and sums of a split tile's side 1
-  static constexpr int OFF_BAR = OFF_SIDE + 2 * ATT_BM * 4;
+  static constexpr int OFF_BOX = OFF_SIDE + 2 * ATT_BM * 4;   // 8 warps x 2 boxes of 32 rows x 32 columns of O
+  static constexpr int OFF_BAR = OFF_BOX + 8 * 2 * 2048;
   static constexpr int SMEM = OFF_BAR + 256;
   static constexpr int T_O = 256;                        // + t * DP
   static constexpr int T_P = ALIAS_P ? 0 : 256 + 2 * DP;
@@ -309,7 +310,8 @@ __device__ __forceinline__ float probs(const uint32_t (&s)[4][32], uint32_t t_p,
 template <typename T, int DP, bool SPLIT>
 __global__ void __launch_bounds__(FwdCfg<DP>::THREADS, 1)
 attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
-                   const __grid_constant__ CUtensorMap tv, const AttnParams p, const int n_items) {
+                   const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap to,
+                   const AttnParams p, const int n_items) {
   using C = FwdCfg<DP>;
   constexpr int NBLK = C::NBLK, TILE = C::TILE, ST = C::ST;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -337,6 +339,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
   }
   if (tid == 0) {
     tma_prefetch_desc(&tq); tma_prefetch_desc(&tk); tma_prefetch_desc(&tv);
+    tma_prefetch_desc(&to);
     for (int i = 0; i < N_BARS; ++i) mbar_init(&bars[i], 1);
     for (int t = 0; t < 2; ++t) { mbar_init(&s_empty[t], 4); mbar_init(&p_full[t], 4); }
     mbar_init(joined, 4);
@@ -490,7 +493,8 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
     const uint32_t t_p = tmem + C::T_P + t * C::P_TILE + lane_off;
     const float c2 = p.scale * LOG2E;
     const int shift = p.Sk - p.Sq;
-    uint32_t cnt = 0;
+    uint8_t* boxes = smem + C::OFF_BOX + warp * 4096;
+    uint32_t cnt = 0, box = 0;
     bool ok = true;
     for (int r = 0; ok && r * (int)gridDim.x < n_items; ++r) {
       const int w = fwd_index(r);
@@ -656,12 +660,20 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
             for (int i = 0; i < 32; ++i)
               o[i] = __float_as_uint(fmaf(__uint_as_float(o1[i]), w1, __uint_as_float(o[i])));
           }
-          if (qi < p.Sq) {
-#pragma unroll
-            for (int v = 0; v < 4; ++v)
-              if (c * 32 + v * 8 < p.D)
-                reinterpret_cast<uint4*>(dst)[c * 4 + v] = pack8<T>(o + v * 8);
+          // Through boxes: 16 bytes of a row per thread and store take longer to leave than a key tile's
+          // products (at head dim 88 8000 cycles from item to item, 3600 between key tiles).  The store
+          // that last used this box must have read it; rows and columns that do not exist are clipped.
+          uint8_t* bx = boxes + (box & 1) * 2048;
+          if (lane == 0 && box >= 2) tma_store_wait_read_but_one();
+          __syncwarp();
+          box_row16<T>(bx, lane, o);
+          fence_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            tma_store_4d(&to, bx, c * 32, it.h, q0 + quad * 32, it.b);
+            tma_store_commit();
           }
+          ++box;
         }
         if (qi < p.Sq) *lse_dst = (l > 0.f) ? (m_used + log2f(l)) * LN2 : -INFINITY;
       }
@@ -669,6 +681,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
       // tile, which overwrites O, is ordered after them by this warp's next arrival on p_full
       tc_fence_before();
     }
+    if (lane == 0) tma_store_wait_all();
   }
 
   // teardown: every role reaches this point (all waits are bounded)
@@ -679,7 +692,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 
 template <typename T, int DP>
 static int launch_fwd_ws(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
-                         const AttnParams& p, bool two_launches, cudaStream_t st) {
+                         const CUtensorMap& to, const AttnParams& p, bool two_launches, cudaStream_t st) {
   using C = FwdCfg<DP>;
   const int pairs = p.q_pairs * p.H * p.B, tiles = 2 * (pairs - p.n_pair);
   static bool done[2][64] = {};
@@ -688,7 +701,7 @@ static int launch_fwd_ws(const CUtensorMap& tq, const CUtensorMap& tk, const CUt
     auto kern = split ? attn_fwd_ws_kernel<T, DP, true> : attn_fwd_ws_kernel<T, DP, false>;
     const int r = set_smem(kern, C::SMEM, done[split]), sms = attn_sm_count();
     if (r) return r;
-    kern<<<n < sms ? n : sms, C::THREADS, C::SMEM, st>>>(tq, tk, tv, q, n);
+    kern<<<n < sms ? n : sms, C::THREADS, C::SMEM, st>>>(tq, tk, tv, to, q, n);
     PF_CHECK_LAUNCH();
     return 0;
   };
@@ -721,14 +734,16 @@ PF_API int pf_attn_fwd(const void* q, const void* k, const void* v, void* o, voi
   if (dtype != PF_F16 && dtype != PF_BF16) return -1;
   if (D % 8 || D > 128) return -3;
   if (!strides_ok(q, sq[0], sq[1], sq[2]) || !strides_ok(k, sk[0], sk[1], sk[2]) ||
-      !strides_ok(v, sv[0], sv[1], sv[2]))
+      !strides_ok(v, sv[0], sv[1], sv[2]) || (reinterpret_cast<uintptr_t>(o) & 15))
     return -2;
   const int fmt = dtype == PF_BF16;
-  CUtensorMap tq, tk, tv;
+  CUtensorMap tq, tk, tv, to;
   int r;
   if ((r = make_tmap_bshd(&tq, q, fmt, B, Sq, H, D, sq[0], sq[1], sq[2]))) return r;
   if ((r = make_tmap_bshd(&tk, k, fmt, B, Sk, H, D, sk[0], sk[1], sk[2]))) return r;
   if ((r = make_tmap_bshd(&tv, v, fmt, B, Sk, H, D, sv[0], sv[1], sv[2]))) return r;
+  const long long so[3] = {(long long)Sq * H * D, (long long)H * D, D};
+  if ((r = make_tmap_box32(&to, o, fmt, B, Sq, H, D, so))) return r;
   AttnParams p = {};
   p.B = B; p.H = H; p.Sq = Sq; p.Sk = Sk; p.D = D; p.causal = causal; p.scale = scale;
   p.fmt = fmt; p.o = o; p.lse = (float*)lse; p.status = status;
@@ -760,5 +775,5 @@ PF_API int pf_attn_fwd(const void* q, const void* k, const void* v, void* o, voi
                       (p.q_rows > ATT_BM || Sk > 2 * ATT_BN));
   p.n_pair = split ? pairs - left_over : pairs;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  PF_ATTN_DISPATCH(launch_fwd_ws, tq, tk, tv, p, two_launches, st);
+  PF_ATTN_DISPATCH(launch_fwd_ws, tq, tk, tv, to, p, two_launches, st);
 }
