@@ -45,7 +45,7 @@ namespace pf {
 
 constexpr int ATT_TAIL_MAX = 4;      // leftover rows handled on CUDA cores
 constexpr int ATT_TWO_LAUNCH_TILES = 12;   // key tiles from which a second launch pays (see FwdItem)
-constexpr int ATT_TAIL_SEQ_MAX = 2048;  // longest other dimension the CUDA-core paths stage in smem
+constexpr int ATT_TAIL_SEQ_MAX = 2048;  // most keys of a leftover row
 
 struct AttnParams {
   int B, H, Sq, Sk, D;
@@ -65,121 +65,130 @@ struct AttnParams {
   long long sq[3], sk[3], sv[3];
 };
 
-__device__ __forceinline__ float block_reduce(float v, float* red, bool is_max) {
-  // red: 32 floats of shared memory; every thread of the CTA calls
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  v = is_max ? warp_max(v) : warp_sum(v);
-  __syncthreads();
-  if (lane == 0) red[warp] = v;
-  __syncthreads();
-  float r = is_max ? -INFINITY : 0.f;
-  for (int i = 0; i < nw; ++i) r = is_max ? fmaxf(r, red[i]) : r + red[i];
-  return r;
-}
-
-// dot product of a 16-bit global row (16-byte aligned, D a multiple of 8) with fp32 values in
-// shared memory
-template <typename T>
-__device__ __forceinline__ float dot_row(const T* row, const float* sv, int D) {
-  // D <= 128: up to 16 vectors, requested together so that one memory latency covers the row
-  uint4 u[16];
-  const int nv = D / 8;
-#pragma unroll
-  for (int c = 0; c < 16; ++c)
-    if (c < nv) u[c] = __ldg(reinterpret_cast<const uint4*>(row) + c);
-  float s = 0.f;
-#pragma unroll
-  for (int c = 0; c < 16; ++c) {
-    if (c < nv) {
-      const T* e = reinterpret_cast<const T*>(&u[c]);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) s = fmaf(to_f32<T>(e[j]), sv[c * 8 + j], s);
-    }
-  }
-  return s;
-}
-
-// acc[0..7] += w * (8 consecutive 16-bit values at `src`)
-template <typename T>
-__device__ __forceinline__ void axpy8(float (&acc)[8], float w, const uint4& u) {
-  const T* e = reinterpret_cast<const T*>(&u);
-#pragma unroll
-  for (int j = 0; j < 8; ++j) acc[j] = fmaf(w, to_f32<T>(e[j]), acc[j]);
-}
-
-// Forward for one leftover query row on CUDA cores (128 threads).
-template <typename T>
-__device__ void attn_fwd_tail_row(const AttnParams& p, uint8_t* smem, int qi, int h, int b) {
-  float* qs = reinterpret_cast<float*>(smem);       // [128]
-  float* red = qs + 128;                            // [32]
-  float* sc = red + 32;                             // [Sk]
-  const int tid = threadIdx.x;
-  const T* qrow = reinterpret_cast<const T*>(p.q) + b * p.sq[0] + (long long)qi * p.sq[1] +
-                  h * p.sq[2];
-  for (int d = tid; d < p.D; d += blockDim.x) qs[d] = to_f32<T>(qrow[d]);
-  __syncthreads();
-  const float c2 = p.scale * LOG2E;
-  const int shift = p.Sk - p.Sq;
-  const T* kb = reinterpret_cast<const T*>(p.k) + b * p.sk[0] + h * p.sk[2];
-  float mx = -INFINITY;
-  for (int j = tid; j < p.Sk; j += blockDim.x) {
-    const bool vis = !(p.causal && j > qi + shift);
-    const float sj = vis ? dot_row<T>(kb + (long long)j * p.sk[1], qs, p.D) * c2 : -INFINITY;
-    sc[j] = sj;
-    mx = fmaxf(mx, sj);
-  }
-  mx = block_reduce(mx, red, true);
-  const float m_use = (mx == -INFINITY) ? 0.f : mx;
-  float sum = 0.f;
-  for (int j = tid; j < p.Sk; j += blockDim.x) {
-    const float pj = exp2f(sc[j] - m_use);
-    sc[j] = pj;
-    sum += pj;
-  }
-  const float l = block_reduce(sum, red, false);    // its barriers also publish sc[]
-  const float inv = l > 0.f ? 1.f / l : 0.f;
-  {
-    // thread = (key group g of 8, column vector cv of 16): keys g, g+8, ... ; 8 columns each
-    const int cv = tid & 15, g = tid >> 4;
-    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    if (cv * 8 < p.D) {
-      const T* vb = reinterpret_cast<const T*>(p.v) + b * p.sv[0] + h * p.sv[2] + cv * 8;
-      int j = g;
-      for (; j + 24 < p.Sk; j += 32) {
-        const uint4 u0 = __ldg(reinterpret_cast<const uint4*>(vb + (long long)j * p.sv[1]));
-        const uint4 u1 = __ldg(reinterpret_cast<const uint4*>(vb + (long long)(j + 8) * p.sv[1]));
-        const uint4 u2 = __ldg(reinterpret_cast<const uint4*>(vb + (long long)(j + 16) * p.sv[1]));
-        const uint4 u3 = __ldg(reinterpret_cast<const uint4*>(vb + (long long)(j + 24) * p.sv[1]));
-        axpy8<T>(acc, sc[j], u0); axpy8<T>(acc, sc[j + 8], u1);
-        axpy8<T>(acc, sc[j + 16], u2); axpy8<T>(acc, sc[j + 24], u3);
-      }
-      for (; j < p.Sk; j += 8)
-        axpy8<T>(acc, sc[j], __ldg(reinterpret_cast<const uint4*>(vb + (long long)j * p.sv[1])));
-    }
-    __syncthreads();                 // sc[] is dead after this point: reuse it for the fold
-    float* fold = sc;                // [8 groups][128 columns]
-#pragma unroll
-    for (int e = 0; e < 8; ++e) fold[g * 128 + cv * 8 + e] = acc[e];
-    __syncthreads();
-    if (tid < p.D) {
-      float a = 0.f;
-#pragma unroll
-      for (int gg = 0; gg < 8; ++gg) a += fold[gg * 128 + tid];
-      T* dst = reinterpret_cast<T*>(p.o) + (((long long)b * p.Sq + qi) * p.H + h) * p.D;
-      dst[tid] = from_f32<T>(a * inv);
-    }
-  }
-  if (tid == 0)
-    p.lse[((long long)b * p.H + h) * p.Sq + qi] = (l > 0.f) ? (mx + log2f(l)) * LN2 : -INFINITY;
-}
-
-// Leftover rows in kernels of their own: small shared memory and block size, so that many of
-// these latency-bound CTAs share an SM instead of each holding a tensor-core CTA's resources.
-template <typename T>
-__global__ void __launch_bounds__(128)
+// One leftover query row per CTA, on CUDA cores.  Four lanes share a key (8 columns to a lane at a time) and
+// fold the keys they meet into a maximum, a sum and an output of their own; the 32 groups are joined at the
+// end.  Bound by memory: a thread asks for the keys and values of its next two tokens while it works on
+// one, in slots of its own, so that the loop has no barrier ([64, 257, 16, 64] 90 -> 72 us with the tiles,
+// causal [1, 2049, 32, 128] 95 -> 78, against one thread per key and staged scores).
+template <int DP>
+struct TailCfg {
+  static constexpr int NV = DP / 32;                     // vectors of 8 columns per lane
+  static constexpr int THREADS = 128, GROUPS = THREADS / 4, DEPTH = 3;
+  static constexpr int RING = DEPTH * 2 * NV * THREADS * 16;
+  static constexpr int SMEM = RING > 4 * (DP + 2) * 4 ? RING : 4 * (DP + 2) * 4;
+};
+template <typename T, int DP>
+__global__ void __launch_bounds__(TailCfg<DP>::THREADS)
 attn_fwd_tail_kernel(const AttnParams p) {
-  extern __shared__ uint8_t tail_smem[];
-  attn_fwd_tail_row<T>(p, tail_smem, p.q_rows + (int)blockIdx.x, blockIdx.y, blockIdx.z);
+  using C = TailCfg<DP>;
+  constexpr int NV = C::NV, THREADS = C::THREADS, GROUPS = C::GROUPS, DEPTH = C::DEPTH;
+  extern __shared__ __align__(16) uint8_t tail_smem[];
+  uint4* ring = reinterpret_cast<uint4*>(tail_smem) + threadIdx.x;     // [DEPTH][K, V][NV][THREADS]
+  float* warps = reinterpret_cast<float*>(tail_smem);                  // after the loop: [4][DP + 2]
+  const int qi = p.q_rows + (int)blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane & 3, grp = threadIdx.x >> 2;
+  const T* qrow = reinterpret_cast<const T*>(p.q) + b * p.sq[0] + (long long)qi * p.sq[1] + h * p.sq[2];
+  const T* kb = reinterpret_cast<const T*>(p.k) + b * p.sk[0] + h * p.sk[2];
+  const T* vb = reinterpret_cast<const T*>(p.v) + b * p.sv[0] + h * p.sv[2];
+  const float c2 = p.scale * LOG2E;
+  const int keys = p.causal ? max(0, min(p.Sk, qi + p.Sk - p.Sq + 1)) : p.Sk;   // visible to this row
+  const int trips = (keys + GROUPS - 1) / GROUPS;                      // the same for every lane
+  auto in = [&](int i) { return (sub + 4 * i) * 8 < p.D; };
+  auto fetch = [&](int trip) {
+    if (trip < trips) {
+      const long long x = min(trip * GROUPS + grp, keys - 1);
+      uint4* slot = ring + (trip % DEPTH) * 2 * NV * THREADS;
+#pragma unroll
+      for (int i = 0; i < NV; ++i)
+        if (in(i)) {
+          cp_async16(slot + i * THREADS, kb + x * p.sk[1] + (sub + 4 * i) * 8);
+          cp_async16(slot + (NV + i) * THREADS, vb + x * p.sv[1] + (sub + 4 * i) * 8);
+        }
+    }
+    cp_async_commit();
+  };
+#pragma unroll
+  for (int i = 0; i < DEPTH * 2 * NV; ++i)                             // columns beyond D count as zeros
+    if (!in(i % NV)) ring[i * THREADS] = make_uint4(0, 0, 0, 0);
+  for (int i = 0; i < DEPTH - 1; ++i) fetch(i);
+  float q[8 * NV], acc[8 * NV] = {}, m = -INFINITY, l = 0.f;
+  auto widen = [](const uint4& u, float* f) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) f[j] = to_f32<T>(reinterpret_cast<const T*>(&u)[j]);
+  };
+#pragma unroll
+  for (int i = 0; i < NV; ++i)
+    widen(in(i) ? __ldg(reinterpret_cast<const uint4*>(qrow) + sub + 4 * i) : make_uint4(0, 0, 0, 0),
+          q + i * 8);
+  for (int trip = 0; trip < trips; ++trip) {
+    fetch(trip + DEPTH - 1);
+    cp_async_wait<DEPTH - 1>();
+    const uint4* slot = ring + (trip % DEPTH) * 2 * NV * THREADS;
+    float f[8], s = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      widen(slot[i * THREADS], f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) s = fmaf(f[j], q[i * 8 + j], s);
+    }
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    s = trip * GROUPS + grp < keys ? s * c2 : -INFINITY;
+    if (s > m) {                                                       // also the first finite score
+      const float alpha = exp2f(m - s);
+      l *= alpha;
+#pragma unroll
+      for (int j = 0; j < 8 * NV; ++j) acc[j] *= alpha;
+      m = s;
+    }
+    const float w = s == -INFINITY ? 0.f : exp2f(s - m);               // a NaN stays one
+    l += w;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      widen(slot[(NV + i) * THREADS], f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[i * 8 + j] = fmaf(w, f[j], acc[i * 8 + j]);
+    }
+  }
+  cp_async_wait<0>();
+  // the eight groups of a warp, then the warps
+  float mw = m;
+#pragma unroll
+  for (int o = 4; o < 32; o <<= 1) mw = fmaxf(mw, __shfl_xor_sync(0xffffffffu, mw, o));
+  const float mine = mw == -INFINITY ? 0.f : exp2f(m - mw);
+  l *= mine;
+#pragma unroll
+  for (int j = 0; j < 8 * NV; ++j) acc[j] *= mine;
+#pragma unroll
+  for (int o = 4; o < 32; o <<= 1) {
+    l += __shfl_xor_sync(0xffffffffu, l, o);
+#pragma unroll
+    for (int j = 0; j < 8 * NV; ++j) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
+  }
+  __syncthreads();                                                     // `warps` lies over the ring
+  float* w = warps + warp * (DP + 2);
+  if (lane < 4) {
+#pragma unroll
+    for (int j = 0; j < 8 * NV; ++j) w[(sub + 4 * (j / 8)) * 8 + j % 8] = acc[j];
+  }
+  if (lane == 0) { w[DP] = mw; w[DP + 1] = l; }
+  __syncthreads();
+  float mx = -INFINITY, sum = 0.f, o = 0.f;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) mx = fmaxf(mx, warps[i * (DP + 2) + DP]);
+  const int d = threadIdx.x;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float* wi = warps + i * (DP + 2);
+    const float e = mx == -INFINITY ? 0.f : exp2f(wi[DP] - mx);
+    sum = fmaf(e, wi[DP + 1], sum);
+    if (d < DP) o = fmaf(e, wi[d], o);
+  }
+  if (d < p.D)
+    (reinterpret_cast<T*>(p.o) + (((long long)b * p.Sq + qi) * p.H + h) * p.D)[d] =
+        from_f32<T>(sum == 0.f ? 0.f : o / sum);
+  if (d == 0)
+    p.lse[((long long)b * p.H + h) * p.Sq + qi] = (sum > 0.f) ? (mx + log2f(sum)) * LN2 : -INFINITY;
 }
 
 template <int DP>
@@ -714,9 +723,10 @@ static int launch_fwd_ws(const CUtensorMap& tq, const CUtensorMap& tk, const CUt
     return r;
   }
   if (p.q_tail > 0) {
-    // [q 128 | red 32 | scores max(Sk, 8 x 128 for the fold)] floats
-    const int bytes = (160 + (p.Sk > 1024 ? p.Sk : 1024)) * 4;
-    attn_fwd_tail_kernel<T><<<dim3(p.q_tail, p.H, p.B), 128, bytes, st>>>(p);
+    static bool tail_done[64] = {};
+    using Tail = TailCfg<DP>;
+    if ((r = set_smem(attn_fwd_tail_kernel<T, DP>, Tail::SMEM, tail_done))) return r;
+    attn_fwd_tail_kernel<T, DP><<<dim3(p.q_tail, p.H, p.B), Tail::THREADS, Tail::SMEM, st>>>(p);
     PF_CHECK_LAUNCH();
   }
   return 0;
@@ -750,7 +760,7 @@ PF_API int pf_attn_fwd(const void* q, const void* k, const void* v, void* o, voi
   p.q = q; p.k = k; p.v = v;
   for (int i = 0; i < 3; ++i) { p.sq[i] = sq[i]; p.sk[i] = sk[i]; p.sv[i] = sv[i]; }
   // A short leftover (at most ATT_TAIL_MAX rows after at least one full tile) goes to the CUDA-core
-  // kernel, which stages the keys' scores in shared memory; otherwise the last tile is ragged.
+  // kernel, whose time grows with the keys; otherwise the last tile is ragged.
   const int left = Sq % ATT_BM;
   p.q_tail = (Sq > ATT_BM && left > 0 && left <= ATT_TAIL_MAX && Sk <= ATT_TAIL_SEQ_MAX) ? left : 0;
   p.q_rows = Sq - p.q_tail;

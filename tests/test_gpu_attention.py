@@ -202,3 +202,30 @@ def test_attention_backward_of_whole_heads(dtype, B, H, Sq, Sk, D, causal):
     o, lse = kx.attn_fwd(q, k, v, causal, D ** -0.5)
     first, second = (kx.attn_bwd(do, q, k, v, o, lse, causal, D ** -0.5) for _ in range(2))
     assert all(torch.equal(a, b) for a, b in zip(first, second))
+
+
+@pytest.mark.parametrize("D,left,causal", [(32, 1, False), (64, 3, True), (88, 4, False), (128, 1, True)])
+def test_attention_forward_of_leftover_rows(D, left, causal):
+    """Rows beyond full tiles against 64 bits (u / 2 on average for rounding the result; the probabilities
+    stay in fp32), fewer keys than lanes among them, and a NaN key, which reaches every row that sees it."""
+    from pfeife_b200.ops import kernels as kx
+    for Sk in (5, 128 + left, 700):
+        q, k, v = (torch.randn(2, S, 3, D, device="cuda").to(torch.bfloat16) for S in (128 + left, Sk, Sk))
+        o, lse = kx.attn_fwd(q, k, v, causal, D ** -0.5)
+        qr, kr, vr = (t.double() for t in (q, k, v))
+        want, lse_want = (t[..., -left:, :, :] if t.dim() == 4 else t[..., -left:]
+                          for t in ref_attn64(qr, kr, vr, causal, D ** -0.5))
+        assert (o[:, -left:].double() - want).norm() <= 2.0 ** -8 * want.norm()
+        assert (lse[..., -left:] - lse_want).abs().max() < 1e-4
+        k[:, 2] = float("nan")
+        o, _ = kx.attn_fwd(q, k, v, causal, D ** -0.5)
+        assert torch.isnan(o[:, -left:].float()).all()
+    kx.check_status()
+
+
+def ref_attn64(q, k, v, causal, scale):
+    s = torch.einsum("bqhd,bkhd->bhqk", q, k) * scale
+    if causal:
+        s = s.masked_fill(~torch.ones(s.shape[-2:], dtype=torch.bool, device="cuda").tril(
+            k.shape[1] - q.shape[1]), float("-inf"))
+    return torch.einsum("bhqk,bkhd->bqhd", s.softmax(-1), v), s.logsumexp(-1)
