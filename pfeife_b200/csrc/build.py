@@ -1,4 +1,4 @@
-"""Builds the native libraries in-tree with nvcc / g++ (no torch headers, seconds per file).
+"""Builds the native libraries in-tree with nvcc / g++ (seconds per file).
 
     python -m pfeife_b200.csrc.build [--force] [--verbose]
 
@@ -7,6 +7,9 @@ Outputs, next to the package's ``__init__.py``:
   * ``libpfeife_b200_host.so``    - host-side C++ (planner evaluator, step executor helpers)
   * ``libpfeife_b200_calls.<abi>.so`` - the kernel library's entry points as a Python module, for the
     Python that builds it; left out where that has no headers (calls then go through ctypes)
+  * ``libpfeife_b200_eager-<torch>.<abi>.so`` - eager calls of the ops with their autograd nodes, for the
+    PyTorch that is installed, whose headers it takes half a minute over; left out where those are
+    missing or other than it was written against (eager calls then go through Python)
 
 Objects are cached under ``build/`` keyed by source mtime, so rebuilding after a one-file edit
 recompiles one file.
@@ -15,6 +18,9 @@ from __future__ import annotations
 
 import argparse
 import concurrent.futures as cf
+import hashlib
+import importlib.metadata
+import importlib.util
 import os
 import shutil
 import subprocess
@@ -30,6 +36,18 @@ KERNEL_LIB = PKG / "libpfeife_b200_kernels.so"
 HOST_LIB = PKG / "libpfeife_b200_host.so"
 CALLS_LIB = PKG / ("libpfeife_b200_calls" + sysconfig.get_config_var("EXT_SUFFIX"))
 CALLS_SRC = CSRC / "calls.cpp"
+EAGER_SRC = CSRC / "eager.cpp"
+
+
+def eager_lib() -> Path:
+    """The name carries the PyTorch and the Python that the module is built for."""
+    return PKG / (f"libpfeife_b200_eager-{importlib.metadata.version('torch')}"
+                  + sysconfig.get_config_var("EXT_SUFFIX"))
+
+
+def eager_sources() -> str:
+    """What the module says that it was built from; the loader takes no module of other sources."""
+    return hashlib.sha256(b"".join(p.read_bytes() for p in (EAGER_SRC, CSRC / "api.h"))).hexdigest()
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -72,7 +90,7 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) 
     BUILD.mkdir(parents=True, exist_ok=True)
     headers = sorted(CSRC.glob("*.h")) + sorted(CSRC.glob("*.cuh"))
     cu = sorted(CSRC.glob("*.cu"))
-    cpp = [p for p in sorted(CSRC.glob("*.cpp")) if p != CALLS_SRC]
+    cpp = [p for p in sorted(CSRC.glob("*.cpp")) if p not in (CALLS_SRC, EAGER_SRC)]
     nvcc = _nvcc()
     jobs = []
     objs_cu, objs_cpp = [], []
@@ -103,6 +121,30 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) 
     elif force or _stale(CALLS_LIB, [CALLS_SRC, CSRC / "api.h"]):
         _run(["g++", *CXX_FLAGS, "-shared", "-I", str(include), "-I", str(CSRC),
               str(CALLS_SRC), "-o", str(CALLS_LIB)], verbose)
+    _build_eager(include, force, verbose)
+
+
+def _build_eager(include: Path, force: bool, verbose: bool) -> None:
+    spec = importlib.util.find_spec("torch")
+    torch_dir = Path(spec.origin).parent if spec and spec.origin else None
+    cuda = Path(_nvcc()).resolve().parent.parent / "include"
+    if torch_dir is None or not (torch_dir / "include" / "torch" / "extension.h").exists() \
+            or not (include / "Python.h").exists():
+        print("no headers of PyTorch or Python: eager calls go through Python")
+        return
+    lib = eager_lib()
+    if not (force or _stale(lib, [EAGER_SRC, CSRC / "api.h"])):
+        return
+    inc = torch_dir / "include"
+    try:
+        _run(["g++", *[f if f != "-O3" else "-O2" for f in CXX_FLAGS], "-shared",
+              f'-DPF_SOURCES="{eager_sources()}"', "-I", str(inc), "-I",
+              str(inc / "torch" / "csrc" / "api" / "include"), "-I", str(cuda), "-I", str(include), "-I",
+              str(CSRC), str(EAGER_SRC), "-o", str(lib), "-L", str(torch_dir / "lib"), "-ltorch",
+              "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-ltorch_python"], verbose)
+    except RuntimeError as e:              # another PyTorch's interfaces
+        lib.unlink(missing_ok=True)
+        print(f"{lib.name} is not built, eager calls go through Python:\n{str(e)[-2000:]}")
 
 
 def main(argv=None) -> int:

@@ -97,7 +97,7 @@ struct Call<F> {
    METH_FASTCALL, nullptr}
 
 PyMethodDef methods[] = {
-    PF_CALL(pf_gemm), PF_CALL(pf_gemm_workspace), PF_CALL(pf_elementwise), PF_CALL(pf_glu_fwd),
+    PF_CALL(pf_bind_device), PF_CALL(pf_gemm), PF_CALL(pf_gemm_workspace), PF_CALL(pf_elementwise), PF_CALL(pf_glu_fwd),
     PF_CALL(pf_glu_bwd),
     PF_CALL(pf_axpy_f32), PF_CALL(pf_cast), PF_CALL(pf_colsum), PF_CALL(pf_transpose16),
     PF_CALL(pf_norm_fwd), PF_CALL(pf_norm_bwd_ctas), PF_CALL(pf_norm_bwd), PF_CALL(pf_nonfinite),

@@ -27,6 +27,8 @@ _CALLS_LIB = _PKG / ("libpfeife_b200_calls" + sysconfig.get_config_var("EXT_SUFF
 
 _lib: Optional[ctypes.CDLL] = None
 _calls = None
+_eager = None
+_eager_tried = False
 _host: Optional[ctypes.CDLL] = None
 _tried = False
 _launches = 0  # kernels launched through this module (reported by bench.py)
@@ -99,8 +101,12 @@ def load_calls(library: ctypes.CDLL):
     """The Python module of the entry points of `library`, which is loaded with its symbols global."""
     if not _CALLS_LIB.exists():
         return _CtypesCalls(library)
-    loader = importlib.machinery.ExtensionFileLoader("pfeife_b200_calls", str(_CALLS_LIB))
-    spec = importlib.util.spec_from_loader("pfeife_b200_calls", loader)
+    return _load("pfeife_b200_calls", _CALLS_LIB)
+
+
+def _load(name: str, path: Path):
+    loader = importlib.machinery.ExtensionFileLoader(name, str(path))
+    spec = importlib.util.spec_from_loader(name, loader)
     module = importlib.util.module_from_spec(spec)
     loader.exec_module(module)
     return module
@@ -113,6 +119,25 @@ def calls():
     if _calls is None and lib() is not None:
         _calls = load_calls(_lib)
     return _calls
+
+
+def eager():
+    """Eager calls of the ops as a Python module (csrc/eager.cpp), or None: on a machine without CUDA, and
+    where the module was not built for this PyTorch from these sources (the calls then go through
+    Python, which takes them 20 us longer in each direction)."""
+    global _eager, _eager_tried
+    if not _eager_tried:
+        _eager_tried = True
+        if lib() is not None:
+            from ..csrc import build
+            path = build.eager_lib()
+            if path.exists():
+                module = _load("pfeife_b200_eager", path)
+                if module.SOURCES == build.eager_sources():
+                    from . import kernels
+                    module.setup(kernels.status_word, check)
+                    _eager = module
+    return _eager
 
 
 def host_lib() -> Optional[ctypes.CDLL]:
@@ -148,11 +173,9 @@ def bind_thread(device_index: Optional[int] = None) -> None:
     """Makes sure the calling thread has the device's context bound inside the library's own
     CUDA runtime (threads created by PyTorch, such as autograd workers, arrive without one)."""
     idx = torch.cuda.current_device() if device_index is None else device_index
-    if getattr(_tls, "dev", None) != idx:
-        code = lib().pf_bind_device(int(idx))
-        if code != 0:
-            raise KernelError(f"pf_bind_device({idx}): CUDA error {code}")
-        _tls.dev = idx
+    code = calls().pf_bind_device(int(idx))          # remembers what the thread is bound to
+    if code != 0:
+        raise KernelError(f"pf_bind_device({idx}): CUDA error {code}")
 
 
 def stream(device: Optional[int] = None) -> ctypes.c_void_p:
@@ -173,8 +196,7 @@ def stream_of(t: torch.Tensor) -> int:
     device = t.get_device()
     if device < 0:
         raise KernelError("a kernel was called on a tensor that is not on a CUDA device")
-    if getattr(_tls, "dev", None) != device:
-        bind_thread(device)
+    bind_thread(device)
     return torch._C._cuda_getCurrentRawStream(device)
 
 
@@ -206,7 +228,7 @@ def check(code: int, what: str) -> None:
 
 
 def launch_count() -> int:
-    return _launches
+    return _launches + (_eager.launches() if _eager is not None else 0)
 
 
 def add_launches(n: int) -> None:

@@ -28,6 +28,7 @@ from torch import Tensor
 from torch._subclasses.fake_tensor import FakeTensor
 from torch.autograd import forward_ad
 
+from . import _lib
 from . import kernels as kx
 
 ACT_NONE, ACT_GELU, ACT_GELU_TANH, ACT_SILU = 0, 1, 2, 3
@@ -313,6 +314,23 @@ def _plain_call(args) -> int:
     return found if device is not None else 0
 
 
+def _native_call(name: str, *args):
+    """The op's outputs where csrc/eager.cpp takes the call, else None (and the call goes on here): plain
+    CUDA tensors of one 16-bit type, without autocast and with nothing that observes ops."""
+    if _is_compiling():
+        return None
+    module = _lib.eager()
+    return None if module is None else getattr(module, name)(*args)
+
+
+def _native_layer(name: str, *args):
+    """``_native_call`` of an op whose weights may be registered: those have shadows and gradient
+    buckets, which the implementations here look after."""
+    if _is_compiling() or _PARAMS:
+        return None
+    return _native_call(name, *args)
+
+
 def _call(op, *args):
     """The first ``n_out`` outputs of `op`."""
     found = _plain_call(args)
@@ -483,6 +501,9 @@ _autograd(linear_fwd, 1, _linear_backward, setup=_linear_setup)
 def linear(x: Tensor, weight: Tensor, bias: Optional[Tensor] = None,
            activation: Optional[str] = None, residual: Optional[Tensor] = None) -> Tensor:
     """act(x @ weight.T + bias) + residual, one GEMM launch with a fused epilogue."""
+    y = _native_layer("linear", x, weight, bias, residual, _ACT_NAMES[activation])
+    if y is not None:
+        return y
     return _call(linear_fwd, x, weight, bias, residual, _ACT_NAMES[activation])
 
 
@@ -572,6 +593,9 @@ def mlp(x: Tensor, w1: Tensor, b1: Optional[Tensor], w2: Tensor, b2: Optional[Te
         activation: str = "gelu", residual: Optional[Tensor] = None) -> Tensor:
     """Transformer feed-forward block: two GEMMs, activation fused into the first epilogue,
     residual into the second, activation derivative into the dgrad epilogue."""
+    y = _native_layer("mlp", x, w1, b1, w2, b2, residual, _ACT_NAMES[activation])
+    if y is not None:
+        return y
     return _call(mlp_fwd, x, w1, b1, w2, b2, residual, _ACT_NAMES[activation])
 
 
@@ -685,11 +709,17 @@ _autograd(norm_fwd, 2, _norm_backward, setup=_norm_setup)
 def layer_norm(x: Tensor, weight: Tensor, bias: Optional[Tensor], eps: float = 1e-5,
                residual: Optional[Tensor] = None):
     """LayerNorm over the last dim.  With ``residual`` returns ``(y, h)``, h = x + residual."""
+    out = _native_layer("norm", x, weight, bias, residual, eps, False)
+    if out is not None:
+        return out
     y, h = _call(norm_fwd, x, weight, bias, residual, eps, False)
     return (y, h) if residual is not None else y
 
 
 def rms_norm(x: Tensor, weight: Tensor, eps: float = 1e-6, residual: Optional[Tensor] = None):
+    out = _native_layer("norm", x, weight, None, residual, eps, True)
+    if out is not None:
+        return out
     y, h = _call(norm_fwd, x, weight, None, residual, eps, True)
     return (y, h) if residual is not None else y
 
@@ -777,12 +807,14 @@ _autograd(
 
 def swiglu(gate_up: Tensor) -> Tensor:
     """silu(gate) * up on a fused [..., 2H] projection (gate first)."""
-    return _call(glu_fwd, gate_up, False)
+    y = _native_call("glu", gate_up, False)
+    return y if y is not None else _call(glu_fwd, gate_up, False)
 
 
 def geglu(gate_up: Tensor) -> Tensor:
     """gelu(gate) * up on a fused [..., 2H] projection (gate first)."""
-    return _call(glu_fwd, gate_up, True)
+    y = _native_call("glu", gate_up, True)
+    return y if y is not None else _call(glu_fwd, gate_up, True)
 
 
 # =========================================================================== losses
@@ -879,6 +911,9 @@ def cross_entropy(logits: Tensor, target: Tensor, ignore_index: int = -100,
     the forward and the backward is one pass over the logits."""
     V = logits.shape[-1]
     if reduction not in ("none", "sum"):
+        loss = _native_call("cross_entropy", logits, target, ignore_index)
+        if loss is not None:
+            return loss
         return _call(ce_mean_fwd, logits.reshape(-1, V), target.reshape(-1), ignore_index)
     loss = _call(ce_fwd, logits.reshape(-1, V), target.reshape(-1), ignore_index)
     return loss.view(target.shape) if reduction == "none" else loss.sum()
@@ -1037,7 +1072,8 @@ _autograd(rope_qkv_apply, 1, _rope_qkv_backward, setup=_rope_setup)
 
 def rope_qkv(qkv: Tensor, cos: Tensor, sin: Tensor) -> Tensor:
     """``rope`` of the queries and keys of a fused projection [B, S, 3, H, D], for ``attention_qkv``."""
-    return _call(rope_qkv_apply, qkv, cos, sin, False)
+    y = _native_call("rope_qkv", qkv, cos, sin)
+    return y if y is not None else _call(rope_qkv_apply, qkv, cos, sin, False)
 
 
 def rope_qkv_in_one(qkv: Tensor) -> bool:
@@ -1138,7 +1174,8 @@ def attention(q: Tensor, k: Tensor, v: Tensor, causal: bool = False,
     Layout [batch, seq, heads, head_dim]; q/k/v may be strided views of a fused projection."""
     if scale is None:
         scale = 1.0 / math.sqrt(q.shape[-1])
-    return _call(attn_fwd, q, k, v, causal, float(scale))
+    o = _native_call("attention", q, k, v, causal, float(scale))
+    return o if o is not None else _call(attn_fwd, q, k, v, causal, float(scale))
 
 
 # --------------------------------------------------------------------------- packed self-attention
@@ -1194,7 +1231,8 @@ def attention_qkv(qkv: Tensor, causal: bool = False, scale: Optional[float] = No
     """Self-attention directly on a fused QKV projection laid out [B, S, 3, H, D]."""
     if scale is None:
         scale = 1.0 / math.sqrt(qkv.shape[-1])
-    return _call(attn_qkv_fwd, qkv, causal, float(scale))
+    o = _native_call("attention_qkv", qkv, causal, float(scale))
+    return o if o is not None else _call(attn_qkv_fwd, qkv, causal, float(scale))
 
 
 # =========================================================================== UNet ops (NHWC)
@@ -1341,7 +1379,8 @@ _autograd(conv2d_fwd, 1, _conv_backward, setup=_conv_setup)
 def conv2d(x: Tensor, weight: Tensor, bias: Optional[Tensor] = None, stride: int = 1,
            padding: int = 0) -> Tensor:
     """NHWC convolution with a standard [Cout, Cin, KH, KW] weight."""
-    return _call(conv2d_fwd, x, weight, bias, stride, padding)
+    y = _native_call("conv2d", x, weight, bias, stride, padding)
+    return y if y is not None else _call(conv2d_fwd, x, weight, bias, stride, padding)
 
 
 @_custom_op("pfeife::group_norm_fwd")
@@ -1421,7 +1460,8 @@ _autograd(group_norm_fwd, 1, _gn_backward, setup=_gn_setup)
 def group_norm(x: Tensor, weight: Tensor, bias: Tensor, groups: int = 32, eps: float = 1e-5,
                silu: bool = False) -> Tensor:
     """GroupNorm over an NHWC tensor, optionally followed by SiLU in the same kernel."""
-    return _call(group_norm_fwd, x, weight, bias, groups, eps, silu)
+    y = _native_call("group_norm", x, weight, bias, groups, eps, silu)
+    return y if y is not None else _call(group_norm_fwd, x, weight, bias, groups, eps, silu)
 
 
 @_custom_op("pfeife::upsample2x_op")
