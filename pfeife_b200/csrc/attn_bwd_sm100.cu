@@ -88,6 +88,7 @@ attn_bwd_prep_kernel(const T* __restrict__ dout, const T* __restrict__ out,
                      const float* __restrict__ lse, float* __restrict__ stats,
                      float* __restrict__ dq_accum, int B, int S, int H, int D, int n_qt,
                      float scale) {
+  after_previous();
   const int lane = threadIdx.x & 31, sub = lane & 7;
   const long long g = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * 4 + (lane >> 3);
   const int s_pad = n_qt * ATT_BM;
@@ -151,6 +152,7 @@ __global__ void __launch_bounds__(EdgeCfg<DP>::THREADS, EdgeCfg<DP>::CTAS)
 attn_bwd_edge_kernel(const AttnBwdParams p, const T* __restrict__ v, const T* __restrict__ out,
                      const float* __restrict__ lse, float* __restrict__ stats, const long long sv0,
                      const long long sv1, const long long sv2) {
+  after_previous();
   using C = EdgeCfg<DP>;
   constexpr int NV = C::NV, THREADS = C::THREADS, GROUPS = C::GROUPS;
   extern __shared__ __align__(16) uint8_t edge_smem[];
@@ -323,6 +325,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 attn_dq_convert_kernel(const float* __restrict__ acc, T* __restrict__ dq, long long rows, int D,
                        int Sq, int H, long long sb, long long ss, long long sh) {
+  after_previous();
   const int dv = D / 8;
   const long long total = rows * dv;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -542,6 +545,7 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_base_of(tmem_slot);
+  after_previous();
   const int shift = p.Sk - p.Sq, rounds = bwd_rounds<MODE>(p, n_items);
   // one split per warpgroup: its four warps execute the same instruction
   if (warp >= 12) {
@@ -813,7 +817,7 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
           __syncwarp();
           if (lane == 0) mbar_arrive(acc_empty);
         }
-        if (MODE == DQ_SUMS) {
+        if constexpr (MODE == DQ_SUMS) {
           if (kj < p.Sk) {
 #pragma unroll
             for (int v = 0; v < 4; ++v)
@@ -822,33 +826,33 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
                 reinterpret_cast<uint4*>(dvp)[c * 4 + v] = pack8<T>(rv + v * 8);
               }
           }
-          continue;
-        }
-        // A row's 16 bytes per thread take some 6800 cycles to leave at head dim 88, more than the products
-        // of a short item: they go through boxes.  Among the boxes of DQ_SUMS they would only wait
-        // ([12, 513, 25, 64] 181 -> 200 us).
-        for (int t = 0; t < p.left; ++t) {       // the leftover queries' part
-          const long long r = p.Sq + t;
-          axpy_row32<T>(rk, edge[(t * 3 + 1) * n_pad + kj],
-                        reinterpret_cast<const T*>(p.q) + (long long)it.b * p.sq[0] + r * p.sq[1] +
-                            (long long)it.h * p.sq[2],
-                        c * 32, p.D);
-          axpy_row32<T>(rv, edge[t * 3 * n_pad + kj],
-                        reinterpret_cast<const T*>(p.dout) +
-                            (((long long)it.b * (p.Sq + p.left) + r) * p.H + it.h) * p.D,
-                        c * 32, p.D);
-        }
-        uint8_t* bx = next_box();                // half a box each
-        box_row16<T>(bx, lane, rk);
-        box_row16<T>(bx + 2048, lane, rv);
-        fence_async_smem();
-        __syncwarp();
-        if (lane == 0) {
-          if (it.k0 + quad * 32 < p.Sk) {
-            tma_store_4d(&tdk, bx, c * 32, it.h, it.k0 + quad * 32, it.b);
-            tma_store_4d(&tdv, bx + 2048, c * 32, it.h, it.k0 + quad * 32, it.b);
+        } else {
+          // A row's 16 bytes per thread take some 6800 cycles to leave at head dim 88, more than the products
+          // of a short item: they go through boxes.  Among the boxes of DQ_SUMS they would only wait
+          // ([12, 513, 25, 64] 181 -> 200 us).
+          for (int t = 0; t < p.left; ++t) {       // the leftover queries' part
+            const long long r = p.Sq + t;
+            axpy_row32<T>(rk, edge[(t * 3 + 1) * n_pad + kj],
+                          reinterpret_cast<const T*>(p.q) + (long long)it.b * p.sq[0] + r * p.sq[1] +
+                              (long long)it.h * p.sq[2],
+                          c * 32, p.D);
+            axpy_row32<T>(rv, edge[t * 3 * n_pad + kj],
+                          reinterpret_cast<const T*>(p.dout) +
+                              (((long long)it.b * (p.Sq + p.left) + r) * p.H + it.h) * p.D,
+                          c * 32, p.D);
           }
-          tma_store_commit();
+          uint8_t* bx = next_box();                // half a box each
+          box_row16<T>(bx, lane, rk);
+          box_row16<T>(bx + 2048, lane, rv);
+          fence_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            if (it.k0 + quad * 32 < p.Sk) {
+              tma_store_4d(&tdk, bx, c * 32, it.h, it.k0 + quad * 32, it.b);
+              tma_store_4d(&tdv, bx + 2048, c * 32, it.h, it.k0 + quad * 32, it.b);
+            }
+            tma_store_commit();
+          }
         }
       }
       ++items;
@@ -1006,7 +1010,7 @@ static int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
     static bool done[64] = {};       // one per instantiation of this lambda
     const int r = set_smem(kern, C::SMEM, done);
     if (r) return r;
-    kern<<<grid, C::THREADS, C::SMEM, st>>>(tq, tk, tv, tdo, tdq, tdk, tdv, p, n_items);
+    after(kern, grid, C::THREADS, C::SMEM, st)(tq, tk, tv, tdo, tdq, tdk, tdv, p, n_items);
     PF_CHECK_LAUNCH();
     return 0;
   };
@@ -1027,7 +1031,7 @@ static int launch_edge(const AttnBwdParams& p, const void* v, const void* out, c
   static bool done[64] = {};
   const int r = set_smem(attn_bwd_edge_kernel<T, DP>, C::SMEM, done);
   if (r) return r;
-  attn_bwd_edge_kernel<T, DP><<<dim3(p.H, p.B), C::THREADS, C::SMEM, st>>>(
+  after(attn_bwd_edge_kernel<T, DP>, dim3(p.H, p.B), C::THREADS, C::SMEM, st)(
       p, (const T*)v, (const T*)out, (const float*)lse, (float*)stats, sv[0], sv[1], sv[2]);
   PF_CHECK_LAUNCH();
   return 0;
@@ -1131,10 +1135,10 @@ PF_API int pf_attn_bwd(const void* dout, const void* q, const void* k, const voi
     const long long pad_rows = (long long)B * p.n_qt * ATT_BM * H;
     const unsigned prep = (unsigned)((pad_rows + 31) / 32);
     if (dtype == PF_F16)
-      attn_bwd_prep_kernel<__half><<<prep, 256, 0, st>>>((const __half*)dout, (const __half*)out,
+      after(attn_bwd_prep_kernel<__half>, prep, 256, 0, st)((const __half*)dout, (const __half*)out,
           (const float*)lse, (float*)stats, sums, B, Sq, H, D, p.n_qt, scale);
     else
-      attn_bwd_prep_kernel<__nv_bfloat16><<<prep, 256, 0, st>>>((const __nv_bfloat16*)dout,
+      after(attn_bwd_prep_kernel<__nv_bfloat16>, prep, 256, 0, st)((const __nv_bfloat16*)dout,
           (const __nv_bfloat16*)out, (const float*)lse, (float*)stats, sums, B, Sq, H, D, p.n_qt,
           scale);
   }
@@ -1149,10 +1153,10 @@ PF_API int pf_attn_bwd(const void* dout, const void* q, const void* k, const voi
   const long long cap = (long long)(sm_count > 0 ? sm_count : 148) * 8;
   if (blocks > cap) blocks = cap;
   if (dtype == PF_F16)
-    attn_dq_convert_kernel<__half><<<(unsigned)blocks, 256, 0, st>>>(
+    after(attn_dq_convert_kernel<__half>, (unsigned)blocks, 256, 0, st)(
         sums, (__half*)dq, rows, D, Sq, H, sdq[0], sdq[1], sdq[2]);
   else
-    attn_dq_convert_kernel<__nv_bfloat16><<<(unsigned)blocks, 256, 0, st>>>(
+    after(attn_dq_convert_kernel<__nv_bfloat16>, (unsigned)blocks, 256, 0, st)(
         sums, (__nv_bfloat16*)dq, rows, D, Sq, H, sdq[0], sdq[1], sdq[2]);
   PF_CHECK_LAUNCH();
   return 0;

@@ -80,6 +80,7 @@ struct TailCfg {
 template <typename T, int DP>
 __global__ void __launch_bounds__(TailCfg<DP>::THREADS)
 attn_fwd_tail_kernel(const AttnParams p) {
+  after_previous();
   using C = TailCfg<DP>;
   constexpr int NV = C::NV, THREADS = C::THREADS, GROUPS = C::GROUPS, DEPTH = C::DEPTH;
   extern __shared__ __align__(16) uint8_t tail_smem[];
@@ -359,6 +360,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_base_of(tmem_slot);
+  after_previous();
 
   // one split per warpgroup: its four warps execute the same instruction
   if (warp >= 8) {
@@ -710,7 +712,7 @@ static int launch_fwd_ws(const CUtensorMap& tq, const CUtensorMap& tk, const CUt
     auto kern = split ? attn_fwd_ws_kernel<T, DP, true> : attn_fwd_ws_kernel<T, DP, false>;
     const int r = set_smem(kern, C::SMEM, done[split]), sms = attn_sm_count();
     if (r) return r;
-    kern<<<n < sms ? n : sms, C::THREADS, C::SMEM, st>>>(tq, tk, tv, to, q, n);
+    after(kern, n < sms ? n : sms, C::THREADS, C::SMEM, st)(tq, tk, tv, to, q, n);
     PF_CHECK_LAUNCH();
     return 0;
   };
@@ -726,7 +728,7 @@ static int launch_fwd_ws(const CUtensorMap& tq, const CUtensorMap& tk, const CUt
     static bool tail_done[64] = {};
     using Tail = TailCfg<DP>;
     if ((r = set_smem(attn_fwd_tail_kernel<T, DP>, Tail::SMEM, tail_done))) return r;
-    attn_fwd_tail_kernel<T, DP><<<dim3(p.q_tail, p.H, p.B), Tail::THREADS, Tail::SMEM, st>>>(p);
+    after(attn_fwd_tail_kernel<T, DP>, dim3(p.q_tail, p.H, p.B), Tail::THREADS, Tail::SMEM, st)(p);
     PF_CHECK_LAUNCH();
   }
   return 0;

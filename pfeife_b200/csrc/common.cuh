@@ -70,6 +70,14 @@ template <int N> __device__ __forceinline__ void regs_dec() {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
 }
 
+// Programmatic dependent launch: a kernel launched by `after` (below) may start when every CTA of the one
+// before it in its stream has left, before that one's end is known everywhere, and calls this before it
+// reads or writes anything that an earlier kernel may have to do with: it returns when all of those have
+// completed and their results are visible.
+__device__ __forceinline__ void after_previous() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // ----------------------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
@@ -635,6 +643,38 @@ __device__ __forceinline__ float warp_max(float v) {
 #define PF_BF16 2
 
 #define PF_API extern "C" __attribute__((visibility("default")))
+
+// `after(kernel, grid, block, smem, stream)(arguments)` launches a kernel that calls after_previous().
+// The launch and the kernel's set-up then lie under the end of the one before, some 2 us of each.  As a
+// caller sees them, without and with: attention [24, 257, 16, 88] 155 -> 146.5 us (four launches), GroupNorm
+// [4, 128, 128, 320] 103 -> 89 (six), a convolution 351 -> 341 (eight), forward and backward each.  No kernel
+// lets the next one start sooner: CTAs that wait on an SM take its place from others (171, 95 and 345).
+template <typename... P>
+struct LaunchAfter {
+  void (*kernel)(P...);
+  cudaLaunchConfig_t cfg;
+  cudaError_t operator()(const P&... args) {
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    for (; n < (int)cfg.numAttrs; ++n) attr[n] = cfg.attrs[n];       // a cluster's size
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = n + 1;
+    void* list[] = {const_cast<void*>(static_cast<const void*>(&args))...};
+    return cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(kernel), list);
+  }
+};
+template <typename... P>
+inline LaunchAfter<P...> after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                               cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  return {kernel, cfg};
+}
 
 #define PF_CHECK_LAUNCH()                            \
   do {                                               \

@@ -16,6 +16,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 im2col_kernel(const T* __restrict__ x, T* __restrict__ cols, int B, int H, int W, int C, int KH,
               int KW, int Ho, int Wo, int stride, int pad, long long ldc) {
+  after_previous();
   const int cv = C / 8;
   const long long total = (long long)B * Ho * Wo * KH * KW * cv;
   const long long gstride = (long long)gridDim.x * blockDim.x;
@@ -42,6 +43,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 col2im_kernel(const T* __restrict__ dcols, T* __restrict__ dx, int B, int H, int W, int C, int KH,
               int KW, int Ho, int Wo, int stride, int pad, long long ldc) {
+  after_previous();
   const int cv = C / 8;
   const long long total = (long long)B * H * W * cv;
   const long long gstride = (long long)gridDim.x * blockDim.x;
@@ -93,6 +95,7 @@ constexpr int CONV_TILE = 4096;        // elements of a tile: 8 channels of 64 t
 __global__ void __launch_bounds__(128)
 conv_pack_kernel(const uint16_t* __restrict__ w, uint16_t* __restrict__ out, int Cout, int Cin,
                  int taps, int cin8, int per, int vec) {
+  after_previous();
   __shared__ __align__(16) uint16_t tile[CONV_TILE];
   const int co = blockIdx.x, ci0 = blockIdx.y * per;
   const int n_in = co < Cout ? max(0, min(per, Cin - ci0)) : 0, n_out = min(per, cin8 - ci0) / 8;
@@ -120,6 +123,7 @@ conv_pack_kernel(const uint16_t* __restrict__ w, uint16_t* __restrict__ out, int
 __global__ void __launch_bounds__(256)
 conv_pack_flip_kernel(const uint16_t* __restrict__ w, uint16_t* __restrict__ out, int Cout, int Cin,
                       int taps, int cout8, int per, int vec) {
+  after_previous();
   // [per][8 * taps + 2]: rows lie an odd number of words apart
   extern __shared__ __align__(16) uint16_t ftile[];
   const int ci0 = blockIdx.x * 8, co0 = blockIdx.y * per;
@@ -159,6 +163,7 @@ template <typename T>
 __global__ void __launch_bounds__(128)
 conv_unpack_kernel(const float* __restrict__ src, T* __restrict__ dw, int Cin, int taps, int cin8,
                    int per, int vec) {
+  after_previous();
   constexpr int V = 16 / sizeof(T);
   __shared__ float tile[CONV_TILE + 64];
   const int co = blockIdx.x, ci0 = blockIdx.y * per, n = min(per, Cin - ci0);
@@ -271,6 +276,7 @@ __device__ __forceinline__ void gn_fold(float* chan, const float (&a)[8], const 
 template <typename T>
 __global__ void gn_stats_kernel(const T* __restrict__ x, float* __restrict__ part, int HW, int C,
                                 int G, int rows) {
+  after_previous();
   extern __shared__ __align__(16) float chan[];       // [rows][2][C]
   const int ncv = C / 8;
   const int cv = threadIdx.x % ncv, r = threadIdx.x / ncv;
@@ -302,6 +308,7 @@ __global__ void __launch_bounds__(128)
 gn_finalize_kernel(const float* __restrict__ part, float* __restrict__ mean,
                    float* __restrict__ rstd, int slabs, int G, int n_groups, float inv_n,
                    float eps) {
+  after_previous();
   const int i = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (i >= n_groups) return;
   const int b = i / G, g = i - b * G;
@@ -327,6 +334,7 @@ __global__ void gn_apply_kernel(const T* __restrict__ x, const float* __restrict
                                 const float* __restrict__ rstd, const float* __restrict__ gamma,
                                 const float* __restrict__ beta, T* __restrict__ y, int HW, int C,
                                 int G, int rows) {
+  after_previous();
   const int ncv = C / 8, cpg = C / G;
   const int cv = threadIdx.x % ncv, r = threadIdx.x / ncv;
   const int b = blockIdx.y, c0 = cv * 8;
@@ -410,6 +418,7 @@ gn_bwd_stats_kernel(const T* __restrict__ dy, const T* __restrict__ x,
                     const float* __restrict__ gamma, const float* __restrict__ beta,
                     float* __restrict__ part, float* __restrict__ gpart, int HW,
                     int C, int G, int rows) {
+  after_previous();
   extern __shared__ __align__(16) float chan[];       // [rows][2][C]: sum dz * xhat, sum dz; the ring
   const int ncv = C / 8, cpg = C / G;
   const int cv = threadIdx.x % ncv, r = threadIdx.x / ncv;
@@ -461,6 +470,7 @@ __global__ void __launch_bounds__(1024)
 gn_bwd_fold_kernel(const float* __restrict__ part, const float* __restrict__ gpart,
                    float* __restrict__ sumA, float* __restrict__ sumB, float* __restrict__ dgamma,
                    float* __restrict__ dbeta, int B, int slabs, int C, int G) {
+  after_previous();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int group_ctas = (B * G + 31) / 32;
   if ((int)blockIdx.x < group_ctas) {
@@ -510,6 +520,7 @@ gn_bwd_apply_kernel(const T* __restrict__ dy, const T* __restrict__ x,
                     const float* __restrict__ gamma, const float* __restrict__ beta,
                     const float* __restrict__ sumA, const float* __restrict__ sumB,
                     T* __restrict__ dx, int HW, int C, int G, int rows) {
+  after_previous();
   extern __shared__ __align__(16) float ring[];
   const int ncv = C / 8, cpg = C / G;
   const float inv_n = 1.f / ((float)HW * cpg);
@@ -551,6 +562,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 upsample2x_kernel(const T* __restrict__ x, T* __restrict__ y, int B, int H, int W, int C,
                   int backward) {
+  after_previous();
   const int cv = C / 8;
   const long long total = backward ? (long long)B * H * W * cv : (long long)B * 4 * H * W * cv;
   const long long gstride = (long long)gridDim.x * blockDim.x;
@@ -610,7 +622,7 @@ PF_API int pf_im2col(const void* x, void* cols, int B, int H, int W, int C, int 
   if (C % 8 || ldc % 8) return -2;
   const long long total = (long long)B * Ho * Wo * KH * KW * (C / 8);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  PF_DISPATCH_H(dtype, (im2col_kernel<T><<<grid_for(total, sm_count), 256, 0, st>>>(
+  PF_DISPATCH_H(dtype, (after(im2col_kernel<T>, grid_for(total, sm_count), 256, 0, st)(
       (const T*)x, (T*)cols, B, H, W, C, KH, KW, Ho, Wo, stride, pad, ldc)));
   PF_CHECK_LAUNCH();
   return 0;
@@ -622,7 +634,7 @@ PF_API int pf_col2im(const void* dcols, void* dx, int B, int H, int W, int C, in
   if (C % 8 || ldc % 8) return -2;
   const long long total = (long long)B * H * W * (C / 8);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  PF_DISPATCH_H(dtype, (col2im_kernel<T><<<grid_for(total, sm_count), 256, 0, st>>>(
+  PF_DISPATCH_H(dtype, (after(col2im_kernel<T>, grid_for(total, sm_count), 256, 0, st)(
       (const T*)dcols, (T*)dx, B, H, W, C, KH, KW, Ho, Wo, stride, pad, ldc)));
   PF_CHECK_LAUNCH();
   return 0;
@@ -636,8 +648,8 @@ PF_API int pf_groupnorm_slabs(int B, int HW, int C, int sm_count) {
 
 #define PF_GN_SILU(KERN, ...)                                 \
   do {                                                        \
-    if (act_silu) KERN<T, true><<<grid, threads, smem, st>>>(__VA_ARGS__); \
-    else KERN<T, false><<<grid, threads, smem, st>>>(__VA_ARGS__);         \
+    if (act_silu) after(KERN<T, true>, grid, threads, smem, st)(__VA_ARGS__); \
+    else after(KERN<T, false>, grid, threads, smem, st)(__VA_ARGS__);         \
   } while (0)
 
 // `done`: per kernel and device, whether it may already use more than 48 KB of shared memory
@@ -652,7 +664,7 @@ static int gn_launch(void (*kern)(P...), bool* done, dim3 grid, int threads, int
     if (e != cudaSuccess) return (int)e;
     if (dev >= 0 && dev < 64) done[dev] = true;
   }
-  kern<<<grid, threads, smem, st>>>(args...);
+  after(kern, grid, threads, smem, st)(args...);
   return (int)cudaGetLastError();
 }
 
@@ -671,7 +683,7 @@ PF_API int pf_groupnorm_fwd(const void* x, const void* gamma, const void* beta, 
     const int r = gn_launch(gn_stats_kernel<T>, done, grid, threads, gn_smem(rows, C), st,
                             (const T*)x, (float*)scratch, HW, C, G, rows);
     if (r) return r;
-    gn_finalize_kernel<<<(B * G + 3) / 4, 128, 0, st>>>(
+    after(gn_finalize_kernel, (B * G + 3) / 4, 128, 0, st)(
         (const float*)scratch, (float*)mean, (float*)rstd, slabs, G, B * G,
         1.f / ((float)HW * (C / G)), eps);
     const int smem = 0;
@@ -720,7 +732,7 @@ PF_API int pf_groupnorm_bwd(const void* dy, const void* x, const void* mean, con
                        (const float*)beta, part, gpart, HW, C, G, rows);
     });
     if (r) return r;
-    gn_bwd_fold_kernel<<<(B * G + 31) / 32 + (C + 31) / 32, 1024, 0, st>>>(
+    after(gn_bwd_fold_kernel, (B * G + 31) / 32 + (C + 31) / 32, 1024, 0, st)(
         part, gpart, sA, sB, (float*)dgamma, (float*)dbeta, B, slabs, C, G);
     r = gn_bwd_launch(act_silu, threads, [&](auto silu, auto most) {
       constexpr bool S = decltype(silu)::value;
@@ -751,13 +763,13 @@ PF_API int pf_conv_pack(const void* w, void* out, int Cout, int Cin, int taps, i
   const int vec = (reinterpret_cast<uintptr_t>(w) & 15) == 0 && (long long)Cin * taps % 8 == 0;
   if (!flip) {
     const int per = conv_share(cin8, CONV_TILE / taps / 8 * 8);
-    conv_pack_kernel<<<dim3(cout8, (cin8 + per - 1) / per), 128, 0, st>>>(
+    after(conv_pack_kernel, dim3(cout8, (cin8 + per - 1) / per), 128, 0, st)(
         (const uint16_t*)w, (uint16_t*)out, Cout, Cin, taps, cin8, per, vec);
   } else {
     // tiles of 5 to 8 thousand elements; 64 channels make whole 128-byte lines of the output
     const int per = taps <= 9 ? 64 : taps <= 25 ? 32 : 16;
-    conv_pack_flip_kernel<<<dim3(cin8 / 8, (cout8 + per - 1) / per), 256,
-                            per * (8 * taps + 2) * 2, st>>>((const uint16_t*)w, (uint16_t*)out,
+    after(conv_pack_flip_kernel, dim3(cin8 / 8, (cout8 + per - 1) / per), 256,
+                            per * (8 * taps + 2) * 2, st)((const uint16_t*)w, (uint16_t*)out,
                                                             Cout, Cin, taps, cout8, per, vec);
   }
   PF_CHECK_LAUNCH();
@@ -776,9 +788,9 @@ PF_API int pf_conv_unpack(const void* src, void* dw, int Cout, int Cin, int taps
                   (long long)Cin * taps % (dtype == PF_F32 ? 4 : 8) == 0;
   const float* s = (const float*)src;
   switch (dtype) {
-    case PF_F32: conv_unpack_kernel<float><<<grid, 128, 0, st>>>(s, (float*)dw, Cin, taps, cin8, per, vec); break;
-    case PF_F16: conv_unpack_kernel<__half><<<grid, 128, 0, st>>>(s, (__half*)dw, Cin, taps, cin8, per, vec); break;
-    case PF_BF16: conv_unpack_kernel<__nv_bfloat16><<<grid, 128, 0, st>>>(s, (__nv_bfloat16*)dw, Cin, taps, cin8, per, vec); break;
+    case PF_F32: after(conv_unpack_kernel<float>, grid, 128, 0, st)(s, (float*)dw, Cin, taps, cin8, per, vec); break;
+    case PF_F16: after(conv_unpack_kernel<__half>, grid, 128, 0, st)(s, (__half*)dw, Cin, taps, cin8, per, vec); break;
+    case PF_BF16: after(conv_unpack_kernel<__nv_bfloat16>, grid, 128, 0, st)(s, (__nv_bfloat16*)dw, Cin, taps, cin8, per, vec); break;
     default: return -1;
   }
   PF_CHECK_LAUNCH();
@@ -790,7 +802,7 @@ PF_API int pf_upsample2x(const void* x, void* y, int B, int H, int W, int C, int
   if (C % 8) return -2;
   const long long total = (long long)B * H * W * (C / 8) * (backward ? 1 : 4);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  PF_DISPATCH_H(dtype, (upsample2x_kernel<T><<<grid_for(total, sm_count), 256, 0, st>>>(
+  PF_DISPATCH_H(dtype, (after(upsample2x_kernel<T>, grid_for(total, sm_count), 256, 0, st)(
       (const T*)x, (T*)y, B, H, W, C, backward)));
   PF_CHECK_LAUNCH();
   return 0;

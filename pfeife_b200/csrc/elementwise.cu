@@ -40,6 +40,7 @@ template <typename T>
 __global__ void __launch_bounds__(EW_THREADS)
 ew_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ out, long long n,
           int op) {
+  after_previous();
   constexpr int V = Vec16<T>::N;
   const long long nvec = n / V;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -98,6 +99,7 @@ ew_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ out,
 template <typename T>
 __global__ void __launch_bounds__(EW_THREADS)
 glu_fwd_kernel(const T* __restrict__ gu, T* __restrict__ out, long long rows, int H, int gelu) {
+  after_previous();
   constexpr int V = Vec16<T>::N;
   const int hv = H / V;
   const long long total = rows * hv;
@@ -121,6 +123,7 @@ template <typename T>
 __global__ void __launch_bounds__(EW_THREADS)
 glu_bwd_kernel(const T* __restrict__ gu, const T* __restrict__ dout, T* __restrict__ dgu,
                long long rows, int H, int gelu) {
+  after_previous();
   constexpr int V = Vec16<T>::N;
   const int hv = H / V;
   const long long total = rows * hv;
@@ -151,6 +154,7 @@ template <typename T>
 __global__ void __launch_bounds__(EW_THREADS)
 axpy_f32_kernel(float* __restrict__ dst, const T* __restrict__ src, long long n, float scale,
                 int accumulate) {
+  after_previous();
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
     const float v = to_f32<T>(src[i]) * scale;
@@ -161,6 +165,7 @@ axpy_f32_kernel(float* __restrict__ dst, const T* __restrict__ src, long long n,
 template <typename TI, typename TO>
 __global__ void __launch_bounds__(EW_THREADS)
 cast_kernel(const TI* __restrict__ src, TO* __restrict__ dst, long long n) {
+  after_previous();
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
     dst[i] = from_f32<TO>(to_f32<TI>(src[i]));
@@ -173,6 +178,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 colsum_kernel(const T* __restrict__ x, float* __restrict__ out, long long rows, int cols,
               long long ld, int rows_per_cta) {
+  after_previous();
   __shared__ float part[8][33];
   const int c = blockIdx.x * 32 + (threadIdx.x & 31);
   const int ry = threadIdx.x >> 5;
@@ -197,6 +203,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 colsum_vec_kernel(const T* __restrict__ x, float* __restrict__ out, long long rows, int cols,
                   long long ld, int rows_per_cta) {
+  after_previous();
   __shared__ float red[8][256];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c0 = blockIdx.x * 256 + lane * 8;
@@ -228,6 +235,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 transpose_kernel(const T* __restrict__ src, T* __restrict__ dst, int rows, int cols,
                  long long ld_src, long long ld_dst) {
+  after_previous();
   __shared__ T tile[32][33];
   const int bx = blockIdx.x * 32, by = blockIdx.y * 32;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -265,7 +273,7 @@ PF_API int pf_elementwise(const void* a, const void* b, void* out, long long n, 
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   PF_DISPATCH_16_32(dtype, {
     const long long nvec = n / Vec16<T>::N + 1;
-    ew_kernel<T><<<ew_grid(nvec, sm_count), EW_THREADS, 0, st>>>(
+    after(ew_kernel<T>, ew_grid(nvec, sm_count), EW_THREADS, 0, st)(
         (const T*)a, (const T*)b, (T*)out, n, op);
   });
   PF_CHECK_LAUNCH();
@@ -279,7 +287,7 @@ PF_API int pf_glu_fwd(const void* gu, void* out, long long rows, int H, int gelu
   PF_DISPATCH_16_32(dtype, {
     if (H % Vec16<T>::N) return -2;
     const long long total = rows * (H / Vec16<T>::N);
-    glu_fwd_kernel<T><<<ew_grid(total, sm_count), EW_THREADS, 0, st>>>((const T*)gu, (T*)out,
+    after(glu_fwd_kernel<T>, ew_grid(total, sm_count), EW_THREADS, 0, st)((const T*)gu, (T*)out,
                                                                        rows, H, gelu);
   });
   PF_CHECK_LAUNCH();
@@ -293,7 +301,7 @@ PF_API int pf_glu_bwd(const void* gu, const void* dout, void* dgu, long long row
   PF_DISPATCH_16_32(dtype, {
     if (H % Vec16<T>::N) return -2;
     const long long total = rows * (H / Vec16<T>::N);
-    glu_bwd_kernel<T><<<ew_grid(total, sm_count), EW_THREADS, 0, st>>>(
+    after(glu_bwd_kernel<T>, ew_grid(total, sm_count), EW_THREADS, 0, st)(
         (const T*)gu, (const T*)dout, (T*)dgu, rows, H, gelu);
   });
   PF_CHECK_LAUNCH();
@@ -305,7 +313,7 @@ PF_API int pf_axpy_f32(void* dst, const void* src, long long n, float scale, int
   if (n <= 0) return 0;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   PF_DISPATCH_16_32(src_dtype, {
-    axpy_f32_kernel<T><<<ew_grid(n, sm_count), EW_THREADS, 0, st>>>((float*)dst, (const T*)src, n,
+    after(axpy_f32_kernel<T>, ew_grid(n, sm_count), EW_THREADS, 0, st)((float*)dst, (const T*)src, n,
                                                                     scale, accumulate);
   });
   PF_CHECK_LAUNCH();
@@ -318,7 +326,7 @@ PF_API int pf_cast(const void* src, void* dst, long long n, int src_dtype, int d
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const int g = ew_grid(n, sm_count);
 #define PF_CAST_CASE(SD, ST, DD, DT) \
-  if (src_dtype == SD && dst_dtype == DD) cast_kernel<ST, DT><<<g, EW_THREADS, 0, st>>>((const ST*)src, (DT*)dst, n);
+  if (src_dtype == SD && dst_dtype == DD) after(cast_kernel<ST, DT>, g, EW_THREADS, 0, st)((const ST*)src, (DT*)dst, n);
   PF_CAST_CASE(PF_F32, float, PF_F16, __half)
   else PF_CAST_CASE(PF_F32, float, PF_BF16, __nv_bfloat16)
   else PF_CAST_CASE(PF_F16, __half, PF_F32, float)
@@ -345,10 +353,10 @@ PF_API int pf_colsum(const void* x, void* out_f32, long long rows, int cols, lon
     if (per < 32) per = 32;
     gyv = (int)((rows + per - 1) / per);
     if (dtype == PF_F16)
-      colsum_vec_kernel<__half><<<dim3(gxv, gyv), 256, 0, st>>>((const __half*)x, (float*)out_f32,
+      after(colsum_vec_kernel<__half>, dim3(gxv, gyv), 256, 0, st)((const __half*)x, (float*)out_f32,
                                                                 rows, cols, ld, per);
     else
-      colsum_vec_kernel<__nv_bfloat16><<<dim3(gxv, gyv), 256, 0, st>>>(
+      after(colsum_vec_kernel<__nv_bfloat16>, dim3(gxv, gyv), 256, 0, st)(
           (const __nv_bfloat16*)x, (float*)out_f32, rows, cols, ld, per);
     PF_CHECK_LAUNCH();
     return 0;
@@ -360,7 +368,7 @@ PF_API int pf_colsum(const void* x, void* out_f32, long long rows, int cols, lon
   if (rows_per < 64) rows_per = 64;
   gy = (int)((rows + rows_per - 1) / rows_per);
   PF_DISPATCH_16_32(dtype, {
-    colsum_kernel<T><<<dim3(gx, gy), 256, 0, st>>>((const T*)x, (float*)out_f32, rows, cols, ld,
+    after(colsum_kernel<T>, dim3(gx, gy), 256, 0, st)((const T*)x, (float*)out_f32, rows, cols, ld,
                                                    rows_per);
   });
   PF_CHECK_LAUNCH();
@@ -372,7 +380,7 @@ PF_API int pf_transpose16(const void* src, void* dst, int rows, int cols, long l
   if (rows <= 0 || cols <= 0) return 0;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   dim3 grid((cols + 31) / 32, (rows + 31) / 32);
-  transpose_kernel<__half><<<grid, 256, 0, st>>>((const __half*)src, (__half*)dst, rows, cols,
+  after(transpose_kernel<__half>, grid, 256, 0, st)((const __half*)src, (__half*)dst, rows, cols,
                                                  ld_src, ld_dst);
   PF_CHECK_LAUNCH();
   return 0;

@@ -269,6 +269,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
   if (PAIR) cluster_sync();   // the peer's barriers exist before anything is sent to them
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_of(tmem_slot);
+  after_previous();
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -705,6 +706,7 @@ template <int V>
 __global__ void __launch_bounds__(256)
 gemm_fold_kernel(const float* __restrict__ ws, float* __restrict__ C, int M, int N, int parts,
                  long long part_size, int pitch, long long ldc, int accumulate) {
+  after_previous();
   const int nv = (N + V - 1) / V;
   const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
   if (i >= (long long)M * nv) return;
@@ -848,14 +850,15 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUten
     }
     const int pairs = num_tiles < max_pairs ? num_tiles : max_pairs;
     cfg.gridDim = dim3(2 * pairs);
-    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, taux, p);
+    cudaError_t e = LaunchAfter<CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, GemmParams>{
+        kern, cfg}(ta, tb, tc, taux, p);
     if (e != cudaSuccess) return (int)e;
     return 0;
   }
   const int num_tiles = ((p.M + GEMM_BM - 1) / GEMM_BM) * ((p.N + BN - 1) / BN) *
                         (p.split_k > 1 ? p.split_k : 1);
   const int grid = num_tiles < sm_count ? num_tiles : sm_count;
-  kern<<<grid, THREADS, S::TOTAL, stream>>>(ta, tb, tc, taux, p);
+  after(kern, grid, THREADS, S::TOTAL, stream)(ta, tb, tc, taux, p);
   PF_CHECK_LAUNCH();
   return 0;
 }
@@ -1103,7 +1106,7 @@ PF_API int pf_gemm(const void* A, const void* B, void* C, int M, int N, int K, l
       const bool wide = quads >= 256ll * sm_count;
       const unsigned grid = (unsigned)(((wide ? quads : (long long)M * N) + 255) / 256);
       auto fold = wide ? gemm_fold_kernel<4> : gemm_fold_kernel<1>;
-      fold<<<grid, 256, 0, st>>>((const float*)workspace, (float*)C, M, N, plan.parts, part,
+      after(fold, grid, 256, 0, st)((const float*)workspace, (float*)C, M, N, plan.parts, part,
                                  plan.pitch, ldc, accumulate);
       PF_CHECK_LAUNCH();
       return 0;

@@ -37,6 +37,7 @@ __global__ void __launch_bounds__(THREADS < 256 ? 256 : THREADS)
 ce_fwd_kernel(const T* __restrict__ logits, const long long* __restrict__ target,
               float* __restrict__ loss, float* __restrict__ lse, long long rows, int V, long long ld,
               long long ignore_index) {
+  after_previous();
   constexpr int W = THREADS / 32, VN = RowSplit<T>::V, U = 4;
   constexpr int ROWS = THREADS < 256 ? 256 / THREADS : 1;       // rows per CTA, whole warps each
   static_assert(ROWS == 1 || W == 1, "rows that share a CTA are a warp each");
@@ -127,6 +128,7 @@ __global__ void __launch_bounds__(1024)
 ce_mean_kernel(const float* __restrict__ loss, const int* __restrict__ counts,
                const long long* __restrict__ target, float* __restrict__ mean,
                float* __restrict__ inv, int n_in, long long ignore_index) {
+  after_previous();
   float s = 0.f;
   int n = 0;
   for (int i = threadIdx.x; i < n_in; i += 1024) {
@@ -144,6 +146,7 @@ __global__ void __launch_bounds__(1024)
 ce_mean_part_kernel(const float* __restrict__ loss, const long long* __restrict__ target,
                     float* __restrict__ sums, int* __restrict__ counts, long long rows,
                     long long ignore_index) {
+  after_previous();
   float s = 0.f;
   int n = 0;
 #pragma unroll 4
@@ -167,6 +170,7 @@ ce_bwd_kernel(const T* __restrict__ logits, const long long* __restrict__ target
               const float* __restrict__ lse, const float* __restrict__ gscale,
               T* __restrict__ dlogits, long long rows, int V, long long ld, long long ignore_index,
               long long gstride) {
+  after_previous();
   constexpr int VN = RowSplit<T>::V, UNROLL = THREADS < 128 ? 1 : THREADS < 256 ? 2 : 4;
   const long long row = (long long)blockIdx.x * (256 / THREADS) + threadIdx.x / THREADS;
   if (row >= rows) return;
@@ -208,6 +212,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 mse_fwd_kernel(const T* __restrict__ a, const T* __restrict__ b, float* __restrict__ out,
                long long n, float inv_n) {
+  after_previous();
   __shared__ float red[8];
   float s = 0.f;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -229,6 +234,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 mse_bwd_kernel(const T* __restrict__ a, const T* __restrict__ b, const float* __restrict__ gout,
                T* __restrict__ da, long long n, float two_inv_n) {
+  after_previous();
   const float g = gout[0] * two_inv_n;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
@@ -240,6 +246,7 @@ template <typename TT, typename T>
 __global__ void __launch_bounds__(256)
 embed_fwd_kernel(const TT* __restrict__ table, const long long* __restrict__ ids,
                  T* __restrict__ out, int D, long long vocab) {
+  after_previous();
   const long long t = blockIdx.x;
   long long id = ids[t];
   if (id < 0 || id >= vocab) id = 0;
@@ -252,6 +259,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 embed_bwd_kernel(const T* __restrict__ dout, const long long* __restrict__ ids,
                  float* __restrict__ dtable, int D, long long vocab) {
+  after_previous();
   const long long t = blockIdx.x;
   const long long id = ids[t];
   if (id < 0 || id >= vocab) return;
@@ -268,6 +276,7 @@ __global__ void __launch_bounds__(256)
 rope_vec_kernel(const T* __restrict__ x, T* __restrict__ out, const float* __restrict__ cos_t,
                 const float* __restrict__ sin_t, long long B, int S, int H, int D,
                 long long stride_b, long long stride_s, long long stride_h, int inverse) {
+  after_previous();
   const int half = D / 2, hv = half / 8;
   const long long total = B * S * H * hv;
   const long long gstride = (long long)gridDim.x * blockDim.x;
@@ -314,6 +323,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 rope_qkv_kernel(const T* __restrict__ x, T* __restrict__ out, const float* __restrict__ cos_t,
                 const float* __restrict__ sin_t, int S, int H, int D, int inverse) {
+  after_previous();
   const int half = D / 2, hv = half / 8;
   const long long row = blockIdx.x;
   const T* src = x + row * 3 * H * D;
@@ -355,6 +365,7 @@ __global__ void __launch_bounds__(256)
 rope_kernel(const T* __restrict__ x, T* __restrict__ out, const float* __restrict__ cos_t,
             const float* __restrict__ sin_t, long long B, int S, int H, int D,
             long long stride_b, long long stride_s, long long stride_h, int inverse) {
+  after_previous();
   const int half = D / 2;
   const long long total = B * S * H * half;
   const long long gstride = (long long)gridDim.x * blockDim.x;
@@ -414,8 +425,8 @@ PF_API int pf_ce_fwd(const void* logits, const void* target, void* loss, void* l
   if (rows <= 0) return 0;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
 #define PF_CE_FWD(THREADS)                                                                       \
-  ce_fwd_kernel<T, THREADS><<<(unsigned)(THREADS < 256 ? (rows + 7) / 8 : rows),                 \
-                              THREADS < 256 ? 256 : THREADS, 0, st>>>(                           \
+  after(ce_fwd_kernel<T, THREADS>, (unsigned)(THREADS < 256 ? (rows + 7) / 8 : rows),                 \
+                              THREADS < 256 ? 256 : THREADS, 0, st)(                           \
       (const T*)logits, (const long long*)target, (float*)loss, (float*)lse, rows, V, ld,        \
       ignore_index)
   PF_DISPATCH3(dtype, {
@@ -444,12 +455,12 @@ PF_API int pf_ce_mean(const void* loss, const void* target, void* scratch, void*
   if (parts > 1) {
     float* sums = (float*)scratch;
     int* counts = (int*)scratch + parts;
-    ce_mean_part_kernel<<<parts, 1024, 0, st>>>((const float*)loss, (const long long*)target, sums,
+    after(ce_mean_part_kernel, parts, 1024, 0, st)((const float*)loss, (const long long*)target, sums,
                                                 counts, rows, ignore_index);
-    ce_mean_kernel<<<1, 1024, 0, st>>>(sums, counts, nullptr, (float*)mean, (float*)inv, parts,
+    after(ce_mean_kernel, 1, 1024, 0, st)(sums, counts, nullptr, (float*)mean, (float*)inv, parts,
                                        ignore_index);
   } else {
-    ce_mean_kernel<<<1, 1024, 0, st>>>((const float*)loss, nullptr, (const long long*)target,
+    after(ce_mean_kernel, 1, 1024, 0, st)((const float*)loss, nullptr, (const long long*)target,
                                        (float*)mean, (float*)inv, (int)rows, ignore_index);
   }
   PF_CHECK_LAUNCH();
@@ -469,7 +480,7 @@ PF_API int pf_ce_bwd(const void* logits, const void* target, const void* lse, co
   if (slabs > most) slabs = most;
   if (slabs < 1) slabs = 1;
 #define PF_CE_BWD(THREADS, GRID)                                                                 \
-  ce_bwd_kernel<T, THREADS><<<GRID, 256, 0, st>>>(                                               \
+  after(ce_bwd_kernel<T, THREADS>, GRID, 256, 0, st)(                                               \
       (const T*)logits, (const long long*)target, (const float*)lse, (const float*)gscale,       \
       (T*)dlogits, rows, V, ld, ignore_index, gstride)
   PF_DISPATCH3(dtype, {
@@ -491,7 +502,7 @@ PF_API int pf_mse_fwd(const void* a, const void* b, void* out_f32, long long n, 
   long long blocks = (n + 255) / 256;
   const long long cap = (long long)(sm_count > 0 ? sm_count : 148) * 8;
   if (blocks > cap) blocks = cap;
-  PF_DISPATCH3(dtype, (mse_fwd_kernel<T><<<(unsigned)blocks, 256, 0, st>>>(
+  PF_DISPATCH3(dtype, (after(mse_fwd_kernel<T>, (unsigned)blocks, 256, 0, st)(
       (const T*)a, (const T*)b, (float*)out_f32, n, 1.0f / (float)n)));
   PF_CHECK_LAUNCH();
   return 0;
@@ -504,7 +515,7 @@ PF_API int pf_mse_bwd(const void* a, const void* b, const void* gout_f32, void* 
   long long blocks = (n + 255) / 256;
   const long long cap = (long long)(sm_count > 0 ? sm_count : 148) * 8;
   if (blocks > cap) blocks = cap;
-  PF_DISPATCH3(dtype, (mse_bwd_kernel<T><<<(unsigned)blocks, 256, 0, st>>>(
+  PF_DISPATCH3(dtype, (after(mse_bwd_kernel<T>, (unsigned)blocks, 256, 0, st)(
       (const T*)a, (const T*)b, (const float*)gout_f32, (T*)da, n, 2.0f / (float)n)));
   PF_CHECK_LAUNCH();
   return 0;
@@ -516,7 +527,7 @@ PF_API int pf_embed_fwd(const void* table, const void* ids, void* out, long long
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const long long* I = (const long long*)ids;
 #define PF_EMB(TD, TT_, OD, OT_) \
-  if (table_dtype == TD && out_dtype == OD) embed_fwd_kernel<TT_, OT_><<<(unsigned)tokens, 256, 0, st>>>((const TT_*)table, I, (OT_*)out, D, vocab);
+  if (table_dtype == TD && out_dtype == OD) after(embed_fwd_kernel<TT_, OT_>, (unsigned)tokens, 256, 0, st)((const TT_*)table, I, (OT_*)out, D, vocab);
   PF_EMB(PF_F32, float, PF_F32, float)
   else PF_EMB(PF_F32, float, PF_F16, __half)
   else PF_EMB(PF_F32, float, PF_BF16, __nv_bfloat16)
@@ -531,7 +542,7 @@ PF_API int pf_embed_bwd(const void* dout, const void* ids, void* dtable_f32, lon
                         int D, long long vocab, int dtype, void* stream) {
   if (tokens <= 0) return 0;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  PF_DISPATCH3(dtype, (embed_bwd_kernel<T><<<(unsigned)tokens, 256, 0, st>>>(
+  PF_DISPATCH3(dtype, (after(embed_bwd_kernel<T>, (unsigned)tokens, 256, 0, st)(
       (const T*)dout, (const long long*)ids, (float*)dtable_f32, D, vocab)));
   PF_CHECK_LAUNCH();
   return 0;
@@ -549,10 +560,10 @@ PF_API int pf_rope_qkv(const void* x, void* out, const void* cos_t, const void* 
     return -2;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (dtype == PF_F16)
-    rope_qkv_kernel<__half><<<(unsigned)rows, 256, 0, st>>>((const __half*)x, (__half*)out,
+    after(rope_qkv_kernel<__half>, (unsigned)rows, 256, 0, st)((const __half*)x, (__half*)out,
         (const float*)cos_t, (const float*)sin_t, S, H, D, inverse);
   else
-    rope_qkv_kernel<__nv_bfloat16><<<(unsigned)rows, 256, 0, st>>>((const __nv_bfloat16*)x,
+    after(rope_qkv_kernel<__nv_bfloat16>, (unsigned)rows, 256, 0, st)((const __nv_bfloat16*)x,
         (__nv_bfloat16*)out, (const float*)cos_t, (const float*)sin_t, S, H, D, inverse);
   PF_CHECK_LAUNCH();
   return 0;
@@ -576,12 +587,12 @@ PF_API int pf_rope(const void* x, void* out, const void* cos_t, const void* sin_
     if (vblocks < 1) vblocks = 1;
     switch (dtype) {
       case PF_F16:
-        rope_vec_kernel<__half><<<(unsigned)vblocks, 256, 0, st>>>(
+        after(rope_vec_kernel<__half>, (unsigned)vblocks, 256, 0, st)(
             (const __half*)x, (__half*)out, (const float*)cos_t, (const float*)sin_t, B, S, H, D,
             stride_b, stride_s, stride_h, inverse);
         break;
       default:
-        rope_vec_kernel<__nv_bfloat16><<<(unsigned)vblocks, 256, 0, st>>>(
+        after(rope_vec_kernel<__nv_bfloat16>, (unsigned)vblocks, 256, 0, st)(
             (const __nv_bfloat16*)x, (__nv_bfloat16*)out, (const float*)cos_t,
             (const float*)sin_t, B, S, H, D, stride_b, stride_s, stride_h, inverse);
     }
@@ -590,7 +601,7 @@ PF_API int pf_rope(const void* x, void* out, const void* cos_t, const void* sin_
   }
   long long blocks = (total + 255) / 256;
   if (blocks > cap) blocks = cap;
-  PF_DISPATCH3(dtype, (rope_kernel<T><<<(unsigned)blocks, 256, 0, st>>>(
+  PF_DISPATCH3(dtype, (after(rope_kernel<T>, (unsigned)blocks, 256, 0, st)(
       (const T*)x, (T*)out, (const float*)cos_t, (const float*)sin_t, B, S, H, D, stride_b,
       stride_s, stride_h, inverse)));
   PF_CHECK_LAUNCH();

@@ -31,6 +31,7 @@ norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ res, const float*
                 const float* __restrict__ beta, T* __restrict__ y, T* __restrict__ h_out,
                 float* __restrict__ mean_out, float* __restrict__ rstd_out, int N, float eps,
                 int rms) {
+  after_previous();
   constexpr int V = 16 / sizeof(T);
   __shared__ float red[32];
   const long long row = blockIdx.x;
@@ -124,6 +125,7 @@ norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ h, const float* 
                 const float* __restrict__ mean, const float* __restrict__ rstd,
                 const T* __restrict__ dres, T* __restrict__ dx, float* __restrict__ scratch,
                 long long rows, int N, int rms) {
+  after_previous();
   constexpr int V = 16 / sizeof(T);
   __shared__ float red[32];
   const int nvec = N / V;
@@ -214,6 +216,7 @@ norm_fwd_warp_kernel(const T* __restrict__ x, const T* __restrict__ res,
                      const float* __restrict__ gamma, const float* __restrict__ beta,
                      T* __restrict__ y, T* __restrict__ h_out, float* __restrict__ mean_out,
                      float* __restrict__ rstd_out, long long rows, int N, float eps, int rms) {
+  after_previous();
   constexpr int V = 8;
   const int nvec = N / V;
   const int lane = threadIdx.x & 31;
@@ -311,6 +314,7 @@ norm_bwd_fused_kernel(const T* __restrict__ dy, const T* __restrict__ h,
                       const float* __restrict__ rstd, const T* __restrict__ dres,
                       T* __restrict__ dx, float* __restrict__ scratch, long long rows, int N,
                       int rms) {
+  after_previous();
   constexpr int V = 8, R = NORM_TILE_ROWS;
   extern __shared__ __align__(128) uint8_t nsmem[];     // [2 stages][dy, h][R][N]
   const int nvec = N / V, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -455,6 +459,7 @@ norm_bwd_wide_kernel(const T* __restrict__ dy, const T* __restrict__ h,
                      const float* __restrict__ rstd, const T* __restrict__ dres,
                      T* __restrict__ dx, float* __restrict__ scratch, long long rows, int N,
                      int rms) {
+  after_previous();
   constexpr int V = 8, R = NORM_WIDE_ROWS, S = NORM_WIDE_STAGES, WARPS = THREADS / 32;
   static_assert(WARPS <= 32 && R == 2, "one lane per warp folds the sums of two rows");
   __shared__ float4 red[2][WARPS];             // per warp: s1, s2 of both rows; two batches
@@ -576,6 +581,7 @@ norm_bwd_wide_kernel(const T* __restrict__ dy, const T* __restrict__ h,
 __global__ void __launch_bounds__(1024)
 norm_bwd_finish_kernel(const float* __restrict__ scratch, float* __restrict__ dgamma,
                        float* __restrict__ dbeta, int G, int N, int accumulate) {
+  after_previous();
   __shared__ float red[2][32][33];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + lane;
@@ -620,7 +626,7 @@ static int norm_bwd_fused_launch(const void* dy, const void* h, const float* gam
     if (e != cudaSuccess) return (int)e;
     if (dev >= 0 && dev < 64) done[dev] = true;
   }
-  kern<<<G, 256, bytes, st>>>((const T*)dy, (const T*)h, gamma, mean, rstd, (const T*)dres,
+  after(kern, G, 256, bytes, st)((const T*)dy, (const T*)h, gamma, mean, rstd, (const T*)dres,
                               (T*)dx, scratch, rows, N, rms);
   return 0;
 }
@@ -640,7 +646,7 @@ static int norm_bwd_wide_launch(const void* dy, const void* h, const float* gamm
     if (e != cudaSuccess) return (int)e;
     if (dev >= 0 && dev < 64) done[dev] = true;
   }
-  kern<<<G, THREADS, bytes, st>>>((const T*)dy, (const T*)h, gamma, mean, rstd, (const T*)dres,
+  after(kern, G, THREADS, bytes, st)((const T*)dy, (const T*)h, gamma, mean, rstd, (const T*)dres,
                                   (T*)dx, scratch, rows, N, rms);
   return 0;
 }
@@ -655,7 +661,7 @@ static int norm_fwd_launch(const void* x, const void* res, const float* gamma, c
   if constexpr (sizeof(T) == 2) if (nvec <= 32 * 8) {
     const unsigned grid = (unsigned)((rows + 7) / 8);
 #define PF_NORM_FWD_WARP(NV, MAY_RES)                                                         \
-    norm_fwd_warp_kernel<T, NV, MAY_RES><<<grid, 256, 0, st>>>((const T*)x, (const T*)res, gamma, \
+    after(norm_fwd_warp_kernel<T, NV, MAY_RES>, grid, 256, 0, st)((const T*)x, (const T*)res, gamma, \
         beta, (T*)y, (T*)h_out, mean, rstd, rows, N, eps, rms)
     if (nvec <= 32 * 2 && !res) PF_NORM_FWD_WARP(2, false);
     else if (nvec <= 32 * 2) PF_NORM_FWD_WARP(2, true);
@@ -666,13 +672,13 @@ static int norm_fwd_launch(const void* x, const void* res, const float* gamma, c
     return 0;
   }
   if (nvec <= 128 * NORM_MAX_VEC)
-    norm_fwd_kernel<T, 128><<<(unsigned)rows, 128, 0, st>>>((const T*)x, (const T*)res, gamma,
+    after(norm_fwd_kernel<T, 128>, (unsigned)rows, 128, 0, st)((const T*)x, (const T*)res, gamma,
         beta, (T*)y, (T*)h_out, mean, rstd, N, eps, rms);
   else if (nvec <= 256 * NORM_MAX_VEC)
-    norm_fwd_kernel<T, 256><<<(unsigned)rows, 256, 0, st>>>((const T*)x, (const T*)res, gamma,
+    after(norm_fwd_kernel<T, 256>, (unsigned)rows, 256, 0, st)((const T*)x, (const T*)res, gamma,
         beta, (T*)y, (T*)h_out, mean, rstd, N, eps, rms);
   else if (nvec <= 1024 * NORM_MAX_VEC)
-    norm_fwd_kernel<T, 1024><<<(unsigned)rows, 1024, 0, st>>>((const T*)x, (const T*)res, gamma,
+    after(norm_fwd_kernel<T, 1024>, (unsigned)rows, 1024, 0, st)((const T*)x, (const T*)res, gamma,
         beta, (T*)y, (T*)h_out, mean, rstd, N, eps, rms);
   else
     return -3;
@@ -704,13 +710,13 @@ static int norm_bwd_launch(const void* dy, const void* h, const float* gamma, co
 #undef PF_NORM_BWD_WIDE
   }
   if (nvec <= 128 * NORM_MAX_VEC)
-    norm_bwd_kernel<T, 128><<<G, 128, 0, st>>>((const T*)dy, (const T*)h, gamma, mean, rstd,
+    after(norm_bwd_kernel<T, 128>, G, 128, 0, st)((const T*)dy, (const T*)h, gamma, mean, rstd,
         (const T*)dres, (T*)dx, scratch, rows, N, rms);
   else if (nvec <= 256 * NORM_MAX_VEC)
-    norm_bwd_kernel<T, 256><<<G, 256, 0, st>>>((const T*)dy, (const T*)h, gamma, mean, rstd,
+    after(norm_bwd_kernel<T, 256>, G, 256, 0, st)((const T*)dy, (const T*)h, gamma, mean, rstd,
         (const T*)dres, (T*)dx, scratch, rows, N, rms);
   else if (nvec <= 1024 * NORM_MAX_VEC)
-    norm_bwd_kernel<T, 1024><<<G, 1024, 0, st>>>((const T*)dy, (const T*)h, gamma, mean, rstd,
+    after(norm_bwd_kernel<T, 1024>, G, 1024, 0, st)((const T*)dy, (const T*)h, gamma, mean, rstd,
         (const T*)dres, (T*)dx, scratch, rows, N, rms);
   else
     return -3;
@@ -762,7 +768,7 @@ PF_API int pf_norm_bwd(const void* dy, const void* h, const void* gamma, const v
   }
   if (r) return r;
   PF_CHECK_LAUNCH();
-  norm_bwd_finish_kernel<<<(N + 31) / 32, 1024, 0, st>>>((const float*)scratch, (float*)dgamma,
+  after(norm_bwd_finish_kernel, (N + 31) / 32, 1024, 0, st)((const float*)scratch, (float*)dgamma,
                                                          (float*)dbeta, G, N, accumulate);
   PF_CHECK_LAUNCH();
   return 0;
