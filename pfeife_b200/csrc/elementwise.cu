@@ -16,6 +16,14 @@ static inline int ew_grid(long long nvec, int sm_count) {
   return (int)blocks;
 }
 
+// A gated unit's three or five streams go faster by CTAs of one vector per thread that end and begin than by
+// resident ones that stride over the tensors, whose addresses drift apart: 2048 x 11008 bf16 forward 27.1 ->
+// 24.9 us, backward 41.0 -> 35.5.  One and two streams do not (16 Mi values through GELU 23.2 and 24.2).
+static inline unsigned glu_grid(long long nvec) {
+  const long long b = (nvec + EW_THREADS - 1) / EW_THREADS;
+  return (unsigned)(b < 1 ? 1 : b > 0x7fffffff ? 0x7fffffff : b);
+}
+
 template <typename T> struct Vec16 {
   static constexpr int N = 16 / sizeof(T);
   uint4 q;
@@ -287,7 +295,7 @@ PF_API int pf_glu_fwd(const void* gu, void* out, long long rows, int H, int gelu
   PF_DISPATCH_16_32(dtype, {
     if (H % Vec16<T>::N) return -2;
     const long long total = rows * (H / Vec16<T>::N);
-    after(glu_fwd_kernel<T>, ew_grid(total, sm_count), EW_THREADS, 0, st)((const T*)gu, (T*)out,
+    after(glu_fwd_kernel<T>, glu_grid(total), EW_THREADS, 0, st)((const T*)gu, (T*)out,
                                                                        rows, H, gelu);
   });
   PF_CHECK_LAUNCH();
@@ -301,7 +309,7 @@ PF_API int pf_glu_bwd(const void* gu, const void* dout, void* dgu, long long row
   PF_DISPATCH_16_32(dtype, {
     if (H % Vec16<T>::N) return -2;
     const long long total = rows * (H / Vec16<T>::N);
-    after(glu_bwd_kernel<T>, ew_grid(total, sm_count), EW_THREADS, 0, st)(
+    after(glu_bwd_kernel<T>, glu_grid(total), EW_THREADS, 0, st)(
         (const T*)gu, (const T*)dout, (T*)dgu, rows, H, gelu);
   });
   PF_CHECK_LAUNCH();
