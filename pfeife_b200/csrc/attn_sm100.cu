@@ -11,7 +11,8 @@
 // SMs idle, one tile whose keys are shared out: see FwdItem).  Its warps:
 //   warps 0-3 / 4-7   softmax of side 0 / 1, thread <-> query row <-> TMEM lane
 //   warp 8            TMA producer (K and V rings; runs ahead, across item boundaries too)
-//   warp 9            MMA issuer, TMEM owner                   warps 10, 11  idle
+//   warp 9            MMA issuer (warp 10: of side 1, where each has its own), TMEM owner
+//   warp 11           idle
 // Per query tile t and key tile j:
 //     S_t = Q_t K_j^T   tcgen05.mma, shared memory x shared memory -> TMEM
 //     online softmax    S_t read once into registers, base-2 exponent, running maximum and sum
@@ -324,6 +325,12 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
                    const AttnParams p, const int n_items) {
   using C = FwdCfg<DP>;
   constexpr int NBLK = C::NBLK, TILE = C::TILE, ST = C::ST;
+  // Pairs with P in columns of its own: a thread per side issues its products, where one thread for both held
+  // a side's products back until the other's were due ([4, 4096, 10, 64] 265 -> 252 us, 77 keys
+  // [4, 1024, 20, 64] 17.7 -> 16.7).  With P in the columns of S that order is what keeps the sides half a step
+  // apart (head dim 128: 176 us so, 208 with two threads), and the form with split tiles lost, too
+  // ([1, 8192, 10, 64] 264 and 290).
+  constexpr bool TWO_ISSUERS = !C::ALIAS_P && !SPLIT;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::OFF_BAR);
   uint64_t* q_full = bars;               // [2] by query tile
@@ -353,6 +360,8 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
     for (int i = 0; i < N_BARS; ++i) mbar_init(&bars[i], 1);
     for (int t = 0; t < 2; ++t) { mbar_init(&s_empty[t], 4); mbar_init(&p_full[t], 4); }
     mbar_init(joined, 4);
+    if (TWO_ISSUERS)                     // both sides free a tile, in either order
+      for (int i = 0; i < ST; ++i) { mbar_init(&k_empty[i], 2); mbar_init(&v_empty[i], 2); }
     mbar_fence_init();
   }
   if (warp == 9) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
@@ -401,7 +410,62 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
         }
       }
       __syncwarp();
-    } else if (warp == 9) {
+    } else if (TWO_ISSUERS && (warp == 9 || warp == 10)) {
+      // ---------------------------------------------------------------- MMA issuers, one per side
+      if (elect_one()) {
+        const int t = warp - 9;
+        const uint32_t id_o = make_idesc_f16(128, DP, p.fmt, 0, 1);
+        const uint32_t t_s = tmem + t * 128, t_o = tmem + C::T_O + t * DP, t_p = tmem + C::T_P + t * C::P_TILE;
+        const uint32_t sQ = smem_u32(smem + t * TILE);
+        uint32_t g = 0, items = 0, cnt = 0;      // ring position; items and steps of this side so far
+        bool ok = true;
+        for (int r = 0; ok && r * (int)gridDim.x < n_items; ++r) {
+          const int w = fwd_index(r);
+          if (w >= n_items) continue;
+          const FwdItem it = fwd_item(p, w);
+          const int n = t ? it.n[1] : it.n[0], other = t ? it.n[0] : it.n[1];
+          auto keys = [&](int j) { return (min(ATT_BN, p.Sk - j * ATT_BN) + 15) / 16 * 16; };
+          // a tile is free when both sides have read it; one that the other does not read counts twice
+          auto free_tile = [&](uint64_t* bar, int j) {
+            tc_commit(bar);
+            if (j >= other) tc_commit(bar);
+          };
+          // S of step j, once the previous scores are in registers
+          auto issue_s = [&](int j) -> bool {
+            const int st = (g + j) % ST;
+            if (!mbar_wait(&k_full[st], ((g + j) / ST) & 1, p.status, PF_ERR_TIMEOUT_FULL)) return false;
+            if (cnt > 0 && !mbar_wait(&s_empty[t], (cnt - 1) & 1, p.status, PF_ERR_TIMEOUT_TMEM_EMPTY))
+              return false;
+            tc_fence_after();
+            mma_kk<DP / 16>(t_s, sQ, smem_u32(smem + C::OFF_K + st * TILE),
+                            make_idesc_f16(128, keys(j), p.fmt, 0, 0));
+            tc_commit(&s_full[t]);
+            free_tile(&k_empty[st], j);
+            if (j == n - 1) tc_commit(&q_empty[t]);
+            ++cnt;
+            return true;
+          };
+          if (n > 0) {
+            ok = mbar_wait(&q_full[t], items & 1, p.status, PF_ERR_TIMEOUT_FULL) && issue_s(0);
+            ++items;
+          }
+          for (int j = 0; j < n && ok; ++j) {
+            const uint32_t c = cnt - 1;          // step j
+            if (j + 1 < n && !(ok = issue_s(j + 1))) break;
+            const int st = (g + j) % ST;
+            ok = mbar_wait(&v_full[st], ((g + j) / ST) & 1, p.status, PF_ERR_TIMEOUT_FULL) &&
+                 mbar_wait(&p_full[t], c & 1, p.status, PF_ERR_TIMEOUT_FULL);
+            if (!ok) break;
+            tc_fence_after();
+            mma_t_mn(t_o, t_p, 32, smem_u32(smem + C::OFF_V + st * TILE), id_o, j > 0, keys(j) / 16);
+            tc_commit(&pv_done[t]);
+            free_tile(&v_empty[st], j);
+          }
+          g += max(n, other);
+        }
+      }
+      __syncwarp();
+    } else if (!TWO_ISSUERS && warp == 9) {
       // ---------------------------------------------------------------- MMA issuer
       if (elect_one()) {
         const uint32_t id_s = make_idesc_f16(128, 128, p.fmt, 0, 0);
