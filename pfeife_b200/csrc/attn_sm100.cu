@@ -24,12 +24,15 @@
 // What bounds it: 16384 exponentials per tile, 1024 cycles of the special-function units, against
 // 8 x head dim cycles of tensor core (512 at head dim 64; at 128 both take 1024).  Two tiles in
 // flight keep one tile's products under the other's exponentials.
-// Measured (B200, CUDA events, L2 flushed), against one query tile per CTA with P in shared
-// memory: [4, 4096, 10, 64] 402 -> 273 us, causal [1, 2048, 32, 128] 87 -> 51,
-// [2, 2048, 16, 128] 114 -> 82, causal [6, 1782, 21, 32] 200 -> 104, 77 keys [4, 1024, 20, 64]
-// 32 -> 20, [24, 257, 16, 88] 62 -> 52.  Steps on the way at [4, 4096, 10, 64]: 346 with two query
-// tiles per CTA, 305 with one elected thread issuing the products, 292 with the maximum found in the
-// pass over the exponentials, 273 with the pairs beyond whole rounds split.
+// Measured (B200, CUDA events, cold L2), against one query tile per CTA with P in shared
+// memory: [4, 4096, 10, 64] 402 -> 236 us, causal [1, 2048, 32, 128] 87 -> 48, causal [6, 1782, 21, 32]
+// 200 -> 101, 77 keys [4, 1024, 20, 64] 32 -> 17.7, [24, 257, 16, 88] 62 -> 39.  Steps on the way at
+// [4, 4096, 10, 64]: 346 with two query tiles per CTA, 305 with one elected thread issuing the products,
+// 292 with the maximum found in the pass over the exponentials, 273 with the pairs beyond whole rounds
+// split, 266 with O leaving through boxes, 249 with an issuing thread per query tile, 236 with the split
+// pairs' launch beside the other.  The two sides
+// of a CTA run in step, so that the 1000 of a step's 3100 cycles in which a side waits, loads and
+// stores find nobody at the exponentials: held half a step apart, a step takes 2770, but they drift back.
 // TMEM (512 columns): S_0, S_1 128 each, O_0, O_1 one head dim each.  Up to head dim 64 P_0, P_1
 // have 64 columns of their own, so S of the next key tile is issued as soon as this one's scores
 // are in registers; above, P_t takes the columns of S_t and the next S_t waits until P_t V has
@@ -38,14 +41,13 @@
 // Short tails.  A sequence length just above a multiple of 128 (ViT: 257 = 2 x 128 + the class
 // token) would spend a whole item on a few rows.  When at most ATT_TAIL_MAX rows are left over, the
 // tensor-core tiles cover only the full multiples and a small CUDA-core kernel computes the
-// leftover query rows ([24, 257, 16, 88]: 68 -> 58 us).
+// leftover query rows (see attn_fwd_tail_kernel).
 #include "attn_common.cuh"
 #include "api.h"
 
 namespace pf {
 
 constexpr int ATT_TAIL_MAX = 4;      // leftover rows handled on CUDA cores
-constexpr int ATT_TWO_LAUNCH_TILES = 12;   // key tiles from which a second launch pays (see FwdItem)
 constexpr int ATT_TAIL_SEQ_MAX = 2048;  // most keys of a leftover row
 
 struct AttnParams {
@@ -61,6 +63,10 @@ struct AttnParams {
   int n_pair;           // the first items are pairs, the others split tiles (see FwdItem)
   int item0;            // first item of this launch
   int q_tail;           // leftover rows
+  // A call's launches need nothing of one another, so that the next one's CTAs start on the SMs that the
+  // last round leaves idle (a CTA of the tensor-core kernel holds an SM to itself).  They find the inputs
+  // complete, which the first launch has waited for, and read them through L2 only.
+  int not_first, not_last;
   // raw views for the leftover rows (element strides: batch, seq, head)
   const void* q; const void* k; const void* v;
   long long sq[3], sk[3], sv[3];
@@ -80,8 +86,7 @@ struct TailCfg {
 };
 template <typename T, int DP>
 __global__ void __launch_bounds__(TailCfg<DP>::THREADS)
-attn_fwd_tail_kernel(const AttnParams p) {
-  after_previous();
+attn_fwd_tail_kernel(const AttnParams p) {       // never a call's first launch
   using C = TailCfg<DP>;
   constexpr int NV = C::NV, THREADS = C::THREADS, GROUPS = C::GROUPS, DEPTH = C::DEPTH;
   extern __shared__ __align__(16) uint8_t tail_smem[];
@@ -120,7 +125,7 @@ attn_fwd_tail_kernel(const AttnParams p) {
   };
 #pragma unroll
   for (int i = 0; i < NV; ++i)
-    widen(in(i) ? __ldg(reinterpret_cast<const uint4*>(qrow) + sub + 4 * i) : make_uint4(0, 0, 0, 0),
+    widen(in(i) ? __ldcg(reinterpret_cast<const uint4*>(qrow) + sub + 4 * i) : make_uint4(0, 0, 0, 0),
           q + i * 8);
   for (int trip = 0; trip < trips; ++trip) {
     fetch(trip + DEPTH - 1);
@@ -191,6 +196,7 @@ attn_fwd_tail_kernel(const AttnParams p) {
         from_f32<T>(sum == 0.f ? 0.f : o / sum);
   if (d == 0)
     p.lse[((long long)b * p.H + h) * p.Sq + qi] = (sum > 0.f) ? (mx + log2f(sum)) * LN2 : -INFINITY;
+  if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) after_previous();
 }
 
 template <int DP>
@@ -369,7 +375,8 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_base_of(tmem_slot);
-  after_previous();
+  if (!p.not_first) after_previous();
+  if (p.not_last && tid == 0) let_next_start();
 
   // one split per warpgroup: its four warps execute the same instruction
   if (warp >= 8) {
@@ -763,6 +770,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
   tc_fence_before();
   __syncthreads();
   if (warp == 9) { tc_fence_after(); tmem_dealloc(tmem, 512); }
+  if (p.not_first && blockIdx.x == 0) after_previous();
 }
 
 template <typename T, int DP>
@@ -781,18 +789,31 @@ static int launch_fwd_ws(const CUtensorMap& tq, const CUtensorMap& tk, const CUt
     return 0;
   };
   int r;
+  AttnParams first = p;
+  first.not_last = two_launches || p.q_tail > 0;
   if (two_launches) {
     AttnParams rest = p;
     rest.item0 = p.n_pair;
-    if ((r = run(p, false, p.n_pair)) || (r = run(rest, true, tiles))) return r;
-  } else if ((r = run(p, tiles > 0, p.n_pair + tiles))) {
+    rest.not_first = 1;
+    rest.not_last = p.q_tail > 0;
+    if ((r = run(first, false, p.n_pair)) || (r = run(rest, true, tiles))) return r;
+  } else if ((r = run(first, tiles > 0, p.n_pair + tiles))) {
     return r;
   }
   if (p.q_tail > 0) {
     static bool tail_done[64] = {};
     using Tail = TailCfg<DP>;
-    if ((r = set_smem(attn_fwd_tail_kernel<T, DP>, Tail::SMEM, tail_done))) return r;
-    after(attn_fwd_tail_kernel<T, DP>, dim3(p.q_tail, p.H, p.B), Tail::THREADS, Tail::SMEM, st)(p);
+    // The leftover rows start on the SMs that the last round leaves idle.  No SM may take many more than
+    // its share of them, or the others would wait for it: shared memory that nobody uses sees to that.
+    // us, after the tiles' end, at once with all that fit on an SM, and with this many: [24, 257, 16, 88]
+    // 42.2, 43.5, 39.1; [64, 257, 16, 64] 66.5, 63.8, 63.8; [16, 513, 16, 64] 54.0, 62.0, 53.4; causal
+    // [4, 1025, 16, 128] 50.8, 55.6, 45.0; [24, 258, 16, 88] 49.1, 47.3, 45.9; [8, 641, 16, 64] 51.3,
+    // 46.9, 44.8.
+    const long long share = (long long)p.q_tail * p.H * p.B / attn_sm_count();
+    const int per_sm = share < 2 ? 2 : share < 8 ? (int)share : 8, room = 228 * 1024 / per_sm - 2048;
+    if ((r = set_smem(attn_fwd_tail_kernel<T, DP>, 112 * 1024, tail_done))) return r;
+    after(attn_fwd_tail_kernel<T, DP>, dim3(p.q_tail, p.H, p.B), Tail::THREADS,
+          room > Tail::SMEM ? room : Tail::SMEM, st)(p);
     PF_CHECK_LAUNCH();
   }
   return 0;
@@ -834,16 +855,18 @@ PF_API int pf_attn_fwd(const void* q, const void* k, const void* v, void* o, voi
   // Pairs left over after whole rounds are split into tiles when these fit one round (FwdItem).  The
   // form of the kernel that can do both takes 4 to 9 % longer over a pair: up to three rounds it gains
   // all the same ([4, 1024, 20, 64] 56 us whole, 48 split, [2, 2048, 20, 128] 116 and 103), after more
-  // it does not.  There the whole rounds go to the form without and the tiles to a second launch.  640
-  // pairs of head dim 64, whole and in two, by key tiles: 8 94 and 94 us, 12 129 and 128, 14 145 and 143,
-  // 16 163 and 159, 24 229 and 220, 32 297 and 282; head dims 32 and 128, 600 and 664 pairs alike, 900
-  // (six rounds) 1 to 3 % from 20 tiles on, 1500 (ten) 3 % at 128 and nothing at 64.  Causal items differ
-  // in length and are dealt by it: there only a call without a whole round is split.
+  // it does not.  There the whole rounds go to the form without and the tiles to a second launch, whose
+  // CTAs start where the first one's leave.  us, by pairs of head dim 64 and key tiles, in one launch and
+  // in two: 640 and 4 51.2 51.5, 8 85.5 79.6, 16 146 133, 32 255 238; 664 and 8 86.5 84.2; 900 and 8 113
+  // 105.5, 16 201 181; 1500 and 8 170 167; head dim 32 alike.  In three rounds: 468 and 8 64.0 62.2, 500 and
+  // 8 63.8 65.7, 464 and 16 107.7 103.5, 496 and 16 109 108.  At head dim 128: 640 and 8 99.5 106, 16 177
+  // 176; 900 and 8 134 141, 16 243 240.  Causal items differ in length and are dealt by it: there only a
+  // call without a whole round is split.
   const int pairs = p.q_pairs * H * B, left_over = pairs % attn_sm_count();
   const int rounds = pairs / attn_sm_count();
   const bool fits = left_over > 0 && 2 * left_over <= attn_sm_count();
-  const bool two_launches =
-      fits && !causal && rounds > 3 && Sk > (ATT_TWO_LAUNCH_TILES - 1) * ATT_BN;
+  const int two_from = D > 64 ? (rounds > 3 ? 12 : INT_MAX) : rounds > 3 ? 8 : rounds == 3 ? 16 : INT_MAX;
+  const bool two_launches = fits && !causal && (Sk + ATT_BN - 1) / ATT_BN >= two_from;
   // One tile per head is no pair to begin with: its keys are shared out from the third key tile on
   // ([1, 128, 4, 128] 7.2 us whole, 7.8 split).
   const bool split = two_launches ||

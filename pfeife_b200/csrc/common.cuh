@@ -77,6 +77,12 @@ template <int N> __device__ __forceinline__ void regs_dec() {
 __device__ __forceinline__ void after_previous() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
+// Called by a CTA after after_previous(): the next kernel may start as soon as every CTA has called it.  Only
+// for a next kernel that needs nothing of this one; that one has a CTA call after_previous() before it
+// leaves, so that whatever comes later finds both completed.
+__device__ __forceinline__ void let_next_start() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 
 // ----------------------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
@@ -648,7 +654,8 @@ __device__ __forceinline__ float warp_max(float v) {
 // The launch and the kernel's set-up then lie under the end of the one before, some 2 us of each.  As a
 // caller sees them, without and with: attention [24, 257, 16, 88] 155 -> 146.5 us (four launches), GroupNorm
 // [4, 128, 128, 320] 103 -> 89 (six), a convolution 351 -> 341 (eight), forward and backward each.  No kernel
-// lets the next one start sooner: CTAs that wait on an SM take its place from others (171, 95 and 345).
+// lets one that depends on it start sooner: CTAs that wait on an SM take its place from others (171, 95 and
+// 345).
 template <typename... P>
 struct LaunchAfter {
   void (*kernel)(P...);

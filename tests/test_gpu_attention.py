@@ -223,6 +223,54 @@ def test_attention_forward_of_leftover_rows(D, left, causal):
     kx.check_status()
 
 
+@pytest.mark.parametrize("S,H,D,causal", [(1024, 160, 32, False), (1025, 152, 64, False), (1537, 110, 128, False),
+                                          (2050, 58, 64, False), (257, 150, 88, True), (129, 1200, 32, False)])
+def test_attention_forward_of_several_launches(S, H, D, causal):
+    """Launches of a call that run beside one another: inputs overwritten before it and right after it, results
+    used at once, eagerly and replayed, give the bits of calls that have the device to themselves; the
+    last rows (of the last launch) and one head are within u of 64 bits."""
+    from pfeife_b200.ops import kernels as kx
+    sets = [[torch.randn(1, S, H, D, device="cuda").to(torch.bfloat16) for _ in range(3)] for _ in range(3)]
+    want = []
+    for q, k, v in sets:
+        torch.cuda.synchronize()
+        want.append(kx.attn_fwd(q, k, v, causal, D ** -0.5))
+        torch.cuda.synchronize()
+    q, k, v = (t.clone() for t in sets[0])
+    outs = [[torch.zeros_like(t) for t in w] for w in want]
+
+    def all_sets():
+        for i, given in enumerate(sets):
+            for t, g in zip((q, k, v), given):
+                t.copy_(g)
+            for t, r in zip(outs[i], kx.attn_fwd(q, k, v, causal, D ** -0.5)):
+                t.copy_(r)
+
+    def check():
+        torch.cuda.synchronize()
+        for o, w in zip(outs, want):
+            assert all(torch.equal(a, b) for a, b in zip(o, w))
+            for t in o:
+                t.zero_()
+
+    for _ in range(3):
+        all_sets()
+        check()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        all_sets()
+    for _ in range(3):
+        graph.replay()
+        check()
+    for h in (0, H - 1):
+        o64, lse64 = ref_attn64(*(t[:, :, h:h + 1].double() for t in sets[0]), causal, D ** -0.5)
+        o, lse = want[0][0][:, :, h:h + 1].double(), want[0][1][:, h:h + 1]
+        for rows in (slice(None), slice(-(S % 128 or 128), None)):
+            assert (o[:, rows] - o64[:, rows]).norm() <= 2.0 ** -8 * o64[:, rows].norm()
+        assert (lse - lse64).abs().max() < 1e-4
+    kx.check_status()
+
+
 def ref_attn64(q, k, v, causal, scale):
     s = torch.einsum("bqhd,bkhd->bhqk", q, k) * scale
     if causal:
