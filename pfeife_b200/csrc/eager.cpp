@@ -3,8 +3,9 @@
 //
 // What bounds a small call is the host: through Python an op took the caller 20 to 30 us forward and as
 // much again backward, where autograd's thread also has to wait for the interpreter lock.  Here it takes
-// a few.  (Forward and backward of a LayerNorm with residual 161 -> EAGER_NORM us, logits of 4 images by
-// ViT-Tiny 2590 -> EAGER_VIT us.)
+// a few: linear 6.1 us, MLP 9.8, LayerNorm with residual 6.1, attention 5.4.  (As a caller sees them, forward
+// and backward of a LayerNorm with residual 160 -> 81 us, what is left being autograd's hop to its thread
+// and back; logits of 4 images by ViT-Tiny 2540 -> 753 us.)
 //
 // Only the usual call is taken: plain CUDA tensors of one device and one 16-bit type, no autocast, nothing
 // that observes ops (dispatch or function modes, transforms, traces, forward-mode gradients).  For every
