@@ -140,15 +140,18 @@ template <int DP>
 struct EdgeCfg {
   static constexpr int NV = DP / 32;                     // vectors of 8 columns per lane
   static constexpr int THREADS = 128, GROUPS = THREADS / 4;
-  static constexpr int CTAS = NV > 3 ? 2 : 3;            // per SM
+  // per SM: shared memory bounds it above head dim 64, registers below.  Four there gain where heads fill
+  // them ([64, 257, 16, 64] 154 -> 150 us with the tiles, [32, 129, 16, 64] 44 -> 40) and lose 1 to 2 %
+  // where they do not ([8, 257, 12, 64] 27.1 -> 27.6).
+  static constexpr int CTAS = NV > 3 ? 2 : 3, CTAS_MANY = NV > 2 ? CTAS : 4;
   static constexpr int RING = 2 * 5 * NV * THREADS * 16;
   static constexpr int OFF_VECS = RING, OFF_LSE = OFF_VECS + 4 * DP * 4;
   static constexpr int SMEM = OFF_LSE + (BWD_WHOLE_TILES * ATT_BM + BWD_LEFT_MAX) * 4;
   static_assert(4 * 3 * DP * 4 <= RING, "the warps' sums lie over the ring");
 };
 
-template <typename T, int DP>
-__global__ void __launch_bounds__(EdgeCfg<DP>::THREADS, EdgeCfg<DP>::CTAS)
+template <typename T, int DP, int CTAS>
+__global__ void __launch_bounds__(EdgeCfg<DP>::THREADS, CTAS)
 attn_bwd_edge_kernel(const AttnBwdParams p, const T* __restrict__ v, const T* __restrict__ out,
                      const float* __restrict__ lse, float* __restrict__ stats, const long long sv0,
                      const long long sv1, const long long sv2) {
@@ -1028,10 +1031,12 @@ template <typename T, int DP>
 static int launch_edge(const AttnBwdParams& p, const void* v, const void* out, const void* lse, void* stats,
                        const long long* sv, cudaStream_t st) {
   using C = EdgeCfg<DP>;
-  static bool done[64] = {};
-  const int r = set_smem(attn_bwd_edge_kernel<T, DP>, C::SMEM, done);
+  static bool done[2][64] = {};
+  const bool many = C::CTAS_MANY > C::CTAS && (long long)p.H * p.B > (long long)C::CTAS * attn_sm_count();
+  auto kern = many ? attn_bwd_edge_kernel<T, DP, C::CTAS_MANY> : attn_bwd_edge_kernel<T, DP, C::CTAS>;
+  const int r = set_smem(kern, C::SMEM, done[many]);
   if (r) return r;
-  after(attn_bwd_edge_kernel<T, DP>, dim3(p.H, p.B), C::THREADS, C::SMEM, st)(
+  after(kern, dim3(p.H, p.B), C::THREADS, C::SMEM, st)(
       p, (const T*)v, (const T*)out, (const float*)lse, (float*)stats, sv[0], sv[1], sv[2]);
   PF_CHECK_LAUNCH();
   return 0;

@@ -204,6 +204,12 @@ def test_attention_backward_of_whole_heads(dtype, B, H, Sq, Sk, D, causal):
     assert all(torch.equal(a, b) for a, b in zip(first, second))
 
 
+@pytest.mark.parametrize("B,H,S,D", [(23, 20, 129, 32), (30, 15, 258, 64)])
+def test_attention_backward_of_leftover_tokens_of_many_heads(B, H, S, D):
+    """More heads than three to an SM of 148, which take the form of fewer registers."""
+    test_attention_backward_of_whole_heads(torch.bfloat16, B, H, S, S, D, False)
+
+
 @pytest.mark.parametrize("D,left,causal", [(32, 1, False), (64, 3, True), (88, 4, False), (128, 1, True)])
 def test_attention_forward_of_leftover_rows(D, left, causal):
     """Rows beyond full tiles against 64 bits (u / 2 on average for rounding the result; the probabilities
