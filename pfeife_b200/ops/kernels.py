@@ -439,7 +439,8 @@ def rope_qkv(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, inverse: boo
     B, S, three, H, D = x.shape
     assert three == 3 and rope_qkv_supported(x, cos, sin)
     out = torch.empty_like(x)
-    fix = lambda t: t if t.is_contiguous() and t.data_ptr() % 16 == 0 else t.clone()
+    fix = lambda t: t if t.is_contiguous() and t.data_ptr() % 16 == 0 else \
+        t.clone(memory_format=torch.contiguous_format)
     check(L.pf_rope_qkv(x, out, fix(cos), fix(sin), B * S, S, H, D,
                         int(inverse), dt(x.dtype), stream_of(x)), "pf_rope_qkv")
     return out

@@ -148,6 +148,27 @@ def test_native_calls_equal_pythons(name, dtype, monkeypatch):
                 torch.testing.assert_close(a, b, rtol=2.0 ** -7 if a.dtype != torch.float32 else 1e-5, atol=1e-5)
 
 
+def _reversed(t):
+    """The same values with the dimensions the other way round in memory."""
+    order = tuple(reversed(range(t.dim())))
+    return t.permute(order).contiguous().permute(order)
+
+
+def _spread(t):
+    """The same values with a gap after each."""
+    return torch.stack([t, t + 1], dim=-1)[..., 0]
+
+
+def test_rotary_tables_in_any_order():
+    x, dy = _r(2, 20, 3, 4, 32).requires_grad_(), _r(2, 20, 3, 4, 32)
+    tables = ops.rope_tables(20, 32, device="cuda")
+    want = ops.rope_qkv(x, *tables)
+    for order in (_reversed, _spread, _strided, _shifted):
+        got = ops.rope_qkv(x, *map(order, tables))
+        assert torch.equal(got, want)
+        assert torch.equal(*(torch.autograd.grad(y, x, dy, retain_graph=True)[0] for y in (got, want)))
+
+
 def test_results_may_be_changed_in_place_and_inputs_may_not():
     x, w = _r(8, 64).requires_grad_(), _r(64, 64).requires_grad_()
     y = ops.linear(x * 1, w)
