@@ -88,6 +88,16 @@ def poll_status(device=None) -> None:
     ent["event"] = ev
 
 
+def _like(t: Optional[torch.Tensor], x: torch.Tensor) -> Optional[torch.Tensor]:
+    """`t` in x's type, as which a kernel reads both.  Hooks on saved tensors may have changed either."""
+    return t if t is None or t.dtype == x.dtype else t.to(x.dtype)
+
+
+def _floats(t: torch.Tensor) -> torch.Tensor:
+    """`t` as the packed fp32 values that a kernel reads."""
+    return (t if t.dtype == torch.float32 else t.float()).contiguous()
+
+
 def _split_workspace(L, M: int, N: int, K: int, accumulate: bool, conv: int, tile_n: int, device
                      ) -> Tuple[Optional[torch.Tensor], int]:
     """(workspace, KiB) in which the parts of a split reduction wait to be added in their order."""
@@ -171,7 +181,7 @@ def glu_fwd(gu: torch.Tensor, gelu: bool) -> torch.Tensor:
 def glu_bwd(gu: torch.Tensor, dout: torch.Tensor, gelu: bool) -> torch.Tensor:
     L = _lib.calls()
     gu = gu.contiguous()
-    dout = dout.contiguous()
+    dout = _like(dout, gu).contiguous()
     H = gu.shape[-1] // 2
     dgu = torch.empty_like(gu)
     rows = gu.numel() // (2 * H)
@@ -253,12 +263,13 @@ def norm_bwd(dy: torch.Tensor, h: torch.Tensor, gamma: torch.Tensor, mean: torch
              ) -> Tuple[torch.Tensor, torch.Tensor, Optional[torch.Tensor]]:
     L = _lib.calls()
     N = h.shape[-1]
+    dy, dres, mean, rstd = _like(dy, h), _like(dres, h), _floats(mean), _floats(rstd)
     dy2 = dy.contiguous().view(-1, N)
     h2 = h.contiguous().view(-1, N)
     rows = h2.shape[0]
     dres2 = dres.contiguous().view(-1, N) if dres is not None else None
     dx = torch.empty_like(h2)
-    g = gamma if gamma.dtype == torch.float32 else gamma.float()
+    g = _floats(gamma)
     if dgamma is None:
         dgamma = torch.empty(N, dtype=torch.float32, device=h.device)
         accumulate = False
@@ -342,8 +353,10 @@ def ce_fwd(logits: torch.Tensor, target: torch.Tensor, ignore_index: int = -100
 def ce_bwd(logits: torch.Tensor, target: torch.Tensor, lse: torch.Tensor,
            gscale: torch.Tensor, ignore_index: int = -100) -> torch.Tensor:
     L = _lib.calls()
+    assert target.dtype == torch.int64
     rows, V = logits.shape
     d = torch.empty_like(logits)
+    lse = _floats(lse)
     if rows > 1 and gscale.stride(0) != 0:       # one value for all rows may come as an expand
         gscale = gscale.contiguous()
     check(L.pf_ce_bwd(logits, target.contiguous(), lse, gscale, d,
@@ -456,6 +469,7 @@ def attention_supported(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> bo
 def _attn_ok(q, k, v) -> bool:
     D = q.shape[-1]
     return (q.dtype in (torch.float16, torch.bfloat16) and D % 8 == 0 and D <= 128
+            and k.dtype == q.dtype and v.dtype == q.dtype
             and q.stride(-1) == 1 and k.stride(-1) == 1 and v.stride(-1) == 1)
 
 
@@ -493,7 +507,7 @@ def attn_bwd(do: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor
     fix = lambda t: t if (t.stride(3) == 1 and t.data_ptr() % 16 == 0 and
                           all(s % 8 == 0 for s in t.stride()[:3])) else t.contiguous()
     q, k, v = fix(q), fix(k), fix(v)
-    do, o = do.contiguous(), o.contiguous()
+    do, o, lse = _like(do, q).contiguous(), _like(o, q).contiguous(), _floats(lse)
     if packed and Sq == Sk:
         if dqkv is None:
             dqkv = torch.empty((B, Sq, 3, H, D), dtype=q.dtype, device=q.device)
@@ -664,15 +678,16 @@ def groupnorm_fwd(x: torch.Tensor, gamma: torch.Tensor, beta: torch.Tensor, grou
 
 def groupnorm_bwd(dy, x, mean, rstd, gamma, beta, groups: int, silu: bool):
     L = _lib.calls()
-    x, dy = x.contiguous(), dy.contiguous()
+    x, dy = x.contiguous(), _like(dy, x).contiguous()
+    mean, rstd, gamma, beta = (_floats(t) for t in (mean, rstd, gamma, beta))
     B, H, W, C = x.shape
     dx = torch.empty_like(x)
     dgamma = torch.empty(C, dtype=torch.float32, device=x.device)
     dbeta = torch.empty(C, dtype=torch.float32, device=x.device)
     sums = torch.empty(2 * B * groups, dtype=torch.float32, device=x.device)
     scratch = _groupnorm_scratch(L, B, H * W, C, C + groups, x.device)
-    check(L.pf_groupnorm_bwd(dy, x, mean, rstd, gamma.float(),
-                             beta.float(), dx, dgamma, dbeta, sums,
+    check(L.pf_groupnorm_bwd(dy, x, mean, rstd, gamma,
+                             beta, dx, dgamma, dbeta, sums,
                              scratch, B, H * W, C, groups, int(silu), dt(x.dtype),
                              sm_count(x.device), stream_of(dy)), "pf_groupnorm_bwd")
     return dx, dgamma, dbeta

@@ -159,6 +159,51 @@ def _spread(t):
     return torch.stack([t, t + 1], dim=-1)[..., 0]
 
 
+def _wider(t):
+    return t.float() if t.dtype in DT.values() else t
+
+
+UNPACK = {"same": lambda t: t, "clone": lambda t: t.clone(), "reversed": _reversed,
+          "rows_apart": lambda t: _strided(t) if t.dim() > 1 else t, "spread": _spread, "wider": _wider,
+          "wider_images": lambda t: _wider(t) if t.dim() > 2 else t,
+          "double": lambda t: t.double() if t.dtype == torch.float32 else t}
+
+
+def _hooked(fn, leaves, how):
+    """(outputs, None), or (None, what was raised) under hooks that unpack `how`."""
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, UNPACK[how]):
+        try:
+            return _outputs(fn, leaves, set(range(len(leaves))))[1], None
+        except (AssertionError, RuntimeError) as e:
+            return None, type(e)
+
+
+def _agree(got, want):
+    for a, b in zip(got, want):
+        assert (a is None) == (b is None)
+        if a is not None:
+            assert a.dtype == b.dtype and a.shape == b.shape
+            # results of 8 bits, and probabilities of 8 bits where a formula in fp32 has more
+            assert (a.double() - b.double()).norm() <= 2.0 ** -7 * b.double().norm()
+
+
+@pytest.mark.parametrize("how", UNPACK)
+@pytest.mark.parametrize("name", list(_cases(torch.bfloat16)) if torch.cuda.is_available() else [])
+def test_what_the_formulas_in_python_unpack(name, how, monkeypatch):
+    """Hooks on saved tensors that return the same values in another order or type: the gradients of a call
+    without hooks.  Products refuse operands with gaps between a row's values, and a pre-activation and
+    logits of another type."""
+    torch.manual_seed(len(name))
+    fn, leaves = _cases(torch.bfloat16)[name]
+    monkeypatch.setattr(_lib, "_eager", None)
+    want = _outputs(fn, leaves, set(range(len(leaves))))[1]
+    got, error = _hooked(fn, leaves, how)
+    if error is None:
+        _agree(got, want)
+    else:
+        assert name.startswith(("linear", "mlp", "loss", "conv_1x1")) and how not in ("same", "clone", "rows_apart")
+
+
 def test_rotary_tables_in_any_order():
     x, dy = _r(2, 20, 3, 4, 32).requires_grad_(), _r(2, 20, 3, 4, 32)
     tables = ops.rope_tables(20, 32, device="cuda")
