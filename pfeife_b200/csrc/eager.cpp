@@ -11,7 +11,9 @@
 // that observes ops (dispatch or function modes, transforms, traces, forward-mode gradients).  For every
 // other call the functions return None, and the caller goes on in Python (ops/functional.py), which
 // defines what each op means.  A backward whose tensors are not plain any more, or that is itself
-// recorded, calls the registered backward op through the dispatcher, as the Python formulas do.
+// recorded, calls the registered backward op through the dispatcher, as the Python formulas do.  So does
+// one that unpacks something in another order or type than the forward saved: hooks on saved tensors may
+// return any tensor, and what the kernels assume of their operands is tested again in each backward.
 //
 // The kernel library is loaded by the caller beforehand with its symbols global.
 #include <ATen/autocast_mode.h>
@@ -117,6 +119,15 @@ bool direct(const Tensor& first, const T&... more) {
   return !at::GradMode::is_enabled() && unobserved() && all_plain(first, more...);
 }
 
+// fp32 values one after the other, as a forward kernel wrote them or as a caller's parameters are taken
+bool packed_floats(const Tensor& t, int64_t n) {
+  return t.scalar_type() == at::kFloat && t.numel() == n && t.is_contiguous();
+}
+// values of the type and sizes of `like`
+bool matches(const Tensor& t, const Tensor& like) {
+  return t.scalar_type() == like.scalar_type() && t.sizes() == like.sizes();
+}
+
 c10::IValue opt(const Tensor& t) { return t.defined() ? c10::IValue(t) : c10::IValue(); }
 
 // A registered op through the dispatcher.
@@ -128,7 +139,8 @@ Tensor given(const c10::IValue& v) {                // an empty tensor stands fo
   const Tensor& t = v.toTensor();
   return t.numel() ? t : Tensor();
 }
-Tensor as(const Tensor& t, at::ScalarType type) {
+Tensor as(const Tensor& t, const c10::IValue& saved) {       // in the type that a forward took down
+  const auto type = static_cast<at::ScalarType>(saved.toInt());
   return !t.defined() || t.scalar_type() == type ? t : t.to(type);
 }
 
@@ -214,6 +226,11 @@ std::pair<Tensor, Tensor> linear_forward(const Tensor& x, const Tensor& w, const
   const auto shape = with_last(x, w.size(0));
   return {y.view(shape), act ? aux.view(shape) : aux};
 }
+// whether linear_gradients can read what a backward unpacked, beside a gradient of the output
+bool gradients_fit(const Tensor& dz, const Tensor& x, const Tensor& w) {
+  return layer_fits(x, w, {}) && x.scalar_type() == dz.scalar_type() && dz.size(-1) == w.size(0) &&
+         x.numel() / x.size(-1) == dz.numel() / dz.size(-1);
+}
 // gradients of x, w, b from that of the pre-activation
 void linear_gradients(const Env& e, const Tensor& dz2, const Tensor& x, const Tensor& w, bool need_dx,
                       bool need_dw, bool need_db, Tensor& dx, Tensor& dw, Tensor& db) {
@@ -230,6 +247,7 @@ struct DirectLinear : torch::autograd::Function<DirectLinear> {
     ctx->set_materialize_grads(false);
     ctx->save_for_backward({x, w, b, aux});
     ctx->saved_data["act"] = act;
+    if (bias) ctx->saved_data["type"] = (int64_t)b.scalar_type();
     ctx->saved_data["res"] = res.defined();
     return y;
   }
@@ -243,13 +261,13 @@ struct DirectLinear : torch::autograd::Function<DirectLinear> {
                nb = b.defined() && ctx->needs_input_grad(2),
                nr = ctx->saved_data["res"].toBool() && ctx->needs_input_grad(2 + b.defined());
     Tensor dx, dw, db;
-    if (direct(dy, x, w, b, aux)) {
+    if (direct(dy, x, w, b, aux) && gradients_fit(dy, x, w) && (!act || matches(aux, dy))) {
       below([&] {
         const Env e(dy);
         Tensor dz = rows(dy);
         if (act) {
           constexpr int DACT[4] = {0, 10, 11, 12};                    // elementwise.cu
-          const Tensor z = rows(aux);
+          const Tensor z = rows(aux).contiguous();
           Tensor out = empty(dz.sizes(), dz);
           dz = dz.contiguous();
           ok(pf_elementwise(dz.data_ptr(), z.data_ptr(), out.data_ptr(), dz.numel(), DACT[act], code_of(dz),
@@ -265,7 +283,7 @@ struct DirectLinear : torch::autograd::Function<DirectLinear> {
                                                    (int64_t)act, nx, nw, nb, opt(b)});
       dx = given(out[0]); dw = given(out[1]); db = given(out[2]);
     }
-    return {nx ? dx : Tensor(), nw ? dw : Tensor(), nb ? as(db, b.scalar_type()) : Tensor(),
+    return {nx ? dx : Tensor(), nw ? dw : Tensor(), nb ? as(db, ctx->saved_data["type"]) : Tensor(),
             nr ? dy : Tensor(), Tensor()};
   }
 };
@@ -281,6 +299,8 @@ struct DirectMlp : torch::autograd::Function<DirectMlp> {
     ctx->set_materialize_grads(false);
     ctx->save_for_backward({x, w1, w2, z1, a1, b1, b2});
     ctx->saved_data["act"] = act;
+    if (bias1) ctx->saved_data["type1"] = (int64_t)b1.scalar_type();
+    if (bias2) ctx->saved_data["type2"] = (int64_t)b2.scalar_type();
     ctx->saved_data["res"] = res.defined();
     return y;
   }
@@ -294,7 +314,8 @@ struct DirectMlp : torch::autograd::Function<DirectMlp> {
                nr = ctx->saved_data["res"].toBool() &&
                     ctx->needs_input_grad(3 + b1.defined() + b2.defined());
     Tensor dx, dw1, db1, dw2, db2, none;
-    if (direct(dy, x, w1, w2, z1, a1, b1, b2)) {
+    if (direct(dy, x, w1, w2, z1, a1, b1, b2) && gradients_fit(dy, a1, w2) && gradients_fit(a1, x, w1) &&
+        matches(z1, a1)) {
       below([&] {
         const Env e(dy);
         const Tensor dy2 = rows(dy);
@@ -308,8 +329,8 @@ struct DirectMlp : torch::autograd::Function<DirectMlp> {
                                                 b2.defined(), opt(b1), opt(b2)});
       dx = given(out[0]); dw1 = given(out[1]); db1 = given(out[2]); dw2 = given(out[3]); db2 = given(out[4]);
     }
-    return {nx ? dx : Tensor(), dw1, b1.defined() ? as(db1, b1.scalar_type()) : Tensor(), dw2,
-            b2.defined() ? as(db2, b2.scalar_type()) : Tensor(), nr ? dy : Tensor(), Tensor()};
+    return {nx ? dx : Tensor(), dw1, b1.defined() ? as(db1, ctx->saved_data["type1"]) : Tensor(), dw2,
+            b2.defined() ? as(db2, ctx->saved_data["type2"]) : Tensor(), nr ? dy : Tensor(), Tensor()};
   }
 };
 
@@ -356,12 +377,15 @@ struct DirectNorm : torch::autograd::Function<DirectNorm> {
       dy = at::zeros_like(h);
     }
     dy = dy.contiguous();
+    const int64_t n = h.numel() / h.size(-1);
     Tensor dx, dg, db;
-    if (direct(dy, dh, h, gamma, beta, mean, rstd)) {
+    if (direct(dy, dh, h, gamma, beta, mean, rstd) && half(h) && matches(h, dy) &&
+        (!dh.defined() || matches(dh, dy)) && packed_floats(gamma, h.size(-1)) && packed_floats(mean, n) &&
+        packed_floats(rstd, n)) {
       below([&] {
         const Env e(dy);
         const Tensor hc = h.contiguous();
-        const int64_t N = h.size(-1), n = h.numel() / N;
+        const int64_t N = h.size(-1);
         dx = empty(h.sizes(), h);
         dg = floats(N, h);
         if (beta.defined() && !rms) db = floats(N, h);
@@ -429,6 +453,12 @@ std::pair<Tensor, Tensor> heads_forward(const Tensor& q, const Tensor& k, const 
                            q.size(2), q.size(3), causal, scale);
 }
 
+// whether a backward can read what it unpacked, beside a gradient of the output
+bool heads_fit(const Tensor& dout, const Tensor& o, const Tensor& lse) {
+  return half(dout) && matches(o, dout) &&
+         packed_floats(lse, dout.size(0) * dout.size(1) * dout.size(2));
+}
+
 struct DirectAttention : torch::autograd::Function<DirectAttention> {
   static Tensor forward(AutogradContext* ctx, Tensor q, Tensor k, Tensor v, bool causal, double scale) {
     at::AutoDispatchBelowADInplaceOrView guard;
@@ -447,7 +477,8 @@ struct DirectAttention : torch::autograd::Function<DirectAttention> {
     const bool causal = ctx->saved_data["causal"].toBool();
     const double scale = ctx->saved_data["scale"].toDouble();
     Tensor dq, dk, dv;
-    if (direct(dout, q, k, v, o, lse)) {
+    if (direct(dout, q, k, v, o, lse) && heads_fit(dout, o, lse) && matches(q, dout) &&
+        matches(k, v) && k.scalar_type() == q.scalar_type()) {
       below([&] {
         const Tensor qr = readable_heads(q), kr = readable_heads(k), vr = readable_heads(v);
         dq = empty(q.sizes(), q);
@@ -493,7 +524,8 @@ struct DirectAttentionQkv : torch::autograd::Function<DirectAttentionQkv> {
     const bool causal = ctx->saved_data["causal"].toBool();
     const double scale = ctx->saved_data["scale"].toDouble();
     Tensor d;
-    if (direct(dout, qkv, o, lse) && packed_fits(qkv)) {
+    if (direct(dout, qkv, o, lse) && heads_fit(dout, o, lse) && qkv.scalar_type() == dout.scalar_type() &&
+        qkv.dim() == 5 && qkv.numel() == 3 * dout.numel() && packed_fits(qkv)) {
       below([&] {
         d = empty(qkv.sizes(), qkv);
         attention_backward(aligned(dout) ? dout : dout.clone(), slice_of(qkv, 0), slice_of(qkv, 1),
@@ -517,6 +549,10 @@ Tensor rope_forward(const Tensor& x, const Tensor& cos, const Tensor& sin, bool 
      "pf_rope_qkv");
   return out;
 }
+bool table_fits(const Tensor& t, const Tensor& x) {  // of cosines or sines, for x [B, S, 3, H, D]
+  return t.scalar_type() == at::kFloat && t.dim() == 2 && t.is_contiguous() && aligned(t) &&
+         t.size(0) >= x.size(1) && t.size(1) == x.size(4) / 2;
+}
 struct DirectRopeQkv : torch::autograd::Function<DirectRopeQkv> {
   static Tensor forward(AutogradContext* ctx, Tensor x, Tensor cos, Tensor sin) {
     at::AutoDispatchBelowADInplaceOrView guard;
@@ -528,7 +564,8 @@ struct DirectRopeQkv : torch::autograd::Function<DirectRopeQkv> {
     const Tensor &cos = s[0], &sin = s[1];
     const Tensor dy = grads[0].contiguous();
     Tensor dx;
-    if (direct(dy, cos, sin) && aligned(dy)) below([&] { dx = rope_forward(dy, cos, sin, true); return 0; });
+    if (direct(dy, cos, sin) && half(dy) && aligned(dy) && table_fits(cos, dy) && table_fits(sin, dy))
+      below([&] { dx = rope_forward(dy, cos, sin, true); return 0; });
     else dx = dispatched("pfeife::rope_qkv_apply", {dy, cos, sin, true})[0].toTensor();
     return {dx, Tensor(), Tensor()};
   }
@@ -555,7 +592,8 @@ struct DirectGlu : torch::autograd::Function<DirectGlu> {
     const Tensor dy = grads[0].contiguous();
     const bool gelu = ctx->saved_data["gelu"].toBool();
     Tensor d;
-    if (direct(dy, gu) && gu.is_contiguous()) {
+    if (direct(dy, gu) && gu.is_contiguous() && half(gu) && gu.scalar_type() == dy.scalar_type() &&
+        gu.numel() == 2 * dy.numel()) {
       below([&] {
         const Env e(dy);
         const int64_t H = gu.size(-1) / 2;
@@ -607,7 +645,9 @@ struct DirectCrossEntropy : torch::autograd::Function<DirectCrossEntropy> {
     const int64_t ignore = ctx->saved_data["ignore"].toInt();
     const Tensor scale = g * inv;
     Tensor d;
-    if (direct(scale, logits, target, lse)) {
+    if (direct(scale, logits, target, lse) && logits.dim() == 2 &&
+        (half(logits) || logits.scalar_type() == at::kFloat) && target.scalar_type() == at::kLong &&
+        target.numel() == logits.size(0) && packed_floats(lse, logits.size(0)) && packed_floats(scale, 1)) {
       below([&] {
         const Env e(scale);
         const Tensor lc = logits.contiguous(), tc = target.contiguous();
@@ -661,12 +701,14 @@ struct DirectGroupNorm : torch::autograd::Function<DirectGroupNorm> {
     const Tensor dy = grads[0].contiguous();
     const int64_t groups = ctx->saved_data["groups"].toInt();
     const bool silu = ctx->saved_data["silu"].toBool();
+    const int64_t stats = dy.size(0) * groups, C = dy.size(3);
     Tensor dx, dg, db;
-    if (direct(dy, x, mean, rstd, gamma, beta)) {
+    if (direct(dy, x, mean, rstd, gamma, beta) && half(x) && matches(x, dy) && packed_floats(mean, stats) &&
+        packed_floats(rstd, stats) && packed_floats(gamma, C) && packed_floats(beta, C)) {
       below([&] {
         const Env e(dy);
         const Tensor xc = x.contiguous();
-        const int64_t B = x.size(0), C = x.size(3), HW = x.size(1) * x.size(2);
+        const int64_t B = x.size(0), HW = x.size(1) * x.size(2);
         dx = empty(x.sizes(), x);
         dg = floats(C, x);
         db = floats(C, x);
@@ -693,6 +735,9 @@ struct ConvShape {
   ConvShape(const Tensor& x, const Tensor& w, int64_t s, int64_t p)
       : B(x.size(0)), H(x.size(1)), W(x.size(2)), C(x.size(3)), N(w.size(0)), KH(w.size(2)), KW(w.size(3)),
         stride(s), pad(p), Ho((H + 2 * p - KH) / s + 1), Wo((W + 2 * p - KW) / s + 1) {}
+  bool output_fits(const Tensor& y) const {
+    return y.dim() == 4 && y.size(0) == B && y.size(1) == Ho && y.size(2) == Wo && y.size(3) == N;
+  }
   bool one() const { return KH == 1 && KW == 1 && stride == 1 && pad == 0; }
   bool forward_fits() const {
     return !one() && C % 64 == 0 && N % 8 == 0 && KH * KW <= 64 && Wo > 0 && Ho > 0 && Wo <= 128 &&
@@ -713,6 +758,11 @@ Tensor conv_pack(const Env& e, const Tensor& w, const ConvShape& s, bool flip) {
                   e.stream),
      "pf_conv_pack");
   return out;
+}
+// images that the implicit GEMM reads in place
+bool operands_fit(const Tensor& x, const Tensor& w) {
+  return x.dim() == 4 && w.dim() == 4 && half(x) && w.scalar_type() == x.scalar_type() &&
+         w.size(1) == x.size(3) && x.is_contiguous() && aligned(x);
 }
 Tensor conv_forward(const Tensor& x, const Tensor& w, const Tensor& b, int64_t stride, int64_t pad) {
   const Env e(x);
@@ -741,7 +791,8 @@ struct DirectConv2d : torch::autograd::Function<DirectConv2d> {
     const bool bias = ctx->saved_data["bias"].toBool();
     const bool nx = ctx->needs_input_grad(0), nw = ctx->needs_input_grad(1);
     Tensor dx, dw, db;
-    if (direct(dy, x, w)) {
+    if (direct(dy, x, w) && operands_fit(x, w) && x.scalar_type() == dy.scalar_type() &&
+        ConvShape(x, w, 1, pad).output_fits(dy)) {
       below([&] {
         const Env e(dy);
         const ConvShape s(x, w, 1, pad);
@@ -947,12 +998,8 @@ PF_OP(rope_qkv) {
   Args a(args, n, 3);
   if (PyErr_Occurred()) return nullptr;
   const Tensor x = a.tensor(0), cos = a.tensor(1), sin = a.tensor(2);
-  auto table = [&](const Tensor& t) {
-    return t.scalar_type() == at::kFloat && t.dim() == 2 && t.is_contiguous() && aligned(t) &&
-           t.size(0) >= x.size(1) && t.size(1) == x.size(4) / 2;
-  };
   if (!a.fits || !all_plain(x, cos, sin) || x.dim() != 5 || !half(x) || x.size(2) != 3 || x.size(4) % 16 ||
-      !x.is_contiguous() || !aligned(x) || !table(cos) || !table(sin))
+      !x.is_contiguous() || !aligned(x) || !table_fits(cos, x) || !table_fits(sin, x))
     Py_RETURN_NONE;
   if (!recorded(x, cos, sin))
     return run(x, [&] { return unrecorded([&] { return rope_forward(x, cos, sin, false); }); });
@@ -1014,9 +1061,8 @@ PF_OP(conv2d) {
   if (PyErr_Occurred()) return nullptr;
   const Tensor x = a.tensor(0), w = a.tensor(1), b = a.tensor(2, true);
   const int64_t stride = a.integer(3), pad = a.integer(4);
-  if (!a.fits || !all_plain(x, w, b) || x.dim() != 4 || w.dim() != 4 || !half(x) ||
-      w.scalar_type() != x.scalar_type() || w.size(1) != x.size(3) || !x.is_contiguous() || !aligned(x) ||
-      stride < 1 || pad < 0 || !ConvShape(x, w, stride, pad).forward_fits() ||
+  if (!a.fits || !all_plain(x, w, b) || !operands_fit(x, w) || stride < 1 || pad < 0 ||
+      !ConvShape(x, w, stride, pad).forward_fits() ||
       (b.defined() && (b.scalar_type() != at::kFloat || !bias_fits(b, w.size(0)))))
     Py_RETURN_NONE;
   if (!recorded(x, w, b))

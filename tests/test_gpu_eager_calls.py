@@ -204,6 +204,21 @@ def test_what_the_formulas_in_python_unpack(name, how, monkeypatch):
         assert name.startswith(("linear", "mlp", "loss", "conv_1x1")) and how not in ("same", "clone", "rows_apart")
 
 
+@pytest.mark.parametrize("how", UNPACK)
+@pytest.mark.parametrize("name", list(_cases(torch.bfloat16)) if torch.cuda.is_available() else [])
+def test_what_native_backwards_unpack(name, how, monkeypatch):
+    """The same of the nodes in C++, which raise what the formulas in Python raise."""
+    torch.manual_seed(len(name))
+    fn, leaves = _cases(torch.bfloat16)[name]
+    want = _outputs(fn, leaves, set(range(len(leaves))))[1]
+    got, error = _hooked(fn, leaves, how)
+    with monkeypatch.context() as m:
+        m.setattr(_lib, "_eager", None)
+        assert error == _hooked(fn, leaves, how)[1]
+    if error is None:
+        _agree(got, want)
+
+
 def test_rotary_tables_in_any_order():
     x, dy = _r(2, 20, 3, 4, 32).requires_grad_(), _r(2, 20, 3, 4, 32)
     tables = ops.rope_tables(20, 32, device="cuda")
