@@ -95,9 +95,13 @@ bool unobserved() {
 }
 
 // A tensor whose memory holds its values: no wrapper, negative view or the like (each is a dispatch key),
-// no forward-mode gradient, and not empty.
+// no forward-mode gradient, and not empty.  The usual keys are those of a tensor made outside inference mode,
+// in which tensors lack some of them, whatever the mode of the first call.
 bool plain(const Tensor& t, int dev) {
-  static const uint64_t usual = at::empty({0}, at::device(at::kCUDA).dtype(at::kHalf)).key_set().raw_repr();
+  static const uint64_t usual = [] {
+    const c10::InferenceMode off(false);
+    return at::empty({0}, at::device(at::kCUDA).dtype(at::kHalf)).key_set().raw_repr();
+  }();
   return (t.key_set().raw_repr() & ~usual) == 0 && t.get_device() == dev && t.data_ptr() != nullptr &&
          !t._fw_grad(0).defined();
 }

@@ -1,6 +1,9 @@
 """Eager calls that csrc/eager.cpp takes give what the Python implementations give, over the forms of
 arguments it accepts; what it does not accept goes on in Python."""
+import subprocess
+import sys
 import threading
+from pathlib import Path
 
 import pytest
 import torch
@@ -276,6 +279,33 @@ def test_refused_calls_raise_what_they_raised():
     y = ops.linear(x.requires_grad_(), w)
     with pytest.raises(_lib.KernelError):
         y.backward(_shifted(torch.ones_like(y)))
+
+
+FIRST_CALL = """
+import torch
+from pfeife_b200 import ops
+from pfeife_b200.ops import _lib
+x, w = (torch.randn(64, 64, device="cuda").bfloat16() for _ in range(2))
+seen = []
+def call(x):
+    ops.linear(x, w)
+    seen.append(_lib._eager.launches())
+with torch.inference_mode():
+    call(x)
+    call(x + 1)
+call(x)
+with torch.no_grad():
+    call(x.requires_grad_())
+y = ops.linear(x, w)
+y.sum().backward()
+assert seen == [1, 2, 3, 4] and _lib._eager.launches() > 5 and type(y.grad_fn).__name__ == "CppFunction", seen
+"""
+
+
+def test_the_first_call_may_be_in_inference_mode():
+    """In a process of its own: what a call learns of tensors does not depend on the mode it is made in."""
+    root = Path(__file__).resolve().parent.parent
+    subprocess.run([sys.executable, "-c", FIRST_CALL], cwd=root, check=True, timeout=300)
 
 
 def test_threads_and_streams():
