@@ -123,20 +123,23 @@ def calls():
 
 def eager():
     """Eager calls of the ops as a Python module (csrc/eager.cpp), or None: on a machine without CUDA, and
-    where the module was not built for this PyTorch from these sources (the calls then go through
-    Python, which takes them 20 us longer in each direction)."""
+    where the module was not built for this PyTorch from these sources, or these are not there to tell
+    (the calls then go through Python, which takes them 20 us longer in each direction)."""
     global _eager, _eager_tried
-    if not _eager_tried:
+    if not _eager_tried and lib() is not None:
         _eager_tried = True
-        if lib() is not None:
-            from ..csrc import build
-            path = build.eager_lib()
-            if path.exists():
-                module = _load("pfeife_b200_eager", path)
-                if module.SOURCES == build.eager_sources():
-                    from . import kernels
-                    module.setup(kernels.status_word, check)
-                    _eager = module
+        from ..csrc import build
+        path = build.eager_lib()
+        if path.exists():
+            try:
+                sources = build.eager_sources()
+            except FileNotFoundError:
+                return None
+            module = _load("pfeife_b200_eager", path)
+            if module.SOURCES == sources:
+                from . import kernels
+                module.setup(kernels.status_word, check)
+                _eager = module
     return _eager
 
 

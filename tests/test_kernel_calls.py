@@ -5,6 +5,7 @@ import ctypes
 import pytest
 import torch
 
+from pfeife_b200 import ops
 from pfeife_b200.csrc import build
 from pfeife_b200.ops import _lib
 
@@ -79,3 +80,40 @@ def test_the_module_is_optional(monkeypatch, tmp_path, capsys):
     monkeypatch.setattr(build, "_stale", lambda *a: False)
     build.build()
     assert not left.exists() and "ctypes" in capsys.readouterr().out
+
+
+@pytest.mark.parametrize("library", ["missing", "of_a_parent"])
+def test_calls_on_the_cpu_load_nothing(library, monkeypatch, tmp_path):
+    """Beside CUDA, whether the library is not built or the process was forked from one that holds CUDA."""
+    monkeypatch.setattr(torch.cuda, "is_available", lambda: True)
+    for name, value in (("_lib", None), ("_tried", False), ("_calls", None), ("_eager", None), ("_eager_tried", False)):
+        monkeypatch.setattr(_lib, name, value)
+    if library == "missing":
+        monkeypatch.setattr(_lib, "_KERNEL_LIB", tmp_path / "missing.so")
+    else:
+        monkeypatch.setattr(_lib, "_KERNEL_LIB", tmp_path)
+
+        def init():
+            raise RuntimeError("Cannot re-initialize CUDA in forked subprocess")
+        monkeypatch.setattr(torch.cuda, "init", init)
+    x, w, g = torch.randn(2, 16, 32, requires_grad=True), torch.randn(32, 32), torch.ones(32)
+    qkv, cos_sin = torch.randn(2, 8, 3, 2, 16), ops.rope_tables(8, 16)
+    image = torch.randn(1, 4, 4, 32)
+    for y in (ops.linear(x, w), ops.mlp(x, w, None, w, None), ops.layer_norm(x, g, g), ops.rms_norm(x, g),
+              ops.swiglu(x), ops.geglu(x), ops.cross_entropy(x[0], torch.zeros(16, dtype=torch.int64)),
+              ops.rope_qkv(qkv, *cos_sin), ops.attention_qkv(qkv), ops.attention(*qkv.unbind(2)),
+              ops.group_norm(image, g, g, 4), ops.conv2d(image, torch.randn(8, 32, 3, 3), padding=1)):
+        assert torch.isfinite(y).all()
+        if y.requires_grad:
+            y.sum().backward()
+    assert not _lib._tried and not _lib._eager_tried
+
+
+def test_eager_calls_without_their_sources(monkeypatch, tmp_path):
+    (tmp_path / "eager.so").write_bytes(b"")
+    monkeypatch.setattr(build, "eager_lib", lambda: tmp_path / "eager.so")
+    monkeypatch.setattr(build, "EAGER_SRC", tmp_path / "eager.cpp")
+    monkeypatch.setattr(_lib, "lib", lambda: object())
+    monkeypatch.setattr(_lib, "_eager", None)
+    monkeypatch.setattr(_lib, "_eager_tried", False)
+    assert _lib.eager() is None and _lib.eager() is None
