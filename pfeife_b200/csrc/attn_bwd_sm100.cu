@@ -247,7 +247,7 @@ attn_bwd_edge_kernel(const AttnBwdParams p, const T* __restrict__ v, const T* __
       fetch(trip + 1);
       cp_async_wait<1>();
       const int x = trip * GROUPS + grp;
-      const bool live = x < S;
+      const bool live = x < S;          // the others hold a copy of the last token and take no part
       const uint4* slot = ring + (trip & 1) * 5 * NV * THREADS;
       auto row = [&](int a, float (&to)[8 * NV]) {
 #pragma unroll
@@ -265,19 +265,23 @@ attn_bwd_edge_kernel(const AttnBwdParams p, const T* __restrict__ v, const T* __
       row(1, f);
       vec(0, w);
       const float s_r = over_lanes(dot(f, w));
-      const float p_r = live ? exp2f(fmaf(s_r, c2, nlse_r)) : 0.f;
+      const float p_r = exp2f(fmaf(s_r, c2, nlse_r));
       const float ds_r = p_r * (dp_r - delta_r) * p.scale;
+      if (live) {
 #pragma unroll
-      for (int j = 0; j < 8 * NV; ++j) dq[j] = fmaf(ds_r, f[j], dq[j]);
+        for (int j = 0; j < 8 * NV; ++j) dq[j] = fmaf(ds_r, f[j], dq[j]);
+      }
       row(0, f);
       vec(1, w);
       const float s_x = over_lanes(dot(f, w));
-      const float p_x = live ? exp2f(fmaf(s_x, c2, nlse_x)) : 0.f;
+      const float p_x = exp2f(fmaf(s_x, c2, nlse_x));
       const float ds_x = p_x * (dp_x - delta_x) * p.scale;
+      if (live) {
 #pragma unroll
-      for (int j = 0; j < 8 * NV; ++j) {
-        dk[j] = fmaf(ds_x, f[j], dk[j]);
-        dv[j] = fmaf(p_x, g[j], dv[j]);
+        for (int j = 0; j < 8 * NV; ++j) {
+          dk[j] = fmaf(ds_x, f[j], dk[j]);
+          dv[j] = fmaf(p_x, g[j], dv[j]);
+        }
       }
       if (sub == 0 && x < n) {
         e[x] = p_r;

@@ -140,21 +140,24 @@ attn_fwd_tail_kernel(const AttnParams p) {       // never a call's first launch
     }
     s += __shfl_xor_sync(0xffffffffu, s, 2);
     s += __shfl_xor_sync(0xffffffffu, s, 1);
-    s = trip * GROUPS + grp < keys ? s * c2 : -INFINITY;
-    if (s > m) {                                                       // also the first finite score
-      const float alpha = exp2f(m - s);
-      l *= alpha;
+    // Lanes beyond the last key hold a copy of it and take no part: no weight is small enough for an infinity.
+    if (trip * GROUPS + grp < keys) {
+      s *= c2;
+      if (s > m) {                                                     // also the first finite score
+        const float alpha = exp2f(m - s);
+        l *= alpha;
 #pragma unroll
-      for (int j = 0; j < 8 * NV; ++j) acc[j] *= alpha;
-      m = s;
-    }
-    const float w = s == -INFINITY ? 0.f : exp2f(s - m);               // a NaN stays one
-    l += w;
+        for (int j = 0; j < 8 * NV; ++j) acc[j] *= alpha;
+        m = s;
+      }
+      const float w = s == -INFINITY ? 0.f : exp2f(s - m);             // a NaN stays one
+      l += w;
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      widen(slot[(NV + i) * THREADS], f);
+      for (int i = 0; i < NV; ++i) {
+        widen(slot[(NV + i) * THREADS], f);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) acc[i * 8 + j] = fmaf(w, f[j], acc[i * 8 + j]);
+        for (int j = 0; j < 8; ++j) acc[i * 8 + j] = fmaf(w, f[j], acc[i * 8 + j]);
+      }
     }
   }
   cp_async_wait<0>();

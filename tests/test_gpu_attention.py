@@ -283,3 +283,27 @@ def ref_attn64(q, k, v, causal, scale):
         s = s.masked_fill(~torch.ones(s.shape[-2:], dtype=torch.bool, device="cuda").tril(
             k.shape[1] - q.shape[1]), float("-inf"))
     return torch.einsum("bhqk,bkhd->bqhd", s.softmax(-1), v), s.logsumexp(-1)
+
+
+@pytest.mark.parametrize("tokens,heads,dim", [(129, 3, 64), (129, 2, 128), (130, 2, 32), (257, 2, 88), (385, 1, 64)])
+def test_infinities_in_the_last_token(tokens, heads, dim):
+    """Leftover rows on CUDA cores: a token whose lane has none beside it is read there too, and must not count.
+    An infinity in its value reaches its own column of every row, and nothing else."""
+    from pfeife_b200 import ops
+
+    torch.manual_seed(tokens + dim)
+    q, k, v, do = (torch.randn(2, tokens, heads, dim, device="cuda").bfloat16() for _ in range(4))
+    inf_v, inf_do = v.clone(), do.clone()
+    inf_v[:, -1, :, 5] = float("inf")
+    inf_do[:, -1, :, 5] = float("-inf")
+
+    def run(v, do):
+        leaves = [t.detach().requires_grad_() for t in (q, k, v)]
+        o = ops.attention(*leaves)
+        return o.detach(), torch.autograd.grad(o, leaves, do)[2]
+
+    (o, dv), (inf_o, _), (_, inf_dv) = run(v, do), run(inf_v, do), run(v, inf_do)
+    other = [c for c in range(dim) if c != 5]
+    for got, finite, inf in ((inf_o, o, float("inf")), (inf_dv, dv, float("-inf"))):
+        assert (got[..., 5] == inf).all()
+        assert torch.equal(got[..., other], finite[..., other])
