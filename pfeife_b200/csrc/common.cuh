@@ -683,6 +683,13 @@ inline LaunchAfter<P...> after(void (*kernel)(P...), dim3 grid, dim3 block, size
   return {kernel, cfg};
 }
 
+// Whether operands that a kernel reads or writes 16 bytes at a time lie on 16 bytes (one that is left out
+// does): an access that does not is a fault which ends the context, so entry points refuse it (-2).
+template <typename... P>
+inline bool on_vectors(const P*... operands) {
+  return ((reinterpret_cast<uintptr_t>(operands) | ...) & 15) == 0;
+}
+
 #define PF_CHECK_LAUNCH()                            \
   do {                                               \
     cudaError_t e__ = cudaGetLastError();            \

@@ -646,7 +646,7 @@ using namespace pf;
 PF_API int pf_im2col(const void* x, void* cols, int B, int H, int W, int C, int KH, int KW, int Ho,
                      int Wo, int stride, int pad, long long ldc, int dtype, int sm_count,
                      void* stream) {
-  if (C % 8 || ldc % 8) return -2;
+  if (C % 8 || ldc % 8 || !on_vectors(x, cols)) return -2;
   const long long total = (long long)B * Ho * Wo * KH * KW * (C / 8);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   PF_DISPATCH_H(dtype, (after(im2col_kernel<T>, grid_for(total, sm_count), 256, 0, st)(
@@ -658,7 +658,7 @@ PF_API int pf_im2col(const void* x, void* cols, int B, int H, int W, int C, int 
 PF_API int pf_col2im(const void* dcols, void* dx, int B, int H, int W, int C, int KH, int KW,
                      int Ho, int Wo, int stride, int pad, long long ldc, int dtype, int sm_count,
                      void* stream) {
-  if (C % 8 || ldc % 8) return -2;
+  if (C % 8 || ldc % 8 || !on_vectors(dcols, dx)) return -2;
   const long long total = (long long)B * H * W * (C / 8);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   PF_DISPATCH_H(dtype, (after(col2im_kernel<T>, grid_for(total, sm_count), 256, 0, st)(
@@ -698,7 +698,7 @@ static int gn_launch(void (*kern)(P...), bool* done, dim3 grid, int threads, int
 PF_API int pf_groupnorm_fwd(const void* x, const void* gamma, const void* beta, void* y,
                             void* mean, void* rstd, void* scratch, int B, int HW, int C, int G,
                             float eps, int act_silu, int dtype, int sm_count, void* stream) {
-  if (C % G || C % 8) return -2;
+  if (C % G || C % 8 || !on_vectors(x, y)) return -2;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const int rows = gn_rows(C);
   const int threads = rows * (C / 8);
@@ -737,7 +737,7 @@ PF_API int pf_groupnorm_bwd(const void* dy, const void* x, const void* mean, con
                             const void* gamma, const void* beta, void* dx, void* dgamma,
                             void* dbeta, void* sums, void* scratch, int B, int HW, int C, int G,
                             int act_silu, int dtype, int sm_count, void* stream) {
-  if (C % G || C % 8) return -2;
+  if (C % G || C % 8 || !on_vectors(dy, x, dx)) return -2;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   float* sA = (float*)sums;
   float* sB = sA + (long long)B * G;
@@ -786,6 +786,7 @@ static inline int conv_share(int channels, int most) {
 PF_API int pf_conv_pack(const void* w, void* out, int Cout, int Cin, int taps, int cout8, int cin8,
                         int flip, void* stream) {
   if (taps < 1 || taps > CONV_PACK_TAPS || cout8 % 8 || cin8 % 8) return -3;
+  if (!on_vectors(out)) return -2;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const int vec = (reinterpret_cast<uintptr_t>(w) & 15) == 0 && (long long)Cin * taps % 8 == 0;
   if (!flip) {
@@ -807,7 +808,7 @@ PF_API int pf_conv_pack(const void* w, void* out, int Cout, int Cin, int taps, i
 PF_API int pf_conv_unpack(const void* src, void* dw, int Cout, int Cin, int taps, int cin8,
                           int dtype, void* stream) {
   if (taps < 1 || taps > CONV_PACK_TAPS || cin8 % 8) return -3;
-  if (reinterpret_cast<uintptr_t>(src) & 15) return -2;
+  if (!on_vectors(src)) return -2;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const int per = conv_share(cin8, CONV_TILE / (taps | 1) / 8 * 8);
   const dim3 grid(Cout, (Cin + per - 1) / per);
@@ -826,7 +827,7 @@ PF_API int pf_conv_unpack(const void* src, void* dw, int Cout, int Cin, int taps
 
 PF_API int pf_upsample2x(const void* x, void* y, int B, int H, int W, int C, int backward,
                          int dtype, int sm_count, void* stream) {
-  if (C % 8) return -2;
+  if (C % 8 || !on_vectors(x, y)) return -2;
   const long long total = (long long)B * H * W * (C / 8) * (backward ? 1 : 4);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   PF_DISPATCH_H(dtype, (after(upsample2x_kernel<T>, grid_for(total, sm_count), 256, 0, st)(

@@ -79,6 +79,11 @@ int code_of(at::ScalarType t) { return t == at::kFloat ? 0 : t == at::kHalf ? 1 
 int code_of(const Tensor& t) { return code_of(t.scalar_type()); }
 const void* at_or_null(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 bool aligned(const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0; }
+// packed values are read 16 bytes at a time; others are packed into memory of their own first
+template <typename... T>
+bool on_vectors(const T&... t) {
+  return ((!t.defined() || !t.is_contiguous() || aligned(t)) && ...);
+}
 bool half(const Tensor& t) { return t.scalar_type() == at::kHalf || t.scalar_type() == at::kBFloat16; }
 
 Tensor empty(at::IntArrayRef sizes, at::ScalarType type, const Tensor& like) {
@@ -384,7 +389,7 @@ struct DirectNorm : torch::autograd::Function<DirectNorm> {
     const int64_t n = h.numel() / h.size(-1);
     Tensor dx, dg, db;
     if (direct(dy, dh, h, gamma, beta, mean, rstd) && half(h) && matches(h, dy) &&
-        (!dh.defined() || matches(dh, dy)) && packed_floats(gamma, h.size(-1)) && packed_floats(mean, n) &&
+        (!dh.defined() || matches(dh, dy)) && on_vectors(dy, dh, h, gamma) && packed_floats(gamma, h.size(-1)) && packed_floats(mean, n) &&
         packed_floats(rstd, n)) {
       below([&] {
         const Env e(dy);
@@ -459,7 +464,7 @@ std::pair<Tensor, Tensor> heads_forward(const Tensor& q, const Tensor& k, const 
 
 // whether a backward can read what it unpacked, beside a gradient of the output
 bool heads_fit(const Tensor& dout, const Tensor& o, const Tensor& lse) {
-  return half(dout) && matches(o, dout) &&
+  return half(dout) && matches(o, dout) && on_vectors(o) &&
          packed_floats(lse, dout.size(0) * dout.size(1) * dout.size(2));
 }
 
@@ -597,7 +602,7 @@ struct DirectGlu : torch::autograd::Function<DirectGlu> {
     const bool gelu = ctx->saved_data["gelu"].toBool();
     Tensor d;
     if (direct(dy, gu) && gu.is_contiguous() && half(gu) && gu.scalar_type() == dy.scalar_type() &&
-        gu.numel() == 2 * dy.numel()) {
+        gu.numel() == 2 * dy.numel() && on_vectors(gu, dy)) {
       below([&] {
         const Env e(dy);
         const int64_t H = gu.size(-1) / 2;
@@ -708,7 +713,7 @@ struct DirectGroupNorm : torch::autograd::Function<DirectGroupNorm> {
     const int64_t stats = dy.size(0) * groups, C = dy.size(3);
     Tensor dx, dg, db;
     if (direct(dy, x, mean, rstd, gamma, beta) && half(x) && matches(x, dy) && packed_floats(mean, stats) &&
-        packed_floats(rstd, stats) && packed_floats(gamma, C) && packed_floats(beta, C)) {
+        packed_floats(rstd, stats) && packed_floats(gamma, C) && packed_floats(beta, C) && on_vectors(dy, x)) {
       below([&] {
         const Env e(dy);
         const Tensor xc = x.contiguous();
@@ -950,7 +955,7 @@ PF_OP(norm) {
                             t.is_contiguous());
   };
   if (!a.fits || !all_plain(x, g, b, r) || x.dim() < 1 || !half(x) || !vector(g) || !vector(b) ||
-      (r.defined() && (r.scalar_type() != x.scalar_type() || r.sizes() != x.sizes())))
+      !on_vectors(x, g, b, r) || (r.defined() && (r.scalar_type() != x.scalar_type() || r.sizes() != x.sizes())))
     Py_RETURN_NONE;
   if (!recorded(x, g, b, r))
     return run(x, [&]() -> variable_list {
@@ -1017,7 +1022,8 @@ PF_OP(glu) {
   if (PyErr_Occurred()) return nullptr;
   const Tensor gu = a.tensor(0);
   const bool gelu = a.boolean(1);
-  if (!a.fits || !all_plain(gu) || gu.dim() < 1 || !half(gu) || gu.size(-1) % 16 || !gu.is_contiguous())
+  if (!a.fits || !all_plain(gu) || gu.dim() < 1 || !half(gu) || gu.size(-1) % 16 || !gu.is_contiguous() ||
+      !on_vectors(gu))
     Py_RETURN_NONE;
   if (!recorded(gu)) return run(gu, [&] { return unrecorded([&] { return glu_forward(gu, gelu); }); });
   return run(gu, [&] { return DirectGlu::apply(gu, gelu); });
@@ -1051,7 +1057,7 @@ PF_OP(group_norm) {
     return t.scalar_type() == at::kFloat && t.dim() == 1 && t.size(0) == x.size(3) && t.is_contiguous();
   };
   if (!a.fits || !all_plain(x, g, b) || x.dim() != 4 || !half(x) || x.size(3) % 8 || x.size(3) > 8192 ||
-      groups <= 0 || x.size(3) % groups || !vector(g) || !vector(b))
+      groups <= 0 || x.size(3) % groups || !vector(g) || !vector(b) || !on_vectors(x))
     Py_RETURN_NONE;
   if (!recorded(x, g, b))
     return run(x, [&] { return unrecorded([&] { return group_norm_forward(x, g, b, groups, eps, silu).y; }); });

@@ -275,9 +275,7 @@ using namespace pf;
 PF_API int pf_elementwise(const void* a, const void* b, void* out, long long n, int op, int dtype,
                           int sm_count, void* stream) {
   if (n <= 0) return 0;
-  if ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) |
-       reinterpret_cast<uintptr_t>(out)) & 15)
-    return -2;
+  if (!on_vectors(a, b, out)) return -2;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   PF_DISPATCH_16_32(dtype, {
     const long long nvec = n / Vec16<T>::N + 1;
@@ -291,6 +289,7 @@ PF_API int pf_elementwise(const void* a, const void* b, void* out, long long n, 
 PF_API int pf_glu_fwd(const void* gu, void* out, long long rows, int H, int gelu, int dtype,
                       int sm_count, void* stream) {
   if (rows <= 0) return 0;
+  if (!on_vectors(gu, out)) return -2;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   PF_DISPATCH_16_32(dtype, {
     if (H % Vec16<T>::N) return -2;
@@ -305,6 +304,7 @@ PF_API int pf_glu_fwd(const void* gu, void* out, long long rows, int H, int gelu
 PF_API int pf_glu_bwd(const void* gu, const void* dout, void* dgu, long long rows, int H, int gelu,
                       int dtype, int sm_count, void* stream) {
   if (rows <= 0) return 0;
+  if (!on_vectors(gu, dout, dgu)) return -2;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   PF_DISPATCH_16_32(dtype, {
     if (H % Vec16<T>::N) return -2;

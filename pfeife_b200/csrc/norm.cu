@@ -731,6 +731,7 @@ PF_API int pf_norm_fwd(const void* x, const void* res, const void* gamma, const 
                        void* y, void* h_out, void* mean, void* rstd, long long rows, int N,
                        float eps, int rms, int dtype, void* stream) {
   if (rows <= 0) return 0;
+  if (!on_vectors(x, res, gamma, beta, y, h_out)) return -2;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   int r = -1;
   switch (dtype) {
@@ -757,6 +758,7 @@ PF_API int pf_norm_bwd(const void* dy, const void* h, const void* gamma, const v
                        void* scratch, long long rows, int N, int rms, int accumulate, int dtype,
                        int sm_count, void* stream) {
   if (rows <= 0) return 0;
+  if (!on_vectors(dy, h, gamma, dres, dx, scratch)) return -2;
   if (sm_count <= 0) sm_count = 148;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   int G = pf_norm_bwd_ctas(rows, sm_count);   // rows of scratch; the launch may use fewer

@@ -189,6 +189,7 @@ using namespace pf;
 
 PF_API int pf_nonfinite(const void* g, long long n, void* found_inf, int sm_count, void* stream) {
   if (n <= 0) return 0;
+  if (n >= 4 && !on_vectors(g)) return -2;
   nonfinite_kernel<<<opt_grid(n, sm_count), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
       (const float*)g, n, (float*)found_inf);
   PF_CHECK_LAUNCH();
@@ -200,6 +201,7 @@ PF_API int pf_adamw(void* p, void* g, void* m, void* v, void* lp, long long n,
                     float weight_decay, int step, const void* applied_steps, float grad_scale,
                     int adamw, int zero_grad, int lp_dtype, int sm_count, void* stream) {
   if (n <= 0) return 0;
+  if (n >= 4 && (!on_vectors(p, g, m, v) || (reinterpret_cast<uintptr_t>(lp) & 7))) return -2;
   AdamArgs a;
   a.lr = lr; a.beta1 = beta1; a.beta2 = beta2; a.eps = eps; a.weight_decay = weight_decay;
   a.step = step;

@@ -98,6 +98,12 @@ def _floats(t: torch.Tensor) -> torch.Tensor:
     return (t if t.dtype == torch.float32 else t.float()).contiguous()
 
 
+def _vectors(t: torch.Tensor) -> torch.Tensor:
+    """`t` packed and on 16 bytes, for a kernel that reads it so; a view into a buffer may be neither."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 def _split_workspace(L, M: int, N: int, K: int, accumulate: bool, conv: int, tile_n: int, device
                      ) -> Tuple[Optional[torch.Tensor], int]:
     """(workspace, KiB) in which the parts of a split reduction wait to be added in their order."""
@@ -169,7 +175,7 @@ def elementwise(op: int, a: torch.Tensor, b: Optional[torch.Tensor] = None,
 
 def glu_fwd(gu: torch.Tensor, gelu: bool) -> torch.Tensor:
     L = _lib.calls()
-    gu = gu.contiguous()
+    gu = _vectors(gu)
     H = gu.shape[-1] // 2
     out = torch.empty(gu.shape[:-1] + (H,), dtype=gu.dtype, device=gu.device)
     rows = gu.numel() // (2 * H)
@@ -180,8 +186,8 @@ def glu_fwd(gu: torch.Tensor, gelu: bool) -> torch.Tensor:
 
 def glu_bwd(gu: torch.Tensor, dout: torch.Tensor, gelu: bool) -> torch.Tensor:
     L = _lib.calls()
-    gu = gu.contiguous()
-    dout = _like(dout, gu).contiguous()
+    gu = _vectors(gu)
+    dout = _vectors(_like(dout, gu))
     H = gu.shape[-1] // 2
     dgu = torch.empty_like(gu)
     rows = gu.numel() // (2 * H)
@@ -236,15 +242,15 @@ def norm_fwd(x: torch.Tensor, gamma: torch.Tensor, beta: Optional[torch.Tensor],
     """Returns (y, h, mean, rstd); h = x + residual (h is x itself when residual is None)."""
     L = _lib.calls()
     N = x.shape[-1]
-    x2 = x.contiguous().view(-1, N)
+    x2 = _vectors(x).view(-1, N)
     rows = x2.shape[0]
     y = torch.empty_like(x2)
-    res2 = residual.contiguous().view(-1, N) if residual is not None else None
+    res2 = _vectors(residual).view(-1, N) if residual is not None else None
     h = torch.empty_like(x2) if residual is not None else x2
     mean = torch.empty(rows, dtype=torch.float32, device=x.device)
     rstd = torch.empty(rows, dtype=torch.float32, device=x.device)
-    g = gamma if gamma.dtype == torch.float32 else gamma.float()
-    b = None if beta is None else (beta if beta.dtype == torch.float32 else beta.float())
+    g = _vectors(_floats(gamma))
+    b = None if beta is None else _vectors(_floats(beta))
     check(L.pf_norm_fwd(x2, res2, g, b, y,
                         h if residual is not None else None, mean, rstd,
                         rows, N, eps, int(rms), dt(x.dtype), stream_of(x2)), "pf_norm_fwd")
@@ -264,12 +270,12 @@ def norm_bwd(dy: torch.Tensor, h: torch.Tensor, gamma: torch.Tensor, mean: torch
     L = _lib.calls()
     N = h.shape[-1]
     dy, dres, mean, rstd = _like(dy, h), _like(dres, h), _floats(mean), _floats(rstd)
-    dy2 = dy.contiguous().view(-1, N)
-    h2 = h.contiguous().view(-1, N)
+    dy2 = _vectors(dy).view(-1, N)
+    h2 = _vectors(h).view(-1, N)
     rows = h2.shape[0]
-    dres2 = dres.contiguous().view(-1, N) if dres is not None else None
+    dres2 = _vectors(dres).view(-1, N) if dres is not None else None
     dx = torch.empty_like(h2)
-    g = _floats(gamma)
+    g = _vectors(_floats(gamma))
     if dgamma is None:
         dgamma = torch.empty(N, dtype=torch.float32, device=h.device)
         accumulate = False
@@ -507,7 +513,7 @@ def attn_bwd(do: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor
     fix = lambda t: t if (t.stride(3) == 1 and t.data_ptr() % 16 == 0 and
                           all(s % 8 == 0 for s in t.stride()[:3])) else t.contiguous()
     q, k, v = fix(q), fix(k), fix(v)
-    do, o, lse = _like(do, q).contiguous(), _like(o, q).contiguous(), _floats(lse)
+    do, o, lse = _vectors(_like(do, q)), _vectors(_like(o, q)), _floats(lse)
     if packed and Sq == Sk:
         if dqkv is None:
             dqkv = torch.empty((B, Sq, 3, H, D), dtype=q.dtype, device=q.device)
@@ -537,7 +543,7 @@ def im2col(x: torch.Tensor, KH: int, KW: int, stride: int, pad: int) -> torch.Te
     Ho = (H + 2 * pad - KH) // stride + 1
     Wo = (W + 2 * pad - KW) // stride + 1
     cols = torch.empty((B * Ho * Wo, KH * KW * C), dtype=x.dtype, device=x.device)
-    check(L.pf_im2col(x.contiguous(), cols, B, H, W, C, KH, KW, Ho, Wo, stride, pad,
+    check(L.pf_im2col(_vectors(x), cols, B, H, W, C, KH, KW, Ho, Wo, stride, pad,
                       cols.stride(0), dt(x.dtype), sm_count(x.device), stream_of(cols)),
           "pf_im2col")
     return cols
@@ -664,13 +670,13 @@ def groupnorm_fwd(x: torch.Tensor, gamma: torch.Tensor, beta: torch.Tensor, grou
                   eps: float, silu: bool):
     """x NHWC [B, H, W, C] -> (y, mean[B*G], rstd[B*G])."""
     L = _lib.calls()
-    x = x.contiguous()
+    x = _vectors(x)
     B, H, W, C = x.shape
     y = torch.empty_like(x)
     mean = torch.empty(B * groups, dtype=torch.float32, device=x.device)
     rstd = torch.empty_like(mean)
     scratch = _groupnorm_scratch(L, B, H * W, C, groups, x.device)
-    check(L.pf_groupnorm_fwd(x, gamma.float(), beta.float(), y, mean,
+    check(L.pf_groupnorm_fwd(x, _floats(gamma), _floats(beta), y, mean,
                              rstd, scratch, B, H * W, C, groups, eps, int(silu),
                              dt(x.dtype), sm_count(x.device), stream_of(x)), "pf_groupnorm_fwd")
     return y, mean, rstd
@@ -678,7 +684,7 @@ def groupnorm_fwd(x: torch.Tensor, gamma: torch.Tensor, beta: torch.Tensor, grou
 
 def groupnorm_bwd(dy, x, mean, rstd, gamma, beta, groups: int, silu: bool):
     L = _lib.calls()
-    x, dy = x.contiguous(), _like(dy, x).contiguous()
+    x, dy = _vectors(x), _vectors(_like(dy, x))
     mean, rstd, gamma, beta = (_floats(t) for t in (mean, rstd, gamma, beta))
     B, H, W, C = x.shape
     dx = torch.empty_like(x)
@@ -695,7 +701,7 @@ def groupnorm_bwd(dy, x, mean, rstd, gamma, beta, groups: int, silu: bool):
 
 def upsample2x(x: torch.Tensor, backward: bool = False) -> torch.Tensor:
     L = _lib.calls()
-    x = x.contiguous()
+    x = _vectors(x)
     B, H, W, C = x.shape
     if backward:
         H, W = H // 2, W // 2

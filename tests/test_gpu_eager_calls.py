@@ -34,7 +34,7 @@ def _strided(t):
 
 
 def _shifted(t):
-    """The same values two bytes off a 16-byte boundary."""
+    """The same values one place off a 16-byte boundary."""
     buf = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)
     return buf[1:].copy_(t.reshape(-1)).view(t.shape)
 
@@ -88,6 +88,10 @@ def _cases(dt):
         "loss_3d": (lambda x: ops.cross_entropy(x, ids[:36].view(4, 9)), (_r(4, 9, 50, dtype=dt),)),
         "group_norm": (lambda x, g, b: ops.group_norm(x, g, b, 32, silu=True), (img, _f(64), _f(64))),
         "group_norm_strided": (lambda x, g, b: ops.group_norm(x.transpose(1, 2), g, b, 8), (img, _f(64), _f(64))),
+        "norm_shifted": (norm, (_shifted(x), _shifted(_f(64)), _shifted(_f(64)), _shifted(x + 1))),
+        "swiglu_shifted": (ops.swiglu, (_shifted(x),)),
+        "loss_shifted": (lambda x: ops.cross_entropy(x, ids), (_shifted(_r(37, 50, dtype=dt)),)),
+        "group_norm_shifted": (lambda x, g, b: ops.group_norm(x, g, b, 8), (_shifted(img), _shifted(_f(64)), _f(64))),
         "conv": (lambda x, w, b: ops.conv2d(x, w, b, 1, 1), (img, cw, _f(128))),
         "conv_no_bias": (lambda x, w: ops.conv2d(x, w, None, 1, 1), (img, cw)),
         "conv_5x5": (lambda x, w: ops.conv2d(x, w, None, 1, 2), (img, _r(128, 64, 5, 5, dtype=dt, scale=.1))),
@@ -101,7 +105,7 @@ def _cases(dt):
 
 
 PYTHON = {"linear_odd_width", "linear_odd_depth", "mlp_silu", "norm_half_gain", "rope_strided", "swiglu_strided",
-          "qkv_shifted", "loss_3d", "conv_stride", "conv_no_padding", "conv_1x1"}
+          "qkv_shifted", "norm_shifted", "swiglu_shifted", "group_norm_shifted", "loss_3d", "conv_stride", "conv_no_padding", "conv_1x1"}
 
 
 def _outputs(fn, leaves, needs):
@@ -167,6 +171,7 @@ def _wider(t):
 
 
 UNPACK = {"same": lambda t: t, "clone": lambda t: t.clone(), "reversed": _reversed,
+          "shifted": lambda t: _shifted(t) if t.dim() > 0 else t,
           "rows_apart": lambda t: _strided(t) if t.dim() > 1 else t, "spread": _spread, "wider": _wider,
           "wider_images": lambda t: _wider(t) if t.dim() > 2 else t,
           "double": lambda t: t.double() if t.dtype == torch.float32 else t}
@@ -203,6 +208,8 @@ def test_what_the_formulas_in_python_unpack(name, how, monkeypatch):
     got, error = _hooked(fn, leaves, how)
     if error is None:
         _agree(got, want)
+    elif how == "shifted":              # what TMA reads has to lie on 16 bytes
+        assert error is _lib.KernelError and name.startswith(("linear", "mlp", "conv", "attention"))
     else:
         assert name.startswith(("linear", "mlp", "loss", "conv_1x1")) and how not in ("same", "clone", "rows_apart")
 
@@ -220,6 +227,22 @@ def test_what_native_backwards_unpack(name, how, monkeypatch):
         assert error == _hooked(fn, leaves, how)[1]
     if error is None:
         _agree(got, want)
+
+
+@pytest.mark.parametrize("python", [False, True])
+@pytest.mark.parametrize("name", ["norm_residual", "rms", "norm_one_row", "swiglu", "geglu", "group_norm", "rope", "qkv",
+                                  "attention"])
+def test_gradients_off_their_vectors(name, python, monkeypatch):
+    """A gradient that is a view into a buffer, off the 16 bytes that the kernels read it by."""
+    fn, leaves = _cases(torch.bfloat16)[name]
+    if python:
+        monkeypatch.setattr(_lib, "_eager", None)
+    leaves = [t.detach().requires_grad_() for t in leaves]
+    out = fn(*leaves)
+    out = out if isinstance(out, tuple) else (out,)
+    dy = [torch.randn(o.shape, device="cuda").to(o.dtype) for o in out]
+    got, want = (torch.autograd.grad(out, leaves, g, retain_graph=True) for g in ([_shifted(t) for t in dy], dy))
+    _agree(got, want)
 
 
 def test_rotary_tables_in_any_order():

@@ -47,6 +47,38 @@ def test_values_arrive(calls):
     assert calls.pf_attn_fwd(*args) == -2
 
 
+VECTORS = {             # entry points that read and write 16 bytes at a time: arguments, and which of them are operands
+    "pf_norm_fwd": (lambda t: [t, t, t, t, t, t, None, None, 1, 64, 0.0, 0, 2, None], range(6)),
+    "pf_norm_bwd": (lambda t: [t, t, t, None, None, t, t, None, None, t, 1, 64, 0, 0, 2, 148, None], (0, 1, 2, 5, 6, 9)),
+    "pf_glu_fwd": (lambda t: [t, t, 1, 64, 0, 2, 148, None], range(2)),
+    "pf_glu_bwd": (lambda t: [t, t, t, 1, 64, 0, 2, 148, None], range(3)),
+    "pf_elementwise": (lambda t: [t, t, t, 64, 20, 2, 148, None], range(3)),
+    "pf_groupnorm_fwd": (lambda t: [t, None, None, t, None, None, None, 1, 1, 64, 8, 0.0, 0, 2, 148, None], (0, 3)),
+    "pf_groupnorm_bwd": (lambda t: [t, t, None, None, None, None, t, None, None, None, None, 1, 1, 64, 8, 0, 2, 148,
+                                    None], (0, 1, 6)),
+    "pf_im2col": (lambda t: [t, t, 1, 1, 1, 64, 1, 1, 1, 1, 1, 0, 64, 2, 148, None], range(2)),
+    "pf_col2im": (lambda t: [t, t, 1, 1, 1, 64, 1, 1, 1, 1, 1, 0, 64, 2, 148, None], range(2)),
+    "pf_upsample2x": (lambda t: [t, t, 1, 1, 1, 64, 0, 2, 148, None], range(2)),
+    "pf_conv_pack": (lambda t: [None, t, 8, 8, 1, 8, 8, 0, None], (1,)),
+    "pf_nonfinite": (lambda t: [t, 64, None, 148, None], (0,)),
+    "pf_adamw": (lambda t: [t, t, t, t, None, 64, None, None, 0.0, 0.0, 0.0, 0.0, 0.0, 1, None, 1.0, 1, 0, 0, 148, None],
+                 range(4)),
+}
+
+
+@pytest.mark.skipif(torch.cuda.is_available(), reason="where there is no device, what is not refused is not launched")
+@pytest.mark.parametrize("name", VECTORS)
+def test_operands_off_their_vectors_are_refused(calls, name):
+    arguments, operands = VECTORS[name]
+    aligned = torch.zeros(256)
+    assert aligned.data_ptr() % 16 == 0
+    for i in operands:
+        for off in (2, 4, 8, 14):
+            args = arguments(aligned.data_ptr())
+            args[i] += off
+            assert getattr(calls, name)(*args) == -2
+
+
 def test_what_does_not_fit_is_refused(calls):
     t = torch.zeros(64, 64, dtype=torch.bfloat16)
     with pytest.raises(TypeError):
