@@ -408,7 +408,7 @@ def mse_bwd(a: torch.Tensor, b: torch.Tensor, gout: torch.Tensor) -> torch.Tenso
 
 def embed_fwd(table: torch.Tensor, ids: torch.Tensor, out_dtype: torch.dtype) -> torch.Tensor:
     L = _lib.calls()
-    ids_c = ids.contiguous()
+    ids_c = ids.long().contiguous()
     D = table.shape[1]
     out = torch.empty(ids.shape + (D,), dtype=out_dtype, device=table.device)
     check(L.pf_embed_fwd(table, ids_c, out, ids_c.numel(), D,
@@ -421,7 +421,7 @@ def embed_bwd(dout: torch.Tensor, ids: torch.Tensor, dtable: torch.Tensor) -> to
     L = _lib.calls()
     assert dtable.dtype == torch.float32 and dtable.is_contiguous()
     dout = dout.contiguous()
-    ids_c = ids.contiguous()
+    ids_c = ids.long().contiguous()
     check(L.pf_embed_bwd(dout, ids_c, dtable, ids_c.numel(),
                          dtable.shape[1], dtable.shape[0], dt(dout.dtype), stream_of(dout)),
           "pf_embed_bwd")

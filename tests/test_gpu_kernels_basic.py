@@ -218,3 +218,17 @@ def test_mse_embedding_rope():
     assert torch.allclose(y.float(), ref, atol=2e-2, rtol=2e-2)
     back = kx.rope(y, cos, sin, inverse=True)
     assert torch.allclose(back.float(), xf, atol=4e-2, rtol=4e-2)
+
+
+def test_embedding_of_32_bit_ids():
+    """Ids of 32 bits give what those of 64 give, forward and backward."""
+    from pfeife_b200 import ops
+
+    torch.manual_seed(0)
+    table, ids = torch.randn(40, 24, device="cuda").requires_grad_(), torch.randint(0, 40, (3, 7), device="cuda")
+    dy = torch.randn(3, 7, 24, device="cuda")
+    for i in (ids.int(), ids.short(), ids.int().t().contiguous().t()):
+        y, want = ops.embedding(i, table, torch.float32), ops.embedding(ids, table, torch.float32)
+        assert torch.equal(y, want) and torch.equal(y, table[ids])
+        for a, b in zip(torch.autograd.grad(y, table, dy), torch.autograd.grad(want, table, dy)):
+            torch.testing.assert_close(a, b)        # sums by atomics
