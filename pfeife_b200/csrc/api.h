@@ -97,7 +97,6 @@ PF_DECL int pf_attn_fwd(const void* q, const void* k, const void* v, void* o, vo
                         void* stream);
 
 // ---- attn_bwd_sm100.cu
-PF_DECL int pf_attn_bwd_direct(int Sq, int Sk, int causal);
 PF_DECL int pf_attn_bwd_scratch(int B, int H, int Sq, int Sk, int D, int causal);
 PF_DECL int pf_attn_bwd(const void* dout, const void* q, const void* k, const void* v,
                         const void* out, const void* lse, void* stats, void* scratch, void* dq,

@@ -1085,8 +1085,6 @@ static BwdPlan bwd_plan(int B, int H, int Sq, int Sk, int D, int causal) {
 
 using namespace pf;
 
-PF_API int pf_attn_bwd_direct(int Sq, int Sk, int causal) { return bwd_direct(Sq, Sk, causal); }
-
 // KiB of scratch that pf_attn_bwd needs on the current device (0: none)
 PF_API int pf_attn_bwd_scratch(int B, int H, int Sq, int Sk, int D, int causal) {
   const BwdPlan g = bwd_plan(B, H, Sq, Sk, D, causal);

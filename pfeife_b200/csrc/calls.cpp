@@ -104,7 +104,7 @@ PyMethodDef methods[] = {
     PF_CALL(pf_adamw), PF_CALL(pf_step_advance), PF_CALL(pf_sgd), PF_CALL(pf_loss_scale_update),
     PF_CALL(pf_ce_fwd), PF_CALL(pf_ce_mean_parts), PF_CALL(pf_ce_mean), PF_CALL(pf_ce_bwd),
     PF_CALL(pf_mse_fwd), PF_CALL(pf_mse_bwd), PF_CALL(pf_embed_fwd), PF_CALL(pf_embed_bwd),
-    PF_CALL(pf_rope), PF_CALL(pf_rope_qkv), PF_CALL(pf_attn_fwd), PF_CALL(pf_attn_bwd_direct),
+    PF_CALL(pf_rope), PF_CALL(pf_rope_qkv), PF_CALL(pf_attn_fwd),
     PF_CALL(pf_attn_bwd_scratch), PF_CALL(pf_attn_bwd), PF_CALL(pf_im2col), PF_CALL(pf_col2im), PF_CALL(pf_groupnorm_slabs),
     PF_CALL(pf_groupnorm_fwd), PF_CALL(pf_groupnorm_bwd), PF_CALL(pf_upsample2x),
     PF_CALL(pf_conv_gemm), PF_CALL(pf_conv_wgrad), PF_CALL(pf_conv_pack), PF_CALL(pf_conv_unpack),

@@ -523,7 +523,7 @@ def attn_bwd(do: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor
         dq = torch.empty((B, Sq, H, D), dtype=q.dtype, device=q.device)
         dk = torch.empty((B, Sk, H, D), dtype=q.dtype, device=q.device)
         dv = torch.empty((B, Sk, H, D), dtype=q.dtype, device=q.device)
-    # row statistics per query tile and, unless one key tile holds every key, fp32 sums of dq
+    # row statistics per query tile; what the kernels need beside them depends on how they go about it
     stats = torch.empty((B, H, (Sq + 127) // 128, 256), dtype=torch.float32, device=q.device)
     stream = stream_of(do)               # binds the thread to the device that the next call asks
     kib = L.pf_attn_bwd_scratch(B, H, Sq, Sk, D, int(causal))

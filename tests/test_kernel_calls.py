@@ -32,8 +32,8 @@ def _gemm(calls, a, b, M=8, dtype=_lib.PF_BF16, lda=64, alpha=1.0):
 def test_values_arrive(calls):
     assert calls.pf_norm_bwd_ctas(1, 148) == 1
     assert calls.pf_norm_bwd_ctas(1 << 40, 148) == calls.pf_norm_bwd_ctas(1 << 20, 148) > 148
-    assert calls.pf_attn_bwd_direct(256, 128, False) == 1
-    assert calls.pf_attn_bwd_direct(256, 129, 0) == 0
+    assert calls.pf_gemm_workspace(320, 72, 65536, False, 0, 148, 0) > 0
+    assert calls.pf_gemm_workspace(320, 72, 65536, 1, 0, 148, 0) == 0
     t = torch.zeros(64, 64, dtype=torch.bfloat16)
     assert _gemm(calls, t, t, M=0) == 0
     assert _gemm(calls, t, t, dtype=7) == -1
