@@ -209,8 +209,8 @@ conv_unpack_kernel(const float* __restrict__ src, T* __restrict__ dw, int Cin, i
 static inline int gn_rows(int C) { const int ncv = C / 8; return ncv >= 256 ? 1 : 256 / ncv; }
 
 // Slabs of pixels per image, at least eight pixels per thread.  `per_sm` CTAs of up to 256 threads per
-// SM make one wave: 4 of the forward's at 56 registers, 3 of the backward's at 80 (4 left a third of
-// them to a second wave: 110 us against 83).
+// SM make one wave: 4 of the forward's, at 41 registers and at 64, which the bound of 1024 threads holds them to,
+// and 3 of the backward's at 80 (4 left a third of them to a second wave: 110 us against 83).
 constexpr int GN_FWD_PER_SM = 4, GN_BWD_PER_SM = 3;
 static inline int gn_slabs(int B, int HW, int rows, int sm_count, int per_sm) {
   int slabs = (per_sm * (sm_count > 0 ? sm_count : 148)) / B;
@@ -273,6 +273,7 @@ __device__ __forceinline__ void gn_fold(float* chan, const float (&a)[8], const 
   __syncthreads();
 }
 
+// 41 registers, without a bound on its CTAs: with one it comes out at 43 and 2 to 7 % slower.
 template <typename T>
 __global__ void gn_stats_kernel(const T* __restrict__ x, float* __restrict__ part, int HW, int C,
                                 int G, int rows) {
@@ -334,7 +335,7 @@ gn_finalize_kernel(const float* __restrict__ part, float* __restrict__ mean,
 // that waited for the stores before).
 constexpr int GN_AHEAD = 2;
 template <typename T, bool SILU>
-__global__ void gn_apply_kernel(const T* __restrict__ x, const float* __restrict__ mean,
+__global__ void __launch_bounds__(1024) gn_apply_kernel(const T* __restrict__ x, const float* __restrict__ mean,
                                 const float* __restrict__ rstd, const float* __restrict__ gamma,
                                 const float* __restrict__ beta, T* __restrict__ y, int HW, int C,
                                 int G, int rows) {
