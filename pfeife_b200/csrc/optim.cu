@@ -162,18 +162,25 @@ __global__ void loss_scale_update_kernel(float* state, float* found_inf, float g
   }
 }
 
-// CTAs of an update: more than are resident, so that the addresses in flight in the eight streams stay close
-// together as CTAs end and begin, but with some eight vectors per thread under their set-up, and no fewer
-// than twice those resident.  AdamW over 64 Mi parameters, cold and after seconds of it: resident CTAs
-// striding over everything 383 and 378 us, a CTA per 256 vectors 350 and 391, this 351 and 355 (a plain
-// copy of as many bytes takes 348); over 5 Mi 34.4, 33.2 and 33.1 cold, 33.9, 35.7 and 34.1 warm.
-static inline unsigned update_grid(long long n, int sm_count) {
-  const long long sms = sm_count > 0 ? sm_count : 148, blocks = (n / 4 + 255) / 256;
-  long long b = blocks / 8;
-  if (b > 64 * sms) b = 64 * sms;
-  if (b < 16 * sms) b = 16 * sms;
-  if (b > blocks) b = blocks;
-  return (unsigned)(b < 1 ? 1 : b);
+// CTAs of an update: eight per SM that stride over everything or, for large ones, more than are resident with
+// seven or eight vectors per thread under their set-up, so that the addresses in flight in the seven or eight
+// streams stay close together as CTAs end and begin.  SGD has all eight on an SM at 32 registers: a last round of
+// them that is nearly empty is felt, so it takes whole rounds (20 Mi 127 us without, 113 so).  AdamW has
+// five at 48 registers and takes twice the eight before it takes more.  us, on buffers that change from call
+// to call, with eight per SM and so: AdamW 2.5 M 18.6 both (20.1 with 16 per SM), 10 Mi 61.7 both, 20 Mi 119.6 and
+// 118.9, 40 Mi 236.9 and 225.9, 64 Mi 387 and 365, 128 Mi 771 and 708; SGD 10 Mi 57.6 both, 20 Mi 115 and 113,
+// 40 Mi 231 and 219, 64 Mi 373 and 346.
+static inline unsigned grid_of(long long ctas, long long blocks) {
+  return (unsigned)(blocks < 1 ? 1 : ctas < blocks ? ctas : blocks);
+}
+static inline unsigned adamw_grid(long long n, int sm_count) {
+  const long long sms = sm_count > 0 ? sm_count : 148, blocks = (n / 4 + 255) / 256, b = blocks / 8;
+  return grid_of(b < 16 * sms ? 8 * sms : b > 64 * sms ? 64 * sms : b, blocks);
+}
+static inline unsigned sgd_grid(long long n, int sm_count) {
+  const long long round = 8ll * (sm_count > 0 ? sm_count : 148), blocks = (n / 4 + 255) / 256;
+  const long long rounds = (blocks / 7 + round / 2) / round;
+  return grid_of((rounds < 1 ? 1 : rounds > 8 ? 8 : rounds) * round, blocks);
 }
 static inline int opt_grid(long long n, int sm_count) {
   long long b = (n / 4 + 255) / 256;
@@ -206,7 +213,7 @@ PF_API int pf_adamw(void* p, void* g, void* m, void* v, void* lp, long long n,
   a.lr = lr; a.beta1 = beta1; a.beta2 = beta2; a.eps = eps; a.weight_decay = weight_decay;
   a.step = step;
   a.grad_scale = grad_scale; a.adamw = adamw; a.zero_grad = zero_grad; a.lp_dtype = lp_dtype;
-  adamw_kernel<<<update_grid(n, sm_count), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+  adamw_kernel<<<adamw_grid(n, sm_count), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
       (float*)p, (float*)g, (float*)m, (float*)v, lp, n, (const float*)found_inf,
       (const float*)loss_scale, (const int*)applied_steps, a);
   PF_CHECK_LAUNCH();
@@ -225,7 +232,7 @@ PF_API int pf_sgd(void* p, void* g, void* mom, void* lp, long long n, const void
                   int first_step, float grad_scale, int zero_grad, int lp_dtype, int sm_count,
                   void* stream) {
   if (n <= 0) return 0;
-  sgd_kernel<<<update_grid(n, sm_count), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+  sgd_kernel<<<sgd_grid(n, sm_count), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
       (float*)p, (float*)g, (float*)mom, lp, n, (const float*)found_inf, lr, momentum, dampening,
       weight_decay, nesterov, first_step, grad_scale, zero_grad, lp_dtype,
       (const float*)loss_scale);
