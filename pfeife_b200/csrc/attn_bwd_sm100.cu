@@ -48,6 +48,7 @@
 // beyond the last query, which makes the probabilities there zero without a test) and clears the fp32
 // dQ sums; a post-pass converts them.  With one key tile the dQ tiles are complete and go straight to
 // their 16-bit destination: no sums, no post-pass.
+#include <climits>
 #include <type_traits>
 #include "attn_common.cuh"
 #include "api.h"
@@ -1055,26 +1056,64 @@ struct BwdPlan {
   int mode, left, n_kt, n_qt;
   long long part, edge;               // floats of scratch: dQ so far (or the fp32 sums), leftover weights
 };
-// Heads are taken whole where that takes no more rounds of key tiles than dealing the key tiles one by one.
-// The leftover token then saves a key tile and a query tile per head; each costs a pass over the head (some
-// 15 us per 200 heads of 257 tokens up to head dim 64, twice that above).  [12, 258, 25, 64] 87 us in tiles
-// and 83 so, [12, 260, 25, 64] 86 and 121; [24, 257, 16, 88] 123 and 107, [24, 258, 16, 88] 125 and 147.
+// Heads are taken whole where that takes no more rounds of key tiles than dealing the key tiles one by one, and
+// while a head's sums of dQ (512 bytes per query tile and column) are small: a CTA reads and writes them once
+// per key tile, and past 200 KB, or 320 with two key tiles, that costs more than adding in memory.  us, dealt and
+// whole, 144 heads: head dim 64, 256 tokens 25.8 21.8, 768 99.9 99.8, 1024 156 176, 1024 queries of 200 keys 1.17
+// times as fast whole; head dim 128, 256 tokens 37.5 32.3, 384 59.8 58.9, 512 86.8 101, 1024 243 409.
+// Under a causal mask a head visits half the pairs of tiles and whole heads gain for longer (head dim 128, 294
+// heads of 512 168 126, of 1024 1.07 times), but dealing, longest first, fills a single round better (head dim
+// 128, 144 heads of 640 1.05 times, of 768 0.98; head dim 32, 132 heads of 898 0.95), and a last tile of a few
+// rows costs it next to nothing (head dim 88, 432 heads of 898 0.92, of 1024 1.03).
+static bool whole_pays(int causal, int dp, int Sq, int n_kt, long long heads, long long sms) {
+  const long long rounds = (heads + sms - 1) / sms, apart = (heads * n_kt + sms - 1) / sms;
+  const int n_qt = (Sq + ATT_BM - 1) / ATT_BM, size = n_qt * dp;
+  if (n_qt > BWD_WHOLE_TILES || rounds * n_kt > apart) return false;
+  if (!causal)
+    return size <= (n_kt == 2 ? 640 : n_kt == 3 && dp <= 96 ? 512 : n_kt <= 4 || dp <= 96 ? 384 : 256);
+  const bool few_rows = Sq % ATT_BM > 0 && Sq % ATT_BM <= 32;
+  if (rounds == 1) return size <= (few_rows ? 512 : 640) && (n_qt <= 6 || 20 * heads >= 19 * sms);
+  return dp <= 64 || !few_rows || size <= 640;
+}
+// Whether the leftover tokens are taken out of the tiles, which saves a key tile and a query tile per head and
+// costs a pass over the head per token.  `rounds` are of heads, of n_kt key tiles without the leftovers.  The pass
+// takes the place of the one that clears and of the one that converts, so that one token pays without a saved
+// round up to head dim 64, and for a fifth of the rounds at 96 and a quarter at 128; two tokens pay for nearly
+// half of them at head dim 64, or for a quarter where the tiles cannot be taken whole, and want several rounds of
+// heads over which the pass spreads.  us, dealt, whole and so: [10, 257, 16, 64] 46.9 54.1 42.5, [24, 257, 16, 88]
+// 114.7 113.7 103.4, [10, 257, 16, 88] 60.1 73.6 67.7, [24, 257, 16, 128] 129.5 127.4 130.1, [3, 129, 19, 64] 13.2
+// 15.0 14.4, [3, 130, 19, 64] 13.3 15.1 20.0, [24, 258, 16, 64] 90.8 87.2 86.0, [16, 386, 19, 32] 106 111 92.5.
+static bool leftover_pays(int left, int dp, int n_qt, int n_kt, long long rounds, long long apart) {
+  const long long r = rounds * n_kt;
+  if (n_qt > BWD_WHOLE_TILES || n_qt * dp > 384) return false;
+  if (left == 1) {
+    const int percent = dp <= 64 ? 100 : dp <= 96 ? 122 : 133;
+    return r * percent <= apart * 100 && (r < apart || n_kt > 1);
+  }
+  if (dp <= 32) return r < apart || (r == apart && rounds > 1);
+  return rounds > 1 && (8 * r <= 5 * apart || (n_kt > 1 && 4 * r <= 3 * apart && rounds * (n_kt + 1) > apart));
+}
 static BwdPlan bwd_plan(int B, int H, int Sq, int Sk, int D, int causal) {
   const long long heads = (long long)B * H, sms = attn_sm_count();
   auto tiles = [](int n) { return (n + ATT_BN - 1) / ATT_BN; };
   BwdPlan g = {bwd_direct(Sq, Sk, causal) ? DQ_DIRECT : DQ_SUMS, 0, tiles(Sk), tiles(Sq), 0, 0};
-  const int left = Sq % ATT_BM, left_max = D > 64 ? 1 : BWD_LEFT_MAX;
-  const bool edge = !causal && Sq == Sk && Sq > ATT_BM && left > 0 && left <= left_max;
-  const int n_kt = edge ? g.n_kt - 1 : g.n_kt, n_qt = edge ? g.n_qt - 1 : g.n_qt;
-  const long long whole = (heads + sms - 1) / sms * n_kt, apart = (heads * g.n_kt + sms - 1) / sms;
-  if (g.mode == DQ_SUMS && n_qt <= BWD_WHOLE_TILES && (!causal || Sk >= Sq) && whole <= apart) {
-    g.mode = DQ_WHOLE;
-    g.left = edge ? left : 0;
-    g.n_kt = n_kt;
-    g.n_qt = n_qt;
-    const int dp = (D + 31) / 32 * 32;
-    g.part = (heads < sms ? heads : sms) * n_qt * ATT_BM * dp;
-    g.edge = heads * g.left * 3 * n_qt * ATT_BM;
+  const int dp = (D + 31) / 32 * 32;
+  const long long rounds = (heads + sms - 1) / sms, apart = (heads * g.n_kt + sms - 1) / sms;
+  if (g.mode == DQ_SUMS && (!causal || Sk >= Sq)) {
+    const int left = !causal && Sq == Sk && Sq > ATT_BM ? Sq % ATT_BM : 0;
+    if (left > 0 && left <= (D > 64 ? 1 : BWD_LEFT_MAX) &&
+        leftover_pays(left, dp, g.n_qt - 1, g.n_kt - 1, rounds, apart)) {
+      g.mode = DQ_WHOLE;
+      g.left = left;
+      --g.n_kt;
+      --g.n_qt;
+    } else if (whole_pays(causal, dp, Sq, g.n_kt, heads, sms)) {
+      g.mode = DQ_WHOLE;
+    }
+  }
+  if (g.mode == DQ_WHOLE) {
+    g.part = (heads < sms ? heads : sms) * g.n_qt * ATT_BM * dp;
+    g.edge = heads * g.left * 3 * g.n_qt * ATT_BM;
   } else if (g.mode == DQ_SUMS) {
     g.part = heads * Sq * D;
   }

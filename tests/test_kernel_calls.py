@@ -79,6 +79,39 @@ def test_operands_off_their_vectors_are_refused(calls, name):
             assert getattr(calls, name)(*args) == -2
 
 
+DEALT, WHOLE, LEFTOVER = "key tiles dealt", "whole heads", "leftover tokens beside them"
+
+
+@pytest.mark.skipif(torch.cuda.is_available(), reason="the plan is asked for 148 SMs, as where there is no device")
+@pytest.mark.parametrize("heads,queries,keys,dim,causal,route", [
+    # whole heads while they cost no round, and while their sums are small
+    (144, 250, 250, 64, 0, WHOLE), (150, 250, 250, 64, 0, DEALT), (8, 250, 250, 64, 0, DEALT), (57, 257, 257, 88, 0, DEALT),
+    (144, 760, 760, 64, 0, WHOLE), (144, 890, 890, 64, 0, DEALT), (144, 1020, 300, 64, 0, WHOLE),
+    (144, 1020, 512, 64, 0, DEALT), (144, 380, 380, 128, 0, WHOLE), (144, 510, 510, 128, 0, DEALT),
+    (144, 1020, 1020, 32, 0, WHOLE), (144, 1100, 1100, 32, 0, DEALT),
+    (144, 630, 630, 128, 1, WHOLE), (144, 760, 760, 128, 1, DEALT), (294, 1020, 1020, 128, 1, WHOLE),
+    (144, 300, 256, 64, 1, DEALT),
+    (144, 630, 200, 128, 0, WHOLE), (144, 760, 200, 128, 0, DEALT), (144, 500, 380, 88, 0, WHOLE), (144, 630, 380, 88, 0, WHOLE),
+    (144, 630, 500, 88, 0, DEALT), (144, 380, 630, 88, 0, WHOLE), (144, 380, 630, 128, 0, DEALT), (144, 250, 630, 128, 0, WHOLE),
+    (132, 898, 898, 32, 1, DEALT), (144, 898, 898, 32, 1, WHOLE), (144, 642, 642, 88, 1, DEALT), (294, 898, 898, 88, 1, DEALT),
+    (294, 898, 898, 64, 1, WHOLE), (294, 642, 642, 88, 1, WHOLE),
+    # leftover tokens where that saves what it costs
+    (160, 257, 257, 64, 0, LEFTOVER), (96, 129, 129, 64, 0, LEFTOVER), (57, 129, 129, 64, 0, DEALT), (57, 257, 257, 64, 0, LEFTOVER),
+    (384, 257, 257, 88, 0, LEFTOVER), (160, 257, 257, 88, 0, DEALT), (140, 257, 257, 128, 0, LEFTOVER),
+    (304, 257, 257, 128, 0, DEALT), (144, 1025, 1025, 64, 0, DEALT),
+    (96, 130, 130, 64, 0, WHOLE), (304, 130, 130, 64, 0, LEFTOVER), (160, 130, 130, 64, 0, DEALT), (384, 258, 258, 64, 0, LEFTOVER),
+    (294, 258, 258, 64, 0, WHOLE), (96, 130, 130, 32, 0, LEFTOVER), (57, 258, 258, 32, 0, DEALT), (304, 386, 386, 32, 0, LEFTOVER),
+    (384, 259, 259, 64, 0, DEALT), (384, 258, 258, 88, 0, DEALT)])
+def test_the_plan_of_the_attention_backward(calls, heads, queries, keys, dim, causal, route):
+    """Which way a call goes, by the scratch that it asks for: the lines were measured from both sides."""
+    tiles, columns, left = (queries + 127) // 128, (dim + 31) // 32 * 32, queries % 128
+    full = queries // 128
+    sizes = {DEALT: heads * queries * dim, WHOLE: min(heads, 148) * tiles * 128 * columns,
+              LEFTOVER: min(heads, 148) * full * 128 * columns + heads * left * 3 * full * 128}
+    assert len(set(sizes.values())) == 3
+    assert calls.pf_attn_bwd_scratch(1, heads, queries, keys, dim, causal) == (sizes[route] + 255) // 256
+
+
 def test_what_does_not_fit_is_refused(calls):
     t = torch.zeros(64, 64, dtype=torch.bfloat16)
     with pytest.raises(TypeError):
