@@ -130,7 +130,13 @@ attn_fwd_tail_kernel(const AttnParams p) {       // never a call's first launch
   for (int trip = 0; trip < trips; ++trip) {
     fetch(trip + DEPTH - 1);
     cp_async_wait<DEPTH - 1>();
-    const uint4* slot = ring + (trip % DEPTH) * 2 * NV * THREADS;
+    uint4* slot = ring + (trip % DEPTH) * 2 * NV * THREADS;
+    // Beyond the last key lies a copy of its value, which a weight of zero does not take out if it is infinite.
+    const bool live = trip * GROUPS + grp < keys;
+    if (!live) {
+#pragma unroll
+      for (int i = 0; i < NV; ++i) slot[(NV + i) * THREADS] = make_uint4(0, 0, 0, 0);
+    }
     float f[8], s = 0.f;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
@@ -140,24 +146,21 @@ attn_fwd_tail_kernel(const AttnParams p) {       // never a call's first launch
     }
     s += __shfl_xor_sync(0xffffffffu, s, 2);
     s += __shfl_xor_sync(0xffffffffu, s, 1);
-    // Lanes beyond the last key hold a copy of it and take no part: no weight is small enough for an infinity.
-    if (trip * GROUPS + grp < keys) {
-      s *= c2;
-      if (s > m) {                                                     // also the first finite score
-        const float alpha = exp2f(m - s);
-        l *= alpha;
+    s = live ? s * c2 : -INFINITY;
+    if (s > m) {                                                       // also the first finite score
+      const float alpha = exp2f(m - s);
+      l *= alpha;
 #pragma unroll
-        for (int j = 0; j < 8 * NV; ++j) acc[j] *= alpha;
-        m = s;
-      }
-      const float w = s == -INFINITY ? 0.f : exp2f(s - m);             // a NaN stays one
-      l += w;
+      for (int j = 0; j < 8 * NV; ++j) acc[j] *= alpha;
+      m = s;
+    }
+    const float w = s == -INFINITY ? 0.f : exp2f(s - m);               // a NaN stays one
+    l += w;
 #pragma unroll
-      for (int i = 0; i < NV; ++i) {
-        widen(slot[(NV + i) * THREADS], f);
+    for (int i = 0; i < NV; ++i) {
+      widen(slot[(NV + i) * THREADS], f);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i * 8 + j] = fmaf(w, f[j], acc[i * 8 + j]);
-      }
+      for (int j = 0; j < 8; ++j) acc[i * 8 + j] = fmaf(w, f[j], acc[i * 8 + j]);
     }
   }
   cp_async_wait<0>();
