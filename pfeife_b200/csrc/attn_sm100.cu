@@ -330,7 +330,7 @@ __device__ __forceinline__ float probs(const uint32_t (&s)[4][32], uint32_t t_p,
   return (a + b) + (d + e);
 }
 
-template <typename T, int DP, bool SPLIT>
+template <typename T, int DP, bool SPLIT, bool ONE_ISSUER>
 __global__ void __launch_bounds__(FwdCfg<DP>::THREADS, 1)
 attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                    const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap to,
@@ -338,11 +338,11 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
   using C = FwdCfg<DP>;
   constexpr int NBLK = C::NBLK, TILE = C::TILE, ST = C::ST;
   // Pairs with P in columns of its own: a thread per side issues its products, where one thread for both held
-  // a side's products back until the other's were due ([4, 4096, 10, 64] 265 -> 252 us, 77 keys
+  // a side's products back until the other's were due ([4, 4096, 10, 64] 266 -> 249 us, 77 keys
   // [4, 1024, 20, 64] 17.7 -> 16.7).  With P in the columns of S that order is what keeps the sides half a step
   // apart (head dim 128: 176 us so, 208 with two threads), and the form with split tiles lost, too
-  // ([1, 8192, 10, 64] 264 and 290).
-  constexpr bool TWO_ISSUERS = !C::ALIAS_P && !SPLIT;
+  // ([1, 8192, 10, 64] 264 and 290); see also one_issues.
+  constexpr bool TWO_ISSUERS = !C::ALIAS_P && !SPLIT && !ONE_ISSUER;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::OFF_BAR);
   uint64_t* q_full = bars;               // [2] by query tile
@@ -779,16 +779,40 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
   if (p.not_first && blockIdx.x == 0) after_previous();
 }
 
+// Whether one thread issues the products of both sides of pairs up to head dim 64.  Where the tiles of a head are
+// odd, a side that has none to itself goes ahead to the next item, and with a ragged key tile the two then
+// keep fetching one another's instructions out: half of the time of a step goes there.  Held together by one
+// thread they do not ([19, 640, 19, 64] over 612 keys 118 us with two, 101 with one; over 640 keys 84 and 90).
+// The more key tiles, the rarer the ragged one, and the more pairs to a head, the rarer the odd tile; four or
+// eight pairs to a head put the shorter items on the same SMs; and over few rounds the sides are never far apart.
+// Two threads against one, us over us, by heads, query tiles and keys: 361, 3 and 172 1.08, 356 1.14, 612 1.15,
+// 868 1.06, 996 1.03; 361, 5 and 172 1.16, 356 1.31, 740 1.11, 996 0.99; 190 (3.9 rounds), 5 and 172 0.99, 356 1.15,
+// 868 0.95; 200, 7 and 300 1.10, 428 0.97; 200, 11 and 356 1.12, 556 1.04, 868 1.00; 100 (4.7), 13 and 356 1.08,
+// 556 1.00; 498 (20), 11 and 708 1.11; 130 (1.8), 3 and 356 0.95.
+static bool one_issues(const AttnParams& p, int Sk) {
+  const int q_tiles = (p.q_rows + ATT_BM - 1) / ATT_BM, n_kt = (Sk + ATT_BN - 1) / ATT_BN;
+  if (p.causal || q_tiles % 2 == 0 || q_tiles == 1 || Sk % ATT_BN == 0) return false;
+  const int pairs = p.q_pairs;
+  const long long tenths = 10ll * pairs * p.H * p.B / attn_sm_count();          // of rounds
+  const int least = tenths >= (pairs == 2 ? 35 : 60) ? 2 : 3;
+  const int most = pairs % 4 == 0 ? 3 : pairs == 2 || tenths >= (pairs <= 5 ? 60 : pairs <= 8 ? 170 : 20 * pairs) ? 7
+                   : pairs <= 5 || tenths >= 80 ? 5 : 3;
+  return tenths >= (pairs == 2 ? 26 : 35) && n_kt >= least && n_kt <= most;
+}
+
 template <typename T, int DP>
 static int launch_fwd_ws(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
-                         const CUtensorMap& to, const AttnParams& p, bool two_launches, cudaStream_t st) {
+                         const CUtensorMap& to, const AttnParams& p, bool two_launches, bool one_issuer,
+                         cudaStream_t st) {
   using C = FwdCfg<DP>;
   const int pairs = p.q_pairs * p.H * p.B, tiles = 2 * (pairs - p.n_pair);
-  static bool done[2][64] = {};
+  static bool done[3][64] = {};
   auto run = [&](const AttnParams& q, bool split, int n) -> int {
     if (n <= 0) return 0;
-    auto kern = split ? attn_fwd_ws_kernel<T, DP, true> : attn_fwd_ws_kernel<T, DP, false>;
-    const int r = set_smem(kern, C::SMEM, done[split]), sms = attn_sm_count();
+    auto kern = split ? attn_fwd_ws_kernel<T, DP, true, false> : attn_fwd_ws_kernel<T, DP, false, false>;
+    const bool one = DP <= 64 && !split && one_issuer;
+    if (one) kern = attn_fwd_ws_kernel<T, DP, false, DP <= 64>;
+    const int r = set_smem(kern, C::SMEM, done[split ? 1 : one ? 2 : 0]), sms = attn_sm_count();
     if (r) return r;
     after(kern, n < sms ? n : sms, C::THREADS, C::SMEM, st)(tq, tk, tv, to, q, n);
     PF_CHECK_LAUNCH();
@@ -880,5 +904,6 @@ PF_API int pf_attn_fwd(const void* q, const void* k, const void* v, void* o, voi
                       (p.q_rows > ATT_BM || Sk > 2 * ATT_BN));
   p.n_pair = split ? pairs - left_over : pairs;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  PF_ATTN_DISPATCH(launch_fwd_ws, tq, tk, tv, to, p, two_launches, st);
+  const bool one_issuer = one_issues(p, Sk);
+  PF_ATTN_DISPATCH(launch_fwd_ws, tq, tk, tv, to, p, two_launches, one_issuer, st);
 }

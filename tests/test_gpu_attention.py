@@ -229,6 +229,26 @@ def test_attention_forward_of_leftover_rows(D, left, causal):
     kx.check_status()
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("Sq,Sk,H,D", [(300, 300, 304, 64), (384, 130, 270, 40), (387, 387, 304, 32), (640, 257, 200, 64),
+                                       (1000, 350, 160, 32), (1300, 800, 420, 64)])
+def test_attention_forward_of_odd_tiles_and_ragged_keys(Sq, Sk, H, D, dtype):
+    """Many heads of an odd number of query tiles, the last key tile ragged: one thread issues the products of both
+    sides of a pair.  Every tile of the first, a middle and the last head against 64 bits."""
+    from pfeife_b200.ops import kernels as kx
+    q = torch.randn(1, Sq, H, D, device="cuda").to(dtype)
+    k, v = (torch.randn(1, Sk, H, D, device="cuda").to(dtype) for _ in range(2))
+    o, lse = kx.attn_fwd(q, k, v, False, D ** -0.5)
+    kx.check_status()
+    for h in (0, H // 2, H - 1):
+        want, lse_want = ref_attn64(*(t[:, :, h:h + 1].double() for t in (q, k, v)), False, D ** -0.5)
+        for r in range(0, Sq, 128):
+            got = o[:, r:r + 128, h:h + 1].double()
+            assert (got - want[:, r:r + 128]).norm() <= 2 * 2.0 ** -8 * want[:, r:r + 128].norm()
+        assert (lse[:, h] - lse_want[:, 0]).abs().max() < 1e-4
+    assert torch.isfinite(o).all()
+
+
 @pytest.mark.parametrize("S,H,D,causal", [(1024, 160, 32, False), (1025, 152, 64, False), (1537, 110, 128, False),
                                           (2050, 58, 64, False), (257, 150, 88, True), (129, 1200, 32, False)])
 def test_attention_forward_of_several_launches(S, H, D, causal):
