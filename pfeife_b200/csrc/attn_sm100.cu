@@ -788,12 +788,16 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 // Two threads against one, us over us, by heads, query tiles and keys: 361, 3 and 172 1.08, 356 1.14, 612 1.15,
 // 868 1.06, 996 1.03; 361, 5 and 172 1.16, 356 1.31, 740 1.11, 996 0.99; 190 (3.9 rounds), 5 and 172 0.99, 356 1.15,
 // 868 0.95; 200, 7 and 300 1.10, 428 0.97; 200, 11 and 356 1.12, 556 1.04, 868 1.00; 100 (4.7), 13 and 356 1.08,
-// 556 1.00; 498 (20), 11 and 708 1.11; 130 (1.8), 3 and 356 0.95.
+// 556 1.00; 498 (20), 11 and 708 1.11; 130 (1.8), 3 and 356 0.95.  Under a causal mask the sides of a pair
+// differ by a masked tile, and over many rounds of long rows they come as far apart: head dim 64, 460 heads of 640
+// 0.90, 896 0.99, 1024 1.08, 1280 1.10, 300 (8.1 rounds) of 931 0.98, 1024 1.02, 150 (5.1) of 1280 1.00; head dim 32,
+// 576 heads of 1024 0.97, 1280 1.03.
 static bool one_issues(const AttnParams& p, int Sk) {
   const int q_tiles = (p.q_rows + ATT_BM - 1) / ATT_BM, n_kt = (Sk + ATT_BN - 1) / ATT_BN;
-  if (p.causal || q_tiles % 2 == 0 || q_tiles == 1 || Sk % ATT_BN == 0) return false;
   const int pairs = p.q_pairs;
   const long long tenths = 10ll * pairs * p.H * p.B / attn_sm_count();          // of rounds
+  if (p.causal) return n_kt >= 8 && n_kt * tenths >= (p.D <= 32 ? 1500 : Sk % ATT_BN ? 900 : 550);
+  if (q_tiles % 2 == 0 || q_tiles == 1 || Sk % ATT_BN == 0) return false;
   const int least = tenths >= (pairs == 2 ? 35 : 60) ? 2 : 3;
   const int most = pairs % 4 == 0 ? 3 : pairs == 2 || tenths >= (pairs <= 5 ? 60 : pairs <= 8 ? 170 : 20 * pairs) ? 7
                    : pairs <= 5 || tenths >= 80 ? 5 : 3;

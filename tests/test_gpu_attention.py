@@ -239,18 +239,19 @@ def test_attention_forward_of_leftover_rows(D, left, causal):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("Sq,Sk,H,D", [(300, 300, 304, 64), (384, 130, 270, 40), (387, 387, 304, 32), (640, 257, 200, 64),
-                                       (1000, 350, 160, 32), (1300, 800, 420, 64)])
-def test_attention_forward_of_odd_tiles_and_ragged_keys(Sq, Sk, H, D, dtype):
-    """Many heads of an odd number of query tiles, the last key tile ragged: one thread issues the products of both
-    sides of a pair.  Every tile of the first, a middle and the last head against 64 bits."""
+@pytest.mark.parametrize("Sq,Sk,H,D,causal", [
+    (300, 300, 304, 64, False), (384, 130, 270, 40, False), (387, 387, 304, 32, False), (640, 257, 200, 64, False),
+    (1000, 350, 160, 32, False), (1300, 800, 420, 64, False), (1024, 1024, 420, 48, True), (1153, 1153, 470, 32, True)])
+def test_attention_forward_of_one_issuing_thread(Sq, Sk, H, D, causal, dtype):
+    """Many heads of an odd number of query tiles, the last key tile ragged, or of long rows under a causal mask:
+    one thread issues the products of both sides of a pair.  Every tile of the first, a middle and the last head against 64 bits."""
     from pfeife_b200.ops import kernels as kx
     q = torch.randn(1, Sq, H, D, device="cuda").to(dtype)
     k, v = (torch.randn(1, Sk, H, D, device="cuda").to(dtype) for _ in range(2))
-    o, lse = kx.attn_fwd(q, k, v, False, D ** -0.5)
+    o, lse = kx.attn_fwd(q, k, v, causal, D ** -0.5)
     kx.check_status()
     for h in (0, H // 2, H - 1):
-        want, lse_want = ref_attn64(*(t[:, :, h:h + 1].double() for t in (q, k, v)), False, D ** -0.5)
+        want, lse_want = ref_attn64(*(t[:, :, h:h + 1].double() for t in (q, k, v)), causal, D ** -0.5)
         for r in range(0, Sq, 128):
             got = o[:, r:r + 128, h:h + 1].double()
             assert (got - want[:, r:r + 128]).norm() <= 2 * 2.0 ** -8 * want[:, r:r + 128].norm()
