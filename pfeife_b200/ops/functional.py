@@ -317,13 +317,19 @@ def _plain_call(args) -> int:
 
 def _native_call(name: str, *args):
     """The op's outputs where csrc/eager.cpp takes the call, else None (and the call goes on here): plain
-    CUDA tensors of one 16-bit type, without autocast and with nothing that observes ops.  Nothing is
-    loaded for a first tensor elsewhere: CPU calls need no library, and a forked child may make them."""
-    x = args[0]
-    if _is_compiling() or (type(x) is not Tensor and type(x) is not _Parameter) or not x.is_cuda:
+    CUDA tensors of one 16-bit type, without autocast and with nothing that observes ops.  The module is not
+    looked for before a first tensor on CUDA: CPU calls need no library, and a forked child may make them."""
+    if _is_compiling():
         return None
-    module = _lib.eager()
-    return None if module is None else getattr(module, name)(*args)
+    module = _lib._eager
+    if module is None:
+        x = args[0]
+        if (type(x) is not Tensor and type(x) is not _Parameter) or not x.is_cuda:
+            return None
+        module = _lib.eager()
+        if module is None:
+            return None
+    return getattr(module, name)(*args)
 
 
 def _native_layer(name: str, *args):
