@@ -106,22 +106,22 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) 
         objs_cpp.append(obj)
         if force or _stale(obj, [src] + headers):
             jobs.append(["g++", *CXX_FLAGS, "-I", str(CSRC), "-c", str(src), "-o", str(obj)])
-    if jobs:
-        with cf.ThreadPoolExecutor(max_workers=min(8, len(jobs))) as ex:
-            list(ex.map(lambda c: _run(c, verbose or ptxas_info), jobs))
+    include = Path(sysconfig.get_paths()["include"])
+    with cf.ThreadPoolExecutor(max_workers=8) as ex:
+        eager = ex.submit(_build_eager, include, force, verbose)       # the longest, and needs no other
+        list(ex.map(lambda c: _run(c, verbose or ptxas_info), jobs))
+        eager.result()
     if objs_cu and (force or jobs or _stale(KERNEL_LIB, objs_cu)):
         _run([nvcc, "-shared", "-o", str(KERNEL_LIB), *map(str, objs_cu),
               "-gencode", "arch=compute_100a,code=sm_100a"], verbose)
     if objs_cpp and (force or jobs or _stale(HOST_LIB, objs_cpp)):
         _run(["g++", "-shared", "-o", str(HOST_LIB), *map(str, objs_cpp), "-pthread"], verbose)
-    include = Path(sysconfig.get_paths()["include"])
     if not (include / "Python.h").exists():
         CALLS_LIB.unlink(missing_ok=True)      # of another state of the sources, perhaps
         print(f"no Python.h in {include}: {CALLS_LIB.name} is not built, calls go through ctypes")
     elif force or _stale(CALLS_LIB, [CALLS_SRC, CSRC / "api.h"]):
         _run(["g++", *CXX_FLAGS, "-shared", "-I", str(include), "-I", str(CSRC),
               str(CALLS_SRC), "-o", str(CALLS_LIB)], verbose)
-    _build_eager(include, force, verbose)
 
 
 def _build_eager(include: Path, force: bool, verbose: bool) -> None:

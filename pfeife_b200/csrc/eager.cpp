@@ -25,8 +25,8 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/autograd/variable.h>
 #include <torch/csrc/jit/frontend/tracer.h>
-#include <torch/torch.h>
 
 #include <atomic>
 
