@@ -17,8 +17,8 @@ static inline int ew_grid(long long nvec, int sm_count) {
 }
 
 // A gated unit's three or five streams go faster by CTAs of one vector per thread that end and begin than by
-// resident ones that stride over the tensors, whose addresses drift apart: 2048 x 11008 bf16 forward 27.1 ->
-// 24.9 us, backward 41.0 -> 35.5.  One and two streams do not (16 Mi values through GELU 23.2 and 24.2).
+// resident ones that stride over the tensors, whose addresses drift apart: 2048 x 11008 bf16 forward 25.8 ->
+// 23.3 us, backward 39.7 -> 33.9.  One and two streams do not (16 Mi values through GELU 23.2 and 24.2).
 static inline unsigned glu_grid(long long nvec) {
   const long long b = (nvec + EW_THREADS - 1) / EW_THREADS;
   return (unsigned)(b < 1 ? 1 : b > 0x7fffffff ? 0x7fffffff : b);
