@@ -82,10 +82,10 @@ struct AttnBwdParams {
 // and writes 16 bits after the last one: nothing to clear, to add in memory or to convert.
 // DQ_TILE: DQ_DIRECT for a few rows in one tile of either kind.  Its outputs leave by 16-byte stores, whose cost goes
 // by the row, and not through boxes, each of which waits for the one before the last.  us over us with boxes and
-// without, 361 heads: head dim 64, 17 tokens 1.09, 64 1.06, 100 0.98, 128 0.90; head dim 128, 17 1.20, 64 1.05, 77
-// 0.99, 128 0.82; 100 queries of 20 keys 1.07.
+// without, 1200 heads: head dim 64, 17 tokens 1.08, 64 1.03, 100 0.94; head dim 128, 17 1.10, 64 1.05, 77 0.96; 96 heads,
+// which no other item follows: head dim 128, 33 tokens 1.04, 49 0.97, 64 0.92.
 enum DqMode : int { DQ_SUMS = 0, DQ_DIRECT = 1, DQ_WHOLE = 2, DQ_TILE = 3 };
-constexpr int BWD_TILE_ROWS = 192;    // most rows of dQ, dK and dV of DQ_TILE
+constexpr int BWD_TILE_ROWS = 192, BWD_TILE_ROWS_ONCE = 112;   // most rows of dQ, dK and dV of DQ_TILE
 
 // One 8-lane group per (batch, padded query, head): delta = dO . O, statistics, cleared dQ sums.
 template <typename T>
@@ -1113,7 +1113,8 @@ static BwdPlan bwd_plan(int B, int H, int Sq, int Sk, int D, int causal) {
   const long long heads = (long long)B * H, sms = attn_sm_count();
   auto tiles = [](int n) { return (n + ATT_BN - 1) / ATT_BN; };
   BwdPlan g = {bwd_direct(Sq, Sk, causal) ? DQ_DIRECT : DQ_SUMS, 0, tiles(Sk), tiles(Sq), 0, 0};
-  if (g.mode == DQ_DIRECT && g.n_qt == 1 && Sq + 2 * Sk <= BWD_TILE_ROWS) g.mode = DQ_TILE;
+  if (g.mode == DQ_DIRECT && g.n_qt == 1 && Sq + 2 * Sk <= (heads > sms ? BWD_TILE_ROWS : BWD_TILE_ROWS_ONCE))
+    g.mode = DQ_TILE;
   const int dp = (D + 31) / 32 * 32;
   const long long rounds = (heads + sms - 1) / sms, apart = (heads * g.n_kt + sms - 1) / sms;
   if (g.mode == DQ_SUMS && (!causal || Sk >= Sq)) {
